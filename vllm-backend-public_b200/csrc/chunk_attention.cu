@@ -39,30 +39,11 @@
 //                        touches only the keys it sees, wherever it stands; a decode row is a sequence with one query.
 // Sequences are described like everywhere in this library: rows cu_q[i] .. cu_q[i+1]-1, ctx_start[i] cached tokens
 // before them (< 0: padding, output rows are zeroed), block_tables[i, :].
-#include "b2_act.cuh"
+#include "b2_mask.cuh"
 
 namespace {
 
 constexpr int kMaxDvPerLane = 16;                    // dv <= 512
-
-// The keys a query at position `pos` may see, as one compact index range [0, n): first the kept keys lo .. lo+nfirst-1
-// (the sequence's first tokens that lie before the window), then wlo .. pos.  Without a window nfirst = 0 and wlo = lo.
-struct KeySpan {
-    int lo, nfirst, wlo, n;
-    __device__ __forceinline__ int key(int c) const { return c < nfirst ? lo + c : wlo + (c - nfirst); }
-};
-__device__ __forceinline__ KeySpan key_span(int pos, int last, int chunk, int window, int keep_first) {
-    KeySpan s;
-    s.lo = chunk > 0 ? (pos / chunk) * chunk : 0;
-    s.wlo = window > 0 ? max(s.lo, pos - window + 1) : s.lo;
-    s.nfirst = (window > 0 && keep_first > s.lo) ? max(0, min(keep_first, s.wlo) - s.lo) : 0;
-    s.n = s.nfirst + (last - s.wlo + 1);
-    return s;
-}
-// what the masks leave of key j for the query at position i
-__device__ __forceinline__ bool key_visible(int i, int j, int lo_i, int window, int keep_first) {
-    return j <= i && j >= lo_i && (window <= 0 || i - j < window || j < keep_first);
-}
 
 // 1 / rms of all H * dk numbers of q and of all G * dk of k, which lie one after the other at `src` (block-wide)
 template <typename T, int W>
@@ -254,21 +235,6 @@ __global__ void qknorm_cache_kernel(const T* __restrict__ qkv, int64_t qkv_strid
         }
     }
 }
-
-// sigmoid of a score that is already in the exponent of 2
-__device__ __forceinline__ float sigmoid2_f(float x2) { return __fdividef(1.f, 1.f + b2::fast_exp2(-x2)); }
-
-// What happens to a score before its weight is taken, and to a head's output after the values are summed.
-struct HeadShape {
-    float cap;               // > 0: scores become cap * tanh(score / cap)
-    float lambda;            // two maps: output = a1 - lambda * a2 ...
-    float eps, out_scale;    // ... / sqrt(mean(output^2) + eps) * out_scale
-};
-// cap * tanh(s / cap); tanh x = 1 - 2 / (1 + e^2x), whose absolute error (times cap) is that of one fp32 rounding
-__device__ __forceinline__ float cap_score(float s, float cap, float e_scale) {
-    return fmaf(-cap, __fdividef(2.f, 1.f + b2::fast_exp2(s * e_scale)), cap);
-}
-__device__ __forceinline__ float cap_score_exact(float s, float cap) { return cap * tanhf(s / cap); }
 
 template <typename T, bool SIG, int MAPS>
 __global__ void chunk_attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
@@ -1292,21 +1258,36 @@ extern "C" int b2_masked_attention(void* out, const void* q, const void* k_cache
         b2_aligned16(q) && b2_aligned16(k_cache) && b2_aligned16(v_cache) && b2_aligned16(out) && out_stride % 8 == 0) {
         skip_from = kTileMinRows;
         int rc = B2_OK;
-#define B2_TILE_RUN(a, b, SIG, MAPS)                                                                                      \
-    launch_tile<a, b, SIG, MAPS>(q, k_cache, v_cache, block_tables, max_nb, cu_q, ctx_start, n_seq, T, H, G, bs, scale, chunk, \
-                                 window, keep_first, sink, sink_logit, sink_logits, head_bias, gate, gate_stride, hs, out, \
-                                 out_stride, st)
-#define B2_TILE(a, b)                                                                                                     \
+        b2_prompt_args pa{};
+        pa.q0 = q;
+        pa.q0_row = (int64_t)H * maps * dk;
+        pa.q0_head = maps * dk;
+        pa.k0 = k_cache;
+        pa.v = v_cache;
+        pa.block_tables = block_tables;
+        pa.max_nb = max_nb; pa.bs = bs; pa.cu_q = cu_q; pa.ctx_start = ctx_start; pa.n_seq = n_seq; pa.T = T;
+        pa.H = H; pa.G = G; pa.dk0 = pa.dk = dk; pa.dv = dv; pa.maps = maps; pa.min_rows = kTileMinRows;
+        pa.scale = scale; pa.chunk = chunk; pa.window = window; pa.keep_first = keep_first;
+        pa.sink = sink; pa.sink_logit = sink_logit; pa.sink_logits = sink_logits; pa.head_bias = head_bias; pa.sigmoid = sig;
+        pa.cap = softcap; pa.map_lambda = map_lambda; pa.map_eps = map_eps; pa.map_scale = map_scale;
+        pa.gate = gate; pa.gate_stride = gate_stride; pa.out = out; pa.out_stride = out_stride;
+        if (b2_internal_prompt_tc5_ok(pa)) {
+            rc = b2_internal_prompt_tc5(pa, stream);
+        } else {
+#define B2_TILE(a, b, MAPS)                                                                                               \
     if (dk == 16 * a && dv == 16 * b)                                                                                     \
-        rc = sig ? B2_TILE_RUN(a, b, true, 1) : (maps == 2 ? B2_TILE_RUN(a, b, false, 2) : B2_TILE_RUN(a, b, false, 1));
-#define B2_TILE_WIDE(a, b) if (dk == 16 * a && dv == 16 * b) rc = B2_TILE_RUN(a, b, false, 1);
-        B2_TILE(2, 2) B2_TILE(2, 4) B2_TILE(2, 6) B2_TILE(2, 8) B2_TILE(4, 2) B2_TILE(4, 4) B2_TILE(4, 6) B2_TILE(4, 8)
-        B2_TILE(6, 2) B2_TILE(6, 4) B2_TILE(6, 6) B2_TILE(6, 8) B2_TILE(8, 2) B2_TILE(8, 4) B2_TILE(8, 6) B2_TILE(8, 8)
-        B2_TILE_WIDE(2, 12) B2_TILE_WIDE(4, 12) B2_TILE_WIDE(6, 12) B2_TILE_WIDE(8, 12)
-        B2_TILE_WIDE(2, 16) B2_TILE_WIDE(4, 16) B2_TILE_WIDE(6, 16) B2_TILE_WIDE(8, 16)
+        rc = launch_tile<a, b, false, MAPS>(q, k_cache, v_cache, block_tables, max_nb, cu_q, ctx_start, n_seq, T, H, G, bs, scale, \
+                                            chunk, window, keep_first, sink, sink_logit, sink_logits, head_bias, gate, gate_stride, \
+                                            hs, out, out_stride, st);
+            if (maps == 2) {
+                B2_TILE(6, 2, 2) B2_TILE(6, 4, 2) B2_TILE(6, 6, 2) B2_TILE(6, 8, 2)
+                B2_TILE(8, 2, 2) B2_TILE(8, 4, 2) B2_TILE(8, 6, 2) B2_TILE(8, 8, 2)
+            } else {
+                B2_TILE(2, 12, 1) B2_TILE(4, 12, 1) B2_TILE(6, 12, 1) B2_TILE(8, 12, 1)
+                B2_TILE(2, 16, 1) B2_TILE(4, 16, 1) B2_TILE(6, 16, 1) B2_TILE(8, 16, 1)
+            }
 #undef B2_TILE
-#undef B2_TILE_WIDE
-#undef B2_TILE_RUN
+        }
         if (rc != B2_OK) return rc;
     }
     if (act_dtype == B2_ACT_BF16 && dk % 32 == 0 && dk <= 256 && b2_aligned16(q) && b2_aligned16(k_cache) && b2_aligned16(v_cache)) {

@@ -1115,6 +1115,16 @@ extern "C" int b2_window_attention(void* out, const void* qn, int64_t qn_row, in
     B2_REQUIRE(!gate || !gate_channels || (gate_stride >= (int64_t)H * dv && gate_stride % 2 == 0 &&
                                            reinterpret_cast<uintptr_t>(gate) % 4 == 0), B2_EINVAL,
                "window_attention: a gate per channel needs 4-byte aligned rows of H * dv columns");
+    b2_prompt_args pa{};
+    pa.q0 = qn; pa.q0_row = qn_row; pa.q0_head = qn_head;
+    pa.q1 = qr; pa.q1_row = qr_row; pa.q1_head = qr_head;
+    pa.k0 = kn; pa.k1 = kt; pa.k1_row = kt_row; pa.v = v;
+    pa.cu_k = cu_k; pa.k_lo = k_lo; pa.cu_q = cu_q; pa.ctx_start = ctx_start; pa.n_seq = n_seq; pa.T = T;
+    pa.H = pa.G = H; pa.bs = 1; pa.dk0 = dn; pa.dk = dn + dr; pa.dv = dv; pa.maps = 1; pa.min_rows = 1;
+    pa.scale = scale; pa.window = window;
+    pa.sink = sink_logits ? 1.f : 0.f; pa.sink_logits = sink_logits;
+    pa.gate = gate; pa.gate_stride = gate_stride; pa.gate_channels = gate_channels; pa.out = out; pa.out_stride = out_stride;
+    if (b2_internal_prompt_tc5_ok(pa)) return b2_internal_prompt_tc5(pa, stream);
     const size_t smem = (size_t)((kWQ + kWK) * (dn + dr + 8) + kWK * (dv + 8)) * sizeof(__nv_bfloat16);
     B2_REQUIRE(smem <= 200 * 1024, B2_EUNSUPPORTED, "window_attention: key size %d too large", dn + dr);
     if (smem > 48 * 1024)
