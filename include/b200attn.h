@@ -521,6 +521,14 @@ B2_API int b2_channel_scan(const float* qkv, const float* beta /* NULL without d
                            int H, int G, int dk, int dv, int decay_per_channel, int delta, const int32_t* cu_q,
                            const int32_t* ctx_start, const int32_t* state_slot, int n_seq, float* state, float* o,
                            void* stream);
+/* The same with fp32 scratch from the caller: b2_channel_scan_workspace floats (0: none is used) let prompts run in chunks of 32
+ * or 64 tokens -- a few products per chunk instead of a chain of tokens -- without it (NULL, or too small) the call is
+ * b2_channel_scan.  The results are the same recurrence summed in another order. */
+B2_API int64_t b2_channel_scan_workspace(int total_rows, int n_seq, int H, int dk, int dv, int decay_per_channel, int delta);
+B2_API int b2_channel_scan_ws(const float* qkv, const float* beta, const float* decay, int total_rows, int H, int G, int dk, int dv,
+                              int decay_per_channel, int delta, const int32_t* cu_q, const int32_t* ctx_start,
+                              const int32_t* state_slot, int n_seq, float* state, float* o, float* workspace,
+                              int64_t workspace_floats, void* stream);
 B2_API int b2_gated_head_norm(const float* o, const void* gate, int64_t gate_stride, int gate_kind, int act_dtype, int T,
                               int H, int dv, const float* norm_w /* or NULL */, float eps, float out_scale, void* out,
                               int64_t out_stride, void* stream);

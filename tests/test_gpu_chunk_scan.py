@@ -1,0 +1,94 @@
+"""The chunked form of the recurrence scan (b2_channel_scan_ws) against fp64 and against the token-by-token scan it stands in for:
+portions around a chunk's edge, several sequences with and without context, padding and stateless sequences, head sizes with
+remainders, grouped keys, decays of one, of zero and so strong that a chunk's product underflows.
+
+Tolerance: both forms sum dk + (tokens that still count) products in fp32, so their error is a small multiple of 2^-24 of the sums of
+absolute values; the chunked one may be twice the other's (other orders) and both stay below 2e-6 of the result's norm, the delta
+correction on unit keys included."""
+import pytest
+import torch
+
+from b200attn import _lib, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(cuda, lens, H, G, dk, dv, per_channel, delta, decay, seed):
+    g = torch.Generator(device=cuda).manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=cuda)           # noqa: E731
+    uni = lambda *s: torch.rand(*s, generator=g, device=cuda)            # noqa: E731
+    T = sum(lens)
+    q, k, v = rnd(T, G, dk), rnd(T, G, dk), rnd(T, H, dv)
+    if delta:
+        q, k = (x / (x.square().sum(-1, keepdim=True) + 1e-6).sqrt() for x in (q, k))
+    wide = H * dk if per_channel else H
+    dec = {"mild": 1.0 - 0.1 * uni(T, wide), "one": torch.ones(T, wide, device=cuda), "strong": torch.exp(-20.0 * uni(T, wide)),
+           "zero": (uni(T, wide) > 0.1).float() * 0.97}[decay].contiguous()
+    qkv = torch.cat([q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1)], 1).contiguous()
+    beta = torch.sigmoid(rnd(T, H)) if delta else None
+    state = rnd(len(lens) + 1, H, dk, dv)
+    return qkv, beta, dec, state
+
+
+def _reference(qkv, beta, dec, state, lens, ctx, slots, H, G, dk, dv):
+    T = qkv.shape[0]
+    x = qkv.double()
+    q = x[:, :G * dk].view(T, G, dk).repeat_interleave(H // G, 1)
+    k = x[:, G * dk:2 * G * dk].view(T, G, dk).repeat_interleave(H // G, 1)
+    v = x[:, 2 * G * dk:].view(T, H, dv)
+    d = dec.double().view(T, H, -1)
+    out, st = torch.zeros(T, H, dv, dtype=torch.float64, device=qkv.device), state.double().clone()
+    at = 0
+    for n, c, s in zip(lens, ctx, slots):
+        if c >= 0:
+            S = st[s].clone() if s >= 0 and c > 0 else torch.zeros(H, dk, dv, dtype=torch.float64, device=qkv.device)
+            for t in range(at, at + n):
+                S = S * d[t][..., None]
+                u = v[t] if beta is None else beta[t].double()[:, None] * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))
+                S = S + k[t][..., None] * u[:, None, :]
+                out[t] = torch.einsum("hkv,hk->hv", S, q[t])
+            if s >= 0:
+                st[s] = S
+        at += n
+    return out, st
+
+
+@pytest.mark.parametrize("delta,per_channel", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("lens,ctx,slots,H,G,dk,dv,decay", [
+    ([200], [0], [0], 2, 2, 128, 128, "mild"),
+    ([31, 32, 33], [0, 7, 3], [0, 1, 2], 3, 3, 64, 20, "mild"),
+    ([63, 64, 65, 129], [5, 0, 9, 2], [3, 0, 1, 2], 4, 2, 128, 48, "mild"),
+    ([1, 300, 2], [40, 0, 6], [1, 0, 2], 2, 1, 96, 16, "mild"),
+    ([100, 50], [-1, 4], [0, 1], 2, 2, 32, 32, "mild"),                  # a padding sequence
+    ([90, 70], [3, 0], [-1, 1], 2, 2, 20, 36, "one"),                    # a sequence without state; sizes with remainders
+    ([257], [8], [1], 2, 2, 128, 64, "strong"),                          # products of a chunk far below the smallest float
+    ([140], [8], [0], 3, 3, 4, 4, "zero"),
+])
+def test_chunked_scan(cuda, lens, ctx, slots, H, G, dk, dv, decay, delta, per_channel):
+    qkv, beta, dec, state = _inputs(cuda, lens, H, G, dk, dv, per_channel, delta, decay, seed=len(lens) * 100 + dk + dv)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    T, cu = qkv.shape[0], [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    batch = ops.SeqBatch(i32(cu), i32(ctx), None, i32(slots), len(lens), T)
+    lib = _lib.load()
+    assert lib.b2_channel_scan_workspace(T, len(lens), H, dk, dv, int(per_channel), int(delta)) > 0, "these sizes are meant for chunks"
+    st_new, st_old = state.clone(), state.clone()
+    new = ops.channel_scan(qkv, beta, dec, H, G, dk, dv, batch, st_new, delta=delta)
+    old = torch.zeros(T, H, dv, device=cuda)
+    _lib.check(lib.b2_channel_scan(qkv.data_ptr(), beta.data_ptr() if delta else None, dec.data_ptr(), T, H, G, dk, dv, int(per_channel),
+                                   int(delta), batch.cu_q.data_ptr(), batch.ctx_start.data_ptr(), batch.state_slots.data_ptr(), len(lens),
+                                   st_old.data_ptr(), old.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    ref, st_ref = _reference(qkv, beta, dec, state, lens, ctx, slots, H, G, dk, dv)
+    rows = torch.cat([torch.arange(cu[i], cu[i + 1], device=cuda) for i in range(len(lens)) if ctx[i] >= 0])
+    for a, b, r in ((new[rows], old[rows], ref[rows]), (st_new, st_old, st_ref)):
+        e_new, e_old = (float((x.double() - r).norm() / r.norm()) for x in (a, b))
+        assert e_new < 2e-6 and e_new <= 2.0 * e_old + 1e-7, (e_new, e_old)
+
+
+def test_chunked_scan_leaves_short_portions_to_the_token_scan():
+    lib = _lib.load()
+    assert lib.b2_channel_scan_workspace(64, 64, 16, 128, 128, 0, 1) == 0
+    assert lib.b2_channel_scan_workspace(4096, 1, 16, 256, 128, 0, 1) == 0
+    assert lib.b2_channel_scan_workspace(4096, 1, 16, 126, 128, 0, 1) == 0
+    assert lib.b2_channel_scan_workspace(0, 1, 16, 128, 128, 0, 1) == 0

@@ -118,6 +118,8 @@ SIGNATURES = {
     "b2_recur_prep": (i32, [vp, i64, i32, i32, i32, i32, i32, i32, i32, vp, i32, i32, f32, f32, f32, vp, i32, i32, i32, i32, i32, i32,
                             vp, i64, vp, vp, f32, vp, vp, vp, i32, vp, vp, vp, vp, vp]),
     "b2_channel_scan": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp, i32, vp, vp, vp]),
+    "b2_channel_scan_workspace": (i64, [i32, i32, i32, i32, i32, i32, i32]),
+    "b2_channel_scan_ws": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp, i32, vp, vp, vp, i64, vp]),
     "b2_gated_head_norm": (i32, [vp, vp, i64, i32, i32, i32, i32, i32, vp, f32, f32, vp, i64, vp]),
     "b2_qk_prep_cache": (i32, [vp, i64, i32, i32, i32, i32, i32, i32, i32, vp, vp, f32, vp, f32, i32, vp, i32, vp, vp, vp, vp]),
     "b2_qknorm_cache": (i32, [vp, i64, i32, i32, i32, i32, i32, i32, vp, vp, f32, vp, i32, vp, vp, vp, vp]),

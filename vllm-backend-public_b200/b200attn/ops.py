@@ -806,9 +806,18 @@ def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, H: in
     _f32(qkv, "qkv", (T, 2 * G * dk + H * dv)), _f32(beta, "beta", (T, H)), _f32(decay, "decay", (T, H))
     if state.dtype != torch.float32 or not state.is_contiguous() or tuple(state.shape[1:]) != (H, dk, dv):
         raise ValueError(f"state must be contiguous fp32 [slots, {H}, {dk}, {dv}]")
+    return _scan(lib, dev, qkv, beta, decay, T, H, G, dk, dv, False, True, batch, state)
+
+
+def _scan(lib, dev, qkv, beta, decay, T: int, H: int, G: int, dk: int, dv: int, per_channel: bool, delta: bool, batch: SeqBatch,
+          state: torch.Tensor) -> torch.Tensor:
+    """b2_channel_scan_ws: prompts run in chunks, for which the call wants fp32 scratch."""
     o = torch.empty(T, H, dv, dtype=torch.float32, device=dev)
-    _lib.check(lib.b2_delta_scan(_ptr(qkv), _ptr(beta), _ptr(decay), T, H, G, dk, dv, _ptr(batch.cu_q), _ptr(batch.ctx_start),
-                                 _ptr(batch.state_slots), batch.n_seq, _ptr(state), _ptr(o), _stream(dev)))
+    nws = lib.b2_channel_scan_workspace(T, batch.n_seq, H, dk, dv, int(per_channel), int(delta))
+    ws = torch.empty(nws, dtype=torch.float32, device=dev) if nws else None
+    _lib.check(lib.b2_channel_scan_ws(_ptr(qkv), _ptr(beta), _ptr(decay), T, H, G, dk, dv, int(per_channel), int(delta), _ptr(batch.cu_q),
+                                      _ptr(batch.ctx_start), _ptr(batch.state_slots), batch.n_seq, _ptr(state), _ptr(o), _ptr(ws), nws,
+                                      _stream(dev)))
     return o
 
 
@@ -1199,11 +1208,7 @@ def channel_scan(qkv: torch.Tensor, beta: Optional[torch.Tensor], decay: torch.T
     per_channel = tuple(decay.shape) == (T, H * dk) and dk > 1
     if state.dtype != torch.float32 or not state.is_contiguous() or tuple(state.shape[1:]) != (H, dk, dv):
         raise ValueError(f"state must be contiguous fp32 [slots, {H}, {dk}, {dv}]")
-    o = torch.empty(T, H, dv, dtype=torch.float32, device=dev)
-    _lib.check(lib.b2_channel_scan(_ptr(qkv), _ptr(beta) if delta else None, _ptr(decay), T, H, G, dk, dv, int(per_channel),
-                                   int(delta), _ptr(batch.cu_q), _ptr(batch.ctx_start), _ptr(batch.state_slots), batch.n_seq,
-                                   _ptr(state), _ptr(o), _stream(dev)))
-    return o
+    return _scan(lib, dev, qkv, beta if delta else None, decay, T, H, G, dk, dv, per_channel, delta, batch, state)
 
 
 def gated_head_norm(o: torch.Tensor, gate: torch.Tensor, norm_w: Optional[torch.Tensor], eps: float, gate_kind: int = GATE_SILU,

@@ -608,12 +608,31 @@ extern "C" int b2_delta_scan(const float* qkv, const float* beta, const float* d
 extern "C" int b2_channel_scan(const float* qkv, const float* beta, const float* decay, int total_rows, int H, int G, int dk,
                                int dv, int decay_per_channel, int delta, const int32_t* cu_q, const int32_t* ctx_start,
                                const int32_t* state_slot, int n_seq, float* state, float* o, void* stream) {
+    return b2_channel_scan_ws(qkv, beta, decay, total_rows, H, G, dk, dv, decay_per_channel, delta, cu_q, ctx_start, state_slot, n_seq,
+                              state, o, nullptr, 0, stream);
+}
+
+// fp32 scratch (in floats) with which b2_channel_scan_ws takes the chunked form for these sizes; 0: it needs none
+extern "C" int64_t b2_channel_scan_workspace(int total_rows, int n_seq, int H, int dk, int dv, int decay_per_channel, int delta) {
+    if (total_rows <= 0 || n_seq <= 0 || H <= 0 || dk <= 0 || dv <= 0) return 0;
+    return b2_internal_chunk_scan_floats(total_rows, n_seq, H, dk, dv, decay_per_channel != 0, delta != 0);
+}
+
+extern "C" int b2_channel_scan_ws(const float* qkv, const float* beta, const float* decay, int total_rows, int H, int G, int dk,
+                                  int dv, int decay_per_channel, int delta, const int32_t* cu_q, const int32_t* ctx_start,
+                                  const int32_t* state_slot, int n_seq, float* state, float* o, float* workspace,
+                                  int64_t workspace_floats, void* stream) {
     B2_REQUIRE(H > 0 && G > 0 && H % G == 0 && dk > 0 && dv > 0, B2_EINVAL, "recurrence scan: bad sizes");
     B2_REQUIRE(dk <= 512, B2_EUNSUPPORTED, "recurrence scan: key size %d above 512", dk);
     if (n_seq == 0) return B2_OK;
     B2_REQUIRE(qkv && decay && cu_q && ctx_start && state_slot && state && o && (beta || !delta), B2_EINVAL,
                "recurrence scan: null pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int64_t need = workspace ? b2_channel_scan_workspace(total_rows, n_seq, H, dk, dv, decay_per_channel, delta) : 0;
+    if (need > 0 && workspace_floats >= need && b2_aligned16(qkv) && b2_aligned16(state) && b2_aligned16(o) && b2_aligned16(workspace) &&
+        (!decay_per_channel || b2_aligned16(decay)))
+        return b2_internal_chunk_scan(qkv, beta, decay, total_rows, H, G, dk, dv, decay_per_channel != 0, delta != 0, cu_q, ctx_start,
+                                      state_slot, n_seq, state, o, workspace, stream);
 #define B2_SCAN_ARGS qkv, beta, decay, total_rows, H, G, dk, dv, cu_q, ctx_start, state_slot, n_seq, state, o, st
     if (decay_per_channel) return delta ? launch_scan<true, true>(B2_SCAN_ARGS) : launch_scan<true, false>(B2_SCAN_ARGS);
     return delta ? launch_scan<false, true>(B2_SCAN_ARGS) : launch_scan<false, false>(B2_SCAN_ARGS);
