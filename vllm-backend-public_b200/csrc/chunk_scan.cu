@@ -1,34 +1,45 @@
 // chunk_scan.cu -- the scan of delta_rule.cu for prompts: S <- g S, u = beta (v - S^T k) (or u = v), S <- S + k u^T, o = S^T q, in
-// chunks of C tokens instead of token after token, everything in fp32 on the FMA pipe.
+// chunks of 64 tokens instead of token after token, everything in fp32 on the FMA pipe.
 //
 // With G_t the product of the chunk's decays up to token t (per head, or per key channel), S_0 the state before the chunk and
-// every ratio G_t / G_s taken as the product g_{s+1} .. g_t (numbers in [0, 1] are only ever multiplied, nothing is divided by a
-// product that may have underflowed):
+// every ratio G_t / G_s taken as the product g_{s+1} .. g_t (decays are only ever multiplied, nothing is divided by a product that
+// may have underflowed):
 //   A[t, s] = beta_t sum_i k_t k_s G_t/G_s  (s < t),    T = (I + A)^-1 diag(beta),     P[t, s] = sum_i q_t k_s G_t/G_s  (s <= t)
-//   R = V - (G K) S_0,   U = T R  (no delta: U = V),   O = (G Q) S_0 + P U,   S = G_C S_0 + (G_C/G K)^T U
-// which is the same recurrence, summed in another order (the WY form of Yang et al., "Parallelizing linear transformers with the
-// delta rule over sequence length", 2024).  Two kernels:
-//   chunk_prep_kernel   A, T, P and the decay products: a CTA per (chunk, head), all chunks at once, into the caller's scratch
-//   chunk_scan_kernel   the chain over a sequence's chunks: a CTA per (sequence, head, 16 columns of S), the next chunk's operands
-//                       in flight by cp.async; three products per chunk of [2C x dk][dk x 16], [C x C][C x 16], [dk x C][C x 16]
-// What bounds it: the chain.  A CTA needs C/32 x 0.23 M FMAs a chunk (1.8k cycles of its SM for C = 32), plus a few barriers; the
-// token-by-token scan it replaces waited 200 - 400 cycles a token for shuffles and shared memory whatever the shape.  Sixteen columns
-// a CTA fill the chip with one sequence of 16 heads of 128; wider slices would halve the reads of K and Q but leave SMs idle.
-// C = 64 without delta and with a decay per head (half the barriers), else 32 (T is C x C and the products per channel cost C dk).
+//   U = T (V - (G K) S_0)   (no delta: U = V),   S = G_C S_0 + (G_C/G K)^T U,   O = (G Q) S_0 + P U
+// which is the same recurrence summed in another order (the WY form of Yang et al., "Parallelizing linear transformers with the
+// delta rule over sequence length", 2024).  Three kernels, only the second of which is a chain:
+//   chunk_prep_kernel    P, T and the decay products; without delta also F = (G_C/G K)^T V: a CTA per (chunk, head)
+//   chunk_state_kernel   without delta: S <- G_C S + F over the chunks, element by element (memory bound)
+//   chunk_delta_kernel   with delta: U and S over the chunks, a CTA per (sequence, head, 16 columns of S)
+//   chunk_out_kernel     O of every chunk from its S_0: a CTA per (chunk, head, 128 columns)
+// What bounds them: the first and last are products on the FMA pipe with 8 x 8 / 4 x 8 tiles a thread (shared-memory reads cost
+// about 0.7 of the FMA cycles); the delta chain is a chain of 64-token steps of [64 x dk][dk x 16], [64 x 64][64 x 16] and
+// [dk x 64][64 x 16], bound by shared-memory reads and their latency.  Sixteen columns a CTA fill the chip with one sequence of 16
+// heads of 128.  The scan token by token waited 200 - 400 cycles a token for shuffles and shared memory whatever the shape.
 #include "b2_act.cuh"
 
 namespace {
 
-constexpr int NC = 16, NT = 256;
+constexpr int C = 64, NC = 16, NT = 256, JB = 128, LP = C + 4;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(b2::smem_u32(dst)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// floats of scratch per (chunk, head): P | T | decay products
-__host__ __device__ constexpr int scratch_floats(int C, int dk, bool ch, bool delta) {
-    return C * C * (delta ? 2 : 1) + (ch ? 3 * C * dk + dk : 2 * C);
-}
+// Scratch of one (chunk, head), in floats: P | T (delta) | products | S_0 (first F) | U (delta)
+struct Scratch {
+    int t, dec, s0, u, total;
+    __host__ __device__ Scratch(int dk, int dv, bool ch, bool delta) {
+        t = C * C;
+        dec = t + (delta ? C * C : 0);
+        s0 = dec + (ch ? 3 * C * dk + dk : 2 * C);   // per channel: G K | G Q | G_C/G K | G_C; per head: G | G_C/G
+        u = s0 + dk * dv;
+        total = u + (delta ? C * dv : 0);
+    }
+};
 
 struct ChunkArgs {
     const float *qkv, *beta, *decay;
@@ -37,43 +48,57 @@ struct ChunkArgs {
     float *state, *o, *ws;
 };
 
+// chunk number -> first batch row and number of rows (row < 0: a spare CTA)
+__device__ __forceinline__ void find_chunk(const ChunkArgs& a, int want, int* at) {
+    at[0] = -1;
+    for (int s = 0; s < a.n_seq; ++s) {
+        if (a.ctx_start[s] < 0) continue;
+        const int len = a.cu_q[s + 1] - a.cu_q[s], nc = (len + C - 1) / C;
+        if (want < nc) {
+            at[0] = a.cu_q[s] + want * C;
+            at[1] = min(C, len - want * C);
+            return;
+        }
+        want -= nc;
+    }
+}
+__device__ __forceinline__ int first_chunk(const ChunkArgs& a, int seq) {
+    int base = 0;
+    for (int s = 0; s < seq; ++s)
+        if (a.ctx_start[s] >= 0) base += (a.cu_q[s + 1] - a.cu_q[s] + C - 1) / C;
+    return base;
+}
+__device__ __forceinline__ void fma4(float (&acc)[4], float x, const float4& y) {
+    acc[0] = fmaf(x, y.x, acc[0]);
+    acc[1] = fmaf(x, y.y, acc[1]);
+    acc[2] = fmaf(x, y.z, acc[2]);
+    acc[3] = fmaf(x, y.w, acc[3]);
+}
+__device__ __forceinline__ float4 scaled(const float4& v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); }
+
 // ---------------------------------------------------------------------------------------------------------------- prep
-template <int C, bool CH, bool DELTA>
+template <bool CH, bool DELTA>
 __global__ void __launch_bounds__(NT)
 chunk_prep_kernel(const ChunkArgs a) {
     extern __shared__ __align__(16) float sm[];
-    __shared__ int s_at[3];
+    __shared__ int s_at[2];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, hh = blockIdx.y;
-    const int dk = a.dk, LD = dk + 4;
-    if (tid == 0) {
-        int want = blockIdx.x;
-        s_at[0] = -1;
-        for (int s = 0; s < a.n_seq; ++s) {
-            if (a.ctx_start[s] < 0) continue;
-            const int len = a.cu_q[s + 1] - a.cu_q[s], nc = (len + C - 1) / C;
-            if (want < nc) {
-                s_at[0] = a.cu_q[s] + want * C;
-                s_at[1] = min(C, len - want * C);
-                break;
-            }
-            want -= nc;
-        }
-    }
+    const int dk = a.dk, dv = a.dv, LD = dk + 4, per = dk / 4;
+    if (tid == 0) find_chunk(a, blockIdx.x, s_at);
     __syncthreads();
     const int r0 = s_at[0], nt = s_at[1];
     if (r0 < 0) return;
     float* ks = sm;                                  // [C][LD]
-    float* qs = ks + C * LD;                         // [C][LD]
-    float* As = qs + C * LD;                         // [C][C + 1]
-    float* Ps = As + C * (C + 1);                    // [C][C + 1]
-    float* gs = Ps + C * (C + 1);                    // [C], CH: [C][LD]
-    float* bs = gs + (CH ? C * LD : C);              // [C]
-    const int Cq = 2 * a.G * dk + a.H * a.dv, kvh = hh / (a.H / a.G);
+    float* qs = ks + C * LD;                         // [C][LD]; later (no delta) the columns of V
+    float* Ps = qs + (DELTA ? C * LD : max(C * LD, C * JB));        // [C][C + 1]
+    float* As = Ps + C * (C + 1);                    // [C][C + 1] (delta)
+    float* gs = As + (DELTA ? C * (C + 1) : 0);      // [C], per channel [C][LD]
+    float* bs = gs + (CH ? C * LD : C);              // [C] beta; per head without delta: G_C/G
+    const int Cq = 2 * a.G * dk + a.H * dv, kvh = hh / (a.H / a.G);
     const float* qrow = a.qkv + (size_t)r0 * Cq + (size_t)kvh * dk;
     const float* krow = qrow + (size_t)a.G * dk;
-    const int per = dk / 4;
     for (int idx = tid; idx < C * per; idx += NT) {
-        const int t = idx / per, c = (idx % per) * 4;
+        const int t = idx / per, c = (idx - t * per) * 4;
         float4 k = make_float4(0.f, 0.f, 0.f, 0.f), q = k, g = make_float4(1.f, 1.f, 1.f, 1.f);
         if (t < nt) {
             k = *reinterpret_cast<const float4*>(krow + (size_t)t * Cq + c);
@@ -88,17 +113,23 @@ chunk_prep_kernel(const ChunkArgs a) {
         if (!CH) gs[tid] = tid < nt ? a.decay[(size_t)(r0 + tid) * a.H + hh] : 1.f;
         if (DELTA) bs[tid] = tid < nt ? a.beta[(size_t)(r0 + tid) * a.H + hh] : 0.f;
     }
-    float* out = a.ws + ((size_t)blockIdx.x * a.H + hh) * scratch_floats(C, dk, CH, DELTA);
-    float* dec = out + C * C * (DELTA ? 2 : 1);
+    const Scratch sc(dk, dv, CH, DELTA);
+    float* out = a.ws + ((size_t)blockIdx.x * a.H + hh) * sc.total;
+    float* dec = out + sc.dec;
     __syncthreads();
+    // sums over dk of rows x (q, and with delta k) times columns k_s: 16 x 16 threads, rows rg + 16 rr, columns cg + 16 cc
+    const int rg = tid >> 4, cg = tid & 15;
     if (CH) {
-        // a warp per column s: k_s times the running product of the decays, dotted with every later row
+        // inside a half of 32 tokens a warp takes a column s: k_s times the running product of the decays, dotted with every later row
         for (int s = wid; s < C; s += NT / 32) {
             float w[4];
 #pragma unroll
             for (int m = 0; m < 4; ++m) w[m] = lane + 32 * m < dk ? ks[s * LD + lane + 32 * m] : 0.f;
-            if (lane < s) Ps[lane * (C + 1) + s] = As[lane * (C + 1) + s] = 0.f;         // C = 32: one lane a row above the diagonal
-            for (int t = s; t < C; ++t) {
+            for (int t = lane; t < s; t += 32) {
+                Ps[t * (C + 1) + s] = 0.f;
+                if (DELTA) As[t * (C + 1) + s] = 0.f;
+            }
+            for (int t = s; t < (s < 32 ? 32 : C); ++t) {
                 float dq = 0.f, dd = 0.f;
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
@@ -122,22 +153,74 @@ chunk_prep_kernel(const ChunkArgs a) {
                 }
             }
         }
-        // decayed copies of the rows: from the chunk's start (k, q) and to its end (k); the whole chunk's product
+        __syncthreads();
+        // across the halves: rows 32 .. 63 decayed from the boundary, columns 0 .. 31 decayed to it, then a plain product; the copies
+        // for the chain are written on the way
         const int i = tid & 127;
         if (i < dk) {
-            float run = 1.f;
             if (tid < 128) {
-                for (int t = 0; t < C; ++t) {
+                float run = 1.f;
+                for (int t = 0; t < 32; ++t) {
                     run *= gs[t * LD + i];
                     dec[t * dk + i] = run * ks[t * LD + i];
                     dec[(C + t) * dk + i] = run * qs[t * LD + i];
                 }
-                dec[3 * C * dk + i] = run;
-            } else {
-                for (int t = C - 1; t >= 0; --t) {
-                    dec[(2 * C + t) * dk + i] = run * ks[t * LD + i];
-                    run *= gs[t * LD + i];
+                float half = 1.f;
+                for (int t = 32; t < C; ++t) {
+                    half *= gs[t * LD + i];
+                    const float k = half * ks[t * LD + i], q = half * qs[t * LD + i];
+                    dec[t * dk + i] = run * k;
+                    dec[(C + t) * dk + i] = run * q;
+                    qs[t * LD + i] = q;              // this thread's channel: nobody else reads it before the barrier
                 }
+                dec[3 * C * dk + i] = run * half;
+            }
+        }
+        __syncthreads();                             // the later half's keys are still as they came: their copy to the chunk's end
+        if (i < dk && tid >= 128) {
+            float run = 1.f;
+            for (int t = C - 1; t >= 32; --t) {
+                const float k = ks[t * LD + i], g = gs[t * LD + i];
+                dec[(2 * C + t) * dk + i] = run * k;
+                run *= g;
+            }
+            float half = 1.f;
+            for (int t = 31; t >= 0; --t) {
+                const float k = half * ks[t * LD + i];
+                dec[(2 * C + t) * dk + i] = run * k;
+                ks[t * LD + i] = k;
+                half *= gs[t * LD + i];
+            }
+            if (DELTA) {                             // keys 32 .. 63 decayed from the boundary
+                float from = 1.f;
+                for (int t = 32; t < C; ++t) {
+                    from *= gs[t * LD + i];
+                    ks[t * LD + i] *= from;
+                }
+            }
+        }
+        __syncthreads();
+        float acc[DELTA ? 4 : 2][2];
+#pragma unroll
+        for (int r = 0; r < (DELTA ? 4 : 2); ++r) acc[r][0] = acc[r][1] = 0.f;
+        for (int x = 0; x < dk; x += 4) {
+            const float4 k0 = *reinterpret_cast<const float4*>(ks + cg * LD + x), k1 = *reinterpret_cast<const float4*>(ks + (cg + 16) * LD + x);
+#pragma unroll
+            for (int r = 0; r < (DELTA ? 4 : 2); ++r) {
+                const float4 v = *reinterpret_cast<const float4*>((r < 2 ? qs : ks) + (32 + rg + 16 * (r & 1)) * LD + x);
+                acc[r][0] = fmaf(v.x, k0.x, acc[r][0]); acc[r][0] = fmaf(v.y, k0.y, acc[r][0]);
+                acc[r][0] = fmaf(v.z, k0.z, acc[r][0]); acc[r][0] = fmaf(v.w, k0.w, acc[r][0]);
+                acc[r][1] = fmaf(v.x, k1.x, acc[r][1]); acc[r][1] = fmaf(v.y, k1.y, acc[r][1]);
+                acc[r][1] = fmaf(v.z, k1.z, acc[r][1]); acc[r][1] = fmaf(v.w, k1.w, acc[r][1]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < (DELTA ? 4 : 2); ++r) {
+            const int t = 32 + rg + 16 * (r & 1);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                if (r < 2) Ps[t * (C + 1) + cg + 16 * c] = acc[r][c];
+                else As[t * (C + 1) + cg + 16 * c] = bs[t] * acc[r][c];
             }
         }
     } else {
@@ -150,29 +233,25 @@ chunk_prep_kernel(const ChunkArgs a) {
                 Ps[t * (C + 1) + tid] = run;
             }
             dec[C + tid] = run;
+            if (!DELTA) bs[tid] = run;
             float from = 1.f;
             for (int t = 0; t <= tid; ++t) from *= gs[t];
             dec[tid] = from;
         }
         __syncthreads();
-        // rows (q, and with delta k) against the columns k_s: 16 x 16 threads, rows rg + 16 rr, columns cg + 16 cc
-        constexpr int RR = (DELTA ? 2 : 1) * C / 16, CC = C / 16;
-        const int rg = tid >> 4, cg = tid & 15;
-        float acc[RR][CC];
+        constexpr int RR = DELTA ? 8 : 4;
+        float acc[RR][4];
 #pragma unroll
-        for (int r = 0; r < RR; ++r)
-#pragma unroll
-            for (int c = 0; c < CC; ++c) acc[r][c] = 0.f;
+        for (int r = 0; r < RR; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
         for (int i = 0; i < dk; i += 4) {
-            float4 kc[CC];
+            float4 kc[4];
 #pragma unroll
-            for (int c = 0; c < CC; ++c) kc[c] = *reinterpret_cast<const float4*>(ks + (cg + 16 * c) * LD + i);
+            for (int c = 0; c < 4; ++c) kc[c] = *reinterpret_cast<const float4*>(ks + (cg + 16 * c) * LD + i);
 #pragma unroll
             for (int r = 0; r < RR; ++r) {
-                const int row = rg + 16 * r;         // q rows first, then k rows
-                const float4 x = *reinterpret_cast<const float4*>((row < C ? qs + row * LD : ks + (row - C) * LD) + i);
+                const float4 x = *reinterpret_cast<const float4*>((r < 4 ? qs : ks) + (rg + 16 * (r & 3)) * LD + i);
 #pragma unroll
-                for (int c = 0; c < CC; ++c) {
+                for (int c = 0; c < 4; ++c) {
                     acc[r][c] = fmaf(x.x, kc[c].x, acc[r][c]);
                     acc[r][c] = fmaf(x.y, kc[c].y, acc[r][c]);
                     acc[r][c] = fmaf(x.z, kc[c].z, acc[r][c]);
@@ -181,112 +260,216 @@ chunk_prep_kernel(const ChunkArgs a) {
             }
         }
 #pragma unroll
-        for (int r = RR - 1; r >= 0; --r) {          // the k rows still need the ratios that the q rows overwrite
+        for (int r = RR - 1; r >= 0; --r) {          // the k rows still need the ratios that the q rows overwrite (same thread)
 #pragma unroll
-            for (int c = 0; c < CC; ++c) {
-                const int row = rg + 16 * r, s = cg + 16 * c, t = row < C ? row : row - C;
+            for (int c = 0; c < 4; ++c) {
+                const int t = rg + 16 * (r & 3), s = cg + 16 * c;
                 const float ratio = Ps[t * (C + 1) + s];
-                if (row < C) Ps[t * (C + 1) + s] = acc[r][c] * ratio;                    // 0 above the diagonal
+                if (r < 4) Ps[t * (C + 1) + s] = acc[r][c] * ratio;                      // 0 above the diagonal
                 else As[t * (C + 1) + s] = t > s ? bs[t] * acc[r][c] * ratio : 0.f;
             }
         }
     }
     __syncthreads();
     for (int idx = tid; idx < C * C; idx += NT) out[idx] = Ps[(idx / C) * (C + 1) + idx % C];
-    if (DELTA && wid == 7) {                         // forward substitution, a lane per column of T
-        float T[C];
-        float* to = out + C * C;
+    if (DELTA) {
+        // the inverse of I + A by halves: forward substitution on the diagonal blocks (a warp each, a lane per column), then
+        // T21 = -T22 A21 T11; Ps is free and takes T
+        if (wid >= 6) {
+            const int o = wid == 6 ? 0 : 32;
+            float T[32];
 #pragma unroll
-        for (int t = 0; t < C; ++t) {
-            float v = t == lane ? bs[t] : 0.f;
+            for (int t = 0; t < 32; ++t) {
+                float v = t == lane ? 1.f : 0.f;
 #pragma unroll
-            for (int s = 0; s < t; ++s) v = fmaf(-As[t * (C + 1) + s], T[s], v);
-            T[t] = v;
-            to[t * C + lane] = v;
+                for (int s = 0; s < t; ++s) v = fmaf(-As[(o + t) * (C + 1) + o + s], T[s], v);
+                T[t] = v;
+            }
+            __syncwarp();
+            asm volatile("bar.sync 1, 64;" ::: "memory");            // both warps are done reading A's diagonal blocks ...
+#pragma unroll
+            for (int t = 0; t < 32; ++t) As[(o + t) * (C + 1) + o + lane] = T[t];        // ... whose place T takes
+        }
+        __syncthreads();
+        float* x = Ps;                               // A21 T11, [32][C + 1]
+        const int row = tid >> 3, c4 = (tid & 7) * 4;
+        {
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int s = 0; s < 32; ++s) {
+                const float l = As[(32 + row) * (C + 1) + s];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[c] = fmaf(l, As[s * (C + 1) + c4 + c], v[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) x[row * (C + 1) + c4 + c] = v[c];
+        }
+        __syncthreads();
+        {
+            float v[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int s = 0; s < 32; ++s) {
+                const float l = As[(32 + row) * (C + 1) + 32 + s];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[c] = fmaf(-l, x[s * (C + 1) + c4 + c], v[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) As[(32 + row) * (C + 1) + c4 + c] = v[c];        // A21 was read before the last barrier
+        }
+        __syncthreads();
+        float* to = out + sc.t;
+        for (int idx = tid; idx < C * C; idx += NT) {
+            const int t = idx / C, s = idx % C;
+            to[idx] = s <= t ? As[t * (C + 1) + s] * bs[s] : 0.f;
+        }
+    } else {
+        // F = (G_C/G K)^T V, 128 columns at a time, 8 x 8 results a thread: rows 8 ti .., columns 4 tj .. and 64 + 4 tj ..
+        const int ti = tid >> 4, tj = tid & 15;
+        const float* vrow = a.qkv + (size_t)r0 * Cq + (size_t)2 * a.G * dk + (size_t)hh * dv;
+        float* f0 = out + sc.s0;
+        if (CH) {                                    // the keys decayed to the chunk's end, from where they were just written
+            for (int idx = tid; idx < C * per; idx += NT) {
+                const int t = idx / per, c = (idx - t * per) * 4;
+                *reinterpret_cast<float4*>(ks + t * LD + c) = *reinterpret_cast<const float4*>(dec + (2 * C + t) * dk + c);
+            }
+        }
+        float* vs = qs;
+        for (int j0 = 0; j0 < dv; j0 += JB) {
+            __syncthreads();
+            for (int idx = tid; idx < C * (JB / 4); idx += NT) {
+                const int t = idx / (JB / 4), c = (idx % (JB / 4)) * 4;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (t < nt && j0 + c < dv) v = *reinterpret_cast<const float4*>(vrow + (size_t)t * Cq + j0 + c);
+                *reinterpret_cast<float4*>(vs + t * JB + c) = CH ? v : scaled(v, bs[t]);
+            }
+            __syncthreads();
+            if (ti * 8 < dk) {
+                float acc[8][2][4];
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[r][0][c] = acc[r][1][c] = 0.f;
+                const int hi = min(ti * 8 + 4, dk - 4);              // heads of 4 (mod 8) entries: a second look at the last four
+#pragma unroll 2
+                for (int t = 0; t < C; ++t) {
+                    const float4 x0 = *reinterpret_cast<const float4*>(ks + t * LD + ti * 8), x1 = *reinterpret_cast<const float4*>(ks + t * LD + hi);
+                    const float4 y0 = *reinterpret_cast<const float4*>(vs + t * JB + tj * 4), y1 = *reinterpret_cast<const float4*>(vs + t * JB + 64 + tj * 4);
+                    const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) {
+                        fma4(acc[r][0], x[r], y0);
+                        fma4(acc[r][1], x[r], y1);
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const int i = r < 4 ? ti * 8 + r : hi + r - 4;
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        const int j = j0 + b * 64 + tj * 4;
+                        if (j < dv) *reinterpret_cast<float4*>(f0 + (size_t)i * dv + j) = make_float4(acc[r][b][0], acc[r][b][1], acc[r][b][2], acc[r][b][3]);
+                    }
+                }
+            }
         }
     }
 }
 
-// ---------------------------------------------------------------------------------------------------------------- scan
-template <int C, bool CH, bool DELTA>
-struct ScanSmem {
-    static constexpr int RB = DELTA ? 2 : C / 32;    // 32-row blocks of the product with the state
-    static constexpr int KS = 8 / RB;                // slices of dk, one a warp
-    static constexpr int LP = C + 4;                 // padded rows of P and T
-    static constexpr int VLD = NC;
-    __host__ __device__ static constexpr int stage(int dk) {
-        return (CH ? 3 : 2) * C * (dk + 4) + C * VLD + (DELTA ? 2 : 1) * C * LP + (CH ? dk : 2 * C);
-    }
-    __host__ __device__ static constexpr int fixed(int dk) { return dk * NC + 2 * 8 * 32 * NC + 3 * C * NC; }
-};
-
-template <int C, bool CH, bool DELTA>
+// ---------------------------------------------------------------------------------------------------------------- state, no delta
+template <bool CH>
 __global__ void __launch_bounds__(NT)
-chunk_scan_kernel(const ChunkArgs a, int stages) {
-    using L = ScanSmem<C, CH, DELTA>;
+chunk_state_kernel(const ChunkArgs a) {
+    const int seq = blockIdx.x, hh = blockIdx.y;
+    const int ctx = a.ctx_start[seq];
+    if (ctx < 0) return;
+    const int dk = a.dk, dv = a.dv, e = (blockIdx.z * NT + threadIdx.x) * 4;
+    if (e >= dk * dv) return;
+    const int nchunks = (a.cu_q[seq + 1] - a.cu_q[seq] + C - 1) / C;
+    if (nchunks == 0) return;
+    const Scratch sc(dk, dv, CH, false);
+    const size_t step = (size_t)a.H * sc.total;
+    float* w = a.ws + ((size_t)first_chunk(a, seq) * a.H + hh) * sc.total;
+    const float* g = w + sc.dec + (CH ? 3 * C * dk + e / dv : C - 1);                    // the chunk's whole product
+    float* f = w + sc.s0 + e;
+    const int slot = a.state_slot[seq];
+    float* sp = slot >= 0 ? a.state + ((size_t)slot * a.H + hh) * dk * dv + e : nullptr;
+    float4 s = sp && ctx > 0 ? *reinterpret_cast<const float4*>(sp) : make_float4(0.f, 0.f, 0.f, 0.f);
+    constexpr int AHEAD = 8;                         // loads in flight: they do not depend on the chain
+    for (int c0 = 0; c0 < nchunks; c0 += AHEAD) {
+        float4 x[AHEAD];
+        float d[AHEAD];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+            if (c0 + u < nchunks) {
+                x[u] = *reinterpret_cast<const float4*>(f + (c0 + u) * step);
+                d[u] = g[(c0 + u) * step];
+            }
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+            if (c0 + u < nchunks) {
+                *reinterpret_cast<float4*>(f + (c0 + u) * step) = s;
+                s = make_float4(fmaf(s.x, d[u], x[u].x), fmaf(s.y, d[u], x[u].y), fmaf(s.z, d[u], x[u].z), fmaf(s.w, d[u], x[u].w));
+            }
+    }
+    if (sp) *reinterpret_cast<float4*>(sp) = s;
+}
+
+// ---------------------------------------------------------------------------------------------------------------- state, delta
+__host__ __device__ constexpr int delta_stage(int dk, bool ch) { return (ch ? 2 : 1) * C * (dk + 4) + C * NC + C * LP + (ch ? dk : 2 * C); }
+__host__ __device__ constexpr int delta_fixed(int dk) { return dk * NC + 2 * 4 * C * NC + 2 * C * NC; }
+
+template <bool CH>
+__global__ void __launch_bounds__(NT)
+chunk_delta_kernel(const ChunkArgs a, int stages) {
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int seq = blockIdx.x, hh = blockIdx.y, j0 = blockIdx.z * NC;
     const int ctx = a.ctx_start[seq];
     if (ctx < 0) return;
     const int dk = a.dk, dv = a.dv, H = a.H, LD = dk + 4, per = dk / 4;
-    const int r0 = a.cu_q[seq], n = a.cu_q[seq + 1] - r0, nchunks = (n + C - 1) / C;
-    int base = 0;                                    // this sequence's first chunk
-    for (int s = 0; s < seq; ++s)
-        if (a.ctx_start[s] >= 0) base += (a.cu_q[s + 1] - a.cu_q[s] + C - 1) / C;
+    const int r0 = a.cu_q[seq], n = a.cu_q[seq + 1] - r0, nchunks = (n + C - 1) / C, base = first_chunk(a, seq);
     const int Cq = 2 * a.G * dk + H * dv, kvh = hh / (H / a.G);
     const int slot = a.state_slot[seq];
     const int cols = min(NC, dv - j0);               // a multiple of 4
+    const Scratch sc(dk, dv, CH, true);
     float* S = sm;                                   // [dk][NC]
-    float* redA = S + dk * NC;                       // [KS][32 RB][NC]: partial products with the state
-    float* redB = redA + 8 * 32 * NC;                // partial products with T, then with P
-    float* Rm = redB + 8 * 32 * NC;                  // [C][NC] R (delta)
-    float* U = Rm + C * NC;                          // [C][NC]
-    float* Ud = U + C * NC;                          // [C][NC] U times the decay to the chunk's end (decay per head)
+    float* redA = S + dk * NC;                       // [4][C][NC]: partial products with the state
+    float* redB = redA + 4 * C * NC;                 // [4][C][NC]: partial products with T
+    float* Rm = redB + 4 * C * NC;                   // [C][NC] V - (G K) S
+    float* Ud = Rm + C * NC;                         // [C][NC] U, times the decay to the chunk's end (decay per head)
     float* st0 = Ud + C * NC;
-    const int stage_floats = L::stage(dk);
+    const int stage_floats = delta_stage(dk, CH);
 
     auto issue = [&](int c, int buf) {
         float* ks = st0 + (size_t)buf * stage_floats;
-        float* qs = ks + C * LD;
-        float* ku = qs + C * LD;                     // CH only
+        float* ku = ks + C * LD;                     // per channel only
         float* vs = ku + (CH ? C * LD : 0);
-        float* ps = vs + C * L::VLD;
-        float* ts = ps + C * L::LP;
-        float* de = ts + (DELTA ? C * L::LP : 0);
+        float* ts = vs + C * NC;
+        float* de = ts + C * LP;
         const int t0 = c * C, nt = min(C, n - t0);
-        const float* ws = a.ws + ((size_t)(base + c) * H + hh) * scratch_floats(C, dk, CH, DELTA);
-        const float* dec = ws + C * C * (DELTA ? 2 : 1);
-        const float* qrow = a.qkv + (size_t)(r0 + t0) * Cq + (size_t)kvh * dk;
-        const float* krow = qrow + (size_t)a.G * dk;
+        const float* ws = a.ws + ((size_t)(base + c) * H + hh) * sc.total;
+        const float* dec = ws + sc.dec;
+        const float* krow = a.qkv + (size_t)(r0 + t0) * Cq + (size_t)(a.G + kvh) * dk;
         const float* vrow = a.qkv + (size_t)(r0 + t0) * Cq + (size_t)2 * a.G * dk + (size_t)hh * dv + j0;
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int idx = tid; idx < C * per; idx += NT) {
             const int t = idx / per, x = (idx - t * per) * 4;
             if (CH) {                                // the decayed copies; rows past the end are zeros there
-                if (DELTA) cp_async16(ks + t * LD + x, dec + t * dk + x);
-                cp_async16(qs + t * LD + x, dec + (C + t) * dk + x);
+                cp_async16(ks + t * LD + x, dec + t * dk + x);
                 cp_async16(ku + t * LD + x, dec + (2 * C + t) * dk + x);
             } else if (t < nt) {
                 cp_async16(ks + t * LD + x, krow + (size_t)t * Cq + x);
-                cp_async16(qs + t * LD + x, qrow + (size_t)t * Cq + x);
             } else {
                 *reinterpret_cast<float4*>(ks + t * LD + x) = zero;
-                *reinterpret_cast<float4*>(qs + t * LD + x) = zero;
             }
         }
-        for (int idx = tid; idx < C * (NC / 4); idx += NT) {
-            const int t = idx / (NC / 4), x = (idx % (NC / 4)) * 4;
-            if (t < nt && x < cols) cp_async16(vs + t * L::VLD + x, vrow + (size_t)t * Cq + x);
-            else *reinterpret_cast<float4*>(vs + t * L::VLD + x) = zero;
+        {
+            const int t = tid / (NC / 4), x = (tid % (NC / 4)) * 4;  // 64 rows x 4 vectors
+            if (t < nt && x < cols) cp_async16(vs + t * NC + x, vrow + (size_t)t * Cq + x);
+            else *reinterpret_cast<float4*>(vs + t * NC + x) = zero;
         }
-        for (int idx = tid; idx < (DELTA ? 2 : 1) * C * (C / 4); idx += NT) {            // P, then T behind it
-            const int row = idx / (C / 4), x = (idx % (C / 4)) * 4;
-            cp_async16(ps + row * L::LP + x, ws + row * C + x);
-        }
-        if (CH) { for (int idx = tid; idx < per; idx += NT) cp_async16(de + idx * 4, dec + 3 * C * dk + idx * 4); }
-        else { for (int idx = tid; idx < 2 * C / 4; idx += NT) cp_async16(de + idx * 4, dec + idx * 4); }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        for (int idx = tid; idx < C * (C / 4); idx += NT) cp_async16(ts + (idx / (C / 4)) * LP + (idx % (C / 4)) * 4, ws + sc.t + idx * 4);
+        const int nd = CH ? per : 2 * C / 4;
+        if (tid < nd) cp_async16(de + tid * 4, dec + (CH ? 3 * C * dk : 0) + tid * 4);
+        cp_commit();
     };
 
     // this thread's part of the state: rows i0 .. i0 + 3, columns jc, jc + 1
@@ -300,25 +483,29 @@ chunk_scan_kernel(const ChunkArgs a, int stages) {
         if (mine && in_cols && sp && ctx > 0) s[r] = *reinterpret_cast<const float2*>(sp + (size_t)(i0 + r) * dv);
         if (mine) *reinterpret_cast<float2*>(S + (i0 + r) * NC + jc) = s[r];
     }
-    const int rg = lane >> 2, cg = lane & 3;         // products: rows rg + 8 rr of a 32-row block, columns 4 cg .. 4 cg + 3
+    const int rg = lane >> 2, cg = lane & 3;         // products: rows 32 (w / 4) + rg + 8 rr, columns 4 cg .. 4 cg + 3
+    const int half = w >> 2, kq = w & 3;
     if (nchunks > 0) issue(0, 0);
     for (int c = 0; c < nchunks; ++c) {
         const int buf = stages == 2 ? c & 1 : 0;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                             // the chunk's operands and S are there; the last chunk's stage and sums are read
+        cp_wait<0>();
+        __syncthreads();                             // the chunk's operands and S are there; the last chunk's stage is read
         if (stages == 2 && c + 1 < nchunks) issue(c + 1, buf ^ 1);
         const float* ks = st0 + (size_t)buf * stage_floats;
-        const float* qs = ks + C * LD;
-        const float* ku = CH ? qs + C * LD : ks;
-        const float* vs = qs + C * LD + (CH ? C * LD : 0);
-        const float* ps = vs + C * L::VLD;
-        const float* ts = ps + C * L::LP;
-        const float* de = ts + (DELTA ? C * L::LP : 0);
-        const int t0 = c * C, nt = min(C, n - t0);
-        {   // rows times the state: block rb (delta: k rows, q rows; else q rows 0 - 31, 32 - 63), slice kq of dk
-            const int rb = w / L::KS, kq = w % L::KS;
-            const float* rows = (DELTA ? (rb == 0 ? ks : qs) : qs + rb * 32 * LD) + rg * LD;
-            const int span = (per + L::KS - 1) / L::KS * 4, k0 = kq * span, k1 = min(k0 + span, dk);
+        const float* ku = CH ? ks + C * LD : ks;
+        const float* vs = ks + (CH ? 2 : 1) * C * LD;
+        const float* ts = vs + C * NC;
+        const float* de = ts + C * LP;
+        const int nt = min(C, n - c * C);
+        float* ws = a.ws + ((size_t)(base + c) * H + hh) * sc.total;
+        if (mine && in_cols) {
+            float* s0 = ws + sc.s0 + (size_t)i0 * dv + j0 + jc;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) *reinterpret_cast<float2*>(s0 + (size_t)r * dv) = s[r];
+        }
+        {   // K S, a quarter of dk a warp
+            const float* rows = ks + (half * 32 + rg) * LD;
+            const int span = (per + 3) / 4 * 4, k0 = kq * span, k1 = min(k0 + span, dk);
             float acc[4][4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
@@ -331,96 +518,65 @@ chunk_scan_kernel(const ChunkArgs a, int stages) {
                 for (int q = 0; q < 4; ++q) y[q] = *reinterpret_cast<const float4*>(S + (i + q) * NC + cg * 4);
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    const float xv[4] = {x[r].x, x[r].y, x[r].z, x[r].w};
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        acc[r][0] = fmaf(xv[q], y[q].x, acc[r][0]);
-                        acc[r][1] = fmaf(xv[q], y[q].y, acc[r][1]);
-                        acc[r][2] = fmaf(xv[q], y[q].z, acc[r][2]);
-                        acc[r][3] = fmaf(xv[q], y[q].w, acc[r][3]);
-                    }
+                    fma4(acc[r], x[r].x, y[0]);
+                    fma4(acc[r], x[r].y, y[1]);
+                    fma4(acc[r], x[r].z, y[2]);
+                    fma4(acc[r], x[r].w, y[3]);
                 }
             }
-            float* dst = redA + ((size_t)kq * 32 * L::RB + rb * 32 + rg) * NC + cg * 4;
+            float* dst = redA + (kq * C + half * 32 + rg) * NC + cg * 4;
 #pragma unroll
             for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(dst + r * 8 * NC) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
         }
-        if (!DELTA && !CH) {                         // U = V: its decayed copy while the products settle
-            for (int idx = tid; idx < C * NC / 4; idx += NT) {
-                const float f = de[C + idx / (NC / 4)];
-                const float4 v = *reinterpret_cast<const float4*>(vs + idx * 4);
-                *reinterpret_cast<float4*>(Ud + idx * 4) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+        __syncthreads();
+        const int t = tid >> 2, x4 = (tid & 3) * 4;  // the small matrices: four columns of a row a thread
+        {
+            const float f = CH ? 1.f : de[t];
+            const float4 v = *reinterpret_cast<const float4*>(vs + t * NC + x4);
+            float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 y = *reinterpret_cast<const float4*>(redA + (q * C + t) * NC + x4);
+                p = make_float4(p.x + y.x, p.y + y.y, p.z + y.z, p.w + y.w);
             }
+            *reinterpret_cast<float4*>(Rm + t * NC + x4) = make_float4(fmaf(-f, p.x, v.x), fmaf(-f, p.y, v.y), fmaf(-f, p.z, v.z), fmaf(-f, p.w, v.w));
         }
         __syncthreads();
-        // partial products of a [C x C] lower-triangular matrix with a [C x NC] one into redB: C = 32: slice w of 4 columns; C = 64:
-        // row half w / 4, columns 16 it + 4 (w % 4)
-        auto tri = [&](const float* m, const float* b) {
+        {   // T R, nothing above the diagonal; columns 16 it + 4 kq of T
             float acc[4][4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
-            const int half = C == 32 ? 0 : w >> 2;
-            const int its = C == 32 ? 1 : (half == 0 ? 2 : 4);          // nothing above the diagonal
-            for (int it = 0; it < its; ++it) {
-                const int s0 = C == 32 ? w * 4 : it * 16 + (w & 3) * 4;
+            for (int it = 0; it < (half == 0 ? 2 : 4); ++it) {
+                const int s0 = it * 16 + kq * 4;
                 float4 x[4], y[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(m + (half * 32 + rg + 8 * r) * L::LP + s0);
+                for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(ts + (half * 32 + rg + 8 * r) * LP + s0);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) y[q] = *reinterpret_cast<const float4*>(b + (s0 + q) * NC + cg * 4);
+                for (int q = 0; q < 4; ++q) y[q] = *reinterpret_cast<const float4*>(Rm + (s0 + q) * NC + cg * 4);
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    const float xv[4] = {x[r].x, x[r].y, x[r].z, x[r].w};
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        acc[r][0] = fmaf(xv[q], y[q].x, acc[r][0]);
-                        acc[r][1] = fmaf(xv[q], y[q].y, acc[r][1]);
-                        acc[r][2] = fmaf(xv[q], y[q].z, acc[r][2]);
-                        acc[r][3] = fmaf(xv[q], y[q].w, acc[r][3]);
-                    }
+                    fma4(acc[r], x[r].x, y[0]);
+                    fma4(acc[r], x[r].y, y[1]);
+                    fma4(acc[r], x[r].z, y[2]);
+                    fma4(acc[r], x[r].w, y[3]);
                 }
             }
-            float* dst = redB + ((size_t)(C == 32 ? w * 32 : (w & 3) * 64 + half * 32) + rg) * NC + cg * 4;
+            float* dst = redB + (kq * C + half * 32 + rg) * NC + cg * 4;
 #pragma unroll
             for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(dst + r * 8 * NC) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
-        };
-        constexpr int NS = C == 32 ? 8 : 4;          // partial products in redB
-        if (DELTA) {
-            {
-                const int t = tid >> 3, x = (tid & 7) * 2;           // C = 32: a pair of columns a thread
-                float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int kq = 0; kq < L::KS; ++kq) {
-                    const float2 p = *reinterpret_cast<const float2*>(redA + (kq * 32 * L::RB + t) * NC + x);
-                    v.x += p.x;
-                    v.y += p.y;
-                }
-                const float f = CH ? 1.f : de[t];
-                const float2 vv = *reinterpret_cast<const float2*>(vs + t * L::VLD + x);
-                *reinterpret_cast<float2*>(Rm + t * NC + x) = make_float2(fmaf(-f, v.x, vv.x), fmaf(-f, v.y, vv.y));
-            }
-            __syncthreads();
-            tri(ts, Rm);
-            __syncthreads();
-            {
-                const int t = tid >> 3, x = (tid & 7) * 2;
-                float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int q = 0; q < NS; ++q) {
-                    const float2 p = *reinterpret_cast<const float2*>(redB + (q * C + t) * NC + x);
-                    v.x += p.x;
-                    v.y += p.y;
-                }
-                *reinterpret_cast<float2*>(U + t * NC + x) = v;
-                if (!CH) {
-                    const float f = de[C + t];
-                    *reinterpret_cast<float2*>(Ud + t * NC + x) = make_float2(v.x * f, v.y * f);
-                }
-            }
-            __syncthreads();
         }
-        const float* u = DELTA ? U : vs;
-        const float* ud = CH ? u : Ud;
+        __syncthreads();
+        {
+            float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 y = *reinterpret_cast<const float4*>(redB + (q * C + t) * NC + x4);
+                p = make_float4(p.x + y.x, p.y + y.y, p.z + y.z, p.w + y.w);
+            }
+            if (x4 < cols) *reinterpret_cast<float4*>(ws + sc.u + (size_t)t * dv + j0 + x4) = p;
+            *reinterpret_cast<float4*>(Ud + t * NC + x4) = CH ? p : scaled(p, de[C + t]);
+        }
+        __syncthreads();
         if (mine) {                                  // S = G_C S + (decayed K)^T U
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
@@ -429,9 +585,9 @@ chunk_scan_kernel(const ChunkArgs a, int stages) {
                 s[r].y *= f;
             }
 #pragma unroll 8
-            for (int t = 0; t < C; ++t) {
-                const float4 k = *reinterpret_cast<const float4*>(ku + t * LD + i0);
-                const float2 x = *reinterpret_cast<const float2*>(ud + t * NC + jc);
+            for (int u = 0; u < nt; ++u) {
+                const float4 k = *reinterpret_cast<const float4*>(ku + u * LD + i0);
+                const float2 x = *reinterpret_cast<const float2*>(Ud + u * NC + jc);
                 s[0].x = fmaf(k.x, x.x, s[0].x); s[0].y = fmaf(k.x, x.y, s[0].y);
                 s[1].x = fmaf(k.y, x.x, s[1].x); s[1].y = fmaf(k.y, x.y, s[1].y);
                 s[2].x = fmaf(k.z, x.x, s[2].x); s[2].y = fmaf(k.z, x.y, s[2].y);
@@ -439,29 +595,6 @@ chunk_scan_kernel(const ChunkArgs a, int stages) {
             }
 #pragma unroll
             for (int r = 0; r < 4; ++r) *reinterpret_cast<float2*>(S + (i0 + r) * NC + jc) = s[r];
-        }
-        tri(ps, u);
-        __syncthreads();
-        for (int idx = tid; idx < nt * (NC / 2); idx += NT) {        // O = G (Q S_0) + P U
-            const int t = idx >> 3, x = (idx & 7) * 2;
-            float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int kq = 0; kq < L::KS; ++kq) {
-                const float2 p = *reinterpret_cast<const float2*>(redA + (kq * 32 * L::RB + (DELTA ? 32 : 0) + t) * NC + x);
-                v.x += p.x;
-                v.y += p.y;
-            }
-            if (!CH) {
-                v.x *= de[t];
-                v.y *= de[t];
-            }
-#pragma unroll
-            for (int q = 0; q < NS; ++q) {
-                const float2 p = *reinterpret_cast<const float2*>(redB + (q * C + t) * NC + x);
-                v.x += p.x;
-                v.y += p.y;
-            }
-            if (x < cols) *reinterpret_cast<float2*>(a.o + ((size_t)(r0 + t0 + t) * H + hh) * dv + j0 + x) = v;
         }
         if (stages == 1 && c + 1 < nchunks) {
             __syncthreads();                         // the single stage is read
@@ -474,36 +607,140 @@ chunk_scan_kernel(const ChunkArgs a, int stages) {
     }
 }
 
-template <int C, bool CH, bool DELTA>
+// ---------------------------------------------------------------------------------------------------------------- output
+// [64 x (dk + 64)] times [(dk + 64) x 128]: the rows [ G Q | P ] stay in shared memory, the rows of S_0 and of U (or V) stream through
+// two stages of 32.  Rows 4 rg .., columns 4 tj .. and 64 + 4 tj .. a thread.
+template <bool CH, bool DELTA>
+__global__ void __launch_bounds__(NT, 2)
+chunk_out_kernel(const ChunkArgs a) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ int s_at[2];
+    const int tid = threadIdx.x, hh = blockIdx.y, j0 = blockIdx.z * JB;
+    const int dk = a.dk, dv = a.dv, LD = dk + 4, per = dk / 4;
+    if (tid == 0) find_chunk(a, blockIdx.x, s_at);
+    __syncthreads();
+    const int r0 = s_at[0], nt = s_at[1];
+    if (r0 < 0) return;
+    float* qs = sm;                                  // [C][LD]
+    float* ps = qs + C * LD;                         // [C][LP]
+    float* bsm = ps + C * LP;                        // [2][32][JB]
+    const int Cq = 2 * a.G * dk + a.H * dv, kvh = hh / (a.H / a.G);
+    const Scratch sc(dk, dv, CH, DELTA);
+    const float* ws = a.ws + ((size_t)blockIdx.x * a.H + hh) * sc.total;
+    const float* dec = ws + sc.dec;
+    const float* vrow = a.qkv + (size_t)r0 * Cq + (size_t)2 * a.G * dk + (size_t)hh * dv;
+    const int n1 = (dk + 31) / 32, n2 = (nt + 31) / 32;              // slices of S_0, slices of U
+    auto issue = [&](int sl, int buf) {
+        const bool second = sl >= n1;
+        const int k0 = (second ? sl - n1 : sl) * 32, rows = second ? nt : dk;
+        for (int idx = tid; idx < 32 * (JB / 4); idx += NT) {
+            const int r = idx / (JB / 4), c = (idx % (JB / 4)) * 4;
+            float* dst = bsm + ((size_t)buf * 32 + r) * JB + c;
+            const float* src = !second ? ws + sc.s0 + (size_t)(k0 + r) * dv + j0 + c
+                             : DELTA ? ws + sc.u + (size_t)(k0 + r) * dv + j0 + c : vrow + (size_t)(k0 + r) * Cq + j0 + c;
+            if (k0 + r < rows && j0 + c < dv) cp_async16(dst, src);
+            else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        cp_commit();
+    };
+    issue(0, 0);
+    for (int idx = tid; idx < C * per; idx += NT) {
+        const int t = idx / per, c = (idx - t * per) * 4;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (CH) q = *reinterpret_cast<const float4*>(dec + (C + t) * dk + c);
+        else if (t < nt) q = scaled(*reinterpret_cast<const float4*>(a.qkv + (size_t)(r0 + t) * Cq + (size_t)kvh * dk + c), dec[t]);
+        *reinterpret_cast<float4*>(qs + t * LD + c) = q;
+    }
+    for (int idx = tid; idx < C * (C / 4); idx += NT)
+        *reinterpret_cast<float4*>(ps + (idx / (C / 4)) * LP + (idx % (C / 4)) * 4) = *reinterpret_cast<const float4*>(ws + idx * 4);
+    const int rg = tid >> 4, tj = tid & 15;
+    float acc[4][2][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[r][0][c] = acc[r][1][c] = 0.f;
+    for (int sl = 0; sl < n1 + n2; ++sl) {
+        cp_wait<0>();
+        __syncthreads();                             // slice sl is there, the other stage is read
+        if (sl + 1 < n1 + n2) issue(sl + 1, (sl + 1) & 1);
+        const bool second = sl >= n1;
+        const int k0 = (second ? sl - n1 : sl) * 32, kn = second ? 32 : min(32, dk - k0);
+        const int ld = second ? LP : LD;
+        const float* rows = (second ? ps : qs) + (size_t)(rg * 4) * ld + k0;
+        const float* b = bsm + (size_t)(sl & 1) * 32 * JB + tj * 4;
+        if (second && k0 > rg * 4 + 3) continue;     // above the diagonal
+#pragma unroll 2
+        for (int k = 0; k < kn; k += 4) {
+            float4 x[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(rows + r * ld + k);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float4 y0 = *reinterpret_cast<const float4*>(b + (k + q) * JB), y1 = *reinterpret_cast<const float4*>(b + (k + q) * JB + 64);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float xv = q == 0 ? x[r].x : q == 1 ? x[r].y : q == 2 ? x[r].z : x[r].w;
+                    fma4(acc[r][0], xv, y0);
+                    fma4(acc[r][1], xv, y1);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int t = rg * 4 + r;
+        if (t < nt) {
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const int j = j0 + b * 64 + tj * 4;
+                if (j < dv)
+                    *reinterpret_cast<float4*>(a.o + ((size_t)(r0 + t) * a.H + hh) * dv + j) =
+                        make_float4(acc[r][b][0], acc[r][b][1], acc[r][b][2], acc[r][b][3]);
+            }
+        }
+    }
+}
+
+template <typename K>
+int allow(K kern, size_t bytes) {
+    if (bytes > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return B2_OK;
+}
+
+template <bool CH, bool DELTA>
 int launch(const ChunkArgs& a, int total_rows, cudaStream_t st) {
+    static const int n_sm = []() { int dev = 0, n = 148; if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); return n; }();
     const int chunks = total_rows / C + a.n_seq;     // upper bound on sum(ceil(len / C)); spare CTAs leave at once
-    const int LD = a.dk + 4;
-    const size_t psm = sizeof(float) * (size_t)(2 * C * LD + 2 * C * (C + 1) + (CH ? C * LD : C) + C);
-    auto prep = chunk_prep_kernel<C, CH, DELTA>;
-    if (psm > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
-    prep<<<dim3(chunks, a.H), NT, psm, st>>>(a);
-    using L = ScanSmem<C, CH, DELTA>;
-    const size_t stage = sizeof(float) * (size_t)L::stage(a.dk), fixed = sizeof(float) * (size_t)L::fixed(a.dk);
-    const int stages = fixed + 2 * stage <= 227 * 1024 ? 2 : 1;
-    const size_t ssm = fixed + stages * stage;
-    auto scan = chunk_scan_kernel<C, CH, DELTA>;
-    if (ssm > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm));
-    scan<<<dim3(a.n_seq, a.H, (a.dv + NC - 1) / NC), NT, ssm, st>>>(a, stages);
+    const size_t LD = a.dk + 4, rows = C * LD;
+    const size_t psm = sizeof(float) * (rows + (DELTA ? rows : (rows > C * JB ? rows : C * JB)) + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows : C) + C);
+    int rc = allow(chunk_prep_kernel<CH, DELTA>, psm);
+    if (rc != B2_OK) return rc;
+    chunk_prep_kernel<CH, DELTA><<<dim3(chunks, a.H), NT, psm, st>>>(a);
+    if constexpr (DELTA) {
+        const dim3 grid(a.n_seq, a.H, (a.dv + NC - 1) / NC);
+        const size_t stage = sizeof(float) * (size_t)delta_stage(a.dk, CH), fixed = sizeof(float) * (size_t)delta_fixed(a.dk);
+        // two CTAs an SM cover each other's copies when there are enough of them; a lone one prefetches
+        const int stages = (long)grid.x * grid.y * grid.z > n_sm || fixed + 2 * stage > 227 * 1024 ? 1 : 2;
+        rc = allow(chunk_delta_kernel<CH>, fixed + stages * stage);
+        if (rc != B2_OK) return rc;
+        chunk_delta_kernel<CH><<<grid, NT, fixed + stages * stage, st>>>(a, stages);
+    } else {
+        chunk_state_kernel<CH><<<dim3(a.n_seq, a.H, (a.dk * a.dv / 4 + NT - 1) / NT), NT, 0, st>>>(a);
+    }
+    const size_t osm = sizeof(float) * (rows + C * LP + 2 * 32 * JB);
+    rc = allow(chunk_out_kernel<CH, DELTA>, osm);
+    if (rc != B2_OK) return rc;
+    chunk_out_kernel<CH, DELTA><<<dim3(chunks, a.H, (a.dv + JB - 1) / JB), NT, osm, st>>>(a);
     B2_CUDA_OK(cudaGetLastError());
     return B2_OK;
 }
 
-int chunk_of(bool ch, bool delta) { return ch || delta ? 32 : 64; }
-
 }  // namespace
 
-// Scratch (floats) of the chunked form, 0 where the token-by-token scan is the one to run: head sizes it is not built for, and
-// batches of short portions -- below about 24 tokens a sequence a chunk's products cost more than the tokens' chain
-// (measured at 64 sequences of 16 heads of 128: 1 token 41 us there, 100+ here).
 int64_t b2_internal_chunk_scan_floats(int total_rows, int n_seq, int H, int dk, int dv, bool ch, bool delta) {
     if (dk % 4 || dv % 4 || dk > 128 || n_seq <= 0 || total_rows < 24 * n_seq) return 0;
-    const int C = chunk_of(ch, delta);
-    return (int64_t)(total_rows / C + n_seq) * H * scratch_floats(C, dk, ch, delta);
+    const int64_t n = (int64_t)(total_rows / C + n_seq) * H * Scratch(dk, dv, ch, delta).total;
+    return n <= (int64_t)1 << 29 ? n : 0;
 }
 
 int b2_internal_chunk_scan(const float* qkv, const float* beta, const float* decay, int total_rows, int H, int G, int dk, int dv,
@@ -511,6 +748,6 @@ int b2_internal_chunk_scan(const float* qkv, const float* beta, const float* dec
                            float* state, float* o, float* ws, void* stream) {
     const ChunkArgs a{qkv, beta, decay, H, G, dk, dv, n_seq, cu_q, ctx_start, state_slot, state, o, ws};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (ch) return delta ? launch<32, true, true>(a, total_rows, st) : launch<32, true, false>(a, total_rows, st);
-    return delta ? launch<32, false, true>(a, total_rows, st) : launch<64, false, false>(a, total_rows, st);
+    if (ch) return delta ? launch<true, true>(a, total_rows, st) : launch<true, false>(a, total_rows, st);
+    return delta ? launch<false, true>(a, total_rows, st) : launch<false, false>(a, total_rows, st);
 }
