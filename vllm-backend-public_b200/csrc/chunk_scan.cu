@@ -68,11 +68,24 @@ __device__ __forceinline__ int first_chunk(const ChunkArgs& a, int seq) {
         if (a.ctx_start[s] >= 0) base += (a.cu_q[s + 1] - a.cu_q[s] + C - 1) / C;
     return base;
 }
-__device__ __forceinline__ void fma4(float (&acc)[4], float x, const float4& y) {
-    acc[0] = fmaf(x, y.x, acc[0]);
-    acc[1] = fmaf(x, y.y, acc[1]);
-    acc[2] = fmaf(x, y.z, acc[2]);
-    acc[3] = fmaf(x, y.w, acc[3]);
+// Two FMAs an instruction on register pairs: the rate is that of two (73 TFLOP/s either way), but half the issue slots, which the
+// shared-memory reads need.
+typedef unsigned long long pair_t;
+__device__ __forceinline__ pair_t dup(float x) {
+    pair_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ void fma2(pair_t& acc, pair_t x, pair_t y) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(y)); }
+__device__ __forceinline__ float2 halves(pair_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ ulonglong2 pairs(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
+__device__ __forceinline__ float4 unpack(pair_t lo, pair_t hi) {
+    const float2 a = halves(lo), b = halves(hi);
+    return make_float4(a.x, a.y, b.x, b.y);
 }
 __device__ __forceinline__ float4 scaled(const float4& v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); }
 
@@ -93,7 +106,7 @@ chunk_prep_kernel(const ChunkArgs a) {
     float* Ps = qs + (DELTA ? C * LD : max(C * LD, C * JB));        // [C][C + 1]
     float* As = Ps + C * (C + 1);                    // [C][C + 1] (delta)
     float* gs = As + (DELTA ? C * (C + 1) : 0);      // [C], per channel [C][LD]
-    float* bs = gs + (CH ? C * LD : C);              // [C] beta; per head without delta: G_C/G
+    float* bs = gs + (CH ? C * LD : C);              // [C] beta; per head without delta: G_C/G; per head 4 + C more
     const int Cq = 2 * a.G * dk + a.H * dv, kvh = hh / (a.H / a.G);
     const float* qrow = a.qkv + (size_t)r0 * Cq + (size_t)kvh * dk;
     const float* krow = qrow + (size_t)a.G * dk;
@@ -224,38 +237,53 @@ chunk_prep_kernel(const ChunkArgs a) {
             }
         }
     } else {
-        if (tid < C) {                               // column s of the decay ratios, and the products from the start / to the end
+        // the decay ratios of all (t, s), and the products from the chunk's start and to its end: by segments of 16 tokens, a chain of
+        // 16 + 16 products instead of 64
+        float* seg = As + (DELTA ? C * (C + 1) : 0) + 2 * C;         // behind g and beta: [4] segments | [C] from s + 1 to the end of its segment
+        float* tail = seg + 4;
+        const int col = tid & (C - 1), sg = tid >> 6, own = col >> 4;
+        if (tid < C) {
             float run = 1.f;
-            for (int t = 0; t < tid; ++t) Ps[t * (C + 1) + tid] = 0.f;
-            Ps[tid * (C + 1) + tid] = 1.f;
-            for (int t = tid + 1; t < C; ++t) {
-                run *= gs[t];
-                Ps[t * (C + 1) + tid] = run;
+            for (int r = tid + 1; r < (tid | 15) + 1; ++r) run *= gs[r];
+            tail[tid] = run;
+            if ((tid & 15) == 0) seg[tid >> 4] = run * gs[tid];
+        }
+        __syncthreads();
+        {
+            float run = tail[col];
+            for (int m = own + 1; m < sg; ++m) run *= seg[m];
+            if (sg == own) run = 1.f;
+#pragma unroll 4
+            for (int t = sg * 16; t < sg * 16 + 16; ++t) {
+                if (t > col) run *= gs[t];
+                Ps[t * (C + 1) + col] = t >= col ? run : 0.f;
             }
-            dec[C + tid] = run;
-            if (!DELTA) bs[tid] = run;
-            float from = 1.f;
-            for (int t = 0; t <= tid; ++t) from *= gs[t];
+        }
+        if (tid < C) {
+            float to = tail[tid], from = 1.f;
+            for (int m = own + 1; m < 4; ++m) to *= seg[m];
+            for (int m = 0; m < own; ++m) from *= seg[m];
+            for (int r = own * 16; r <= tid; ++r) from *= gs[r];
             dec[tid] = from;
+            dec[C + tid] = to;
+            if (!DELTA) bs[tid] = to;
         }
         __syncthreads();
         constexpr int RR = DELTA ? 8 : 4;
-        float acc[RR][4];
+        pair_t acc[RR][4];                           // sums over even and odd entries; blocks above the diagonal are left out
 #pragma unroll
-        for (int r = 0; r < RR; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+        for (int r = 0; r < RR; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0;
         for (int i = 0; i < dk; i += 4) {
-            float4 kc[4];
+            ulonglong2 kc[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) kc[c] = *reinterpret_cast<const float4*>(ks + (cg + 16 * c) * LD + i);
+            for (int c = 0; c < 4; ++c) kc[c] = pairs(ks + (cg + 16 * c) * LD + i);
 #pragma unroll
             for (int r = 0; r < RR; ++r) {
-                const float4 x = *reinterpret_cast<const float4*>((r < 4 ? qs : ks) + (rg + 16 * (r & 3)) * LD + i);
+                const ulonglong2 x = pairs((r < 4 ? qs : ks) + (rg + 16 * (r & 3)) * LD + i);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    acc[r][c] = fmaf(x.x, kc[c].x, acc[r][c]);
-                    acc[r][c] = fmaf(x.y, kc[c].y, acc[r][c]);
-                    acc[r][c] = fmaf(x.z, kc[c].z, acc[r][c]);
-                    acc[r][c] = fmaf(x.w, kc[c].w, acc[r][c]);
+                for (int c = 0; c <= (r & 3); ++c) {
+                    fma2(acc[r][c], x.x, kc[c].x);
+                    fma2(acc[r][c], x.y, kc[c].y);
                 }
             }
         }
@@ -263,10 +291,11 @@ chunk_prep_kernel(const ChunkArgs a) {
         for (int r = RR - 1; r >= 0; --r) {          // the k rows still need the ratios that the q rows overwrite (same thread)
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const int t = rg + 16 * (r & 3), s = cg + 16 * c;
-                const float ratio = Ps[t * (C + 1) + s];
-                if (r < 4) Ps[t * (C + 1) + s] = acc[r][c] * ratio;                      // 0 above the diagonal
-                else As[t * (C + 1) + s] = t > s ? bs[t] * acc[r][c] * ratio : 0.f;
+                const int t = rg + 16 * (r & 3), x = cg + 16 * c;
+                const float2 h = halves(acc[r][c]);
+                const float v = (h.x + h.y) * Ps[t * (C + 1) + x];   // 0 above the diagonal
+                if (r < 4) Ps[t * (C + 1) + x] = v;
+                else As[t * (C + 1) + x] = t > x ? bs[t] * v : 0.f;
             }
         }
     }
@@ -342,21 +371,22 @@ chunk_prep_kernel(const ChunkArgs a) {
             }
             __syncthreads();
             if (ti * 8 < dk) {
-                float acc[8][2][4];
+                pair_t acc[8][4];
 #pragma unroll
-                for (int r = 0; r < 8; ++r)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[r][0][c] = acc[r][1][c] = 0.f;
+                for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0;
                 const int hi = min(ti * 8 + 4, dk - 4);              // heads of 4 (mod 8) entries: a second look at the last four
-#pragma unroll 2
+#pragma unroll 4
                 for (int t = 0; t < C; ++t) {
                     const float4 x0 = *reinterpret_cast<const float4*>(ks + t * LD + ti * 8), x1 = *reinterpret_cast<const float4*>(ks + t * LD + hi);
-                    const float4 y0 = *reinterpret_cast<const float4*>(vs + t * JB + tj * 4), y1 = *reinterpret_cast<const float4*>(vs + t * JB + 64 + tj * 4);
+                    const ulonglong2 y0 = pairs(vs + t * JB + tj * 4), y1 = pairs(vs + t * JB + 64 + tj * 4);
                     const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
                     for (int r = 0; r < 8; ++r) {
-                        fma4(acc[r][0], x[r], y0);
-                        fma4(acc[r][1], x[r], y1);
+                        const pair_t xx = dup(x[r]);
+                        fma2(acc[r][0], xx, y0.x);
+                        fma2(acc[r][1], xx, y0.y);
+                        fma2(acc[r][2], xx, y1.x);
+                        fma2(acc[r][3], xx, y1.y);
                     }
                 }
 #pragma unroll
@@ -365,7 +395,7 @@ chunk_prep_kernel(const ChunkArgs a) {
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
                         const int j = j0 + b * 64 + tj * 4;
-                        if (j < dv) *reinterpret_cast<float4*>(f0 + (size_t)i * dv + j) = make_float4(acc[r][b][0], acc[r][b][1], acc[r][b][2], acc[r][b][3]);
+                        if (j < dv) *reinterpret_cast<float4*>(f0 + (size_t)i * dv + j) = unpack(acc[r][2 * b], acc[r][2 * b + 1]);
                     }
                 }
             }
@@ -380,7 +410,7 @@ chunk_state_kernel(const ChunkArgs a) {
     const int seq = blockIdx.x, hh = blockIdx.y;
     const int ctx = a.ctx_start[seq];
     if (ctx < 0) return;
-    const int dk = a.dk, dv = a.dv, e = (blockIdx.z * NT + threadIdx.x) * 4;
+    const int dk = a.dk, dv = a.dv, e = (blockIdx.z * blockDim.x + threadIdx.x) * 4;
     if (e >= dk * dv) return;
     const int nchunks = (a.cu_q[seq + 1] - a.cu_q[seq] + C - 1) / C;
     if (nchunks == 0) return;
@@ -392,22 +422,28 @@ chunk_state_kernel(const ChunkArgs a) {
     const int slot = a.state_slot[seq];
     float* sp = slot >= 0 ? a.state + ((size_t)slot * a.H + hh) * dk * dv + e : nullptr;
     float4 s = sp && ctx > 0 ? *reinterpret_cast<const float4*>(sp) : make_float4(0.f, 0.f, 0.f, 0.f);
-    constexpr int AHEAD = 8;                         // loads in flight: they do not depend on the chain
+    constexpr int AHEAD = 6;                         // loads in flight: they do not depend on the chain
+    float4 x[AHEAD];
+    float d[AHEAD];
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u)
+        if (u < nchunks) {
+            x[u] = *reinterpret_cast<const float4*>(f + u * step);
+            d[u] = g[u * step];
+        }
     for (int c0 = 0; c0 < nchunks; c0 += AHEAD) {
-        float4 x[AHEAD];
-        float d[AHEAD];
 #pragma unroll
-        for (int u = 0; u < AHEAD; ++u)
-            if (c0 + u < nchunks) {
-                x[u] = *reinterpret_cast<const float4*>(f + (c0 + u) * step);
-                d[u] = g[(c0 + u) * step];
-            }
-#pragma unroll
-        for (int u = 0; u < AHEAD; ++u)
-            if (c0 + u < nchunks) {
-                *reinterpret_cast<float4*>(f + (c0 + u) * step) = s;
+        for (int u = 0; u < AHEAD; ++u) {
+            const int c = c0 + u;
+            if (c < nchunks) {
+                *reinterpret_cast<float4*>(f + c * step) = s;
                 s = make_float4(fmaf(s.x, d[u], x[u].x), fmaf(s.y, d[u], x[u].y), fmaf(s.z, d[u], x[u].z), fmaf(s.w, d[u], x[u].w));
+                if (c + AHEAD < nchunks) {
+                    x[u] = *reinterpret_cast<const float4*>(f + (c + AHEAD) * step);
+                    d[u] = g[(c + AHEAD) * step];
+                }
             }
+        }
     }
     if (sp) *reinterpret_cast<float4*>(sp) = s;
 }
@@ -506,27 +542,31 @@ chunk_delta_kernel(const ChunkArgs a, int stages) {
         {   // K S, a quarter of dk a warp
             const float* rows = ks + (half * 32 + rg) * LD;
             const int span = (per + 3) / 4 * 4, k0 = kq * span, k1 = min(k0 + span, dk);
-            float acc[4][4];
+            pair_t acc[4][2];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+            for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0;
 #pragma unroll 2
             for (int i = k0; i < k1; i += 4) {
-                float4 x[4], y[4];
+                float4 x[4];
+                ulonglong2 y[4];
 #pragma unroll
                 for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(rows + r * 8 * LD + i);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) y[q] = *reinterpret_cast<const float4*>(S + (i + q) * NC + cg * 4);
+                for (int q = 0; q < 4; ++q) y[q] = pairs(S + (i + q) * NC + cg * 4);
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    fma4(acc[r], x[r].x, y[0]);
-                    fma4(acc[r], x[r].y, y[1]);
-                    fma4(acc[r], x[r].z, y[2]);
-                    fma4(acc[r], x[r].w, y[3]);
+                    const float xv[4] = {x[r].x, x[r].y, x[r].z, x[r].w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const pair_t xx = dup(xv[q]);
+                        fma2(acc[r][0], xx, y[q].x);
+                        fma2(acc[r][1], xx, y[q].y);
+                    }
                 }
             }
             float* dst = redA + (kq * C + half * 32 + rg) * NC + cg * 4;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(dst + r * 8 * NC) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+            for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(dst + r * 8 * NC) = unpack(acc[r][0], acc[r][1]);
         }
         __syncthreads();
         const int t = tid >> 2, x4 = (tid & 3) * 4;  // the small matrices: four columns of a row a thread
@@ -543,27 +583,31 @@ chunk_delta_kernel(const ChunkArgs a, int stages) {
         }
         __syncthreads();
         {   // T R, nothing above the diagonal; columns 16 it + 4 kq of T
-            float acc[4][4];
+            pair_t acc[4][2];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+            for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0;
             for (int it = 0; it < (half == 0 ? 2 : 4); ++it) {
                 const int s0 = it * 16 + kq * 4;
-                float4 x[4], y[4];
+                float4 x[4];
+                ulonglong2 y[4];
 #pragma unroll
                 for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(ts + (half * 32 + rg + 8 * r) * LP + s0);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) y[q] = *reinterpret_cast<const float4*>(Rm + (s0 + q) * NC + cg * 4);
+                for (int q = 0; q < 4; ++q) y[q] = pairs(Rm + (s0 + q) * NC + cg * 4);
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    fma4(acc[r], x[r].x, y[0]);
-                    fma4(acc[r], x[r].y, y[1]);
-                    fma4(acc[r], x[r].z, y[2]);
-                    fma4(acc[r], x[r].w, y[3]);
+                    const float xv[4] = {x[r].x, x[r].y, x[r].z, x[r].w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const pair_t xx = dup(xv[q]);
+                        fma2(acc[r][0], xx, y[q].x);
+                        fma2(acc[r][1], xx, y[q].y);
+                    }
                 }
             }
             float* dst = redB + (kq * C + half * 32 + rg) * NC + cg * 4;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(dst + r * 8 * NC) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+            for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(dst + r * 8 * NC) = unpack(acc[r][0], acc[r][1]);
         }
         __syncthreads();
         {
@@ -654,11 +698,9 @@ chunk_out_kernel(const ChunkArgs a) {
     for (int idx = tid; idx < C * (C / 4); idx += NT)
         *reinterpret_cast<float4*>(ps + (idx / (C / 4)) * LP + (idx % (C / 4)) * 4) = *reinterpret_cast<const float4*>(ws + idx * 4);
     const int rg = tid >> 4, tj = tid & 15;
-    float acc[4][2][4];
+    pair_t acc[4][4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][0][c] = acc[r][1][c] = 0.f;
+    for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0;
     for (int sl = 0; sl < n1 + n2; ++sl) {
         cp_wait<0>();
         __syncthreads();                             // slice sl is there, the other stage is read
@@ -676,12 +718,14 @@ chunk_out_kernel(const ChunkArgs a) {
             for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(rows + r * ld + k);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const float4 y0 = *reinterpret_cast<const float4*>(b + (k + q) * JB), y1 = *reinterpret_cast<const float4*>(b + (k + q) * JB + 64);
+                const ulonglong2 y0 = pairs(b + (k + q) * JB), y1 = pairs(b + (k + q) * JB + 64);
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    const float xv = q == 0 ? x[r].x : q == 1 ? x[r].y : q == 2 ? x[r].z : x[r].w;
-                    fma4(acc[r][0], xv, y0);
-                    fma4(acc[r][1], xv, y1);
+                    const pair_t xx = dup(q == 0 ? x[r].x : q == 1 ? x[r].y : q == 2 ? x[r].z : x[r].w);
+                    fma2(acc[r][0], xx, y0.x);
+                    fma2(acc[r][1], xx, y0.y);
+                    fma2(acc[r][2], xx, y1.x);
+                    fma2(acc[r][3], xx, y1.y);
                 }
             }
         }
@@ -694,8 +738,7 @@ chunk_out_kernel(const ChunkArgs a) {
             for (int b = 0; b < 2; ++b) {
                 const int j = j0 + b * 64 + tj * 4;
                 if (j < dv)
-                    *reinterpret_cast<float4*>(a.o + ((size_t)(r0 + t) * a.H + hh) * dv + j) =
-                        make_float4(acc[r][b][0], acc[r][b][1], acc[r][b][2], acc[r][b][3]);
+                    *reinterpret_cast<float4*>(a.o + ((size_t)(r0 + t) * a.H + hh) * dv + j) = unpack(acc[r][2 * b], acc[r][2 * b + 1]);
             }
         }
     }
@@ -712,7 +755,7 @@ int launch(const ChunkArgs& a, int total_rows, cudaStream_t st) {
     static const int n_sm = []() { int dev = 0, n = 148; if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); return n; }();
     const int chunks = total_rows / C + a.n_seq;     // upper bound on sum(ceil(len / C)); spare CTAs leave at once
     const size_t LD = a.dk + 4, rows = C * LD;
-    const size_t psm = sizeof(float) * (rows + (DELTA ? rows : (rows > C * JB ? rows : C * JB)) + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows : C) + C);
+    const size_t psm = sizeof(float) * (rows + (DELTA ? rows : (rows > C * JB ? rows : C * JB)) + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows : 2 * C + 4) + C);
     int rc = allow(chunk_prep_kernel<CH, DELTA>, psm);
     if (rc != B2_OK) return rc;
     chunk_prep_kernel<CH, DELTA><<<dim3(chunks, a.H), NT, psm, st>>>(a);
@@ -725,7 +768,7 @@ int launch(const ChunkArgs& a, int total_rows, cudaStream_t st) {
         if (rc != B2_OK) return rc;
         chunk_delta_kernel<CH><<<grid, NT, fixed + stages * stage, st>>>(a, stages);
     } else {
-        chunk_state_kernel<CH><<<dim3(a.n_seq, a.H, (a.dk * a.dv / 4 + NT - 1) / NT), NT, 0, st>>>(a);
+        chunk_state_kernel<CH><<<dim3(a.n_seq, a.H, (a.dk * a.dv / 4 + 127) / 128), 128, 0, st>>>(a);
     }
     const size_t osm = sizeof(float) * (rows + C * LP + 2 * 32 * JB);
     rc = allow(chunk_out_kernel<CH, DELTA>, osm);

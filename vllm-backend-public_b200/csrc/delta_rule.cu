@@ -131,6 +131,173 @@ __global__ void recur_prep_kernel(const T* __restrict__ proj, int64_t proj_strid
     }
 }
 
+// The same for channels in vectors of eight whose heads are 1, 2, .. 32 lanes of a warp (dk = 8 .. 256, a power of two): a thread keeps
+// its eight channels over `run` consecutive batch rows, the last taps - 1 inputs and the weights in registers, so every input is
+// read once and 16 bytes at a time; the sums over a head and the partners of a rotation are shuffles.  Vectors behind the q | k | v
+// columns are those of a decay per key channel; small per-head outputs are left to the first column block.
+// Bound: memory (2 or 4 bytes in and 4 out per channel), with the exact exponentials and divisions of the activation close behind.
+// One CTA a row with scalar accesses and a staging pass took 89 us at 4096 rows of 6144 channels (rotation, no convolution) and
+// 175 us at 3001 (four taps, SiLU, unit vectors); this one 31 and 38.
+template <typename T>
+__device__ __forceinline__ void ld_vec8(const T* p, float (&v)[8]) {
+    if constexpr (sizeof(T) == 2) {
+        b2::ld8(p, v);
+    } else {
+        float a[4], b[4];
+        b2::ld4(p, a);
+        b2::ld4(p + 4, b);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { v[c] = a[c]; v[4 + c] = b[c]; }
+    }
+}
+
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(256)
+recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec sp, const float* __restrict__ conv_w,
+                      const int32_t* __restrict__ cu_q, const int32_t* __restrict__ ctx_start, const int32_t* __restrict__ state_slot,
+                      int n_seq, int rows, int run, const T* __restrict__ conv_state, float* __restrict__ qkv, float* __restrict__ beta,
+                      float* __restrict__ decay) {
+    const int H = sp.H, G = sp.G, dk = sp.dk, C = 2 * G * dk + H * sp.dv;
+    const int vec = blockIdx.y * 256 + threadIdx.x, lane = threadIdx.x & 31;
+    const int c0 = vec * 8, qk = 2 * G * dk;
+    const int r_begin = blockIdx.x * run, r_end = min(rows, r_begin + run);
+    const int P = dk / 8, i0 = c0 % dk, half = sp.rot_dims / 2;          // lanes a head, first entry of this lane's head part
+    const bool channel = c0 < C, head = c0 < qk;
+    const bool turns = head && i0 < sp.rot_dims;
+    const bool second = !sp.interleaved && i0 >= half;
+    const float scale = c0 < G * dk ? sp.q_scale : sp.k_scale;
+    float w[TAPS][8], hist[TAPS][8];                 // hist[j]: the input j rows back
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j)
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            hist[j][c] = 0.f;
+            w[j][c] = conv_w && channel ? conv_w[(size_t)(c0 + c) * TAPS + (TAPS - 1 - j)] : 1.f;
+        }
+    // a decay per key channel: vectors [C / 8, C / 8 + H dk / 8)
+    const int d0 = c0 - C;
+    const bool per_channel = !channel && (sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS || sp.decay_mode == B2_DECAY_CHANNEL_SIGMOID_POW) && d0 < H * dk;
+    float dbias[8];
+    float rate = 0.f;
+    if (per_channel) {
+        if (sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS) rate = -expf(sp.A_log[d0 / dk]);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) dbias[c] = sp.bias ? sp.bias[d0 + c] : 0.f;
+    }
+    int seq = -1, seq_end = r_begin, seq_begin = 0, ctx = -1;
+    for (int row = r_begin; row < r_end; ++row) {
+        bool fresh = row == r_begin;
+        if (row >= seq_end) {                        // the next sequence with rows
+            seq = b2::seq_of_row(cu_q, n_seq, row);
+            seq_begin = cu_q[seq];
+            seq_end = cu_q[seq + 1];
+            ctx = ctx_start[seq];
+            fresh = true;
+        }
+        if (ctx < 0) continue;
+        const int li = row - seq_begin;
+        if (channel) {
+            if (TAPS > 1) {
+                if (fresh) {                         // inputs before this row: earlier rows of the portion, then the state's tail
+                    const int slot = state_slot[seq];
+                    const T* st = slot >= 0 && ctx > 0 ? conv_state + (size_t)slot * (TAPS - 1) * C : nullptr;
+#pragma unroll
+                    for (int j = 1; j < TAPS; ++j) {
+                        const int l = li - j;
+                        if (l >= 0) {
+                            ld_vec8(proj + (size_t)(row - j) * proj_stride + c0, hist[j]);
+                        } else if (ctx + l >= 0 && st) {
+                            ld_vec8(st + (size_t)(l + TAPS - 1) * C + c0, hist[j]);
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) hist[j][c] = 0.f;
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int j = TAPS - 1; j > 0; --j)
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) hist[j][c] = hist[j - 1][c];
+                }
+            }
+            ld_vec8(proj + (size_t)row * proj_stride + c0, hist[0]);
+        }
+        float x[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            x[c] = hist[0][c];
+            if (TAPS > 1 || conv_w) {
+                x[c] = 0.f;
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) x[c] = fmaf(w[j][c], hist[j][c], x[c]);
+            }
+            if (sp.act && channel) x[c] = b2::silu_f(x[c]);
+        }
+        float sc = scale;
+        if (sp.unit) {                               // every lane takes part: heads and value columns may share a warp
+            float ss = 0.f;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) ss = fmaf(x[c], x[c], ss);
+            for (int m = 1; m < P; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+            sc *= rsqrtf(ss + sp.unit_eps);
+        }
+        if (sp.rot_dims) {
+            const float* cs = sp.cos_sin + (size_t)min(ctx + li, sp.max_pos - 1) * sp.rot_dims;
+            if (sp.interleaved) {
+                if (turns) {
+#pragma unroll
+                    for (int c = 0; c < 8; c += 2) {
+                        const float co = cs[(i0 + c) >> 1], si = cs[half + ((i0 + c) >> 1)], u = x[c], v = x[c + 1];
+                        x[c] = fmaf(u, co, -v * si);
+                        x[c + 1] = fmaf(v, co, u * si);
+                    }
+                }
+            } else {
+                const int src = turns ? (second ? lane - half / 8 : lane + half / 8) : lane;
+                float y[8];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) y[c] = __shfl_sync(0xffffffffu, x[c], src);
+                if (turns) {
+                    float co[8], si[8];
+                    const int pr = second ? i0 - half : i0;
+                    ld_vec8(cs + pr, co);
+                    ld_vec8(cs + half + pr, si);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) x[c] = second ? fmaf(x[c], co[c], y[c] * si[c]) : fmaf(x[c], co[c], -y[c] * si[c]);
+                }
+            }
+        }
+        if (channel) {
+            const float f = head ? sc : 1.f;
+            float* o = qkv + (size_t)row * C + c0;
+            *reinterpret_cast<float4*>(o) = make_float4(x[0] * f, x[1] * f, x[2] * f, x[3] * f);
+            *reinterpret_cast<float4*>(o + 4) = make_float4(x[4] * f, x[5] * f, x[6] * f, x[7] * f);
+        } else if (per_channel) {
+            float z[8];
+            ld_vec8(sp.a + (size_t)row * sp.a_stride + d0, z);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                z[c] += dbias[c];
+                z[c] = sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS ? expf(rate * b2::softplus_f(z[c])) : expf(-b2::softplus_f(-z[c]) * sp.inv_tau);
+            }
+            float* o = decay + (size_t)row * H * dk + d0;
+            *reinterpret_cast<float4*>(o) = make_float4(z[0], z[1], z[2], z[3]);
+            *reinterpret_cast<float4*>(o + 4) = make_float4(z[4], z[5], z[6], z[7]);
+        }
+    }
+    if (blockIdx.y) return;
+    for (int idx = threadIdx.x; idx < (r_end - r_begin) * H; idx += 256) {
+        const int row = r_begin + idx / H, hh = idx % H;
+        if (ctx_start[b2::seq_of_row(cu_q, n_seq, row)] < 0) continue;
+        const T* pr = proj + (size_t)row * proj_stride;
+        if (sp.off_beta >= 0) beta[(size_t)row * H + hh] = b2::sigmoid_f(b2::ld(pr + sp.off_beta + hh));
+        if (sp.decay_mode == B2_DECAY_HEAD_SOFTPLUS)
+            decay[(size_t)row * H + hh] = expf(-expf(sp.A_log[hh]) * b2::softplus_f(b2::ld(pr + sp.off_a + hh) + sp.bias[hh]));
+        else if (sp.decay_mode == B2_DECAY_HEAD_CONST)
+            decay[(size_t)row * H + hh] = sp.bias[hh];
+    }
+}
+
 template <typename T>
 __global__ void delta_conv_state_kernel(const T* __restrict__ proj, int64_t proj_stride, int C, int taps,
                                         const int32_t* __restrict__ cu_q, const int32_t* __restrict__ ctx_start,
@@ -442,6 +609,43 @@ __global__ void gated_head_norm_kernel(const float* __restrict__ o, const T* __r
     }
 }
 
+// The same with a head in 1, 2, .. 32 lanes of eight entries (dv = 8 .. 256, a power of two): 16-byte accesses, the row read once.
+// Scalar accesses and a warp per head took 27 us at 4096 rows of 16 heads of 128, this 13 (0.78 of the copy rate).
+template <typename T>
+__global__ void __launch_bounds__(256)
+gated_head_norm_vec_kernel(const float* __restrict__ o, const T* __restrict__ gate, int64_t gate_stride, int gate_kind, int H, int dv,
+                           const float* __restrict__ norm_w, float eps, float out_scale, T* __restrict__ out, int64_t out_stride, int64_t total) {
+    const int64_t e = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 8;
+    const bool ok = e < total;
+    const int width = H * dv, P = dv / 8;
+    const int64_t row = ok ? e / width : 0;
+    const int c0 = ok ? (int)(e - row * width) : 0;
+    float v[8], ss = 0.f;
+    ld_vec8(o + (ok ? e : 0), v);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) ss = fmaf(v[c], v[c], ss);
+    for (int m = 1; m < P; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+    if (!ok) return;
+    const float inv = rsqrtf(ss / (float)dv + eps);
+    float z[8], wv[8];
+    ld_vec8(gate + row * gate_stride + c0, z);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) wv[c] = 1.f;
+    if (norm_w) ld_vec8(norm_w + c0 % dv, wv);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float g = b2::sigmoid_as<T>(z[c]);
+        v[c] = v[c] * inv * wv[c] * (gate_kind == B2_GATE_SIGMOID ? g : z[c] * g) * out_scale;
+    }
+    T* dst = out + row * out_stride + c0;
+    if constexpr (sizeof(T) == 2) {
+        b2::st8(dst, v);
+    } else {
+        *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    }
+}
+
 // The same for wide rows (a norm over all the heads of a token at once is one "head" of H * dv entries): a CTA per
 // (row, head), four entries a thread per access when the sizes and addresses allow.
 template <typename T, int W>
@@ -528,11 +732,31 @@ int launch_prep(const void* proj, int64_t proj_stride, const PrepSpec& sp, int T
                 float* decay, cudaStream_t st) {
     const int C = 2 * sp.G * sp.dk + sp.H * sp.dv;
     const size_t smem = (size_t)C * sizeof(float);
+    const bool channel_decay = sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS || sp.decay_mode == B2_DECAY_CHANNEL_SIGMOID_POW;
+    const int P = sp.dk / 8;
+    const bool vec = sp.dk % 8 == 0 && P <= 32 && (P & (P - 1)) == 0 && sp.dv % 8 == 0 && sp.taps <= 4 && (conv_w || sp.taps == 1) &&
+                     sp.rot_dims % (sp.interleaved ? 8 : 16) == 0 && b2_aligned16(proj) && (proj_stride * sizeof(A)) % 16 == 0 && b2_aligned16(qkv) &&
+                     (sp.taps == 1 || b2_aligned16(conv_state)) && (!sp.rot_dims || b2_aligned16(sp.cos_sin)) &&
+                     (!channel_decay || (b2_aligned16(sp.a) && sp.a_stride % 4 == 0 && b2_aligned16(decay)));
+    if (vec) {
+        // rows a CTA: long runs read the convolution's inputs once; small batches spread over the SMs instead
+        const int run = T >= 2048 ? 8 : T >= 512 ? 4 : 1;
+        const dim3 grid((T + run - 1) / run, ((C + (channel_decay ? sp.H * sp.dk : 0)) / 8 + 255) / 256);
+#define B2_PREP_VEC(TAPS)                                                                                                    \
+    recur_prep_vec_kernel<A, TAPS><<<grid, 256, 0, st>>>(static_cast<const A*>(proj), proj_stride, sp, conv_w, cu_q, ctx_start, state_slot, \
+                                                         n_seq, T, run, static_cast<const A*>(conv_state), qkv, beta, decay)
+        if (sp.taps == 1) B2_PREP_VEC(1);
+        else if (sp.taps == 2) B2_PREP_VEC(2);
+        else if (sp.taps == 3) B2_PREP_VEC(3);
+        else B2_PREP_VEC(4);
+#undef B2_PREP_VEC
+    } else {
     B2_REQUIRE(smem <= 200 * 1024, B2_EUNSUPPORTED, "recurrence prep: %d channels do not fit shared memory", C);
     auto kern = recur_prep_kernel<A>;
     if (smem > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<T, 256, smem, st>>>(static_cast<const A*>(proj), proj_stride, sp, conv_w, cu_q, ctx_start, state_slot, n_seq,
                                static_cast<const A*>(conv_state), qkv, beta, decay);
+    }
     B2_CUDA_OK(cudaGetLastError());
     if (sp.taps > 1) {
         const int by = (C + 255) / 256;
@@ -667,6 +891,15 @@ extern "C" int b2_gated_head_norm(const float* o, const void* gate, int64_t gate
                 gated_row_norm_kernel<A, 1><<<T * H, 256, 0, st>>>(o, static_cast<const A*>(gate), gate_stride, gate_kind, H, dv,
                                                                   norm_w, eps, out_scale, static_cast<A*>(out), out_stride);
         });
+        B2_CUDA_OK(cudaGetLastError());
+        return B2_OK;
+    }
+    const size_t esz = act_dtype == B2_ACT_BF16 ? 2 : 4;
+    if (dv % 8 == 0 && dv <= 256 && (dv & (dv - 1)) == 0 && b2_aligned16(o) && b2_aligned16(gate) && b2_aligned16(out) && b2_aligned16(norm_w) &&
+        gate_stride * esz % 16 == 0 && out_stride * esz % 16 == 0) {
+        const int64_t total = (int64_t)T * H * dv;
+        B2_DISPATCH_ACT(act_dtype, A, (gated_head_norm_vec_kernel<A><<<(unsigned)((total / 8 + 255) / 256), 256, 0, st>>>(
+            o, static_cast<const A*>(gate), gate_stride, gate_kind, H, dv, norm_w, eps, out_scale, static_cast<A*>(out), out_stride, total)));
         B2_CUDA_OK(cudaGetLastError());
         return B2_OK;
     }
