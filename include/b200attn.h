@@ -521,8 +521,8 @@ B2_API int b2_channel_scan(const float* qkv, const float* beta /* NULL without d
                            int H, int G, int dk, int dv, int decay_per_channel, int delta, const int32_t* cu_q,
                            const int32_t* ctx_start, const int32_t* state_slot, int n_seq, float* state, float* o,
                            void* stream);
-/* The same with fp32 scratch from the caller: b2_channel_scan_workspace floats (0: none is used) let prompts run in chunks of 32
- * or 64 tokens -- a few products per chunk instead of a chain of tokens -- without it (NULL, or too small) the call is
+/* The same with fp32 scratch from the caller: b2_channel_scan_workspace floats (0: none is used) let prompts run in chunks of 64
+ * tokens -- a few products per chunk instead of a chain of tokens -- without it (NULL, or too small) the call is
  * b2_channel_scan.  The results are the same recurrence summed in another order. */
 B2_API int64_t b2_channel_scan_workspace(int total_rows, int n_seq, int H, int dk, int dv, int decay_per_channel, int delta);
 B2_API int b2_channel_scan_ws(const float* qkv, const float* beta, const float* decay, int total_rows, int H, int G, int dk, int dv,

@@ -72,13 +72,15 @@ def test_chunked_scan(cuda, lens, ctx, slots, H, G, dk, dv, decay, delta, per_ch
         cu.append(cu[-1] + n)
     batch = ops.SeqBatch(i32(cu), i32(ctx), None, i32(slots), len(lens), T)
     lib = _lib.load()
-    assert lib.b2_channel_scan_workspace(T, len(lens), H, dk, dv, int(per_channel), int(delta)) > 0, "these sizes are meant for chunks"
     st_new, st_old = state.clone(), state.clone()
-    new = ops.channel_scan(qkv, beta, dec, H, G, dk, dv, batch, st_new, delta=delta)
-    old = torch.zeros(T, H, dv, device=cuda)
-    _lib.check(lib.b2_channel_scan(qkv.data_ptr(), beta.data_ptr() if delta else None, dec.data_ptr(), T, H, G, dk, dv, int(per_channel),
-                                   int(delta), batch.cu_q.data_ptr(), batch.ctx_start.data_ptr(), batch.state_slots.data_ptr(), len(lens),
-                                   st_old.data_ptr(), old.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    new, old = torch.zeros(T, H, dv, device=cuda), torch.zeros(T, H, dv, device=cuda)
+    ws = torch.empty(1 << 25, device=cuda)               # enough for every case: the chunked form, though most are too short to gain by it
+    args = lambda st, o: (qkv.data_ptr(), beta.data_ptr() if delta else None, dec.data_ptr(), T, H, G, dk, dv, int(per_channel),  # noqa: E731
+                          int(delta), batch.cu_q.data_ptr(), batch.ctx_start.data_ptr(), batch.state_slots.data_ptr(), len(lens),
+                          st.data_ptr(), o.data_ptr())
+    stream = torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.b2_channel_scan_ws(*args(st_new, new), ws.data_ptr(), ws.numel(), stream))
+    _lib.check(lib.b2_channel_scan(*args(st_old, old), stream))
     ref, st_ref = _reference(qkv, beta, dec, state, lens, ctx, slots, H, G, dk, dv)
     rows = torch.cat([torch.arange(cu[i], cu[i + 1], device=cuda) for i in range(len(lens)) if ctx[i] >= 0])
     for a, b, r in ((new[rows], old[rows], ref[rows]), (st_new, st_old, st_ref)):
@@ -88,6 +90,10 @@ def test_chunked_scan(cuda, lens, ctx, slots, H, G, dk, dv, decay, delta, per_ch
 
 def test_chunked_scan_leaves_short_portions_to_the_token_scan():
     lib = _lib.load()
+    for per_channel in (0, 1):
+        for delta in (0, 1):
+            assert lib.b2_channel_scan_workspace(4096, 1, 16, 128, 128, per_channel, delta) > 0
+            assert lib.b2_channel_scan_workspace(1536, 64, 16, 128, 128, per_channel, delta) == 0
     assert lib.b2_channel_scan_workspace(64, 64, 16, 128, 128, 0, 1) == 0
     assert lib.b2_channel_scan_workspace(4096, 1, 16, 256, 128, 0, 1) == 0
     assert lib.b2_channel_scan_workspace(4096, 1, 16, 126, 128, 0, 1) == 0

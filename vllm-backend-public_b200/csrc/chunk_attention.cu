@@ -563,37 +563,48 @@ chunk_attention_group_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
 // ------------------------------------------------------------------------------------------------- head-tile decode kernel
 // The same rows for head sizes the tensor cores take (dk a multiple of 32, dv one of the prompt kernel's sizes): one CTA per
 // (row, kv head), the query heads of that kv head as the rows of a 16-row operand (two maps: rows 0 - 7 hold the first maps of
-// eight heads, rows 8 - 15 their second), so a K or V row is read once and multiplied for all of them at once.  Four warps take
-// 32 visible keys at a time each, gather their K and V rows from the pages with cp.async (four lanes a row, one page lookup per
-// key), run S = Q K^T and O += P V on mma.sync with the softmax in the accumulator registers, and merge through shared
+// eight heads, rows 8 - 15 their second), so a K or V row is read once and multiplied for all of them at once.  NW warps take
+// 16 visible keys at a time each, gather their K and V rows from the pages with cp.async (four lanes a row, one page lookup per
+// key, a tile ahead), run S = Q K^T and O += P V on mma.sync with the softmax in the accumulator registers, and merge through shared
 // memory, which by then no longer holds tiles.  The keys a single row sees are one exact range: nothing to mask but its end.
-constexpr int kHeadRows = 16, kHeadKeys = 32;
+// Bound: the bytes of K and V.  A warp has one buffer for K and one for V and refills each as soon as it is multiplied, so one of the
+// two is always in flight under the other's arithmetic; 16 keys a tile and 128 registers let 16 warps share an SM.  With 32 keys
+// copied and then multiplied, three CTAs of four warps an SM, 64 rows x 8 kv heads x 1028 keys of 128 took 73 us: two waves, each
+// warp idle while its tile arrived.  NW is 16, 8 or 4 so that a small batch's rows are still shared by 16 warps an SM.
+constexpr int kHeadRows = 16, kHeadKeys = 16;
 
-template <int DVT, bool SIG, int MAPS>
-__global__ void __launch_bounds__(128)
+template <int DVT, bool SIG, int MAPS, int NW>
+__global__ void __launch_bounds__(32 * NW, DVT <= 8 ? 16 / NW : (NW < 8 ? 8 / NW : 1))
 chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
                              const __nv_bfloat16* __restrict__ v_cache, const int32_t* __restrict__ block_tables, int max_nb,
                              const int32_t* __restrict__ cu_q, const int32_t* __restrict__ ctx_start, int n_seq, int H, int G,
                              int dk, int bs, float scale_log2, int chunk, int window, int keep_first, float sink,
                              float sink_logit, const float* __restrict__ sink_logits, const float* __restrict__ head_bias,
-                             const __nv_bfloat16* __restrict__ gate, int64_t gate_stride, HeadShape hs, int skip_rows_from,
+                             const __nv_bfloat16* __restrict__ gate, int64_t gate_stride, HeadShape hs, int skip_rows_from, bool by_seq,
                              __nv_bfloat16* __restrict__ out, int64_t out_stride) {
-    constexpr int DV = 16 * DVT, LDV = DV + 8, PASS = kHeadRows / MAPS, PW = 2 + DV;
+    constexpr int DV = 16 * DVT, LDV = DV + 8, PASS = kHeadRows / MAPS, PW = 2 + DV, NTH = 32 * NW;
     constexpr float kLog2e = 1.4426950408889634f;
-    // q [16][dk + 8], then per warp: K tile [32][MAPS * dk + 8], V tile [32][DV + 8]; the merge reuses the tiles' place
+    // q [16][dk + 8], then per warp: K tile [16][MAPS * dk + 8], V tile [16][DV + 8]; the merge reuses the tiles' place
     extern __shared__ __align__(16) unsigned char head_sm[];
-    const int row = blockIdx.x, g = blockIdx.y;
+    const int g = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int seq = b2::seq_of_row(cu_q, n_seq, row);
-    const int ctx = ctx_start[seq];
     const int QHall = H / G;
-    if (skip_rows_from > 0 && ctx >= 0 && cu_q[seq + 1] - cu_q[seq] >= skip_rows_from) return;    // the tile kernel's
+    // by_seq: a batch with prompt portions for the tile kernel -- the CTAs are the up to skip_rows_from - 1 rows of every short sequence
+    const int per = skip_rows_from - 1;
+    const int seq = by_seq ? blockIdx.x / per : b2::seq_of_row(cu_q, n_seq, blockIdx.x);
+    const int r0 = cu_q[seq], len = cu_q[seq + 1] - r0;
+    int row = by_seq ? r0 + blockIdx.x % per : blockIdx.x;
+    const int ctx = ctx_start[seq];
+    if (by_seq && row >= r0 + len) return;
+    if (skip_rows_from > 0 && ctx >= 0 && len >= skip_rows_from) return;         // the tile kernel's
     if (ctx < 0) {
-        for (int i = tid; i < QHall * DV; i += 128)
-            out[(size_t)row * out_stride + (size_t)g * QHall * DV + i] = __float2bfloat16_rn(0.f);
+        do {
+            for (int i = tid; i < QHall * DV; i += NTH)
+                out[(size_t)row * out_stride + (size_t)g * QHall * DV + i] = __float2bfloat16_rn(0.f);
+        } while (by_seq && (row += per) < r0 + len);
         return;
     }
-    const int pos = ctx + row - cu_q[seq];
+    const int pos = ctx + row - r0;
     const KeySpan span = key_span(pos, pos, chunk, window, keep_first);
     const int32_t* bt = block_tables + (size_t)seq * max_nb;
     const int ldq = dk + 8, ldk = MAPS * dk + 8;
@@ -601,15 +612,59 @@ chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
     __nv_bfloat16* tiles = q_sm + kHeadRows * ldq;
     __nv_bfloat16* kt = tiles + (size_t)w * kHeadKeys * (ldk + LDV);
     __nv_bfloat16* vt = kt + kHeadKeys * ldk;
-    float* part = reinterpret_cast<float*>(tiles);       // [4][16][m, l, O (DV)]
+    float* part = reinterpret_cast<float*>(tiles);       // [NW][16][m, l, O (DV)]
     const uint32_t q_base = b2::smem_u32(q_sm), k_base = b2::smem_u32(kt), v_base = b2::smem_u32(vt);
     const int gq = lane >> 2, tq = lane & 3;
     const float cap_log2 = hs.cap * kLog2e, cap_e = hs.cap > 0.f ? 2.f / hs.cap : 0.f;
+    constexpr int STEP = NW * kHeadKeys;
 
     for (int h0 = 0; h0 < QHall; h0 += PASS) {
         const int QH = min(PASS, QHall - h0);
+        // keys past the end repeat the last one: finite numbers that the mask drops
+        auto key_at = [&](int c) { return span.key(min(c + (lane & 15), span.n - 1)); };
+        auto page_of = [&](int j, int& off) {
+            const int pg = j / bs;
+            off = j - pg * bs;
+            return bt[pg];
+        };
+        int off, page, next_off = 0, next_page = 0;      // of the tile in flight, and of the one behind it
+        auto issue_k = [&]() {
+#pragma unroll
+            for (int kq = 0; kq < kHeadKeys / 8; ++kq) {
+                const int key = kq * 8 + (lane >> 2), c = (lane & 3) * 8;
+                const size_t pg = __shfl_sync(0xffffffffu, page, key);
+                const int of = __shfl_sync(0xffffffffu, off, key);
+#pragma unroll
+                for (int mp = 0; mp < MAPS; ++mp) {
+                    const __nv_bfloat16* ks = k_cache + ((pg * (G * MAPS) + g * MAPS + mp) * bs + of) * dk + c;
+                    __nv_bfloat16* kd = kt + key * ldk + mp * dk + c;
+                    for (int t = 0; t < dk; t += 32) cp_async16(kd + t, ks + t);
+                }
+            }
+        };
+        auto issue_v = [&]() {
+#pragma unroll
+            for (int kq = 0; kq < kHeadKeys / 8; ++kq) {
+                const int key = kq * 8 + (lane >> 2), c = (lane & 3) * 8;
+                const size_t pg = __shfl_sync(0xffffffffu, page, key);
+                const int of = __shfl_sync(0xffffffffu, off, key);
+                const __nv_bfloat16* vs = v_cache + ((pg * G + g) * bs + of) * DV + c;
+                __nv_bfloat16* vd = vt + key * LDV + c;
+#pragma unroll
+                for (int t = 0; t < DV; t += 32) cp_async16(vd + t, vs + t);
+            }
+        };
+        const int first = w * kHeadKeys;
         __syncthreads();                                 // a previous pass is done with the shared memory
-        for (int idx = tid; idx < kHeadRows * (dk / 8); idx += 128) {
+        if (first < span.n) {
+            page = page_of(key_at(first), off);
+            issue_k();
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            issue_v();
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            next_page = page_of(key_at(first + STEP), next_off);
+        }
+        for (int idx = tid; idx < kHeadRows * (dk / 8); idx += NTH) {
             const int r = idx / (dk / 8), c = (idx % (dk / 8)) * 8, h = r % PASS, mp = r / PASS;
             uint4 v = make_uint4(0, 0, 0, 0);
             if (h < QH) v = *reinterpret_cast<const uint4*>(q + (((size_t)row * H + (size_t)g * QHall + h0 + h) * MAPS + mp) * dk + c);
@@ -632,64 +687,49 @@ chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
 #pragma unroll
         for (int n = 0; n < 2 * DVT; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
 
-        for (int c0 = w * kHeadKeys; c0 < span.n; c0 += 4 * kHeadKeys) {
-            // keys past the end repeat the last one: finite numbers that the mask drops
-            const int j = span.key(min(c0 + lane, span.n - 1));
-            const int page = bt[j / bs], off = j % bs;
-            __syncwarp();                                // the previous tile has been read
-#pragma unroll
-            for (int kq = 0; kq < kHeadKeys / 8; ++kq) {
-                const int key = kq * 8 + (lane >> 2), c = (lane & 3) * 8;
-                const size_t pg = __shfl_sync(0xffffffffu, page, key);
-                const int of = __shfl_sync(0xffffffffu, off, key);
-#pragma unroll
-                for (int mp = 0; mp < MAPS; ++mp) {
-                    const __nv_bfloat16* ks = k_cache + ((pg * (G * MAPS) + g * MAPS + mp) * bs + of) * dk + c;
-                    __nv_bfloat16* kd = kt + key * ldk + mp * dk + c;
-                    for (int t = 0; t < dk; t += 32) cp_async16(kd + t, ks + t);
-                }
-                const __nv_bfloat16* vs = v_cache + ((pg * G + g) * bs + of) * DV + c;
-                __nv_bfloat16* vd = vt + key * LDV + c;
-#pragma unroll
-                for (int t = 0; t < DV; t += 32) cp_async16(vd + t, vs + t);
-            }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        for (int c0 = first; c0 < span.n; c0 += STEP) {
+            const bool more = c0 + STEP < span.n;
+            asm volatile("cp.async.wait_group 1;" ::: "memory");     // K is there, V may still be on its way
             __syncwarp();
-            float sc[4][4], sd[MAPS > 1 ? 4 : 1][4];
+            float sc[2][4], sd[MAPS > 1 ? 2 : 1][4];
 #pragma unroll
-            for (int n = 0; n < 4; ++n) {
+            for (int n = 0; n < 2; ++n) {
                 sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
                 if (MAPS > 1) sd[MAPS > 1 ? n : 0][0] = sd[MAPS > 1 ? n : 0][1] = sd[MAPS > 1 ? n : 0][2] = sd[MAPS > 1 ? n : 0][3] = 0.f;
             }
+#pragma unroll 4
             for (int kk = 0; kk < dk; kk += 16) {
-                uint32_t a0, a1, a2, a3;
+                uint32_t a0, a1, a2, a3, b0, b1, b2_, b3;
                 b2::ldmatrix_x4(q_base + 2u * ((lane & 15) * ldq + kk + (lane >> 4) * 8), a0, a1, a2, a3);
-#pragma unroll
-                for (int n2 = 0; n2 < 2; ++n2) {
-                    uint32_t b0, b1, b2_, b3;
-                    const int key = n2 * 16 + (lane >> 4) * 8 + (lane & 7), dim = kk + ((lane >> 3) & 1) * 8;
-                    b2::ldmatrix_x4(k_base + 2u * (key * ldk + dim), b0, b1, b2_, b3);
-                    b2::mma_bf16_16816(sc[2 * n2], a0, a1, a2, a3, b0, b1);
-                    b2::mma_bf16_16816(sc[2 * n2 + 1], a0, a1, a2, a3, b2_, b3);
-                    if (MAPS > 1) {                      // rows 8 - 15 belong to the second maps and take their keys
-                        b2::ldmatrix_x4(k_base + 2u * (key * ldk + dk + dim), b0, b1, b2_, b3);
-                        b2::mma_bf16_16816(sd[MAPS > 1 ? 2 * n2 : 0], a0, a1, a2, a3, b0, b1);
-                        b2::mma_bf16_16816(sd[MAPS > 1 ? 2 * n2 + 1 : 0], a0, a1, a2, a3, b2_, b3);
-                    }
+                const int key = (lane >> 4) * 8 + (lane & 7), dim = kk + ((lane >> 3) & 1) * 8;
+                b2::ldmatrix_x4(k_base + 2u * (key * ldk + dim), b0, b1, b2_, b3);
+                b2::mma_bf16_16816(sc[0], a0, a1, a2, a3, b0, b1);
+                b2::mma_bf16_16816(sc[1], a0, a1, a2, a3, b2_, b3);
+                if (MAPS > 1) {                          // rows 8 - 15 belong to the second maps and take their keys
+                    b2::ldmatrix_x4(k_base + 2u * (key * ldk + dk + dim), b0, b1, b2_, b3);
+                    b2::mma_bf16_16816(sd[0], a0, a1, a2, a3, b0, b1);
+                    b2::mma_bf16_16816(sd[MAPS > 1 ? 1 : 0], a0, a1, a2, a3, b2_, b3);
                 }
             }
             if (MAPS > 1) {
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
+                for (int n = 0; n < 2; ++n) {
                     sc[n][2] = sd[MAPS > 1 ? n : 0][2];
                     sc[n][3] = sd[MAPS > 1 ? n : 0][3];
                 }
             }
+            __syncwarp();                                // the K tile is multiplied: the next one takes its place
+            if (more) {
+                page = next_page;
+                off = next_off;
+                issue_k();
+                next_page = page_of(key_at(c0 + 2 * STEP), next_off);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
             const bool whole = c0 + kHeadKeys <= span.n;
             float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-            for (int n = 0; n < 4; ++n) {
+            for (int n = 0; n < 2; ++n) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     float x = sc[n][e] * scale_log2;
@@ -717,7 +757,7 @@ chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
                 l0 *= f0;
                 l1 *= f1;
 #pragma unroll
-                for (int n = 0; n < 4; ++n) {
+                for (int n = 0; n < 2; ++n) {
                     sc[n][0] = b2::fast_exp2(sc[n][0] - mn0);
                     sc[n][1] = b2::fast_exp2(sc[n][1] - mn0);
                     sc[n][2] = b2::fast_exp2(sc[n][2] - mn1);
@@ -733,20 +773,23 @@ chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
                     o[n][3] *= f1;
                 }
             }
-#pragma unroll
-            for (int ks = 0; ks < 2; ++ks) {
-                const uint32_t a0 = b2::pack_bf16x2(sc[2 * ks][0], sc[2 * ks][1]), a1 = b2::pack_bf16x2(sc[2 * ks][2], sc[2 * ks][3]);
-                const uint32_t a2 = b2::pack_bf16x2(sc[2 * ks + 1][0], sc[2 * ks + 1][1]),
-                               a3 = b2::pack_bf16x2(sc[2 * ks + 1][2], sc[2 * ks + 1][3]);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");     // V is there, the next K may still be on its way
+            __syncwarp();
+            {
+                const uint32_t a0 = b2::pack_bf16x2(sc[0][0], sc[0][1]), a1 = b2::pack_bf16x2(sc[0][2], sc[0][3]);
+                const uint32_t a2 = b2::pack_bf16x2(sc[1][0], sc[1][1]), a3 = b2::pack_bf16x2(sc[1][2], sc[1][3]);
 #pragma unroll
                 for (int n2 = 0; n2 < DVT; ++n2) {
                     uint32_t b0, b1, b2_, b3;
-                    const int key = ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), col = n2 * 16 + (lane >> 4) * 8;
+                    const int key = ((lane >> 3) & 1) * 8 + (lane & 7), col = n2 * 16 + (lane >> 4) * 8;
                     b2::ldmatrix_x4_trans(v_base + 2u * (key * LDV + col), b0, b1, b2_, b3);
                     b2::mma_bf16_16816(o[2 * n2], a0, a1, a2, a3, b0, b1);
                     b2::mma_bf16_16816(o[2 * n2 + 1], a0, a1, a2, a3, b2_, b3);
                 }
             }
+            __syncwarp();                                // the V tile is multiplied
+            if (more) issue_v();
+            asm volatile("cp.async.commit_group;" ::: "memory");
         }
 #pragma unroll
         for (int x = 1; x < 4; x <<= 1) {
@@ -768,37 +811,33 @@ chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
         }
         __syncthreads();
         // a warp per head: merged output of operand row r at column col
-        for (int h = w; h < QH; h += 4) {
+        for (int h = w; h < QH; h += NW) {
             const size_t head = (size_t)g * QHall + h0 + h;
-            float f[MAPS][4];
+            float v[DV / 32], ss = 0.f;
+#pragma unroll
+            for (int c = 0; c < DV / 32; ++c) v[c] = 0.f;
 #pragma unroll
             for (int mp = 0; mp < MAPS; ++mp) {
                 const float* px = part + (size_t)(h + mp * PASS) * PW;
                 float M = -INFINITY, L = 0.f;
 #pragma unroll
-                for (int x = 0; x < 4; ++x) M = fmaxf(M, px[(size_t)x * kHeadRows * PW]);
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
+                for (int x = 0; x < NW; ++x) M = fmaxf(M, px[(size_t)x * kHeadRows * PW]);
+                auto weight = [&](int x) {
                     const float mx = px[(size_t)x * kHeadRows * PW];
-                    f[mp][x] = SIG ? 1.f : (mx == -INFINITY ? 0.f : b2::fast_exp2(mx - M));
-                    L = fmaf(px[(size_t)x * kHeadRows * PW + 1], f[mp][x], L);
-                }
+                    return SIG ? 1.f : (mx == -INFINITY ? 0.f : b2::fast_exp2(mx - M));
+                };
+#pragma unroll
+                for (int x = 0; x < NW; ++x) L = fmaf(px[(size_t)x * kHeadRows * PW + 1], weight(x), L);
                 const float inv = (SIG ? 1.f : (L > 0.f ? 1.f / L : 0.f)) * (mp == 0 ? 1.f : -hs.lambda);
 #pragma unroll
-                for (int x = 0; x < 4; ++x) f[mp][x] *= inv;
-            }
-            float v[DV / 32], ss = 0.f;
+                for (int x = 0; x < NW; ++x) {
+                    const float f = weight(x) * inv;
 #pragma unroll
-            for (int c = 0; c < DV / 32; ++c) {
-                v[c] = 0.f;
-#pragma unroll
-                for (int mp = 0; mp < MAPS; ++mp) {
-                    const float* px = part + (size_t)(h + mp * PASS) * PW + 2 + lane + 32 * c;
-#pragma unroll
-                    for (int x = 0; x < 4; ++x) v[c] = fmaf(px[(size_t)x * kHeadRows * PW], f[mp][x], v[c]);
+                    for (int c = 0; c < DV / 32; ++c) v[c] = fmaf(px[(size_t)x * kHeadRows * PW + 2 + lane + 32 * c], f, v[c]);
                 }
-                ss = fmaf(v[c], v[c], ss);
             }
+#pragma unroll
+            for (int c = 0; c < DV / 32; ++c) ss = fmaf(v[c], v[c], ss);
             float inv = MAPS > 1 ? rsqrtf(b2::warp_sum(ss) / (float)DV + hs.eps) * hs.out_scale : 1.f;
             if (gate) inv *= b2::sigmoid_f(__bfloat162float(gate[(size_t)row * gate_stride + head]));
 #pragma unroll
@@ -808,25 +847,53 @@ chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
     }
 }
 
+template <int DVT, bool SIG, int MAPS, int NW>
+int launch_heads_nw(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables, int max_nb,
+                    const int32_t* cu_q, const int32_t* ctx_start, int n_seq, int ctas, int H, int G, int dk, int bs, float scale, int chunk,
+                    int window, int keep_first, float sink, float sink_logit, const float* sink_logits, const float* head_bias,
+                    const void* gate, int64_t gate_stride, const HeadShape& hs, int skip_from, bool by_seq, void* out, int64_t out_stride,
+                    cudaStream_t st) {
+    constexpr int DV = 16 * DVT;
+    const size_t tiles = (size_t)NW * kHeadKeys * (MAPS * dk + 8 + DV + 8) * sizeof(__nv_bfloat16);
+    const size_t merge = (size_t)NW * kHeadRows * (2 + DV) * sizeof(float);
+    const size_t smem = (size_t)kHeadRows * (dk + 8) * sizeof(__nv_bfloat16) + (tiles > merge ? tiles : merge);
+    auto kern = chunk_attention_heads_kernel<DVT, SIG, MAPS, NW>;
+    if (smem > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<dim3(ctas, G), 32 * NW, smem, st>>>(static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k_cache),
+                                              static_cast<const __nv_bfloat16*>(v_cache), block_tables, max_nb, cu_q, ctx_start, n_seq, H,
+                                              G, dk, bs, scale * 1.4426950408889634f, chunk, window, keep_first, sink, sink_logit, sink_logits,
+                                              head_bias, static_cast<const __nv_bfloat16*>(gate), gate_stride, hs, skip_from, by_seq,
+                                              static_cast<__nv_bfloat16*>(out), out_stride);
+    B2_CUDA_OK(cudaGetLastError());
+    return B2_OK;
+}
+
 template <int DVT, bool SIG, int MAPS>
 int launch_heads(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables, int max_nb,
                  const int32_t* cu_q, const int32_t* ctx_start, int n_seq, int T, int H, int G, int dk, int bs, float scale, int chunk,
                  int window, int keep_first, float sink, float sink_logit, const float* sink_logits, const float* head_bias,
                  const void* gate, int64_t gate_stride, const HeadShape& hs, int skip_from, void* out, int64_t out_stride,
                  cudaStream_t st) {
-    constexpr int DV = 16 * DVT;
-    const size_t tiles = (size_t)4 * kHeadKeys * (MAPS * dk + 8 + DV + 8) * sizeof(__nv_bfloat16);
-    const size_t merge = (size_t)4 * kHeadRows * (2 + DV) * sizeof(float);
-    const size_t smem = (size_t)kHeadRows * (dk + 8) * sizeof(__nv_bfloat16) + (tiles > merge ? tiles : merge);
-    auto kern = chunk_attention_heads_kernel<DVT, SIG, MAPS>;
-    if (smem > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<dim3(T, G), 128, smem, st>>>(static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k_cache),
-                                       static_cast<const __nv_bfloat16*>(v_cache), block_tables, max_nb, cu_q, ctx_start, n_seq, H,
-                                       G, dk, bs, scale * 1.4426950408889634f, chunk, window, keep_first, sink, sink_logit, sink_logits,
-                                       head_bias, static_cast<const __nv_bfloat16*>(gate), gate_stride, hs, skip_from,
-                                       static_cast<__nv_bfloat16*>(out), out_stride);
-    B2_CUDA_OK(cudaGetLastError());
-    return B2_OK;
+    // beside the tile kernel only the rows of sequences below skip_from are left, at most skip_from - 1 a sequence: a CTA for each of
+    // those and not for every row of the batch (4096 rows x 8 kv heads of CTAs that leave at once took 31 us)
+    const bool by_seq = skip_from > 1 && (int64_t)n_seq * (skip_from - 1) < T;
+    const int ctas = by_seq ? n_seq * (skip_from - 1) : T;
+    // warps a CTA: 16 an SM together, as long as each still has a few tiles of keys
+    int64_t keys = (int64_t)max_nb * bs;
+    if (chunk > 0 && chunk < keys) keys = chunk;
+    if (window > 0 && window + keep_first < keys) keys = window + keep_first;
+    const int64_t items = (int64_t)ctas * G;
+    const int nw = items <= 148 && keys >= 512 ? 16 : items <= 296 && keys >= 256 ? 8 : 4;
+#define B2_HEADS_NW(NW)                                                                                                      \
+    return launch_heads_nw<DVT, SIG, MAPS, NW>(q, k_cache, v_cache, block_tables, max_nb, cu_q, ctx_start, n_seq, ctas, H, G, dk, bs, scale, \
+                                               chunk, window, keep_first, sink, sink_logit, sink_logits, head_bias, gate, gate_stride, hs, \
+                                               skip_from, by_seq, out, out_stride, st)
+    if constexpr (DVT <= 8 && MAPS == 1) {               // elsewhere 16 warps would not have the registers or the shared memory
+        if (nw == 16) B2_HEADS_NW(16);
+    }
+    if (nw >= 8) B2_HEADS_NW(8);
+    B2_HEADS_NW(4);
+#undef B2_HEADS_NW
 }
 
 // ------------------------------------------------------------------------------------------------- tiled prompt kernel

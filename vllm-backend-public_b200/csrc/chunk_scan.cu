@@ -18,6 +18,8 @@
 // heads of 128.  The scan token by token waited 200 - 400 cycles a token for shuffles and shared memory whatever the shape.
 #include "b2_act.cuh"
 
+#include <math.h>
+
 namespace {
 
 constexpr int C = 64, NC = 16, NT = 256, JB = 128, LP = C + 4;
@@ -780,10 +782,31 @@ int launch(const ChunkArgs& a, int total_rows, cudaStream_t st) {
 
 }  // namespace
 
+// Scratch (floats) of the chunked form; 0 for sizes it is not built for and for scratch above 2 GiB
 int64_t b2_internal_chunk_scan_floats(int total_rows, int n_seq, int H, int dk, int dv, bool ch, bool delta) {
-    if (dk % 4 || dv % 4 || dk > 128 || n_seq <= 0 || total_rows < 24 * n_seq) return 0;
+    if (dk % 4 || dv % 4 || dk > 128 || n_seq <= 0 || total_rows <= 0) return 0;
     const int64_t n = (int64_t)(total_rows / C + n_seq) * H * Scratch(dk, dv, ch, delta).total;
     return n <= (int64_t)1 << 29 ? n : 0;
+}
+
+// Where the chunked form is the faster one.  Both times are estimated in us from what they measured for heads of 128 x 128 on
+// one B200 (w = dk dv / 16384 scales the products); the host knows the rows and the number of sequences, so lengths are taken equal:
+//   tokens   a chain of 0.20 (delta 0.285, per channel 0.235 / 0.31) a token, or, with many sequences, 5.0 (6.3 / 6.8 / 8.3) ns a
+//            token and head
+//   chunks   0.23 (0.16 / 0.55 / 0.70) a chunk and head for the products, 0.11 a sequence and head for its state, with delta 4.8 a
+//            step of the chain and SM's share of CTAs; at least 40 (80 per channel, 110 with delta too): three launches
+// Measured, tokens -> chunks: 1 x 4096 tokens, 16 heads: 804 -> 250, 1160 -> 470, 963 -> 572, 1254 -> 1006; 1 x 500: 101 -> 43,
+// 146 -> 74, 121 -> 82, 158 -> 144; 64 x 64: 328 -> 377, 413 -> 567: left to the tokens, as are 64 x 24: 147 -> 317.
+bool b2_internal_chunk_scan_pays(int total_rows, int n_seq, int H, int dk, int dv, bool ch, bool delta) {
+    if (total_rows < 2 * n_seq) return false;
+    const float len = (float)total_rows / n_seq, w = dk * dv / 16384.f, steps = ceilf(len / C), heads = (float)n_seq * H;
+    const int kind = (ch ? 2 : 0) + (delta ? 1 : 0);
+    const float chain_tok[4] = {0.20f, 0.285f, 0.235f, 0.31f}, rate_tok[4] = {5.0e-3f, 6.3e-3f, 6.8e-3f, 8.3e-3f};
+    const float per_chunk[4] = {0.23f, 0.16f, 0.55f, 0.70f}, least[4] = {40.f, 40.f, 80.f, 110.f};
+    const float tokens = fmaxf(chain_tok[kind] * (dk <= 64 ? 0.75f : 1.f) * len, rate_tok[kind] * (float)total_rows * H * w);
+    float chunks = (per_chunk[kind] * (0.35f + 0.65f * w) * steps + 0.11f * w) * heads;
+    if (delta) chunks += steps * (3.4f + 1.4f * w) * fmaxf(1.f, heads * ((dv + NC - 1) / NC) / 148.f);
+    return tokens >= 1.1f * fmaxf(chunks, least[kind]);
 }
 
 int b2_internal_chunk_scan(const float* qkv, const float* beta, const float* decay, int total_rows, int H, int G, int dk, int dv,

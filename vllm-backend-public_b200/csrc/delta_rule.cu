@@ -131,61 +131,67 @@ __global__ void recur_prep_kernel(const T* __restrict__ proj, int64_t proj_strid
     }
 }
 
-// The same for channels in vectors of eight whose heads are 1, 2, .. 32 lanes of a warp (dk = 8 .. 256, a power of two): a thread keeps
-// its eight channels over `run` consecutive batch rows, the last taps - 1 inputs and the weights in registers, so every input is
-// read once and 16 bytes at a time; the sums over a head and the partners of a rotation are shuffles.  Vectors behind the q | k | v
-// columns are those of a decay per key channel; small per-head outputs are left to the first column block.
+// The same for channels in vectors of four whose heads are 1, 2, .. 32 lanes of a warp (dk = 4 .. 128, a power of two): a thread keeps
+// its four channels over `run` consecutive batch rows, the last taps - 1 inputs and the weights in registers and the next row in
+// flight, so every input is read once; the sums over a head and the partners of a rotation are shuffles.  Vectors behind the
+// q | k | v columns are those of a decay per key channel; small per-head outputs are left to the first column block.  Four channels
+// and not eight: 64 registers let four CTAs share an SM, and a warp's stores are 512 consecutive bytes.
 // Bound: memory (2 or 4 bytes in and 4 out per channel), with the exact exponentials and divisions of the activation close behind.
-// One CTA a row with scalar accesses and a staging pass took 89 us at 4096 rows of 6144 channels (rotation, no convolution) and
-// 175 us at 3001 (four taps, SiLU, unit vectors); this one 31 and 38.
-template <typename T>
-__device__ __forceinline__ void ld_vec8(const T* p, float (&v)[8]) {
-    if constexpr (sizeof(T) == 2) {
-        b2::ld8(p, v);
-    } else {
-        float a[4], b[4];
-        b2::ld4(p, a);
-        b2::ld4(p + 4, b);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) { v[c] = a[c]; v[4 + c] = b[c]; }
-    }
-}
-
 template <typename T, int TAPS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec sp, const float* __restrict__ conv_w,
                       const int32_t* __restrict__ cu_q, const int32_t* __restrict__ ctx_start, const int32_t* __restrict__ state_slot,
                       int n_seq, int rows, int run, const T* __restrict__ conv_state, float* __restrict__ qkv, float* __restrict__ beta,
                       float* __restrict__ decay) {
     const int H = sp.H, G = sp.G, dk = sp.dk, C = 2 * G * dk + H * sp.dv;
     const int vec = blockIdx.y * 256 + threadIdx.x, lane = threadIdx.x & 31;
-    const int c0 = vec * 8, qk = 2 * G * dk;
+    const int c0 = vec * 4, qk = 2 * G * dk;
     const int r_begin = blockIdx.x * run, r_end = min(rows, r_begin + run);
-    const int P = dk / 8, i0 = c0 % dk, half = sp.rot_dims / 2;          // lanes a head, first entry of this lane's head part
+    const int P = dk / 4, i0 = c0 % dk, half = sp.rot_dims / 2;          // lanes a head, first entry of this lane's head part
     const bool channel = c0 < C, head = c0 < qk;
     const bool turns = head && i0 < sp.rot_dims;
     const bool second = !sp.interleaved && i0 >= half;
     const float scale = c0 < G * dk ? sp.q_scale : sp.k_scale;
-    float w[TAPS][8], hist[TAPS][8];                 // hist[j]: the input j rows back
+    float w[TAPS][4], hist[TAPS][4];                 // hist[j]: the input j rows back
 #pragma unroll
     for (int j = 0; j < TAPS; ++j)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < 4; ++c) {
             hist[j][c] = 0.f;
-            w[j][c] = conv_w && channel ? conv_w[(size_t)(c0 + c) * TAPS + (TAPS - 1 - j)] : 1.f;
+            w[j][c] = 1.f;
         }
-    // a decay per key channel: vectors [C / 8, C / 8 + H dk / 8)
+    if (conv_w && channel) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if constexpr (TAPS == 4) {
+                const float4 t = *reinterpret_cast<const float4*>(conv_w + (size_t)(c0 + c) * 4);
+                w[3][c] = t.x; w[2][c] = t.y; w[1][c] = t.z; w[0][c] = t.w;
+            } else {
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) w[j][c] = conv_w[(size_t)(c0 + c) * TAPS + (TAPS - 1 - j)];
+            }
+        }
+    }
+    // a decay per key channel: vectors [C / 4, C / 4 + H dk / 4)
     const int d0 = c0 - C;
     const bool per_channel = !channel && (sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS || sp.decay_mode == B2_DECAY_CHANNEL_SIGMOID_POW) && d0 < H * dk;
-    float dbias[8];
+    float dbias[4];
     float rate = 0.f;
     if (per_channel) {
         if (sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS) rate = -expf(sp.A_log[d0 / dk]);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) dbias[c] = sp.bias ? sp.bias[d0 + c] : 0.f;
+        for (int c = 0; c < 4; ++c) dbias[c] = sp.bias ? sp.bias[d0 + c] : 0.f;
     }
     int seq = -1, seq_end = r_begin, seq_begin = 0, ctx = -1;
+    float next[4];                                   // a row ahead: nothing of it depends on the row before
+#pragma unroll
+    for (int c = 0; c < 4; ++c) next[c] = 0.f;
+    if (channel) b2::ld4(proj + (size_t)r_begin * proj_stride + c0, next);
     for (int row = r_begin; row < r_end; ++row) {
+        float now[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) now[c] = next[c];
+        if (channel && row + 1 < r_end) b2::ld4(proj + (size_t)(row + 1) * proj_stride + c0, next);
         bool fresh = row == r_begin;
         if (row >= seq_end) {                        // the next sequence with rows
             seq = b2::seq_of_row(cu_q, n_seq, row);
@@ -205,26 +211,27 @@ recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec 
                     for (int j = 1; j < TAPS; ++j) {
                         const int l = li - j;
                         if (l >= 0) {
-                            ld_vec8(proj + (size_t)(row - j) * proj_stride + c0, hist[j]);
+                            b2::ld4(proj + (size_t)(row - j) * proj_stride + c0, hist[j]);
                         } else if (ctx + l >= 0 && st) {
-                            ld_vec8(st + (size_t)(l + TAPS - 1) * C + c0, hist[j]);
+                            b2::ld4(st + (size_t)(l + TAPS - 1) * C + c0, hist[j]);
                         } else {
 #pragma unroll
-                            for (int c = 0; c < 8; ++c) hist[j][c] = 0.f;
+                            for (int c = 0; c < 4; ++c) hist[j][c] = 0.f;
                         }
                     }
                 } else {
 #pragma unroll
                     for (int j = TAPS - 1; j > 0; --j)
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) hist[j][c] = hist[j - 1][c];
+                        for (int c = 0; c < 4; ++c) hist[j][c] = hist[j - 1][c];
                 }
             }
-            ld_vec8(proj + (size_t)row * proj_stride + c0, hist[0]);
-        }
-        float x[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < 4; ++c) hist[0][c] = now[c];
+        }
+        float x[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
             x[c] = hist[0][c];
             if (TAPS > 1 || conv_w) {
                 x[c] = 0.f;
@@ -237,7 +244,7 @@ recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec 
         if (sp.unit) {                               // every lane takes part: heads and value columns may share a warp
             float ss = 0.f;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) ss = fmaf(x[c], x[c], ss);
+            for (int c = 0; c < 4; ++c) ss = fmaf(x[c], x[c], ss);
             for (int m = 1; m < P; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
             sc *= rsqrtf(ss + sp.unit_eps);
         }
@@ -246,24 +253,24 @@ recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec 
             if (sp.interleaved) {
                 if (turns) {
 #pragma unroll
-                    for (int c = 0; c < 8; c += 2) {
+                    for (int c = 0; c < 4; c += 2) {
                         const float co = cs[(i0 + c) >> 1], si = cs[half + ((i0 + c) >> 1)], u = x[c], v = x[c + 1];
                         x[c] = fmaf(u, co, -v * si);
                         x[c + 1] = fmaf(v, co, u * si);
                     }
                 }
             } else {
-                const int src = turns ? (second ? lane - half / 8 : lane + half / 8) : lane;
-                float y[8];
+                const int src = turns ? (second ? lane - half / 4 : lane + half / 4) : lane;
+                float y[4];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) y[c] = __shfl_sync(0xffffffffu, x[c], src);
+                for (int c = 0; c < 4; ++c) y[c] = __shfl_sync(0xffffffffu, x[c], src);
                 if (turns) {
-                    float co[8], si[8];
+                    float co[4], si[4];
                     const int pr = second ? i0 - half : i0;
-                    ld_vec8(cs + pr, co);
-                    ld_vec8(cs + half + pr, si);
+                    b2::ld4(cs + pr, co);
+                    b2::ld4(cs + half + pr, si);
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) x[c] = second ? fmaf(x[c], co[c], y[c] * si[c]) : fmaf(x[c], co[c], -y[c] * si[c]);
+                    for (int c = 0; c < 4; ++c) x[c] = second ? fmaf(x[c], co[c], y[c] * si[c]) : fmaf(x[c], co[c], -y[c] * si[c]);
                 }
             }
         }
@@ -271,18 +278,16 @@ recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec 
             const float f = head ? sc : 1.f;
             float* o = qkv + (size_t)row * C + c0;
             *reinterpret_cast<float4*>(o) = make_float4(x[0] * f, x[1] * f, x[2] * f, x[3] * f);
-            *reinterpret_cast<float4*>(o + 4) = make_float4(x[4] * f, x[5] * f, x[6] * f, x[7] * f);
         } else if (per_channel) {
-            float z[8];
-            ld_vec8(sp.a + (size_t)row * sp.a_stride + d0, z);
+            float z[4];
+            b2::ld4(sp.a + (size_t)row * sp.a_stride + d0, z);
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < 4; ++c) {
                 z[c] += dbias[c];
                 z[c] = sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS ? expf(rate * b2::softplus_f(z[c])) : expf(-b2::softplus_f(-z[c]) * sp.inv_tau);
             }
             float* o = decay + (size_t)row * H * dk + d0;
             *reinterpret_cast<float4*>(o) = make_float4(z[0], z[1], z[2], z[3]);
-            *reinterpret_cast<float4*>(o + 4) = make_float4(z[4], z[5], z[6], z[7]);
         }
     }
     if (blockIdx.y) return;
@@ -609,6 +614,19 @@ __global__ void gated_head_norm_kernel(const float* __restrict__ o, const T* __r
     }
 }
 
+template <typename T>
+__device__ __forceinline__ void ld_vec8(const T* p, float (&v)[8]) {
+    if constexpr (sizeof(T) == 2) {
+        b2::ld8(p, v);
+    } else {
+        float a[4], b[4];
+        b2::ld4(p, a);
+        b2::ld4(p + 4, b);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) { v[c] = a[c]; v[4 + c] = b[c]; }
+    }
+}
+
 // The same with a head in 1, 2, .. 32 lanes of eight entries (dv = 8 .. 256, a power of two): 16-byte accesses, the row read once.
 // Scalar accesses and a warp per head took 27 us at 4096 rows of 16 heads of 128, this 13 (0.78 of the copy rate).
 template <typename T>
@@ -733,15 +751,15 @@ int launch_prep(const void* proj, int64_t proj_stride, const PrepSpec& sp, int T
     const int C = 2 * sp.G * sp.dk + sp.H * sp.dv;
     const size_t smem = (size_t)C * sizeof(float);
     const bool channel_decay = sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS || sp.decay_mode == B2_DECAY_CHANNEL_SIGMOID_POW;
-    const int P = sp.dk / 8;
-    const bool vec = sp.dk % 8 == 0 && P <= 32 && (P & (P - 1)) == 0 && sp.dv % 8 == 0 && sp.taps <= 4 && (conv_w || sp.taps == 1) &&
-                     sp.rot_dims % (sp.interleaved ? 8 : 16) == 0 && b2_aligned16(proj) && (proj_stride * sizeof(A)) % 16 == 0 && b2_aligned16(qkv) &&
-                     (sp.taps == 1 || b2_aligned16(conv_state)) && (!sp.rot_dims || b2_aligned16(sp.cos_sin)) &&
+    const int P = sp.dk / 4;
+    const bool vec = sp.dk % 4 == 0 && P <= 32 && (P & (P - 1)) == 0 && sp.dv % 4 == 0 && sp.taps <= 4 && (conv_w || sp.taps == 1) &&
+                     sp.rot_dims % (sp.interleaved ? 4 : 8) == 0 && b2_aligned16(proj) && proj_stride % 4 == 0 && b2_aligned16(qkv) &&
+                     (sp.taps == 1 || (b2_aligned16(conv_state) && b2_aligned16(conv_w))) && (!sp.rot_dims || b2_aligned16(sp.cos_sin)) &&
                      (!channel_decay || (b2_aligned16(sp.a) && sp.a_stride % 4 == 0 && b2_aligned16(decay)));
     if (vec) {
         // rows a CTA: long runs read the convolution's inputs once; small batches spread over the SMs instead
         const int run = T >= 2048 ? 8 : T >= 512 ? 4 : 1;
-        const dim3 grid((T + run - 1) / run, ((C + (channel_decay ? sp.H * sp.dk : 0)) / 8 + 255) / 256);
+        const dim3 grid((T + run - 1) / run, ((C + (channel_decay ? sp.H * sp.dk : 0)) / 4 + 255) / 256);
 #define B2_PREP_VEC(TAPS)                                                                                                    \
     recur_prep_vec_kernel<A, TAPS><<<grid, 256, 0, st>>>(static_cast<const A*>(proj), proj_stride, sp, conv_w, cu_q, ctx_start, state_slot, \
                                                          n_seq, T, run, static_cast<const A*>(conv_state), qkv, beta, decay)
@@ -836,9 +854,10 @@ extern "C" int b2_channel_scan(const float* qkv, const float* beta, const float*
                               state, o, nullptr, 0, stream);
 }
 
-// fp32 scratch (in floats) with which b2_channel_scan_ws takes the chunked form for these sizes; 0: it needs none
+// fp32 scratch (in floats) to give to b2_channel_scan_ws for these sizes; 0: the scan token by token, which needs none, is the faster
 extern "C" int64_t b2_channel_scan_workspace(int total_rows, int n_seq, int H, int dk, int dv, int decay_per_channel, int delta) {
     if (total_rows <= 0 || n_seq <= 0 || H <= 0 || dk <= 0 || dv <= 0) return 0;
+    if (!b2_internal_chunk_scan_pays(total_rows, n_seq, H, dk, dv, decay_per_channel != 0, delta != 0)) return 0;
     return b2_internal_chunk_scan_floats(total_rows, n_seq, H, dk, dv, decay_per_channel != 0, delta != 0);
 }
 
@@ -852,7 +871,7 @@ extern "C" int b2_channel_scan_ws(const float* qkv, const float* beta, const flo
     B2_REQUIRE(qkv && decay && cu_q && ctx_start && state_slot && state && o && (beta || !delta), B2_EINVAL,
                "recurrence scan: null pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int64_t need = workspace ? b2_channel_scan_workspace(total_rows, n_seq, H, dk, dv, decay_per_channel, delta) : 0;
+    const int64_t need = workspace ? b2_internal_chunk_scan_floats(total_rows, n_seq, H, dk, dv, decay_per_channel != 0, delta != 0) : 0;
     if (need > 0 && workspace_floats >= need && b2_aligned16(qkv) && b2_aligned16(state) && b2_aligned16(o) && b2_aligned16(workspace) &&
         (!decay_per_channel || b2_aligned16(decay)))
         return b2_internal_chunk_scan(qkv, beta, decay, total_rows, H, G, dk, dv, decay_per_channel != 0, delta != 0, cu_q, ctx_start,
