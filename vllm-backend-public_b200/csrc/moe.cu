@@ -720,6 +720,13 @@ extern "C" int b2_moe_experts(const void* h, int64_t h_stride, const void* w_gat
     const bool vec1 = D % ve == 0 && h_stride % ve == 0 && w13_expert_stride % ve == 0 && b2_aligned16(h) &&
                       (!gated || b2_aligned16(w_gate)) && b2_aligned16(w_up);
     const bool vec2 = F % ve == 0 && b2_aligned16(act) && b2_aligned16(w_down);
+    if (act_dtype == B2_ACT_BF16 && b2_internal_moe_tc5_ok(h, h_stride, gated ? w_gate : nullptr, w_up, w_down, w13_expert_stride, D, F, act)) {
+        rc = b2_internal_moe_gate_up_tc5(h, h_stride, w_gate, w_up, w13_expert_stride, sorted, tile_expert, tiles, top, D, F, glu, glu_alpha,
+                                         glu_limit, in_w, act, stream);
+        if (rc == B2_OK) rc = b2_internal_moe_down_tc5(act, w_down, sorted, tile_expert, tiles, D, F, rows, stream);
+        if (rc != B2_OK) return rc;
+        return launch_combine<__nv_bfloat16, float>(rows, place, weight_on_input ? nullptr : weights, T, top, D, add, add_stride, y, y_stride, st);
+    }
     B2_DISPATCH_ACT(act_dtype, A, {
         if (gated)
             moe_gate_up_kernel<A, 2><<<dim3(tiles, (F + kMoeBN - 1) / kMoeBN), 128, 0, st>>>(
