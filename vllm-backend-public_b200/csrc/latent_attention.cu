@@ -480,6 +480,10 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ qa, const __nv_bfl
 // tile against all 16 rows, the row maxima meet in shared memory, every warp writes its 16 x 8 slice of P (bf16) to a
 // shared P tile, and then multiplies the whole P tile with ITS R / 8 output columns of the key rows.  No score is computed
 // twice, and the chain of dependent instructions per tile is an eighth of what one warp per row group would run.
+// Bound: the bytes of the latent rows; behind them shared memory, from which a tile is read twice (scores, values).  Every warp needs
+// all of Q for its keys: it stays in registers (4 per 16 entries and thread, up to R + 64 entries), the scores of a tile add up in four
+// chains, and three barriers a tile remain: the next tile is asked for behind the first, when the one before it is surely read.
+// With Q read from shared memory again for every tile, one chain and four barriers, 64 sequences x 32 heads x 2560 keys took 140 us.
 constexpr int kPLD = kLK + 8;
 
 __device__ __forceinline__ void ldmatrix_x2(uint32_t addr, uint32_t& r0, uint32_t& r1) {
@@ -487,7 +491,7 @@ __device__ __forceinline__ void ldmatrix_x2(uint32_t addr, uint32_t& r0, uint32_
 }
 
 template <int RT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, RT >= 32 ? 1 : 2)
 latent_attention_decode_kernel(const __nv_bfloat16* __restrict__ qa, const __nv_bfloat16* __restrict__ cache,
                                const int32_t* __restrict__ block_tables, int max_nb, const int32_t* __restrict__ cu_q,
                                const int32_t* __restrict__ ctx_start, int H, int dr, int bs, float scale_log2, int window,
@@ -542,39 +546,71 @@ latent_attention_decode_kernel(const __nv_bfloat16* __restrict__ qa, const __nv_
     for (int n = 0; n < NTO; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
     const uint32_t q_base = b2::smem_u32(q_sm), k_base0 = b2::smem_u32(k_sm), p_base = b2::smem_u32(p_sm);
     const int ksteps = Dc / 16;
+    constexpr int QK = RT + 4;                                              // k-steps of Q in registers (R + 64 entries)
     const int ld_key = tid >> 2, ld_sub = (tid & 3) * 8;
+    int page_next = 0, off_next = 0;                                        // of the tile behind the one in flight
+    auto lookup = [&](int kv0) {
+        const int j = min(kv0 + ld_key, pos), pg = j / bs;
+        off_next = j - pg * bs;
+        page_next = bt[pg];
+    };
     auto issue = [&](int kv0, int buf) {
         const int j = kv0 + ld_key;
         __nv_bfloat16* dst = k_sm + (size_t)buf * kLK * LD + ld_key * LD;
         if (j <= pos) {
-            const __nv_bfloat16* src = cache + ((size_t)bt[j / bs] * bs + j % bs) * Dc;
+            const __nv_bfloat16* src = cache + ((size_t)page_next * bs + off_next) * Dc;
             for (int c = ld_sub; c < Dc; c += 32) cp_async16(dst + c, src + c);
         } else {
             for (int c = ld_sub; c < Dc; c += 32) *reinterpret_cast<uint4*>(dst + c) = make_uint4(0, 0, 0, 0);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
+        lookup(kv0 + kLK);
     };
     const int all_tiles = (pos - klo) / kLK + 1, per = (all_tiles + nsplit - 1) / nsplit;
     const int t_begin = zs * per, ntiles = min(all_tiles, t_begin + per);
-    if (t_begin < ntiles) issue(klo + t_begin * kLK, 0);
+    if (t_begin < ntiles) {
+        lookup(klo + t_begin * kLK);
+        issue(klo + t_begin * kLK, 0);
+    }
+    __syncthreads();                                                        // Q is in shared memory
+    uint32_t qf[QK][4];
+#pragma unroll
+    for (int kk = 0; kk < QK; ++kk) {
+        qf[kk][0] = qf[kk][1] = qf[kk][2] = qf[kk][3] = 0u;
+        if (kk < ksteps) b2::ldmatrix_x4(q_base + 2u * ((lane & 15) * LD + kk * 16 + (lane >> 4) * 8), qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3]);
+    }
     for (int t = t_begin; t < ntiles; ++t) {
         const int kv0 = klo + t * kLK, buf = (t - t_begin) & 1;
-        if (t + 1 < ntiles) {
-            issue(kv0 + kLK, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();                                                    // the tile (and, first time, Q) is in shared memory
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                                    // the tile is there; the one before, P and the maxima are consumed
+        if (t + 1 < ntiles) issue(kv0 + kLK, buf ^ 1);
         const uint32_t k_base = k_base0 + (uint32_t)buf * kLK * LD * 2u;
-        float sc[4] = {0.f, 0.f, 0.f, 0.f};                                 // 16 rows x this warp's 8 keys
-#pragma unroll 4
-        for (int kk = 0; kk < ksteps; ++kk) {
+        const uint32_t k_row = k_base + 2u * ((w * 8 + (lane & 7)) * LD + (lane >> 3) * 8);
+        float part[4][4];                                                   // 16 rows x this warp's 8 keys
+#pragma unroll
+        for (int c = 0; c < 4; ++c) part[c][0] = part[c][1] = part[c][2] = part[c][3] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < QK; kk += 2) {
+            if (kk + 1 < ksteps) {
+                uint32_t b0, b1, b2_, b3;
+                b2::ldmatrix_x4(k_row + kk * 32u, b0, b1, b2_, b3);
+                b2::mma_bf16_16816(part[kk & 3], qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], b0, b1);
+                b2::mma_bf16_16816(part[(kk + 1) & 3], qf[kk + 1][0], qf[kk + 1][1], qf[kk + 1][2], qf[kk + 1][3], b2_, b3);
+            } else if (kk < ksteps) {
+                uint32_t b0, b1;
+                ldmatrix_x2(k_row - 2u * (lane >> 4) * 16 + kk * 32u, b0, b1);
+                b2::mma_bf16_16816(part[kk & 3], qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], b0, b1);
+            }
+        }
+        for (int kk = QK; kk < ksteps; ++kk) {
             uint32_t a0, a1, a2, a3, b0, b1;
             b2::ldmatrix_x4(q_base + 2u * ((lane & 15) * LD + kk * 16 + (lane >> 4) * 8), a0, a1, a2, a3);
-            ldmatrix_x2(k_base + 2u * ((w * 8 + (lane & 7)) * LD + kk * 16 + ((lane >> 3) & 1) * 8), b0, b1);
-            b2::mma_bf16_16816(sc, a0, a1, a2, a3, b0, b1);
+            ldmatrix_x2(k_row - 2u * (lane >> 4) * 16 + kk * 32u, b0, b1);
+            b2::mma_bf16_16816(part[0], a0, a1, a2, a3, b0, b1);
         }
+        float sc[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sc[e] = (part[0][e] + part[1][e]) + (part[2][e] + part[3][e]);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int j = kv0 + w * 8 + 2 * tq + (e & 1);
@@ -629,8 +665,8 @@ latent_attention_decode_kernel(const __nv_bfloat16* __restrict__ qa, const __nv_
                 b2::mma_bf16_16816(o[2 * n2 + 1], a0, a1, a2, a3, b2_, b3);
             }
         }
-        __syncthreads();                                                    // the tile, P and the maxima are consumed
     }
+    __syncthreads();                                                        // the maxima are consumed: their place takes the sums
     // the row sums of the eight key slices
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
     l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
