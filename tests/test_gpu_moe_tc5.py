@@ -33,7 +33,8 @@ def test_experts(cuda, rows, D, F, E, top, stacked, on_input, glu):
     ids = torch.stack([torch.randperm(E, generator=g, device=cuda)[:top] for _ in range(rows)]).int().contiguous()
     wts = torch.rand(rows, top, generator=g, device=cuda)
     add = rnd(rows, D).bfloat16()
-    y = ops.moe_experts(h, ids, wts, gate if gated else None, up, down, glu=glu, weight_on_input=on_input, add=add)
+    y = ops.moe_experts(h, ids, wts, gate if gated else None, up, down, glu=glu, glu_alpha=1.702, glu_limit=7.0, weight_on_input=on_input,
+                        add=add)
     ref = add.double()
     for t in range(rows):
         for j in range(top):
