@@ -107,6 +107,7 @@ __device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&v)[8]) {
 
 // Sequence of batch row `row` when rows are grouped by cu[0..n] (cu[0] = 0, cu[n] = rows in the batch).
 __device__ __forceinline__ int seq_of_row(const int32_t* cu, int n, int row) {
+    if (row < n && cu[row] == row && cu[row + 1] > row) return row;      // rows of one each up to here, as in a decode step: no search
     int lo = 0, hi = n - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;

@@ -45,17 +45,8 @@ namespace {
 
 constexpr int kMaxDvPerLane = 16;                    // dv <= 512
 
-// 1 / rms of all H * dk numbers of q and of all G * dk of k, which lie one after the other at `src` (block-wide)
-template <typename T, int W>
-__device__ __forceinline__ void qk_row_scales(const T* src, int nq, int nk, float eps, float* red, float& inv_q, float& inv_k) {
-    float sq = 0.f, sk = 0.f;
-    for (int i = threadIdx.x * W; i < nq + nk; i += blockDim.x * W) {
-        float v[4] = {0.f, 0.f, 0.f, 0.f}, ss = 0.f;
-        if (W == 4) b2::ld4(src + i, v); else v[0] = b2::ld(src + i);
-#pragma unroll
-        for (int c = 0; c < W; ++c) ss = fmaf(v[c], v[c], ss);
-        if (i < nq) sq += ss; else sk += ss;
-    }
+// 1 / rms of nq and of nk numbers whose squares the threads of the block have summed up in parts
+__device__ __forceinline__ void block_scales(float sq, float sk, int nq, int nk, float eps, float* red, float& inv_q, float& inv_k) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     sq = b2::warp_sum(sq);
     sk = b2::warp_sum(sk);
@@ -71,6 +62,20 @@ __device__ __forceinline__ void qk_row_scales(const T* src, int nq, int nk, floa
     }
     inv_q = rsqrtf(sq / (float)nq + eps);
     inv_k = rsqrtf(sk / (float)nk + eps);
+}
+
+// 1 / rms of all H * dk numbers of q and of all G * dk of k, which lie one after the other at `src` (block-wide)
+template <typename T, int W>
+__device__ __forceinline__ void qk_row_scales(const T* src, int nq, int nk, float eps, float* red, float& inv_q, float& inv_k) {
+    float sq = 0.f, sk = 0.f;
+    for (int i = threadIdx.x * W; i < nq + nk; i += blockDim.x * W) {
+        float v[4] = {0.f, 0.f, 0.f, 0.f}, ss = 0.f;
+        if (W == 4) b2::ld4(src + i, v); else v[0] = b2::ld(src + i);
+#pragma unroll
+        for (int c = 0; c < W; ++c) ss = fmaf(v[c], v[c], ss);
+        if (i < nq) sq += ss; else sk += ss;
+    }
+    block_scales(sq, sk, nq, nk, eps, red, inv_q, inv_k);
 }
 
 // Rows [q | k] (+ [v]): partial rotation of the q and k heads, K (rotated) and V pool writes; see the file comment.  NORM:
@@ -124,37 +129,87 @@ __global__ void qk_rope_cache_kernel(const T* __restrict__ qkv, int64_t qkv_stri
 // The same with four entries per access (8 or 16 bytes): every size a multiple of four, the rotated entries a multiple of
 // eight in the (i, i + rot_dims/2) layout so that a group of four and its partners never straddle the halves.
 // A thread takes two groups of four of a head, where they rotate one another the two partners, and the same two in every head it
-// visits: their cosines and sines stay in registers and each input is read once (twice with NORM: the row's sums come first).
-// Bound: memory.  With one group a thread, its partner read again beside it and the table entry by entry, 4096 rows of 32 + 8 heads
-// of 128 with NORM took 56 us; the bytes alone need 14.
+// visits: their cosines and sines stay in registers.  `held`: at most kRopeHeld heads a thread, whose inputs it keeps in registers
+// from the row's sums to the stores, so a row is read once.
+// Bound: memory, and the instructions around it.  With one group a thread, its partner read again beside it, the table entry by entry
+// and the row read a second time behind the norm, 4096 rows of 32 + 8 heads of 128 with NORM took 56 us; the bytes alone need 14.
+constexpr int kRopeHeld = 4;
+
+template <typename T> struct Raw4;
+template <> struct Raw4<float> { using type = float4; };
+template <> struct Raw4<__nv_bfloat16> { using type = uint2; };
+
 template <typename T, bool NORM>
 __global__ void __launch_bounds__(256)
 qk_rope_cache_vec_kernel(const T* __restrict__ qkv, int64_t qkv_stride, int H, int G, int Gv, int dk, int dv, bool v_from_k, int rot_dims,
                          bool interleaved, const int32_t* __restrict__ positions, const float* __restrict__ cos_sin, int max_pos,
                          const int64_t* __restrict__ slots, int bs, const float* __restrict__ q_w, const float* __restrict__ k_w,
                          float eps, T* __restrict__ q_out, T* __restrict__ k_cache, T* __restrict__ v_cache) {
+    using Raw = typename Raw4<T>::type;
     __shared__ float red[16];
     const int row = blockIdx.x;
     const T* src = qkv + (size_t)row * qkv_stride;
     const int64_t slot = slots[row];
-    const int64_t blk = slot >= 0 ? slot / bs : 0;
-    const int off = slot >= 0 ? (int)(slot % bs) : 0;
     int pos = positions[row];
-    pos = pos < 0 ? 0 : (pos >= max_pos ? max_pos - 1 : pos);
-    const float* cs = cos_sin + (size_t)pos * rot_dims;
     const int half = rot_dims / 2, per = (dk + 7) / 8, heads = slot >= 0 ? H + G : H;
     // heads of at most 256 groups of eight: a thread keeps its place in the head; larger ones step through it
-    const int wide = per < (int)blockDim.x ? blockDim.x / per * per : blockDim.x;
-    float inv_q = 1.f, inv_k = 1.f;
-    if (NORM) qk_row_scales<T, 4>(src, H * dk, G * dk, eps, red, inv_q, inv_k);
-    for (int j0 = 0; j0 < per; j0 += wide) {
-        const int j = j0 + (per < wide ? threadIdx.x % per : threadIdx.x), step = per < wide ? wide / per : 1;
-        int hd = per < wide ? threadIdx.x / per : 0;
-        if ((int)threadIdx.x >= wide || j >= per) continue;
+    const int step = per < (int)blockDim.x ? blockDim.x / per : 1, wide = per < (int)blockDim.x ? step * per : blockDim.x;
+    const bool held = per <= wide && H + G <= kRopeHeld * step;
+    const int hd0 = per < (int)blockDim.x ? threadIdx.x / per : 0, jt = threadIdx.x - hd0 * per;
+    const bool in = (int)threadIdx.x < wide;
+    auto place = [&](int j, int& i, int& i2) {
         const bool pairs = !interleaved && j < half / 4;
-        const int i = pairs || interleaved ? (pairs ? 4 * j : 8 * j) : rot_dims + 8 * (j - half / 4);
-        const int i2 = pairs ? i + half : i + 4;
-        const bool two = i2 < dk;
+        i = pairs ? 4 * j : interleaved ? 8 * j : rot_dims + 8 * (j - half / 4);
+        i2 = pairs ? i + half : i + 4;
+        return pairs;
+    };
+    auto load = [&](int hd, int i, int i2, Raw& a, Raw& b) {
+        const T* v = src + (size_t)hd * dk;
+        a = *reinterpret_cast<const Raw*>(v + i);
+        b = i2 < dk ? *reinterpret_cast<const Raw*>(v + i2) : Raw{};
+    };
+    Raw ra[kRopeHeld], rb[kRopeHeld];
+    float inv_q = 1.f, inv_k = 1.f;
+    if (held) {
+        int i, i2;
+        place(jt, i, i2);
+#pragma unroll
+        for (int u = 0; u < kRopeHeld; ++u) {
+            ra[u] = rb[u] = Raw{};
+            if (in && hd0 + u * step < heads) load(hd0 + u * step, i, i2, ra[u], rb[u]);
+        }
+    }
+    pos = pos < 0 ? 0 : (pos >= max_pos ? max_pos - 1 : pos);
+    const float* cs = cos_sin + (size_t)pos * rot_dims;
+    int64_t blk = 0;
+    int off = 0;
+    if (slot >= 0) {                                 // a 64-bit division only where it has to be one
+        if (slot >> 31) { blk = slot / bs; off = (int)(slot % bs); }
+        else { blk = (int)slot / bs; off = (int)slot - (int)blk * bs; }
+    }
+    if (NORM) {
+        if (held) {
+            float sq = 0.f, sk = 0.f;
+#pragma unroll
+            for (int u = 0; u < kRopeHeld; ++u) {
+                float x[4], y[4];
+                b2::ld4(reinterpret_cast<const T*>(&ra[u]), x);
+                b2::ld4(reinterpret_cast<const T*>(&rb[u]), y);
+                float s = 0.f;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) s = fmaf(x[c], x[c], fmaf(y[c], y[c], s));
+                if (hd0 + u * step < H) sq += s; else sk += s;
+            }
+            block_scales(sq, sk, H * dk, G * dk, eps, red, inv_q, inv_k);
+        } else {
+            qk_row_scales<T, 4>(src, H * dk, G * dk, eps, red, inv_q, inv_k);
+        }
+    }
+    for (int j0 = 0; j0 < per; j0 += wide) {
+        const int j = j0 + jt;
+        if (!in || j >= per) continue;
+        int i, i2;
+        const bool pairs = place(j, i, i2), two = i2 < dk;
         float co[4], si[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) { co[c] = 1.f; si[c] = 0.f; }
@@ -166,12 +221,10 @@ qk_rope_cache_vec_kernel(const T* __restrict__ qkv, int64_t qkv_stride, int H, i
             for (int c = 0; c < 4; ++c)
                 if (i + 2 * c < rot_dims) { co[c] = cs[i / 2 + c]; si[c] = cs[half + i / 2 + c]; }
         }
-#pragma unroll 2
-        for (; hd < heads; hd += step) {
-            const T* v = src + (size_t)hd * dk;
-            float x[4], y[4] = {0.f, 0.f, 0.f, 0.f};
-            b2::ld4(v + i, x);
-            if (two) b2::ld4(v + i2, y);
+        auto turn = [&](int hd, const Raw& a0, const Raw& b0) {
+            float x[4], y[4];
+            b2::ld4(reinterpret_cast<const T*>(&a0), x);
+            b2::ld4(reinterpret_cast<const T*>(&b0), y);
             if (NORM) {
                 const float* w = hd < H ? q_w + (size_t)hd * dk : k_w + (size_t)(hd - H) * dk;
                 const float inv = hd < H ? inv_q : inv_k;
@@ -206,16 +259,25 @@ qk_rope_cache_vec_kernel(const T* __restrict__ qkv, int64_t qkv_stride, int H, i
             T* dst = hd < H ? q_out + ((size_t)row * H + hd) * dk : k_cache + (((size_t)blk * G + (hd - H)) * bs + off) * dk;
             b2::st4(dst + i, x);
             if (two) b2::st4(dst + i2, y);
+        };
+        if (held) {
+#pragma unroll
+            for (int u = 0; u < kRopeHeld; ++u)
+                if (hd0 + u * step < heads) turn(hd0 + u * step, ra[u], rb[u]);
+        } else {
+            for (int hd = hd0; hd < heads; hd += step) {
+                Raw a0, b0;
+                load(hd, i, i2, a0, b0);
+                turn(hd, a0, b0);
+            }
         }
     }
     if (slot < 0) return;
     const T* vsrc = v_from_k ? src + (size_t)H * dk : src + (size_t)(H + G) * dk;
     const int pv = dv / 4;
     for (int idx = threadIdx.x; idx < Gv * pv; idx += blockDim.x) {
-        const int g = idx / pv, i = (idx % pv) * 4;
-        float x[4];
-        b2::ld4(vsrc + (size_t)g * dv + i, x);
-        b2::st4(v_cache + (((size_t)blk * Gv + g) * bs + off) * dv + i, x);
+        const int g = idx / pv, i = (idx - g * pv) * 4;
+        *reinterpret_cast<Raw*>(v_cache + (((size_t)blk * Gv + g) * bs + off) * dv + i) = *reinterpret_cast<const Raw*>(vsrc + (size_t)idx * 4);
     }
 }
 
@@ -603,6 +665,253 @@ chunk_attention_group_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
 // warp idle while its tile arrived.  NW is 16, 8 or 4 so that a small batch's rows are still shared by 16 warps an SM.
 constexpr int kHeadRows = 16, kHeadKeys = 16;
 
+// At most eight query heads a kv head (and one map, dk <= 128): the keys are the 16 rows of the operand and the heads its 8 columns,
+// S^T = K Q^T and O^T += V^T P^T.  No half of the tile is padding: half the products, scores, rescales and accumulators of the form
+// below, Q in registers, and P^T turns into an operand by two 8 x 8 transpositions.
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
+    uint32_t y;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+    return y;
+}
+
+constexpr int kFewHeads = 8, kFewDk = 128;
+
+template <int DVT, bool SIG, int NW>
+__global__ void __launch_bounds__(32 * NW, DVT <= 8 && NW < 16 ? 20 / NW : 16 / NW)
+chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
+                             const __nv_bfloat16* __restrict__ v_cache, const int32_t* __restrict__ block_tables, int max_nb,
+                             const int32_t* __restrict__ cu_q, const int32_t* __restrict__ ctx_start, int n_seq, int H, int G,
+                             int dk, int bs, float scale_log2, int chunk, int window, int keep_first, float sink,
+                             float sink_logit, const float* __restrict__ sink_logits, const float* __restrict__ head_bias,
+                             const __nv_bfloat16* __restrict__ gate, int64_t gate_stride, HeadShape hs, int skip_rows_from, bool by_seq,
+                             __nv_bfloat16* __restrict__ out, int64_t out_stride) {
+    constexpr int DV = 16 * DVT, LDV = DV + 8, PW = 2 + DV, NTH = 32 * NW;
+    constexpr float kLog2e = 1.4426950408889634f;
+    // q [8][dk + 8], then per warp: K tile [16][dk + 8], V tile [16][DV + 8]; the merge reuses the tiles' place
+    extern __shared__ __align__(16) unsigned char head_sm[];
+    const int g = blockIdx.y;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int QHall = H / G;
+    // by_seq: a batch with prompt portions for the tile kernel -- the CTAs are the up to skip_rows_from - 1 rows of every short sequence
+    const int per = skip_rows_from - 1;
+    const int seq = by_seq ? blockIdx.x / per : b2::seq_of_row(cu_q, n_seq, blockIdx.x);
+    const int r0 = cu_q[seq], len = cu_q[seq + 1] - r0;
+    int row = by_seq ? r0 + blockIdx.x % per : blockIdx.x;
+    const int ctx = ctx_start[seq];
+    if (by_seq && row >= r0 + len) return;
+    if (skip_rows_from > 0 && ctx >= 0 && len >= skip_rows_from) return;         // the tile kernel's
+    if (ctx < 0) {
+        do {
+            for (int i = tid; i < QHall * DV; i += NTH)
+                out[(size_t)row * out_stride + (size_t)g * QHall * DV + i] = __float2bfloat16_rn(0.f);
+        } while (by_seq && (row += per) < r0 + len);
+        return;
+    }
+    const int pos = ctx + row - r0;
+    const KeySpan span = key_span(pos, pos, chunk, window, keep_first);
+    const int32_t* bt = block_tables + (size_t)seq * max_nb;
+    const int ldq = dk + 8, ldk = dk + 8;
+    __nv_bfloat16* q_sm = reinterpret_cast<__nv_bfloat16*>(head_sm);
+    __nv_bfloat16* tiles = q_sm + kFewHeads * ldq;
+    __nv_bfloat16* kt = tiles + (size_t)w * kHeadKeys * (ldk + LDV);
+    __nv_bfloat16* vt = kt + kHeadKeys * ldk;
+    float* part = reinterpret_cast<float*>(tiles);       // [NW][8][m, l, O (DV)]
+    const uint32_t q_base = b2::smem_u32(q_sm), k_base = b2::smem_u32(kt), v_base = b2::smem_u32(vt);
+    const int gq = lane >> 2, tq = lane & 3;
+    const float cap_log2 = hs.cap * kLog2e, cap_e = hs.cap > 0.f ? 2.f / hs.cap : 0.f;
+    constexpr int STEP = NW * kHeadKeys;
+
+    // keys past the end repeat the last one: finite numbers that the mask drops
+    auto key_at = [&](int c) { return span.key(min(c + (lane & 15), span.n - 1)); };
+    auto page_of = [&](int j, int& off) {
+        const int pg = j / bs;
+        off = j - pg * bs;
+        return bt[pg];
+    };
+    int off, page, next_off = 0, next_page = 0;      // of the tile in flight, and of the one behind it
+    auto issue_k = [&]() {
+#pragma unroll
+        for (int kq = 0; kq < kHeadKeys / 8; ++kq) {
+            const int key = kq * 8 + (lane >> 2), c = (lane & 3) * 8;
+            const size_t pg = __shfl_sync(0xffffffffu, page, key);
+            const int of = __shfl_sync(0xffffffffu, off, key);
+            const __nv_bfloat16* ks = k_cache + ((pg * G + g) * bs + of) * dk + c;
+            __nv_bfloat16* kd = kt + key * ldk + c;
+            for (int t = 0; t < dk; t += 32) cp_async16(kd + t, ks + t);
+        }
+    };
+    auto issue_v = [&]() {
+#pragma unroll
+        for (int kq = 0; kq < kHeadKeys / 8; ++kq) {
+            const int key = kq * 8 + (lane >> 2), c = (lane & 3) * 8;
+            const size_t pg = __shfl_sync(0xffffffffu, page, key);
+            const int of = __shfl_sync(0xffffffffu, off, key);
+            const __nv_bfloat16* vs = v_cache + ((pg * G + g) * bs + of) * DV + c;
+            __nv_bfloat16* vd = vt + key * LDV + c;
+#pragma unroll
+            for (int t = 0; t < DV; t += 32) cp_async16(vd + t, vs + t);
+        }
+    };
+    const int first = w * kHeadKeys;
+    if (first < span.n) {
+        page = page_of(key_at(first), off);
+        issue_k();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        issue_v();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        next_page = page_of(key_at(first + STEP), next_off);
+    }
+    for (int idx = tid; idx < kFewHeads * (dk / 8); idx += NTH) {
+        const int r = idx / (dk / 8), c = (idx % (dk / 8)) * 8;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (r < QHall) v = *reinterpret_cast<const uint4*>(q + ((size_t)row * H + (size_t)g * QHall + r) * dk + c);
+        *reinterpret_cast<uint4*>(q_sm + r * ldq + c) = v;
+    }
+    __syncthreads();
+    uint32_t qf[kFewDk / 16][2];
+#pragma unroll
+    for (int kk = 0; kk < kFewDk / 16; kk += 2) {
+        qf[kk][0] = qf[kk][1] = qf[kk + 1][0] = qf[kk + 1][1] = 0u;
+        if (kk * 16 < dk) b2::ldmatrix_x4(q_base + 2u * ((lane & 7) * ldq + kk * 16 + (lane >> 3) * 8), qf[kk][0], qf[kk][1], qf[kk + 1][0], qf[kk + 1][1]);
+    }
+    // this thread's two heads (of S^T and O^T columns 2 tq and 2 tq + 1)
+    const int ha = g * QHall + min(2 * tq, QHall - 1), hb = g * QHall + min(2 * tq + 1, QHall - 1);
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f, ba = 0.f, bb = 0.f;
+    if (w == 0 && sink > 0.f) {                      // the sink enters once, through the first warp
+        m0 = (sink_logits ? sink_logits[ha] : sink_logit) * kLog2e;
+        m1 = (sink_logits ? sink_logits[hb] : sink_logit) * kLog2e;
+        l0 = l1 = gq == 0 ? sink : 0.f;
+    }
+    if (SIG && head_bias) {
+        ba = head_bias[ha] * kLog2e;
+        bb = head_bias[hb] * kLog2e;
+    }
+    float o[DVT][4];
+#pragma unroll
+    for (int n = 0; n < DVT; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+
+    for (int c0 = first; c0 < span.n; c0 += STEP) {
+        const bool more = c0 + STEP < span.n;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");     // K is there, V may still be on its way
+        __syncwarp();
+        float sc[2][4];                              // two chains
+        sc[0][0] = sc[0][1] = sc[0][2] = sc[0][3] = sc[1][0] = sc[1][1] = sc[1][2] = sc[1][3] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < kFewDk / 16; ++kk) {
+            if (kk * 16 >= dk) break;
+            uint32_t a0, a1, a2, a3;
+            b2::ldmatrix_x4(k_base + 2u * ((lane & 15) * ldk + kk * 16 + (lane >> 4) * 8), a0, a1, a2, a3);
+            b2::mma_bf16_16816(sc[kk & 1], a0, a1, a2, a3, qf[kk][0], qf[kk][1]);
+        }
+        __syncwarp();                                // the K tile is multiplied: the next one takes its place
+        if (more) {
+            page = next_page;
+            off = next_off;
+            issue_k();
+            next_page = page_of(key_at(c0 + 2 * STEP), next_off);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        float p[4], mx0 = -INFINITY, mx1 = -INFINITY;            // keys gq (0, 1) and gq + 8 (2, 3), heads ha and hb
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            float x = (sc[0][e] + sc[1][e]) * scale_log2;
+            const bool in = c0 + gq + (e < 2 ? 0 : 8) < span.n;
+            if (SIG) {
+                x = in ? sigmoid2_f(x + (e & 1 ? bb : ba)) : 0.f;
+            } else {
+                if (hs.cap > 0.f) x = cap_score(x, cap_log2, cap_e);
+                if (!in) x = -INFINITY;
+                if (e & 1) mx1 = fmaxf(mx1, x); else mx0 = fmaxf(mx0, x);
+            }
+            p[e] = x;
+        }
+        if (!SIG) {
+#pragma unroll
+            for (int x = 4; x < 32; x <<= 1) {
+                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, x));
+                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, x));
+            }
+            if (__any_sync(0xffffffffu, mx0 > m0 || mx1 > m1)) {            // else every factor is one
+                const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);     // finite: the tile has at least one key
+                const float f0 = b2::fast_exp2(m0 - mn0), f1 = b2::fast_exp2(m1 - mn1);
+                m0 = mn0;
+                m1 = mn1;
+                l0 *= f0;
+                l1 *= f1;
+#pragma unroll
+                for (int n = 0; n < DVT; ++n) {
+                    o[n][0] *= f0;
+                    o[n][1] *= f1;
+                    o[n][2] *= f0;
+                    o[n][3] *= f1;
+                }
+            }
+            p[0] = b2::fast_exp2(p[0] - m0);
+            p[1] = b2::fast_exp2(p[1] - m1);
+            p[2] = b2::fast_exp2(p[2] - m0);
+            p[3] = b2::fast_exp2(p[3] - m1);
+            l0 += p[0] + p[2];
+            l1 += p[1] + p[3];
+        }
+        const uint32_t b0 = transpose_8x8(b2::pack_bf16x2(p[0], p[1])), b1 = transpose_8x8(b2::pack_bf16x2(p[2], p[3]));
+        asm volatile("cp.async.wait_group 1;" ::: "memory");     // V is there, the next K may still be on its way
+        __syncwarp();
+#pragma unroll
+        for (int n = 0; n < DVT; ++n) {
+            uint32_t a0, a1, a2, a3;
+            const int key = (lane >> 4) * 8 + (lane & 7), col = n * 16 + ((lane >> 3) & 1) * 8;
+            b2::ldmatrix_x4_trans(v_base + 2u * (key * LDV + col), a0, a1, a2, a3);
+            b2::mma_bf16_16816(o[n], a0, a1, a2, a3, b0, b1);
+        }
+        __syncwarp();                                // the V tile is multiplied
+        if (more) issue_v();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+#pragma unroll
+    for (int x = 4; x < 32; x <<= 1) {
+        l0 += __shfl_xor_sync(0xffffffffu, l0, x);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, x);
+    }
+    __syncthreads();                                 // every warp is done with its tiles: the partial results take their place
+    float* pa = part + (size_t)(w * kFewHeads + 2 * tq) * PW;
+    float* pb = pa + PW;
+    if (gq == 0) {
+        pa[0] = m0; pa[1] = l0;
+        pb[0] = m1; pb[1] = l1;
+    }
+#pragma unroll
+    for (int n = 0; n < DVT; ++n) {
+        const int col = 2 + n * 16 + gq;
+        pa[col] = o[n][0];
+        pb[col] = o[n][1];
+        pa[col + 8] = o[n][2];
+        pb[col + 8] = o[n][3];
+    }
+    __syncthreads();
+    for (int h = w; h < QHall; h += NW) {            // a warp per head
+        const size_t head = (size_t)g * QHall + h;
+        const float* px = part + (size_t)h * PW;
+        float v[DV / 32], M = -INFINITY, L = 0.f;
+#pragma unroll
+        for (int c = 0; c < DV / 32; ++c) v[c] = 0.f;
+#pragma unroll
+        for (int x = 0; x < NW; ++x) M = fmaxf(M, px[(size_t)x * kFewHeads * PW]);
+#pragma unroll
+        for (int x = 0; x < NW; ++x) {
+            const float* pw = px + (size_t)x * kFewHeads * PW;
+            const float f = SIG ? 1.f : (pw[0] == -INFINITY ? 0.f : b2::fast_exp2(pw[0] - M));
+            L = fmaf(pw[1], f, L);
+#pragma unroll
+            for (int c = 0; c < DV / 32; ++c) v[c] = fmaf(pw[2 + lane + 32 * c], f, v[c]);
+        }
+        float inv = SIG ? 1.f : (L > 0.f ? 1.f / L : 0.f);
+        if (gate) inv *= b2::sigmoid_f(__bfloat162float(gate[(size_t)row * gate_stride + head]));
+#pragma unroll
+        for (int c = 0; c < DV / 32; ++c)
+            out[(size_t)row * out_stride + head * DV + lane + 32 * c] = __float2bfloat16_rn(v[c] * inv);
+    }
+}
+
 template <int DVT, bool SIG, int MAPS, int NW>
 __global__ void __launch_bounds__(32 * NW, DVT <= 8 ? 16 / NW : (NW < 8 ? 8 / NW : 1))
 chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
@@ -877,17 +1186,21 @@ chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
     }
 }
 
-template <int DVT, bool SIG, int MAPS, int NW>
+template <int DVT, bool SIG, int MAPS, int NW, bool FEW>
 int launch_heads_nw(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables, int max_nb,
                     const int32_t* cu_q, const int32_t* ctx_start, int n_seq, int ctas, int H, int G, int dk, int bs, float scale, int chunk,
                     int window, int keep_first, float sink, float sink_logit, const float* sink_logits, const float* head_bias,
                     const void* gate, int64_t gate_stride, const HeadShape& hs, int skip_from, bool by_seq, void* out, int64_t out_stride,
                     cudaStream_t st) {
     constexpr int DV = 16 * DVT;
+    constexpr int ROWS = FEW ? kFewHeads : kHeadRows;
     const size_t tiles = (size_t)NW * kHeadKeys * (MAPS * dk + 8 + DV + 8) * sizeof(__nv_bfloat16);
-    const size_t merge = (size_t)NW * kHeadRows * (2 + DV) * sizeof(float);
-    const size_t smem = (size_t)kHeadRows * (dk + 8) * sizeof(__nv_bfloat16) + (tiles > merge ? tiles : merge);
-    auto kern = chunk_attention_heads_kernel<DVT, SIG, MAPS, NW>;
+    const size_t merge = (size_t)NW * ROWS * (2 + DV) * sizeof(float);
+    const size_t smem = (size_t)ROWS * (dk + 8) * sizeof(__nv_bfloat16) + (tiles > merge ? tiles : merge);
+    auto kern = [] {
+        if constexpr (FEW) return chunk_attention_few_heads_kernel<DVT, SIG, NW>;
+        else return chunk_attention_heads_kernel<DVT, SIG, MAPS, NW>;
+    }();
     if (smem > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<dim3(ctas, G), 32 * NW, smem, st>>>(static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k_cache),
                                               static_cast<const __nv_bfloat16*>(v_cache), block_tables, max_nb, cu_q, ctx_start, n_seq, H,
@@ -914,15 +1227,21 @@ int launch_heads(const void* q, const void* k_cache, const void* v_cache, const 
     if (window > 0 && window + keep_first < keys) keys = window + keep_first;
     const int64_t items = (int64_t)ctas * G;
     const int nw = items <= 148 && keys >= 512 ? 16 : items <= 296 && keys >= 256 ? 8 : 4;
-#define B2_HEADS_NW(NW)                                                                                                      \
-    return launch_heads_nw<DVT, SIG, MAPS, NW>(q, k_cache, v_cache, block_tables, max_nb, cu_q, ctx_start, n_seq, ctas, H, G, dk, bs, scale, \
+#define B2_HEADS_NW(NW, FEW)                                                                                                      \
+    return launch_heads_nw<DVT, SIG, MAPS, NW, FEW>(q, k_cache, v_cache, block_tables, max_nb, cu_q, ctx_start, n_seq, ctas, H, G, dk, bs, scale, \
                                                chunk, window, keep_first, sink, sink_logit, sink_logits, head_bias, gate, gate_stride, hs, \
                                                skip_from, by_seq, out, out_stride, st)
-    if constexpr (DVT <= 8 && MAPS == 1) {               // elsewhere 16 warps would not have the registers or the shared memory
-        if (nw == 16) B2_HEADS_NW(16);
+    if constexpr (MAPS == 1) {
+        if (H / G <= kFewHeads && dk <= kFewDk) {
+            if constexpr (DVT <= 8) {                    // else 16 warps would not have the shared memory
+                if (nw == 16) B2_HEADS_NW(16, true);
+            }
+            if (nw >= 8) B2_HEADS_NW(8, true);
+            B2_HEADS_NW(4, true);
+        }
     }
-    if (nw >= 8) B2_HEADS_NW(8);
-    B2_HEADS_NW(4);
+    if (nw >= 8) B2_HEADS_NW(8, false);
+    B2_HEADS_NW(4, false);
 #undef B2_HEADS_NW
 }
 

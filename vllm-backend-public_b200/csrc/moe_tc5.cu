@@ -10,8 +10,6 @@
 #include "b2_act.cuh"
 #include "b2_tc5.cuh"
 
-#include <stdlib.h>
-
 namespace {
 using namespace b2tc;
 using bf16 = __nv_bfloat16;
@@ -198,21 +196,14 @@ int encode(CUtensorMap* map, const void* w, int64_t stride, int N, int K) {
     return b2_internal_encode_bf16_sw128(map, w, 3, dims, st, box);
 }
 
-template <int KIND, int ST>
-int launch_st(const ExpertArgs& p, int tiles, cudaStream_t st) {
-    constexpr int OUT = KIND == PAIR ? 64 : 128, SMEM = ST * (W_STAGE + A_STAGE) + 1024;
+template <int KIND>
+int launch(const ExpertArgs& p, int tiles, cudaStream_t st) {
+    constexpr int ST = 3, OUT = KIND == PAIR ? 64 : 128, SMEM = ST * (W_STAGE + A_STAGE) + 1024;
     auto kern = moe_tc5_kernel<KIND, ST>;
     B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     kern<<<dim3(tiles, (p.N + OUT - 1) / OUT), NT, SMEM, st>>>(p);
     B2_CUDA_OK(cudaGetLastError());
     return B2_OK;
-}
-template <int KIND>
-int launch(const ExpertArgs& p, int tiles, cudaStream_t st) {
-    static const int stages = getenv("MOEST") ? atoi(getenv("MOEST")) : 3;
-    if (stages == 4) return launch_st<KIND, 4>(p, tiles, st);
-    if (stages == 5) return launch_st<KIND, 5>(p, tiles, st);
-    return launch_st<KIND, 3>(p, tiles, st);
 }
 
 }  // namespace
