@@ -1,0 +1,73 @@
+"""Decode rows of b2_latent_attention (one row a sequence) against fp64: latents of 128, 256 and 512 numbers with rotated parts that do
+and do not fill their 64 columns, more and fewer heads than a CTA takes, key counts around tiles of 64 and boxes of 16, pages TMA boxes
+fit and do not fit, windows that begin inside a page, keys split over CTAs, and scores that outgrow the first tile's by 2^60 and more.
+
+Tolerance: queries and rows are bf16 in both; the kernel rounds the weights and the result, 2^-9 each of its own:
+|error| <= 2^-8 (sum_j p_j |c_j| + |out|), with 2^-10 more where fp32 scores in the hundreds move the weights."""
+import math
+
+import pytest
+import torch
+
+from b200attn import ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ctx,H,R,dr,bs,window,sink,gate,rise", [
+    ([0, 1, 15, 16, 17, 62, 63, 64, 65, 127, 128, 129], 16, 512, 64, 16, 0, False, False, 0.0),
+    ([700, -1, 3], 32, 512, 64, 16, 0, True, True, 0.0),                 # split over CTAs, padding between
+    ([2000], 33, 512, 64, 32, 0, True, False, 0.0),                      # one head more than a CTA takes, up to 16 shares
+    ([300, 1000, 77, 16], 5, 512, 64, 16, 70, False, True, 0.0),         # windows that begin inside a page
+    ([300, 1000, 77, 64], 40, 256, 32, 24, 100, True, True, 0.0),        # pages of 24: no boxes
+    ([90, 333], 8, 128, 16, 8, 0, False, False, 0.0),
+    ([500] * 80, 32, 128, 64, 64, 0, False, True, 0.0),                  # more CTAs than SMs
+    ([200, 65, 640], 32, 512, 128, 16, 0, False, False, 0.0),
+    ([1500, 130], 16, 512, 64, 16, 0, True, False, 400.0),               # computed a second time
+    ([1500] * 150, 4, 256, 64, 16, 0, False, False, 400.0),              # ... without a split, an odd number of tiles
+    ([1500, 130], 16, 512, 64, 16, 0, True, False, -400.0),              # falling scores: late weights vanish
+])
+def test_latent_decode(cuda, ctx, H, R, dr, bs, window, sink, gate, rise):
+    g = torch.Generator(device=cuda).manual_seed(len(ctx) * 100 + H + window)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=cuda)           # noqa: E731
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    n, Dc = len(ctx), R + dr
+    nb = max(ctx) // bs + 1
+    scale = Dc ** -0.5
+    cache = rnd(n * nb, bs, Dc).bfloat16()
+    tables = torch.randperm(n * nb, generator=g, device=cuda).to(torch.int32).view(n, nb)
+    qa = rnd(n, H, Dc).bfloat16()
+    if rise:                                                             # one column makes the scores climb from the first key to the last
+        qa[:, :, 0] = 8.0
+    for i, c in enumerate(ctx):
+        rows = torch.arange(nb * bs, device=cuda)
+        page, off = tables[i].long()[rows // bs], rows % bs
+        if rise:
+            cache[page, off, 0] = (rows.float() / (c + 1) * rise / 8.0 / scale * math.log(2.0)).bfloat16()
+        lo = max(0, c - window + 1) if window else 0
+        dead = (rows > c) | (rows // bs < lo // bs)                      # behind the end, and pages before the window's first
+        cache[page[dead], off[dead]] = float("nan")
+    sinks = rnd(H) if sink else None
+    wide = rnd(n, H + 3).bfloat16()
+    batch = ops.SeqBatch(i32(list(range(n + 1))), i32(ctx), tables, None, n, n)
+    out = ops.latent_attention(qa, cache, batch, R, scale, window, gate=wide[:, :H] if gate else None, sink_logits=sinks).double()
+    for i, c in enumerate(ctx):
+        if c < 0:
+            assert bool((out[i] == 0).all())
+            continue
+        lo = max(0, c - window + 1) if window else 0
+        rows = torch.arange(lo, c + 1, device=cuda)
+        K = cache[tables[i].long()[rows // bs], rows % bs].double()
+        s = qa[i].double() @ K.T * scale
+        m = s.amax(-1, keepdim=True)
+        if sink:
+            m = torch.maximum(m, sinks.double()[:, None])
+        e = torch.exp(s - m)
+        w = e / (e.sum(-1, keepdim=True) + (torch.exp(sinks.double()[:, None] - m) if sink else 0.0))
+        ref, spr = w @ K[:, :R], w @ K[:, :R].abs()
+        if gate:
+            z = torch.sigmoid(wide[i, :H].double())[:, None]
+            ref, spr = ref * z, spr * z
+        bound = (2.0 ** -8 + (2.0 ** -10 if rise else 0.0)) * (spr + ref.abs()) + 1e-6
+        err = (out[i] - ref).abs()
+        assert bool((err <= bound).all()), (i, c, float((err / bound).max()))

@@ -474,243 +474,6 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ qa, const __nv_bfl
     }
 }
 
-// ------------------------------------------------------------------------------------------------- decode rows
-// bf16, R >= 128, every sequence of the batch has ONE row: a CTA takes one token x up to 16 heads (one m16 row group), so
-// the eight warps cannot share rows -- they share the KEYS of a tile instead.  Warp w scores keys 8w .. 8w+7 of the 64-key
-// tile against all 16 rows, the row maxima meet in shared memory, every warp writes its 16 x 8 slice of P (bf16) to a
-// shared P tile, and then multiplies the whole P tile with ITS R / 8 output columns of the key rows.  No score is computed
-// twice, and the chain of dependent instructions per tile is an eighth of what one warp per row group would run.
-// Bound: the bytes of the latent rows; behind them shared memory, from which a tile is read twice (scores, values).  Every warp needs
-// all of Q for its keys: it stays in registers (4 per 16 entries and thread, up to R + 64 entries), the scores of a tile add up in four
-// chains, and three barriers a tile remain: the next tile is asked for behind the first, when the one before it is surely read.
-// With Q read from shared memory again for every tile, one chain and four barriers, 64 sequences x 32 heads x 2560 keys took 140 us.
-constexpr int kPLD = kLK + 8;
-
-__device__ __forceinline__ void ldmatrix_x2(uint32_t addr, uint32_t& r0, uint32_t& r1) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
-}
-
-template <int RT>
-__global__ void __launch_bounds__(256, RT >= 32 ? 1 : 2)
-latent_attention_decode_kernel(const __nv_bfloat16* __restrict__ qa, const __nv_bfloat16* __restrict__ cache,
-                               const int32_t* __restrict__ block_tables, int max_nb, const int32_t* __restrict__ cu_q,
-                               const int32_t* __restrict__ ctx_start, int H, int dr, int bs, float scale_log2, int window,
-                               const float* __restrict__ sink_logits, const __nv_bfloat16* __restrict__ gate,
-                               int64_t gate_stride, __nv_bfloat16* __restrict__ out, float* __restrict__ ws_o,
-                               float* __restrict__ ws_ml) {
-    constexpr int R = 16 * RT, CW = R / 8, NTO = CW / 8;                    // output columns / n-tiles per warp
-    static_assert(CW % 16 == 0, "a warp owns whole pairs of n-tiles");
-    const int Dc = R + dr, LD = Dc + 8, vecs = Dc / 8;
-    extern __shared__ __align__(16) unsigned char lat_smem[];
-    __nv_bfloat16* q_sm = reinterpret_cast<__nv_bfloat16*>(lat_smem);       // [16][LD]
-    __nv_bfloat16* k_sm = q_sm + 16 * LD;                                   // [2][64][LD]
-    __nv_bfloat16* p_sm = k_sm + 2 * kLK * LD;                              // [16][kPLD]
-    float* mx_sm = reinterpret_cast<float*>(p_sm + 16 * kPLD);              // [8][16]: row maxima, later row sums, per warp
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int seq = blockIdx.x, tok = cu_q[seq];
-    const int h0 = blockIdx.y * 16, nh = min(16, H - h0);
-    const int nsplit = gridDim.z, zs = blockIdx.z;
-    const int ctx = ctx_start[seq];
-    if (ctx < 0) {                                                          // padding
-        if (nsplit > 1) {
-            for (int rr = tid; rr < nh; rr += 256) {
-                float* ml = ws_ml + (((size_t)tok * H + h0 + rr) * nsplit + zs) * 2;
-                ml[0] = -INFINITY;
-                ml[1] = 0.f;
-            }
-        } else {
-            for (int idx = tid; idx < nh * (R / 8); idx += 256)
-                *reinterpret_cast<uint4*>(out + ((size_t)tok * H + h0 + idx / (R / 8)) * R + (idx % (R / 8)) * 8) =
-                    make_uint4(0, 0, 0, 0);
-        }
-        return;
-    }
-    const int pos = ctx;
-    const int klo = window > 0 ? max(pos - window + 1, 0) : 0;
-    const int32_t* bt = block_tables + (size_t)seq * max_nb;
-    for (int idx = tid; idx < 16 * vecs; idx += 256) {
-        const int r = idx / vecs, c = (idx % vecs) * 8;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r < nh) v = *reinterpret_cast<const uint4*>(qa + ((size_t)tok * H + h0 + r) * Dc + c);
-        *reinterpret_cast<uint4*>(q_sm + r * LD + c) = v;
-    }
-    const int gq = lane >> 2, tq = lane & 3;
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-    if (sink_logits && zs == 0) {                                           // every warp keeps the same maximum, its own sums
-        m0 = sink_logits[h0 + min(gq, nh - 1)] * kLog2e;
-        m1 = sink_logits[h0 + min(gq + 8, nh - 1)] * kLog2e;
-        if (w == 0 && tq == 0) l0 = l1 = 1.f;
-    }
-    float o[NTO][4];
-#pragma unroll
-    for (int n = 0; n < NTO; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-    const uint32_t q_base = b2::smem_u32(q_sm), k_base0 = b2::smem_u32(k_sm), p_base = b2::smem_u32(p_sm);
-    const int ksteps = Dc / 16;
-    constexpr int QK = RT + 4;                                              // k-steps of Q in registers (R + 64 entries)
-    const int ld_key = tid >> 2, ld_sub = (tid & 3) * 8;
-    int page_next = 0, off_next = 0;                                        // of the tile behind the one in flight
-    auto lookup = [&](int kv0) {
-        const int j = min(kv0 + ld_key, pos), pg = j / bs;
-        off_next = j - pg * bs;
-        page_next = bt[pg];
-    };
-    auto issue = [&](int kv0, int buf) {
-        const int j = kv0 + ld_key;
-        __nv_bfloat16* dst = k_sm + (size_t)buf * kLK * LD + ld_key * LD;
-        if (j <= pos) {
-            const __nv_bfloat16* src = cache + ((size_t)page_next * bs + off_next) * Dc;
-            for (int c = ld_sub; c < Dc; c += 32) cp_async16(dst + c, src + c);
-        } else {
-            for (int c = ld_sub; c < Dc; c += 32) *reinterpret_cast<uint4*>(dst + c) = make_uint4(0, 0, 0, 0);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        lookup(kv0 + kLK);
-    };
-    const int all_tiles = (pos - klo) / kLK + 1, per = (all_tiles + nsplit - 1) / nsplit;
-    const int t_begin = zs * per, ntiles = min(all_tiles, t_begin + per);
-    if (t_begin < ntiles) {
-        lookup(klo + t_begin * kLK);
-        issue(klo + t_begin * kLK, 0);
-    }
-    __syncthreads();                                                        // Q is in shared memory
-    uint32_t qf[QK][4];
-#pragma unroll
-    for (int kk = 0; kk < QK; ++kk) {
-        qf[kk][0] = qf[kk][1] = qf[kk][2] = qf[kk][3] = 0u;
-        if (kk < ksteps) b2::ldmatrix_x4(q_base + 2u * ((lane & 15) * LD + kk * 16 + (lane >> 4) * 8), qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3]);
-    }
-    for (int t = t_begin; t < ntiles; ++t) {
-        const int kv0 = klo + t * kLK, buf = (t - t_begin) & 1;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                                                    // the tile is there; the one before, P and the maxima are consumed
-        if (t + 1 < ntiles) issue(kv0 + kLK, buf ^ 1);
-        const uint32_t k_base = k_base0 + (uint32_t)buf * kLK * LD * 2u;
-        const uint32_t k_row = k_base + 2u * ((w * 8 + (lane & 7)) * LD + (lane >> 3) * 8);
-        float part[4][4];                                                   // 16 rows x this warp's 8 keys
-#pragma unroll
-        for (int c = 0; c < 4; ++c) part[c][0] = part[c][1] = part[c][2] = part[c][3] = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < QK; kk += 2) {
-            if (kk + 1 < ksteps) {
-                uint32_t b0, b1, b2_, b3;
-                b2::ldmatrix_x4(k_row + kk * 32u, b0, b1, b2_, b3);
-                b2::mma_bf16_16816(part[kk & 3], qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], b0, b1);
-                b2::mma_bf16_16816(part[(kk + 1) & 3], qf[kk + 1][0], qf[kk + 1][1], qf[kk + 1][2], qf[kk + 1][3], b2_, b3);
-            } else if (kk < ksteps) {
-                uint32_t b0, b1;
-                ldmatrix_x2(k_row - 2u * (lane >> 4) * 16 + kk * 32u, b0, b1);
-                b2::mma_bf16_16816(part[kk & 3], qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], b0, b1);
-            }
-        }
-        for (int kk = QK; kk < ksteps; ++kk) {
-            uint32_t a0, a1, a2, a3, b0, b1;
-            b2::ldmatrix_x4(q_base + 2u * ((lane & 15) * LD + kk * 16 + (lane >> 4) * 8), a0, a1, a2, a3);
-            ldmatrix_x2(k_row - 2u * (lane >> 4) * 16 + kk * 32u, b0, b1);
-            b2::mma_bf16_16816(part[0], a0, a1, a2, a3, b0, b1);
-        }
-        float sc[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sc[e] = (part[0][e] + part[1][e]) + (part[2][e] + part[3][e]);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int j = kv0 + w * 8 + 2 * tq + (e & 1);
-            sc[e] = (j >= klo && j <= pos) ? sc[e] * scale_log2 : -INFINITY;
-        }
-        float mx0 = fmaxf(sc[0], sc[1]), mx1 = fmaxf(sc[2], sc[3]);
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        if (tq == 0) {
-            mx_sm[w * 16 + gq] = mx0;
-            mx_sm[w * 16 + gq + 8] = mx1;
-        }
-        __syncthreads();                                                    // every warp's row maxima of this tile
-        float mn0 = m0, mn1 = m1;
-#pragma unroll
-        for (int x = 0; x < 8; ++x) {
-            mn0 = fmaxf(mn0, mx_sm[x * 16 + gq]);
-            mn1 = fmaxf(mn1, mx_sm[x * 16 + gq + 8]);
-        }
-        const float mu0 = mn0 == -INFINITY ? 0.f : mn0, mu1 = mn1 == -INFINITY ? 0.f : mn1;
-        const float c0 = exp2f(m0 - mu0), c1 = exp2f(m1 - mu1);
-        m0 = mn0;
-        m1 = mn1;
-        sc[0] = exp2f(sc[0] - mu0);
-        sc[1] = exp2f(sc[1] - mu0);
-        sc[2] = exp2f(sc[2] - mu1);
-        sc[3] = exp2f(sc[3] - mu1);
-        l0 = l0 * c0 + sc[0] + sc[1];                                       // sums over this warp's keys only
-        l1 = l1 * c1 + sc[2] + sc[3];
-        *reinterpret_cast<uint32_t*>(p_sm + gq * kPLD + w * 8 + 2 * tq) = b2::pack_bf16x2(sc[0], sc[1]);
-        *reinterpret_cast<uint32_t*>(p_sm + (gq + 8) * kPLD + w * 8 + 2 * tq) = b2::pack_bf16x2(sc[2], sc[3]);
-#pragma unroll
-        for (int n = 0; n < NTO; ++n) {
-            o[n][0] *= c0;
-            o[n][1] *= c0;
-            o[n][2] *= c1;
-            o[n][3] *= c1;
-        }
-        __syncthreads();                                                    // the P tile is complete
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            uint32_t a0, a1, a2, a3;
-            b2::ldmatrix_x4(p_base + 2u * ((lane & 15) * kPLD + ks * 16 + (lane >> 4) * 8), a0, a1, a2, a3);
-#pragma unroll
-            for (int n2 = 0; n2 < NTO / 2; ++n2) {
-                uint32_t b0, b1, b2_, b3;
-                const int key = ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), col = w * CW + n2 * 16 + (lane >> 4) * 8;
-                b2::ldmatrix_x4_trans(k_base + 2u * (key * LD + col), b0, b1, b2_, b3);
-                b2::mma_bf16_16816(o[2 * n2], a0, a1, a2, a3, b0, b1);
-                b2::mma_bf16_16816(o[2 * n2 + 1], a0, a1, a2, a3, b2_, b3);
-            }
-        }
-    }
-    __syncthreads();                                                        // the maxima are consumed: their place takes the sums
-    // the row sums of the eight key slices
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-    if (tq == 0) {
-        mx_sm[w * 16 + gq] = l0;
-        mx_sm[w * 16 + gq + 8] = l1;
-    }
-    __syncthreads();
-    l0 = l1 = 0.f;
-#pragma unroll
-    for (int x = 0; x < 8; ++x) {
-        l0 += mx_sm[x * 16 + gq];
-        l1 += mx_sm[x * 16 + gq + 8];
-    }
-    const bool va = gq < nh, vb = gq + 8 < nh;
-    const size_t ra = (size_t)tok * H + h0 + gq, rb = ra + 8;
-    if (nsplit > 1) {
-        if (w == 0 && tq == 0) {
-            if (va) { ws_ml[(ra * nsplit + zs) * 2] = m0; ws_ml[(ra * nsplit + zs) * 2 + 1] = l0; }
-            if (vb) { ws_ml[(rb * nsplit + zs) * 2] = m1; ws_ml[(rb * nsplit + zs) * 2 + 1] = l1; }
-        }
-#pragma unroll
-        for (int n = 0; n < NTO; ++n) {
-            const int col = w * CW + n * 8 + 2 * tq;
-            if (va) *reinterpret_cast<float2*>(ws_o + (ra * nsplit + zs) * R + col) = make_float2(o[n][0], o[n][1]);
-            if (vb) *reinterpret_cast<float2*>(ws_o + (rb * nsplit + zs) * R + col) = make_float2(o[n][2], o[n][3]);
-        }
-        return;
-    }
-    float f0 = l0 > 0.f ? 1.f / l0 : 0.f, f1 = l1 > 0.f ? 1.f / l1 : 0.f;
-    if (gate) {
-        if (va) f0 *= b2::sigmoid_f(__bfloat162float(gate[(size_t)tok * gate_stride + h0 + gq]));
-        if (vb) f1 *= b2::sigmoid_f(__bfloat162float(gate[(size_t)tok * gate_stride + h0 + gq + 8]));
-    }
-#pragma unroll
-    for (int n = 0; n < NTO; ++n) {
-        const int col = w * CW + n * 8 + 2 * tq;
-        if (va) *reinterpret_cast<uint32_t*>(out + ra * R + col) = b2::pack_bf16x2(o[n][0] * f0, o[n][1] * f0);
-        if (vb) *reinterpret_cast<uint32_t*>(out + rb * R + col) = b2::pack_bf16x2(o[n][2] * f1, o[n][3] * f1);
-    }
-}
-
 // ------------------------------------------------------------------------------------------------- prompt portions, per-head keys
 // Long prompt portions are cheaper with keys and values rebuilt per head: a (query, key) pair then costs dn + dr + dv
 // multiplications instead of 2 R + dr.  The latent rows a portion can see are gathered from the pages into one
@@ -970,16 +733,17 @@ inline int latent_sm_count() {
 }
 
 // Which kernel and how many shares of the key tiles per CTA row: a batch that cannot fill the GPU (decode rows) splits its
-// keys over CTAs.  decode: every sequence has one row and the latent is wide enough for eight column slices.
+// keys over CTAs.  decode: every sequence has one row and latent_tc5.cu takes the sizes.
 struct LatentPlan {
     bool decode;
     int nsplit;
 };
-inline LatentPlan latent_plan(int T, int n_seq, int H, int R, int window, int max_nb, int bs) {
+inline LatentPlan latent_plan(int T, int n_seq, int H, int R, int dr, int window, int max_nb, int bs) {
     LatentPlan p;
-    p.decode = T == n_seq && R >= 128;
+    p.decode = T == n_seq && b2_internal_latent_tc5_ok(R, dr);
     const int Hc = H < kLQ ? H : kLQ, Gt = kLQ / Hc;
-    const long ctas = p.decode ? (long)T * ((H + 15) / 16) : (long)(T < T / Gt + n_seq ? T : T / Gt + n_seq) * ((H + Hc - 1) / Hc);
+    const int group = b2_internal_latent_tc5_heads();
+    const long ctas = p.decode ? (long)T * ((H + group - 1) / group) : (long)(T < T / Gt + n_seq ? T : T / Gt + n_seq) * ((H + Hc - 1) / Hc);
     long keys = (long)max_nb * bs;
     const int span = p.decode ? 1 : Gt;
     if (window > 0 && window + span < keys) keys = window + span;
@@ -1007,14 +771,9 @@ int launch_latent_mma(void* out, const void* qa, const void* cache, const int32_
     float* ws_ml = ws ? ws + (size_t)T * H * nsplit * 16 * RT : nullptr;
     if constexpr (RT >= 8) {
         if (decode) {
-            const size_t dsm = (size_t)(16 + 2 * kLK) * (Dc + 8) * sizeof(__nv_bfloat16) + 16 * kPLD * sizeof(__nv_bfloat16) +
-                               128 * sizeof(float);
-            auto dk = latent_attention_decode_kernel<RT>;
-            if (dsm > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(dk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
-            dk<<<dim3(T, (H + 15) / 16, nsplit), 256, dsm, st>>>(
-                static_cast<const __nv_bfloat16*>(qa), static_cast<const __nv_bfloat16*>(cache), block_tables, max_nb, cu_q, ctx_start,
-                H, dr, bs, scale * kLog2e, window, sink_logits, static_cast<const __nv_bfloat16*>(gate), gate_stride,
-                static_cast<__nv_bfloat16*>(out), ws_o, ws_ml);
+            const int rc = b2_internal_latent_tc5(out, qa, cache, block_tables, max_nb, cu_q, ctx_start, T, H, 16 * RT, dr, bs, scale, window,
+                                                  sink_logits, gate, gate_stride, nsplit, ws_o, ws_ml, st);
+            if (rc != B2_OK) return rc;
             if (nsplit > 1)
                 latent_merge_kernel<<<T * H, 128, 0, st>>>(ws_o, ws_ml, nsplit, 16 * RT, H, static_cast<const __nv_bfloat16*>(gate),
                                                            gate_stride, static_cast<__nv_bfloat16*>(out));
@@ -1044,7 +803,7 @@ inline bool latent_mma_ok(int act_dtype, int R, int dr, const void* qa, const vo
 extern "C" int64_t b2_latent_attention_workspace(int act_dtype, int T, int n_seq, int H, int R, int dr, int bs, int window,
                                                  int max_nb) {
     if (T <= 0 || n_seq <= 0 || H <= 0 || !latent_mma_ok(act_dtype, R, dr, nullptr, nullptr, nullptr)) return 0;
-    const int n = latent_plan(T, n_seq, H, R, window, max_nb, bs).nsplit;
+    const int n = latent_plan(T, n_seq, H, R, dr, window, max_nb, bs).nsplit;
     return n > 1 ? (int64_t)T * H * n * (R + 2) : 0;
 }
 
@@ -1097,7 +856,7 @@ extern "C" int b2_latent_attention(void* out, const void* qa, const void* cache,
     B2_REQUIRE(out && qa && cache && block_tables && cu_q && ctx_start, B2_EINVAL, "latent_attention: null pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (latent_mma_ok(act_dtype, R, dr, qa, cache, out)) {
-        const LatentPlan plan = latent_plan(T, n_seq, H, R, window, max_nb, bs);
+        const LatentPlan plan = latent_plan(T, n_seq, H, R, dr, window, max_nb, bs);
         int nsplit = plan.nsplit;
         if (nsplit > 1 && (!workspace || workspace_floats < (int64_t)T * H * nsplit * (R + 2))) nsplit = 1;
 #define B2_LAT(RT)                                                                                                            \
