@@ -140,7 +140,7 @@ template <> struct Raw4<float> { using type = float4; };
 template <> struct Raw4<__nv_bfloat16> { using type = uint2; };
 
 template <typename T, bool NORM>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 4 : 3)
 qk_rope_cache_vec_kernel(const T* __restrict__ qkv, int64_t qkv_stride, int H, int G, int Gv, int dk, int dv, bool v_from_k, int rot_dims,
                          bool interleaved, const int32_t* __restrict__ positions, const float* __restrict__ cos_sin, int max_pos,
                          const int64_t* __restrict__ slots, int bs, const float* __restrict__ q_w, const float* __restrict__ k_w,

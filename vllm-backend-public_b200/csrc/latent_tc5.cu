@@ -199,8 +199,14 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
 #pragma unroll 1
             for (int t = 0; t < nt; ++t) {
                 const int it = it0 + t, s = it & 1;
-                if (t + 1 < nt) scores(t + 1);
-                wait(bar(PR + s), (it >> 1) & 1, failed);
+                bool ahead = t + 1 < nt;             // the next scores go first if their tile is there, else behind this output
+                for (uint32_t spins = 0; !b2::mbar_try_wait(bar(PR + s), (it >> 1) & 1);) {
+                    if (ahead && b2::mbar_try_wait(bar(FULL + (s ^ 1)), ((it + 1) >> 1) & 1)) {
+                        scores(t + 1);
+                        ahead = false;
+                    }
+                    if (*failed || ++spins > (1u << 22)) { *failed = 1; break; }
+                }
                 tc_fence_after();
                 if (elect_one()) {
                     const uint32_t vl = desc_lo(ring + s * (KT * 128), SUB), pl = desc_lo(p_sm + s * (KT * 128), 16);
@@ -214,6 +220,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
                     if (t + 1 == nt) mma_commit(bar(END));
                 }
                 __syncwarp();
+                if (ahead) scores(t + 1);
             }
             wait(bar(END), pass, failed);
         } else {
