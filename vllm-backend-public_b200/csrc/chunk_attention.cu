@@ -737,7 +737,9 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
             const int of = __shfl_sync(0xffffffffu, off, key);
             const __nv_bfloat16* ks = k_cache + ((pg * G + g) * bs + of) * dk + c;
             __nv_bfloat16* kd = kt + key * ldk + c;
-            for (int t = 0; t < dk; t += 32) cp_async16(kd + t, ks + t);
+#pragma unroll
+            for (int t = 0; t < kFewDk; t += 32)
+                if (t < dk) cp_async16(kd + t, ks + t);
         }
     };
     auto issue_v = [&]() {
@@ -794,14 +796,15 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
         const bool more = c0 + STEP < span.n;
         asm volatile("cp.async.wait_group 1;" ::: "memory");     // K is there, V may still be on its way
         __syncwarp();
-        float sc[2][4];                              // two chains
-        sc[0][0] = sc[0][1] = sc[0][2] = sc[0][3] = sc[1][0] = sc[1][1] = sc[1][2] = sc[1][3] = 0.f;
+        float sc[4][4];                              // four chains
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sc[c][0] = sc[c][1] = sc[c][2] = sc[c][3] = 0.f;
 #pragma unroll
         for (int kk = 0; kk < kFewDk / 16; ++kk) {
             if (kk * 16 >= dk) break;
             uint32_t a0, a1, a2, a3;
             b2::ldmatrix_x4(k_base + 2u * ((lane & 15) * ldk + kk * 16 + (lane >> 4) * 8), a0, a1, a2, a3);
-            b2::mma_bf16_16816(sc[kk & 1], a0, a1, a2, a3, qf[kk][0], qf[kk][1]);
+            b2::mma_bf16_16816(sc[kk & 3], a0, a1, a2, a3, qf[kk][0], qf[kk][1]);
         }
         __syncwarp();                                // the K tile is multiplied: the next one takes its place
         if (more) {
@@ -814,7 +817,7 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
         float p[4], mx0 = -INFINITY, mx1 = -INFINITY;            // keys gq (0, 1) and gq + 8 (2, 3), heads ha and hb
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            float x = (sc[0][e] + sc[1][e]) * scale_log2;
+            float x = ((sc[0][e] + sc[1][e]) + (sc[2][e] + sc[3][e])) * scale_log2;
             const bool in = c0 + gq + (e < 2 ? 0 : 8) < span.n;
             if (SIG) {
                 x = in ? sigmoid2_f(x + (e & 1 ? bb : ba)) : 0.f;
@@ -826,12 +829,12 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
             p[e] = x;
         }
         if (!SIG) {
+            if (__any_sync(0xffffffffu, mx0 > m0 || mx1 > m1)) {            // a lane's keys exceed the maximum: else every factor is one
 #pragma unroll
-            for (int x = 4; x < 32; x <<= 1) {
-                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, x));
-                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, x));
-            }
-            if (__any_sync(0xffffffffu, mx0 > m0 || mx1 > m1)) {            // else every factor is one
+                for (int x = 4; x < 32; x <<= 1) {
+                    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, x));
+                    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, x));
+                }
                 const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);     // finite: the tile has at least one key
                 const float f0 = b2::fast_exp2(m0 - mn0), f1 = b2::fast_exp2(m1 - mn1);
                 m0 = mn0;

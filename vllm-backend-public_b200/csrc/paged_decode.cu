@@ -926,54 +926,62 @@ __device__ __forceinline__ uint32_t dyn_runs_of_item_fast(uint32_t ci0, uint32_t
 // every partial run's end sit on the consumers' critical path, the merging CTA stalls its own pipeline, and the extra
 // code cost the 128-register fp8 instantiation its spill-free allocation.)
 // thread -> (head tid128/16 [+8], 8 consecutive d); partials were written by other CTAs: read through L2 (ld.cg).
+// merge_runs: the runs that start at the chunks [c, cend) of the item beginning at chunk ci0
+template <int HEADS>
+__device__ __forceinline__ void merge_runs(const float* ws_o, const float* ws_lse, uint32_t ci0, uint32_t c, uint32_t cend, uint32_t S,
+                                           uint32_t stat_total, uint32_t NC, int h, int dc, float& m_run, float& den, float (&num)[8]) {
+    constexpr int MAXC = 4;
+    m_run = -INFINITY;
+    den = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) num[i] = 0.f;
+    while (c < cend) {
+        float lse[MAXC];
+        float4 o0[MAXC], o1[MAXC];
+#pragma unroll
+        for (int i = 0; i < MAXC; ++i) {
+            while (c < cend && !dyn_is_start(c, c - ci0, S, stat_total)) ++c;
+            lse[i] = -INFINITY;
+            o0[i] = o1[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c < cend) {
+                const int64_t slot = dyn_slot(c, S, stat_total, NC);
+                lse[i] = __ldcg(ws_lse + slot * HEADS + h);
+                const float4* po = reinterpret_cast<const float4*>(ws_o + (slot * HEADS + h) * D + dc);
+                o0[i] = __ldcg(po);
+                o1[i] = __ldcg(po + 1);
+                ++c;
+            }
+        }
+        float mx = m_run;
+#pragma unroll
+        for (int i = 0; i < MAXC; ++i) mx = fmaxf(mx, lse[i]);
+        if (mx == -INFINITY) continue;
+        const float a = m_run == -INFINITY ? 0.f : exp2f(m_run - mx);
+        den *= a;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) num[i] *= a;
+#pragma unroll
+        for (int i = 0; i < MAXC; ++i) {
+            const float w = lse[i] == -INFINITY ? 0.f : exp2f(lse[i] - mx);
+            den += w;
+            num[0] = fmaf(w, o0[i].x, num[0]); num[1] = fmaf(w, o0[i].y, num[1]);
+            num[2] = fmaf(w, o0[i].z, num[2]); num[3] = fmaf(w, o0[i].w, num[3]);
+            num[4] = fmaf(w, o1[i].x, num[4]); num[5] = fmaf(w, o1[i].y, num[5]);
+            num[6] = fmaf(w, o1[i].z, num[6]); num[7] = fmaf(w, o1[i].w, num[7]);
+        }
+        m_run = mx;
+    }
+}
+
 template <int HEADS>
 __device__ __forceinline__ void merge_item(__nv_bfloat16* __restrict__ out_rows, const float* ws_o, const float* ws_lse,
                                            uint32_t ci0, uint32_t nck, uint32_t S, uint32_t stat_total, uint32_t NC,
                                            int nheads, int tid128) {
-    constexpr int MAXC = 4;
     const uint32_t cend = ci0 + nck;
     const int dc = (tid128 & 15) * 8;
     for (int h = tid128 >> 4; h < nheads; h += 8) {
-        float m_run = -INFINITY, den = 0.f, num[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) num[i] = 0.f;
-        uint32_t c = ci0;
-        while (c < cend) {
-            float lse[MAXC];
-            float4 o0[MAXC], o1[MAXC];
-#pragma unroll
-            for (int i = 0; i < MAXC; ++i) {
-                while (c < cend && !dyn_is_start(c, c - ci0, S, stat_total)) ++c;
-                lse[i] = -INFINITY;
-                o0[i] = o1[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (c < cend) {
-                    const int64_t slot = dyn_slot(c, S, stat_total, NC);
-                    lse[i] = __ldcg(ws_lse + slot * HEADS + h);
-                    const float4* po = reinterpret_cast<const float4*>(ws_o + (slot * HEADS + h) * D + dc);
-                    o0[i] = __ldcg(po);
-                    o1[i] = __ldcg(po + 1);
-                    ++c;
-                }
-            }
-            float mx = m_run;
-#pragma unroll
-            for (int i = 0; i < MAXC; ++i) mx = fmaxf(mx, lse[i]);
-            if (mx == -INFINITY) continue;
-            const float a = m_run == -INFINITY ? 0.f : exp2f(m_run - mx);
-            den *= a;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) num[i] *= a;
-#pragma unroll
-            for (int i = 0; i < MAXC; ++i) {
-                const float w = lse[i] == -INFINITY ? 0.f : exp2f(lse[i] - mx);
-                den += w;
-                num[0] = fmaf(w, o0[i].x, num[0]); num[1] = fmaf(w, o0[i].y, num[1]);
-                num[2] = fmaf(w, o0[i].z, num[2]); num[3] = fmaf(w, o0[i].w, num[3]);
-                num[4] = fmaf(w, o1[i].x, num[4]); num[5] = fmaf(w, o1[i].y, num[5]);
-                num[6] = fmaf(w, o1[i].z, num[6]); num[7] = fmaf(w, o1[i].w, num[7]);
-            }
-            m_run = mx;
-        }
+        float m_run, den, num[8];
+        merge_runs<HEADS>(ws_o, ws_lse, ci0, ci0, cend, S, stat_total, NC, h, dc, m_run, den, num);
         const float inv = den > 0.f ? 1.f / den : 0.f;
         uint4 pk;
         pk.x = b2::pack_bf16x2(num[0] * inv, num[1] * inv);
@@ -1234,14 +1242,42 @@ __global__ void zero_counter_kernel(uint32_t* counter) {
     if (threadIdx.x == 0) *counter = 0u;
 }
 
-// One block per item (sequence b = blockIdx.y, item j = blockIdx.x): combine its partial runs unless one
-// run covered it.  Which chunks start a run, and where their partials live, follows from (Ctot, S, NC)
+// One head of an item in a block: the eight groups of 16 threads take an eighth of its chunks each and meet in shared memory.
+template <int HEADS>
+__device__ __forceinline__ void merge_head(__nv_bfloat16* __restrict__ out_row, const float* ws_o, const float* ws_lse, uint32_t ci0,
+                                           uint32_t nck, uint32_t S, uint32_t stat_total, uint32_t NC, int h, int tid) {
+    __shared__ float s_m[8], s_den[8], s_num[8][D];
+    const int grp = tid >> 4, dc = (tid & 15) * 8;
+    const uint32_t part = (nck + 7) / 8, c = min(nck, grp * part), cend = min(nck, c + part);
+    float m_run, den, num[8];
+    merge_runs<HEADS>(ws_o, ws_lse, ci0, ci0 + c, ci0 + cend, S, stat_total, NC, h, dc, m_run, den, num);
+    if ((tid & 15) == 0) {
+        s_m[grp] = m_run;
+        s_den[grp] = den;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s_num[grp][dc + i] = num[i];
+    __syncthreads();
+    float mx = -INFINITY, sum = 0.f, v = 0.f;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) mx = fmaxf(mx, s_m[g]);
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+        const float w = s_m[g] == -INFINITY ? 0.f : exp2f(s_m[g] - mx);
+        sum = fmaf(w, s_den[g], sum);
+        v = fmaf(w, s_num[g][tid], v);
+    }
+    out_row[tid] = __float2bfloat16_rn(sum > 0.f ? v / sum : 0.f);
+}
+
+// One block per item (sequence b = blockIdx.y, item j = blockIdx.x) or, with per_head, per head of one: combine its partial
+// runs unless one run covered it.  Which chunks start a run, and where their partials live, follows from (Ctot, S, NC)
 // -- the same arithmetic as the main kernel, no flags in memory.
 template <int HEADS>
 __global__ void __launch_bounds__(128)
 merge_chunks_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ ws_o,
                     const float* __restrict__ ws_lse, const int32_t* __restrict__ seq_lens, int B, int Hkv, int G,
-                    int HG, int64_t out_stride, int ct, int static_pct, uint32_t NC, uint32_t* counter) {
+                    int HG, int64_t out_stride, int ct, int static_pct, uint32_t NC, uint32_t* counter, bool per_head) {
     __shared__ uint32_t s_red[2][4];
     const int tid = threadIdx.x, b = blockIdx.y, j = blockIdx.x;
     const int IPB = Hkv * HG;
@@ -1267,7 +1303,7 @@ merge_chunks_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ w
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // the decode grid is complete: leave the claim counter at zero for the next call on this workspace
     // (b2_decode_plan_run relies on it and launches no zeroing kernel; b2_paged_decode zeroes it itself)
-    if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) *counter = 0u;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && tid == 0) *counter = 0u;
     const uint32_t nck = chunks_of(seq_lens[b], ct);
     if (nck <= 1) return;                                 // a single chunk is always written directly
     const uint32_t S = dyn_static_chunks(total, NC, static_pct);
@@ -1276,8 +1312,10 @@ merge_chunks_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ w
     if (dyn_runs_of_item_fast(ci0, nck, S, stat_total) == 1) return;   // one run covered the item: already in `out`
     const int kvh = j / HG, hg = j - kvh * HG;
     const int head0 = kvh * G + hg * HEADS;
-    merge_item<HEADS>(out + b * out_stride + (int64_t)head0 * D, ws_o, ws_lse, ci0, nck, S, stat_total, NC,
-                      min(HEADS, G - hg * HEADS), tid);
+    const int nheads = min(HEADS, G - hg * HEADS), h = blockIdx.z;
+    __nv_bfloat16* rows = out + b * out_stride + (int64_t)head0 * D;
+    if (!per_head) merge_item<HEADS>(rows, ws_o, ws_lse, ci0, nck, S, stat_total, NC, nheads, tid);
+    else if (h < nheads) merge_head<HEADS>(rows + (int64_t)h * D, ws_o, ws_lse, ci0, nck, S, stat_total, NC, h, tid);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1522,14 +1560,17 @@ int launch_decode(const CUtensorMap& tmK, const CUtensorMap& tmV, const DecodePa
         cfg.numAttrs = zero_first ? 1 : 0;
         B2_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmK, tmV, p));
         cudaLaunchConfig_t cfg2 = {};
-        cfg2.gridDim = dim3(p.Hkv * p.HG, p.B);
+        // few items have many runs each (chunks shrink to 64 tokens): a block per item walked them four at a time, 32 us of the 45
+        // that 4 sequences of 8192 tokens on 2 kv heads took; a block per head shares them out.  Many items have few runs.
+        const bool per_head = p.Hkv * p.HG * p.B < sm_count();
+        cfg2.gridDim = dim3(p.Hkv * p.HG, p.B, per_head ? std::min(8 * NT, p.G) : 1);
         cfg2.blockDim = dim3(128);
         cfg2.stream = st;
         cfg2.attrs = at;
         cfg2.numAttrs = 1;
         B2_CUDA_OK(cudaLaunchKernelEx(&cfg2, merge_chunks_kernel<8 * NT>, p.out, (const float*)p.ws_o,
                                       (const float*)p.ws_lse, p.seq_lens, p.B, p.Hkv, p.G, p.HG, p.out_stride,
-                                      p.chunk_tokens, p.static_pct, (uint32_t)grid, p.counter));
+                                      p.chunk_tokens, p.static_pct, (uint32_t)grid, p.counter, per_head));
         return B2_OK;
     }
     auto kern = paged_decode_split_kernel<BS, FP8, NT, NSTAGE>;
@@ -1769,6 +1810,12 @@ extern "C" int b2_paged_decode_plan_splits(const int32_t* seq_lens_host, int B, 
             streamed += L * ipb;
         }
     }
+    // Short sequences in one wave: the single-pass grid is one launch (KV write included) and streams a CTA's tokens at about 10.7 ns
+    // each behind 3.3 us; the dynamic schedule starts at 9.6 us whatever the batch (write, counter, decode, merge).  Measured bf16, 1 - 32
+    // sequences, single / dynamic, in a graph: 4.7 / 10.5 us at 128 tokens, 8.4 / 11.6 at 512, 13.8 / 13.7 at 1024; fp8 4.9 / 10.2,
+    // 7.8 / 11.7, 12.5 / 13.5.  Launched one by one the three extra launches cost another 5 us.
+    constexpr int64_t SHORT_TOK = 640;
+    if (makespan <= SHORT_TOK + OVERHEAD_TOK) return 1;
     const double ideal = (double)total / NC;
     // fp8 (three CTAs per SM) is paced by its consumer warps, not by HBM: an idle slot is lost throughput, so the
     // single-pass grid only wins when its waves are nearly full (measured: config 3 dynamic 6.4 vs grid 6.1 TB/s)
