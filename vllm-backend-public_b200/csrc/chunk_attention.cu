@@ -32,10 +32,10 @@
 //   b2_qk_norm_rope_cache  rows [q | k | v]: all of q (H * dk numbers) and all of k (G * dk) are RMS-normed as one row each,
 //                        before the split into heads (fp32 weights of those sizes), then rotated and written as above; the
 //                        numbers stay in fp32 between the norm and the rotation.
-//   b2_chunk_attention   four kernels: prompt rows of bf16 models on mma.sync tiles of 64 rows; decode rows and short portions
-//                        of bf16 models on mma.sync with a kv head's query heads as operand rows, or (head sizes the tensor
-//                        cores do not take) one CTA per (row, kv head) on fp32 FMAs; fp32 and odd sizes one warp per
-//                        (token, head).  Scores, softmax state and accumulators are fp32 in all of them.  With a mask a query
+//   b2_chunk_attention   prompt rows of bf16 models: prompt_tc5.cu (tcgen05), or mma.sync tiles of 64 rows for the head sizes that
+//                        one does not take; decode rows and short portions of bf16 models on mma.sync with the keys (up to eight
+//                        query heads a kv head) or the query heads as operand rows, or (head sizes the tensor cores do not
+//                        take) one CTA per (row, kv head) on fp32 FMAs; fp32 and odd sizes one warp per (token, head). Scores, softmax state and accumulators are fp32 in all of them.  With a mask a query
 //                        touches only the keys it sees, wherever it stands; a decode row is a sequence with one query.
 // Sequences are described like everywhere in this library: rows cu_q[i] .. cu_q[i+1]-1, ctx_start[i] cached tokens
 // before them (< 0: padding, output rows are zeroed), block_tables[i, :].
@@ -132,7 +132,8 @@ __global__ void qk_rope_cache_kernel(const T* __restrict__ qkv, int64_t qkv_stri
 // visits: their cosines and sines stay in registers.  `held`: at most kRopeHeld heads a thread, whose inputs it keeps in registers
 // from the row's sums to the stores, so a row is read once.
 // Bound: memory, and the instructions around it.  With one group a thread, its partner read again beside it, the table entry by entry
-// and the row read a second time behind the norm, 4096 rows of 32 + 8 heads of 128 with NORM took 56 us; the bytes alone need 14.
+// and the row read a second time behind the norm, 4096 rows of 32 + 8 heads of 128 with NORM took 56 us, this one 40; the bytes need 14.
+// 64 registers and four CTAs an SM: with 120 registers it took 54.
 constexpr int kRopeHeld = 4;
 
 template <typename T> struct Raw4;
@@ -662,7 +663,7 @@ chunk_attention_group_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
 // Bound: the bytes of K and V.  A warp has one buffer for K and one for V and refills each as soon as it is multiplied, so one of the
 // two is always in flight under the other's arithmetic; 16 keys a tile and 128 registers let 16 warps share an SM.  With 32 keys
 // copied and then multiplied, three CTAs of four warps an SM, 64 rows x 8 kv heads x 1028 keys of 128 took 73 us: two waves, each
-// warp idle while its tile arrived.  NW is 16, 8 or 4 so that a small batch's rows are still shared by 16 warps an SM.
+// warp idle while its tile arrived (62 us with this form, 60 with the keys as rows, below).  NW is 16, 8 or 4 so that a small batch's rows are still shared by 16 warps an SM.
 constexpr int kHeadRows = 16, kHeadKeys = 16;
 
 // At most eight query heads a kv head (and one map, dk <= 128): the keys are the 16 rows of the operand and the heads its 8 columns,
@@ -1249,7 +1250,8 @@ int launch_heads(const void* q, const void* k_cache, const void* v_cache, const 
 }
 
 // ------------------------------------------------------------------------------------------------- tiled prompt kernel
-// bf16, dk and dv multiples of 16: one CTA = 64 consecutive query rows of one sequence x one head, four warps of 16 rows.
+// What the tcgen05 prompt kernel does not take: two maps of more than 64 numbers, and values of 192 or 256.
+// bf16, dk and dv multiples of 16, softmax weights: one CTA = 64 consecutive query rows of one sequence x one head, four warps of 16 rows.
 // Keys are walked 64 at a time from the first row's block start to the last row's position (at most chunk + 63 keys
 // with a mask, the whole prefix without): K and V tiles are gathered from the pages into shared memory (cp.async, two
 // threads per key row with one page lookup each, the next tile in flight while this one is multiplied), S = Q K^T and
@@ -1259,13 +1261,13 @@ int launch_heads(const void* q, const void* k_cache, const void* v_cache, const 
 // kernel above.
 constexpr int kTQ = 64, kTK = 64, kTileMinRows = 16;
 
-template <int DKT, int DVT, bool SIG, int MAPS>
+template <int DKT, int DVT, int MAPS>
 __global__ void __launch_bounds__(128)
 chunk_attention_tile_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
                             const __nv_bfloat16* __restrict__ v_cache, const int32_t* __restrict__ block_tables, int max_nb,
                             const int32_t* __restrict__ cu_q, const int32_t* __restrict__ ctx_start, int n_seq, int H, int G,
                             int bs, float scale_log2, int chunk, int window, int keep_first, float sink,
-                            float sink_logit_log2, const float* __restrict__ sink_logits, const float* __restrict__ head_bias,
+                            float sink_logit_log2, const float* __restrict__ sink_logits,
                             const __nv_bfloat16* __restrict__ gate, int64_t gate_stride, HeadShape hs, __nv_bfloat16* __restrict__ out,
                             int64_t out_stride) {
     constexpr int DK = 16 * DKT, DV = 16 * DVT, LDK = MAPS * DK + 8, LDV = DV + 8;
@@ -1320,7 +1322,6 @@ chunk_attention_tile_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
 #pragma unroll
         for (int n = 0; n < 2 * DVT; ++n) o[mp][n][0] = o[mp][n][1] = o[mp][n][2] = o[mp][n][3] = 0.f;
     }
-    const float bias_log2 = SIG && head_bias ? head_bias[hh] * 1.4426950408889634f : 0.f;
     const float cap_log2 = hs.cap * 1.4426950408889634f, cap_e = hs.cap > 0.f ? 2.f / hs.cap : 0.f;
     const uint32_t q_base = b2::smem_u32(q_sm), k_base0 = b2::smem_u32(k_sm), v_base0 = b2::smem_u32(v_sm);
 
@@ -1384,81 +1385,62 @@ chunk_attention_tile_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
                         b2::mma_bf16_16816(sc[2 * n2 + 1], a0, a1, a2, a3, b2_, b3);
                     }
                 }
-                if (SIG) {                                                          // every weight by itself: nothing to rescale
+                float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+                for (int n = 0; n < 8; ++n) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) sc[n][e] *= scale_log2;
+                }
+                if (hs.cap > 0.f) {
 #pragma unroll
                     for (int n = 0; n < 8; ++n) {
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) sc[n][e] = sigmoid2_f(fmaf(sc[n][e], scale_log2, bias_log2));
+                        for (int e = 0; e < 4; ++e) sc[n][e] = cap_score(sc[n][e], cap_log2, cap_e);
                     }
-                    if (!full) {
+                }
+                if (!full) {
 #pragma unroll
-                        for (int n = 0; n < 8; ++n) {
+                    for (int n = 0; n < 8; ++n) {
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int j = span.key(kv0 + n * 8 + 2 * tq + (e & 1));
-                                const bool ok = e < 2 ? key_visible(i0, j, lo0, window, keep_first) : key_visible(i1, j, lo1, window, keep_first);
-                                if (!ok) sc[n][e] = 0.f;
-                            }
+                        for (int e = 0; e < 4; ++e) {
+                            const int j = span.key(kv0 + n * 8 + 2 * tq + (e & 1));
+                            const bool ok = e < 2 ? key_visible(i0, j, lo0, window, keep_first) : key_visible(i1, j, lo1, window, keep_first);
+                            if (!ok) sc[n][e] = -INFINITY;
                         }
                     }
-                } else {
-                    float mx0 = -INFINITY, mx1 = -INFINITY;
+                }
 #pragma unroll
-                    for (int n = 0; n < 8; ++n) {
+                for (int n = 0; n < 8; ++n) {
+                    mx0 = fmaxf(mx0, fmaxf(sc[n][0], sc[n][1]));
+                    mx1 = fmaxf(mx1, fmaxf(sc[n][2], sc[n][3]));
+                }
+                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+                mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+                mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+                const float mn0 = fmaxf(m0[mp], mx0), mn1 = fmaxf(m1[mp], mx1);
+                const float mu0 = mn0 == -INFINITY ? 0.f : mn0, mu1 = mn1 == -INFINITY ? 0.f : mn1;
+                const float c0 = b2::fast_exp2(m0[mp] - mu0), c1 = b2::fast_exp2(m1[mp] - mu1);             // exp2(-inf) = 0: nothing accumulated yet
+                m0[mp] = mn0;
+                m1[mp] = mn1;
+                float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) sc[n][e] *= scale_log2;
-                    }
-                    if (hs.cap > 0.f) {
+                for (int n = 0; n < 8; ++n) {
+                    sc[n][0] = b2::fast_exp2(sc[n][0] - mu0);
+                    sc[n][1] = b2::fast_exp2(sc[n][1] - mu0);
+                    sc[n][2] = b2::fast_exp2(sc[n][2] - mu1);
+                    sc[n][3] = b2::fast_exp2(sc[n][3] - mu1);
+                    s0 += sc[n][0] + sc[n][1];
+                    s1 += sc[n][2] + sc[n][3];
+                }
+                l0[mp] = l0[mp] * c0 + s0;
+                l1[mp] = l1[mp] * c1 + s1;
 #pragma unroll
-                        for (int n = 0; n < 8; ++n) {
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) sc[n][e] = cap_score(sc[n][e], cap_log2, cap_e);
-                        }
-                    }
-                    if (!full) {
-#pragma unroll
-                        for (int n = 0; n < 8; ++n) {
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int j = span.key(kv0 + n * 8 + 2 * tq + (e & 1));
-                                const bool ok = e < 2 ? key_visible(i0, j, lo0, window, keep_first) : key_visible(i1, j, lo1, window, keep_first);
-                                if (!ok) sc[n][e] = -INFINITY;
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int n = 0; n < 8; ++n) {
-                        mx0 = fmaxf(mx0, fmaxf(sc[n][0], sc[n][1]));
-                        mx1 = fmaxf(mx1, fmaxf(sc[n][2], sc[n][3]));
-                    }
-                    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-                    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-                    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-                    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-                    const float mn0 = fmaxf(m0[mp], mx0), mn1 = fmaxf(m1[mp], mx1);
-                    const float mu0 = mn0 == -INFINITY ? 0.f : mn0, mu1 = mn1 == -INFINITY ? 0.f : mn1;
-                    const float c0 = b2::fast_exp2(m0[mp] - mu0), c1 = b2::fast_exp2(m1[mp] - mu1);             // exp2(-inf) = 0: nothing accumulated yet
-                    m0[mp] = mn0;
-                    m1[mp] = mn1;
-                    float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-                    for (int n = 0; n < 8; ++n) {
-                        sc[n][0] = b2::fast_exp2(sc[n][0] - mu0);
-                        sc[n][1] = b2::fast_exp2(sc[n][1] - mu0);
-                        sc[n][2] = b2::fast_exp2(sc[n][2] - mu1);
-                        sc[n][3] = b2::fast_exp2(sc[n][3] - mu1);
-                        s0 += sc[n][0] + sc[n][1];
-                        s1 += sc[n][2] + sc[n][3];
-                    }
-                    l0[mp] = l0[mp] * c0 + s0;
-                    l1[mp] = l1[mp] * c1 + s1;
-#pragma unroll
-                    for (int n = 0; n < 2 * DVT; ++n) {
-                        o[mp][n][0] *= c0;
-                        o[mp][n][1] *= c0;
-                        o[mp][n][2] *= c1;
-                        o[mp][n][3] *= c1;
-                    }
+                for (int n = 0; n < 2 * DVT; ++n) {
+                    o[mp][n][0] *= c0;
+                    o[mp][n][1] *= c0;
+                    o[mp][n][2] *= c1;
+                    o[mp][n][3] *= c1;
                 }
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
@@ -1486,8 +1468,8 @@ chunk_attention_tile_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
             l0[mp] += __shfl_xor_sync(0xffffffffu, l0[mp], x);
             l1[mp] += __shfl_xor_sync(0xffffffffu, l1[mp], x);
         }
-        inv0 = SIG ? 1.f : (l0[mp] > 0.f ? 1.f / l0[mp] : 0.f);
-        inv1 = SIG ? 1.f : (l1[mp] > 0.f ? 1.f / l1[mp] : 0.f);
+        inv0 = l0[mp] > 0.f ? 1.f / l0[mp] : 0.f;
+        inv1 = l1[mp] > 0.f ? 1.f / l1[mp] : 0.f;
         if (MAPS > 1) {
             const float f0 = mp == 0 ? inv0 : -hs.lambda * inv0, f1 = mp == 0 ? inv1 : -hs.lambda * inv1;
 #pragma unroll
@@ -1533,20 +1515,20 @@ chunk_attention_tile_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bflo
     }
 }
 
-template <int DKT, int DVT, bool SIG, int MAPS>
+template <int DKT, int DVT, int MAPS>
 int launch_tile(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables, int max_nb,
                 const int32_t* cu_q, const int32_t* ctx_start, int n_seq, int T, int H, int G, int bs, float scale, int chunk,
-                int window, int keep_first, float sink, float sink_logit, const float* sink_logits, const float* head_bias,
+                int window, int keep_first, float sink, float sink_logit, const float* sink_logits,
                 const void* gate, int64_t gate_stride, const HeadShape& hs, void* out, int64_t out_stride, cudaStream_t st) {
     constexpr int DK = 16 * DKT, DV = 16 * DVT;
     const size_t smem = (size_t)(kTQ * (MAPS * DK + 8) + 2 * kTK * (MAPS * DK + 8) + 2 * kTK * (DV + 8)) * sizeof(__nv_bfloat16);
-    auto kern = chunk_attention_tile_kernel<DKT, DVT, SIG, MAPS>;
+    auto kern = chunk_attention_tile_kernel<DKT, DVT, MAPS>;
     if (smem > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int tiles = (T + kTQ - 1) / kTQ + n_seq;          // upper bound on sum(ceil(len / 64)); spare CTAs leave at once
     kern<<<dim3(tiles, H), 128, smem, st>>>(static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k_cache),
                                            static_cast<const __nv_bfloat16*>(v_cache), block_tables, max_nb, cu_q, ctx_start,
                                            n_seq, H, G, bs, scale * 1.4426950408889634f, chunk, window, keep_first, sink,
-                                           sink_logit * 1.4426950408889634f, sink_logits, head_bias,
+                                           sink_logit * 1.4426950408889634f, sink_logits,
                                            static_cast<const __nv_bfloat16*>(gate), gate_stride, hs, static_cast<__nv_bfloat16*>(out),
                                            out_stride);
     B2_CUDA_OK(cudaGetLastError());
@@ -1695,8 +1677,8 @@ extern "C" int b2_masked_attention(void* out, const void* q, const void* k_cache
         } else {
 #define B2_TILE(a, b, MAPS)                                                                                               \
     if (dk == 16 * a && dv == 16 * b)                                                                                     \
-        rc = launch_tile<a, b, false, MAPS>(q, k_cache, v_cache, block_tables, max_nb, cu_q, ctx_start, n_seq, T, H, G, bs, scale, \
-                                            chunk, window, keep_first, sink, sink_logit, sink_logits, head_bias, gate, gate_stride, \
+        rc = launch_tile<a, b, MAPS>(q, k_cache, v_cache, block_tables, max_nb, cu_q, ctx_start, n_seq, T, H, G, bs, scale, \
+                                            chunk, window, keep_first, sink, sink_logit, sink_logits, gate, gate_stride, \
                                             hs, out, out_stride, st);
             if (maps == 2) {
                 B2_TILE(6, 2, 2) B2_TILE(6, 4, 2) B2_TILE(6, 6, 2) B2_TILE(6, 8, 2)

@@ -137,6 +137,8 @@ __global__ void recur_prep_kernel(const T* __restrict__ proj, int64_t proj_strid
 // q | k | v columns are those of a decay per key channel; small per-head outputs are left to the first column block.  Four channels
 // and not eight: 64 registers let four CTAs share an SM, and a warp's stores are 512 consecutive bytes.
 // Bound: memory (2 or 4 bytes in and 4 out per channel), with the exact exponentials and divisions of the activation close behind.
+// One CTA a row with scalar accesses and a staging pass took 88 us at 4096 rows of 6144 channels (rotation, no convolution), 174 at 3001
+// rows (four taps, SiLU, unit vectors) and 59 at 64 rows; this one 58, 63 and 27.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(256, 4)
 recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec sp, const float* __restrict__ conv_w,
@@ -628,7 +630,7 @@ __device__ __forceinline__ void ld_vec8(const T* p, float (&v)[8]) {
 }
 
 // The same with a head in 1, 2, .. 32 lanes of eight entries (dv = 8 .. 256, a power of two): 16-byte accesses, the row read once.
-// Scalar accesses and a warp per head took 27 us at 4096 rows of 16 heads of 128, this 13 (0.78 of the copy rate).
+// Scalar accesses and a warp per head took 27 us at 4096 rows of 16 heads of 128, this 14 (0.72 of the copy rate).
 template <typename T>
 __global__ void __launch_bounds__(256)
 gated_head_norm_vec_kernel(const float* __restrict__ o, const T* __restrict__ gate, int64_t gate_stride, int gate_kind, int H, int dv,
@@ -757,7 +759,8 @@ int launch_prep(const void* proj, int64_t proj_stride, const PrepSpec& sp, int T
                      (sp.taps == 1 || (b2_aligned16(conv_state) && b2_aligned16(conv_w))) && (!sp.rot_dims || b2_aligned16(sp.cos_sin)) &&
                      (!channel_decay || (b2_aligned16(sp.a) && sp.a_stride % 4 == 0 && b2_aligned16(decay)));
     if (vec) {
-        // rows a CTA: long runs read the convolution's inputs once; small batches spread over the SMs instead
+        // rows a CTA: long runs read the convolution's inputs once; small batches spread over the SMs instead.  Runs of 1 / 4 / 16 rows:
+        // 349 / 140 / 85 us at 3001 rows of four taps, 128 / 57 / 46 at 1000, 38 / 42 / 72 at 64 (before the channels went from eight to four)
         const int run = T >= 2048 ? 8 : T >= 512 ? 4 : 1;
         const dim3 grid((T + run - 1) / run, ((C + (channel_decay ? sp.H * sp.dk : 0)) / 4 + 255) / 256);
 #define B2_PREP_VEC(TAPS)                                                                                                    \

@@ -23,7 +23,7 @@
 // Sequences are described like everywhere in this library: rows cu_q[i] .. cu_q[i+1]-1, ctx_start[i] cached tokens before
 // them (< 0: padding, output rows are zeroed), block_tables[i, :].
 // Every sequence of a batch has at least one row; a batch with as many rows as sequences is therefore one row each (a
-// decode step) and may take the decode kernel.  b2_latent_attention_workspace tells how much fp32 scratch a call can use
+// decode step) and may take the decode kernel of latent_tc5.cu.  b2_latent_attention_workspace tells how much fp32 scratch a call can use
 // to split the keys of a row over CTAs; without it the call runs unsplit.
 #include "b2_act.cuh"
 

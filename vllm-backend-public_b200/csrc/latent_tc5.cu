@@ -11,7 +11,9 @@
 // bf16 and fp32 keep their relative precision for every weight from 2^-100 to 2^60.  If a later score exceeds m by more than 60 (in
 // powers of two), the share is computed again with the maxima found.
 // Bound: the bytes of the cached rows (74 KB a tile and SM).  The form on mma.sync with Q in registers waited for its own chain of
-// ldmatrix, MMA and barriers, two warps a scheduler: 64 sequences x 32 heads x 2560 keys of 576 took 120 us (140 with Q in shared memory).
+// ldmatrix, MMA and barriers, two warps a scheduler: 64 sequences x 32 heads x 2560 keys of 576 took 120 us (140 with Q in shared memory); this one 60 (3.2 TB/s, two shares a row on 128
+// SMs: a tile's load, scores, softmax and output follow one another in each half of the ring).  An output goes before the next scores
+// whenever those still wait for their tile: always behind them, it took 88.
 #include "b2_act.cuh"
 #include "b2_tc5.cuh"
 

@@ -1452,6 +1452,8 @@ struct Plan {
     int nc;            // dynamic: CTAs of the persistent grid the plan was made for
 };
 
+constexpr int SHORT_ROW_TOKENS = 640;                // rows that a CTA streams faster than further launches start
+
 // dynamic schedule: workspace header (claim counter)
 constexpr size_t WS_HEADER_BYTES = 256;
 
@@ -1560,8 +1562,8 @@ int launch_decode(const CUtensorMap& tmK, const CUtensorMap& tmV, const DecodePa
         cfg.numAttrs = zero_first ? 1 : 0;
         B2_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tmK, tmV, p));
         cudaLaunchConfig_t cfg2 = {};
-        // few items have many runs each (chunks shrink to 64 tokens): a block per item walked them four at a time, 32 us of the 45
-        // that 4 sequences of 8192 tokens on 2 kv heads took; a block per head shares them out.  Many items have few runs.
+        // few items have many runs each (chunks shrink to 64 tokens), and a block per item walks them four at a time: of the 45 us
+        // that 4 sequences of 8192 tokens on 2 kv heads took more than half.  A block per head shares them out.  Many items have few runs.
         const bool per_head = p.Hkv * p.HG * p.B < sm_count();
         cfg2.gridDim = dim3(p.Hkv * p.HG, p.B, per_head ? std::min(8 * NT, p.G) : 1);
         cfg2.blockDim = dim3(128);
@@ -1679,6 +1681,13 @@ int run_decode(const DecodeGeom& g, const CacheMaps& maps, const Knobs& kn, bool
     const bool fp8 = g.kv_dtype == B2_KV_FP8_E4M3;
     Plan pl;
     make_plan(&pl, B, g.Hkv, G, g.bs, g.max_nb, num_splits, ctas_per_sm(fp8, G, kn.fp8_ctas), kn);
+    const Plan asked = pl;                               // what the workspace is checked against
+    // Block tables too narrow for long rows, and all items in one wave: the single-pass grid whatever was asked.  It is one launch (KV
+    // write included) and streams a CTA's tokens at about 10.7 ns each behind 3.3 us; the dynamic schedule starts at 9.6 us whatever the
+    // batch (write, counter, decode, merge).  Measured with 1 - 32 rows in a graph, single / dynamic, bf16: 4.7 / 10.5 us at 128 tokens,
+    // 8.4 / 11.6 at 512, 13.8 / 13.7 at 1024; fp8: 4.9 / 10.2, 7.8 / 11.7, 12.5 / 13.5.  Launched one by one 20 / 29 at 512.
+    if (pl.num_splits == 0 && (int64_t)g.max_nb * g.bs <= SHORT_ROW_TOKENS && (int64_t)B * pl.ipb <= 2 * (int64_t)sm_count())
+        make_plan(&pl, B, g.Hkv, G, g.bs, g.max_nb, 1, ctas_per_sm(fp8, G, kn.fp8_ctas), kn);
 
     DecodeParams p;
     p.out = static_cast<__nv_bfloat16*>(out);
@@ -1719,15 +1728,15 @@ int run_decode(const DecodeGeom& g, const CacheMaps& maps, const Knobs& kn, bool
     p.two_box = maps.two_box;
     // a plan handle keeps its zeroed claim counter in the workspace header: the partials of every schedule start
     // behind it (the stateless call re-zeroes the counter itself and uses the header only for the dynamic schedule)
-    const bool header = pl.num_splits == 0 || !zero_first;
-    const size_t body = plan_workspace(pl, B, g.Hq) - (pl.num_splits == 0 ? WS_HEADER_BYTES : 0);
+    const bool header = asked.num_splits == 0 || !zero_first;
+    const size_t body = plan_workspace(asked, B, g.Hq) - (asked.num_splits == 0 ? WS_HEADER_BYTES : 0);
     if (body) {
         const size_t need = body + (header ? WS_HEADER_BYTES : 0);
         B2_REQUIRE(g.workspace && g.workspace_bytes >= need && b2_aligned16(g.workspace), B2_ENOMEM,
                    "paged_decode: workspace %zu bytes < required %zu", g.workspace_bytes, need);
         char* base = static_cast<char*>(g.workspace);
-        if (pl.num_splits == 0) {
-            B2_REQUIRE(pl.slots < (1LL << 27), B2_EUNSUPPORTED, "paged_decode: %lld partial slots", (long long)pl.slots);
+        if (asked.num_splits == 0) {
+            B2_REQUIRE(asked.slots < (1LL << 27), B2_EUNSUPPORTED, "paged_decode: %lld partial slots", (long long)asked.slots);
             p.counter = reinterpret_cast<uint32_t*>(base);
         }
         if (header) base += WS_HEADER_BYTES;
@@ -1810,12 +1819,6 @@ extern "C" int b2_paged_decode_plan_splits(const int32_t* seq_lens_host, int B, 
             streamed += L * ipb;
         }
     }
-    // Short sequences in one wave: the single-pass grid is one launch (KV write included) and streams a CTA's tokens at about 10.7 ns
-    // each behind 3.3 us; the dynamic schedule starts at 9.6 us whatever the batch (write, counter, decode, merge).  Measured bf16, 1 - 32
-    // sequences, single / dynamic, in a graph: 4.7 / 10.5 us at 128 tokens, 8.4 / 11.6 at 512, 13.8 / 13.7 at 1024; fp8 4.9 / 10.2,
-    // 7.8 / 11.7, 12.5 / 13.5.  Launched one by one the three extra launches cost another 5 us.
-    constexpr int64_t SHORT_TOK = 640;
-    if (makespan <= SHORT_TOK + OVERHEAD_TOK) return 1;
     const double ideal = (double)total / NC;
     // fp8 (three CTAs per SM) is paced by its consumer warps, not by HBM: an idle slot is lost throughput, so the
     // single-pass grid only wins when its waves are nearly full (measured: config 3 dynamic 6.4 vs grid 6.1 TB/s)
