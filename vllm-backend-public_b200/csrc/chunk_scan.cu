@@ -459,7 +459,19 @@ __global__ void __launch_bounds__(NT)
 chunk_delta_kernel(const ChunkArgs a, int stages) {
     extern __shared__ __align__(16) float sm[];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int seq = blockIdx.x, hh = blockIdx.y, j0 = blockIdx.z * NC;
+    // CTAs start in the order of their sequences' lengths, the longest first: 3 sequences of 16 heads are 384 chains on 296 places
+    __shared__ int s_seq;
+    for (int i = tid; i < a.n_seq; i += NT) {
+        const int len = a.cu_q[i + 1] - a.cu_q[i];
+        int rank = 0;
+        for (int j = 0; j < a.n_seq; ++j) {
+            const int other = a.cu_q[j + 1] - a.cu_q[j];
+            rank += other > len || (other == len && j < i);
+        }
+        if (rank == blockIdx.z) s_seq = i;
+    }
+    __syncthreads();
+    const int seq = s_seq, hh = blockIdx.y, j0 = blockIdx.x * NC;
     const int ctx = a.ctx_start[seq];
     if (ctx < 0) return;
     const int dk = a.dk, dv = a.dv, H = a.H, LD = dk + 4, per = dk / 4;
@@ -762,7 +774,7 @@ int launch(const ChunkArgs& a, int total_rows, cudaStream_t st) {
     if (rc != B2_OK) return rc;
     chunk_prep_kernel<CH, DELTA><<<dim3(chunks, a.H), NT, psm, st>>>(a);
     if constexpr (DELTA) {
-        const dim3 grid(a.n_seq, a.H, (a.dv + NC - 1) / NC);
+        const dim3 grid((a.dv + NC - 1) / NC, a.H, a.n_seq);
         const size_t stage = sizeof(float) * (size_t)delta_stage(a.dk, CH), fixed = sizeof(float) * (size_t)delta_fixed(a.dk);
         // two CTAs an SM cover each other's copies when there are enough of them; a lone one prefetches
         const int stages = (long)grid.x * grid.y * grid.z > n_sm || fixed + 2 * stage > 227 * 1024 ? 1 : 2;
@@ -790,9 +802,9 @@ int64_t b2_internal_chunk_scan_floats(int total_rows, int n_seq, int H, int dk, 
 }
 
 // Where the chunked form is the faster one.  Both times are estimated in us from what they measured for heads of 128 x 128 on
-// one B200 (w = dk dv / 16384 scales the products); the host knows the rows and the number of sequences, so lengths are taken equal:
-//   tokens   a chain of 0.20 (delta 0.285, per channel 0.235 / 0.31) a token, or, with many sequences, 5.0 (6.3 / 6.8 / 8.3) ns a
-//            token and head
+// one B200 (w = dk dv / 16384 scales the products); the host knows the rows and the number of sequences, so the longest of several is taken to be 1.25 times the mean:
+//   tokens   a chain of 0.20 (delta 0.285, per channel 0.235 / 0.31) a token, or, with several sequences, 5.2 (7.1 / 10.6 / 12.4) ns a
+//            token and head, down to 5.0 (6.3 / 6.8 / 8.3) from 64 sequences on
 //   chunks   0.23 (0.16 / 0.55 / 0.70) a chunk and head for the products, 0.11 a sequence and head for its state, with delta 4.8 a
 //            step of the chain and SM's share of CTAs; at least 40 (80 per channel, 110 with delta too): three launches
 // Measured, tokens -> chunks: 1 x 4096 tokens, 16 heads: 804 -> 250, 1160 -> 470, 963 -> 572, 1254 -> 1006; 1 x 500: 101 -> 43,
@@ -801,12 +813,14 @@ bool b2_internal_chunk_scan_pays(int total_rows, int n_seq, int H, int dk, int d
     if (total_rows < 2 * n_seq) return false;
     const float len = (float)total_rows / n_seq, w = dk * dv / 16384.f, steps = ceilf(len / C), heads = (float)n_seq * H;
     const int kind = (ch ? 2 : 0) + (delta ? 1 : 0);
-    const float chain_tok[4] = {0.20f, 0.285f, 0.235f, 0.31f}, rate_tok[4] = {5.0e-3f, 6.3e-3f, 6.8e-3f, 8.3e-3f};
+    const float chain_tok[4] = {0.20f, 0.285f, 0.235f, 0.31f}, rate_few[4] = {5.2e-3f, 7.1e-3f, 10.6e-3f, 12.4e-3f}, rate_many[4] = {5.0e-3f, 6.3e-3f, 6.8e-3f, 8.3e-3f};
     const float per_chunk[4] = {0.23f, 0.16f, 0.55f, 0.70f}, least[4] = {40.f, 40.f, 80.f, 110.f};
-    const float tokens = fmaxf(chain_tok[kind] * (dk <= 64 ? 0.75f : 1.f) * len, rate_tok[kind] * (float)total_rows * H * w);
+    const float many = fminf(1.f, fmaxf(0.f, log2f(n_seq / 4.f) / 4.f)), rate = rate_few[kind] + (rate_many[kind] - rate_few[kind]) * many;
+    const float longest = len * (n_seq > 1 ? 1.25f : 1.f);
+    const float tokens = fmaxf(chain_tok[kind] * (dk <= 64 ? 0.75f : 1.f) * longest, rate * (float)total_rows * H * w);
     float chunks = (per_chunk[kind] * (0.35f + 0.65f * w) * steps + 0.11f * w) * heads;
-    if (delta) chunks += steps * (3.4f + 1.4f * w) * fmaxf(1.f, heads * ((dv + NC - 1) / NC) / 148.f);
-    return tokens >= 1.1f * fmaxf(chunks, least[kind]);
+    if (delta) chunks += (3.4f + 1.4f * w) * fmaxf(ceilf(longest / C), steps * heads * ((dv + NC - 1) / NC) / 148.f);
+    return tokens >= fmaxf(chunks, least[kind]);
 }
 
 int b2_internal_chunk_scan(const float* qkv, const float* beta, const float* decay, int total_rows, int H, int G, int dk, int dv,
