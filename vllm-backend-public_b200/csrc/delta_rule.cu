@@ -917,7 +917,8 @@ extern "C" int b2_gated_head_norm(const float* o, const void* gate, int64_t gate
         return B2_OK;
     }
     const size_t esz = act_dtype == B2_ACT_BF16 ? 2 : 4;
-    if (dv % 8 == 0 && dv <= 256 && (dv & (dv - 1)) == 0 && b2_aligned16(o) && b2_aligned16(gate) && b2_aligned16(out) && b2_aligned16(norm_w) &&
+    // from a prompt's size on: below it a launch is all that either takes, and the warp per head keeps its order of summation
+    if (T >= 256 && dv % 8 == 0 && dv <= 256 && (dv & (dv - 1)) == 0 && b2_aligned16(o) && b2_aligned16(gate) && b2_aligned16(out) && b2_aligned16(norm_w) &&
         gate_stride * esz % 16 == 0 && out_stride * esz % 16 == 0) {
         const int64_t total = (int64_t)T * H * dv;
         B2_DISPATCH_ACT(act_dtype, A, (gated_head_norm_vec_kernel<A><<<(unsigned)((total / 8 + 255) / 256), 256, 0, st>>>(
