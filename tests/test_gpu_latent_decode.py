@@ -71,3 +71,20 @@ def test_latent_decode(cuda, ctx, H, R, dr, bs, window, sink, gate, rise):
         bound = (2.0 ** -8 + (2.0 ** -10 if rise else 0.0)) * (spr + ref.abs()) + 1e-6
         err = (out[i] - ref).abs()
         assert bool((err <= bound).all()), (i, c, float((err / bound).max()))
+
+
+def test_long_rows_repeat_to_the_bit(cuda):
+    """Some forty tiles a share, many times: the issuing warp's choice between the next scores and this output is timing, and neither
+    order changes what is summed, so every call returns the same bits."""
+    g = torch.Generator(device=cuda).manual_seed(7)
+    n, H, R, dr, bs, c = 64, 32, 512, 64, 16, 2559
+    nb = c // bs + 1
+    cache = torch.randn(n * nb, bs, R + dr, generator=g, device=cuda).bfloat16()
+    tables = torch.randperm(n * nb, generator=g, device=cuda).to(torch.int32).view(n, nb)
+    qa = torch.randn(n, H, R + dr, generator=g, device=cuda).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    batch = ops.SeqBatch(i32(list(range(n + 1))), i32([c] * n), tables, None, n, n)
+    first = ops.latent_attention(qa, cache, batch, R, (R + dr) ** -0.5, 0)
+    assert bool(torch.isfinite(first).all())
+    for _ in range(40):
+        assert torch.equal(first, ops.latent_attention(qa, cache, batch, R, (R + dr) ** -0.5, 0))

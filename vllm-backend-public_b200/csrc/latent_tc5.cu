@@ -201,13 +201,15 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
 #pragma unroll 1
             for (int t = 0; t < nt; ++t) {
                 const int it = it0 + t, s = it & 1;
-                bool ahead = t + 1 < nt;             // the next scores go first if their tile is there, else behind this output
-                for (uint32_t spins = 0; !b2::mbar_try_wait(bar(PR + s), (it >> 1) & 1);) {
-                    if (ahead && b2::mbar_try_wait(bar(FULL + (s ^ 1)), ((it + 1) >> 1) & 1)) {
+                // The next scores go first if their tile is there, else behind this output.  Lanes may see a phase end at different
+                // probes, and both branches hold instructions of the whole warp: every answer is the warp's vote, not the lane's.
+                bool ahead = t + 1 < nt;
+                for (uint32_t spins = 0; !__all_sync(0xffffffffu, b2::mbar_try_wait(bar(PR + s), (it >> 1) & 1));) {
+                    if (ahead && __all_sync(0xffffffffu, b2::mbar_try_wait(bar(FULL + (s ^ 1)), ((it + 1) >> 1) & 1))) {
                         scores(t + 1);
                         ahead = false;
                     }
-                    if (*failed || ++spins > (1u << 22)) { *failed = 1; break; }
+                    if (__any_sync(0xffffffffu, *failed || ++spins > (1u << 22))) { *failed = 1; break; }
                 }
                 tc_fence_after();
                 if (elect_one()) {
