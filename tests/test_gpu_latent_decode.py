@@ -88,3 +88,21 @@ def test_long_rows_repeat_to_the_bit(cuda):
     assert bool(torch.isfinite(first).all())
     for _ in range(40):
         assert torch.equal(first, ops.latent_attention(qa, cache, batch, R, (R + dr) ** -0.5, 0))
+
+
+def test_as_many_rows_as_sequences_but_not_one_each(cuda):
+    """Rows [2, 0, 1, 3, 0, 0]: every row is its own sequence's, at its own position; the same rows asked one by one give the same bits."""
+    g = torch.Generator(device=cuda).manual_seed(9)
+    lens, ctx, H, R, dr, bs = [2, 0, 1, 3, 0, 0], [40, 5, 0, 130, 7, 9], 20, 256, 64, 16
+    n, nb = len(lens), 10
+    cache = torch.randn(n * nb, bs, R + dr, generator=g, device=cuda).bfloat16()
+    tables = torch.randperm(n * nb, generator=g, device=cuda).to(torch.int32).view(n, nb)
+    qa = torch.randn(n, H, R + dr, generator=g, device=cuda).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    cu = [sum(lens[:i]) for i in range(n + 1)]
+    owner = [i for i, k in enumerate(lens) for _ in range(k)]
+    pos = [ctx[i] + r for i, k in enumerate(lens) for r in range(k)]
+    scale = (R + dr) ** -0.5
+    out = ops.latent_attention(qa, cache, ops.SeqBatch(i32(cu), i32(ctx), tables, None, n, n), R, scale, 0)
+    single = ops.SeqBatch(i32(list(range(n + 1))), i32(pos), tables[owner].contiguous(), None, n, n)
+    assert torch.equal(out, ops.latent_attention(qa, cache, single, R, scale, 0))

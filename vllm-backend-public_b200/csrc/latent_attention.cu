@@ -22,8 +22,8 @@
 //                         Softmax state, scores and the accumulator are fp32.
 // Sequences are described like everywhere in this library: rows cu_q[i] .. cu_q[i+1]-1, ctx_start[i] cached tokens before
 // them (< 0: padding, output rows are zeroed), block_tables[i, :].
-// Every sequence of a batch has at least one row; a batch with as many rows as sequences is therefore one row each (a
-// decode step) and may take the decode kernel of latent_tc5.cu.  b2_latent_attention_workspace tells how much fp32 scratch a call can use
+// A batch with as many rows as sequences (a decode step: one row each) may take the decode kernel of latent_tc5.cu, which looks up
+// the sequence of every row and so takes any division of them.  b2_latent_attention_workspace tells how much fp32 scratch a call can use
 // to split the keys of a row over CTAs; without it the call runs unsplit.
 #include "b2_act.cuh"
 
@@ -745,7 +745,7 @@ inline int latent_sm_count() {
 }
 
 // Which kernel and how many shares of the key tiles per CTA row: a batch that cannot fill the GPU (decode rows) splits its
-// keys over CTAs.  decode: every sequence has one row and latent_tc5.cu takes the sizes.
+// keys over CTAs.  decode: as many rows as sequences and latent_tc5.cu takes the sizes.
 struct LatentPlan {
     bool decode;
     int nsplit;
@@ -783,7 +783,7 @@ int launch_latent_mma(void* out, const void* qa, const void* cache, const int32_
     float* ws_ml = ws ? ws + (size_t)T * H * nsplit * 16 * RT : nullptr;
     if constexpr (RT >= 8) {
         if (decode) {
-            const int rc = b2_internal_latent_tc5(out, qa, cache, block_tables, max_nb, cu_q, ctx_start, T, H, 16 * RT, dr, bs, scale, window,
+            const int rc = b2_internal_latent_tc5(out, qa, cache, block_tables, max_nb, cu_q, ctx_start, n_seq, T, H, 16 * RT, dr, bs, scale, window,
                                                   sink_logits, gate, gate_stride, nsplit, ws_o, ws_ml, st);
             if (rc != B2_OK) return rc;
             if (nsplit > 1)

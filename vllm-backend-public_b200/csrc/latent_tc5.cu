@@ -1,4 +1,4 @@
-// latent_tc5.cu -- decode rows of b2_latent_attention in bf16 on the 5th-gen tensor cores (every sequence has one row, R a multiple
+// latent_tc5.cu -- decode rows of b2_latent_attention in bf16 on the 5th-gen tensor cores (as many rows as sequences, R a multiple
 // of 128): out[t, h] = sum_j softmax_j(qa[t, h] . c_j) c_j[0..R) over the cached rows c_j of R + dr numbers.
 //
 // A CTA takes one token, up to 32 heads and one share of its keys, 64 keys at a time.  The keys are the M side of the scores and the
@@ -29,7 +29,7 @@ struct LatentArgs {
     CUtensorMap map;                                 // the pool as rows of Dc numbers, boxes of 16 rows x 64 columns
     const bf16 *qa, *cache;
     const int32_t *block_tables, *cu_q, *ctx_start;
-    int max_nb, H, dr, bs, window, tma;
+    int n_seq, max_nb, H, dr, bs, window, tma;
     float scale_log2;
     const float* sink_logits;
     const bf16* gate;
@@ -62,9 +62,10 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
     __shared__ __align__(16) float s_ref[HEADS];
     __shared__ float s_f[HEADS];
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int seq = blockIdx.x, tok = p.cu_q[seq], h0 = blockIdx.y * HEADS, nh = min(HEADS, p.H - h0);
+    // a CTA belongs to a row: as many rows as sequences is one row each as a rule, but [2, 0] is as many too
+    const int tok = blockIdx.x, seq = b2::seq_of_row(p.cu_q, p.n_seq, tok), h0 = blockIdx.y * HEADS, nh = min(HEADS, p.H - h0);
     const int nsplit = gridDim.z, zs = blockIdx.z, ctx = p.ctx_start[seq], bs = p.bs;
-    const int pos = ctx, klo = p.window > 0 ? max(pos - p.window + 1, 0) : 0, kbase = klo & ~15;
+    const int pos = ctx + tok - p.cu_q[seq], klo = p.window > 0 ? max(pos - p.window + 1, 0) : 0, kbase = klo & ~15;
     const int all_tiles = ctx < 0 ? 0 : (pos - kbase) / KT + 1, per = (all_tiles + nsplit - 1) / nsplit;
     const int t0 = zs * per, nt = min(all_tiles, t0 + per) - t0;
     if (nt <= 0) {                                   // padding, or a share without keys
@@ -358,20 +359,20 @@ size_t smem_bytes(int Dc) { return (size_t)((Dc + 63) / 64) * (SUB + Q_SUB) + SU
 
 }  // namespace
 
-// one row a sequence; R = 128, 256 or 512, dr a multiple of 16; pointers and rows of 16 bytes
+// R = 128, 256 or 512, dr a multiple of 16; pointers and rows of 16 bytes
 bool b2_internal_latent_tc5_ok(int R, int dr) {
     return (R == 128 || R == 256 || R == 512) && dr % 16 == 0 && smem_bytes(R + dr) <= 226 * 1024;
 }
 int b2_internal_latent_tc5_heads(void) { return HEADS; }
 
 int b2_internal_latent_tc5(void* out, const void* qa, const void* cache, const int32_t* block_tables, int max_nb, const int32_t* cu_q,
-                           const int32_t* ctx_start, int T, int H, int R, int dr, int bs, float scale, int window, const float* sink_logits,
+                           const int32_t* ctx_start, int n_seq, int T, int H, int R, int dr, int bs, float scale, int window, const float* sink_logits,
                            const void* gate, int64_t gate_stride, int nsplit, float* ws_o, float* ws_ml, void* stream) {
     LatentArgs p{};
     const int Dc = R + dr;
     p.qa = static_cast<const bf16*>(qa);
     p.cache = static_cast<const bf16*>(cache);
-    p.block_tables = block_tables; p.cu_q = cu_q; p.ctx_start = ctx_start; p.max_nb = max_nb;
+    p.block_tables = block_tables; p.cu_q = cu_q; p.ctx_start = ctx_start; p.n_seq = n_seq; p.max_nb = max_nb;
     p.H = H; p.dr = dr; p.bs = bs; p.window = window; p.scale_log2 = scale * kLog2e;
     p.sink_logits = sink_logits;
     p.gate = static_cast<const bf16*>(gate);
