@@ -106,3 +106,20 @@ def test_as_many_rows_as_sequences_but_not_one_each(cuda):
     out = ops.latent_attention(qa, cache, ops.SeqBatch(i32(cu), i32(ctx), tables, None, n, n), R, scale, 0)
     single = ops.SeqBatch(i32(list(range(n + 1))), i32(pos), tables[owner].contiguous(), None, n, n)
     assert torch.equal(out, ops.latent_attention(qa, cache, single, R, scale, 0))
+
+
+@pytest.mark.parametrize("n", [3, 160])                                  # keys split over CTAs, and not
+@pytest.mark.parametrize("where", [0, 1, 700])
+def test_a_nan_in_a_cached_row_stays_one(cuda, n, where):
+    """A NaN in the rotated part of a cached row reaches every output of its sequence and no other's, however the keys are shared."""
+    g = torch.Generator(device=cuda).manual_seed(11)
+    H, R, dr, bs, c = 8, 512, 64, 16, 900
+    nb = c // bs + 1
+    cache = torch.randn(n * nb, bs, R + dr, generator=g, device=cuda).bfloat16()
+    tables = torch.arange(n * nb, dtype=torch.int32, device=cuda).view(n, nb)
+    cache[nb + where // bs, where % bs, R + 5] = float("nan")
+    qa = torch.randn(n, H, R + dr, generator=g, device=cuda).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    out = ops.latent_attention(qa, cache, ops.SeqBatch(i32(list(range(n + 1))), i32([c] * n), tables, None, n, n), R, 0.04, 0)
+    nan = torch.isnan(out).flatten(1)
+    assert bool(nan[1].all()) and not bool(nan[0].any()) and not bool(nan[2:].any())

@@ -713,9 +713,9 @@ __global__ void latent_merge_kernel(const float* __restrict__ ws_o, const float*
         const float M = b2::warp_max(ml.x);
         const float e = ml.x == -INFINITY ? 0.f : exp2f(ml.x - M);
         const float L = b2::warp_sum(ml.y * e);
-        float f = L > 0.f ? 1.f / L : 0.f;
+        float f = L > 0.f ? 1.f / L : L == 0.f ? 0.f : L;                   // NaN stays NaN, as in a row of one share
         if (gate) f *= b2::sigmoid_f(__bfloat162float(gate[(size_t)(row / H) * gate_stride + row % H]));
-        if (z < nsplit) s_w[z] = e * f;
+        if (z < nsplit) s_w[z] = ml.x == -INFINITY ? 0.f : e * f;
     }
     __syncthreads();
     const float* o = ws_o + (size_t)row * nsplit * R;
