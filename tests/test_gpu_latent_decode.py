@@ -123,3 +123,27 @@ def test_a_nan_in_a_cached_row_stays_one(cuda, n, where):
     out = ops.latent_attention(qa, cache, ops.SeqBatch(i32(list(range(n + 1))), i32([c] * n), tables, None, n, n), R, 0.04, 0)
     nan = torch.isnan(out).flatten(1)
     assert bool(nan[1].all()) and not bool(nan[0].any()) and not bool(nan[2:].any())
+
+
+@pytest.mark.parametrize("n", [2, 150])                                  # keys split over CTAs, and not
+def test_a_sink_far_above_the_first_share(cuda, n):
+    """Scores that climb by 400 (in powers of two) over the row and a sink between: above the first share's scores by more than fp32
+    holds, far below the last's, so that it weighs nothing; and a sink above all of them, which leaves nothing to the keys."""
+    g = torch.Generator(device=cuda).manual_seed(13)
+    H, R, dr, bs, c = 4, 256, 64, 16, 1535
+    nb = c // bs + 1
+    scale = 1.0 / 16
+    cache = torch.randn(n * nb, bs, R + dr, generator=g, device=cuda).bfloat16()
+    tables = torch.arange(n * nb, dtype=torch.int32, device=cuda).view(n, nb)
+    qa = torch.randn(n, H, R + dr, generator=g, device=cuda).bfloat16()
+    qa[:, :, R] = 8.0
+    row = torch.arange(nb * bs, device=cuda).float()
+    cache[..., R] = ((row / c - 0.5) * 400.0 / 8.0 / scale * math.log(2.0)).bfloat16().view(nb, bs).repeat(n, 1)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    batch = ops.SeqBatch(i32(list(range(n + 1))), i32([c] * n), tables, None, n, n)
+    plain = ops.latent_attention(qa, cache, batch, R, scale, 0)
+    between = ops.latent_attention(qa, cache, batch, R, scale, 0, sink_logits=torch.full((H,), 0.0, device=cuda))
+    above = ops.latent_attention(qa, cache, batch, R, scale, 0, sink_logits=torch.full((H,), 300.0, device=cuda))
+    assert bool(torch.isfinite(plain).all())
+    assert bool(((between.float() - plain.float()).abs() <= 2.0 ** -6 * plain.float().abs() + 1e-3).all())
+    assert bool((above.float().abs() <= 1e-6).all())

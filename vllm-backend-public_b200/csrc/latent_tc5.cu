@@ -7,7 +7,7 @@
 // scores are computed on all 128 rows and read from its own 64 lanes.  Warps 0, 1 and 2, 3 do the softmax of the halves in turn (a lane
 // a key), warp 4 issues the MMAs, warps 5 - 8 fetch: whole tiles by TMA boxes of 16 rows, tiles with an end (or pages whose size is no
 // multiple of 16) by cp.async with zeros outside.
-// The softmax needs no running maximum: weights are taken against a reference m per head, the maximum of the share's first tile, and
+// The softmax needs no running maximum: weights are taken against a reference m per head, the maximum of the share's first tile (and the sink), and
 // bf16 and fp32 keep their relative precision for every weight from 2^-100 to 2^60.  If a later score exceeds m by more than 60 (in
 // powers of two), the share is computed again with the maxima found.
 // Bound: the bytes of the cached rows (74 KB a tile and SM).  The form on mma.sync with Q in registers waited for its own chain of
@@ -98,7 +98,8 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
         b2::mbar_init(bar(END), 1);
         b2::fence_mbar_init();
     }
-    if (tid < HEADS) s_max[tid] = ordered(__float_as_int(-INFINITY));
+    // the sink counts among the scores the reference is taken from: a sum is at least one and finite, which the merge relies on
+    if (tid < HEADS) s_max[tid] = ordered(__float_as_int(p.sink_logits && zs == 0 ? p.sink_logits[h0 + min(tid, nh - 1)] * kLog2e : -INFINITY));
     if (warp == 4) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(b2::smem_u32(&s_tmem)), "n"(COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
