@@ -98,3 +98,39 @@ def test_chunked_scan_leaves_short_portions_to_the_token_scan():
     assert lib.b2_channel_scan_workspace(4096, 1, 16, 256, 128, 0, 1) == 0
     assert lib.b2_channel_scan_workspace(4096, 1, 16, 126, 128, 0, 1) == 0
     assert lib.b2_channel_scan_workspace(0, 1, 16, 128, 128, 0, 1) == 0
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("delta,per_channel", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("at", [1, 5, 31, 34, 63, 64, 100])
+def test_nothing_runs_backwards(cuda, at, delta, per_channel, bad):
+    """An infinity or NaN in one token's query, key, value, decay or beta: the tokens before it are bit-equal to the same call without it,
+    and so are all tokens but its own where only its query is bad, and the other heads'."""
+    H, G, dk, dv, T = 2, 2, 64, 32, 130
+    qkv, beta, dec, state = _inputs(cuda, [T], H, G, dk, dv, per_channel, delta, "mild", seed=at)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    cu, ctx, slot = i32([0, T]), i32([5]), i32([0])
+    lib = _lib.load()
+    ws = torch.empty(1 << 22, device=cuda)
+
+    def scan(x, b, d):
+        st, o = state.clone(), torch.zeros(T, H, dv, device=cuda)
+        _lib.check(lib.b2_channel_scan_ws(x.data_ptr(), b.data_ptr() if delta else None, d.data_ptr(), T, H, G, dk, dv, int(per_channel),
+                                          int(delta), cu.data_ptr(), ctx.data_ptr(), slot.data_ptr(), 1, st.data_ptr(), o.data_ptr(),
+                                          ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
+        return o
+
+    good = scan(qkv, beta, dec)
+    for what in ("q", "k", "v", "decay") + (("beta",) if delta else ()):
+        x, b, d = qkv.clone(), beta.clone() if delta else None, dec.clone()
+        if what == "decay":
+            d[at, 0] = bad
+        elif what == "beta":
+            b[at, 0] = bad
+        else:
+            x[at, {"q": 3, "k": G * dk + 3, "v": 2 * G * dk + 3}[what]] = bad
+        out = scan(x, b, d)
+        assert torch.equal(out[:at], good[:at]) and torch.equal(out[:, 1], good[:, 1]), what
+        assert what in ("decay", "beta") or not bool(torch.isfinite(out[at, 0]).all()), what
+        if what == "q":
+            assert torch.equal(out[at + 1:], good[at + 1:])

@@ -6,7 +6,9 @@
 // may have underflowed):
 //   A[t, s] = beta_t sum_i k_t k_s G_t/G_s  (s < t),    T = (I + A)^-1 diag(beta),     P[t, s] = sum_i q_t k_s G_t/G_s  (s <= t)
 //   U = T (V - (G K) S_0)   (no delta: U = V),   S = G_C S_0 + (G_C/G K)^T U,   O = (G Q) S_0 + P U
-// which is the same recurrence summed in another order (the WY form of Yang et al., "Parallelizing linear transformers with the
+// Nothing above a diagonal is multiplied: a product that counts no later token must not become NaN by an infinity or NaN in one, so zeros
+// there are selected or left out, and a token's output depends on it and earlier ones alone, as in the scan token by token.
+// It is the same recurrence summed in another order (the WY form of Yang et al., "Parallelizing linear transformers with the
 // delta rule over sequence length", 2024).  Three kernels, only the second of which is a chain:
 //   chunk_prep_kernel    P, T and the decay products; without delta also F = (G_C/G K)^T V: a CTA per (chunk, head)
 //   chunk_state_kernel   without delta: S <- G_C S + F over the chunks, element by element (memory bound)
@@ -295,7 +297,7 @@ chunk_prep_kernel(const ChunkArgs a) {
             for (int c = 0; c < 4; ++c) {
                 const int t = rg + 16 * (r & 3), x = cg + 16 * c;
                 const float2 h = halves(acc[r][c]);
-                const float v = (h.x + h.y) * Ps[t * (C + 1) + x];   // 0 above the diagonal
+                const float v = t >= x ? (h.x + h.y) * Ps[t * (C + 1) + x] : 0.f;
                 if (r < 4) Ps[t * (C + 1) + x] = v;
                 else As[t * (C + 1) + x] = t > x ? bs[t] * v : 0.f;
             }
@@ -337,7 +339,7 @@ chunk_prep_kernel(const ChunkArgs a) {
         __syncthreads();
         {
             float v[4] = {0.f, 0.f, 0.f, 0.f};
-            for (int s = 0; s < 32; ++s) {
+            for (int s = 0; s <= row; ++s) {
                 const float l = As[(32 + row) * (C + 1) + 32 + s];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) v[c] = fmaf(-l, x[s * (C + 1) + c4 + c], v[c]);
@@ -612,11 +614,14 @@ chunk_delta_kernel(const ChunkArgs a, int stages) {
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     const float xv[4] = {x[r].x, x[r].y, x[r].z, x[r].w};
+                    const int last = half * 32 + rg + 8 * r - s0;    // of the four columns, those up to the row's own
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        const pair_t xx = dup(xv[q]);
-                        fma2(acc[r][0], xx, y[q].x);
-                        fma2(acc[r][1], xx, y[q].y);
+                        if (q <= last) {
+                            const pair_t xx = dup(xv[q]);
+                            fma2(acc[r][0], xx, y[q].x);
+                            fma2(acc[r][1], xx, y[q].y);
+                        }
                     }
                 }
             }
@@ -721,13 +726,13 @@ chunk_out_kernel(const ChunkArgs a) {
         __syncthreads();                             // slice sl is there, the other stage is read
         if (sl + 1 < n1 + n2) issue(sl + 1, (sl + 1) & 1);
         const bool second = sl >= n1;
-        const int k0 = (second ? sl - n1 : sl) * 32, kn = second ? 32 : min(32, dk - k0);
+        const int k0 = (second ? sl - n1 : sl) * 32, kn = second ? min(32, rg * 4 + 4 - k0) : min(32, dk - k0);
         const int ld = second ? LP : LD;
         const float* rows = (second ? ps : qs) + (size_t)(rg * 4) * ld + k0;
         const float* b = bsm + (size_t)(sl & 1) * 32 * JB + tj * 4;
-        if (second && k0 > rg * 4 + 3) continue;     // above the diagonal
 #pragma unroll 2
-        for (int k = 0; k < kn; k += 4) {
+        for (int k = 0; k < kn; k += 4) {            // of P nothing above the diagonal
+            const bool edge = second && k0 + k == rg * 4;
             float4 x[4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(rows + r * ld + k);
@@ -736,6 +741,7 @@ chunk_out_kernel(const ChunkArgs a) {
                 const ulonglong2 y0 = pairs(b + (k + q) * JB), y1 = pairs(b + (k + q) * JB + 64);
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
+                    if (q > r && edge) continue;
                     const pair_t xx = dup(q == 0 ? x[r].x : q == 1 ? x[r].y : q == 2 ? x[r].z : x[r].w);
                     fma2(acc[r][0], xx, y0.x);
                     fma2(acc[r][1], xx, y0.y);
