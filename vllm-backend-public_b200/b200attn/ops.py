@@ -811,34 +811,14 @@ def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, H: in
 
 def _scan(lib, dev, qkv, beta, decay, T: int, H: int, G: int, dk: int, dv: int, per_channel: bool, delta: bool, batch: SeqBatch,
           state: torch.Tensor) -> torch.Tensor:
-    """b2_channel_scan_ws where it wants fp32 scratch for prompts in chunks, b2_channel_scan elsewhere: decode rows, fewer than two a
-    sequence, never do, and are not asked about."""
+    """b2_channel_scan_ws: prompts run in chunks, for which the call wants fp32 scratch."""
     o = torch.empty(T, H, dv, dtype=torch.float32, device=dev)
-    nws = 0 if T < 2 * batch.n_seq else lib.b2_channel_scan_workspace(T, batch.n_seq, H, dk, dv, per_channel, delta)
-    if not nws:
-        _lib.check(lib.b2_channel_scan(_ptr(qkv), _ptr(beta), _ptr(decay), T, H, G, dk, dv, per_channel, delta, _ptr(batch.cu_q),
-                                       _ptr(batch.ctx_start), _ptr(batch.state_slots), batch.n_seq, _ptr(state), _ptr(o), _stream(dev)))
-        return o
-    ws = torch.empty(nws, dtype=torch.float32, device=dev)
-    _lib.check(lib.b2_channel_scan_ws(_ptr(qkv), _ptr(beta), _ptr(decay), T, H, G, dk, dv, per_channel, delta, _ptr(batch.cu_q),
+    nws = lib.b2_channel_scan_workspace(T, batch.n_seq, H, dk, dv, int(per_channel), int(delta))
+    ws = torch.empty(nws, dtype=torch.float32, device=dev) if nws else None
+    _lib.check(lib.b2_channel_scan_ws(_ptr(qkv), _ptr(beta), _ptr(decay), T, H, G, dk, dv, int(per_channel), int(delta), _ptr(batch.cu_q),
                                       _ptr(batch.ctx_start), _ptr(batch.state_slots), batch.n_seq, _ptr(state), _ptr(o), _ptr(ws), nws,
                                       _stream(dev)))
     return o
-
-
-def scan_scratch_bytes(rows: int, seqs: int, mixers) -> int:
-    """The most scratch in bytes that one scan of the `mixers` -- (H, dk, dv, per_channel, delta) each -- over up to `rows` batch rows of
-    up to `seqs` sequences asks for.  Scratch grows with rows and sequences wherever the chunked form is taken, so only where its
-    rule ends has to be found: for every number of sequences, all rows and the most rows whose mean length just fills its chunks
-    of 64."""
-    lib = _lib.load()
-    most = 0
-    for H, dk, dv, per_channel, delta in set(mixers):
-        for n in range(1, min(rows, seqs) + 1):
-            for T in (rows, rows // n // 64 * 64 * n):
-                if T > 0:
-                    most = max(most, lib.b2_channel_scan_workspace(T, n, H, dk, dv, per_channel, delta))
-    return 4 * most
 
 
 def delta_out(o: torch.Tensor, proj: torch.Tensor, off_g: int, norm_w: torch.Tensor, eps: float) -> torch.Tensor:

@@ -1,6 +1,6 @@
 // b2_tc5.cuh -- tcgen05 / TMEM wrappers and the packed fp32 pipe, shared by the attention kernels on the 5th-gen tensor cores.
 #pragma once
-#include "b2_common.cuh"
+#include <stdint.h>
 
 #ifdef __CUDACC__
 namespace b2tc {
@@ -36,11 +36,6 @@ __device__ __forceinline__ uint64_t desc_join(uint32_t lo) {           // SBO = 
 }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {       // arrives on `bar` when all MMAs issued so far are done
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// After a wait has given up: shared memory and TMEM must not go while copies or MMAs are on their way to them.  Polls the phase they
-// complete for a millisecond at most, which is longer than any of them takes, in case it lacks an arrival and never ends.
-__device__ __forceinline__ void drain(uint32_t bar, uint32_t parity) {
-    for (int spins = 0; spins < 4096 && !b2::mbar_try_wait(bar, parity); ++spins) __nanosleep(256);
 }
 __device__ __forceinline__ bool elect_one() {                   // true in exactly one lane of the (converged) warp
     uint32_t pred;

@@ -87,10 +87,6 @@ moe_tc5_kernel(const __grid_constant__ ExpertArgs p) {
             for (int it = 0; it < nk; ++it) {
                 const int s = it % ST;
                 if (it >= ST) wait(empty(s), (it / ST - 1) & 1, failed);
-                if (*failed) {                       // no more copies; the last ones end before the shared memory goes
-                    for (int back = 1; back <= min(ST, it); ++back) drain(full((it - back) % ST), ((it - back) / ST) & 1);
-                    break;
-                }
                 b2::mbar_arrive_expect_tx(full(s), W_STAGE);         // columns and rows past the matrix are zero-filled and count
                 tma_load_3d(sm + s * W_STAGE, &p.map0, full(s), it * KSTEP, n0, e);
                 tma_load_3d(sm + s * W_STAGE + W_STAGE / 2, &p.map1, full(s), it * KSTEP, KIND == PAIR ? n0 : n0 + 64, e);
@@ -183,7 +179,10 @@ moe_tc5_kernel(const __grid_constant__ ExpertArgs p) {
             b2::st(static_cast<bf16*>(p.out) + (size_t)(m0 + r) * p.N + n0 + c, bad ? __int_as_float(0x7fc00000) : v);
         }
     }
-    if (bad) drain(b2::smem_u32(&s_end), 0);
+    if (bad && tid < ST && tid < nk) {               // copies still in flight end before the shared memory goes
+        const int last = (nk - 1 - tid) / ST;
+        for (uint32_t spins = 0; spins < (1u << 20) && !b2::mbar_try_wait(full(tid), last & 1); ++spins) {}
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

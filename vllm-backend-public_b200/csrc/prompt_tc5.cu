@@ -30,8 +30,6 @@
 #include "b2_mask.cuh"
 #include "b2_tc5.cuh"
 
-#include <algorithm>
-
 namespace {
 
 using namespace b2tc;
@@ -39,6 +37,7 @@ using namespace b2tc;
 constexpr int BM = 128, BN = 128, NTHREADS = 384;
 constexpr int SUB = 128 * 128;                       // bytes of a [128 rows][64 el] sub-tile
 constexpr float LOG2E = 1.4426950408889634f;
+constexpr float RESCALE_THRESHOLD = 8.f;             // log2 units
 constexpr float FLOOR = -1e30f;                      // a row that has seen no key yet: exp2(-inf - FLOOR) = 0, not NaN
 enum { KIND_SOFTMAX = 0, KIND_CAPPED = 1, KIND_SIGMOID = 2 };
 
@@ -117,6 +116,7 @@ __device__ __forceinline__ RowRange range_of(const KeySpan& span, int i, int chu
 }
 // what one thread works out for the CTA
 struct Plan {
+    int seq, q0, len, ctx, row0;
     KeySpan span;
     int keep;                                        // compact index below which keys are kept for every row of their mask block
     int first_row[2], rows[2];                       // position of a slot's first row, number of rows
@@ -142,53 +142,36 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
     auto bar = [&](int i) { return bars + 8u * i; };
     volatile int* failed = &s_failed;
 
-    // This CTA's tile: counted from the batch's last row backwards (late rows see more keys, and the spare CTAs of a grid that is an
-    // upper bound come behind all tiles), by every warp for itself, 32 sequences at a time, so that a spare CTA leaves at once.
-    const int groups = a.H / prm.heads_per_cta, group = blockIdx.x % groups;
-    int seq = -1, q0 = 0, len = 0;
-    {
-        int want = blockIdx.x / groups;
-#pragma unroll 1
-        for (int top = a.n_seq - 1; top >= 0; top -= 32) {
-            const int s = top - lane, n = s >= 0 ? a.cu_q[s + 1] - a.cu_q[s] : 0;
-            const int nt = n >= a.min_rows ? (n + prm.rows_per_cta - 1) / prm.rows_per_cta : 0;
-            int upto = nt;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int below = __shfl_up_sync(0xffffffffu, upto, d);
-                if (lane >= d) upto += below;
-            }
-            const uint32_t hit = __ballot_sync(0xffffffffu, want < upto);
-            if (hit) {
-                const int who = __ffs(hit) - 1;
-                seq = top - who;
-                len = __shfl_sync(0xffffffffu, n, who);
-                q0 = (__shfl_sync(0xffffffffu, upto, who) - 1 - want) * prm.rows_per_cta;
-                break;
-            }
-            want -= __shfl_sync(0xffffffffu, upto, 31);
-        }
-    }
-    if (seq < 0) return;
-    const int ctx = a.ctx_start[seq], row0 = a.cu_q[seq] + q0;
-    if (ctx < 0) {                                                   // padding: zero rows (the paged form's are another kernel's)
-        const int rows = GATHERED ? min(len - q0, prm.rows_per_cta) : 0, v8 = a.dv / 8;
-        for (int idx = tid; idx < rows * v8; idx += NTHREADS)
-            *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + (size_t)(row0 + idx / v8) * a.out_stride + (size_t)group * a.dv + (idx % v8) * 8) =
-                make_uint4(0, 0, 0, 0);
-        return;
-    }
-
     if (tid == 0) {
         s_failed = 0;
         Plan& pl = s_plan;
+        int want = (int)(gridDim.y - 1 - blockIdx.y), q0 = 0;        // late rows, which see more keys, first
+        pl.seq = -1;
+        pl.ctx = -1;
+        pl.row0 = 0;
+        pl.span.n = 0;
+        for (int s = 0; s < a.n_seq; ++s) {
+            const int len = a.cu_q[s + 1] - a.cu_q[s];
+            if (len < a.min_rows) continue;
+            const int nt = (len + prm.rows_per_cta - 1) / prm.rows_per_cta;
+            if (want < nt) {
+                q0 = want * prm.rows_per_cta;
+                pl.seq = s;
+                pl.len = len;
+                pl.ctx = a.ctx_start[s];
+                pl.row0 = a.cu_q[s] + q0;
+                break;
+            }
+            want -= nt;
+        }
+        pl.q0 = q0;
         pl.rows[0] = pl.rows[1] = pl.t0[0] = pl.t0[1] = pl.t1[0] = pl.t1[1] = 0;
-        {
-            const int left = len - q0, p0 = ctx + q0, p_last = p0 + min(left, prm.rows_per_cta) - 1;
+        if (pl.seq >= 0 && pl.ctx >= 0) {
+            const int left = pl.len - q0, p0 = pl.ctx + q0, p_last = p0 + min(left, prm.rows_per_cta) - 1;
             const bool two = prm.rows_per_cta > BM;
             KeySpan span = key_span(p0, p_last, a.chunk, a.window, a.keep_first);
-            if (GATHERED && span.wlo < a.k_lo[seq]) {                // the gathered rows begin at k_lo
-                span.wlo = span.lo = a.k_lo[seq];
+            if (GATHERED && span.wlo < a.k_lo[pl.seq]) {             // the gathered rows begin at k_lo
+                span.wlo = span.lo = a.k_lo[pl.seq];
                 span.n = p_last - span.lo + 1;
             }
             pl.span = span;
@@ -227,14 +210,23 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
+    const int seq = s_plan.seq, row0 = s_plan.row0;
+    const bool active = seq >= 0 && s_plan.ctx >= 0;                 // CTA-uniform
     const int hpc = prm.heads_per_cta;
     const bool two_rows = prm.rows_per_cta > BM;
     const int n_tiles = max(s_plan.t1[0], s_plan.t1[1]), n_keys = s_plan.span.n;
-    const int kvh = (group * hpc) / (a.H / a.G);                // kv head of the paged pools
+    const int kvh = (blockIdx.x * hpc) / (a.H / a.G);                // kv head of the paged pools
+
+    if (GATHERED && seq >= 0 && !active) {                           // padding: zero rows (the paged form's are another kernel's)
+        const int rows = min(s_plan.len - s_plan.q0, prm.rows_per_cta), v8 = a.dv / 8, hh = blockIdx.x;
+        for (int idx = tid; idx < rows * v8; idx += NTHREADS)
+            *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + (size_t)(row0 + idx / v8) * a.out_stride + (size_t)hh * a.dv + (idx % v8) * 8) =
+                make_uint4(0, 0, 0, 0);
+    }
 
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-        if (warp != 9) {
+        if (active && warp != 9) {
             // ------------------------------------------ copies: warps 8 and 11 the even and odd groups of K rows, warp 10 V
             // Eight lanes copy the 128 bytes of a row and sub-tile, four rows (a group) an instruction.  The pool rows of a tile's
             // 128 keys (four a lane, through the page table) are looked up before the stage is free: a lookup in front of its
@@ -270,7 +262,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             {                                                        // Q, by all three warps: rows past the tile are zeros
 #pragma unroll 1
                 for (int x = 0; x < 2; ++x) {
-                    const int hh = group * hpc + (hpc == 2 ? x : 0), nrows = s_plan.rows[x];
+                    const int hh = blockIdx.x * hpc + (hpc == 2 ? x : 0), nrows = s_plan.rows[x];
                     const int rbase = row0 + (two_rows && x ? BM : 0);
                     if (nrows == 0) continue;
                     const int col0 = TWO_MAPS ? x * a.dk : 0;
@@ -296,24 +288,19 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             const int nst = is_v ? L::VST : L::KST;
             const int n_sub = is_v ? DVH : L::KSUBS, width = is_v ? a.dv : a.dk, split = GATHERED && !is_v ? a.dk0 : width;
             const uint32_t ld = 2u * (uint32_t)(GATHERED ? a.H * split : width), ld1 = 2u * (uint32_t)a.k1_row;    // bytes between pool rows
-            const char* p0 = reinterpret_cast<const char*>(static_cast<const bf16*>(is_v ? a.v : a.k0) + (GATHERED ? (size_t)group * split : 0) + c8 * 8);
+            const char* p0 = reinterpret_cast<const char*>(static_cast<const bf16*>(is_v ? a.v : a.k0) + (GATHERED ? (size_t)blockIdx.x * split : 0) + c8 * 8);
             const char* p1 = GATHERED && !is_v ? reinterpret_cast<const char*>(static_cast<const bf16*>(a.k1) + c8 * 8) - 2 * split : p0;
             const uint32_t map2 = 2u * (uint32_t)a.bs * (uint32_t)a.dk;                  // the second map's rows lie a page of the first behind
 #pragma unroll 1
             for (int it = 0; it < n_tiles; ++it) {
                 const int s = it % nst, ph = (it / nst) & 1;
                 wait(bar((is_v ? L::BAR_VE : L::BAR_KE) + s), ph ^ 1, failed);
-                if (__any_sync(0xffffffffu, *failed)) {              // no more copies; the last boxes end before the shared memory goes
-                    for (int back = 1; GATHERED && lane == 0 && back <= min(nst, it); ++back)
-                        drain(bar((is_v ? L::BAR_V : L::BAR_K) + (it - back) % nst), ((it - back) / nst) & 1);
-                    break;
-                }
                 const uint32_t base = is_v ? v_ring + s * L::V_STAGE : k_ring + s * L::K_STAGE;
                 const uint32_t full = bar((is_v ? L::BAR_V : L::BAR_K) + s);
                 const bool whole = GATHERED && prm.tma && (it + 1) * BN <= n_keys;      // all 128 rows are this sequence's
                 if (whole && !odd) {
                     if (lane == 0) {
-                        const int row = (int)g0 + span.wlo + it * BN, hh = group;
+                        const int row = (int)g0 + span.wlo + it * BN, hh = blockIdx.x;
                         b2::mbar_arrive_expect_tx(full, (uint32_t)n_sub * SUB);          // columns past the head are zero-filled and count
 #pragma unroll 1
                         for (int h = 0; h < n_sub; ++h) {
@@ -364,7 +351,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                 __syncwarp();
                 if (lane == 0 && !(whole && !odd)) b2::mbar_arrive(full);
             }
-        } else {
+        } else if (active && warp == 9) {
             // ------------------------------------------ MMA issuer: the whole warp, warp-uniform operands, one elected lane
             // step j: P_0 V(j), Q_0 K(j+1), P_1 V(j), Q_1 K(j+1) -- the softmax of one slot runs under the MMAs of the other
             constexpr uint32_t ID_QK = idesc_bf16(128, 128, 0), ID_PV = idesc_bf16(128, 64 * DVH, 1);
@@ -429,7 +416,6 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             if (elect_one()) mma_commit(bar(L::BAR_END));            // nothing in flight when the TMEM is given back
             __syncwarp();
             wait(bar(L::BAR_END), 0, failed);
-            if (*failed) drain(bar(L::BAR_END), 0);
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
@@ -440,7 +426,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             const int row = wq * 32 + lane;                          // query row of the slot = TMEM lane
             const uint32_t lane_off = (uint32_t)(wq * 32) << 16;
             const uint32_t s_addr = tmem + lane_off + x * 128, o_addr = tmem + lane_off + 256 + x * 128;
-            const int hh = group * hpc + (hpc == 2 ? x : 0);
+            const int hh = blockIdx.x * hpc + (hpc == 2 ? x : 0);
             const RowRange mine = range_of(s_plan.span, s_plan.first_row[x] + min(row, nrows - 1), a.chunk, a.window);
             const int all_hi = s_plan.all_hi[x], all_low = s_plan.all_low[x], keep = s_plan.keep;
             const float sl2 = prm.scale_log2;
@@ -464,6 +450,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                 auto reduce = [&]() {
                     return fmaxf(fmaxf(fmaxf(mp[0], mp[1]), fmaxf(mp[2], mp[3])), fmaxf(fmaxf(mp[4], mp[5]), fmaxf(mp[6], mp[7])));
                 };
+                float mx = -INFINITY;
                 bool small = false;
                 uint32_t see[4] = {~0u, ~0u, ~0u, ~0u};
                 if (KIND == KIND_CAPPED) {
@@ -472,12 +459,13 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
 #pragma unroll
                         for (int k = 0; k < 32; ++k) mp[k & 7] = fmaxf(mp[k & 7], fabsf(__uint_as_float(sr[c][k])));
                     const float am = reduce();
-                    small = __all_sync(0xffffffffu, cx > 0.f && am * cx <= 0.1875f);
+                    small = __all_sync(0xffffffffu, cx > 0.f && am * cx <= 0.1875f && am * eff <= 30.f);
                     if (small) {
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
 #pragma unroll
                             for (int k = 0; k < 32; k += 2) tanh_small_x2(sr[c][k], sr[c][k + 1], a1, a2, a3);
+                        mx = am * eff;                               // no score of the row is above it, none 2^60 below
                     } else {                                         // any score, any scale: through TMEM, a rolled loop
                         eff = 1.f;
 #pragma unroll 1
@@ -512,18 +500,26 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                     }
                 }
                 if (KIND != KIND_SIGMOID) {
+                    if (!small) {
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) mp[k] = -INFINITY;
+                        for (int k = 0; k < 8; ++k) mp[k] = -INFINITY;
 #pragma unroll
-                    for (int c = 0; c < 4; ++c)
+                        for (int c = 0; c < 4; ++c)
 #pragma unroll
-                        for (int k = 0; k < 32; ++k) mp[k & 7] = fmaxf(mp[k & 7], __uint_as_float(sr[c][k]));
-                    const float m_new = fmaxf(fmaxf(m, reduce() * eff), FLOOR), alpha = b2::fast_exp2(m - m_new);
-                    l *= alpha;                                      // at first the sink's share, if any; exp2(-inf) = 0
-                    if (i > 0) {
-                        if (__any_sync(0xffffffffu, m_new > m)) {    // else every factor is one
+                            for (int k = 0; k < 32; ++k) mp[k & 7] = fmaxf(mp[k & 7], __uint_as_float(sr[c][k]));
+                        mx = reduce() * eff;
+                    }
+                    const float m_new = fmaxf(fmaxf(m, mx), FLOOR);
+                    if (i == 0) {
+                        l *= b2::fast_exp2(m - m_new);               // the sink's share, if any; exp2(-inf) = 0
+                        m = m_new;
+                    } else {
+                        const bool need = m_new - m > RESCALE_THRESHOLD;
+                        if (__any_sync(0xffffffffu, need)) {         // rare after the first tiles
                             wait(bar(L::BAR_PV + x), (i - 1) & 1, failed);
                             tc_fence_after();
+                            const float alpha = need ? b2::fast_exp2(m - m_new) : 1.f;
+                            if (need) { m = m_new; l *= alpha; }
 #pragma unroll 1
                             for (int c = 0; c < 2 * DVH; ++c) {
                                 uint32_t o[32];
@@ -535,7 +531,6 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                             }
                         }
                     }
-                    m = m_new;
                 }
                 float sum[4] = {0.f, 0.f, 0.f, 0.f};                 // the denominator sums the fp32 weights
 #pragma unroll
@@ -568,12 +563,12 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                 if (KIND != KIND_SIGMOID) l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
             }
             // ------------------------------------------ output rows
+            float inv = KIND == KIND_SIGMOID ? 1.f : (l > 0.f ? 1.f / l : 0.f);
+            if (*failed) inv = __int_as_float(0x7fc00000);
             const int n = te - tb;
             const bool valid = row < nrows;
             const size_t brow = (size_t)row0 + (two_rows && x ? BM : 0) + row;
             wait(bar(L::BAR_PV + x), (n - 1) & 1, failed);
-            float inv = KIND == KIND_SIGMOID ? 1.f : (l > 0.f ? 1.f / l : 0.f);
-            if (*failed) inv = __int_as_float(0x7fc00000);           // behind the last wait, which may be the one that gave up
             if (TWO_MAPS && x == 1) {                                // slot 0 writes: it reads both outputs from its own TMEM lane
                 s_inv[TWO_MAPS ? row : 0] = inv;
                 tc_fence_after();
@@ -715,8 +710,7 @@ int b2_internal_prompt_tc5(const b2_prompt_args& a, void* stream) {
     }
     // Two slots a CTA share the copies of a key tile and cover each other's softmax; a launch of fewer than one wave of such CTAs
     // takes one slot each (twice the CTAs, each a little faster).  Two heads of a kv head before two row tiles: see above.
-    const int64_t longs = std::min(a.n_seq, a.T / a.min_rows);       // sequences of min_rows rows or more
-    const int64_t tiles128 = (int64_t)a.T / BM + longs, tiles256 = (int64_t)a.T / (2 * BM) + longs;
+    const int64_t tiles128 = (int64_t)a.T / BM + a.n_seq, tiles256 = (int64_t)a.T / (2 * BM) + a.n_seq;
     p.rows_per_cta = BM;
     p.heads_per_cta = 1;
     if (a.maps == 1) {
@@ -725,10 +719,8 @@ int b2_internal_prompt_tc5(const b2_prompt_args& a, void* stream) {
         else if (!pair && tiles256 * a.H >= n_sm) p.rows_per_cta = 2 * BM;
     }
     const int64_t tiles = p.rows_per_cta == BM ? tiles128 : tiles256;        // upper bound on sum(ceil(len / rows)); spare CTAs leave at once
-    if (tiles == 0) return B2_OK;
-    const int64_t ctas = tiles * (a.H / p.heads_per_cta);
-    B2_REQUIRE(ctas <= 0x7fffffff, B2_EUNSUPPORTED, "prompt attention: %lld row tiles exceed the grid", (long long)tiles);
-    const dim3 grid((unsigned)ctas);
+    B2_REQUIRE(tiles <= 65535, B2_EUNSUPPORTED, "prompt attention: %lld row tiles exceed the grid", (long long)tiles);
+    const dim3 grid((unsigned)(a.H / p.heads_per_cta), (unsigned)tiles);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nh = (a.dk + 63) / 64, dvh = (a.dv + 63) / 64;
     const bool one_by_one = a.cap > 0.f || !(a.scale > 0.f);         // the capped form takes any score and any sign of the scale
