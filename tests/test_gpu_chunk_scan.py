@@ -134,3 +134,21 @@ def test_nothing_runs_backwards(cuda, at, delta, per_channel, bad):
         assert what in ("decay", "beta") or not bool(torch.isfinite(out[at, 0]).all()), what
         if what == "q":
             assert torch.equal(out[at + 1:], good[at + 1:])
+
+
+@pytest.mark.parametrize("delta", [False, True])
+def test_decode_rows_do_not_ask_for_scratch(cuda, monkeypatch, delta):
+    """A decode step's scan is one call into the library, as many of them are launched one by one."""
+    n, H, dk, dv = 3, 2, 32, 32
+    qkv, beta, dec, state = _inputs(cuda, [1] * n, H, H, dk, dv, False, delta, "mild", seed=5)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    batch = ops.SeqBatch(i32(list(range(n + 1))), i32([4] * n), None, i32(list(range(n))), n, n)
+
+    def asked(*_):
+        raise AssertionError("a scan of decode rows asked for scratch")
+
+    monkeypatch.setattr(_lib.load(), "b2_channel_scan_workspace", asked)
+    st, ref = state.clone(), state.clone()
+    out = ops.channel_scan(qkv, beta, dec, H, H, dk, dv, batch, st, delta=delta)
+    want, ref = _reference(qkv, beta, dec, ref, [1] * n, [4] * n, list(range(n)), H, H, dk, dv)
+    assert float((out.double() - want).norm() / want.norm()) < 2e-6 and float((st.double() - ref).norm() / ref.norm()) < 2e-6

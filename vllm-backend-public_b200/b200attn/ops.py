@@ -811,11 +811,16 @@ def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, H: in
 
 def _scan(lib, dev, qkv, beta, decay, T: int, H: int, G: int, dk: int, dv: int, per_channel: bool, delta: bool, batch: SeqBatch,
           state: torch.Tensor) -> torch.Tensor:
-    """b2_channel_scan_ws: prompts run in chunks, for which the call wants fp32 scratch."""
+    """b2_channel_scan_ws where it wants fp32 scratch for prompts in chunks, b2_channel_scan elsewhere: decode rows, fewer than two a
+    sequence, never do, and are not asked about."""
     o = torch.empty(T, H, dv, dtype=torch.float32, device=dev)
-    nws = lib.b2_channel_scan_workspace(T, batch.n_seq, H, dk, dv, int(per_channel), int(delta))
-    ws = torch.empty(nws, dtype=torch.float32, device=dev) if nws else None
-    _lib.check(lib.b2_channel_scan_ws(_ptr(qkv), _ptr(beta), _ptr(decay), T, H, G, dk, dv, int(per_channel), int(delta), _ptr(batch.cu_q),
+    nws = 0 if T < 2 * batch.n_seq else lib.b2_channel_scan_workspace(T, batch.n_seq, H, dk, dv, per_channel, delta)
+    if not nws:
+        _lib.check(lib.b2_channel_scan(_ptr(qkv), _ptr(beta), _ptr(decay), T, H, G, dk, dv, per_channel, delta, _ptr(batch.cu_q),
+                                       _ptr(batch.ctx_start), _ptr(batch.state_slots), batch.n_seq, _ptr(state), _ptr(o), _stream(dev)))
+        return o
+    ws = torch.empty(nws, dtype=torch.float32, device=dev)
+    _lib.check(lib.b2_channel_scan_ws(_ptr(qkv), _ptr(beta), _ptr(decay), T, H, G, dk, dv, per_channel, delta, _ptr(batch.cu_q),
                                       _ptr(batch.ctx_start), _ptr(batch.state_slots), batch.n_seq, _ptr(state), _ptr(o), _ptr(ws), nws,
                                       _stream(dev)))
     return o
