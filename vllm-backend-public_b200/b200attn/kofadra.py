@@ -108,7 +108,9 @@ class KofadraConfig:
         wide = max([self.hidden] + [2 * (2 * m.kv_heads * m.dim + 2 * m.heads * m.vdim + m.heads * m.dim)
                                     for m in (L.mixer for L in self.layer_specs)])
         moe = max([0] + [L.mlp.top * (L.mlp.ff * elem_bytes + self.hidden * 4) for L in self.layer_specs if L.mlp])
-        return tokens * (max(self.streams, 1) * self.hidden * 4 + 6 * wide * 4 + 2 * moe) + seqs * self.vocab * 8 + (1 << 28)
+        scan = ops.scan_scratch_bytes(tokens, seqs, [(m.heads, m.dim, m.vdim, False, True) for m in (L.mixer for L in self.layer_specs)
+                                                     if m.kind == "delta"])
+        return tokens * (max(self.streams, 1) * self.hidden * 4 + 6 * wide * 4 + 2 * moe) + scan + seqs * self.vocab * 8 + (1 << 28)
 
     def build_model(self, device, **kw):
         return KofadraModel(self, device, **kw)

@@ -229,7 +229,9 @@ class LizazenConfig:
                 n = max(n, 3 * f.shared_ff)
                 moe.append(f.top * (3 * f.ff * elem_bytes + self.hidden * 4))
             wide.append(n)
-        return tokens * (self.hidden * 12 + 2 * max(wide) * elem_bytes + 2 * max(moe)) + seqs * self.vocab * 8 + (1 << 28)
+        scan = ops.scan_scratch_bytes(tokens, seqs, [(m.right.heads, m.right.dim, m.right.vdim, False, False)
+                                                     for m in (L.mixer for L in self.layer_specs) if isinstance(m, ParallelSpec)])
+        return tokens * (self.hidden * 12 + 2 * max(wide) * elem_bytes + 2 * max(moe)) + scan + seqs * self.vocab * 8 + (1 << 28)
 
     def build_model(self, device, **kw):
         return LizazenModel(self, device, **kw)

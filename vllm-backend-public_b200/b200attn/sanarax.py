@@ -158,7 +158,9 @@ class SanaraxConfig:
                 wide.append(m.q_rank + m.row + m.heads * (m.dim + m.rot_dim + 1 + 2 * m.row + m.vdim))
             if L.mlp is not None:
                 wide.append(2 * L.mlp.ff)
-        return tokens * (self.hidden * 8 + 2 * max(wide) * elem_bytes) + seqs * self.vocab * 8 + (1 << 28)
+        scan = ops.scan_scratch_bytes(tokens, seqs, [(m.heads, m.dim, m.vdim, False, False) for m in (L.mixer for L in self.layer_specs)
+                                                     if isinstance(m, LightningSpec)])
+        return tokens * (self.hidden * 8 + 2 * max(wide) * elem_bytes) + scan + seqs * self.vocab * 8 + (1 << 28)
 
     def build_model(self, device, **kw):
         return SanaraxModel(self, device, **kw)

@@ -169,7 +169,10 @@ class TonilixConfig:
                 wide.append(3 * L.mlp.ff)
         moe = max([0] + [L.mlp.top * (L.mlp.ff * elem_bytes + self.hidden * 4) for L in self.layer_specs
                          if isinstance(L.mlp, ExpertsSpec)])
-        return tokens * (self.hidden * 12 + 4 * max(wide) + 2 * moe) + seqs * self.vocab * 8 + (1 << 28)
+        scan = ops.scan_scratch_bytes(tokens, seqs, [(m.heads, m.dim, m.vdim, True, True) if isinstance(m, DeltaSpec) else
+                                                     (m.right.heads, m.right.dim, m.right.vdim, True, False)
+                                                     for m in (L.mixer for L in self.layer_specs)])
+        return tokens * (self.hidden * 12 + 4 * max(wide) + 2 * moe) + scan + seqs * self.vocab * 8 + (1 << 28)
 
     def build_model(self, device, **kw):
         return TonilixModel(self, device, **kw)
