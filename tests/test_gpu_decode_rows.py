@@ -1,5 +1,5 @@
 """Short portions of b2_masked_attention (fewer rows than the prompt kernel takes): the forms with the keys or the query heads as the
-16 rows of the operand, 4, 8 and 16 warps a CTA, key counts around their tiles of 16, several rows a sequence, and batches in which
+16 rows of the operand, 4, 8 and 16 warps a CTA, key counts around their tiles of 16 and 32, several rows a sequence, and batches in which
 they stand beside prompts and padding; against fp64 by the same check and bound as the prompt rows."""
 import pytest
 import torch
@@ -25,6 +25,10 @@ pytestmark = pytest.mark.gpu
     ([1, 5], [700, 90], 8, 2, 64, 256, 16, 0, 0, 0, 0.0, False, 1, False, False, 1.0),
     ([1, 7], [300, 20], 12, 1, 128, 64, 16, 0, 0, 0, 0.0, False, 2, False, False, 1.0),                  # two maps
     ([200, 1, 3, 90, 2], [0, 300, 40, 7, 0], 8, 2, 128, 128, 16, 0, 0, 0, 0.0, True, 1, False, False, 1.0),      # beside prompts
+    ([1] * 12, [0, 15, 16, 30, 31, 32, 33, 62, 63, 64, 127, 128], 16, 2, 64, 64, 16, 0, 0, 0, 0.0, True, 1, False, False, 1.0),  # keys of 64: 32 a tile
+    ([1, 2, 14], [1000, 255, 256], 8, 4, 64, 128, 16, 0, 0, 0, 25.0, True, 1, False, True, 1.0),         # ... 16 warps a CTA
+    ([1] * 30, list(range(300, 600, 10)), 32, 8, 32, 256, 16, 0, 200, 3, 0.0, False, 1, False, False, 1.0),      # ... 8
+    ([1, 5], [700, 90], 8, 2, 64, 192, 16, 0, 0, 0, 0.0, False, 1, True, True, 1.0),                     # ... sigmoid
 ])
 def test_short_portions(cuda, c):
     _check(cuda, c)

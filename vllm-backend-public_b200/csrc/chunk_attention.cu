@@ -668,17 +668,20 @@ constexpr int kHeadRows = 16, kHeadKeys = 16;
 
 // At most eight query heads a kv head (and one map, dk <= 128): the keys are the 16 rows of the operand and the heads its 8 columns,
 // S^T = K Q^T and O^T += V^T P^T.  No half of the tile is padding: half the products, scores, rescales and accumulators of the form
-// below, Q in registers, and P^T turns into an operand by two 8 x 8 transpositions.
+// below, Q in registers, and P^T turns into an operand by 8 x 8 transpositions.  Keys of 64
+// numbers and less go 32 at a time: the same bytes in flight as 16 of 128, and the weights' rounding is that of tiles of 32, which these
+// sizes always had (a router behind such a layer may stand within it of another choice).  128 rows x 8 kv heads x 2000 keys of 64: 92 us,
+// 108 in tiles of 16.
 __device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
     uint32_t y;
     asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
     return y;
 }
 
-constexpr int kFewHeads = 8, kFewDk = 128;
+constexpr int kFewHeads = 8, kFewDk = 128, kShortDk = 64;
 
-template <int DVT, bool SIG, int NW>
-__global__ void __launch_bounds__(32 * NW, DVT <= 8 && NW < 16 ? 20 / NW : 16 / NW)
+template <int DVT, bool SIG, int NW, int KEYS>
+__global__ void __launch_bounds__(32 * NW, DVT <= 8 && NW < 16 && KEYS == kHeadKeys ? 20 / NW : 16 / NW)
 chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
                              const __nv_bfloat16* __restrict__ v_cache, const int32_t* __restrict__ block_tables, int max_nb,
                              const int32_t* __restrict__ cu_q, const int32_t* __restrict__ ctx_start, int n_seq, int H, int G,
@@ -686,9 +689,9 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
                              float sink_logit, const float* __restrict__ sink_logits, const float* __restrict__ head_bias,
                              const __nv_bfloat16* __restrict__ gate, int64_t gate_stride, HeadShape hs, int skip_rows_from, bool by_seq,
                              __nv_bfloat16* __restrict__ out, int64_t out_stride) {
-    constexpr int DV = 16 * DVT, LDV = DV + 8, PW = 2 + DV, NTH = 32 * NW;
+    constexpr int DV = 16 * DVT, LDV = DV + 8, PW = 2 + DV, NTH = 32 * NW, MAXDK = KEYS > kHeadKeys ? kShortDk : kFewDk;
     constexpr float kLog2e = 1.4426950408889634f;
-    // q [8][dk + 8], then per warp: K tile [16][dk + 8], V tile [16][DV + 8]; the merge reuses the tiles' place
+    // q [8][dk + 8], then per warp: K tile [KEYS][dk + 8], V tile [KEYS][DV + 8]; the merge reuses the tiles' place
     extern __shared__ __align__(16) unsigned char head_sm[];
     const int g = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -714,16 +717,16 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
     const int ldq = dk + 8, ldk = dk + 8;
     __nv_bfloat16* q_sm = reinterpret_cast<__nv_bfloat16*>(head_sm);
     __nv_bfloat16* tiles = q_sm + kFewHeads * ldq;
-    __nv_bfloat16* kt = tiles + (size_t)w * kHeadKeys * (ldk + LDV);
-    __nv_bfloat16* vt = kt + kHeadKeys * ldk;
+    __nv_bfloat16* kt = tiles + (size_t)w * KEYS * (ldk + LDV);
+    __nv_bfloat16* vt = kt + KEYS * ldk;
     float* part = reinterpret_cast<float*>(tiles);       // [NW][8][m, l, O (DV)]
     const uint32_t q_base = b2::smem_u32(q_sm), k_base = b2::smem_u32(kt), v_base = b2::smem_u32(vt);
     const int gq = lane >> 2, tq = lane & 3;
     const float cap_log2 = hs.cap * kLog2e, cap_e = hs.cap > 0.f ? 2.f / hs.cap : 0.f;
-    constexpr int STEP = NW * kHeadKeys;
+    constexpr int STEP = NW * KEYS;
 
     // keys past the end repeat the last one: finite numbers that the mask drops
-    auto key_at = [&](int c) { return span.key(min(c + (lane & 15), span.n - 1)); };
+    auto key_at = [&](int c) { return span.key(min(c + (lane & (KEYS - 1)), span.n - 1)); };
     auto page_of = [&](int j, int& off) {
         const int pg = j / bs;
         off = j - pg * bs;
@@ -732,20 +735,20 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
     int off, page, next_off = 0, next_page = 0;      // of the tile in flight, and of the one behind it
     auto issue_k = [&]() {
 #pragma unroll
-        for (int kq = 0; kq < kHeadKeys / 8; ++kq) {
+        for (int kq = 0; kq < KEYS / 8; ++kq) {
             const int key = kq * 8 + (lane >> 2), c = (lane & 3) * 8;
             const size_t pg = __shfl_sync(0xffffffffu, page, key);
             const int of = __shfl_sync(0xffffffffu, off, key);
             const __nv_bfloat16* ks = k_cache + ((pg * G + g) * bs + of) * dk + c;
             __nv_bfloat16* kd = kt + key * ldk + c;
 #pragma unroll
-            for (int t = 0; t < kFewDk; t += 32)
+            for (int t = 0; t < MAXDK; t += 32)
                 if (t < dk) cp_async16(kd + t, ks + t);
         }
     };
     auto issue_v = [&]() {
 #pragma unroll
-        for (int kq = 0; kq < kHeadKeys / 8; ++kq) {
+        for (int kq = 0; kq < KEYS / 8; ++kq) {
             const int key = kq * 8 + (lane >> 2), c = (lane & 3) * 8;
             const size_t pg = __shfl_sync(0xffffffffu, page, key);
             const int of = __shfl_sync(0xffffffffu, off, key);
@@ -755,7 +758,7 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
             for (int t = 0; t < DV; t += 32) cp_async16(vd + t, vs + t);
         }
     };
-    const int first = w * kHeadKeys;
+    const int first = w * KEYS;
     if (first < span.n) {
         page = page_of(key_at(first), off);
         issue_k();
@@ -771,9 +774,9 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
         *reinterpret_cast<uint4*>(q_sm + r * ldq + c) = v;
     }
     __syncthreads();
-    uint32_t qf[kFewDk / 16][2];
+    uint32_t qf[MAXDK / 16][2];
 #pragma unroll
-    for (int kk = 0; kk < kFewDk / 16; kk += 2) {
+    for (int kk = 0; kk < MAXDK / 16; kk += 2) {
         qf[kk][0] = qf[kk][1] = qf[kk + 1][0] = qf[kk + 1][1] = 0u;
         if (kk * 16 < dk) b2::ldmatrix_x4(q_base + 2u * ((lane & 7) * ldq + kk * 16 + (lane >> 3) * 8), qf[kk][0], qf[kk][1], qf[kk + 1][0], qf[kk + 1][1]);
     }
@@ -797,15 +800,20 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
         const bool more = c0 + STEP < span.n;
         asm volatile("cp.async.wait_group 1;" ::: "memory");     // K is there, V may still be on its way
         __syncwarp();
-        float sc[4][4];                              // four chains
+        float sc[KEYS / 16][4][4];                   // four chains
 #pragma unroll
-        for (int c = 0; c < 4; ++c) sc[c][0] = sc[c][1] = sc[c][2] = sc[c][3] = 0.f;
+        for (int n = 0; n < KEYS / 16; ++n)
 #pragma unroll
-        for (int kk = 0; kk < kFewDk / 16; ++kk) {
+            for (int c = 0; c < 4; ++c) sc[n][c][0] = sc[n][c][1] = sc[n][c][2] = sc[n][c][3] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < MAXDK / 16; ++kk) {
             if (kk * 16 >= dk) break;
-            uint32_t a0, a1, a2, a3;
-            b2::ldmatrix_x4(k_base + 2u * ((lane & 15) * ldk + kk * 16 + (lane >> 4) * 8), a0, a1, a2, a3);
-            b2::mma_bf16_16816(sc[kk & 3], a0, a1, a2, a3, qf[kk][0], qf[kk][1]);
+#pragma unroll
+            for (int n = 0; n < KEYS / 16; ++n) {
+                uint32_t a0, a1, a2, a3;
+                b2::ldmatrix_x4(k_base + 2u * ((n * 16 + (lane & 15)) * ldk + kk * 16 + (lane >> 4) * 8), a0, a1, a2, a3);
+                b2::mma_bf16_16816(sc[n][kk & 3], a0, a1, a2, a3, qf[kk][0], qf[kk][1]);
+            }
         }
         __syncwarp();                                // the K tile is multiplied: the next one takes its place
         if (more) {
@@ -815,11 +823,12 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
             next_page = page_of(key_at(c0 + 2 * STEP), next_off);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        float p[4], mx0 = -INFINITY, mx1 = -INFINITY;            // keys gq (0, 1) and gq + 8 (2, 3), heads ha and hb
+        float p[KEYS / 4], mx0 = -INFINITY, mx1 = -INFINITY;     // of every 16 keys gq (0, 1) and gq + 8 (2, 3), heads ha and hb
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            float x = ((sc[0][e] + sc[1][e]) + (sc[2][e] + sc[3][e])) * scale_log2;
-            const bool in = c0 + gq + (e < 2 ? 0 : 8) < span.n;
+        for (int e = 0; e < KEYS / 4; ++e) {
+            const float(&s4)[4][4] = sc[e / 4];
+            float x = ((s4[0][e & 3] + s4[1][e & 3]) + (s4[2][e & 3] + s4[3][e & 3])) * scale_log2;
+            const bool in = c0 + e / 4 * 16 + gq + (e & 2 ? 8 : 0) < span.n;
             if (SIG) {
                 x = in ? sigmoid2_f(x + (e & 1 ? bb : ba)) : 0.f;
             } else {
@@ -850,22 +859,30 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
                     o[n][3] *= f1;
                 }
             }
-            p[0] = b2::fast_exp2(p[0] - m0);
-            p[1] = b2::fast_exp2(p[1] - m1);
-            p[2] = b2::fast_exp2(p[2] - m0);
-            p[3] = b2::fast_exp2(p[3] - m1);
-            l0 += p[0] + p[2];
-            l1 += p[1] + p[3];
+#pragma unroll
+            for (int e = 0; e < KEYS / 4; e += 4) {
+                p[e] = b2::fast_exp2(p[e] - m0);
+                p[e + 1] = b2::fast_exp2(p[e + 1] - m1);
+                p[e + 2] = b2::fast_exp2(p[e + 2] - m0);
+                p[e + 3] = b2::fast_exp2(p[e + 3] - m1);
+                l0 += p[e] + p[e + 2];
+                l1 += p[e + 1] + p[e + 3];
+            }
         }
-        const uint32_t b0 = transpose_8x8(b2::pack_bf16x2(p[0], p[1])), b1 = transpose_8x8(b2::pack_bf16x2(p[2], p[3]));
+        uint32_t pt[KEYS / 8];
+#pragma unroll
+        for (int n = 0; n < KEYS / 8; ++n) pt[n] = transpose_8x8(b2::pack_bf16x2(p[2 * n], p[2 * n + 1]));
         asm volatile("cp.async.wait_group 1;" ::: "memory");     // V is there, the next K may still be on its way
         __syncwarp();
 #pragma unroll
         for (int n = 0; n < DVT; ++n) {
-            uint32_t a0, a1, a2, a3;
             const int key = (lane >> 4) * 8 + (lane & 7), col = n * 16 + ((lane >> 3) & 1) * 8;
-            b2::ldmatrix_x4_trans(v_base + 2u * (key * LDV + col), a0, a1, a2, a3);
-            b2::mma_bf16_16816(o[n], a0, a1, a2, a3, b0, b1);
+#pragma unroll
+            for (int ks = 0; ks < KEYS / 16; ++ks) {
+                uint32_t a0, a1, a2, a3;
+                b2::ldmatrix_x4_trans(v_base + 2u * ((ks * 16 + key) * LDV + col), a0, a1, a2, a3);
+                b2::mma_bf16_16816(o[n], a0, a1, a2, a3, pt[2 * ks], pt[2 * ks + 1]);
+            }
         }
         __syncwarp();                                // the V tile is multiplied
         if (more) issue_v();
@@ -1190,7 +1207,7 @@ chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
     }
 }
 
-template <int DVT, bool SIG, int MAPS, int NW, bool FEW>
+template <int DVT, bool SIG, int MAPS, int NW, bool FEW, int KEYS>
 int launch_heads_nw(const void* q, const void* k_cache, const void* v_cache, const int32_t* block_tables, int max_nb,
                     const int32_t* cu_q, const int32_t* ctx_start, int n_seq, int ctas, int H, int G, int dk, int bs, float scale, int chunk,
                     int window, int keep_first, float sink, float sink_logit, const float* sink_logits, const float* head_bias,
@@ -1198,11 +1215,11 @@ int launch_heads_nw(const void* q, const void* k_cache, const void* v_cache, con
                     cudaStream_t st) {
     constexpr int DV = 16 * DVT;
     constexpr int ROWS = FEW ? kFewHeads : kHeadRows;
-    const size_t tiles = (size_t)NW * kHeadKeys * (MAPS * dk + 8 + DV + 8) * sizeof(__nv_bfloat16);
+    const size_t tiles = (size_t)NW * KEYS * (MAPS * dk + 8 + DV + 8) * sizeof(__nv_bfloat16);
     const size_t merge = (size_t)NW * ROWS * (2 + DV) * sizeof(float);
     const size_t smem = (size_t)ROWS * (dk + 8) * sizeof(__nv_bfloat16) + (tiles > merge ? tiles : merge);
     auto kern = [] {
-        if constexpr (FEW) return chunk_attention_few_heads_kernel<DVT, SIG, NW>;
+        if constexpr (FEW) return chunk_attention_few_heads_kernel<DVT, SIG, NW, KEYS>;
         else return chunk_attention_heads_kernel<DVT, SIG, MAPS, NW>;
     }();
     if (smem > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1232,7 +1249,8 @@ int launch_heads(const void* q, const void* k_cache, const void* v_cache, const 
     const int64_t items = (int64_t)ctas * G;
     const int nw = items <= 148 && keys >= 512 ? 16 : items <= 296 && keys >= 256 ? 8 : 4;
 #define B2_HEADS_NW(NW, FEW)                                                                                                      \
-    return launch_heads_nw<DVT, SIG, MAPS, NW, FEW>(q, k_cache, v_cache, block_tables, max_nb, cu_q, ctx_start, n_seq, ctas, H, G, dk, bs, scale, \
+    return (FEW && dk <= kShortDk ? launch_heads_nw<DVT, SIG, MAPS, NW, FEW, FEW ? 2 * kHeadKeys : kHeadKeys>                     \
+                                  : launch_heads_nw<DVT, SIG, MAPS, NW, FEW, kHeadKeys>)(q, k_cache, v_cache, block_tables, max_nb, cu_q, ctx_start, n_seq, ctas, H, G, dk, bs, scale, \
                                                chunk, window, keep_first, sink, sink_logit, sink_logits, head_bias, gate, gate_stride, hs, \
                                                skip_from, by_seq, out, out_stride, st)
     if constexpr (MAPS == 1) {
