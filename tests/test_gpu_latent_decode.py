@@ -147,3 +147,21 @@ def test_a_sink_far_above_the_first_share(cuda, n):
     assert bool(torch.isfinite(plain).all())
     assert bool(((between.float() - plain.float()).abs() <= 2.0 ** -6 * plain.float().abs() + 1e-3).all())
     assert bool((above.float().abs() <= 1e-6).all())
+
+
+@pytest.mark.parametrize("n", [4, 150])                                  # keys split over CTAs, and not
+def test_the_error_is_the_rounding_of_the_result(cuda, n):
+    """Weights are kept to 16 bits, so what is left against fp64 is the result's own rounding to bf16: 5 % above it are allowed for the
+    fp32 sums.  (Weights of eight bits against another reference than the row's maximum: 24 % above.)"""
+    g = torch.Generator(device=cuda).manual_seed(17)
+    H, R, dr, bs, c = 16, 512, 64, 16, 1000
+    nb = c // bs + 1
+    cache = torch.randn(n * nb, bs, R + dr, generator=g, device=cuda).bfloat16()
+    tables = torch.arange(n * nb, dtype=torch.int32, device=cuda).view(n, nb)
+    qa = torch.randn(n, H, R + dr, generator=g, device=cuda).bfloat16()
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    out = ops.latent_attention(qa, cache, ops.SeqBatch(i32(list(range(n + 1))), i32([c] * n), tables, None, n, n), R, 0.1, 0).double()
+    K = cache.view(n, nb * bs, R + dr)[:, :c + 1].double()
+    ref = torch.softmax(torch.bmm(qa.double(), K.transpose(1, 2)) * 0.1, -1) @ K[:, :, :R]
+    err, rounding = float((out - ref).norm()), float((ref.bfloat16().double() - ref).norm())
+    assert err <= 1.05 * rounding, err / rounding

@@ -9,7 +9,9 @@
 // multiple of 16) by cp.async with zeros outside.
 // The softmax needs no running maximum: weights are taken against a reference m per head, the maximum of the share's first tile (and the sink), and
 // bf16 and fp32 keep their relative precision for every weight from 2^-100 to 2^60.  If a later score exceeds m by more than 60 (in
-// powers of two), the share is computed again with the maxima found.
+// powers of two), the share is computed again with the maxima found.  A weight is two bf16 numbers, its rounding and what that left
+// over, side by side in the 128 bytes of a key's row of P: with one, the largest weights, which a running maximum makes exactly one,
+// are rounded too (error against 64 bits 0.00210, 0.00206 with a running maximum, 0.0018 with both halves).
 // Bound: the bytes of the cached rows (74 KB a tile and SM).  The form on mma.sync with Q in registers waited for its own chain of
 // ldmatrix, MMA and barriers, two warps a scheduler: 64 sequences x 32 heads x 2560 keys of 576 took 120 us (140 with Q in shared memory); this one 60 (3.2 TB/s, two shares a row on 128
 // SMs: a tile's load, scores, softmax and output follow one another in each half of the ring).  An output goes before the next scores
@@ -47,13 +49,17 @@ __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, volatile int
         if (++spins > (1u << 22)) { *failed = 1; return; }
     }
 }
+// what two floats lose when they are rounded to the pair `hi` of bf16, as bf16
+__device__ __forceinline__ uint32_t left_over(float a, float b, uint32_t hi) {
+    return b2::pack_bf16x2(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+}
 // order of floats as order of ints (its own inverse)
 __device__ __forceinline__ int ordered(int bits) { return bits ^ ((bits >> 31) & 0x7fffffff); }
 
 template <int RT>                                    // R = 128 RT
 __global__ void __launch_bounds__(NTHREADS, 1)
 latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
-    constexpr int R = 128 * RT, COLS = RT == 4 ? 256 : 128;          // TMEM: S of the halves at 0 and 32, O^T at 64
+    constexpr int R = 128 * RT, COLS = RT == 4 ? 512 : RT == 2 ? 256 : 128;      // TMEM: S of the halves at 0 and 32, O^T at 64
     extern __shared__ unsigned char lat_sm_raw[];
     __shared__ __align__(8) uint64_t s_bar[9];
     __shared__ uint32_t s_tmem;
@@ -183,7 +189,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
             }
         } else if (warp == 4) {
             // ---------------------------------------------- MMA issuer
-            constexpr uint32_t ID_S = idesc_bf16(128, HEADS, 0), ID_O = idesc_bf16(128, HEADS, 1) | (1u << 15);      // O^T: A MN-major too
+            constexpr uint32_t ID_S = idesc_bf16(128, HEADS, 0), ID_O = idesc_bf16(128, 2 * HEADS, 1) | (1u << 15);  // O^T: A MN-major too
             const int ksteps = Dc / 16;
             auto scores = [&](int t) {
                 const int it = it0 + t, s = it & 1;
@@ -220,7 +226,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
                     for (int m = 0; m < RT; ++m)
 #pragma unroll
                         for (int kk = 0; kk < KT / 16; ++kk)
-                            mma_ss(tmem + 64 + 32 * m, desc_join(vl + ((m * 2 * SUB + kk * 2048) >> 4)), desc_join(pl + (kk * 2048 >> 4)), ID_O,
+                            mma_ss(tmem + 64 + 64 * m, desc_join(vl + ((m * 2 * SUB + kk * 2048) >> 4)), desc_join(pl + (kk * 2048 >> 4)), ID_O,
                                    t > 0 || kk > 0);
                     mma_commit(bar(EMPTY + s));
                     if (t + 1 == nt) mma_commit(bar(END));
@@ -259,7 +265,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
                 const bool in = j >= klo && j <= pos;
                 wait(bar(SC + s), (it >> 1) & 1, failed);
                 tc_fence_after();
-                uint32_t acc[32];
+                uint32_t acc[32], rest[16];
                 tmem_ld32(tmem + 32 * s + ((uint32_t)(warp * 32) << 16), acc);
                 tmem_wait_ld();
 #pragma unroll
@@ -283,11 +289,15 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
                     l[h + 3] += e3;
                     acc[h / 2] = b2::pack_bf16x2(e0, e1);
                     acc[h / 2 + 1] = b2::pack_bf16x2(e2, e3);
+                    rest[h / 2] = left_over(e0, e1, acc[h / 2]);
+                    rest[h / 2 + 1] = left_over(e2, e3, acc[h / 2 + 1]);
                 }
-                unsigned char* prow = gen + (p_sm - ring) + (s * KT + r) * 128;      // [key][heads], as C's sub-tiles
+                unsigned char* prow = gen + (p_sm - ring) + (s * KT + r) * 128;      // [key][heads, heads' rests], as C's sub-tiles
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
+                for (int c = 0; c < 4; ++c) {
                     *reinterpret_cast<uint4*>(prow + ((c ^ (r & 7)) << 4)) = make_uint4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+                    *reinterpret_cast<uint4*>(prow + (((4 + c) ^ (r & 7)) << 4)) = make_uint4(rest[4 * c], rest[4 * c + 1], rest[4 * c + 2], rest[4 * c + 3]);
+                }
                 b2::fence_proxy_async();
                 tc_fence_before();
                 __syncwarp();
@@ -335,16 +345,18 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
     if (warp < 4) {
 #pragma unroll 1
         for (int m = 0; m < RT; ++m) {
-            uint32_t acc[32];
-            tmem_ld32(tmem + 64 + 32 * m + ((uint32_t)(warp * 32) << 16), acc);
+            uint32_t acc[32], rest[32];
+            tmem_ld32(tmem + 64 + 64 * m + ((uint32_t)(warp * 32) << 16), acc);
+            tmem_ld32(tmem + 96 + 64 * m + ((uint32_t)(warp * 32) << 16), rest);
             tmem_wait_ld();
             const int c = 128 * m + tid;
             const size_t row = (size_t)tok * p.H + h0;
 #pragma unroll
             for (int h = 0; h < HEADS; ++h) {
                 if (h >= nh) break;
-                if (nsplit > 1) p.ws_o[((row + h) * nsplit + zs) * R + c] = __uint_as_float(acc[h]);
-                else p.out[(row + h) * R + c] = __float2bfloat16_rn(__uint_as_float(acc[h]) * s_f[h]);
+                const float v = __uint_as_float(acc[h]) + __uint_as_float(rest[h]);
+                if (nsplit > 1) p.ws_o[((row + h) * nsplit + zs) * R + c] = v;
+                else p.out[(row + h) * R + c] = __float2bfloat16_rn(v * s_f[h]);
             }
         }
     }
