@@ -894,19 +894,22 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
         l1 += __shfl_xor_sync(0xffffffffu, l1, x);
     }
     __syncthreads();                                 // every warp is done with its tiles: the partial results take their place
-    float* pa = part + (size_t)(w * kFewHeads + 2 * tq) * PW;
-    float* pb = pa + PW;
-    if (gq == 0) {
-        pa[0] = m0; pa[1] = l0;
-        pb[0] = m1; pb[1] = l1;
-    }
+    const int used = min(NW, (span.n + KEYS - 1) / KEYS);        // warps that had a tile: NW follows the width of the table, not this row
+    if (w < used) {
+        float* pa = part + (size_t)(w * kFewHeads + 2 * tq) * PW;
+        float* pb = pa + PW;
+        if (gq == 0) {
+            pa[0] = m0; pa[1] = l0;
+            pb[0] = m1; pb[1] = l1;
+        }
 #pragma unroll
-    for (int n = 0; n < DVT; ++n) {
-        const int col = 2 + n * 16 + gq;
-        pa[col] = o[n][0];
-        pb[col] = o[n][1];
-        pa[col + 8] = o[n][2];
-        pb[col + 8] = o[n][3];
+        for (int n = 0; n < DVT; ++n) {
+            const int col = 2 + n * 16 + gq;
+            pa[col] = o[n][0];
+            pb[col] = o[n][1];
+            pa[col + 8] = o[n][2];
+            pb[col + 8] = o[n][3];
+        }
     }
     __syncthreads();
     for (int h = w; h < QHall; h += NW) {            // a warp per head
@@ -916,9 +919,11 @@ chunk_attention_few_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv
 #pragma unroll
         for (int c = 0; c < DV / 32; ++c) v[c] = 0.f;
 #pragma unroll
-        for (int x = 0; x < NW; ++x) M = fmaxf(M, px[(size_t)x * kFewHeads * PW]);
+        for (int x = 0; x < NW; ++x)
+            if (x < used) M = fmaxf(M, px[(size_t)x * kFewHeads * PW]);
 #pragma unroll
         for (int x = 0; x < NW; ++x) {
+            if (x >= used) break;
             const float* pw = px + (size_t)x * kFewHeads * PW;
             const float f = SIG ? 1.f : (pw[0] == -INFINITY ? 0.f : b2::fast_exp2(pw[0] - M));
             L = fmaf(pw[1], f, L);
@@ -1157,17 +1162,20 @@ chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
             l1 += __shfl_xor_sync(0xffffffffu, l1, x);
         }
         __syncthreads();                                 // every warp is done with its tiles: the partial results take their place
-        float* pa = part + (size_t)(w * kHeadRows + gq) * PW;
-        float* pb = pa + 8 * PW;
-        if (tq == 0) {
-            pa[0] = m0; pa[1] = l0;
-            pb[0] = m1; pb[1] = l1;
-        }
+        const int used = min(NW, (span.n + kHeadKeys - 1) / kHeadKeys);  // warps that had a tile
+        if (w < used) {
+            float* pa = part + (size_t)(w * kHeadRows + gq) * PW;
+            float* pb = pa + 8 * PW;
+            if (tq == 0) {
+                pa[0] = m0; pa[1] = l0;
+                pb[0] = m1; pb[1] = l1;
+            }
 #pragma unroll
-        for (int n = 0; n < 2 * DVT; ++n) {
-            const int col = 2 + n * 8 + 2 * tq;
-            *reinterpret_cast<float2*>(pa + col) = make_float2(o[n][0], o[n][1]);
-            *reinterpret_cast<float2*>(pb + col) = make_float2(o[n][2], o[n][3]);
+            for (int n = 0; n < 2 * DVT; ++n) {
+                const int col = 2 + n * 8 + 2 * tq;
+                *reinterpret_cast<float2*>(pa + col) = make_float2(o[n][0], o[n][1]);
+                *reinterpret_cast<float2*>(pb + col) = make_float2(o[n][2], o[n][3]);
+            }
         }
         __syncthreads();
         // a warp per head: merged output of operand row r at column col
@@ -1181,16 +1189,19 @@ chunk_attention_heads_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfl
                 const float* px = part + (size_t)(h + mp * PASS) * PW;
                 float M = -INFINITY, L = 0.f;
 #pragma unroll
-                for (int x = 0; x < NW; ++x) M = fmaxf(M, px[(size_t)x * kHeadRows * PW]);
+                for (int x = 0; x < NW; ++x)
+                    if (x < used) M = fmaxf(M, px[(size_t)x * kHeadRows * PW]);
                 auto weight = [&](int x) {
                     const float mx = px[(size_t)x * kHeadRows * PW];
                     return SIG ? 1.f : (mx == -INFINITY ? 0.f : b2::fast_exp2(mx - M));
                 };
 #pragma unroll
-                for (int x = 0; x < NW; ++x) L = fmaf(px[(size_t)x * kHeadRows * PW + 1], weight(x), L);
+                for (int x = 0; x < NW; ++x)
+                    if (x < used) L = fmaf(px[(size_t)x * kHeadRows * PW + 1], weight(x), L);
                 const float inv = (SIG ? 1.f : (L > 0.f ? 1.f / L : 0.f)) * (mp == 0 ? 1.f : -hs.lambda);
 #pragma unroll
                 for (int x = 0; x < NW; ++x) {
+                    if (x >= used) break;
                     const float f = weight(x) * inv;
 #pragma unroll
                     for (int c = 0; c < DV / 32; ++c) v[c] = fmaf(px[(size_t)x * kHeadRows * PW + 2 + lane + 32 * c], f, v[c]);
