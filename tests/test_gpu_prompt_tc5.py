@@ -163,3 +163,33 @@ def test_gathered_padding_rows_are_zero(cuda):
     q, kn, kt, v = (torch.randn(*s, device=cuda).bfloat16() for s in ((40, 2, 64), (20, 2, 48), (20, 16), (20, 2, 64)))
     out = ops.window_attention(q[:, :, :48], q[:, :, 48:], kn, kt, v, i32([0, 20, 40]), i32([0, -1]), i32([0, 20, 20]), i32([0, 0]), 2, 0.1)
     assert bool((out[20:] == 0).all()) and bool(out[:20].isfinite().all()) and bool((out[:20] != 0).any())
+
+
+@pytest.mark.parametrize("cap,low", [(0.0, -30.0), (400.0, -30.0), (8.0, -100.0)])
+def test_the_largest_weight_is_exactly_one(cuda, cap, low):
+    """A key of the second tile outweighs one of the first by 2^2 to 2^7.9, all others weigh nothing: relative to the row's maximum its
+    weight is one and only the small one is rounded (2^-9 of it, at most 2^-11 of the result), so the error is the result's own
+    rounding and little more.  Against another reference both are rounded."""
+    g = torch.Generator(device=cuda).manual_seed(21)
+    n, T, G, H, d, bs, scale = 24, 300, 2, 4, 64, 16, 0.125
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    nb = -(-T // bs)
+    q, K = torch.zeros(n, T, H, d, device=cuda), torch.zeros(n, G, nb * bs, d, device=cuda)
+    V = torch.randn(n, G, nb * bs, d, generator=g, device=cuda).bfloat16()
+    q[..., 0] = 1.0 / scale
+    K[..., 0] = low
+    K[:, :, 5, 0] = 0.5
+    K[:, :, 200, 0] = 0.5 + (2.0 + 5.9 * torch.rand(n, G, generator=g, device=cuda)) * math.log(2.0)
+    q, K = q.bfloat16(), K.bfloat16()
+    pages = lambda x: x.view(n, G, nb, bs, d).transpose(1, 2).reshape(n * nb, G, bs, d).contiguous()        # noqa: E731
+    batch = ops.SeqBatch(i32([T * i for i in range(n + 1)]), i32([0] * n), torch.arange(n * nb, dtype=torch.int32, device=cuda).view(n, nb), None, n, n * T)
+    out = ops.chunk_attention(q.view(n * T, H, d), pages(K), pages(V), batch, scale, softcap=cap).view(n, T, H, d)[:, 200:].double()
+    s = K[:, :, :201, 0].double()                                        # every row's score of key j
+    s = (cap * torch.tanh(s / cap) if cap else s)[:, :, None].expand(-1, -1, T - 200, -1)
+    own = torch.full((n, G, T - 200, nb * bs), float(low), device=cuda, dtype=torch.float64)
+    own = cap * torch.tanh(own / cap) if cap else own
+    own[..., :201] = s
+    own = own.masked_fill(torch.arange(nb * bs, device=cuda)[None] > torch.arange(200, T, device=cuda)[:, None], -math.inf)
+    ref = (torch.softmax(own, -1) @ V.double()).repeat_interleave(H // G, 1).transpose(1, 2)
+    err, rounding = float((out - ref).norm()), float((ref.bfloat16().double() - ref).norm())
+    assert err <= 1.1 * rounding, err / rounding

@@ -14,16 +14,18 @@
 // per key row, written in the 128-byte swizzle that the MMA descriptors name (gathered rows: TMA boxes).  A mask is tested per
 // score only in tiles that the slot's rows see in part.
 // S = Q K^T and O += P V are tcgen05.mma 128x128x16 (bf16 -> fp32 in TMEM); P replaces S in TMEM and is the A operand of the
-// second product; the online softmax rescales O lazily (a row keeps its maximum until the true one exceeds it by 2^8).
+// second product.  The online softmax takes a row's weights against its maximum so far, whatever that costs in rescales of O: the largest
+// weight is exactly one then and loses nothing in bf16.  (A row that kept its maximum until the true one exceeded it by 2^8 saved 7 us of
+// 124 at 4096 capped rows, and its error against 64 bits was 0.0029 instead of 0.0028.)
 //
 // Bound: tensor pipe (2 (dk + dv) flops per visible pair) and, for the exponentials, the XU pipe, 16 a clock and SM.  A capped
 // score would need two more XU operations (the exponential and the division of tanh): where a whole warp's scores are below 3/16
 // of the cap, tanh is its Taylor polynomial to x^7 on the packed FMA pipe instead (remainder below 7e-9; the exponential form's
-// error is one fp32 rounding, 6e-8), and the bound max|s| takes the place of the row's maximum.
+// error is one fp32 rounding, 6e-8).
 // Measured (clock64, 128 keys x two slots): 3.3k cycles with heads of 192 / 128, of which the tensor pipe is busy 2.6k; 4.8k with
 // capped scores (the packed polynomial and the exponentials of both slots share the issue slots).
-//   4096 rows x 16 heads of 128 + 64 / 128, causal: 270 us (mma.sync, 64-row tiles) -> 59 us
-//   4096 rows x 32 heads of 128, window 1024, capped: 460 us (mma.sync) -> 110 us
+//   4096 rows x 16 heads of 128 + 64 / 128, causal: 648 us (mma.sync, 64-row tiles) -> 78 us, in a graph
+//   4096 rows x 32 heads of 128, window 1024, capped: 461 us (mma.sync) -> 124 us; causal, not capped 877 -> 152 us
 // What cost most on the way: code size (95 - 145 KB with everything unrolled: every warp waited for instructions, 10.9k cycles per
 // tile; loops are rolled wherever registers are not indexed), and a divergent branch per row in the copies (~100 cycles an
 // instruction, serialised; zero-filling copies need none).
@@ -37,7 +39,6 @@ using namespace b2tc;
 constexpr int BM = 128, BN = 128, NTHREADS = 384;
 constexpr int SUB = 128 * 128;                       // bytes of a [128 rows][64 el] sub-tile
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr float RESCALE_THRESHOLD = 8.f;             // log2 units
 constexpr float FLOOR = -1e30f;                      // a row that has seen no key yet: exp2(-inf - FLOOR) = 0, not NaN
 enum { KIND_SOFTMAX = 0, KIND_CAPPED = 1, KIND_SIGMOID = 2 };
 
@@ -450,7 +451,6 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                 auto reduce = [&]() {
                     return fmaxf(fmaxf(fmaxf(mp[0], mp[1]), fmaxf(mp[2], mp[3])), fmaxf(fmaxf(mp[4], mp[5]), fmaxf(mp[6], mp[7])));
                 };
-                float mx = -INFINITY;
                 bool small = false;
                 uint32_t see[4] = {~0u, ~0u, ~0u, ~0u};
                 if (KIND == KIND_CAPPED) {
@@ -459,13 +459,12 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
 #pragma unroll
                         for (int k = 0; k < 32; ++k) mp[k & 7] = fmaxf(mp[k & 7], fabsf(__uint_as_float(sr[c][k])));
                     const float am = reduce();
-                    small = __all_sync(0xffffffffu, cx > 0.f && am * cx <= 0.1875f && am * eff <= 30.f);
+                    small = __all_sync(0xffffffffu, cx > 0.f && am * cx <= 0.1875f);
                     if (small) {
 #pragma unroll
                         for (int c = 0; c < 4; ++c)
 #pragma unroll
                             for (int k = 0; k < 32; k += 2) tanh_small_x2(sr[c][k], sr[c][k + 1], a1, a2, a3);
-                        mx = am * eff;                               // no score of the row is above it, none 2^60 below
                     } else {                                         // any score, any scale: through TMEM, a rolled loop
                         eff = 1.f;
 #pragma unroll 1
@@ -500,26 +499,18 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                     }
                 }
                 if (KIND != KIND_SIGMOID) {
-                    if (!small) {
 #pragma unroll
-                        for (int k = 0; k < 8; ++k) mp[k] = -INFINITY;
+                    for (int k = 0; k < 8; ++k) mp[k] = -INFINITY;
 #pragma unroll
-                        for (int c = 0; c < 4; ++c)
+                    for (int c = 0; c < 4; ++c)
 #pragma unroll
-                            for (int k = 0; k < 32; ++k) mp[k & 7] = fmaxf(mp[k & 7], __uint_as_float(sr[c][k]));
-                        mx = reduce() * eff;
-                    }
-                    const float m_new = fmaxf(fmaxf(m, mx), FLOOR);
-                    if (i == 0) {
-                        l *= b2::fast_exp2(m - m_new);               // the sink's share, if any; exp2(-inf) = 0
-                        m = m_new;
-                    } else {
-                        const bool need = m_new - m > RESCALE_THRESHOLD;
-                        if (__any_sync(0xffffffffu, need)) {         // rare after the first tiles
+                        for (int k = 0; k < 32; ++k) mp[k & 7] = fmaxf(mp[k & 7], __uint_as_float(sr[c][k]));
+                    const float m_new = fmaxf(fmaxf(m, reduce() * eff), FLOOR), alpha = b2::fast_exp2(m - m_new);
+                    l *= alpha;                                      // at first the sink's share, if any; exp2(-inf) = 0
+                    if (i > 0) {
+                        if (__any_sync(0xffffffffu, m_new > m)) {    // else every factor is one
                             wait(bar(L::BAR_PV + x), (i - 1) & 1, failed);
                             tc_fence_after();
-                            const float alpha = need ? b2::fast_exp2(m - m_new) : 1.f;
-                            if (need) { m = m_new; l *= alpha; }
 #pragma unroll 1
                             for (int c = 0; c < 2 * DVH; ++c) {
                                 uint32_t o[32];
@@ -531,6 +522,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                             }
                         }
                     }
+                    m = m_new;
                 }
                 float sum[4] = {0.f, 0.f, 0.f, 0.f};                 // the denominator sums the fp32 weights
 #pragma unroll
