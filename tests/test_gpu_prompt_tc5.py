@@ -53,6 +53,8 @@ CASES = [
     ([400, 64], [0, 9], 4, 2, 128, 64, 16, 0, 150, 0, 0.0, False, 1, True, True, 1.0),
     ([1300], [0], 16, 16, 96, 96, 16, 0, 0, 0, 0.0, False, 1, True, False, 1.0),                         # two row tiles a CTA
     ([130], [64], 2, 1, 128, 128, 16, 0, 0, 0, 0.0, True, 1, False, False, -1.0),
+    ([1] * 40 + [200] + [15] * 20 + [16] + [3] * 9 + [130, 2], [30] * 73, 8, 4, 64, 64, 16, 0, 64, 2, 0.0, True, 1, False, False, 1.0),
+    ([0, 0, 40] + [0] * 60 + [16, 0, 17] + [0] * 20, [3] * 86, 2, 2, 32, 32, 16, 0, 0, 0, 0.0, False, 1, False, False, 1.0),      # most are empty
 ]
 
 
@@ -163,6 +165,23 @@ def test_gathered_padding_rows_are_zero(cuda):
     q, kn, kt, v = (torch.randn(*s, device=cuda).bfloat16() for s in ((40, 2, 64), (20, 2, 48), (20, 16), (20, 2, 64)))
     out = ops.window_attention(q[:, :, :48], q[:, :, 48:], kn, kt, v, i32([0, 20, 40]), i32([0, -1]), i32([0, 20, 20]), i32([0, 0]), 2, 0.1)
     assert bool((out[20:] == 0).all()) and bool(out[:20].isfinite().all()) and bool((out[:20] != 0).any())
+
+
+def test_more_row_tiles_than_a_grid_dimension_holds(cuda):
+    """70000 portions of 16 rows: above the 65535 blocks of a grid's second dimension."""
+    g = torch.Generator(device=cuda).manual_seed(3)
+    n, m, d = 70000, 16, 32
+    rnd = lambda *s: torch.randn(*s, generator=g, device=cuda).bfloat16()        # noqa: E731
+    q, kc, vc = rnd(n * m, 1, d), rnd(n, 1, m, d), rnd(n, 1, m, d)
+    tables = torch.randperm(n, generator=g, device=cuda).to(torch.int32).view(n, 1)
+    cu = torch.arange(n + 1, dtype=torch.int32, device=cuda) * m
+    batch = ops.SeqBatch(cu, torch.zeros(n, dtype=torch.int32, device=cuda), tables, None, n, n * m)
+    out = ops.chunk_attention(q, kc, vc, batch, d ** -0.5).view(n, m, d).double()
+    K, V = kc[tables[:, 0].long(), 0].double(), vc[tables[:, 0].long(), 0].double()
+    s = torch.bmm(q.view(n, m, d).double(), K.transpose(1, 2)) * d ** -0.5
+    w = torch.softmax(s.masked_fill(~torch.ones(m, m, dtype=torch.bool, device=cuda).tril(), -math.inf), -1)
+    ref, spr = torch.bmm(w, V), torch.bmm(w, V.abs())
+    assert bool(((out - ref).abs() <= 2.0 ** -8 * (spr + ref.abs()) + 1e-6).all())
 
 
 @pytest.mark.parametrize("cap,low", [(0.0, -30.0), (400.0, -30.0), (8.0, -100.0)])

@@ -32,6 +32,8 @@
 #include "b2_mask.cuh"
 #include "b2_tc5.cuh"
 
+#include <algorithm>
+
 namespace {
 
 using namespace b2tc;
@@ -117,7 +119,6 @@ __device__ __forceinline__ RowRange range_of(const KeySpan& span, int i, int chu
 }
 // what one thread works out for the CTA
 struct Plan {
-    int seq, q0, len, ctx, row0;
     KeySpan span;
     int keep;                                        // compact index below which keys are kept for every row of their mask block
     int first_row[2], rows[2];                       // position of a slot's first row, number of rows
@@ -143,36 +144,53 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
     auto bar = [&](int i) { return bars + 8u * i; };
     volatile int* failed = &s_failed;
 
+    // This CTA's tile: counted from the batch's last row backwards (late rows see more keys, and the spare CTAs of a grid that is an
+    // upper bound come behind all tiles), by every warp for itself, 32 sequences at a time, so that a spare CTA leaves at once.
+    const int groups = a.H / prm.heads_per_cta, group = blockIdx.x % groups;
+    int seq = -1, q0 = 0, len = 0;
+    {
+        int want = blockIdx.x / groups;
+#pragma unroll 1
+        for (int top = a.n_seq - 1; top >= 0; top -= 32) {
+            const int s = top - lane, n = s >= 0 ? a.cu_q[s + 1] - a.cu_q[s] : 0;
+            const int nt = n >= a.min_rows ? (n + prm.rows_per_cta - 1) / prm.rows_per_cta : 0;
+            int upto = nt;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, d);
+                if (lane >= d) upto += below;
+            }
+            const uint32_t hit = __ballot_sync(0xffffffffu, want < upto);
+            if (hit) {
+                const int who = __ffs(hit) - 1;
+                seq = top - who;
+                len = __shfl_sync(0xffffffffu, n, who);
+                q0 = (__shfl_sync(0xffffffffu, upto, who) - 1 - want) * prm.rows_per_cta;
+                break;
+            }
+            want -= __shfl_sync(0xffffffffu, upto, 31);
+        }
+    }
+    if (seq < 0) return;
+    const int ctx = a.ctx_start[seq], row0 = a.cu_q[seq] + q0;
+    if (ctx < 0) {                                                   // padding: zero rows (the paged form's are another kernel's)
+        const int rows = GATHERED ? min(len - q0, prm.rows_per_cta) : 0, v8 = a.dv / 8;
+        for (int idx = tid; idx < rows * v8; idx += NTHREADS)
+            *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + (size_t)(row0 + idx / v8) * a.out_stride + (size_t)group * a.dv + (idx % v8) * 8) =
+                make_uint4(0, 0, 0, 0);
+        return;
+    }
+
     if (tid == 0) {
         s_failed = 0;
         Plan& pl = s_plan;
-        int want = (int)(gridDim.y - 1 - blockIdx.y), q0 = 0;        // late rows, which see more keys, first
-        pl.seq = -1;
-        pl.ctx = -1;
-        pl.row0 = 0;
-        pl.span.n = 0;
-        for (int s = 0; s < a.n_seq; ++s) {
-            const int len = a.cu_q[s + 1] - a.cu_q[s];
-            if (len < a.min_rows) continue;
-            const int nt = (len + prm.rows_per_cta - 1) / prm.rows_per_cta;
-            if (want < nt) {
-                q0 = want * prm.rows_per_cta;
-                pl.seq = s;
-                pl.len = len;
-                pl.ctx = a.ctx_start[s];
-                pl.row0 = a.cu_q[s] + q0;
-                break;
-            }
-            want -= nt;
-        }
-        pl.q0 = q0;
         pl.rows[0] = pl.rows[1] = pl.t0[0] = pl.t0[1] = pl.t1[0] = pl.t1[1] = 0;
-        if (pl.seq >= 0 && pl.ctx >= 0) {
-            const int left = pl.len - q0, p0 = pl.ctx + q0, p_last = p0 + min(left, prm.rows_per_cta) - 1;
+        {
+            const int left = len - q0, p0 = ctx + q0, p_last = p0 + min(left, prm.rows_per_cta) - 1;
             const bool two = prm.rows_per_cta > BM;
             KeySpan span = key_span(p0, p_last, a.chunk, a.window, a.keep_first);
-            if (GATHERED && span.wlo < a.k_lo[pl.seq]) {             // the gathered rows begin at k_lo
-                span.wlo = span.lo = a.k_lo[pl.seq];
+            if (GATHERED && span.wlo < a.k_lo[seq]) {                // the gathered rows begin at k_lo
+                span.wlo = span.lo = a.k_lo[seq];
                 span.n = p_last - span.lo + 1;
             }
             pl.span = span;
@@ -211,23 +229,14 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    const int seq = s_plan.seq, row0 = s_plan.row0;
-    const bool active = seq >= 0 && s_plan.ctx >= 0;                 // CTA-uniform
     const int hpc = prm.heads_per_cta;
     const bool two_rows = prm.rows_per_cta > BM;
     const int n_tiles = max(s_plan.t1[0], s_plan.t1[1]), n_keys = s_plan.span.n;
-    const int kvh = (blockIdx.x * hpc) / (a.H / a.G);                // kv head of the paged pools
-
-    if (GATHERED && seq >= 0 && !active) {                           // padding: zero rows (the paged form's are another kernel's)
-        const int rows = min(s_plan.len - s_plan.q0, prm.rows_per_cta), v8 = a.dv / 8, hh = blockIdx.x;
-        for (int idx = tid; idx < rows * v8; idx += NTHREADS)
-            *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + (size_t)(row0 + idx / v8) * a.out_stride + (size_t)hh * a.dv + (idx % v8) * 8) =
-                make_uint4(0, 0, 0, 0);
-    }
+    const int kvh = (group * hpc) / (a.H / a.G);                // kv head of the paged pools
 
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-        if (active && warp != 9) {
+        if (warp != 9) {
             // ------------------------------------------ copies: warps 8 and 11 the even and odd groups of K rows, warp 10 V
             // Eight lanes copy the 128 bytes of a row and sub-tile, four rows (a group) an instruction.  The pool rows of a tile's
             // 128 keys (four a lane, through the page table) are looked up before the stage is free: a lookup in front of its
@@ -263,7 +272,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             {                                                        // Q, by all three warps: rows past the tile are zeros
 #pragma unroll 1
                 for (int x = 0; x < 2; ++x) {
-                    const int hh = blockIdx.x * hpc + (hpc == 2 ? x : 0), nrows = s_plan.rows[x];
+                    const int hh = group * hpc + (hpc == 2 ? x : 0), nrows = s_plan.rows[x];
                     const int rbase = row0 + (two_rows && x ? BM : 0);
                     if (nrows == 0) continue;
                     const int col0 = TWO_MAPS ? x * a.dk : 0;
@@ -289,7 +298,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             const int nst = is_v ? L::VST : L::KST;
             const int n_sub = is_v ? DVH : L::KSUBS, width = is_v ? a.dv : a.dk, split = GATHERED && !is_v ? a.dk0 : width;
             const uint32_t ld = 2u * (uint32_t)(GATHERED ? a.H * split : width), ld1 = 2u * (uint32_t)a.k1_row;    // bytes between pool rows
-            const char* p0 = reinterpret_cast<const char*>(static_cast<const bf16*>(is_v ? a.v : a.k0) + (GATHERED ? (size_t)blockIdx.x * split : 0) + c8 * 8);
+            const char* p0 = reinterpret_cast<const char*>(static_cast<const bf16*>(is_v ? a.v : a.k0) + (GATHERED ? (size_t)group * split : 0) + c8 * 8);
             const char* p1 = GATHERED && !is_v ? reinterpret_cast<const char*>(static_cast<const bf16*>(a.k1) + c8 * 8) - 2 * split : p0;
             const uint32_t map2 = 2u * (uint32_t)a.bs * (uint32_t)a.dk;                  // the second map's rows lie a page of the first behind
 #pragma unroll 1
@@ -301,7 +310,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                 const bool whole = GATHERED && prm.tma && (it + 1) * BN <= n_keys;      // all 128 rows are this sequence's
                 if (whole && !odd) {
                     if (lane == 0) {
-                        const int row = (int)g0 + span.wlo + it * BN, hh = blockIdx.x;
+                        const int row = (int)g0 + span.wlo + it * BN, hh = group;
                         b2::mbar_arrive_expect_tx(full, (uint32_t)n_sub * SUB);          // columns past the head are zero-filled and count
 #pragma unroll 1
                         for (int h = 0; h < n_sub; ++h) {
@@ -352,7 +361,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                 __syncwarp();
                 if (lane == 0 && !(whole && !odd)) b2::mbar_arrive(full);
             }
-        } else if (active && warp == 9) {
+        } else {
             // ------------------------------------------ MMA issuer: the whole warp, warp-uniform operands, one elected lane
             // step j: P_0 V(j), Q_0 K(j+1), P_1 V(j), Q_1 K(j+1) -- the softmax of one slot runs under the MMAs of the other
             constexpr uint32_t ID_QK = idesc_bf16(128, 128, 0), ID_PV = idesc_bf16(128, 64 * DVH, 1);
@@ -427,7 +436,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             const int row = wq * 32 + lane;                          // query row of the slot = TMEM lane
             const uint32_t lane_off = (uint32_t)(wq * 32) << 16;
             const uint32_t s_addr = tmem + lane_off + x * 128, o_addr = tmem + lane_off + 256 + x * 128;
-            const int hh = blockIdx.x * hpc + (hpc == 2 ? x : 0);
+            const int hh = group * hpc + (hpc == 2 ? x : 0);
             const RowRange mine = range_of(s_plan.span, s_plan.first_row[x] + min(row, nrows - 1), a.chunk, a.window);
             const int all_hi = s_plan.all_hi[x], all_low = s_plan.all_low[x], keep = s_plan.keep;
             const float sl2 = prm.scale_log2;
@@ -702,7 +711,8 @@ int b2_internal_prompt_tc5(const b2_prompt_args& a, void* stream) {
     }
     // Two slots a CTA share the copies of a key tile and cover each other's softmax; a launch of fewer than one wave of such CTAs
     // takes one slot each (twice the CTAs, each a little faster).  Two heads of a kv head before two row tiles: see above.
-    const int64_t tiles128 = (int64_t)a.T / BM + a.n_seq, tiles256 = (int64_t)a.T / (2 * BM) + a.n_seq;
+    const int64_t longs = std::min(a.n_seq, a.T / a.min_rows);       // sequences of min_rows rows or more
+    const int64_t tiles128 = (int64_t)a.T / BM + longs, tiles256 = (int64_t)a.T / (2 * BM) + longs;
     p.rows_per_cta = BM;
     p.heads_per_cta = 1;
     if (a.maps == 1) {
@@ -711,8 +721,10 @@ int b2_internal_prompt_tc5(const b2_prompt_args& a, void* stream) {
         else if (!pair && tiles256 * a.H >= n_sm) p.rows_per_cta = 2 * BM;
     }
     const int64_t tiles = p.rows_per_cta == BM ? tiles128 : tiles256;        // upper bound on sum(ceil(len / rows)); spare CTAs leave at once
-    B2_REQUIRE(tiles <= 65535, B2_EUNSUPPORTED, "prompt attention: %lld row tiles exceed the grid", (long long)tiles);
-    const dim3 grid((unsigned)(a.H / p.heads_per_cta), (unsigned)tiles);
+    if (tiles == 0) return B2_OK;
+    const int64_t ctas = tiles * (a.H / p.heads_per_cta);
+    B2_REQUIRE(ctas <= 0x7fffffff, B2_EUNSUPPORTED, "prompt attention: %lld row tiles exceed the grid", (long long)tiles);
+    const dim3 grid((unsigned)ctas);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nh = (a.dk + 63) / 64, dvh = (a.dv + 63) / 64;
     const bool one_by_one = a.cap > 0.f || !(a.scale > 0.f);         // the capped form takes any score and any sign of the scale
