@@ -1,6 +1,6 @@
 // b2_tc5.cuh -- tcgen05 / TMEM wrappers and the packed fp32 pipe, shared by the attention kernels on the 5th-gen tensor cores.
 #pragma once
-#include <stdint.h>
+#include "b2_common.cuh"
 
 #ifdef __CUDACC__
 namespace b2tc {
@@ -36,6 +36,30 @@ __device__ __forceinline__ uint64_t desc_join(uint32_t lo) {           // SBO = 
 }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {       // arrives on `bar` when all MMAs issued so far are done
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// A wait that gives up after some seconds (false): it raises the CTA's flag, every later wait returns at once, the kernel issues no more
+// copies, runs to its end on whatever the buffers hold and writes NaN: a fault of the protocol ends in an error and not in a hang.
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity, volatile int* failed) {
+    uint32_t spins = 0;
+#pragma unroll 1
+    while (!b2::mbar_try_wait(bar, parity)) {
+        if (*failed) return false;
+        if (++spins > (1u << 22)) { *failed = 1; return false; }
+    }
+    return true;
+}
+// After a wait has given up: shared memory and TMEM must not go while copies or MMAs are on their way to them.  Polls the phase they
+// complete for a millisecond at most, which is longer than any of them takes, in case it lacks an arrival and never ends.
+__device__ __forceinline__ void drain(uint32_t bar, uint32_t parity) {
+    for (int spins = 0; spins < 4096 && !b2::mbar_try_wait(bar, parity); ++spins) __nanosleep(256);
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
 }
 __device__ __forceinline__ bool elect_one() {                   // true in exactly one lane of the (converged) warp
     uint32_t pred;

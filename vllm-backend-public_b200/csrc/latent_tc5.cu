@@ -40,15 +40,6 @@ struct LatentArgs {
     float *ws_o, *ws_ml;
 };
 
-// gives up after some seconds; the CTA then runs to its end and writes NaN
-__device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, volatile int* failed) {
-    uint32_t spins = 0;
-#pragma unroll 1
-    while (!b2::mbar_try_wait(bar, parity)) {
-        if (*failed) return;
-        if (++spins > (1u << 22)) { *failed = 1; return; }
-    }
-}
 // what two floats lose when they are rounded to the pair `hi` of bf16, as bf16
 __device__ __forceinline__ uint32_t left_over(float a, float b, uint32_t hi) {
     return b2::pack_bf16x2(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
@@ -148,7 +139,10 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
             for (int t = 0; t < nt; ++t) {
                 const int it = it0 + t, s = it & 1, kv0 = kbase + (t0 + t) * KT;
                 const uint32_t base = ring + s * (KT * 128), full = bar(FULL + s);
-                if (it >= 2) wait(bar(EMPTY + s), ((it >> 1) - 1) & 1, failed);
+                if (it >= 2 && !__all_sync(0xffffffffu, wait(bar(EMPTY + s), ((it >> 1) - 1) & 1, failed))) {
+                    for (int back = 1; lane == 0 && back <= 2; ++back) drain(bar(FULL + ((it - back) & 1)), ((it - back) >> 1) & 1);
+                    break;
+                }
                 if (whole(t)) {
                     if (cw == 0) {
                         if (lane == 0) b2::mbar_arrive_expect_tx(full, (uint32_t)NS * KT * 128);      // columns past Dc are zero-filled and count
@@ -156,9 +150,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
 #pragma unroll
                         for (int u = 0; u < 2; ++u) {
                             const int idx = lane + 32 * u, sub = idx % NS, pg = idx / NS;
-                            if (idx < 4 * NS)
-                                asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                                             ::"r"(base + sub * SUB + pg * 2048), "l"(&p.map), "r"(full), "r"(sub * 64), "r"(u ? row_b : row_a) : "memory");
+                            if (idx < 4 * NS) tma_load_2d(base + sub * SUB + pg * 2048, &p.map, full, sub * 64, u ? row_b : row_a);
                         }
                         __syncwarp();
                     } else if (lane == 0) {
@@ -234,7 +226,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
                 __syncwarp();
                 if (ahead) scores(t + 1);
             }
-            wait(bar(END), pass, failed);
+            if (!wait(bar(END), pass, failed)) drain(bar(END), pass);
         } else {
             // ---------------------------------------------- softmax: lane = key; warps 0, 1 the first half of the ring, 2, 3 the second
             float mx[HEADS];
@@ -360,8 +352,6 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
             }
         }
     }
-    if (s_failed && tid < 2)                         // copies still in flight end before the shared memory goes
-        for (uint32_t spins = 0; spins < (1u << 20) && !b2::mbar_try_wait(bar(FULL + tid), 0) && !b2::mbar_try_wait(bar(FULL + tid), 1); ++spins) {}
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

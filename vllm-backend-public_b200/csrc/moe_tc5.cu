@@ -29,21 +29,6 @@ struct ExpertArgs {
     float alpha, limit;
 };
 
-// gives up after some seconds; the CTA then runs to its end and writes NaN
-__device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, volatile int* failed) {
-    uint32_t spins = 0;
-#pragma unroll 1
-    while (!b2::mbar_try_wait(bar, parity)) {
-        if (*failed) return;
-        if (++spins > (1u << 22)) { *failed = 1; return; }
-    }
-}
-
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
-}
-
 enum { PAIR, SINGLE, DOWN };                         // glu of two products; relu^2 of one; one product in fp32
 
 template <int KIND, int ST>
@@ -86,7 +71,10 @@ moe_tc5_kernel(const __grid_constant__ ExpertArgs p) {
 #pragma unroll 1
             for (int it = 0; it < nk; ++it) {
                 const int s = it % ST;
-                if (it >= ST) wait(empty(s), (it / ST - 1) & 1, failed);
+                if (it >= ST && !wait(empty(s), (it / ST - 1) & 1, failed)) {
+                    for (int back = 1; back <= ST; ++back) drain(full((it - back) % ST), ((it - back) / ST) & 1);
+                    break;
+                }
                 b2::mbar_arrive_expect_tx(full(s), W_STAGE);         // columns and rows past the matrix are zero-filled and count
                 tma_load_3d(sm + s * W_STAGE, &p.map0, full(s), it * KSTEP, n0, e);
                 tma_load_3d(sm + s * W_STAGE + W_STAGE / 2, &p.map1, full(s), it * KSTEP, KIND == PAIR ? n0 : n0 + 64, e);
@@ -179,10 +167,7 @@ moe_tc5_kernel(const __grid_constant__ ExpertArgs p) {
             b2::st(static_cast<bf16*>(p.out) + (size_t)(m0 + r) * p.N + n0 + c, bad ? __int_as_float(0x7fc00000) : v);
         }
     }
-    if (bad && tid < ST && tid < nk) {               // copies still in flight end before the shared memory goes
-        const int last = (nk - 1 - tid) / ST;
-        for (uint32_t spins = 0; spins < (1u << 20) && !b2::mbar_try_wait(full(tid), last & 1); ++spins) {}
-    }
+    if (bad) drain(b2::smem_u32(&s_end), 0);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();

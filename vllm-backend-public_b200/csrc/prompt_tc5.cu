@@ -65,30 +65,10 @@ struct Params {
     CUtensorMap map_k0, map_k1, map_v;
 };
 
-// A wait that gives up after some seconds: it raises the CTA's flag, every later wait returns at once, the kernel runs to its end on
-// whatever the buffers hold and writes NaN, so that a fault of the protocol ends in an error and not in a hang.
-__device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, volatile int* failed) {
-    uint32_t spins = 0;
-#pragma unroll 1
-    while (!b2::mbar_try_wait(bar, parity)) {
-        if (*failed) return;
-        if (++spins > (1u << 22)) { *failed = 1; return; }
-    }
-}
-
 // 16 bytes, or zeros without reading `src` (no branch: a divergent one would serialise the copies of a warp)
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool ok) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
-}
-
 // (s0, s1) (1 + z a1 + z^2 a2 + z^3 a3), z = s^2, on the packed pipe: s tanh(x) / x of a score s = x / c, a_i = t_i c^2i with the
 // Taylor coefficients -1/3, 2/15, -17/315
 __device__ __forceinline__ void tanh_small_x2(uint32_t& s0, uint32_t& s1, float a1, float a2, float a3) {
@@ -304,7 +284,11 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
 #pragma unroll 1
             for (int it = 0; it < n_tiles; ++it) {
                 const int s = it % nst, ph = (it / nst) & 1;
-                wait(bar((is_v ? L::BAR_VE : L::BAR_KE) + s), ph ^ 1, failed);
+                if (!__all_sync(0xffffffffu, wait(bar((is_v ? L::BAR_VE : L::BAR_KE) + s), ph ^ 1, failed))) {
+                    for (int back = 1; GATHERED && lane == 0 && back <= min(nst, it); ++back)
+                        drain(bar((is_v ? L::BAR_V : L::BAR_K) + (it - back) % nst), ((it - back) / nst) & 1);
+                    break;
+                }
                 const uint32_t base = is_v ? v_ring + s * L::V_STAGE : k_ring + s * L::K_STAGE;
                 const uint32_t full = bar((is_v ? L::BAR_V : L::BAR_K) + s);
                 const bool whole = GATHERED && prm.tma && (it + 1) * BN <= n_keys;      // all 128 rows are this sequence's
@@ -425,7 +409,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             }
             if (elect_one()) mma_commit(bar(L::BAR_END));            // nothing in flight when the TMEM is given back
             __syncwarp();
-            wait(bar(L::BAR_END), 0, failed);
+            if (!wait(bar(L::BAR_END), 0, failed)) drain(bar(L::BAR_END), 0);
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
@@ -564,12 +548,12 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                 if (KIND != KIND_SIGMOID) l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
             }
             // ------------------------------------------ output rows
-            float inv = KIND == KIND_SIGMOID ? 1.f : (l > 0.f ? 1.f / l : 0.f);
-            if (*failed) inv = __int_as_float(0x7fc00000);
             const int n = te - tb;
             const bool valid = row < nrows;
             const size_t brow = (size_t)row0 + (two_rows && x ? BM : 0) + row;
             wait(bar(L::BAR_PV + x), (n - 1) & 1, failed);
+            float inv = KIND == KIND_SIGMOID ? 1.f : (l > 0.f ? 1.f / l : 0.f);
+            if (*failed) inv = __int_as_float(0x7fc00000);           // behind the last wait, which may be the one that gave up
             if (TWO_MAPS && x == 1) {                                // slot 0 writes: it reads both outputs from its own TMEM lane
                 s_inv[TWO_MAPS ? row : 0] = inv;
                 tc_fence_after();
