@@ -20,7 +20,9 @@
 // heads of 128.  The scan token by token waited 200 - 400 cycles a token for shuffles and shared memory whatever the shape.
 #include "b2_act.cuh"
 
+#include <float.h>
 #include <math.h>
+#include <type_traits>
 
 namespace {
 
@@ -587,6 +589,7 @@ chunk_delta_kernel(const ChunkArgs a, int stages) {
         }
         __syncthreads();
         const int t = tid >> 2, x4 = (tid & 3) * 4;  // the small matrices: four columns of a row a thread
+        bool bad;
         {
             const float f = CH ? 1.f : de[t];
             const float4 v = *reinterpret_cast<const float4*>(vs + t * NC + x4);
@@ -596,35 +599,39 @@ chunk_delta_kernel(const ChunkArgs a, int stages) {
                 const float4 y = *reinterpret_cast<const float4*>(redA + (q * C + t) * NC + x4);
                 p = make_float4(p.x + y.x, p.y + y.y, p.z + y.z, p.w + y.w);
             }
-            *reinterpret_cast<float4*>(Rm + t * NC + x4) = make_float4(fmaf(-f, p.x, v.x), fmaf(-f, p.y, v.y), fmaf(-f, p.z, v.z), fmaf(-f, p.w, v.w));
+            p = make_float4(fmaf(-f, p.x, v.x), fmaf(-f, p.y, v.y), fmaf(-f, p.z, v.z), fmaf(-f, p.w, v.w));
+            *reinterpret_cast<float4*>(Rm + t * NC + x4) = p;
+            bad = !(fabsf(p.x) + fabsf(p.y) + fabsf(p.z) + fabsf(p.w) <= FLT_MAX);
         }
-        __syncthreads();
-        {   // T R, nothing above the diagonal; columns 16 it + 4 kq of T
+        bad = __syncthreads_or(bad);                 // only then T's zeros above the diagonal have to be left out
+        {   // T R, columns 16 it + 4 kq of T
             pair_t acc[4][2];
 #pragma unroll
             for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0;
-            for (int it = 0; it < (half == 0 ? 2 : 4); ++it) {
-                const int s0 = it * 16 + kq * 4;
-                float4 x[4];
-                ulonglong2 y[4];
+            auto product = [&](auto select) {
+                for (int it = 0; it < (half == 0 ? 2 : 4); ++it) {
+                    const int s0 = it * 16 + kq * 4;
+                    float4 x[4];
+                    ulonglong2 y[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(ts + (half * 32 + rg + 8 * r) * LP + s0);
+                    for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(ts + (half * 32 + rg + 8 * r) * LP + s0);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) y[q] = pairs(Rm + (s0 + q) * NC + cg * 4);
+                    for (int q = 0; q < 4; ++q) y[q] = pairs(Rm + (s0 + q) * NC + cg * 4);
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float xv[4] = {x[r].x, x[r].y, x[r].z, x[r].w};
-                    const int last = half * 32 + rg + 8 * r - s0;    // of the four columns, those up to the row's own
+                    for (int r = 0; r < 4; ++r) {
+                        const float xv[4] = {x[r].x, x[r].y, x[r].z, x[r].w};
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        if (q <= last) {
+                        for (int q = 0; q < 4; ++q) {
+                            if (decltype(select)::value && s0 + q > half * 32 + rg + 8 * r) continue;
                             const pair_t xx = dup(xv[q]);
                             fma2(acc[r][0], xx, y[q].x);
                             fma2(acc[r][1], xx, y[q].y);
                         }
                     }
                 }
-            }
+            };
+            if (bad) product(std::true_type());
+            else product(std::false_type());
             float* dst = redB + (kq * C + half * 32 + rg) * NC + cg * 4;
 #pragma unroll
             for (int r = 0; r < 4; ++r) *reinterpret_cast<float4*>(dst + r * 8 * NC) = unpack(acc[r][0], acc[r][1]);
@@ -726,13 +733,11 @@ chunk_out_kernel(const ChunkArgs a) {
         __syncthreads();                             // slice sl is there, the other stage is read
         if (sl + 1 < n1 + n2) issue(sl + 1, (sl + 1) & 1);
         const bool second = sl >= n1;
-        const int k0 = (second ? sl - n1 : sl) * 32, kn = second ? min(32, rg * 4 + 4 - k0) : min(32, dk - k0);
+        const int k0 = (second ? sl - n1 : sl) * 32;
         const int ld = second ? LP : LD;
         const float* rows = (second ? ps : qs) + (size_t)(rg * 4) * ld + k0;
         const float* b = bsm + (size_t)(sl & 1) * 32 * JB + tj * 4;
-#pragma unroll 2
-        for (int k = 0; k < kn; k += 4) {            // of P nothing above the diagonal
-            const bool edge = second && k0 + k == rg * 4;
+        auto block = [&](int k, auto diagonal) {     // four columns; on P's diagonal a row takes those up to its own
             float4 x[4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) x[r] = *reinterpret_cast<const float4*>(rows + r * ld + k);
@@ -740,8 +745,7 @@ chunk_out_kernel(const ChunkArgs a) {
             for (int q = 0; q < 4; ++q) {
                 const ulonglong2 y0 = pairs(b + (k + q) * JB), y1 = pairs(b + (k + q) * JB + 64);
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    if (q > r && edge) continue;
+                for (int r = decltype(diagonal)::value ? q : 0; r < 4; ++r) {
                     const pair_t xx = dup(q == 0 ? x[r].x : q == 1 ? x[r].y : q == 2 ? x[r].z : x[r].w);
                     fma2(acc[r][0], xx, y0.x);
                     fma2(acc[r][1], xx, y0.y);
@@ -749,7 +753,11 @@ chunk_out_kernel(const ChunkArgs a) {
                     fma2(acc[r][3], xx, y1.y);
                 }
             }
-        }
+        };
+        const int kn = second ? min(32, rg * 4 - k0) : min(32, dk - k0);     // of P nothing above the diagonal
+#pragma unroll 2
+        for (int k = 0; k < kn; k += 4) block(k, std::false_type());
+        if (second && kn >= 0 && kn < 32) block(kn, std::true_type());
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
