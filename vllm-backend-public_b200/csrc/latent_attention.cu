@@ -931,7 +931,11 @@ extern "C" int b2_window_attention(void* out, const void* qn, int64_t qn_row, in
     pa.scale = scale; pa.window = window;
     pa.sink = sink_logits ? 1.f : 0.f; pa.sink_logits = sink_logits;
     pa.gate = gate; pa.gate_stride = gate_stride; pa.gate_channels = gate_channels; pa.out = out; pa.out_stride = out_stride;
-    if (b2_internal_prompt_tc5_ok(pa)) return b2_internal_prompt_tc5(pa, stream);
+    // The tcgen05 kernel's CTA is one an SM and takes 9 us from its start to its end with a single tile of keys; three CTAs of the other
+    // share an SM.  More than two waves of CTAs with fewer than 80 rows a sequence go to the other one: 64 x 40 rows, 16 heads 47 us
+    // against 62, 200 x 20 160 against 197, 30 x 64 30 against 35; 30 x 100 50 against 37, and one wave takes the same in both.
+    const bool many_short = (int64_t)T < 80 * (int64_t)n_seq && ((int64_t)T / 128 + n_seq) * H > 2 * (int64_t)latent_sm_count();
+    if (!many_short && b2_internal_prompt_tc5_ok(pa)) return b2_internal_prompt_tc5(pa, stream);
     const size_t smem = (size_t)((kWQ + kWK) * (dn + dr + 8) + kWK * (dv + 8)) * sizeof(__nv_bfloat16);
     B2_REQUIRE(smem <= 200 * 1024, B2_EUNSUPPORTED, "window_attention: key size %d too large", dn + dr);
     if (smem > 48 * 1024)
