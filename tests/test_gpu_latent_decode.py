@@ -1,4 +1,5 @@
-"""Decode rows of b2_latent_attention (one row a sequence) against fp64: latents of 128, 256 and 512 numbers with rotated parts that do
+"""Decode rows of b2_latent_attention (one row a sequence) against fp64, by both kernels that take them (block tables as wide as the rows,
+and so wide that they promise enough work for the tcgen05 kernel): latents of 128, 256 and 512 numbers with rotated parts that do
 and do not fill their 64 columns, more and fewer heads than a CTA takes, key counts around tiles of 64 and boxes of 16, pages TMA boxes
 fit and do not fit, windows that begin inside a page, keys split over CTAs, and scores that outgrow the first tile's by 2^60 and more.
 
@@ -14,6 +15,12 @@ from b200attn import ops
 pytestmark = pytest.mark.gpu
 
 
+def _widen(tables, bs, wide):
+    """Columns up to 100000 tokens, behind every row's end: the rule between the kernels goes by the table's width."""
+    return torch.nn.functional.pad(tables, (0, 100000 // bs - tables.shape[1])).contiguous() if wide else tables
+
+
+@pytest.mark.parametrize("wide", [False, True])
 @pytest.mark.parametrize("ctx,H,R,dr,bs,window,sink,gate,rise", [
     ([0, 1, 15, 16, 17, 62, 63, 64, 65, 127, 128, 129], 16, 512, 64, 16, 0, False, False, 0.0),
     ([700, -1, 3], 32, 512, 64, 16, 0, True, True, 0.0),                 # split over CTAs, padding between
@@ -26,8 +33,12 @@ pytestmark = pytest.mark.gpu
     ([1500, 130], 16, 512, 64, 16, 0, True, False, 400.0),               # computed a second time
     ([1500] * 150, 4, 256, 64, 16, 0, False, False, 400.0),              # ... without a split, an odd number of tiles
     ([1500, 130], 16, 512, 64, 16, 0, True, False, -400.0),              # falling scores: late weights vanish
+    ([3000 - i for i in range(32)], 32, 512, 64, 16, 700, True, False, 0.0),     # windows in the tcgen05 kernel
+    ([1500 - 7 * i for i in range(16)], 64, 256, 32, 24, 1100, False, True, 0.0),        # ... pages of 24
+    ([700, 40, 3], 18, 512, 256, 16, 0, True, True, 0.0),                # keys of more than 640 numbers
+    ([300, 9], 20, 128, 768, 16, 0, False, False, 0.0),                  # ... of more than either kernel takes
 ])
-def test_latent_decode(cuda, ctx, H, R, dr, bs, window, sink, gate, rise):
+def test_latent_decode(cuda, ctx, H, R, dr, bs, window, sink, gate, rise, wide):
     g = torch.Generator(device=cuda).manual_seed(len(ctx) * 100 + H + window)
     rnd = lambda *s: torch.randn(*s, generator=g, device=cuda)           # noqa: E731
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
@@ -49,7 +60,7 @@ def test_latent_decode(cuda, ctx, H, R, dr, bs, window, sink, gate, rise):
         cache[page[dead], off[dead]] = float("nan")
     sinks = rnd(H) if sink else None
     wide = rnd(n, H + 3).bfloat16()
-    batch = ops.SeqBatch(i32(list(range(n + 1))), i32(ctx), tables, None, n, n)
+    batch = ops.SeqBatch(i32(list(range(n + 1))), i32(ctx), _widen(tables, bs, wide), None, n, n)
     out = ops.latent_attention(qa, cache, batch, R, scale, window, gate=wide[:, :H] if gate else None, sink_logits=sinks).double()
     for i, c in enumerate(ctx):
         if c < 0:
@@ -90,13 +101,14 @@ def test_long_rows_repeat_to_the_bit(cuda):
         assert torch.equal(first, ops.latent_attention(qa, cache, batch, R, (R + dr) ** -0.5, 0))
 
 
-def test_as_many_rows_as_sequences_but_not_one_each(cuda):
+@pytest.mark.parametrize("wide", [False, True])
+def test_as_many_rows_as_sequences_but_not_one_each(cuda, wide):
     """Rows [2, 0, 1, 3, 0, 0]: every row is its own sequence's, at its own position; the same rows asked one by one give the same bits."""
     g = torch.Generator(device=cuda).manual_seed(9)
     lens, ctx, H, R, dr, bs = [2, 0, 1, 3, 0, 0], [40, 5, 0, 130, 7, 9], 20, 256, 64, 16
     n, nb = len(lens), 10
     cache = torch.randn(n * nb, bs, R + dr, generator=g, device=cuda).bfloat16()
-    tables = torch.randperm(n * nb, generator=g, device=cuda).to(torch.int32).view(n, nb)
+    tables = _widen(torch.randperm(n * nb, generator=g, device=cuda).to(torch.int32).view(n, nb), bs, wide)
     qa = torch.randn(n, H, R + dr, generator=g, device=cuda).bfloat16()
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
     cu = [sum(lens[:i]) for i in range(n + 1)]
@@ -110,7 +122,8 @@ def test_as_many_rows_as_sequences_but_not_one_each(cuda):
 
 @pytest.mark.parametrize("n", [3, 160])                                  # keys split over CTAs, and not
 @pytest.mark.parametrize("where", [0, 1, 700])
-def test_a_nan_in_a_cached_row_stays_one(cuda, n, where):
+@pytest.mark.parametrize("wide", [False, True])
+def test_a_nan_in_a_cached_row_stays_one(cuda, wide, n, where):
     """A NaN in the rotated part of a cached row reaches every output of its sequence and no other's, however the keys are shared."""
     g = torch.Generator(device=cuda).manual_seed(11)
     H, R, dr, bs, c = 8, 512, 64, 16, 900
@@ -120,13 +133,14 @@ def test_a_nan_in_a_cached_row_stays_one(cuda, n, where):
     cache[nb + where // bs, where % bs, R + 5] = float("nan")
     qa = torch.randn(n, H, R + dr, generator=g, device=cuda).bfloat16()
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
-    out = ops.latent_attention(qa, cache, ops.SeqBatch(i32(list(range(n + 1))), i32([c] * n), tables, None, n, n), R, 0.04, 0)
+    out = ops.latent_attention(qa, cache, ops.SeqBatch(i32(list(range(n + 1))), i32([c] * n), _widen(tables, bs, wide), None, n, n), R, 0.04, 0)
     nan = torch.isnan(out).flatten(1)
     assert bool(nan[1].all()) and not bool(nan[0].any()) and not bool(nan[2:].any())
 
 
 @pytest.mark.parametrize("n", [2, 150])                                  # keys split over CTAs, and not
-def test_a_sink_far_above_the_first_share(cuda, n):
+@pytest.mark.parametrize("wide", [False, True])
+def test_a_sink_far_above_the_first_share(cuda, wide, n):
     """Scores that climb by 400 (in powers of two) over the row and a sink between: above the first share's scores by more than fp32
     holds, far below the last's, so that it weighs nothing; and a sink above all of them, which leaves nothing to the keys."""
     g = torch.Generator(device=cuda).manual_seed(13)
@@ -140,7 +154,7 @@ def test_a_sink_far_above_the_first_share(cuda, n):
     row = torch.arange(nb * bs, device=cuda).float()
     cache[..., R] = ((row / c - 0.5) * 400.0 / 8.0 / scale * math.log(2.0)).bfloat16().view(nb, bs).repeat(n, 1)
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
-    batch = ops.SeqBatch(i32(list(range(n + 1))), i32([c] * n), tables, None, n, n)
+    batch = ops.SeqBatch(i32(list(range(n + 1))), i32([c] * n), _widen(tables, bs, wide), None, n, n)
     plain = ops.latent_attention(qa, cache, batch, R, scale, 0)
     between = ops.latent_attention(qa, cache, batch, R, scale, 0, sink_logits=torch.full((H,), 0.0, device=cuda))
     above = ops.latent_attention(qa, cache, batch, R, scale, 0, sink_logits=torch.full((H,), 300.0, device=cuda))
@@ -149,12 +163,12 @@ def test_a_sink_far_above_the_first_share(cuda, n):
     assert bool((above.float().abs() <= 1e-6).all())
 
 
-@pytest.mark.parametrize("n", [4, 150])                                  # keys split over CTAs, and not
-def test_the_error_is_the_rounding_of_the_result(cuda, n):
-    """Weights are kept to 16 bits, so what is left against fp64 is the result's own rounding to bf16: 5 % above it are allowed for the
+@pytest.mark.parametrize("n,H,c", [(8, 64, 3000), (150, 16, 1000)])     # keys split over CTAs, and not
+def test_the_error_is_the_rounding_of_the_result(cuda, n, H, c):
+    """The tcgen05 kernel: weights are kept to 16 bits, so what is left against fp64 is the result's own rounding to bf16: 5 % above it are allowed for the
     fp32 sums.  (Weights of eight bits against another reference than the row's maximum: 24 % above.)"""
     g = torch.Generator(device=cuda).manual_seed(17)
-    H, R, dr, bs, c = 16, 512, 64, 16, 1000
+    R, dr, bs = 512, 64, 16
     nb = c // bs + 1
     cache = torch.randn(n * nb, bs, R + dr, generator=g, device=cuda).bfloat16()
     tables = torch.arange(n * nb, dtype=torch.int32, device=cuda).view(n, nb)

@@ -22,8 +22,8 @@
 //                         Softmax state, scores and the accumulator are fp32.
 // Sequences are described like everywhere in this library: rows cu_q[i] .. cu_q[i+1]-1, ctx_start[i] cached tokens before
 // them (< 0: padding, output rows are zeroed), block_tables[i, :].
-// A batch with as many rows as sequences (a decode step: one row each) may take the decode kernel of latent_tc5.cu, which looks up
-// the sequence of every row and so takes any division of them.  b2_latent_attention_workspace tells how much fp32 scratch a call can use
+// A batch with as many rows as sequences (a decode step: one row each) may take the decode kernels, here and in latent_tc5.cu, which look
+// up the sequence of every row and so take any division of them.  b2_latent_attention_workspace tells how much fp32 scratch a call can use
 // to split the keys of a row over CTAs; without it the call runs unsplit.
 #include "b2_act.cuh"
 
@@ -474,6 +474,208 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ qa, const __nv_bfl
     }
 }
 
+// ------------------------------------------------------------------------------------------------- decode rows
+// Decode rows (as many rows as sequences) that do not go to latent_tc5.cu: batches with little work and keys of more than 640 numbers.
+// bf16, R >= 128: a CTA takes one token x up to 16 heads (one m16 row group), so
+// the eight warps cannot share rows -- they share the KEYS of a tile instead.  Warp w scores keys 8w .. 8w+7 of the 64-key
+// tile against all 16 rows, the row maxima meet in shared memory, every warp writes its 16 x 8 slice of P (bf16) to a
+// shared P tile, and then multiplies the whole P tile with ITS R / 8 output columns of the key rows.  No score is computed
+// twice, and the chain of dependent instructions per tile is an eighth of what one warp per row group would run.
+constexpr int kPLD = kLK + 8;
+
+__device__ __forceinline__ void ldmatrix_x2(uint32_t addr, uint32_t& r0, uint32_t& r1) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
+}
+
+template <int RT>
+__global__ void __launch_bounds__(256)
+latent_attention_decode_kernel(const __nv_bfloat16* __restrict__ qa, const __nv_bfloat16* __restrict__ cache,
+                               const int32_t* __restrict__ block_tables, int max_nb, const int32_t* __restrict__ cu_q,
+                               const int32_t* __restrict__ ctx_start, int n_seq, int H, int dr, int bs, float scale_log2, int window,
+                               const float* __restrict__ sink_logits, const __nv_bfloat16* __restrict__ gate,
+                               int64_t gate_stride, __nv_bfloat16* __restrict__ out, float* __restrict__ ws_o,
+                               float* __restrict__ ws_ml) {
+    constexpr int R = 16 * RT, CW = R / 8, NTO = CW / 8;                    // output columns / n-tiles per warp
+    static_assert(CW % 16 == 0, "a warp owns whole pairs of n-tiles");
+    const int Dc = R + dr, LD = Dc + 8, vecs = Dc / 8;
+    extern __shared__ __align__(16) unsigned char lat_smem[];
+    __nv_bfloat16* q_sm = reinterpret_cast<__nv_bfloat16*>(lat_smem);       // [16][LD]
+    __nv_bfloat16* k_sm = q_sm + 16 * LD;                                   // [2][64][LD]
+    __nv_bfloat16* p_sm = k_sm + 2 * kLK * LD;                              // [16][kPLD]
+    float* mx_sm = reinterpret_cast<float*>(p_sm + 16 * kPLD);              // [8][16]: row maxima, later row sums, per warp
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int tok = blockIdx.x, seq = b2::seq_of_row(cu_q, n_seq, tok);
+    const int h0 = blockIdx.y * 16, nh = min(16, H - h0);
+    const int nsplit = gridDim.z, zs = blockIdx.z;
+    const int ctx = ctx_start[seq];
+    if (ctx < 0) {                                                          // padding
+        if (nsplit > 1) {
+            for (int rr = tid; rr < nh; rr += 256) {
+                float* ml = ws_ml + (((size_t)tok * H + h0 + rr) * nsplit + zs) * 2;
+                ml[0] = -INFINITY;
+                ml[1] = 0.f;
+            }
+        } else {
+            for (int idx = tid; idx < nh * (R / 8); idx += 256)
+                *reinterpret_cast<uint4*>(out + ((size_t)tok * H + h0 + idx / (R / 8)) * R + (idx % (R / 8)) * 8) =
+                    make_uint4(0, 0, 0, 0);
+        }
+        return;
+    }
+    const int pos = ctx + tok - cu_q[seq];
+    const int klo = window > 0 ? max(pos - window + 1, 0) : 0;
+    const int32_t* bt = block_tables + (size_t)seq * max_nb;
+    for (int idx = tid; idx < 16 * vecs; idx += 256) {
+        const int r = idx / vecs, c = (idx % vecs) * 8;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (r < nh) v = *reinterpret_cast<const uint4*>(qa + ((size_t)tok * H + h0 + r) * Dc + c);
+        *reinterpret_cast<uint4*>(q_sm + r * LD + c) = v;
+    }
+    const int gq = lane >> 2, tq = lane & 3;
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+    if (sink_logits && zs == 0) {                                           // every warp keeps the same maximum, its own sums
+        m0 = sink_logits[h0 + min(gq, nh - 1)] * kLog2e;
+        m1 = sink_logits[h0 + min(gq + 8, nh - 1)] * kLog2e;
+        if (w == 0 && tq == 0) l0 = l1 = 1.f;
+    }
+    float o[NTO][4];
+#pragma unroll
+    for (int n = 0; n < NTO; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+    const uint32_t q_base = b2::smem_u32(q_sm), k_base0 = b2::smem_u32(k_sm), p_base = b2::smem_u32(p_sm);
+    const int ksteps = Dc / 16;
+    const int ld_key = tid >> 2, ld_sub = (tid & 3) * 8;
+    auto issue = [&](int kv0, int buf) {
+        const int j = kv0 + ld_key;
+        __nv_bfloat16* dst = k_sm + (size_t)buf * kLK * LD + ld_key * LD;
+        if (j <= pos) {
+            const __nv_bfloat16* src = cache + ((size_t)bt[j / bs] * bs + j % bs) * Dc;
+            for (int c = ld_sub; c < Dc; c += 32) cp_async16(dst + c, src + c);
+        } else {
+            for (int c = ld_sub; c < Dc; c += 32) *reinterpret_cast<uint4*>(dst + c) = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int all_tiles = (pos - klo) / kLK + 1, per = (all_tiles + nsplit - 1) / nsplit;
+    const int t_begin = zs * per, ntiles = min(all_tiles, t_begin + per);
+    if (t_begin < ntiles) issue(klo + t_begin * kLK, 0);
+    for (int t = t_begin; t < ntiles; ++t) {
+        const int kv0 = klo + t * kLK, buf = (t - t_begin) & 1;
+        if (t + 1 < ntiles) {
+            issue(kv0 + kLK, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();                                                    // the tile (and, first time, Q) is in shared memory
+        const uint32_t k_base = k_base0 + (uint32_t)buf * kLK * LD * 2u;
+        float sc[4] = {0.f, 0.f, 0.f, 0.f};                                 // 16 rows x this warp's 8 keys
+#pragma unroll 4
+        for (int kk = 0; kk < ksteps; ++kk) {
+            uint32_t a0, a1, a2, a3, b0, b1;
+            b2::ldmatrix_x4(q_base + 2u * ((lane & 15) * LD + kk * 16 + (lane >> 4) * 8), a0, a1, a2, a3);
+            ldmatrix_x2(k_base + 2u * ((w * 8 + (lane & 7)) * LD + kk * 16 + ((lane >> 3) & 1) * 8), b0, b1);
+            b2::mma_bf16_16816(sc, a0, a1, a2, a3, b0, b1);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int j = kv0 + w * 8 + 2 * tq + (e & 1);
+            sc[e] = (j >= klo && j <= pos) ? sc[e] * scale_log2 : -INFINITY;
+        }
+        float mx0 = fmaxf(sc[0], sc[1]), mx1 = fmaxf(sc[2], sc[3]);
+        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+        if (tq == 0) {
+            mx_sm[w * 16 + gq] = mx0;
+            mx_sm[w * 16 + gq + 8] = mx1;
+        }
+        __syncthreads();                                                    // every warp's row maxima of this tile
+        float mn0 = m0, mn1 = m1;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+            mn0 = fmaxf(mn0, mx_sm[x * 16 + gq]);
+            mn1 = fmaxf(mn1, mx_sm[x * 16 + gq + 8]);
+        }
+        const float mu0 = mn0 == -INFINITY ? 0.f : mn0, mu1 = mn1 == -INFINITY ? 0.f : mn1;
+        const float c0 = exp2f(m0 - mu0), c1 = exp2f(m1 - mu1);
+        m0 = mn0;
+        m1 = mn1;
+        sc[0] = exp2f(sc[0] - mu0);
+        sc[1] = exp2f(sc[1] - mu0);
+        sc[2] = exp2f(sc[2] - mu1);
+        sc[3] = exp2f(sc[3] - mu1);
+        l0 = l0 * c0 + sc[0] + sc[1];                                       // sums over this warp's keys only
+        l1 = l1 * c1 + sc[2] + sc[3];
+        *reinterpret_cast<uint32_t*>(p_sm + gq * kPLD + w * 8 + 2 * tq) = b2::pack_bf16x2(sc[0], sc[1]);
+        *reinterpret_cast<uint32_t*>(p_sm + (gq + 8) * kPLD + w * 8 + 2 * tq) = b2::pack_bf16x2(sc[2], sc[3]);
+#pragma unroll
+        for (int n = 0; n < NTO; ++n) {
+            o[n][0] *= c0;
+            o[n][1] *= c0;
+            o[n][2] *= c1;
+            o[n][3] *= c1;
+        }
+        __syncthreads();                                                    // the P tile is complete
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+            uint32_t a0, a1, a2, a3;
+            b2::ldmatrix_x4(p_base + 2u * ((lane & 15) * kPLD + ks * 16 + (lane >> 4) * 8), a0, a1, a2, a3);
+#pragma unroll
+            for (int n2 = 0; n2 < NTO / 2; ++n2) {
+                uint32_t b0, b1, b2_, b3;
+                const int key = ks * 16 + ((lane >> 3) & 1) * 8 + (lane & 7), col = w * CW + n2 * 16 + (lane >> 4) * 8;
+                b2::ldmatrix_x4_trans(k_base + 2u * (key * LD + col), b0, b1, b2_, b3);
+                b2::mma_bf16_16816(o[2 * n2], a0, a1, a2, a3, b0, b1);
+                b2::mma_bf16_16816(o[2 * n2 + 1], a0, a1, a2, a3, b2_, b3);
+            }
+        }
+        __syncthreads();                                                    // the tile, P and the maxima are consumed
+    }
+    // the row sums of the eight key slices
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+    if (tq == 0) {
+        mx_sm[w * 16 + gq] = l0;
+        mx_sm[w * 16 + gq + 8] = l1;
+    }
+    __syncthreads();
+    l0 = l1 = 0.f;
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+        l0 += mx_sm[x * 16 + gq];
+        l1 += mx_sm[x * 16 + gq + 8];
+    }
+    const bool va = gq < nh, vb = gq + 8 < nh;
+    const size_t ra = (size_t)tok * H + h0 + gq, rb = ra + 8;
+    if (nsplit > 1) {
+        if (w == 0 && tq == 0) {
+            if (va) { ws_ml[(ra * nsplit + zs) * 2] = m0; ws_ml[(ra * nsplit + zs) * 2 + 1] = l0; }
+            if (vb) { ws_ml[(rb * nsplit + zs) * 2] = m1; ws_ml[(rb * nsplit + zs) * 2 + 1] = l1; }
+        }
+#pragma unroll
+        for (int n = 0; n < NTO; ++n) {
+            const int col = w * CW + n * 8 + 2 * tq;
+            if (va) *reinterpret_cast<float2*>(ws_o + (ra * nsplit + zs) * R + col) = make_float2(o[n][0], o[n][1]);
+            if (vb) *reinterpret_cast<float2*>(ws_o + (rb * nsplit + zs) * R + col) = make_float2(o[n][2], o[n][3]);
+        }
+        return;
+    }
+    float f0 = l0 > 0.f ? 1.f / l0 : 0.f, f1 = l1 > 0.f ? 1.f / l1 : 0.f;
+    if (gate) {
+        if (va) f0 *= b2::sigmoid_f(__bfloat162float(gate[(size_t)tok * gate_stride + h0 + gq]));
+        if (vb) f1 *= b2::sigmoid_f(__bfloat162float(gate[(size_t)tok * gate_stride + h0 + gq + 8]));
+    }
+#pragma unroll
+    for (int n = 0; n < NTO; ++n) {
+        const int col = w * CW + n * 8 + 2 * tq;
+        if (va) *reinterpret_cast<uint32_t*>(out + ra * R + col) = b2::pack_bf16x2(o[n][0] * f0, o[n][1] * f0);
+        if (vb) *reinterpret_cast<uint32_t*>(out + rb * R + col) = b2::pack_bf16x2(o[n][2] * f1, o[n][3] * f1);
+    }
+}
+
 // ------------------------------------------------------------------------------------------------- prompt portions, per-head keys
 // Long prompt portions are cheaper with keys and values rebuilt per head: a (query, key) pair then costs dn + dr + dv
 // multiplications instead of 2 R + dr.  The latent rows a portion can see are gathered from the pages into one
@@ -745,20 +947,28 @@ inline int latent_sm_count() {
 }
 
 // Which kernel and how many shares of the key tiles per CTA row: a batch that cannot fill the GPU (decode rows) splits its
-// keys over CTAs.  decode: as many rows as sequences and latent_tc5.cu takes the sizes.
+// keys over CTAs.  decode: as many rows as sequences and a latent wide enough for eight column slices; tc5: by latent_tc5.cu.
 struct LatentPlan {
-    bool decode;
+    bool decode, tc5;
     int nsplit;
 };
+inline size_t latent_decode_smem(int Dc) { return ((size_t)(16 + 2 * kLK) * (Dc + 8) + 16 * kPLD) * sizeof(__nv_bfloat16) + 128 * sizeof(float); }
 inline LatentPlan latent_plan(int T, int n_seq, int H, int R, int dr, int window, int max_nb, int bs) {
     LatentPlan p;
-    p.decode = T == n_seq && b2_internal_latent_tc5_ok(R, dr);
     const int Hc = H < kLQ ? H : kLQ, Gt = kLQ / Hc;
-    const int group = b2_internal_latent_tc5_heads();
-    const long ctas = p.decode ? (long)T * ((H + group - 1) / group) : (long)(T < T / Gt + n_seq ? T : T / Gt + n_seq) * ((H + Hc - 1) / Hc);
     long keys = (long)max_nb * bs;
-    const int span = p.decode ? 1 : Gt;
+    const bool rows = T == n_seq && R >= 128;
+    const int span = rows ? 1 : Gt;
     if (window > 0 && window + span < keys) keys = window + span;
+    // The tcgen05 kernel reads a row's keys at twice the other's rate and more but takes 4 us longer from its start to its end (13 us with
+    // a single tile, the other 7 - 9).  Both measured over 1 - 128 rows, 4 - 64 heads, 40 - 6000 keys: it is the faster one from these
+    // products of rows, groups of 16 heads and keys on (at them 0.92 - 1.0 of the other's time, at four times them 0.4 - 0.8).  The host
+    // knows the width of the block table, not the rows' lengths: short rows in a wide table take those 4 us.
+    const long from = R == 512 ? 36000 : R == 256 ? 64000 : 90000;
+    p.tc5 = rows && b2_internal_latent_tc5_ok(R, dr) && (double)keys * T * ((H + 15) / 16) >= from;
+    p.decode = p.tc5 || (rows && latent_decode_smem(R + dr) <= 227 * 1024);
+    const int group = p.tc5 ? b2_internal_latent_tc5_heads() : 16;
+    const long ctas = p.decode ? (long)T * ((H + group - 1) / group) : (long)(T < T / Gt + n_seq ? T : T / Gt + n_seq) * ((H + Hc - 1) / Hc);
     const long tiles = (keys + kLK - 1) / kLK;
     long n = latent_sm_count() / (ctas > 0 ? ctas : 1);
     if (n > tiles / 2) n = tiles / 2;
@@ -770,7 +980,7 @@ inline LatentPlan latent_plan(int T, int n_seq, int H, int R, int dr, int window
 template <int RT>
 int launch_latent_mma(void* out, const void* qa, const void* cache, const int32_t* block_tables, int max_nb, const int32_t* cu_q,
                       const int32_t* ctx_start, int n_seq, int T, int H, int dr, int bs, float scale, int window,
-                      const float* sink_logits, const void* gate, int64_t gate_stride, bool decode, int nsplit, float* ws,
+                      const float* sink_logits, const void* gate, int64_t gate_stride, const LatentPlan& plan, int nsplit, float* ws,
                       cudaStream_t st) {
     const int Dc = 16 * RT + dr, Hc = H < kLQ ? H : kLQ, Gt = kLQ / Hc;
     const size_t tile = (size_t)kLK * (Dc + 8) * sizeof(__nv_bfloat16);
@@ -782,10 +992,20 @@ int launch_latent_mma(void* out, const void* qa, const void* cache, const int32_
     float* ws_o = ws;
     float* ws_ml = ws ? ws + (size_t)T * H * nsplit * 16 * RT : nullptr;
     if constexpr (RT >= 8) {
-        if (decode) {
-            const int rc = b2_internal_latent_tc5(out, qa, cache, block_tables, max_nb, cu_q, ctx_start, n_seq, T, H, 16 * RT, dr, bs, scale, window,
-                                                  sink_logits, gate, gate_stride, nsplit, ws_o, ws_ml, st);
-            if (rc != B2_OK) return rc;
+        if (plan.decode) {
+            if (plan.tc5) {
+                const int rc = b2_internal_latent_tc5(out, qa, cache, block_tables, max_nb, cu_q, ctx_start, n_seq, T, H, 16 * RT, dr, bs, scale,
+                                                      window, sink_logits, gate, gate_stride, nsplit, ws_o, ws_ml, st);
+                if (rc != B2_OK) return rc;
+            } else {
+                const size_t dsm = latent_decode_smem(Dc);
+                auto dk = latent_attention_decode_kernel<RT>;
+                if (dsm > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(dk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
+                dk<<<dim3(T, (H + 15) / 16, nsplit), 256, dsm, st>>>(
+                    static_cast<const __nv_bfloat16*>(qa), static_cast<const __nv_bfloat16*>(cache), block_tables, max_nb, cu_q, ctx_start,
+                    n_seq, H, dr, bs, scale * kLog2e, window, sink_logits, static_cast<const __nv_bfloat16*>(gate), gate_stride,
+                    static_cast<__nv_bfloat16*>(out), ws_o, ws_ml);
+            }
             if (nsplit > 1)
                 latent_merge_kernel<<<T * H, 128, 0, st>>>(ws_o, ws_ml, nsplit, 16 * RT, H, static_cast<const __nv_bfloat16*>(gate),
                                                            gate_stride, static_cast<__nv_bfloat16*>(out));
@@ -873,7 +1093,7 @@ extern "C" int b2_latent_attention(void* out, const void* qa, const void* cache,
         if (nsplit > 1 && (!workspace || !b2_aligned16(workspace) || workspace_floats < (int64_t)T * H * nsplit * (R + 2))) nsplit = 1;
 #define B2_LAT(RT)                                                                                                            \
     return launch_latent_mma<RT>(out, qa, cache, block_tables, max_nb, cu_q, ctx_start, n_seq, T, H, dr, bs, scale, window, \
-                                 sink_logits, gate, gate_stride, plan.decode, nsplit, nsplit > 1 ? workspace : nullptr, st)
+                                 sink_logits, gate, gate_stride, plan, nsplit, nsplit > 1 ? workspace : nullptr, st)
         if (R == 64) B2_LAT(4);
         if (R == 128) B2_LAT(8);
         if (R == 256) B2_LAT(16);

@@ -52,16 +52,18 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
     constexpr int R = 128 * RT, COLS = RT == 4 ? 512 : RT == 2 ? 256 : 128;      // TMEM: S of the halves at 0 and 32, O^T at 64
     extern __shared__ unsigned char lat_sm_raw[];
-    __shared__ __align__(8) uint64_t s_bar[9];
+    __shared__ __align__(8) uint64_t s_bar[10];
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed, s_redo;
     __shared__ int s_max[HEADS];                     // ordered(): maxima found
     __shared__ __align__(16) float s_ref[HEADS];
-    __shared__ float s_f[HEADS];
+    __shared__ __align__(16) float s_f[HEADS];
+    __shared__ float s_sum[4][HEADS];
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     // a CTA belongs to a row: as many rows as sequences is one row each as a rule, but [2, 0] is as many too
-    const int tok = blockIdx.x, seq = b2::seq_of_row(p.cu_q, p.n_seq, tok), h0 = blockIdx.y * HEADS, nh = min(HEADS, p.H - h0);
-    const int nsplit = gridDim.z, zs = blockIdx.z, ctx = p.ctx_start[seq], bs = p.bs;
+    const int tok = blockIdx.x, guess = p.ctx_start[tok];            // asked for beside the row's sequence: nearly always its own
+    const int seq = b2::seq_of_row(p.cu_q, p.n_seq, tok), h0 = blockIdx.y * HEADS, nh = min(HEADS, p.H - h0);
+    const int nsplit = gridDim.z, zs = blockIdx.z, ctx = seq == tok ? guess : p.ctx_start[seq], bs = p.bs;
     const int pos = ctx + tok - p.cu_q[seq], klo = p.window > 0 ? max(pos - p.window + 1, 0) : 0, kbase = klo & ~15;
     const int all_tiles = ctx < 0 ? 0 : (pos - kbase) / KT + 1, per = (all_tiles + nsplit - 1) / nsplit;
     const int t0 = zs * per, nt = min(all_tiles, t0 + per) - t0;
@@ -83,7 +85,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
     unsigned char* gen = lat_sm_raw + (ring - b2::smem_u32(lat_sm_raw));
     volatile int* failed = &s_failed;
     auto bar = [&](int i) { return b2::smem_u32(&s_bar[i]); };
-    enum { FULL = 0, EMPTY = 2, SC = 4, PR = 6, END = 8 };
+    enum { FULL = 0, EMPTY = 2, SC = 4, PR = 6, END = 8, QUERY = 9 };
     if (tid == 0) {
         s_failed = s_redo = 0;
         for (int s = 0; s < 2; ++s) {
@@ -93,6 +95,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
             b2::mbar_init(bar(PR + s), 2);           // ... per softmax warp of the half
         }
         b2::mbar_init(bar(END), 1);
+        b2::mbar_init(bar(QUERY), 5);                // one arrive per warp that loads queries
         b2::fence_mbar_init();
     }
     // the sink counts among the scores the reference is taken from: a sum is at least one and finite, which the merge relies on
@@ -101,19 +104,35 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(b2::smem_u32(&s_tmem)), "n"(COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    for (int idx = tid; idx < HEADS * (Dc / 8); idx += NTHREADS) {
-        const int r = idx / (Dc / 8), c = idx % (Dc / 8);
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (r < nh) v = *reinterpret_cast<const uint4*>(p.qa + ((size_t)tok * p.H + h0 + r) * Dc + c * 8);
-        *reinterpret_cast<uint4*>(gen + (q_sm - ring) + (c >> 3) * Q_SUB + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = v;
-    }
-    b2::fence_proxy_async();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
     const int32_t* bt = p.block_tables + (size_t)seq * p.max_nb;
-    float l[HEADS];
+    float l[HEADS], mx[HEADS];
+    if (warp < 5) {                                  // the queries, five loads in flight, while the other warps fetch the first tiles
+        const int qc = Dc / 8;
+        const bf16* q = p.qa + ((size_t)tok * p.H + h0) * Dc;
+        for (int first = tid; first < HEADS * qc; first += 5 * 160) {
+            uint4 v[5];
+#pragma unroll
+            for (int u = 0; u < 5; ++u) {
+                const int idx = first + u * 160;
+                v[u] = make_uint4(0, 0, 0, 0);
+                if (idx < nh * qc) v[u] = *reinterpret_cast<const uint4*>(q + idx * 8);
+            }
+#pragma unroll
+            for (int u = 0; u < 5; ++u) {
+                const int idx = first + u * 160, r = idx / qc, c = idx - r * qc;
+                if (idx < HEADS * qc) *reinterpret_cast<uint4*>(gen + (q_sm - ring) + (c >> 3) * Q_SUB + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = v[u];
+            }
+        }
+        b2::fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) b2::mbar_arrive(bar(QUERY));
+    }
+#pragma unroll
+    for (int h = 0; h < HEADS; ++h) mx[h] = -INFINITY;
 
     for (int pass = 0, it0 = 0; pass < 2; ++pass, it0 += nt) {           // `it` counts the tiles of both passes: half it & 1
         if (warp >= 5) {
@@ -197,6 +216,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
                 }
                 __syncwarp();
             };
+            wait(bar(QUERY), 0, failed);
             scores(0);
 #pragma unroll 1
             for (int t = 0; t < nt; ++t) {
@@ -229,12 +249,8 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
             if (!wait(bar(END), pass, failed)) drain(bar(END), pass);
         } else {
             // ---------------------------------------------- softmax: lane = key; warps 0, 1 the first half of the ring, 2, 3 the second
-            float mx[HEADS];
 #pragma unroll
-            for (int h = 0; h < HEADS; ++h) {
-                l[h] = 0.f;
-                mx[h] = -INFINITY;
-            }
+            for (int h = 0; h < HEADS; ++h) l[h] = 0.f;
             auto publish = [&]() {                   // s_max: the maxima over this warp's lanes
 #pragma unroll
                 for (int h = 0; h < HEADS; ++h) {
@@ -250,6 +266,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
                 }
                 asm volatile("bar.sync 1, 128;" ::: "memory");
             };
+            if (pass == 1) publish();                // all the maxima found
             if (pass == 1 || warp >= 2) settle();
 #pragma unroll 1
             for (int t = (it0 ^ (warp >> 1)) & 1; t < nt; t += 2) {
@@ -299,7 +316,6 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
                 bool far = false;
 #pragma unroll
                 for (int h = 0; h < HEADS; ++h) far |= mx[h] > s_ref[h] + kRedo;
-                publish();
                 if (__any_sync(0xffffffffu, far) && lane == 0) s_redo = 1;
             }
         }
@@ -314,9 +330,15 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
 #pragma unroll
         for (int h = 0; h < HEADS; ++h) part[tid * (HEADS + 1) + h] = l[h];
     __syncthreads();
-    if (tid < HEADS) {
+    if (warp < 4) {                                  // a quarter of the lanes' parts a warp
         float sum = 0.f;
-        for (int r = 0; r < 128; ++r) sum += part[r * (HEADS + 1) + tid];
+#pragma unroll 8
+        for (int r = 0; r < 32; ++r) sum += part[(warp * 32 + r) * (HEADS + 1) + lane];
+        s_sum[warp][lane] = sum;
+    }
+    __syncthreads();
+    if (tid < HEADS) {
+        float sum = (s_sum[0][tid] + s_sum[1][tid]) + (s_sum[2][tid] + s_sum[3][tid]);
         const int h = h0 + min(tid, nh - 1);
         if (p.sink_logits && zs == 0) sum += b2::fast_exp2(p.sink_logits[h] * kLog2e - s_ref[tid]);
         if (s_failed) sum = __int_as_float(0x7fc00000);
@@ -341,14 +363,23 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
             tmem_ld32(tmem + 64 + 64 * m + ((uint32_t)(warp * 32) << 16), acc);
             tmem_ld32(tmem + 96 + 64 * m + ((uint32_t)(warp * 32) << 16), rest);
             tmem_wait_ld();
-            const int c = 128 * m + tid;
             const size_t row = (size_t)tok * p.H + h0;
+            if (nsplit > 1) {
+                float* o = p.ws_o + (row * nsplit + zs) * R + 128 * m + tid;
+                const size_t step = (size_t)nsplit * R;
 #pragma unroll
-            for (int h = 0; h < HEADS; ++h) {
-                if (h >= nh) break;
-                const float v = __uint_as_float(acc[h]) + __uint_as_float(rest[h]);
-                if (nsplit > 1) p.ws_o[((row + h) * nsplit + zs) * R + c] = v;
-                else p.out[(row + h) * R + c] = __float2bfloat16_rn(v * s_f[h]);
+                for (int h = 0; h < HEADS; ++h)
+                    if (h < nh) o[h * step] = __uint_as_float(acc[h]) + __uint_as_float(rest[h]);
+            } else {
+                bf16* o = p.out + row * R + 128 * m + tid;
+#pragma unroll
+                for (int h = 0; h < HEADS; h += 4) {
+                    const float4 f4 = *reinterpret_cast<const float4*>(s_f + h);
+                    const float f[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (h + u < nh) o[(h + u) * R] = __float2bfloat16_rn((__uint_as_float(acc[h + u]) + __uint_as_float(rest[h + u])) * f[u]);
+                }
             }
         }
     }
