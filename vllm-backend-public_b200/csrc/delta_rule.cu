@@ -752,6 +752,7 @@ int launch_prep(const void* proj, int64_t proj_stride, const PrepSpec& sp, int T
                 float* decay, cudaStream_t st) {
     const int C = 2 * sp.G * sp.dk + sp.H * sp.dv;
     const size_t smem = (size_t)C * sizeof(float);
+    B2_REQUIRE(smem <= 200 * 1024, B2_EUNSUPPORTED, "recurrence prep: %d channels do not fit shared memory", C);
     const bool channel_decay = sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS || sp.decay_mode == B2_DECAY_CHANNEL_SIGMOID_POW;
     const int P = sp.dk / 4;
     const bool vec = sp.dk % 4 == 0 && P <= 32 && (P & (P - 1)) == 0 && sp.dv % 4 == 0 && sp.taps <= 4 && (conv_w || sp.taps == 1) &&
@@ -772,11 +773,10 @@ int launch_prep(const void* proj, int64_t proj_stride, const PrepSpec& sp, int T
         else B2_PREP_VEC(4);
 #undef B2_PREP_VEC
     } else {
-    B2_REQUIRE(smem <= 200 * 1024, B2_EUNSUPPORTED, "recurrence prep: %d channels do not fit shared memory", C);
-    auto kern = recur_prep_kernel<A>;
-    if (smem > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<T, 256, smem, st>>>(static_cast<const A*>(proj), proj_stride, sp, conv_w, cu_q, ctx_start, state_slot, n_seq,
-                               static_cast<const A*>(conv_state), qkv, beta, decay);
+        auto kern = recur_prep_kernel<A>;
+        if (smem > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<T, 256, smem, st>>>(static_cast<const A*>(proj), proj_stride, sp, conv_w, cu_q, ctx_start, state_slot, n_seq,
+                                   static_cast<const A*>(conv_state), qkv, beta, decay);
     }
     B2_CUDA_OK(cudaGetLastError());
     if (sp.taps > 1) {
