@@ -100,7 +100,8 @@ B2_API int b2_reshape_and_cache_decode(const void* k_new, const void* v_new, voi
  * per-GPU head counts after tensor_parallel_size sharding (models.py:11).
  *   out[b][hq] = softmax_j(scale * <q[b][hq], K[b][j][hq / G]>) . V[b][j][hq / G],  j < seq_lens[b]
  *   G = Hq / Hkv; fp32 softmax and accumulation; out rounded to bf16 once; seq_len 0 -> zeros.
- * num_splits: 0 = choose automatically, 1 = single pass ("v1"), >1 = split-K over the KV length
+ * num_splits: 0 = choose automatically (the dynamic persistent schedule, or a single pass where the block tables hold 640 tokens a
+ * row at most and the items fit one wave; b2_paged_decode_auto_splits tells), 1 = single pass ("v1"), >1 = split-K over the KV length
  * with a log-sum-exp merge ("v2").  The workspace (device memory, 16-byte aligned) must hold
  * b2_paged_decode_workspace_bytes(...) bytes for the same B/Hq/d/max_nb/bs/num_splits; it is
  * scratch (no state survives the call) and may be NULL when that size is 0.
@@ -111,13 +112,13 @@ B2_API int b2_reshape_and_cache_decode(const void* k_new, const void* v_new, voi
 B2_API size_t b2_paged_decode_workspace_bytes(int B, int Hq, int Hkv, int d, int bs, int max_nb,
                                        int num_splits);
 
-/* the split count b2_paged_decode will actually use for num_splits = 0 */
+/* the split count b2_paged_decode will actually use for num_splits = 0; 0: the dynamic persistent schedule */
 B2_API int b2_paged_decode_auto_splits(int B, int Hq, int Hkv, int d, int bs, int max_nb, int kv_dtype);
 
 /* Host-side schedule choice for callers that hold seq_lens on the host (the scheduler always does; it is the
  * role `max_seq_len` plays for vLLM's paged_attention_v1/v2 choice).  Returns the num_splits to pass to
  * b2_paged_decode: 1 when the single-pass grid (one CTA per (sequence, kv head)) keeps the machine balanced
- * for these lengths, 0 (dynamic persistent schedule) otherwise; negative on bad arguments.  Pure host code. */
+ * for these lengths, 0 (the call's own choice, see num_splits) otherwise; negative on bad arguments.  Pure host code. */
 B2_API int b2_paged_decode_plan_splits(const int32_t* seq_lens_host, int B, int Hq, int Hkv, int d, int bs,
                                 int kv_dtype);
 
@@ -144,7 +145,8 @@ B2_API int b2_paged_decode(void* out, const void* q,
  * With num_splits = 1 (the single-pass grid; b2_paged_decode_plan_splits picks it for long uniform batches) and
  * Hq / Hkv <= 16 it is ONE kernel launch: the CTA that owns (row, kv head) stores the new K/V row itself and issues
  * the TMA copy of the stage that holds it only once the store is visible to the async proxy (fence.proxy.async) -- the step has no second launch
- * and no kernel boundary.  b2_paged_decode_append_fused tells (1 / 0; negative on bad arguments).  Every other schedule
+ * and no kernel boundary.  b2_paged_decode_append_fused tells (1 / 0; negative on bad arguments); with num_splits = 0 it answers for
+ * the dynamic schedule, though a call that takes a single pass is one launch as well.  Every other schedule
  * cuts a row over several CTAs: the call then launches the KV write in front of the decode grid (same results). */
 B2_API int b2_paged_decode_append_fused(int Hq, int Hkv, int num_splits);
 B2_API int b2_paged_decode_append(void* out, const void* q,

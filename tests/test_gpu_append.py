@@ -130,6 +130,22 @@ def test_append_unfused_schedules(cuda, splits, Hq, Hkv):
     _check(_case(cuda, EDGE_LENS, Hq, Hkv, 16, False, seed=splits + Hq), splits=splits)
 
 
+def _widen(c, columns=48):
+    """The same rows under block tables of 768 tokens: num_splits = 0 takes the single pass for tables of 640 and less."""
+    extra = columns - c["bt"].shape[1]
+    assert extra > 0
+    pad = lambda bt: torch.cat([bt, bt.new_zeros(bt.shape[0], extra)], 1).contiguous()       # noqa: E731
+    return dict(c, bt=pad(c["bt"]), host=dict(c["host"], bt=pad(c["host"]["bt"])))
+
+
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("Hq,Hkv", [(8, 2), (32, 8), (40, 2)])
+def test_append_before_the_dynamic_schedule(cuda, Hq, Hkv, fp8):
+    c = _widen(_case(cuda, EDGE_LENS, Hq, Hkv, 16, fp8, seed=Hq))
+    assert b200attn.decode_auto_splits(len(EDGE_LENS), Hq, Hkv, 128, 16, c["bt"].shape[1]) == 0
+    _check(c, splits=0)
+
+
 def test_append_padding_rows_and_strides(cuda):
     """slot < 0 rows write nothing (their newest token is already cached here); k_new / v_new as strided views of a fused
     q|k|v buffer, the way an engine holds them."""
@@ -150,8 +166,8 @@ def test_append_many_short_rows_config_shape(cuda):
 
 
 @pytest.mark.parametrize("fp8", [False, True])
-@pytest.mark.parametrize("splits", [1, 0])
-def test_plan_run_append_resident_tables(cuda, fp8, splits):
+@pytest.mark.parametrize("splits,wide", [(1, False), (0, False), (0, True)], ids=["1", "0", "0-dynamic"])
+def test_plan_run_append_resident_tables(cuda, fp8, splits, wide):
     """b2_decode_plan_run_append over device-RESIDENT block tables: rows whose new token opens a block (length = n * bs + 1)
     arrive with a stale table entry for it (a wrong block id here), exactly what an engine's resident table holds before
     the step.  Bar: out, both caches and the table bit-identical to b2_reshape_and_cache_decode + b2_decode_plan_run."""
@@ -159,6 +175,8 @@ def test_plan_run_append_resident_tables(cuda, fp8, splits):
     bs = 16
     lens = [1, 17, 33, 16, 65, 64, 129, 300, 2, 49]
     c = _case(cuda, lens, 8, 2, bs, fp8, seed=21 + splits)
+    if wide:                                                  # tables too wide for the single pass that num_splits = 0 takes for short ones
+        c = _widen(c)
     ks, vs = c["scales"]
     stale = c["bt"].clone()
     for b, L in enumerate(lens):

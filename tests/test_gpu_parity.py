@@ -559,6 +559,20 @@ def test_decode_two_box_fallback_map(cuda, monkeypatch):
         assert torch.equal(bits(outs["0", splits]), bits(outs["1", splits]))
 
 
+def test_decode_two_box_fallback_map_dynamic_schedule(cuda, monkeypatch):
+    """The same with tables of 1000 tokens, for which num_splits = 0 is the dynamic schedule (those of 640 and less take the single pass)."""
+    inp = R.make_inputs(6, 16, 2, 128, 16, 1000, seed=44, ragged=True)
+    assert b200attn.decode_auto_splits(6, 16, 2, 128, 16, inp["block_tables"].shape[1]) == 0
+    kc, vc, kc_ref, vc_ref, _ = build_caches(inp, cuda)
+    ref = R.paged_decode_ref(inp["q"], kc_ref, vc_ref, inp["block_tables"], inp["seq_lens"], return_f32=True)
+    outs = []
+    for two in ("0", "1"):
+        monkeypatch.setenv("B2_TWO_BOX", two)
+        outs.append(run_decode(inp, kc, vc, cuda, num_splits=0))
+        assert_close(outs[-1], ref, what=f"two_box={two}")
+    assert torch.equal(bits(outs[0]), bits(outs[1]))
+
+
 def test_workspace_for_max_batch_serves_every_smaller_batch(cuda):
     """one workspace sized for max_num_seqs = 32 at max_model_len 8192 must be accepted by every
     batch size below it under the dynamic schedule (B = 24 needs more partial slots than B = 32)."""

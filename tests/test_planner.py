@@ -55,3 +55,13 @@ def test_append_fused_rule():
     assert not b200attn.append_is_fused(40, 2, 1)        # G = 20: two head-group CTAs share a kv head
     with pytest.raises(b200attn.B2Error):
         b200attn.append_is_fused(30, 8, 1)               # Hq not a multiple of Hkv
+
+
+def test_auto_splits_tells_what_the_call_takes():
+    """num_splits = 0: a single pass where the tables hold 640 tokens at most and the items fit one wave of two CTAs an SM (no device
+    here: 148 SMs), the dynamic schedule elsewhere."""
+    auto = b200attn.decode_auto_splits
+    assert auto(4, 8, 2, 128, 16, 32) == 1 and auto(4, 8, 2, 128, 16, 40) == 1 and auto(1, 32, 8, 128, 32, 20) == 1
+    assert auto(4, 8, 2, 128, 16, 41) == 0 and auto(4, 8, 2, 128, 32, 21) == 0 and auto(4, 8, 2, 128, 16, 512) == 0
+    assert auto(37, 32, 8, 128, 16, 40) == 1 and auto(38, 32, 8, 128, 16, 40) == 0       # 296 items, 304
+    assert auto(74, 48, 2, 128, 16, 40) == 1 and auto(75, 48, 2, 128, 16, 40) == 0       # 24 heads a kv head: two items each

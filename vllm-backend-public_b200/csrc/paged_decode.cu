@@ -1452,7 +1452,12 @@ struct Plan {
     int nc;            // dynamic: CTAs of the persistent grid the plan was made for
 };
 
-constexpr int SHORT_ROW_TOKENS = 640;                // rows that a CTA streams faster than further launches start
+// num_splits = 0 with block tables too narrow for long rows and all items in one wave: the single-pass grid.  It is one launch (KV
+// write included) and streams a CTA's tokens at about 10.7 ns each behind 3.3 us; the dynamic schedule starts at 9.6 us whatever the
+// batch (write, counter, decode, merge).  Measured with 1 - 32 rows in a graph, single / dynamic, bf16: 4.7 / 10.5 us at 128 tokens,
+// 8.4 / 11.6 at 512, 13.8 / 13.7 at 1024; fp8: 4.9 / 10.2, 7.8 / 11.7, 12.5 / 13.5.  Launched one by one 20 / 29 at 512.
+constexpr int SHORT_ROW_TOKENS = 640;
+bool short_rows(int64_t B, int ipb, int bs, int max_nb) { return (int64_t)max_nb * bs <= SHORT_ROW_TOKENS && B * ipb <= 2 * (int64_t)sm_count(); }
 
 // dynamic schedule: workspace header (claim counter)
 constexpr size_t WS_HEADER_BYTES = 256;
@@ -1682,11 +1687,7 @@ int run_decode(const DecodeGeom& g, const CacheMaps& maps, const Knobs& kn, bool
     Plan pl;
     make_plan(&pl, B, g.Hkv, G, g.bs, g.max_nb, num_splits, ctas_per_sm(fp8, G, kn.fp8_ctas), kn);
     const Plan asked = pl;                               // what the workspace is checked against
-    // Block tables too narrow for long rows, and all items in one wave: the single-pass grid whatever was asked.  It is one launch (KV
-    // write included) and streams a CTA's tokens at about 10.7 ns each behind 3.3 us; the dynamic schedule starts at 9.6 us whatever the
-    // batch (write, counter, decode, merge).  Measured with 1 - 32 rows in a graph, single / dynamic, bf16: 4.7 / 10.5 us at 128 tokens,
-    // 8.4 / 11.6 at 512, 13.8 / 13.7 at 1024; fp8: 4.9 / 10.2, 7.8 / 11.7, 12.5 / 13.5.  Launched one by one 20 / 29 at 512.
-    if (pl.num_splits == 0 && (int64_t)g.max_nb * g.bs <= SHORT_ROW_TOKENS && (int64_t)B * pl.ipb <= 2 * (int64_t)sm_count())
+    if (pl.num_splits == 0 && short_rows(B, pl.ipb, g.bs, g.max_nb))
         make_plan(&pl, B, g.Hkv, G, g.bs, g.max_nb, 1, ctas_per_sm(fp8, G, kn.fp8_ctas), kn);
 
     DecodeParams p;
@@ -1772,7 +1773,8 @@ int b2_internal_make_cache_tmap(CUtensorMap* tm, const void* cache, int kv_dtype
 extern "C" int b2_paged_decode_auto_splits(int B, int Hq, int Hkv, int d, int bs, int max_nb, int kv_dtype) {
     (void)kv_dtype;
     if (!shape_ok(B, Hq, Hkv, d, bs, max_nb)) return B2_EINVAL;
-    return 0;   // num_splits = 0 selects the persistent schedule: no fixed split count
+    const int hpc = Hq / Hkv <= 8 ? 8 : 16;
+    return short_rows(B, Hkv * ((Hq / Hkv + hpc - 1) / hpc), bs, max_nb) ? 1 : 0;      // 0: the persistent schedule, no fixed split count
 }
 
 // Host-side schedule choice from the scheduler's own (host) copy of seq_lens -- the same role max_seq_len plays
