@@ -20,8 +20,7 @@ def _widen(tables, bs, wide):
     return torch.nn.functional.pad(tables, (0, 100000 // bs - tables.shape[1])).contiguous() if wide else tables
 
 
-@pytest.mark.parametrize("wide", [False, True])
-@pytest.mark.parametrize("ctx,H,R,dr,bs,window,sink,gate,rise", [
+CASES = [
     ([0, 1, 15, 16, 17, 62, 63, 64, 65, 127, 128, 129], 16, 512, 64, 16, 0, False, False, 0.0),
     ([700, -1, 3], 32, 512, 64, 16, 0, True, True, 0.0),                 # split over CTAs, padding between
     ([2000], 33, 512, 64, 32, 0, True, False, 0.0),                      # one head more than a CTA takes, up to 16 shares
@@ -37,8 +36,20 @@ def _widen(tables, bs, wide):
     ([1500 - 7 * i for i in range(16)], 64, 256, 32, 24, 1100, False, True, 0.0),        # ... pages of 24
     ([700, 40, 3], 18, 512, 256, 16, 0, True, True, 0.0),                # keys of more than 640 numbers
     ([300, 9], 20, 128, 768, 16, 0, False, False, 0.0),                  # ... of more than either kernel takes
-])
-def test_latent_decode(cuda, ctx, H, R, dr, bs, window, sink, gate, rise, wide):
+]
+
+
+@pytest.mark.parametrize("ctx,H,R,dr,bs,window,sink,gate,rise", CASES)
+def test_latent_decode(cuda, ctx, H, R, dr, bs, window, sink, gate, rise):
+    _check(cuda, ctx, H, R, dr, bs, window, sink, gate, rise, False)
+
+
+@pytest.mark.parametrize("ctx,H,R,dr,bs,window,sink,gate,rise", CASES)
+def test_latent_decode_wide_tables(cuda, ctx, H, R, dr, bs, window, sink, gate, rise):
+    _check(cuda, ctx, H, R, dr, bs, window, sink, gate, rise, True)
+
+
+def _check(cuda, ctx, H, R, dr, bs, window, sink, gate, rise, wide):
     g = torch.Generator(device=cuda).manual_seed(len(ctx) * 100 + H + window)
     rnd = lambda *s: torch.randn(*s, generator=g, device=cuda)           # noqa: E731
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
