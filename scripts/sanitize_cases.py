@@ -5,8 +5,7 @@
 
 All three decode schedules (single pass, grid split + merge, dynamic persistent + merge), bf16 and fp8 caches, ragged
 lengths incl. 0 and 1, KV write (both encodings, skipped slots), the decode-step write over resident block tables,
-tcgen05 and mma.sync prompt-chunk attention, the element-wise layer ops, sampling, and the tensor-parallel exchange
-kernels with two emulated ranks on one device.  Every case is also checked against the CPU oracle."""
+tcgen05 and mma.sync prompt-chunk attention, the element-wise layer ops and sampling.  Every case is also checked against the CPU oracle."""
 import os
 import sys
 from pathlib import Path
@@ -162,11 +161,6 @@ def layer_cases():
     print("layer cases ok")
 
 
-def comm_cases():
-    import test_gpu_comm as TC
-    TC._two_rank_protocol()
-
-
 if __name__ == "__main__":
     if want("decode"):
         decode_cases()
@@ -174,7 +168,5 @@ if __name__ == "__main__":
         step_cases()
     if want("layer"):
         layer_cases()
-    if want("comm"):
-        comm_cases()
     torch.cuda.synchronize()
     print("sanitize cases done")

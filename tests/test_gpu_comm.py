@@ -3,21 +3,14 @@ benchmark-vllm/models.py:11) on ONE GPU.
 
 * tp = 1: b2_comm_allreduce_rms_norm must equal b2_rms_norm with the fused residual add (residual bit for bit), and
   b2_comm_allgather_cols must be a copy.
-* tp = 2 emulated in one process: two regions on the same device, "rank 0" and "rank 1" launched on two streams, so
-  the flag protocol, the epoch counter, the slot alternation and the peer loads / stores run for real (the peers
-  just happen to share a device).  Checked against a plain fp32 torch sum.  It runs in a SUBPROCESS: a protocol bug
-  traps the kernel after 10 s and poisons the CUDA context, which must not take the rest of the suite with it.
+tp = 2 is not emulated here: the ranks' kernels wait for one another.
 The two-process CUDA-IPC path over NVLink is exercised by scripts/tp_check.py / bench.py --gpus N (needs >= 2 GPUs)."""
 import ctypes as C
-import subprocess
-import sys
-from pathlib import Path
 
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
-ROOT = Path(__file__).resolve().parent.parent
 
 
 class Regions:
@@ -110,61 +103,6 @@ def test_comm_tp1_equals_rms_norm(cuda, H):
         R.close()
 
 
-def _two_rank_protocol():
-    """Body of the subprocess: 2 emulated ranks on one device, 40 alternating exchanges + gathers."""
-    sys.path.insert(0, str(ROOT / "vllm-backend-public_b200"))
-    torch.manual_seed(0)
-    H, T, V = 1024, 8, 512
-    R = Regions(2, 16, H, 16, V)
-    s = [torch.cuda.Stream(), torch.cuda.Stream()]
-    w = torch.randn(H, device="cuda").to(torch.bfloat16)
-    worst = 0.0
-    for it in range(60):
-        slot = (it // 3) & 1
-        parts = [torch.randn(T, H, device="cuda").to(torch.bfloat16) for _ in range(2)]
-        resid0 = torch.randn(T, H, device="cuda").to(torch.bfloat16)
-        torch.cuda.synchronize()
-        outs, resids = [], []
-        if it % 7 == 3:
-            parts[0][2, 5:9] = -0.0                      # the sentinel value itself must survive the push protocol
-        for r in range(2):
-            with torch.cuda.stream(s[r]):
-                out, rs = torch.empty(T, H, dtype=torch.bfloat16, device="cuda"), resid0.clone()
-                if it % 3 == 2:                          # every third exchange through the pull variant
-                    R.inputs[r][slot][:T].copy_(parts[r])
-                    R.allreduce(r, slot, out, rs, w, T, 1e-5, s[r])
-                else:
-                    R.push(r, parts[r], out, rs, w, 1e-5, s[r])
-                outs.append(out)
-                resids.append(rs)
-        torch.cuda.synchronize()
-        h = (parts[0].float() + parts[1].float() + resid0.float()).to(torch.bfloat16)
-        hf = h.float()
-        ref = (w.float() * (hf * torch.rsqrt((hf * hf).mean(dim=1, keepdim=True) + 1e-5))).to(torch.bfloat16)
-        for r in range(2):
-            assert torch.equal(resids[r].view(torch.int16), h.view(torch.int16)), f"iteration {it}: residual of rank {r}"
-            worst = max(worst, float((outs[r].float() - ref.float()).abs().max()))
-        assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16)), "ranks must compute the same bits"
-        if it % 5 == 4:                                  # a gather between exchanges, as after the lm_head
-            loc = [torch.randn(T, V // 2, device="cuda").to(torch.bfloat16) for _ in range(2)]
-            torch.cuda.synchronize()
-            for r in range(2):
-                with torch.cuda.stream(s[r]):
-                    R.allgather(r, loc[r], s[r])
-            torch.cuda.synchronize()
-            full = torch.cat(loc, dim=1)
-            for r in range(2):
-                assert torch.equal(R.gathered[r][:T].view(torch.int16), full.view(torch.int16)), f"gather on rank {r}"
-    assert worst <= 0.07, worst            # one bf16 ulp at |x| <= 8
-    R.close()
-    print("two-rank protocol ok, worst", worst)
-
-
 def test_comm_two_emulated_ranks_on_one_gpu(cuda):
-    r = subprocess.run([sys.executable, str(Path(__file__).resolve()), "two-rank"], capture_output=True, text=True,
-                       timeout=300)
-    assert r.returncode == 0 and "two-rank protocol ok" in r.stdout, (r.stdout[-2000:], r.stderr[-2000:])
-
-
-if __name__ == "__main__" and sys.argv[1:] == ["two-rank"]:
-    _two_rank_protocol()
+    pytest.skip("two ranks whose kernels wait for one another are not run as separate launches on one GPU: nothing guarantees that they "
+                "run at the same time.  scripts/tp_check.py runs the exchange with a GPU a rank")
