@@ -29,7 +29,7 @@ def test_small_or_skewed_batches_take_the_dynamic_schedule():
 
 def test_ragged_serving_batches_take_the_dynamic_schedule():
     """log-uniform 128..ctx lengths: the per-item pipeline ramp of the single-pass grid costs more than the dynamic
-    schedule's ~4 % (measured +9 % / +7 % for configs[3] / configs[1] shapes, scripts/gpu_ragged.sh)."""
+    schedule's ~4 % (measured +9 % / +7 % for configs[3] / configs[1] shapes, bench.py --ragged)."""
     import math
     g = torch.Generator().manual_seed(1234)
     for B, ctx, Hq, Hkv in ((256, 8192, 64, 8), (64, 4096, 32, 8)):

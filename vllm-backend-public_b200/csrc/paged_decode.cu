@@ -1828,7 +1828,7 @@ extern "C" int b2_paged_decode_plan_splits(const int32_t* seq_lens_host, int B, 
     const double est = std::max(ideal, (double)makespan / slack);
     // the dynamic schedule keeps its pipelines full across items (no per-item ramp) at ~4 % for chunk boundaries, the
     // claim counter and the merge: measured -4 % on uniform config 2, +9 % / +7 % / +56 % on log-uniform 128..ctx
-    // batches of configs 4 / 2 / 3 (scripts/gpu_ragged.sh)
+    // batches of configs 4 / 2 / 3 (bench.py --ragged)
     const double est_dynamic = 1.04 * (double)streamed / NC;
     return est <= est_dynamic ? 1 : 0;
 }

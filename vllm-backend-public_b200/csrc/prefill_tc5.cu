@@ -18,8 +18,8 @@
 // Round 2, what bounded the kernel and what did not (8k chunk over an 8k prefix, Llama-3-8B heads, block_size 16;
 // clock64 timeline from `make trace` + scripts/trace_prefill.py, profiles/r2_trace_prefill_issuer*.txt):
 //   1055 TF/s  round-1 kernel.  ncu: tensor pipe 48 %, XU pipe 48 %, softmax warps waiting for S in 56 % of samples.
-//   not it     softmax latency hiding: TWO threads per query row (scripts/experiments_prefill_two_threads_per_row.cu.txt,
-//              profiles/r2_ncu_prefill_two_threads_per_row.md) 1038; maximum pass off the chain (speculative maximum) 947;
+//   not it     softmax latency hiding: TWO threads per query row (profiles/r2_ncu_prefill_two_threads_per_row.md)
+//              1038; maximum pass off the chain (speculative maximum) 947;
 //              polynomial exp2 for 1-3 of every 4 weights (B2_PREFILL_POLY) slower then and now (1371 / 1266 / 1164).
 //   not it     shared-memory operand bandwidth of cta_group::1 (an earlier reading of the timeline, WRONG):
 //              scripts/umma_rate.cu shows SS, TS, MN-major B, the kernel's own P.V | Q.K^T mix and all of them under
