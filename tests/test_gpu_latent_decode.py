@@ -49,7 +49,7 @@ def test_latent_decode_wide_tables(cuda, ctx, H, R, dr, bs, window, sink, gate, 
     _check(cuda, ctx, H, R, dr, bs, window, sink, gate, rise, True)
 
 
-def _check(cuda, ctx, H, R, dr, bs, window, sink, gate, rise, wide):
+def _check(cuda, ctx, H, R, dr, bs, window, sink, gate, rise, wide_table):
     g = torch.Generator(device=cuda).manual_seed(len(ctx) * 100 + H + window)
     rnd = lambda *s: torch.randn(*s, generator=g, device=cuda)           # noqa: E731
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
@@ -71,7 +71,7 @@ def _check(cuda, ctx, H, R, dr, bs, window, sink, gate, rise, wide):
         cache[page[dead], off[dead]] = float("nan")
     sinks = rnd(H) if sink else None
     wide = rnd(n, H + 3).bfloat16()
-    batch = ops.SeqBatch(i32(list(range(n + 1))), i32(ctx), _widen(tables, bs, wide), None, n, n)
+    batch = ops.SeqBatch(i32(list(range(n + 1))), i32(ctx), _widen(tables, bs, wide_table), None, n, n)
     out = ops.latent_attention(qa, cache, batch, R, scale, window, gate=wide[:, :H] if gate else None, sink_logits=sinks).double()
     for i, c in enumerate(ctx):
         if c < 0:
