@@ -1258,7 +1258,7 @@ int launch_heads(const void* q, const void* k_cache, const void* v_cache, const 
     if (chunk > 0 && chunk < keys) keys = chunk;
     if (window > 0 && window + keep_first < keys) keys = window + keep_first;
     const int64_t items = (int64_t)ctas * G;
-    const int nw = items <= 148 && keys >= 512 ? 16 : items <= 296 && keys >= 256 ? 8 : 4;
+    const int nw = items <= b2_sm_count() && keys >= 512 ? 16 : items <= 2 * b2_sm_count() && keys >= 256 ? 8 : 4;
 #define B2_HEADS_NW(NW, FEW)                                                                                                      \
     return (FEW && dk <= kShortDk ? launch_heads_nw<DVT, SIG, MAPS, NW, FEW, FEW ? 2 * kHeadKeys : kHeadKeys>                     \
                                   : launch_heads_nw<DVT, SIG, MAPS, NW, FEW, kHeadKeys>)(q, k_cache, v_cache, block_tables, max_nb, cu_q, ctx_start, n_seq, ctas, H, G, dk, bs, scale, \

@@ -781,7 +781,7 @@ int allow(K kern, size_t bytes) {
 
 template <bool CH, bool DELTA>
 int launch(const ChunkArgs& a, int total_rows, cudaStream_t st) {
-    static const int n_sm = []() { int dev = 0, n = 148; if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); return n; }();
+    const int n_sm = b2_sm_count();
     const int chunks = total_rows / C + a.n_seq;     // upper bound on sum(ceil(len / C)); spare CTAs leave at once
     const size_t LD = a.dk + 4, rows = C * LD;
     const size_t psm = sizeof(float) * (rows + (DELTA ? rows : (rows > C * JB ? rows : C * JB)) + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows : 2 * C + 4) + C);
@@ -834,7 +834,7 @@ bool b2_internal_chunk_scan_pays(int total_rows, int n_seq, int H, int dk, int d
     const float longest = len * (n_seq > 1 ? 1.25f : 1.f);
     const float tokens = fmaxf(chain_tok[kind] * (dk <= 64 ? 0.75f : 1.f) * longest, rate * (float)total_rows * H * w);
     float chunks = (per_chunk[kind] * (0.35f + 0.65f * w) * steps + 0.11f * w) * heads;
-    if (delta) chunks += (3.4f + 1.4f * w) * fmaxf(ceilf(longest / C), steps * heads * ((dv + NC - 1) / NC) / 148.f);
+    if (delta) chunks += (3.4f + 1.4f * w) * fmaxf(ceilf(longest / C), steps * heads * ((dv + NC - 1) / NC) / b2_sm_count());
     return tokens >= fmaxf(chunks, least[kind]);
 }
 

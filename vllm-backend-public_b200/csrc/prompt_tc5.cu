@@ -661,7 +661,7 @@ bool b2_internal_prompt_tc5_ok(const b2_prompt_args& a) {
 }
 
 int b2_internal_prompt_tc5(const b2_prompt_args& a, void* stream) {
-    static const int n_sm = []() { int dev = 0, n = 148; if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); return n; }();
+    const int n_sm = b2_sm_count();
     Params p;
     p.a = a;
     p.scale_log2 = a.scale * LOG2E;
