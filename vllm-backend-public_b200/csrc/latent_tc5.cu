@@ -12,10 +12,11 @@
 // powers of two), the share is computed again with the maxima found.  A weight is two bf16 numbers, its rounding and what that left
 // over, side by side in the 128 bytes of a key's row of P: with one, the largest weights, which a running maximum makes exactly one,
 // are rounded too (error against 64 bits 0.00210, 0.00206 with a running maximum, 0.0018 with both halves).
-// Bound: the bytes of the cached rows (74 KB a tile and SM).  The form on mma.sync with Q in registers waited for its own chain of
-// ldmatrix, MMA and barriers, two warps a scheduler: 64 sequences x 32 heads x 2560 keys of 576 took 120 us (140 with Q in shared memory); this one 60 (3.2 TB/s, two shares a row on 128
-// SMs: a tile's load, scores, softmax and output follow one another in each half of the ring).  An output goes before the next scores
-// whenever those still wait for their tile: always behind them, it took 88.
+// Bound: the bytes of the cached rows (74 KB a tile and SM).  64 sequences x 32 heads x 2560 keys of 576 in a graph, merge of two shares a
+// row included: 137 us on mma.sync (its own chain of ldmatrix, MMA and barriers, two warps a scheduler), 60 here (on 128 SMs: a tile's
+// load, scores, softmax and output follow one another in each half of the ring).  An output goes before the next scores whenever those
+// still wait for their tile: always behind them, it took 88.  Start and end take 13 us with a single tile; they took 20 with the queries
+// loaded one after another in front of the first tile, row sums by one warp and a branch around every store.
 #include "b2_act.cuh"
 #include "b2_tc5.cuh"
 
