@@ -127,8 +127,10 @@ def test_masked_prompt_rows(cuda, c):
     ([200], [10], 5, 40, 24, 48, 77, False, 1),                          # a sub-tile across both parts of the key: no TMA boxes
     ([200, 30], [0, 10], 2, 24, 8, 112, 0, True, 2),
     ([30, 1, 64, 40] * 12, [0, 20, 0, 9] * 12, 8, 128, 64, 128, 0, True, 1),     # many short portions: the mma.sync kernel
-    ([90, 65] * 12, [0, 20] * 12, 12, 64, 64, 96, 50, False, 2),                 # ... and so many that are not quite
-    ([100, 65] * 12, [0, 20] * 12, 12, 64, 64, 96, 50, False, 2),
+    ([70, 57] * 12, [0, 0] * 12, 12, 64, 64, 96, 50, False, 2),                  # ... 64 keys a portion, and more
+    ([70, 57] * 12, [0, 9] * 12, 12, 64, 64, 96, 50, False, 2),
+    ([3, 8, 1] * 20, [100, 9, 260] * 20, 6, 128, 64, 128, 0, False, 1),          # ... a few rows each, up to 160 keys, and more
+    ([3, 8, 1] * 20, [100, 99, 360] * 20, 6, 128, 64, 128, 0, False, 1),
 ])
 def test_gathered_prompt_rows(cuda, lens, ctx, H, dn, dr, dv, window, sink, gate):
     g = torch.Generator(device=cuda).manual_seed(sum(lens) + H)

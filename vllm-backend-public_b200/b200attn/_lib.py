@@ -160,6 +160,8 @@ SIGNATURES = {
     "b2_latent_gather": (i32, [vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, vp]),
     "b2_window_attention": (i32, [vp, vp, i64, i32, vp, i64, i32, vp, vp, i64, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32,
                                   f32, i32, vp, vp, i64, i32, i64, vp]),
+    "b2_window_attention_rows": (i32, [vp, vp, i64, i32, vp, i64, i32, vp, vp, i64, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32,
+                                       f32, i32, vp, vp, i64, i32, i64, i64, vp]),
     "b2_latent_attention_workspace": (i64, [i32, i32, i32, i32, i32, i32, i32, i32, i32]),
 }
 

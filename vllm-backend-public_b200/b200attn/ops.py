@@ -1581,7 +1581,7 @@ def window_attention(qn: torch.Tensor, qr: torch.Tensor, kn: torch.Tensor, kt: t
     (shared by the heads; may be a column slice), v [N, H, dv] over the gathered rows (see latent_gather).  The row at
     position p sees positions max(0, p - window + 1) .. p (window 0: 0 .. p); sink_logits fp32 [H]: exp(sink_logits[h]) joins the
     denominator.  Returns sigmoid(gate) * softmax(..) v as bf16 [T, H, dv], gate [T, H] or one column per channel [T, H * dv]; or
-    `out`: rows of H * dv values (a column range of a wider buffer).  b2_window_attention."""
+    `out`: rows of H * dv values (a column range of a wider buffer).  b2_window_attention_rows."""
     lib = _lib.load()
     dev = _need_cuda(qn=qn, qr=qr, kn=kn, kt=kt, v=v, gate=gate, sink_logits=sink_logits, out=out)
     T, H, dn = qn.shape
@@ -1603,8 +1603,8 @@ def window_attention(qn: torch.Tensor, qr: torch.Tensor, kn: torch.Tensor, kt: t
     if out is None:
         out = torch.empty(T, H, dv, dtype=torch.bfloat16, device=dev)
     os_ = _out_rows(out, T, H * dv, torch.bfloat16)
-    _lib.check(lib.b2_window_attention(_ptr(out), _ptr(qn), qn.stride(0), qn.stride(1), _ptr(qr), qr.stride(0), qr.stride(1),
-                                       _ptr(kn), _ptr(kt), kt.stride(0), _ptr(v), _ptr(cu_q), _ptr(ctx_start), _ptr(cu_k),
-                                       _ptr(k_lo), n_seq, T, H, dn, dr, dv, float(scale), int(window), _ptr(sink_logits),
-                                       _ptr(gate), gs, int(channels), os_, _stream(dev)))
+    _lib.check(lib.b2_window_attention_rows(_ptr(out), _ptr(qn), qn.stride(0), qn.stride(1), _ptr(qr), qr.stride(0), qr.stride(1),
+                                            _ptr(kn), _ptr(kt), kt.stride(0), _ptr(v), _ptr(cu_q), _ptr(ctx_start), _ptr(cu_k),
+                                            _ptr(k_lo), n_seq, T, H, dn, dr, dv, float(scale), int(window), _ptr(sink_logits),
+                                            _ptr(gate), gs, int(channels), os_, N, _stream(dev)))
     return out

@@ -1129,6 +1129,16 @@ extern "C" int b2_window_attention(void* out, const void* qn, int64_t qn_row, in
                                    int n_seq, int T, int H, int dn, int dr, int dv, float scale, int window,
                                    const float* sink_logits, const void* gate, int64_t gate_stride, int gate_channels,
                                    int64_t out_stride, void* stream) {
+    return b2_window_attention_rows(out, qn, qn_row, qn_head, qr, qr_row, qr_head, kn, kt, kt_row, v, cu_q, ctx_start, cu_k, k_lo, n_seq, T, H,
+                                    dn, dr, dv, scale, window, sink_logits, gate, gate_stride, gate_channels, out_stride, 0, stream);
+}
+
+extern "C" int b2_window_attention_rows(void* out, const void* qn, int64_t qn_row, int qn_head, const void* qr, int64_t qr_row,
+                                        int qr_head, const void* kn, const void* kt, int64_t kt_row, const void* v,
+                                        const int32_t* cu_q, const int32_t* ctx_start, const int32_t* cu_k, const int32_t* k_lo,
+                                        int n_seq, int T, int H, int dn, int dr, int dv, float scale, int window,
+                                        const float* sink_logits, const void* gate, int64_t gate_stride, int gate_channels,
+                                        int64_t out_stride, int64_t n_keys, void* stream) {
     B2_REQUIRE(T >= 0 && n_seq >= 0 && H > 0 && dn >= 0 && dr >= 0 && dv > 0 && window >= 0, B2_EINVAL, "window_attention: bad sizes");
     B2_REQUIRE(dn % 8 == 0 && dr % 8 == 0 && (dn + dr) % 16 == 0 && dn + dr > 0 && dv % 16 == 0 && dv <= 16 * kWMaxDVT, B2_EUNSUPPORTED,
                "window_attention: head sizes %d + %d / %d", dn, dr, dv);
@@ -1151,10 +1161,14 @@ extern "C" int b2_window_attention(void* out, const void* qn, int64_t qn_row, in
     pa.scale = scale; pa.window = window;
     pa.sink = sink_logits ? 1.f : 0.f; pa.sink_logits = sink_logits;
     pa.gate = gate; pa.gate_stride = gate_stride; pa.gate_channels = gate_channels; pa.out = out; pa.out_stride = out_stride;
-    // The tcgen05 kernel's CTA is one an SM and takes 9 us from its start to its end with a single tile of keys; three CTAs of the other
-    // share an SM.  More than two waves of CTAs with fewer than 80 rows a sequence go to the other one: 64 x 40 rows, 16 heads 47 us
-    // against 62, 200 x 20 160 against 197, 30 x 64 30 against 35; 30 x 100 50 against 37, and one wave takes the same in both.
-    const bool many_short = (int64_t)T < 80 * (int64_t)n_seq && ((int64_t)T / 128 + n_seq) * H > 2 * (int64_t)latent_sm_count();
+    // The tcgen05 kernel's CTA is one an SM and takes 9 us from its start to its end with a single tile of keys; three CTAs of the other,
+    // whose tiles are 64 keys and not 128, share an SM.  More than two waves of CTAs with a tile of 64 keys a portion go to the other one,
+    // and portions of a few rows with up to 160.  16 heads, other / tcgen05 kernel: 64 x 40 rows without context 47 / 62 us, behind 100
+    // keys 85 / 76, behind 300 141 / 92; 200 x 20 162 / 197, behind 50 222 / 202; 30 x 64 31 / 35; 24 x 75 37 / 27; 100 x 8 57 / 95, behind
+    // 150 108 / 116, behind 200 131 / 117.  One wave takes the same in both.
+    const int64_t keys = n_keys > T ? n_keys : T;
+    const bool many_short = keys <= (T < 16 * (int64_t)n_seq ? 160 : 64) * (int64_t)n_seq &&
+                            ((int64_t)T / 128 + n_seq) * H > 2 * (int64_t)latent_sm_count();
     if (!many_short && b2_internal_prompt_tc5_ok(pa)) return b2_internal_prompt_tc5(pa, stream);
     const size_t smem = (size_t)((kWQ + kWK) * (dn + dr + 8) + kWK * (dv + 8)) * sizeof(__nv_bfloat16);
     B2_REQUIRE(smem <= 200 * 1024, B2_EUNSUPPORTED, "window_attention: key size %d too large", dn + dr);
