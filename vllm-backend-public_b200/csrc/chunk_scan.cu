@@ -9,7 +9,8 @@
 // Nothing above a diagonal is multiplied: a product that counts no later token must not become NaN by an infinity or NaN in one, so zeros
 // there are selected or left out, and a token's output depends on it and earlier ones alone, as in the scan token by token.
 // It is the same recurrence summed in another order (the WY form of Yang et al., "Parallelizing linear transformers with the
-// delta rule over sequence length", 2024).  Three kernels, only the second of which is a chain:
+// delta rule over sequence length", 2024).  One decay per head without delta goes to chunk_tc5.cu; the others are three kernels, only the
+// second of which is a chain:
 //   chunk_prep_kernel    P, T and the decay products; without delta also F = (G_C/G K)^T V: a CTA per (chunk, head)
 //   chunk_state_kernel   without delta: S <- G_C S + F over the chunks, element by element (memory bound)
 //   chunk_delta_kernel   with delta: U and S over the chunks, a CTA per (sequence, head, 16 columns of S)
@@ -99,6 +100,7 @@ __device__ __forceinline__ float4 scaled(const float4& v, float f) { return make
 template <bool CH, bool DELTA>
 __global__ void __launch_bounds__(NT)
 chunk_prep_kernel(const ChunkArgs a) {
+    static_assert(CH || DELTA, "chunk_tc5.cu");
     extern __shared__ __align__(16) float sm[];
     __shared__ int s_at[2];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, hh = blockIdx.y;
@@ -112,7 +114,7 @@ chunk_prep_kernel(const ChunkArgs a) {
     float* Ps = qs + (DELTA ? C * LD : max(C * LD, C * JB));        // [C][C + 1]
     float* As = Ps + C * (C + 1);                    // [C][C + 1] (delta)
     float* gs = As + (DELTA ? C * (C + 1) : 0);      // [C], per channel [C][LD]
-    float* bs = gs + (CH ? C * LD : C);              // [C] beta; per head without delta: G_C/G; per head 4 + C more
+    float* bs = gs + (CH ? C * LD : C);              // [C] beta; per head 4 + C more
     const int Cq = 2 * a.G * dk + a.H * dv, kvh = hh / (a.H / a.G);
     const float* qrow = a.qkv + (size_t)r0 * Cq + (size_t)kvh * dk;
     const float* krow = qrow + (size_t)a.G * dk;
@@ -272,19 +274,17 @@ chunk_prep_kernel(const ChunkArgs a) {
             for (int r = own * 16; r <= tid; ++r) from *= gs[r];
             dec[tid] = from;
             dec[C + tid] = to;
-            if (!DELTA) bs[tid] = to;
         }
         __syncthreads();
-        constexpr int RR = DELTA ? 8 : 4;
-        pair_t acc[RR][4];                           // sums over even and odd entries; blocks above the diagonal are left out
+        pair_t acc[8][4];                            // sums over even and odd entries; blocks above the diagonal are left out
 #pragma unroll
-        for (int r = 0; r < RR; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0;
+        for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0;
         for (int i = 0; i < dk; i += 4) {
             ulonglong2 kc[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) kc[c] = pairs(ks + (cg + 16 * c) * LD + i);
 #pragma unroll
-            for (int r = 0; r < RR; ++r) {
+            for (int r = 0; r < 8; ++r) {
                 const ulonglong2 x = pairs((r < 4 ? qs : ks) + (rg + 16 * (r & 3)) * LD + i);
 #pragma unroll
                 for (int c = 0; c <= (r & 3); ++c) {
@@ -294,7 +294,7 @@ chunk_prep_kernel(const ChunkArgs a) {
             }
         }
 #pragma unroll
-        for (int r = RR - 1; r >= 0; --r) {          // the k rows still need the ratios that the q rows overwrite (same thread)
+        for (int r = 7; r >= 0; --r) {          // the k rows still need the ratios that the q rows overwrite (same thread)
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int t = rg + 16 * (r & 3), x = cg + 16 * c;
@@ -360,11 +360,9 @@ chunk_prep_kernel(const ChunkArgs a) {
         const int ti = tid >> 4, tj = tid & 15;
         const float* vrow = a.qkv + (size_t)r0 * Cq + (size_t)2 * a.G * dk + (size_t)hh * dv;
         float* f0 = out + sc.s0;
-        if (CH) {                                    // the keys decayed to the chunk's end, from where they were just written
-            for (int idx = tid; idx < C * per; idx += NT) {
-                const int t = idx / per, c = (idx - t * per) * 4;
-                *reinterpret_cast<float4*>(ks + t * LD + c) = *reinterpret_cast<const float4*>(dec + (2 * C + t) * dk + c);
-            }
+        for (int idx = tid; idx < C * per; idx += NT) {              // the keys decayed to the chunk's end, from where they were just written
+            const int t = idx / per, c = (idx - t * per) * 4;
+            *reinterpret_cast<float4*>(ks + t * LD + c) = *reinterpret_cast<const float4*>(dec + (2 * C + t) * dk + c);
         }
         float* vs = qs;
         for (int j0 = 0; j0 < dv; j0 += JB) {
@@ -373,7 +371,7 @@ chunk_prep_kernel(const ChunkArgs a) {
                 const int t = idx / (JB / 4), c = (idx % (JB / 4)) * 4;
                 float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (t < nt && j0 + c < dv) v = *reinterpret_cast<const float4*>(vrow + (size_t)t * Cq + j0 + c);
-                *reinterpret_cast<float4*>(vs + t * JB + c) = CH ? v : scaled(v, bs[t]);
+                *reinterpret_cast<float4*>(vs + t * JB + c) = v;
             }
             __syncthreads();
             if (ti * 8 < dk) {
@@ -410,7 +408,6 @@ chunk_prep_kernel(const ChunkArgs a) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------- state, no delta
-template <bool CH>
 __global__ void __launch_bounds__(NT)
 chunk_state_kernel(const ChunkArgs a) {
     const int seq = blockIdx.x, hh = blockIdx.y;
@@ -420,10 +417,10 @@ chunk_state_kernel(const ChunkArgs a) {
     if (e >= dk * dv) return;
     const int nchunks = (a.cu_q[seq + 1] - a.cu_q[seq] + C - 1) / C;
     if (nchunks == 0) return;
-    const Scratch sc(dk, dv, CH, false);
+    const Scratch sc(dk, dv, true, false);
     const size_t step = (size_t)a.H * sc.total;
     float* w = a.ws + ((size_t)first_chunk(a, seq) * a.H + hh) * sc.total;
-    const float* g = w + sc.dec + (CH ? 3 * C * dk + e / dv : C - 1);                    // the chunk's whole product
+    const float* g = w + sc.dec + 3 * C * dk + e / dv;        // the chunk's whole product
     float* f = w + sc.s0 + e;
     const int slot = a.state_slot[seq];
     float* sp = slot >= 0 ? a.state + ((size_t)slot * a.H + hh) * dk * dv + e : nullptr;
@@ -797,7 +794,7 @@ int launch(const ChunkArgs& a, int total_rows, cudaStream_t st) {
         if (rc != B2_OK) return rc;
         chunk_delta_kernel<CH><<<grid, NT, fixed + stages * stage, st>>>(a, stages);
     } else {
-        chunk_state_kernel<CH><<<dim3(a.n_seq, a.H, (a.dk * a.dv / 4 + 127) / 128), 128, 0, st>>>(a);
+        chunk_state_kernel<<<dim3(a.n_seq, a.H, (a.dk * a.dv / 4 + 127) / 128), 128, 0, st>>>(a);
     }
     const size_t osm = sizeof(float) * (rows + C * LP + 2 * 32 * JB);
     rc = allow(chunk_out_kernel<CH, DELTA>, osm);
@@ -812,29 +809,38 @@ int launch(const ChunkArgs& a, int total_rows, cudaStream_t st) {
 // Scratch (floats) of the chunked form; 0 for sizes it is not built for and for scratch above 2 GiB
 int64_t b2_internal_chunk_scan_floats(int total_rows, int n_seq, int H, int dk, int dv, bool ch, bool delta) {
     if (dk % 4 || dv % 4 || dk > 128 || n_seq <= 0 || total_rows <= 0) return 0;
-    const int64_t n = (int64_t)(total_rows / C + n_seq) * H * Scratch(dk, dv, ch, delta).total;
+    const int64_t n = !ch && !delta ? b2_internal_chunk_tc5_floats(total_rows, n_seq, H, dk, dv)
+                                    : (int64_t)(total_rows / C + n_seq) * H * Scratch(dk, dv, ch, delta).total;
     return n <= (int64_t)1 << 29 ? n : 0;
 }
 
 // Where the chunked form is the faster one.  Both times are estimated in us from what they measured for heads of 128 x 128 on
 // one B200 (w = dk dv / 16384 scales the products); the host knows the rows and the number of sequences, so the longest of several is taken to be 1.25 times the mean:
 //   tokens   a chain of 0.20 (delta 0.285, per channel 0.235 / 0.31) a token, or, with several sequences, 5.2 (7.1 / 10.6 / 12.4) ns a
-//            token and head, down to 5.0 (6.3 / 6.8 / 8.3) from 64 sequences on
-//   chunks   0.23 (0.16 / 0.55 / 0.70) a chunk and head for the products, 0.11 a sequence and head for its state, with delta 4.8 a
-//            step of the chain and SM's share of CTAs; at least 40 (80 per channel, 110 with delta too): three launches
-// Measured, tokens -> chunks: 1 x 4096 tokens, 16 heads: 804 -> 250, 1160 -> 470, 963 -> 572, 1254 -> 1006; 1 x 500: 101 -> 43,
-// 146 -> 74, 121 -> 82, 158 -> 144; 64 x 64: 328 -> 377, 413 -> 567: left to the tokens, as are 64 x 24: 147 -> 317.
+//            token and head, down to 5.0 (6.3 / 6.8 / 8.3) from 64 sequences on; keys of other sizes than 32, 64, 128 run as the next one, a third slower
+//   chunks   one decay per head without delta (chunk_tc5.cu): 20, 0.2 a chunk of 128 and head for the products (0.14 at 64 x 64) and 0.03 a
+//            sequence and head for its state; at least 33 (29 to dk = 64): three launches
+//            else 0.16 (per channel 0.55 / 0.70) a chunk of 64 and head for the products, 0.11 a sequence and head for its state, with delta
+//            4.8 a step of the chain and SM's share of CTAs; at least 40 (80 per channel, 110 with delta too)
+// Measured, tokens -> chunks: 1 x 4096 tokens, 16 heads: 804 -> 121, 1160 -> 470, 963 -> 572, 1254 -> 1006; 1 x 500: 102 -> 34,
+// 146 -> 74, 121 -> 82, 158 -> 144; 16 x 100: 121 -> 74 the first; 64 x 64: 330 -> 258, 413 -> 567: the second is left to the tokens, as are 64 x 24: 148 -> 250,
+// 147 -> 317, and 1 x 130: 29 -> 33 the first.
 bool b2_internal_chunk_scan_pays(int total_rows, int n_seq, int H, int dk, int dv, bool ch, bool delta) {
     if (total_rows < 2 * n_seq) return false;
     const float len = (float)total_rows / n_seq, w = dk * dv / 16384.f, steps = ceilf(len / C), heads = (float)n_seq * H;
-    const int kind = (ch ? 2 : 0) + (delta ? 1 : 0);
+    const int kind = (ch ? 2 : 0) + (delta ? 1 : 0), run_as = dk <= 32 ? 32 : dk <= 64 ? 64 : 128;
     const float chain_tok[4] = {0.20f, 0.285f, 0.235f, 0.31f}, rate_few[4] = {5.2e-3f, 7.1e-3f, 10.6e-3f, 12.4e-3f}, rate_many[4] = {5.0e-3f, 6.3e-3f, 6.8e-3f, 8.3e-3f};
-    const float per_chunk[4] = {0.23f, 0.16f, 0.55f, 0.70f}, least[4] = {40.f, 40.f, 80.f, 110.f};
+    const float per_chunk[4] = {0.f, 0.16f, 0.55f, 0.70f}, least[4] = {dk <= 64 ? 29.f : 33.f, 40.f, 80.f, 110.f};
     const float many = fminf(1.f, fmaxf(0.f, log2f(n_seq / 4.f) / 4.f)), rate = rate_few[kind] + (rate_many[kind] - rate_few[kind]) * many;
     const float longest = len * (n_seq > 1 ? 1.25f : 1.f);
-    const float tokens = fmaxf(chain_tok[kind] * (dk <= 64 ? 0.75f : 1.f) * longest, rate * (float)total_rows * H * w);
-    float chunks = (per_chunk[kind] * (0.35f + 0.65f * w) * steps + 0.11f * w) * heads;
-    if (delta) chunks += (3.4f + 1.4f * w) * fmaxf(ceilf(longest / C), steps * heads * ((dv + NC - 1) / NC) / b2_sm_count());
+    const float tokens = (run_as == dk ? 1.f : 1.33f) * fmaxf(chain_tok[kind] * (dk <= 64 ? 0.75f : 1.f) * longest, rate * (float)total_rows * H * run_as * dv / 16384.f);
+    float chunks;
+    if (kind == 0) {
+        chunks = 20.f + (0.2f * (0.6f + 0.4f * w) * ceilf(len / 128) + 0.03f * w) * heads;
+    } else {
+        chunks = (per_chunk[kind] * (0.35f + 0.65f * w) * steps + 0.11f * w) * heads;
+        if (delta) chunks += (3.4f + 1.4f * w) * fmaxf(ceilf(longest / C), steps * heads * ((dv + NC - 1) / NC) / b2_sm_count());
+    }
     return tokens >= fmaxf(chunks, least[kind]);
 }
 
@@ -844,5 +850,6 @@ int b2_internal_chunk_scan(const float* qkv, const float* beta, const float* dec
     const ChunkArgs a{qkv, beta, decay, H, G, dk, dv, n_seq, cu_q, ctx_start, state_slot, state, o, ws};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (ch) return delta ? launch<true, true>(a, total_rows, st) : launch<true, false>(a, total_rows, st);
-    return delta ? launch<false, true>(a, total_rows, st) : launch<false, false>(a, total_rows, st);
+    if (!delta) return b2_internal_chunk_tc5(qkv, decay, total_rows, H, G, dk, dv, cu_q, ctx_start, state_slot, n_seq, state, o, ws, stream);
+    return launch<false, true>(a, total_rows, st);
 }
