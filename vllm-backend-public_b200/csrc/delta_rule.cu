@@ -138,7 +138,7 @@ __global__ void recur_prep_kernel(const T* __restrict__ proj, int64_t proj_strid
 // and not eight: 64 registers let four CTAs share an SM, and a warp's stores are 512 consecutive bytes.
 // Bound: memory (2 or 4 bytes in and 4 out per channel), with the exact exponentials and divisions of the activation close behind.
 // One CTA a row with scalar accesses and a staging pass took 88 us at 4096 rows of 6144 channels (rotation, no convolution), 174 at 3001
-// rows (four taps, SiLU, unit vectors) and 59 at 64 rows; this one 58, 63 and 27.
+// rows (four taps, SiLU, unit vectors) and 59 at 64 rows; this one 58, 63 and 27.  Without a convolution recur_prep_heads_kernel takes prompts.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(256, 4)
 recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec sp, const float* __restrict__ conv_w,
@@ -300,6 +300,120 @@ recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec 
         if (sp.off_beta >= 0) beta[(size_t)row * H + hh] = b2::sigmoid_f(b2::ld(pr + sp.off_beta + hh));
         if (sp.decay_mode == B2_DECAY_HEAD_SOFTPLUS)
             decay[(size_t)row * H + hh] = expf(-expf(sp.A_log[hh]) * b2::softplus_f(b2::ld(pr + sp.off_a + hh) + sp.bias[hh]));
+        else if (sp.decay_mode == B2_DECAY_HEAD_CONST)
+            decay[(size_t)row * H + hh] = sp.bias[hh];
+    }
+}
+
+// The same without a convolution: nothing depends on the row before, so a thread goes over the heads of its row and not over rows.
+// It keeps its place in the head, and with it the cosines and sines of the row; four heads and the values after them are in flight at
+// once.  ROT: 0 no rotation, 1 pairs (i, i + rot_dims / 2), 2 neighbours.
+// Bound: memory (150 MB of 4096 rows of 6144 channels: 23 us); by rows with everything that a row may need, 143 instructions a vector of
+// four channels and 57 us, this one 33 (a decay per channel, SiLU and unit vectors 94 -> 65).
+template <typename T, int ROT, bool UNIT>
+__global__ void __launch_bounds__(256, 5)
+recur_prep_heads_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec sp, const float* __restrict__ conv_w,
+                        const int32_t* __restrict__ cu_q, const int32_t* __restrict__ ctx_start, int n_seq, float* __restrict__ qkv,
+                        float* __restrict__ beta, float* __restrict__ decay) {
+    constexpr int AHEAD = 4;
+    const int H = sp.H, G = sp.G, dk = sp.dk, qk = 2 * G * dk, C = qk + H * sp.dv, row = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const int seq = b2::seq_of_row(cu_q, n_seq, row), ctx = ctx_start[seq];
+    if (ctx < 0) return;
+    const T* src = proj + (size_t)row * proj_stride;
+    float* dst = qkv + (size_t)row * C;
+    const int P = dk / 4, i0 = tid % P * 4, half = sp.rot_dims / 2, step = 1024;               // P divides 32: a thread keeps its place
+    const bool turns = ROT && i0 < sp.rot_dims, second = ROT == 1 && i0 >= half;
+    float co[4], si[4];
+    if (turns) {
+        const float* cs = sp.cos_sin + (size_t)min(ctx + row - cu_q[seq], sp.max_pos - 1) * sp.rot_dims;
+        if (ROT == 1) {
+            const int pr = second ? i0 - half : i0;
+            b2::ld4(cs + pr, co);
+            b2::ld4(cs + half + pr, si);
+            if (!second) { si[0] = -si[0]; si[1] = -si[1]; si[2] = -si[2]; si[3] = -si[3]; }
+        } else {
+            const float2 c2 = *reinterpret_cast<const float2*>(cs + i0 / 2), s2 = *reinterpret_cast<const float2*>(cs + half + i0 / 2);
+            co[0] = c2.x; co[1] = c2.y; si[0] = s2.x; si[1] = s2.y;
+        }
+    }
+    auto raw = [&](int c0, float (&x)[4]) {
+        if (conv_w) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) x[c] *= conv_w[c0 + c];
+        }
+        if (sp.act) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) x[c] = b2::silu_f(x[c]);
+        }
+    };
+    // q and k heads: whole warps take part in the shuffles, past the last head with zeros
+    for (int first = tid * 4; first - lane * 4 < qk; first += AHEAD * step) {
+        float x[AHEAD][4];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            x[u][0] = x[u][1] = x[u][2] = x[u][3] = 0.f;
+            if (first + u * step < qk) b2::ld4(src + first + u * step, x[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            const int c0 = first + u * step;
+            if (c0 - lane * 4 >= qk) break;
+            if (c0 < qk) raw(c0, x[u]);
+            float sc = c0 < G * dk ? sp.q_scale : sp.k_scale;
+            if (UNIT) {
+                float ss = 0.f;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) ss = fmaf(x[u][c], x[u][c], ss);
+                for (int m = 1; m < P; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+                sc *= rsqrtf(ss + sp.unit_eps);
+            }
+            if (ROT == 1) {
+                const int from = turns ? (second ? lane - half / 4 : lane + half / 4) : lane;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float y = __shfl_sync(0xffffffffu, x[u][c], from);
+                    if (turns) x[u][c] = fmaf(x[u][c], co[c], y * si[c]);
+                }
+            } else if (ROT == 2 && turns) {
+#pragma unroll
+                for (int c = 0; c < 4; c += 2) {
+                    const float a = x[u][c], b = x[u][c + 1];
+                    x[u][c] = fmaf(a, co[c / 2], -b * si[c / 2]);
+                    x[u][c + 1] = fmaf(b, co[c / 2], a * si[c / 2]);
+                }
+            }
+            if (c0 < qk) *reinterpret_cast<float4*>(dst + c0) = make_float4(x[u][0] * sc, x[u][1] * sc, x[u][2] * sc, x[u][3] * sc);
+        }
+    }
+    for (int first = qk + tid * 4; first < C; first += AHEAD * 1024) {
+        float x[AHEAD][4];
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+            if (first + u * 1024 < C) b2::ld4(src + first + u * 1024, x[u]);
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+            if (first + u * 1024 < C) {
+                raw(first + u * 1024, x[u]);
+                *reinterpret_cast<float4*>(dst + first + u * 1024) = make_float4(x[u][0], x[u][1], x[u][2], x[u][3]);
+            }
+    }
+    if (sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS || sp.decay_mode == B2_DECAY_CHANNEL_SIGMOID_POW) {
+        for (int d0 = tid * 4; d0 < H * dk; d0 += 1024) {
+            float z[4];
+            b2::ld4(sp.a + (size_t)row * sp.a_stride + d0, z);
+            const float rate = sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS ? -expf(sp.A_log[d0 / dk]) : 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                z[c] += sp.bias ? sp.bias[d0 + c] : 0.f;
+                z[c] = sp.decay_mode == B2_DECAY_CHANNEL_SOFTPLUS ? expf(rate * b2::softplus_f(z[c])) : expf(-b2::softplus_f(-z[c]) * sp.inv_tau);
+            }
+            *reinterpret_cast<float4*>(decay + (size_t)row * H * dk + d0) = make_float4(z[0], z[1], z[2], z[3]);
+        }
+    }
+    for (int hh = tid; hh < H; hh += 256) {
+        if (sp.off_beta >= 0) beta[(size_t)row * H + hh] = b2::sigmoid_f(b2::ld(src + sp.off_beta + hh));
+        if (sp.decay_mode == B2_DECAY_HEAD_SOFTPLUS)
+            decay[(size_t)row * H + hh] = expf(-expf(sp.A_log[hh]) * b2::softplus_f(b2::ld(src + sp.off_a + hh) + sp.bias[hh]));
         else if (sp.decay_mode == B2_DECAY_HEAD_CONST)
             decay[(size_t)row * H + hh] = sp.bias[hh];
     }
@@ -767,11 +881,18 @@ int launch_prep(const void* proj, int64_t proj_stride, const PrepSpec& sp, int T
 #define B2_PREP_VEC(TAPS)                                                                                                    \
     recur_prep_vec_kernel<A, TAPS><<<grid, 256, 0, st>>>(static_cast<const A*>(proj), proj_stride, sp, conv_w, cu_q, ctx_start, state_slot, \
                                                          n_seq, T, run, static_cast<const A*>(conv_state), qkv, beta, decay)
-        if (sp.taps == 1) B2_PREP_VEC(1);
+#define B2_PREP_HEADS(ROT, UNIT)                                                                                             \
+    recur_prep_heads_kernel<A, ROT, UNIT><<<T, 256, 0, st>>>(static_cast<const A*>(proj), proj_stride, sp, conv_w, cu_q, ctx_start, n_seq, qkv, beta, decay)
+        if (sp.taps == 1 && T >= 256) {              // below it the columns of a row have to be spread: 64 rows 4.3 - 6.3 us by rows, 6.3 - 8.4 by heads
+            const int rot = sp.rot_dims == 0 ? 0 : sp.interleaved ? 2 : 1;
+            if (sp.unit) { if (rot == 0) B2_PREP_HEADS(0, true); else if (rot == 1) B2_PREP_HEADS(1, true); else B2_PREP_HEADS(2, true); }
+            else { if (rot == 0) B2_PREP_HEADS(0, false); else if (rot == 1) B2_PREP_HEADS(1, false); else B2_PREP_HEADS(2, false); }
+        } else if (sp.taps == 1) B2_PREP_VEC(1);
         else if (sp.taps == 2) B2_PREP_VEC(2);
         else if (sp.taps == 3) B2_PREP_VEC(3);
         else B2_PREP_VEC(4);
 #undef B2_PREP_VEC
+#undef B2_PREP_HEADS
     } else {
         auto kern = recur_prep_kernel<A>;
         if (smem > 48 * 1024) B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
