@@ -88,25 +88,26 @@ def test_chunked_scan(cuda, lens, ctx, slots, H, G, dk, dv, decay, delta, per_ch
         assert e_new < 2e-6 and e_new <= 2.0 * e_old + 1e-7, (e_new, e_old)
 
 
+@pytest.mark.parametrize("delta,per_channel", [(False, False), (True, False), (False, True), (True, True)])
 @pytest.mark.parametrize("lens,H,G,dk,dv", [
     ([127, 128, 129, 256, 1], 16, 16, 128, 128),                         # edges of a chunk of 128 tokens
     ([2100], 16, 4, 64, 136),                                            # more items than SMs; two blocks of columns, the second of eight
     ([9] * 40 + [300] + [2] * 30, 2, 2, 68, 12),                         # more sequences than lanes; one feature past a slice
     ([520, 33], 8, 8, 124, 260),
 ])
-def test_chunked_scan_sizes(cuda, lens, H, G, dk, dv):
-    """One decay per head, no delta: the chunked form on the tensor cores, whose sums are those of test_chunked_scan."""
+def test_chunked_scan_sizes(cuda, lens, H, G, dk, dv, delta, per_channel):
+    """Sizes at which the kernels on the tensor cores go on to another item, block or slice; the bound is test_chunked_scan's."""
     n, T = len(lens), sum(lens)
-    qkv, _, dec, state = _inputs(cuda, lens, H, G, dk, dv, False, False, "mild", seed=T + dk)
+    qkv, beta, dec, state = _inputs(cuda, lens, H, G, dk, dv, per_channel, delta, "mild", seed=T + dk)
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
     cu, ctx, slots = [0], [(5 * i) % 3 for i in range(n)], list(range(n))
     for m in lens:
         cu.append(cu[-1] + m)
-    st, o, ws = state.clone(), torch.zeros(T, H, dv, device=cuda), torch.empty(1 << 26, device=cuda)
+    st, o, ws = state.clone(), torch.zeros(T, H, dv, device=cuda), torch.empty(1 << 27, device=cuda)
     keep = i32(cu), i32(ctx), i32(slots)
-    _lib.check(_lib.load().b2_channel_scan_ws(qkv.data_ptr(), None, dec.data_ptr(), T, H, G, dk, dv, 0, 0, *(x.data_ptr() for x in keep), n, st.data_ptr(),
-                                              o.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
-    ref, st_ref = _reference(qkv, None, dec, state, lens, ctx, slots, H, G, dk, dv)
+    _lib.check(_lib.load().b2_channel_scan_ws(qkv.data_ptr(), beta.data_ptr() if delta else None, dec.data_ptr(), T, H, G, dk, dv, int(per_channel),
+                                              int(delta), *(x.data_ptr() for x in keep), n, st.data_ptr(), o.data_ptr(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
+    ref, st_ref = _reference(qkv, beta, dec, state, lens, ctx, slots, H, G, dk, dv)
     assert float((o.double() - ref).norm() / ref.norm()) < 2e-6 and float((st.double() - st_ref).norm() / st_ref.norm()) < 2e-6
 
 

@@ -22,108 +22,11 @@ using namespace chunk_tc5;
 
 constexpr int CS = 128, NT = 512, SMEM = 12 * PART + 1024;
 
-struct Args {
-    const float *qkv, *decay;
-    int H, G, dk, dv, n_seq, blocks, items;          // blocks of 128 columns; items = chunks (an upper bound) x heads x blocks
-    const int32_t *cu_q, *ctx_start, *state_slot;
-    float *state, *o, *ws;
-};
 // Scratch of a (chunk, head), in floats: G_C | F | S_0 as out_kernel's operand: the parts of 64 rows x 128 columns after one another, per
 // block of the columns and slice of the rows.  All three start on 128 bytes.
 constexpr int F_AT = 32;
 __host__ __device__ constexpr int image(int dk, int dv) { return F_AT + (dk * dv + 31) / 32 * 32; }
 __host__ __device__ constexpr int scratch(int dk, int dv) { return image(dk, dv) + (dk + 63) / 64 * ((dv + 127) / 128) * (3 * PART / 4); }
-
-// Where an item lies.  The whole warp works.
-struct At {
-    int row, nt, chunk, head, block, fresh;          // first row, rows (0: none, and none follow), fresh: the state before it is zero
-};
-__device__ __forceinline__ At locate(const Args& a, int item) {
-    At at{0, 0, 0, 0, 0, 0};
-    if (item >= a.items) return at;
-    const int lane = threadIdx.x & 31, hz = a.H * a.blocks;
-    at.chunk = item / hz;
-    at.head = (item - at.chunk * hz) / a.blocks;
-    at.block = (item - at.chunk * hz) % a.blocks;
-    int want = at.chunk;
-    for (int s0 = 0; s0 < a.n_seq; s0 += 32) {
-        int lo = 0, len = 0, ctx = -1;
-        if (s0 + lane < a.n_seq) {
-            lo = a.cu_q[s0 + lane];
-            ctx = a.ctx_start[s0 + lane];
-            len = ctx < 0 ? 0 : a.cu_q[s0 + lane + 1] - lo;
-        }
-        const int own = (len + CS - 1) / CS;
-        int c = own;                                 // chunks up to this sequence's last
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, c, d);
-            if (lane >= d) c += u;
-        }
-        const unsigned has = __ballot_sync(0xffffffffu, want < c);
-        if (has) {
-            const int src = __ffs(has) - 1, in = want - __shfl_sync(0xffffffffu, c - own, src);
-            at.row = __shfl_sync(0xffffffffu, lo, src) + in * CS;
-            at.nt = min(CS, __shfl_sync(0xffffffffu, len, src) - in * CS);
-            at.fresh = in == 0 && __shfl_sync(0xffffffffu, ctx, src) == 0;
-            return at;
-        }
-        want -= __shfl_sync(0xffffffffu, c, 31);
-    }
-    return at;
-}
-
-// Products of neighbours in a warp: up to the lane, from the lane on, of all.  In 64 bits: a tree of products squares its rounding errors
-// where the decays are alike (a fixed decay per head: 0.9961^128 off by 2e-6, the state of 4096 tokens by 6.8e-7; 1.5e-7 so, 4.1e-7 with chains)
-__device__ __forceinline__ double product_up_to(double g) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const double u = __shfl_up_sync(0xffffffffu, g, d);
-        if ((threadIdx.x & 31) >= d) g *= u;
-    }
-    return g;
-}
-__device__ __forceinline__ double product_from(double g) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const double u = __shfl_down_sync(0xffffffffu, g, d);
-        if ((threadIdx.x & 31) + d < 32) g *= u;
-    }
-    return g;
-}
-__device__ __forceinline__ double product_of_all(double g) {
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) g *= __shfl_xor_sync(0xffffffffu, g, d);
-    return g;
-}
-
-// What this warp wrote to shared memory and read from TMEM is handed over; true (in all lanes) in the last of the CTA's warps to do so
-__device__ __forceinline__ bool hand_over(unsigned* count) {
-    b2::fence_proxy_async();
-    tc_fence_before();
-    __syncwarp();
-    unsigned before = 0;
-    if ((threadIdx.x & 31) == 0) asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(b2::smem_u32(count)) : "memory");
-    const bool last = (__shfl_sync(0xffffffffu, before, 0) & 15) == 15;
-    if (last) tc_fence_after();
-    return last;
-}
-__device__ __forceinline__ uint32_t tmem_alloc(uint32_t* at, int warp) {         // all 512 columns; the whole CTA
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(b2::smem_u32(at)) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    return *at;
-}
-__device__ __forceinline__ void tmem_free(uint32_t tmem, int warp) {
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
-}
 
 // ---------------------------------------------------------------------------------------------------------------- F
 // Two slices of 64 tokens, each with its own tiles of V and K and its own accumulator; while one is multiplied, the next is split,
@@ -136,7 +39,7 @@ kv_kernel(const Args a) {
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    At at = locate(a, blockIdx.x);
+    At at = locate<CS>(a, blockIdx.x);
     if (at.nt == 0) return;
     const uint32_t sm = (b2::smem_u32(sm_raw) + 1023u) & ~1023u;
     unsigned char* const gen = sm_raw + (sm - b2::smem_u32(sm_raw));
@@ -222,7 +125,7 @@ kv_kernel(const Args a) {
             __syncwarp();
             if (u == 0) {
                 load(at, 1);
-                next = locate(a, item += gridDim.x);
+                next = locate<CS>(a, item += gridDim.x);
                 if (n > 0) finish();
             } else if (next.nt > 0) {
                 load(next, 0);
@@ -272,15 +175,7 @@ state_kernel(const Args a) {
         for (int u = 0; u < AHEAD; ++u) {
             const int c = c0 + u;
             if (c < nchunks) {
-                uint32_t m[4], l[4];
-                split(s.x, m[0], l[0]);
-                split(s.y, m[1], l[1]);
-                split(s.z, m[2], l[2]);
-                split(s.w, m[3], l[3]);
-                unsigned char* dst = to + (size_t)c * step * 4;
-                *reinterpret_cast<uint2*>(dst) = make_uint2(tops(__float_as_uint(s.x), __float_as_uint(s.y)), tops(__float_as_uint(s.z), __float_as_uint(s.w)));
-                *reinterpret_cast<uint2*>(dst + PART) = make_uint2(tops(m[0], m[1]), tops(m[2], m[3]));
-                *reinterpret_cast<uint2*>(dst + 2 * PART) = make_uint2(tops(l[0], l[1]), tops(l[2], l[3]));
+                store_parts4(to + (size_t)c * step * 4, PART, s);
                 if (pad) continue;
                 s = make_float4(fmaf(s.x, d[u], x[u].x), fmaf(s.y, d[u], x[u].y), fmaf(s.z, d[u], x[u].z), fmaf(s.w, d[u], x[u].w));
                 if (c + AHEAD < nchunks) {
@@ -305,7 +200,7 @@ out_kernel(const Args a) {
     __shared__ int s_failed, s_again;                // s_again: number of the last item (from 1) with a result that was not finite
     __shared__ int s_bad_from[128];                  // first token whose value in this column is not finite
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    At at = locate(a, blockIdx.x);
+    At at = locate<CS>(a, blockIdx.x);
     if (at.nt == 0) return;
     const uint32_t sm = (b2::smem_u32(sm_raw) + 1023u) & ~1023u, q_sm = sm + 6 * PART;
     unsigned char* const gen = sm_raw + (sm - b2::smem_u32(sm_raw)), * const qb = gen + 6 * PART;
@@ -441,7 +336,7 @@ out_kernel(const Args a) {
             __syncwarp();
         };
         if (hand_over(&s_full[3])) values();
-        const At next = locate(a, item += gridDim.x);
+        const At next = locate<CS>(a, item += gridDim.x);
         if (next.nt > 0) load_q(next);
         const int j = at.block * 128 + qd * 32 + lane;
 #pragma unroll 1
@@ -516,7 +411,7 @@ int64_t b2_internal_chunk_tc5_floats(int total_rows, int n_seq, int H, int dk, i
 int b2_internal_chunk_tc5(const float* qkv, const float* decay, int total_rows, int H, int G, int dk, int dv, const int32_t* cu_q,
                           const int32_t* ctx_start, const int32_t* state_slot, int n_seq, float* state, float* o, float* ws, void* stream) {
     const int blocks = (dv + 127) / 128, items = (total_rows / CS + n_seq) * H * blocks;
-    const Args a{qkv, decay, H, G, dk, dv, n_seq, blocks, items, cu_q, ctx_start, state_slot, state, o, ws};
+    const Args a{qkv, nullptr, decay, H, G, dk, dv, n_seq, blocks, items, cu_q, ctx_start, state_slot, state, o, ws};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     B2_CUDA_OK(cudaFuncSetAttribute(kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     B2_CUDA_OK(cudaFuncSetAttribute(out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));

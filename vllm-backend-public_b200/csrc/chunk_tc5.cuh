@@ -1,10 +1,11 @@
 // chunk_tc5.cuh -- fp32 products on the bf16 tensor cores, as the chunked recurrence uses them.
 //
-// A float is the sum of three bf16 numbers (its leading 8 bits, the next 8, the last 8: truncation, so exact), and a product of two
-// floats is six of the nine products of their parts: what is left out is below 2^-22 of it.  Products of parts are exact in fp32, but
+// A float is the sum of three bf16 numbers (its rounding to 8 bits, that of the rest, and what is left: exact), and a product of two
+// floats is six of the nine products of their parts: what is left out is below 2^-25 of it.  (Parts by truncation instead of rounding
+// take as many instructions and are all of one sign: errors a third higher.)  Products of parts are exact in fp32, but
 // the tensor core truncates its accumulator at every instruction, so the leading parts' products have an accumulator of their own, which
 // takes one addition per 16 entries, or the small products come first.  Sums of 128 products of normal numbers against 64 bits, relative to
-// the result's norm: 1.6e-7 with two accumulators, 1.3e-7 with one per 64 entries and the small products first, 9.8e-7 with one for all;
+// the result's norm: 1.2e-7 with two accumulators, 0.8e-7 with one per 64 entries and the small products first, 8.2e-7 with one for all;
 // a chain of 128 FMAs 2.0e-7.
 //
 // Operands are tiles of 128-byte rows in the 128-byte swizzle: rows of 64 entries of the summed index (K-major), or rows of 64 entries of
@@ -17,23 +18,32 @@
 namespace chunk_tc5 {
 using namespace b2tc;
 
-// two floats' leading 16 bits
-__device__ __forceinline__ uint32_t tops(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
-// what x's leading part leaves, and what that one's leaves; the leading parts are the upper halves of x and m
-__device__ __forceinline__ void split(float x, uint32_t& m, uint32_t& l) {
-    const float r = x - __uint_as_float(__float_as_uint(x) & 0xffff0000u);
-    m = __float_as_uint(r);
-    l = __float_as_uint(r - __uint_as_float(m & 0xffff0000u));
+// two floats -> their parts, packed
+__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    hi = b2::pack_bf16x2(x, y);
+    x -= __uint_as_float(hi << 16);
+    y -= __uint_as_float(hi & 0xffff0000u);
+    mid = b2::pack_bf16x2(x, y);
+    lo = b2::pack_bf16x2(x - __uint_as_float(mid << 16), y - __uint_as_float(mid & 0xffff0000u));
 }
 struct Split8 { uint4 hi, mid, lo; };
 // eight floats -> their parts, packed in order
 __device__ __forceinline__ Split8 split8(const float (&x)[8]) {
-    uint32_t m[8], l[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) split(x[i], m[i], l[i]);
-    auto x2 = [&](int i) { return tops(__float_as_uint(x[i]), __float_as_uint(x[i + 1])); };
-    return {make_uint4(x2(0), x2(2), x2(4), x2(6)), make_uint4(tops(m[0], m[1]), tops(m[2], m[3]), tops(m[4], m[5]), tops(m[6], m[7])),
-            make_uint4(tops(l[0], l[1]), tops(l[2], l[3]), tops(l[4], l[5]), tops(l[6], l[7]))};
+    Split8 s;
+    split2(x[0], x[1], s.hi.x, s.mid.x, s.lo.x);
+    split2(x[2], x[3], s.hi.y, s.mid.y, s.lo.y);
+    split2(x[4], x[5], s.hi.z, s.mid.z, s.lo.z);
+    split2(x[6], x[7], s.hi.w, s.mid.w, s.lo.w);
+    return s;
+}
+// four floats -> 8 bytes of each part, `part_bytes` apart
+__device__ __forceinline__ void store_parts4(unsigned char* dst, int part_bytes, const float4& x) {
+    uint2 hi, mid, lo;
+    split2(x.x, x.y, hi.x, mid.x, lo.x);
+    split2(x.z, x.w, hi.y, mid.y, lo.y);
+    *reinterpret_cast<uint2*>(dst) = hi;
+    *reinterpret_cast<uint2*>(dst + part_bytes) = mid;
+    *reinterpret_cast<uint2*>(dst + 2 * part_bytes) = lo;
 }
 __device__ __forceinline__ void store_parts(unsigned char* dst, int part_bytes, const Split8& s) {
     *reinterpret_cast<uint4*>(dst) = s.hi;
@@ -97,6 +107,20 @@ __device__ __forceinline__ void mma_parts(uint32_t d, uint32_t a_lo, uint32_t b_
     }
 }
 
+// The same with 64 columns: D (three accumulators of 64 columns: products of the parts' order 0, 1, 2) += A B over `ksteps` times 16
+// entries, the parts of B side by side as 192 columns.  A_PART: bytes from one part of A to the next.
+template <int A_PART, int AK, int BK>
+__device__ __forceinline__ void mma_orders(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t majors, int ksteps, bool acc) {
+    const uint32_t n64 = idesc_bf16(128, 64, 0) | majors, n128 = idesc_bf16(128, 128, 0) | majors, n192 = idesc_bf16(128, 192, 0) | majors;
+#pragma unroll 1
+    for (int k = 0; k < ksteps; ++k) {
+        const uint64_t b = desc_join(b_lo + k * BK);
+        mma_ss(d, desc_join(a_lo + k * AK), b, n192, acc || k > 0);
+        mma_ss(d + 64, desc_join(a_lo + k * AK + (A_PART >> 4)), b, n128, true);
+        mma_ss(d + 128, desc_join(a_lo + k * AK + (2 * A_PART >> 4)), b, n64, true);
+    }
+}
+
 // 32 lanes x 8 columns
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&r)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -126,7 +150,115 @@ __device__ __forceinline__ void read_parts(uint32_t d, float (&s)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) s[i] += r[i];
 }
+__device__ __forceinline__ void read_orders(uint32_t d, float (&s)[16]) {         // the three accumulators of mma_orders, the smallest first
+    float r[16], q[16];
+    tmem_ld16(d + 128, s);
+    tmem_ld16(d + 64, r);
+    tmem_ld16(d, q);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s[i] = (s[i] + r[i]) + q[i];
+}
 __device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+
+struct Args {
+    const float *qkv, *beta, *decay;
+    int H, G, dk, dv, n_seq, blocks, items;          // blocks of 128 columns; items = chunks (an upper bound) x heads x blocks
+    const int32_t *cu_q, *ctx_start, *state_slot;
+    float *state, *o, *ws;
+};
+
+// Where an item lies.  The whole warp works.
+struct At {
+    int row, nt, chunk, head, block, fresh;          // first row, rows (0: none, and none follow), fresh: the state before it is zero
+};
+template <int TILE>
+__device__ __forceinline__ At locate(const Args& a, int item) {
+    At at{0, 0, 0, 0, 0, 0};
+    if (item >= a.items) return at;
+    const int lane = threadIdx.x & 31, hz = a.H * a.blocks;
+    at.chunk = item / hz;
+    at.head = (item - at.chunk * hz) / a.blocks;
+    at.block = (item - at.chunk * hz) % a.blocks;
+    int want = at.chunk;
+    for (int s0 = 0; s0 < a.n_seq; s0 += 32) {
+        int lo = 0, len = 0, ctx = -1;
+        if (s0 + lane < a.n_seq) {
+            lo = a.cu_q[s0 + lane];
+            ctx = a.ctx_start[s0 + lane];
+            len = ctx < 0 ? 0 : a.cu_q[s0 + lane + 1] - lo;
+        }
+        const int own = (len + TILE - 1) / TILE;
+        int c = own;                                 // chunks up to this sequence's last
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, c, d);
+            if (lane >= d) c += u;
+        }
+        const unsigned has = __ballot_sync(0xffffffffu, want < c);
+        if (has) {
+            const int src = __ffs(has) - 1, in = want - __shfl_sync(0xffffffffu, c - own, src);
+            at.row = __shfl_sync(0xffffffffu, lo, src) + in * TILE;
+            at.nt = min(TILE, __shfl_sync(0xffffffffu, len, src) - in * TILE);
+            at.fresh = in == 0 && __shfl_sync(0xffffffffu, ctx, src) == 0;
+            return at;
+        }
+        want -= __shfl_sync(0xffffffffu, c, 31);
+    }
+    return at;
+}
+
+// Products of neighbours in a warp: up to the lane, from the lane on, of all.  In 64 bits: a tree of products squares its rounding errors
+// where the decays are alike (a fixed decay per head: 0.9961^128 off by 2e-6, the state of 4096 tokens by 6.8e-7; 1.5e-7 so, 4.1e-7 with chains)
+__device__ __forceinline__ double product_up_to(double g) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const double u = __shfl_up_sync(0xffffffffu, g, d);
+        if ((threadIdx.x & 31) >= d) g *= u;
+    }
+    return g;
+}
+__device__ __forceinline__ double product_from(double g) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const double u = __shfl_down_sync(0xffffffffu, g, d);
+        if ((threadIdx.x & 31) + d < 32) g *= u;
+    }
+    return g;
+}
+__device__ __forceinline__ double product_of_all(double g) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) g *= __shfl_xor_sync(0xffffffffu, g, d);
+    return g;
+}
+
+// What this warp wrote to shared memory and read from TMEM is handed over; true (in all lanes) in the last of the CTA's warps to do so
+__device__ __forceinline__ bool hand_over(unsigned* count) {
+    b2::fence_proxy_async();
+    tc_fence_before();
+    __syncwarp();
+    unsigned before = 0;
+    if ((threadIdx.x & 31) == 0) asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(before) : "r"(b2::smem_u32(count)) : "memory");
+    const bool last = (__shfl_sync(0xffffffffu, before, 0) & 15) == 15;
+    if (last) tc_fence_after();
+    return last;
+}
+__device__ __forceinline__ uint32_t tmem_alloc(uint32_t* at, int warp) {         // all 512 columns; the whole CTA
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(b2::smem_u32(at)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    return *at;
+}
+__device__ __forceinline__ void tmem_free(uint32_t tmem, int warp) {
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
 
 }  // namespace chunk_tc5
 #endif
