@@ -10,15 +10,18 @@
 // delta rule over sequence length", 2024).
 //
 // One decay per head without delta is all in chunk_tc5.cu, chunks of 128 tokens.  For the others chunk_prep_kernel here computes P, T and the
-// decay products of every chunk of 64 tokens, a CTA per (chunk, head), on the FMA pipe with 8 x 8 / 4 x 8 tiles a thread (shared-memory
-// reads cost about 0.7 of the FMA cycles); the rest is delta_tc5.cu's.  The choice between chunks and tokens is at the end.
+// decay products of every chunk of 64 tokens, a CTA per (chunk, head), on the FMA pipe; the rest is delta_tc5.cu's.  Per head: tiles of
+// 8 x 8 / 4 x 8 a thread (shared-memory reads cost about 0.7 of the FMA cycles).  Per channel the decays stand between k and q, so
+// pairs of tokens of a segment of 16 are taken one by one, and those of different segments as products of rows decayed to and
+// from a boundary between them.  A warp per column with its sums in butterflies, over segments of 32, took 350 us of 4096 tokens'
+// scan (16 heads of 128), this one about 110: a third of the pairs, and one transposing sum for 16 of them.  The choice between chunks and tokens is at the end.
 #include "b2_act.cuh"
 
 #include <math.h>
 
 namespace {
 
-constexpr int C = 64, NT = 256;
+constexpr int C = 64;
 
 struct ChunkArgs {
     const float *qkv, *beta, *decay;
@@ -54,8 +57,9 @@ __device__ __forceinline__ float2 halves(pair_t v) {
 __device__ __forceinline__ ulonglong2 pairs(const float* p) { return *reinterpret_cast<const ulonglong2*>(p); }
 // ---------------------------------------------------------------------------------------------------------------- prep
 template <bool CH, bool DELTA>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(CH ? 512 : 256)
 chunk_prep_kernel(const ChunkArgs a) {
+    constexpr int NT = CH ? 512 : 256;
     static_assert(CH || DELTA, "chunk_tc5.cu");
     extern __shared__ __align__(16) float sm[];
     __shared__ int s_at[2];
@@ -96,108 +100,154 @@ chunk_prep_kernel(const ChunkArgs a) {
     // sums over dk of rows x (q, and with delta k) times columns k_s: 16 x 16 threads, rows rg + 16 rr, columns cg + 16 cc
     const int rg = tid >> 4, cg = tid & 15;
     if (CH) {
-        // inside a half of 32 tokens a warp takes a column s: k_s times the running product of the decays, dotted with every later row
-        for (int s = wid; s < C; s += NT / 32) {
-            float w[4];
+        // Inside a segment of 16 tokens: a lane takes a column s and eight channels (4 l .. and 64 + 4 l ..), and multiplies k_s by one
+        // decay after the other on its way to the later rows; 16 lanes' parts of the 16 rows are then summed, a row a lane.
+        for (int idx = tid; idx < C * (C + 1); idx += NT) {
+            Ps[idx] = 0.f;
+            if (DELTA) As[idx] = 0.f;
+        }
+        __syncthreads();
+        {
+            const int l = lane & 15;
+            const bool in0 = 4 * l < dk, in1 = 64 + 4 * l < dk;
+            auto row8 = [&](const float* m, int t, float fill, float (&x)[8]) {
+                const float* p = m + t * LD + 4 * l;
+                const float4 none = make_float4(fill, fill, fill, fill);
+                const float4 u = in0 ? *reinterpret_cast<const float4*>(p) : none, v = in1 ? *reinterpret_cast<const float4*>(p + 64) : none;
+                x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w; x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+            };
+#pragma unroll 1
+            for (int s0 = wid * 2; s0 < C; s0 += NT / 16) {
+                const int s = s0 + (lane >> 4), tb = s & ~15, from = s0 & 15;
+                float w[8], sq[16], sk[16];
+                row8(ks, s, 0.f, w);
 #pragma unroll
-            for (int m = 0; m < 4; ++m) w[m] = lane + 32 * m < dk ? ks[s * LD + lane + 32 * m] : 0.f;
-            for (int t = lane; t < s; t += 32) {
-                Ps[t * (C + 1) + s] = 0.f;
-                if (DELTA) As[t * (C + 1) + s] = 0.f;
-            }
-            for (int t = s; t < (s < 32 ? 32 : C); ++t) {
-                float dq = 0.f, dd = 0.f;
+                for (int t = 0; t < 16; ++t) {
+                    sq[t] = sk[t] = 0.f;
+                    if (t < from) continue;
+                    float x[8];
+                    if (t > from) {                  // (the second half's s is one more: it starts a step later)
+                        row8(gs, tb + t, 1.f, x);
+                        const bool step = tb + t > s;
 #pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const int i = lane + 32 * m;
-                    if (i < dk) {
-                        if (t > s) w[m] *= gs[t * LD + i];
-                        dq = fmaf(w[m], qs[t * LD + i], dq);
-                        if (DELTA) dd = fmaf(w[m], ks[t * LD + i], dd);
+                        for (int e = 0; e < 8; ++e) w[e] = step ? w[e] * x[e] : w[e];
+                    }
+                    if (tb + t < s) continue;
+                    row8(qs, tb + t, 0.f, x);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) sq[t] = fmaf(w[e], x[e], sq[t]);
+                    if (DELTA) {
+                        row8(ks, tb + t, 0.f, x);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) sk[t] = fmaf(w[e], x[e], sk[t]);
                     }
                 }
-                if (DELTA) {                         // both sums in one butterfly: the lower half carries the first, the upper the second
-                    const float other = __shfl_xor_sync(0xffffffffu, lane < 16 ? dd : dq, 16);
-                    float v = (lane < 16 ? dq : dd) + other;
+                __syncwarp();
+                auto gather = [&](float (&v)[16]) {  // lane l: the sum of row l
 #pragma unroll
-                    for (int x = 8; x > 0; x >>= 1) v += __shfl_xor_sync(0xffffffffu, v, x);
-                    if (lane == 0) Ps[t * (C + 1) + s] = v;
-                    if (lane == 16) As[t * (C + 1) + s] = t > s ? bs[t] * v : 0.f;
-                } else {
-                    dq = b2::warp_sum(dq);
-                    if (lane == 0) Ps[t * (C + 1) + s] = dq;
+                    for (int d = 8; d > 0; d >>= 1)
+#pragma unroll
+                        for (int i = 0; i < d; ++i) {
+                            const bool up = l & d;
+                            const float send = up ? v[i] : v[i + d], keep = up ? v[i + d] : v[i];
+                            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+                        }
+                    return v[0];
+                };
+                const int t = tb + l;
+                const float vq = gather(sq);
+                if (t >= s) Ps[t * (C + 1) + s] = vq;
+                if (DELTA) {
+                    const float vk = gather(sk);
+                    if (t > s) As[t * (C + 1) + s] = bs[t] * vk;
                 }
             }
         }
         __syncthreads();
-        // across the halves: rows 32 .. 63 decayed from the boundary, columns 0 .. 31 decayed to it, then a plain product; the copies
-        // for the chain are written on the way
-        const int i = tid & 127;
-        if (i < dk) {
-            if (tid < 128) {
+        // A thread takes a channel of a segment: its decays from the segment's start and to its end, then the copies for delta_tc5.cu.
+        // Rows decayed from their segment's start replace q and (in the decays' place) k, k decayed to its segment's end replaces k.
+        float* total = bs + C;                       // [4][128] the segments' whole products
+        {
+            const int i = tid & 127, b = tid >> 7, t0 = b * 16;
+            float f[16], k[16];
+            if (i < dk) {
                 float run = 1.f;
-                for (int t = 0; t < 32; ++t) {
-                    run *= gs[t * LD + i];
-                    dec[t * dk + i] = run * ks[t * LD + i];
-                    dec[(C + t) * dk + i] = run * qs[t * LD + i];
+#pragma unroll
+                for (int t = 0; t < 16; ++t) {
+                    run *= gs[(t0 + t) * LD + i];
+                    f[t] = run;
+                    k[t] = ks[(t0 + t) * LD + i];
                 }
-                float half = 1.f;
-                for (int t = 32; t < C; ++t) {
-                    half *= gs[t * LD + i];
-                    const float k = half * ks[t * LD + i], q = half * qs[t * LD + i];
-                    dec[t * dk + i] = run * k;
-                    dec[(C + t) * dk + i] = run * q;
-                    qs[t * LD + i] = q;              // this thread's channel: nobody else reads it before the barrier
+                total[b * 128 + i] = run;
+            }
+            __syncthreads();
+            if (i < dk) {
+                float before = 1.f, after = 1.f;
+                for (int m = 0; m < b; ++m) before *= total[m * 128 + i];
+                for (int m = 3; m > b; --m) after *= total[m * 128 + i];
+                if (b == 3) dec[3 * C * dk + i] = before * f[15];
+                float run = 1.f;
+#pragma unroll
+                for (int t = 15; t >= 0; --t) {
+                    const float to = run * k[t];
+                    dec[(2 * C + t0 + t) * dk + i] = after * to;
+                    ks[(t0 + t) * LD + i] = to;
+                    run *= gs[(t0 + t) * LD + i];
                 }
-                dec[3 * C * dk + i] = run * half;
-            }
-        }
-        __syncthreads();                             // the later half's keys are still as they came: their copy to the chunk's end
-        if (i < dk && tid >= 128) {
-            float run = 1.f;
-            for (int t = C - 1; t >= 32; --t) {
-                const float k = ks[t * LD + i], g = gs[t * LD + i];
-                dec[(2 * C + t) * dk + i] = run * k;
-                run *= g;
-            }
-            float half = 1.f;
-            for (int t = 31; t >= 0; --t) {
-                const float k = half * ks[t * LD + i];
-                dec[(2 * C + t) * dk + i] = run * k;
-                ks[t * LD + i] = k;
-                half *= gs[t * LD + i];
-            }
-            if (DELTA) {                             // keys 32 .. 63 decayed from the boundary
-                float from = 1.f;
-                for (int t = 32; t < C; ++t) {
-                    from *= gs[t * LD + i];
-                    ks[t * LD + i] *= from;
+#pragma unroll
+                for (int t = 0; t < 16; ++t) {
+                    const float kf = f[t] * k[t], qf = f[t] * qs[(t0 + t) * LD + i];
+                    dec[(t0 + t) * dk + i] = before * kf;
+                    dec[(C + t0 + t) * dk + i] = before * qf;
+                    gs[(t0 + t) * LD + i] = kf;
+                    qs[(t0 + t) * LD + i] = qf;
                 }
             }
         }
         __syncthreads();
-        float acc[DELTA ? 4 : 2][2];
+        // a block of 4 rows x 2 columns a thread, all channels; `rows` of q and, with delta, of k
+        auto block = [&](int t0, int s0, const float* rows, float* to, bool scale) {
+            float acc[4][2];
 #pragma unroll
-        for (int r = 0; r < (DELTA ? 4 : 2); ++r) acc[r][0] = acc[r][1] = 0.f;
-        for (int x = 0; x < dk; x += 4) {
-            const float4 k0 = *reinterpret_cast<const float4*>(ks + cg * LD + x), k1 = *reinterpret_cast<const float4*>(ks + (cg + 16) * LD + x);
+            for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0.f;
+            for (int x = 0; x < dk; x += 4) {
+                const float4 k0 = *reinterpret_cast<const float4*>(ks + s0 * LD + x), k1 = *reinterpret_cast<const float4*>(ks + (s0 + 1) * LD + x);
 #pragma unroll
-            for (int r = 0; r < (DELTA ? 4 : 2); ++r) {
-                const float4 v = *reinterpret_cast<const float4*>((r < 2 ? qs : ks) + (32 + rg + 16 * (r & 1)) * LD + x);
-                acc[r][0] = fmaf(v.x, k0.x, acc[r][0]); acc[r][0] = fmaf(v.y, k0.y, acc[r][0]);
-                acc[r][0] = fmaf(v.z, k0.z, acc[r][0]); acc[r][0] = fmaf(v.w, k0.w, acc[r][0]);
-                acc[r][1] = fmaf(v.x, k1.x, acc[r][1]); acc[r][1] = fmaf(v.y, k1.y, acc[r][1]);
-                acc[r][1] = fmaf(v.z, k1.z, acc[r][1]); acc[r][1] = fmaf(v.w, k1.w, acc[r][1]);
+                for (int r = 0; r < 4; ++r) {
+                    const float4 v = *reinterpret_cast<const float4*>(rows + (t0 + r) * LD + x);
+                    acc[r][0] = fmaf(v.x, k0.x, acc[r][0]); acc[r][0] = fmaf(v.y, k0.y, acc[r][0]);
+                    acc[r][0] = fmaf(v.z, k0.z, acc[r][0]); acc[r][0] = fmaf(v.w, k0.w, acc[r][0]);
+                    acc[r][1] = fmaf(v.x, k1.x, acc[r][1]); acc[r][1] = fmaf(v.y, k1.y, acc[r][1]);
+                    acc[r][1] = fmaf(v.z, k1.z, acc[r][1]); acc[r][1] = fmaf(v.w, k1.w, acc[r][1]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) to[(t0 + r) * (C + 1) + s0 + c] = scale ? bs[t0 + r] * acc[r][c] : acc[r][c];
+        };
+        // neighbouring segments of a half: 16 x 16 results, 32 threads; [half][q, k]
+        if (wid < (DELTA ? 4 : 2)) {
+            const int h = wid & 1, t0 = 32 * h + 16 + (lane & 3) * 4, s0 = 32 * h + (lane >> 2) * 2;
+            if (wid < 2) block(t0, s0, qs, Ps, false);
+            else block(t0, s0, gs, As, true);
+        }
+        __syncthreads();
+        // across the halves: on to the boundary, and from it
+        if (tid < 128 && tid < dk) {
+            const float to = total[128 + tid], from = total[2 * 128 + tid];
+#pragma unroll 4
+            for (int t = 0; t < 16; ++t) {
+                ks[t * LD + tid] *= to;
+                qs[(48 + t) * LD + tid] *= from;
+                if (DELTA) gs[(48 + t) * LD + tid] *= from;
             }
         }
-#pragma unroll
-        for (int r = 0; r < (DELTA ? 4 : 2); ++r) {
-            const int t = 32 + rg + 16 * (r & 1);
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                if (r < 2) Ps[t * (C + 1) + cg + 16 * c] = acc[r][c];
-                else As[t * (C + 1) + cg + 16 * c] = bs[t] * acc[r][c];
-            }
+        __syncthreads();
+        if (wid < (DELTA ? 8 : 4)) {                 // 32 x 32 results, 128 threads
+            const int u = tid & 127, t0 = 32 + (u & 7) * 4, s0 = (u >> 3) * 2;
+            if (wid < 4) block(t0, s0, qs, Ps, false);
+            else block(t0, s0, gs, As, true);
         }
     } else {
         // the decay ratios of all (t, s), and the products from the chunk's start and to its end: by segments of 16 tokens, a chain of
@@ -265,7 +315,7 @@ chunk_prep_kernel(const ChunkArgs a) {
     if (DELTA) {
         // the inverse of I + A by halves: forward substitution on the diagonal blocks (a warp each, a lane per column), then
         // T21 = -T22 A21 T11; Ps is free and takes T
-        if (wid >= 6) {
+        if (wid == 6 || wid == 7) {
             const int o = wid == 6 ? 0 : 32;
             float T[32];
 #pragma unroll
@@ -282,8 +332,8 @@ chunk_prep_kernel(const ChunkArgs a) {
         }
         __syncthreads();
         float* x = Ps;                               // A21 T11, [32][C + 1]
-        const int row = tid >> 3, c4 = (tid & 7) * 4;
-        {
+        const int row = tid >> 3, c4 = (tid & 7) * 4;                // 256 threads
+        if (tid < 256) {
             float v[4] = {0.f, 0.f, 0.f, 0.f};
             for (int s = 0; s < 32; ++s) {
                 const float l = As[(32 + row) * (C + 1) + s];
@@ -294,7 +344,7 @@ chunk_prep_kernel(const ChunkArgs a) {
             for (int c = 0; c < 4; ++c) x[row * (C + 1) + c4 + c] = v[c];
         }
         __syncthreads();
-        {
+        if (tid < 256) {
             float v[4] = {0.f, 0.f, 0.f, 0.f};
             for (int s = 0; s <= row; ++s) {
                 const float l = As[(32 + row) * (C + 1) + 32 + s];
@@ -323,10 +373,10 @@ template <bool CH, bool DELTA>
 int launch_prep(const ChunkArgs& a, int total_rows, cudaStream_t st) {
     const int chunks = total_rows / C + a.n_seq;     // upper bound on sum(ceil(len / C)); spare CTAs leave at once
     const size_t LD = a.dk + 4, rows = C * LD;
-    const size_t psm = sizeof(float) * (2 * rows + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows : 2 * C + 4) + C);
+    const size_t psm = sizeof(float) * (2 * rows + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows + 4 * 128 : 2 * C + 4) + C);
     int rc = allow(chunk_prep_kernel<CH, DELTA>, psm);
     if (rc != B2_OK) return rc;
-    chunk_prep_kernel<CH, DELTA><<<dim3(chunks, a.H), NT, psm, st>>>(a);
+    chunk_prep_kernel<CH, DELTA><<<dim3(chunks, a.H), CH ? 512 : 256, psm, st>>>(a);
     B2_CUDA_OK(cudaGetLastError());
     return B2_OK;
 }
@@ -348,25 +398,26 @@ int64_t b2_internal_chunk_scan_floats(int total_rows, int n_seq, int H, int dk, 
 //            token and head, down to 5.0 (6.3 / 6.8 / 8.3) from 64 sequences on; keys of other sizes than 32, 64, 128 run as the next one, a third slower
 //   chunks   one decay per head without delta (chunk_tc5.cu): 20, 0.2 a chunk of 128 and head for the products (0.14 at 64 x 64) and 0.03 a
 //            sequence and head for its state; at least 33 (29 to dk = 64): three launches
-//            else 0.3 (per channel 0.55 / 0.70) a chunk of 64 and head for the products, 0.11 a sequence and head for its state, with delta
-//            2.7 a step of the chain and SM's share of CTAs; at least 60 (49 to dk = 64; 80 per channel, 110 with delta too): four launches
-// Measured, tokens -> chunks: 1 x 4096 tokens, 16 heads: 804 -> 121, 1160 -> 442, 963 -> 536, 1255 -> 886; 1 x 500: 102 -> 34,
-// 146 -> 72, 121 -> 76, 158 -> 129; 1500 + 1000 + 501: 411 -> 92, 573 -> 290, 503 -> 436, 630 -> 668: the last is left to the tokens, as are 16 x 100 but for the
-// first (121 -> 74, 160 -> 196, 181 -> 299, 223 -> 446), 64 x 24: 148 -> 250, 180 -> 415, and 1 x 130: 29 -> 33, 41 -> 58.
+//            else 0.3 (per channel 20 and 0.27 / 0.46) a chunk of 64 and head for the products, 0.11 a sequence and head for its state, with
+//            delta 2.7 a step of the chain and SM's share of CTAs; at least 60 (39 / 72 per channel; to dk = 64 49, 33 / 58): four launches
+// Measured, tokens -> chunks: 1 x 4096 tokens, 16 heads: 804 -> 121, 1160 -> 442, 963 -> 298, 1255 -> 582; 1 x 500: 102 -> 34,
+// 146 -> 72, 121 -> 43, 158 -> 88; 1500 + 1000 + 501: 411 -> 92, 573 -> 290, 503 -> 235, 631 -> 407; 16 x 100: 121 -> 74, 181 -> 166, but 160 -> 196 and
+// 223 -> 274 with delta, which are left to the tokens, as are 64 x 24: 148 -> 250, 180 -> 415, 193 -> 379, and 1 x 130: 29 -> 33, 41 -> 58, 35 -> 40.
 bool b2_internal_chunk_scan_pays(int total_rows, int n_seq, int H, int dk, int dv, bool ch, bool delta) {
     if (total_rows < 2 * n_seq) return false;
     const float len = (float)total_rows / n_seq, w = dk * dv / 16384.f, steps = ceilf(len / C), heads = (float)n_seq * H;
     const int kind = (ch ? 2 : 0) + (delta ? 1 : 0), run_as = dk <= 32 ? 32 : dk <= 64 ? 64 : 128;
     const float chain_tok[4] = {0.20f, 0.285f, 0.235f, 0.31f}, rate_few[4] = {5.2e-3f, 7.1e-3f, 10.6e-3f, 12.4e-3f}, rate_many[4] = {5.0e-3f, 6.3e-3f, 6.8e-3f, 8.3e-3f};
-    const float per_chunk[4] = {0.f, 0.3f, 0.55f, 0.70f}, least[4] = {dk <= 64 ? 29.f : 33.f, dk <= 64 ? 49.f : 60.f, 80.f, 110.f};
-    const float many = fminf(1.f, fmaxf(0.f, log2f(n_seq / 4.f) / 4.f)), rate = rate_few[kind] + (rate_many[kind] - rate_few[kind]) * many;
+    const float per_chunk[4] = {0.f, 0.3f, 0.27f, 0.46f};
+    const float least[4] = {dk <= 64 ? 29.f : 33.f, dk <= 64 ? 49.f : 60.f, dk <= 64 ? 33.f : 39.f, dk <= 64 ? 58.f : 72.f};
+    const float many = fminf(1.f, fmaxf(0.f, log2f(n_seq / 2.5f) / 4.f)), rate = rate_few[kind] + (rate_many[kind] - rate_few[kind]) * many;
     const float longest = len * (n_seq > 1 ? 1.25f : 1.f);
     const float tokens = (run_as == dk ? 1.f : 1.33f) * fmaxf(chain_tok[kind] * (dk <= 64 ? 0.75f : 1.f) * longest, rate * (float)total_rows * H * run_as * dv / 16384.f);
     float chunks;
     if (kind == 0) {
         chunks = 20.f + (0.2f * (0.6f + 0.4f * w) * ceilf(len / 128) + 0.03f * w) * heads;
     } else {
-        chunks = (per_chunk[kind] * (0.35f + 0.65f * w) * steps + 0.11f * w) * heads;
+        chunks = (ch ? 20.f : 0.f) + (per_chunk[kind] * (ch ? 0.55f + 0.45f * w : 0.35f + 0.65f * w) * steps + 0.11f * w) * heads;
         if (delta) chunks += 2.7f * fmaxf(ceilf(longest / C), steps * heads * ((dv + 63) / 64) / b2_sm_count());
     }
     return tokens >= fmaxf(chunks, least[kind]);
