@@ -16,6 +16,13 @@ from . import _lib
 from ._lib import KV_BF16, KV_FP8_E4M3
 
 
+try:
+    _raw_stream = torch._C._cuda_getCurrentRawStream
+except AttributeError:                               # a torch without it
+    def _raw_stream(index: int) -> int:
+        return torch.cuda.current_stream(index).cuda_stream
+
+
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
@@ -26,6 +33,19 @@ _PINNED_OK = ("q", "k_new", "v_new")
 
 
 def _need_cuda(**tensors) -> torch.device:
+    """The one GPU that all of them are on.  Small steps are bound by the host, so the common case is one integer a tensor."""
+    first, index = None, -2
+    for t in tensors.values():
+        if t is not None:
+            i = t.get_device()
+            if i != index:
+                if first is not None or i < 0:
+                    return _which_device(tensors)
+                first, index = t, i
+    return None if first is None else first.device
+
+
+def _which_device(tensors) -> torch.device:
     dev = None
     for name, t in tensors.items():
         if t is None:
@@ -42,7 +62,7 @@ def _need_cuda(**tensors) -> torch.device:
 
 
 def _stream(dev: torch.device) -> int:
-    return torch.cuda.current_stream(dev).cuda_stream
+    return _raw_stream(dev.index)                    # current_stream(dev).cuda_stream without an object around it: 2.3 -> 0.1 us
 
 
 def _kv_dtype_of(cache: torch.Tensor) -> int:
@@ -54,15 +74,22 @@ def _kv_dtype_of(cache: torch.Tensor) -> int:
 
 
 def _check_cache(k_cache: torch.Tensor, v_cache: torch.Tensor):
-    if k_cache.dim() != 4 or k_cache.shape != v_cache.shape or k_cache.dtype != v_cache.dtype:
+    shape, s = k_cache.shape, k_cache.stride()
+    if len(shape) != 4 or shape != v_cache.shape or k_cache.dtype != v_cache.dtype:
         raise ValueError("k_cache / v_cache must both be [num_blocks, Hkv, bs, d] of one dtype")
-    if k_cache.stride() != v_cache.stride():
+    if s != v_cache.stride():
         raise ValueError("k_cache / v_cache must share strides")
-    nb, Hkv, bs, d = k_cache.shape
-    s = k_cache.stride()
+    nb, Hkv, bs, d = shape
     if s[3] != 1 or s[2] != d:
         raise ValueError("each (block, head) tile of the KV cache must be contiguous [bs, d]")
     return nb, Hkv, bs, d, s[0], s[1]
+
+
+def _head_strides(t: torch.Tensor, d: int, name: str):
+    s = t.stride()
+    if s[2] != 1 or s[1] != d:
+        raise ValueError(f"{name}: head and dim axes must be contiguous")
+    return s
 
 
 def reshape_and_cache(k_new: torch.Tensor, v_new: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
@@ -234,30 +261,33 @@ def paged_decode_append(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tenso
                      workspace=workspace)
     nb, Hkv, bs, d, bstride, hstride = _check_cache(k_cache, v_cache)
     kvd = _kv_dtype_of(k_cache)
-    if q.dtype != torch.bfloat16 or q.dim() != 3 or q.shape[2] != d:
+    shape = q.shape
+    if q.dtype != torch.bfloat16 or len(shape) != 3 or shape[2] != d:
         raise ValueError(f"q must be bf16 [B, Hq, {d}]")
-    B, Hq, _ = q.shape
-    if q.stride(2) != 1 or q.stride(1) != d:
-        raise ValueError("q: head and dim axes must be contiguous")
+    B, Hq, _ = shape
+    qs, _, _ = _head_strides(q, d, "q")
     if k_new.dtype != torch.bfloat16 or v_new.dtype != torch.bfloat16:
         raise ValueError("k_new / v_new must be bf16")
-    if k_new.shape != (B, Hkv, d) or v_new.shape != (B, Hkv, d):
+    row = (B, Hkv, d)
+    if k_new.shape != row or v_new.shape != row:
         raise ValueError(f"k_new / v_new must be [{B}, {Hkv}, {d}] (one new token per row)")
-    for t in (k_new, v_new):
-        if t.stride(2) != 1 or t.stride(1) != d:
-            raise ValueError("k_new / v_new: head and dim axes must be contiguous")
+    ks, _, _ = _head_strides(k_new, d, "k_new / v_new")
+    vs, _, _ = _head_strides(v_new, d, "k_new / v_new")
     if slot_mapping.dtype != torch.int64 or slot_mapping.shape != (B,) or not slot_mapping.is_contiguous():
         raise ValueError("slot_mapping must be a contiguous int64 [B]")
-    if block_tables.dtype != torch.int32 or block_tables.dim() != 2 or block_tables.shape[0] != B \
-            or not block_tables.is_contiguous():
+    shape = block_tables.shape
+    if block_tables.dtype != torch.int32 or len(shape) != 2 or shape[0] != B or not block_tables.is_contiguous():
         raise ValueError("block_tables must be a contiguous int32 [B, max_nb]")
+    max_nb = shape[1]
     if seq_lens.dtype != torch.int32 or seq_lens.shape != (B,) or not seq_lens.is_contiguous():
         raise ValueError("seq_lens must be a contiguous int32 [B]")
-    max_nb = block_tables.shape[1]
+    os_ = Hq * d
     if out is None:
         out = torch.empty(B, Hq, d, dtype=torch.bfloat16, device=dev)
     elif out.dtype != torch.bfloat16 or out.shape != (B, Hq, d) or out.stride(2) != 1 or out.stride(1) != d:
         raise ValueError("out must be bf16 [B, Hq, d] with contiguous head/dim axes")
+    else:
+        os_ = out.stride(0)
     if scale is None:
         scale = 1.0 / math.sqrt(d)
     if kvd == KV_FP8_E4M3:
@@ -266,18 +296,18 @@ def paged_decode_append(q: torch.Tensor, k_new: torch.Tensor, v_new: torch.Tenso
                 raise ValueError("fp8 KV cache needs 1-element fp32 device tensors k_scale / v_scale")
     if B == 0:
         return out
-    need = lib.b2_paged_decode_workspace_bytes(B, Hq, Hkv, d, bs, max_nb, num_splits)
+    need = 0 if num_splits == 1 else lib.b2_paged_decode_workspace_bytes(B, Hq, Hkv, d, bs, max_nb, num_splits)
     if need and (workspace is None or workspace.numel() * workspace.element_size() < need):
         if workspace is not None:
             raise ValueError(f"workspace holds {workspace.numel() * workspace.element_size()} bytes, {need} required")
         workspace = torch.empty(need, dtype=torch.uint8, device=dev)
-    wbytes = 0 if workspace is None else workspace.numel() * workspace.element_size()
+    wbytes = 0 if workspace is None else workspace.nbytes
     one = Hkv * d
     _lib.check(lib.b2_paged_decode_append(
         _ptr(out), _ptr(q), _ptr(k_new), _ptr(v_new), _ptr(slot_mapping),
-        k_new.stride(0) if B > 1 else one, v_new.stride(0) if B > 1 else one,
+        ks if B > 1 else one, vs if B > 1 else one,
         _ptr(k_cache), _ptr(v_cache), _ptr(block_tables), _ptr(seq_lens),
-        B, Hq, Hkv, d, bs, max_nb, nb, q.stride(0) if B > 1 else Hq * d, out.stride(0) if B > 1 else Hq * d,
+        B, Hq, Hkv, d, bs, max_nb, nb, qs if B > 1 else Hq * d, os_ if B > 1 else Hq * d,
         bstride, hstride, float(scale), kvd, _ptr(k_scale), _ptr(v_scale), _ptr(workspace), wbytes, num_splits,
         _stream(dev)))
     return out
@@ -411,7 +441,7 @@ def dequant_kv_blocks(k_cache: torch.Tensor, v_cache: torch.Tensor, src_blocks: 
     for o in (k_out, v_out):
         if o is None:
             o = torch.empty(shape, dtype=torch.bfloat16, device=dev)
-        elif o.dtype != torch.bfloat16 or tuple(o.shape) != shape or not o.is_contiguous():
+        elif o.dtype != torch.bfloat16 or o.shape != shape or not o.is_contiguous():
             raise ValueError(f"k_out / v_out must be contiguous bf16 {list(shape)}")
         outs.append(o)
     _lib.check(lib.b2_dequant_kv_blocks(_ptr(outs[0]), _ptr(outs[1]), _ptr(k_cache), _ptr(v_cache), _ptr(src_blocks),
@@ -658,15 +688,17 @@ def _act(t: torch.Tensor, name: str) -> int:
 def _f32(t: Optional[torch.Tensor], name: str, shape=None) -> Optional[torch.Tensor]:
     if t is None:
         return None
-    if t.dtype != torch.float32 or not t.is_contiguous() or (shape is not None and tuple(t.shape) != tuple(shape)):
+    if t.dtype != torch.float32 or not t.is_contiguous() or (shape is not None and t.shape != shape):
         raise ValueError(f"{name} must be a contiguous fp32 tensor" + (f" of shape {tuple(shape)}" if shape else ""))
     return t
 
 
 def _mat(t: torch.Tensor, name: str):
-    if t.dim() != 2 or (t.shape[1] > 1 and t.stride(1) != 1):
+    shape, strides = t.shape, t.stride()
+    if len(shape) != 2 or (shape[1] > 1 and strides[1] != 1):
         raise ValueError(f"{name} must be [rows, cols] with a contiguous last axis")
-    return t.shape[0], t.shape[1], (t.stride(0) if t.shape[0] > 1 else t.shape[1])
+    rows, cols = shape
+    return rows, cols, strides[0] if rows > 1 else cols
 
 
 def _out_rows(out: torch.Tensor, T: int, cols: int, dtype: torch.dtype) -> int:
@@ -784,7 +816,7 @@ def delta_prep(proj: torch.Tensor, off_b: int, off_a: int, H: int, G: int, dk: i
     _f32(conv_w, "conv_w", (C, taps)), _f32(A_log, "A_log", (H,)), _f32(dt_bias, "dt_bias", (H,))
     if taps > 1:
         if conv_state is None or conv_state.dtype != proj.dtype or not conv_state.is_contiguous() \
-                or tuple(conv_state.shape[1:]) != (taps - 1, C):
+                or conv_state.shape[1:] != (taps - 1, C):
             raise ValueError(f"conv_state must be contiguous [slots, {taps - 1}, {C}] of proj's dtype")
     qkv = torch.empty(T, C, dtype=torch.float32, device=dev)
     beta = torch.empty(T, H, dtype=torch.float32, device=dev)
@@ -804,7 +836,7 @@ def delta_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, H: in
     dev = _need_cuda(qkv=qkv, beta=beta, decay=decay, state=state)
     T = qkv.shape[0]
     _f32(qkv, "qkv", (T, 2 * G * dk + H * dv)), _f32(beta, "beta", (T, H)), _f32(decay, "decay", (T, H))
-    if state.dtype != torch.float32 or not state.is_contiguous() or tuple(state.shape[1:]) != (H, dk, dv):
+    if state.dtype != torch.float32 or not state.is_contiguous() or state.shape[1:] != (H, dk, dv):
         raise ValueError(f"state must be contiguous fp32 [slots, {H}, {dk}, {dv}]")
     return _scan(lib, dev, qkv, beta, decay, T, H, G, dk, dv, False, True, batch, state)
 
@@ -868,7 +900,7 @@ def qknorm_cache(qkv: torch.Tensor, H: int, G: int, dk: int, dv: int, q_w: Optio
         raise ValueError("qkv width differs from H*dk + G*dk + G*dv")
     _f32(q_w, "q_w", (dk,)), _f32(k_w, "k_w", (dk,))
     nb, bs = k_cache.shape[0], k_cache.shape[2]
-    if tuple(k_cache.shape) != (nb, G, bs, dk) or tuple(v_cache.shape) != (nb, G, bs, dv) or not k_cache.is_contiguous() \
+    if k_cache.shape != (nb, G, bs, dk) or v_cache.shape != (nb, G, bs, dv) or not k_cache.is_contiguous() \
             or not v_cache.is_contiguous() or k_cache.dtype != qkv.dtype or v_cache.dtype != qkv.dtype:
         raise ValueError("k_cache / v_cache must be contiguous [nb, G, bs, dk] / [nb, G, bs, dv] of qkv's dtype")
     if slots.dtype != torch.int64 or slots.shape != (T,) or not slots.is_contiguous():
@@ -898,7 +930,7 @@ def chunk_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     T, H, dk = q.shape
     nb, G, bs, dv = v_cache.shape
     if maps < 1 or H % maps or not q.is_contiguous() or k_cache.dtype != q.dtype or v_cache.dtype != q.dtype \
-            or tuple(k_cache.shape) != (nb, G * maps, bs, dk):
+            or k_cache.shape != (nb, G * maps, bs, dk):
         raise ValueError("q must be contiguous and the pools of its dtype, k_cache [nb, maps * G, bs, dk]")
     H //= maps
     bt = batch.block_tables
@@ -908,13 +940,15 @@ def chunk_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     _f32(sink_logits, "sink_logits", (H,))
     gs = 0
     if gate is not None:
-        if gate.dtype != q.dtype or gate.dim() != 2 or tuple(gate.shape) != (T, H) or (H > 1 and gate.stride(1) != 1):
+        if gate.dtype != q.dtype or gate.dim() != 2 or gate.shape != (T, H) or (H > 1 and gate.stride(1) != 1):
             raise ValueError("gate must be [T, H] of q's dtype with a contiguous last axis")
         gs = gate.stride(0) if T > 1 else H
     _f32(head_bias, "head_bias", (H,))
+    os_ = H * dv
     if out is None:
         out = torch.empty(T, H, dv, dtype=q.dtype, device=dev)
-    os_ = _out_rows(out, T, H * dv, q.dtype)
+    else:
+        os_ = _out_rows(out, T, H * dv, q.dtype)
     _lib.check(lib.b2_masked_attention(_ptr(out), _ptr(q), _ptr(k_cache), _ptr(v_cache), _act(q, "q"), _ptr(bt), bt.shape[1],
                                        _ptr(batch.cu_q), _ptr(batch.ctx_start), batch.n_seq, T, H, G, dk, dv, bs,
                                        float(scale), int(chunk), int(window), int(keep_first), float(sink), float(sink_logit),
@@ -940,7 +974,7 @@ def qk_rope_cache(qkv: torch.Tensor, H: int, G: int, dk: int, dv: int, positions
     nb, bs, Gv = k_cache.shape[0], k_cache.shape[2], v_cache.shape[1]
     if P < H * dk + G * dk + (0 if v_from_k else Gv * dv):
         raise ValueError("qkv is narrower than its heads")
-    if tuple(k_cache.shape) != (nb, G, bs, dk) or tuple(v_cache.shape) != (nb, Gv, bs, dv) or Gv > G or not k_cache.is_contiguous() \
+    if k_cache.shape != (nb, G, bs, dk) or v_cache.shape != (nb, Gv, bs, dv) or Gv > G or not k_cache.is_contiguous() \
             or not v_cache.is_contiguous() or k_cache.dtype != qkv.dtype or v_cache.dtype != qkv.dtype:
         raise ValueError("k_cache / v_cache must be contiguous [nb, G, bs, dk] / [nb, Gv, bs, dv] of qkv's dtype")
     if slots.dtype != torch.int64 or slots.shape != (T,) or not slots.is_contiguous():
@@ -969,7 +1003,7 @@ def moe_route(h: torch.Tensor, w_router: torch.Tensor, bias: Optional[torch.Tens
     dev = _need_cuda(h=h, w_router=w_router, bias=bias)
     T, D, hs = _mat(h, "h")
     E = w_router.shape[0]
-    if w_router.dtype != h.dtype or tuple(w_router.shape) != (E, D) or not w_router.is_contiguous():
+    if w_router.dtype != h.dtype or w_router.shape != (E, D) or not w_router.is_contiguous():
         raise ValueError("w_router must be contiguous [E, D] of h's dtype")
     _f32(bias, "bias", (E,))
     ids = torch.empty(T, top, dtype=torch.int32, device=dev)
@@ -1017,11 +1051,11 @@ def moe_experts(h: torch.Tensor, ids: torch.Tensor, wts: torch.Tensor, w_gate: O
     if gated == (w_gate is None):
         raise ValueError("gated experts need w_gate, experts without a gate take none")
     for name, w, shape in (("w_gate", w_gate, (E, F, D)), ("w_up", w_up, (E, F, D)), ("w_down", w_down, (E, D, F))):
-        if w is not None and (w.dtype != h.dtype or tuple(w.shape) != shape or w.stride(2) != 1 or w.stride(1) != shape[2]):
+        if w is not None and (w.dtype != h.dtype or w.shape != shape or w.stride(2) != 1 or w.stride(1) != shape[2]):
             raise ValueError(f"{name} must be {shape} of h's dtype with contiguous rows")
     if (gated and w_gate.stride(0) != w_up.stride(0)) or not w_down.is_contiguous():
         raise ValueError("w_gate / w_up must share their expert stride, w_down must be contiguous")
-    if ids.dtype != torch.int32 or not ids.is_contiguous() or tuple(ids.shape) != (T, top):
+    if ids.dtype != torch.int32 or not ids.is_contiguous() or ids.shape != (T, top):
         raise ValueError("ids must be contiguous int32 [T, top]")
     _f32(wts, "wts", (T, top))
     as_ = 0
@@ -1037,16 +1071,17 @@ def moe_experts(h: torch.Tensor, ids: torch.Tensor, wts: torch.Tensor, w_gate: O
         w_gate_up = w_up if w_up.is_contiguous() else None
     grouped = (w_gate_up is not None and h.dtype == torch.bfloat16 and n >= MOE_GROUPED_GEMM_MIN_PAIRS and D % 8 == 0
                and F % 8 == 0 and hasattr(torch, "_grouped_mm"))
-    meta = torch.empty(cap + tiles + n + E, dtype=torch.int32, device=dev)
-    srt, tile_e, place, ends = meta[:cap], meta[cap:cap + tiles], meta[cap + tiles:cap + tiles + n], meta[cap + tiles + n:]
-    _lib.check(lib.b2_moe_align(_ptr(ids), n, E, cap, _ptr(srt), _ptr(tile_e), _ptr(place), _ptr(ends) if grouped else None,
-                                _stream(dev)))
+    meta = torch.empty(cap + tiles + n + E, dtype=torch.int32, device=dev)          # sorted pairs | experts of the tiles | places | ends
+    srt = meta.data_ptr()
+    tile_e, place = srt + 4 * cap, srt + 4 * (cap + tiles)
+    _lib.check(lib.b2_moe_align(_ptr(ids), n, E, cap, srt, tile_e, place, place + 4 * n if grouped else None, _stream(dev)))
     y = torch.empty(T, D, dtype=h.dtype, device=dev)
     if grouped:
-        if tuple(w_gate_up.shape) != (E, (2 if gated else 1) * F, D) or not w_gate_up.is_contiguous() or w_gate_up.dtype != h.dtype:
+        if w_gate_up.shape != (E, (2 if gated else 1) * F, D) or not w_gate_up.is_contiguous() or w_gate_up.dtype != h.dtype:
             raise ValueError("w_gate_up must be contiguous [E, 2F, D] of h's dtype")
+        ends = meta[cap + tiles + n:]
         a = torch.empty(cap, D, dtype=h.dtype, device=dev)
-        _lib.check(lib.b2_moe_gather(_ptr(h), hs, _act(h, "h"), _ptr(srt), _ptr(wts) if weight_on_input else None, cap, top, D,
+        _lib.check(lib.b2_moe_gather(_ptr(h), hs, _act(h, "h"), srt, _ptr(wts) if weight_on_input else None, cap, top, D,
                                      _ptr(a), _stream(dev)))
         gu = torch._grouped_mm(a, w_gate_up.transpose(1, 2), offs=ends)              # [cap, 2F]; rows past the last group unset
         if not gated:
@@ -1054,13 +1089,13 @@ def moe_experts(h: torch.Tensor, ids: torch.Tensor, wts: torch.Tensor, w_gate: O
         else:
             act = silu_and_mul(gu) if glu == GLU_SILU else glu_and_mul(gu, glu, glu_alpha, glu_limit)
         rows = torch._grouped_mm(act, w_down.transpose(1, 2), offs=ends)             # [cap, D]
-        _lib.check(lib.b2_moe_combine(_ptr(rows), 0, _ptr(place), None if weight_on_input else _ptr(wts), T, top, D, _ptr(add), as_,
+        _lib.check(lib.b2_moe_combine(_ptr(rows), 0, place, None if weight_on_input else _ptr(wts), T, top, D, _ptr(add), as_,
                                       _ptr(y), D, _act(h, "h"), _stream(dev)))
         return y
     act = torch.empty(cap, F, dtype=h.dtype, device=dev)
     rows = torch.empty(cap, D, dtype=torch.float32, device=dev)
     _lib.check(lib.b2_moe_experts(_ptr(h), hs, _ptr(w_gate), _ptr(w_up), _ptr(w_down), w_up.stride(0), _act(h, "h"), T, D, F,
-                                  top, cap, _ptr(srt), _ptr(tile_e), _ptr(place), _ptr(wts), _ptr(act), _ptr(rows), _ptr(add), as_,
+                                  top, cap, srt, tile_e, place, _ptr(wts), _ptr(act), _ptr(rows), _ptr(add), as_,
                                   _ptr(y), D, int(glu), float(glu_alpha), float(glu_limit), int(weight_on_input), _stream(dev)))
     return y
 
@@ -1176,7 +1211,7 @@ def recur_prep(proj: torch.Tensor, H: int, G: int, dk: int, dv: int, batch: SeqB
     if conv_w is not None:
         _f32(conv_w, "conv_w", (C, taps))
     if taps > 1 and (conv_w is None or conv_state is None or conv_state.dtype != proj.dtype or not conv_state.is_contiguous()
-                     or tuple(conv_state.shape[1:]) != (taps - 1, C)):
+                     or conv_state.shape[1:] != (taps - 1, C)):
         raise ValueError(f"a convolution needs conv_w and a contiguous conv_state [slots, {taps - 1}, {C}] of proj's dtype")
     per_channel = decay_mode not in (DECAY_HEAD_SOFTPLUS, DECAY_HEAD_CONST)
     a_stride = 0
@@ -1223,10 +1258,10 @@ def channel_scan(qkv: torch.Tensor, beta: Optional[torch.Tensor], decay: torch.T
     _f32(qkv, "qkv", (T, 2 * G * dk + H * dv))
     if delta:
         _f32(beta, "beta", (T, H))
-    if decay.dtype != torch.float32 or not decay.is_contiguous() or tuple(decay.shape) not in ((T, H), (T, H * dk)):
+    if decay.dtype != torch.float32 or not decay.is_contiguous() or decay.shape not in ((T, H), (T, H * dk)):
         raise ValueError("decay must be contiguous fp32 [T, H] or [T, H*dk]")
-    per_channel = tuple(decay.shape) == (T, H * dk) and dk > 1
-    if state.dtype != torch.float32 or not state.is_contiguous() or tuple(state.shape[1:]) != (H, dk, dv):
+    per_channel = decay.shape == (T, H * dk) and dk > 1
+    if state.dtype != torch.float32 or not state.is_contiguous() or state.shape[1:] != (H, dk, dv):
         raise ValueError(f"state must be contiguous fp32 [slots, {H}, {dk}, {dv}]")
     return _scan(lib, dev, qkv, beta if delta else None, decay, T, H, G, dk, dv, per_channel, delta, batch, state)
 
@@ -1242,11 +1277,13 @@ def gated_head_norm(o: torch.Tensor, gate: torch.Tensor, norm_w: Optional[torch.
     Tg, W, gs = _mat(gate, "gate")
     if (Tg, W) != (T, H * dv):
         raise ValueError("gate must be [T, H*dv]")
+    os_ = H * dv
     if out is None:
         out = torch.empty(T, H * dv, dtype=gate.dtype, device=dev)
-    To, Wo, os_ = _mat(out, "out")
-    if (To, Wo) != (T, H * dv) or out.dtype != gate.dtype:
-        raise ValueError("out must be [T, H*dv] of gate's dtype")
+    else:
+        To, Wo, os_ = _mat(out, "out")
+        if (To, Wo) != (T, H * dv) or out.dtype != gate.dtype:
+            raise ValueError("out must be [T, H*dv] of gate's dtype")
     _lib.check(lib.b2_gated_head_norm(_ptr(o), _ptr(gate), gs, int(gate_kind), _act(gate, "gate"), T, H, dv, _ptr(norm_w),
                                       float(eps), float(out_scale), _ptr(out), os_, _stream(dev)))
     return out
@@ -1264,7 +1301,7 @@ def qk_prep_cache(qkv: torch.Tensor, H: int, G: int, dk: int, dv: int, slots: to
     if P != H * dk + G * dk + G * dv:
         raise ValueError("qkv width differs from H*dk + G*dk + G*dv")
     nb, bs = k_cache.shape[0], k_cache.shape[2]
-    if tuple(k_cache.shape) != (nb, G, bs, dk) or tuple(v_cache.shape) != (nb, G, bs, dv) or not k_cache.is_contiguous() \
+    if k_cache.shape != (nb, G, bs, dk) or v_cache.shape != (nb, G, bs, dv) or not k_cache.is_contiguous() \
             or not v_cache.is_contiguous() or k_cache.dtype != qkv.dtype or v_cache.dtype != qkv.dtype:
         raise ValueError("k_cache / v_cache must be contiguous [nb, G, bs, dk] / [nb, G, bs, dv] of qkv's dtype")
     if slots.dtype != torch.int64 or slots.shape != (T,) or not slots.is_contiguous():
@@ -1494,7 +1531,7 @@ def latent_prep(proj: torch.Tensor, H: int, dn: int, dr: int, rot_dims: int, R: 
         bs = cache.shape[1]
     if qa is None:
         qa = torch.empty(T, H, R + dr, dtype=proj.dtype, device=dev)
-    elif tuple(qa.shape) != (T, H, R + dr) or qa.dtype != proj.dtype or not qa.is_contiguous():
+    elif qa.shape != (T, H, R + dr) or qa.dtype != proj.dtype or not qa.is_contiguous():
         raise ValueError("qa must be contiguous [T, H, R + dr] of proj's dtype")
     _lib.check(lib.b2_latent_prep_rows(_ptr(proj), ps, _ptr(kv), ks, _act(proj, "proj"), T, H, dn, dr, rot_dims, int(interleaved), R, q_off,
                                        dkv_off, _ptr(norm_w), float(eps), _ptr(positions), _ptr(cos_sin), cos_sin.shape[0], _ptr(slots),
@@ -1520,7 +1557,7 @@ def latent_attention(qa: torch.Tensor, cache: torch.Tensor, batch: SeqBatch, R: 
         raise ValueError("block_tables must be a contiguous int32 [n_seq, max_nb]")
     gs = 0
     if gate is not None:
-        if gate.dtype != qa.dtype or gate.dim() != 2 or tuple(gate.shape) != (T, H) or (H > 1 and gate.stride(1) != 1):
+        if gate.dtype != qa.dtype or gate.dim() != 2 or gate.shape != (T, H) or (H > 1 and gate.stride(1) != 1):
             raise ValueError("gate must be [T, H] of qa's dtype with a contiguous last axis")
         gs = gate.stride(0) if T > 1 else H
     out = torch.empty(T, H, R, dtype=qa.dtype, device=dev)
@@ -1586,7 +1623,7 @@ def window_attention(qn: torch.Tensor, qr: torch.Tensor, kn: torch.Tensor, kt: t
     dev = _need_cuda(qn=qn, qr=qr, kn=kn, kt=kt, v=v, gate=gate, sink_logits=sink_logits, out=out)
     T, H, dn = qn.shape
     dr, dv, N = qr.shape[2], v.shape[2], kn.shape[0]
-    if tuple(qr.shape) != (T, H, dr) or tuple(kn.shape) != (N, H, dn) or tuple(kt.shape) != (N, dr) or tuple(v.shape) != (N, H, dv):
+    if qr.shape != (T, H, dr) or kn.shape != (N, H, dn) or kt.shape != (N, dr) or v.shape != (N, H, dv):
         raise ValueError("qn [T, H, dn], qr [T, H, dr], kn [N, H, dn], kt [N, dr], v [N, H, dv]")
     for name, t in (("qn", qn), ("qr", qr), ("kn", kn), ("kt", kt), ("v", v)):
         if t.dtype != torch.bfloat16 or t.stride(-1) != 1:
@@ -1596,7 +1633,7 @@ def window_attention(qn: torch.Tensor, qr: torch.Tensor, kn: torch.Tensor, kt: t
     _f32(sink_logits, "sink_logits", (H,))
     gs, channels = 0, False
     if gate is not None:
-        if gate.dtype != torch.bfloat16 or tuple(gate.shape) not in ((T, H), (T, H * dv)) or (gate.shape[1] > 1 and gate.stride(1) != 1):
+        if gate.dtype != torch.bfloat16 or gate.shape not in ((T, H), (T, H * dv)) or (gate.shape[1] > 1 and gate.stride(1) != 1):
             raise ValueError("gate must be bf16 [T, H] or [T, H * dv] with a contiguous last axis")
         channels = gate.shape[1] != H
         gs = gate.stride(0) if T > 1 else gate.shape[1]
