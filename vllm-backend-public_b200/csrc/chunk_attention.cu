@@ -40,6 +40,7 @@
 // Sequences are described like everywhere in this library: rows cu_q[i] .. cu_q[i+1]-1, ctx_start[i] cached tokens
 // before them (< 0: padding, output rows are zeroed), block_tables[i, :].
 #include "b2_mask.cuh"
+#include "b2_tc5.cuh"
 
 namespace {
 
@@ -280,6 +281,190 @@ qk_rope_cache_vec_kernel(const T* __restrict__ qkv, int64_t qkv_stride, int H, i
         const int g = idx / pv, i = (idx - g * pv) * 4;
         *reinterpret_cast<Raw*>(v_cache + (((size_t)blk * Gv + g) * bs + off) * dv + i) = *reinterpret_cast<const Raw*>(vsrc + (size_t)idx * 4);
     }
+}
+
+// The same in bf16 with sixteen entries a thread: every size a multiple of sixteen, at most 1024 threads a row.  A thread keeps its
+// head, its place in it and its norm weights; with the rotation in halves its entries are 8 j .. and their partners.
+// RING: a CTA goes over rows gridDim.x apart, which come with their cosines and sines by bulk copies, kRopeStages ahead; without, a CTA
+// takes one row and loads it itself (a decode step has too few rows for the copies to run ahead).
+// Bound: memory, and the norm, which needs a whole row before its first result.  4096 rows of 32 + 8 heads of 128 with NORM (92 MB): kernel
+// above 39 us, this one 31; without NORM 16 + 4 heads 20.6 -> 10.4, 32 + 8 in neighbours 33 -> 27; a row ahead in registers instead of
+// the ring took 36 with NORM.  380 instructions a warp and row are half of the issue slots.
+constexpr int kRopeStages = 6;
+struct RopeArgs {
+    const __nv_bfloat16* qkv;
+    int64_t qkv_stride;
+    int rows, H, G, Gv, dk, dv, v_from_k, rot_dims;
+    const int32_t* positions;
+    const float* cos_sin;
+    int max_pos;
+    const int64_t* slots;
+    int bs, bs_log2;                                 // bs_log2 < 0: bs is no power of two
+    const float *q_w, *k_w;
+    float eps;
+    __nv_bfloat16 *q_out, *k_cache, *v_cache;
+    __host__ __device__ int width() const { return (H + G) * dk + (v_from_k ? 0 : Gv * dv); }
+    __host__ __device__ int stage_bytes() const { return (width() * 2 + rot_dims * 4 + 127) / 128 * 128; }
+};
+
+template <bool NORM, bool INTERLEAVED, bool RING>
+__global__ void __launch_bounds__(1024)
+qk_rope_cache_rows_kernel(const RopeArgs p) {
+    extern __shared__ __align__(128) unsigned char rope_sm[];
+    __shared__ __align__(8) uint64_t s_full[kRopeStages];
+    __shared__ float red[2][2][32];                  // [row's parity][q, k][warp]
+    __shared__ int s_failed;
+    using bf16 = __nv_bfloat16;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, dk = p.dk, per = dk / 16, half = p.rot_dims / 2;
+    const bool mine = tid < (p.H + p.G) * per;
+    const int hd = mine ? tid / per : 0, j = tid - (tid / per) * per;
+    const bool pairs = !INTERLEAVED && j < half / 8, is_q = hd < p.H;
+    const int ia = pairs ? 8 * j : INTERLEAVED ? 16 * j : p.rot_dims + 16 * (j - half / 8), ib = pairs ? ia + half : ia + 8;
+    const bool turns = mine && (INTERLEAVED ? ia < p.rot_dims : pairs);
+    const int count = RING ? (p.rows - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 1, stage = p.stage_bytes(), row_bytes = p.width() * 2;
+    auto position = [&](int row) {
+        const int pos = p.positions[row];
+        return pos < 0 ? 0 : (pos >= p.max_pos ? p.max_pos - 1 : pos);
+    };
+    auto full = [&](int s) { return b2::smem_u32(&s_full[s]); };
+    auto fetch = [&](int n, int pos) {               // one thread
+        const uint32_t dst = b2::smem_u32(rope_sm) + n % kRopeStages * stage, bar = full(n % kRopeStages);
+        b2::mbar_arrive_expect_tx(bar, row_bytes + p.rot_dims * 4);
+        b2::bulk_load(dst, p.qkv + (size_t)(blockIdx.x + n * gridDim.x) * p.qkv_stride, row_bytes, bar);
+        if (p.rot_dims) b2::bulk_load(dst + row_bytes, p.cos_sin + (size_t)pos * p.rot_dims, p.rot_dims * 4, bar);
+    };
+    int ahead_pos = 0;                               // thread 0: position of the next row to be fetched
+    if (NORM && tid < 128) red[tid >> 6][(tid >> 5) & 1][lane] = 0.f;
+    if (RING && tid == 0) {
+        s_failed = 0;
+        for (int s = 0; s < kRopeStages; ++s) b2::mbar_init(full(s), 1);
+        b2::fence_mbar_init();
+        for (int n = 0; n < min(count, kRopeStages); ++n) fetch(n, position(blockIdx.x + n * gridDim.x));
+        if (count > kRopeStages) ahead_pos = position(blockIdx.x + kRopeStages * gridDim.x);
+    }
+    if (RING || NORM) __syncthreads();
+    float wa[8], wb[8];
+    if (NORM && mine) {
+        const float* w = is_q ? p.q_w + (size_t)hd * dk : p.k_w + (size_t)(hd - p.H) * dk;
+#pragma unroll
+        for (int c = 0; c < 8; c += 4) {
+            const float4 u = *reinterpret_cast<const float4*>(w + ia + c), v = *reinterpret_cast<const float4*>(w + ib + c);
+            wa[c] = u.x; wa[c + 1] = u.y; wa[c + 2] = u.z; wa[c + 3] = u.w;
+            wb[c] = v.x; wb[c + 1] = v.y; wb[c + 2] = v.z; wb[c + 3] = v.w;
+        }
+    }
+    const bool some_q = __any_sync(0xffffffffu, mine && is_q), some_k = __any_sync(0xffffffffu, mine && !is_q);
+    int64_t next_slot = p.slots[blockIdx.x];
+    for (int n = 0; n < count; ++n) {
+        const int row = blockIdx.x + n * gridDim.x;
+        const int64_t slot = next_slot;
+        if (RING && n + 1 < count) next_slot = p.slots[row + gridDim.x];
+        const unsigned char* src = RING ? rope_sm + n % kRopeStages * stage : reinterpret_cast<const unsigned char*>(p.qkv + (size_t)row * p.qkv_stride);
+        const float* cs = RING ? reinterpret_cast<const float*>(src + row_bytes) : p.cos_sin + (turns ? (size_t)position(row) * p.rot_dims : 0);
+        if (RING) b2tc::wait(full(n % kRopeStages), n / kRopeStages & 1, &s_failed);
+        const bf16* head = reinterpret_cast<const bf16*>(src) + hd * dk;
+        uint4 ra = make_uint4(0, 0, 0, 0), rb = ra, rv = ra;
+        if (mine) {
+            ra = *reinterpret_cast<const uint4*>(head + ia);
+            rb = *reinterpret_cast<const uint4*>(head + ib);
+        }
+        const bool own_v = !p.v_from_k && tid < p.Gv * p.dv / 8;
+        if (own_v) rv = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(src) + (p.H + p.G) * dk + tid * 8);
+        float co[8], si[8];
+        if (turns)
+#pragma unroll
+            for (int c = 0; c < 8; c += 4) {
+                const float4 u = *reinterpret_cast<const float4*>(cs + 8 * j + c), v = *reinterpret_cast<const float4*>(cs + half + 8 * j + c);
+                co[c] = u.x; co[c + 1] = u.y; co[c + 2] = u.z; co[c + 3] = u.w;
+                si[c] = v.x; si[c + 1] = v.y; si[c + 2] = v.z; si[c + 3] = v.w;
+            }
+        float x[8], y[8];
+        {
+            const uint32_t u[8] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                x[2 * c] = __uint_as_float(u[c] << 16);
+                x[2 * c + 1] = __uint_as_float(u[c] & 0xffff0000u);
+                y[2 * c] = __uint_as_float(u[4 + c] << 16);
+                y[2 * c + 1] = __uint_as_float(u[4 + c] & 0xffff0000u);
+            }
+        }
+        float (&part)[2][32] = red[n & 1];
+        if (NORM) {
+            float s = 0.f;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) s = fmaf(x[c], x[c], fmaf(y[c], y[c], s));
+            if (some_q) {
+                const float t = b2::warp_sum(is_q ? s : 0.f);
+                if (lane == 0) part[0][wid] = t;
+            }
+            if (some_k) {
+                const float t = b2::warp_sum(is_q ? 0.f : s);
+                if (lane == 0) part[1][wid] = t;
+            }
+        }
+        if (NORM || RING) __syncthreads();           // the row is read; its sums are there (two sets of them: the next row's are not these)
+        if (RING && tid == 0 && n + kRopeStages < count && !*(volatile int*)&s_failed) {
+            fetch(n + kRopeStages, ahead_pos);
+            if (n + kRopeStages + 1 < count) ahead_pos = position(row + (kRopeStages + 1) * gridDim.x);
+        }
+        if (NORM) {
+            float t = 0.f;
+            if (some_q) t = b2::warp_sum(part[0][lane]);
+            if (some_k) {
+                const float tk = b2::warp_sum(part[1][lane]);
+                if (!is_q) t = tk;
+            }
+            const float inv = rsqrtf(t / (float)((is_q ? p.H : p.G) * dk) + p.eps);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                x[c] *= inv * wa[c];
+                y[c] *= inv * wb[c];
+            }
+        }
+        if (turns) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                if (!INTERLEAVED) {
+                    const float u = x[c], v = y[c];
+                    x[c] = fmaf(u, co[c], -v * si[c]);
+                    y[c] = fmaf(v, co[c], u * si[c]);
+                } else if (c % 2 == 0) {
+                    const float u = x[c], v = x[c + 1], u2 = y[c], v2 = y[c + 1];
+                    x[c] = fmaf(u, co[c / 2], -v * si[c / 2]);
+                    x[c + 1] = fmaf(v, co[c / 2], u * si[c / 2]);
+                    y[c] = fmaf(u2, co[4 + c / 2], -v2 * si[4 + c / 2]);
+                    y[c + 1] = fmaf(v2, co[4 + c / 2], u2 * si[4 + c / 2]);
+                }
+            }
+        }
+        if (RING && *(volatile int*)&s_failed) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) x[c] = y[c] = __int_as_float(0x7fc00000);
+        }
+        int64_t blk = 0;
+        int off = 0;
+        if (slot >= 0) {
+            if (p.bs_log2 >= 0) { blk = slot >> p.bs_log2; off = (int)slot & (p.bs - 1); }
+            else { blk = slot / p.bs; off = (int)(slot % p.bs); }
+        }
+        if (mine && (is_q || slot >= 0)) {
+            const size_t pool = ((size_t)blk * p.G + (hd - p.H)) * p.bs + off;
+            bf16* dst = is_q ? p.q_out + ((size_t)row * p.H + hd) * dk : p.k_cache + pool * dk;
+            b2::st8(dst + ia, x);
+            b2::st8(dst + ib, y);
+            if (p.v_from_k && !is_q) {               // a value head per key head, of its size
+                *reinterpret_cast<uint4*>(p.v_cache + pool * p.dv + ia) = ra;
+                *reinterpret_cast<uint4*>(p.v_cache + pool * p.dv + ib) = rb;
+            }
+        }
+        if (own_v && slot >= 0) {
+            const int g = tid * 8 / p.dv, i = tid * 8 - g * p.dv;
+            *reinterpret_cast<uint4*>(p.v_cache + (((size_t)blk * p.Gv + g) * p.bs + off) * p.dv + i) = rv;
+        }
+    }
+    if (RING && *(volatile int*)&s_failed)           // what is still on its way to this CTA's memory
+        for (int n = max(0, count - kRopeStages); n < count; ++n) b2tc::drain(full(n % kRopeStages), n / kRopeStages & 1);
 }
 
 template <typename T>
@@ -1632,6 +1817,34 @@ extern "C" int b2_qk_norm_rope_cache(const void* qkv, int64_t qkv_stride, int ac
     KERN<A, NORM><<<T, threads, 0, st>>>(static_cast<const A*>(qkv), qkv_stride, H, G, Gv, dk, dv, v_from_k != 0, rot_dims,         \
                                          interleaved != 0, positions, cos_sin, max_pos > 0 ? max_pos : 1, slots, bs, q_w, k_w, eps, \
                                          static_cast<A*>(q_out), static_cast<A*>(k_cache), static_cast<A*>(v_cache))
+    const int row_threads = ((H + G) * (dk / 16) + 31) / 32 * 32;
+    if (act_dtype == B2_ACT_BF16 && dk % 16 == 0 && rot_dims % 16 == 0 && dv % 8 == 0 && qkv_stride % 8 == 0 && row_threads <= 1024 && row_threads >= 128 &&
+        (v_from_k || Gv * dv / 8 <= row_threads) && b2_aligned16(qkv) && b2_aligned16(q_out) && b2_aligned16(k_cache) && b2_aligned16(v_cache) &&
+        b2_aligned16(q_w) && b2_aligned16(k_w) && b2_aligned16(cos_sin)) {
+        const RopeArgs a{static_cast<const __nv_bfloat16*>(qkv), qkv_stride, T, H, G, Gv, dk, dv, v_from_k != 0, rot_dims, positions, cos_sin,
+                         max_pos > 0 ? max_pos : 1, slots, bs, bs & (bs - 1) ? -1 : __builtin_ctz(bs), q_w, k_w, eps,
+                         static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache)};
+        // the ring where every CTA has several rows: 64 rows 4.2 us without it, and its copies could not run ahead
+        const int smem = kRopeStages * a.stage_bytes(), per_sm = 1024 / row_threads, fit = 216 * 1024 / (smem + 2048);
+        const int ctas = (fit < per_sm ? fit : per_sm) * b2_sm_count();
+        const bool ring = ctas > 0 && T >= 2 * ctas;
+#define B2_ROPE_ROWS(NORM, IL)                                                                                                  \
+    do {                                                                                                                        \
+        if (ring) {                                                                                                             \
+            auto kern = qk_rope_cache_rows_kernel<NORM, IL, true>;                                                                \
+            B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));                           \
+            kern<<<ctas, row_threads, smem, st>>>(a);                                                                             \
+        } else {                                                                                                                \
+            qk_rope_cache_rows_kernel<NORM, IL, false><<<T, row_threads, 0, st>>>(a);                                             \
+        }                                                                                                                       \
+    } while (0)
+        if (q_w) { if (interleaved) B2_ROPE_ROWS(true, true); else B2_ROPE_ROWS(true, false); }
+        else if (interleaved) B2_ROPE_ROWS(false, true);
+        else B2_ROPE_ROWS(false, false);
+#undef B2_ROPE_ROWS
+        B2_CUDA_OK(cudaGetLastError());
+        return B2_OK;
+    }
     B2_DISPATCH_ACT(act_dtype, A, {
         if (vec && q_w) B2_ROPE(qk_rope_cache_vec_kernel, true);
         else if (vec) B2_ROPE(qk_rope_cache_vec_kernel, false);
