@@ -14,7 +14,9 @@
 // 8 x 8 / 4 x 8 a thread (shared-memory reads cost about 0.7 of the FMA cycles).  Per channel the decays stand between k and q, so
 // pairs of tokens of a segment of 16 are taken one by one, and those of different segments as products of rows decayed to and
 // from a boundary between them.  A warp per column with its sums in butterflies, over segments of 32, took 350 us of 4096 tokens'
-// scan (16 heads of 128), this one about 110: a third of the pairs, and one transposing sum for 16 of them.  The choice between chunks and tokens is at the end.
+// scan (16 heads of 128), this one about 110: a third of the pairs, and one transposing sum for 16 of them.  Keys and queries come four vectors in flight, P and T
+// leave as vectors, and the triangular solve takes two rows at a time: 76 -> 66 us per head (3001 tokens, delta).  The choice between chunks
+// and tokens is at the end.
 #include "b2_act.cuh"
 
 #include <math.h>
@@ -63,6 +65,7 @@ chunk_prep_kernel(const ChunkArgs a) {
     static_assert(CH || DELTA, "chunk_tc5.cu");
     extern __shared__ __align__(16) float sm[];
     __shared__ int s_at[2];
+    __shared__ double s_tail[CH ? 1 : C], s_seg[4];  // per head: the decays from s + 1 to the end of its segment; segments
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, hh = blockIdx.y;
     const int dk = a.dk, dv = a.dv, LD = dk + 4, per = dk / 4;
     if (tid == 0) find_chunk(a, blockIdx.x, s_at);
@@ -74,21 +77,31 @@ chunk_prep_kernel(const ChunkArgs a) {
     float* Ps = qs + C * LD;                         // [C][C + 1]
     float* As = Ps + C * (C + 1);                    // [C][C + 1] (delta)
     float* gs = As + (DELTA ? C * (C + 1) : 0);      // [C], per channel [C][LD]
-    float* bs = gs + (CH ? C * LD : C);              // [C] beta; per head 4 + C more
+    float* bs = gs + (CH ? C * LD : C);              // [C] beta
     const int Cq = 2 * a.G * dk + a.H * dv, kvh = hh / (a.H / a.G);
     const float* qrow = a.qkv + (size_t)r0 * Cq + (size_t)kvh * dk;
     const float* krow = qrow + (size_t)a.G * dk;
-    for (int idx = tid; idx < C * per; idx += NT) {
-        const int t = idx / per, c = (idx - t * per) * 4;
-        float4 k = make_float4(0.f, 0.f, 0.f, 0.f), q = k, g = make_float4(1.f, 1.f, 1.f, 1.f);
-        if (t < nt) {
-            k = *reinterpret_cast<const float4*>(krow + (size_t)t * Cq + c);
-            q = *reinterpret_cast<const float4*>(qrow + (size_t)t * Cq + c);
-            if (CH) g = *reinterpret_cast<const float4*>(a.decay + ((size_t)(r0 + t) * a.H + hh) * dk + c);
+    for (int base = tid; base < C * per; base += 4 * NT) {           // four vectors a thread in flight
+        float4 k[4], q[4], g[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int idx = base + u * NT, t = idx / per, c = (idx - t * per) * 4;
+            k[u] = q[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            g[u] = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (t < nt) {
+                k[u] = *reinterpret_cast<const float4*>(krow + (size_t)t * Cq + c);
+                q[u] = *reinterpret_cast<const float4*>(qrow + (size_t)t * Cq + c);
+                if (CH) g[u] = *reinterpret_cast<const float4*>(a.decay + ((size_t)(r0 + t) * a.H + hh) * dk + c);
+            }
         }
-        *reinterpret_cast<float4*>(ks + t * LD + c) = k;
-        *reinterpret_cast<float4*>(qs + t * LD + c) = q;
-        if (CH) *reinterpret_cast<float4*>(gs + t * LD + c) = g;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int idx = base + u * NT, t = idx / per, c = (idx - t * per) * 4;
+            if (t >= C) break;
+            *reinterpret_cast<float4*>(ks + t * LD + c) = k[u];
+            *reinterpret_cast<float4*>(qs + t * LD + c) = q[u];
+            if (CH) *reinterpret_cast<float4*>(gs + t * LD + c) = g[u];
+        }
     }
     if (tid < C) {
         if (!CH) gs[tid] = tid < nt ? a.decay[(size_t)(r0 + tid) * a.H + hh] : 1.f;
@@ -251,34 +264,32 @@ chunk_prep_kernel(const ChunkArgs a) {
         }
     } else {
         // the decay ratios of all (t, s), and the products from the chunk's start and to its end: by segments of 16 tokens, a chain of
-        // 16 + 16 products instead of 64
-        float* seg = As + (DELTA ? C * (C + 1) : 0) + 2 * C;         // behind g and beta: [4] segments | [C] from s + 1 to the end of its segment
-        float* tail = seg + 4;
+        // 16 + 16 products instead of 64, in 64 bits
         const int col = tid & (C - 1), sg = tid >> 6, own = col >> 4;
         if (tid < C) {
-            float run = 1.f;
+            double run = 1.;
             for (int r = tid + 1; r < (tid | 15) + 1; ++r) run *= gs[r];
-            tail[tid] = run;
-            if ((tid & 15) == 0) seg[tid >> 4] = run * gs[tid];
+            s_tail[tid] = run;
+            if ((tid & 15) == 0) s_seg[tid >> 4] = run * gs[tid];
         }
         __syncthreads();
         {
-            float run = tail[col];
-            for (int m = own + 1; m < sg; ++m) run *= seg[m];
-            if (sg == own) run = 1.f;
+            double run = s_tail[col];
+            for (int m = own + 1; m < sg; ++m) run *= s_seg[m];
+            if (sg == own) run = 1.;
 #pragma unroll 4
             for (int t = sg * 16; t < sg * 16 + 16; ++t) {
                 if (t > col) run *= gs[t];
-                Ps[t * (C + 1) + col] = t >= col ? run : 0.f;
+                Ps[t * (C + 1) + col] = t >= col ? (float)run : 0.f;
             }
         }
         if (tid < C) {
-            float to = tail[tid], from = 1.f;
-            for (int m = own + 1; m < 4; ++m) to *= seg[m];
-            for (int m = 0; m < own; ++m) from *= seg[m];
+            double to = s_tail[tid], from = 1.;
+            for (int m = own + 1; m < 4; ++m) to *= s_seg[m];
+            for (int m = 0; m < own; ++m) from *= s_seg[m];
             for (int r = own * 16; r <= tid; ++r) from *= gs[r];
-            dec[tid] = from;
-            dec[C + tid] = to;
+            dec[tid] = (float)from;
+            dec[C + tid] = (float)to;
         }
         __syncthreads();
         pair_t acc[8][4];                            // sums over even and odd entries; blocks above the diagonal are left out
@@ -311,7 +322,10 @@ chunk_prep_kernel(const ChunkArgs a) {
         }
     }
     __syncthreads();
-    for (int idx = tid; idx < C * C; idx += NT) out[idx] = Ps[(idx / C) * (C + 1) + idx % C];
+    for (int idx = tid * 4; idx < C * C; idx += NT * 4) {
+        const float* p = Ps + (idx / C) * (C + 1) + idx % C;
+        *reinterpret_cast<float4*>(out + idx) = make_float4(p[0], p[1], p[2], p[3]);
+    }
     if (DELTA) {
         // the inverse of I + A by halves: forward substitution on the diagonal blocks (a warp each, a lane per column), then
         // T21 = -T22 A21 T11; Ps is free and takes T
@@ -320,10 +334,10 @@ chunk_prep_kernel(const ChunkArgs a) {
             float T[32];
 #pragma unroll
             for (int t = 0; t < 32; ++t) {
-                float v = t == lane ? 1.f : 0.f;
+                float v = t == lane ? 1.f : 0.f, v1 = 0.f;           // two chains
 #pragma unroll
-                for (int s = 0; s < t; ++s) v = fmaf(-As[(o + t) * (C + 1) + o + s], T[s], v);
-                T[t] = v;
+                for (int s = 0; s < t; ++s) (s & 1 ? v1 : v) = fmaf(-As[(o + t) * (C + 1) + o + s], T[s], s & 1 ? v1 : v);
+                T[t] = v + v1;
             }
             __syncwarp();
             asm volatile("bar.sync 1, 64;" ::: "memory");            // both warps are done reading A's diagonal blocks ...
@@ -356,9 +370,13 @@ chunk_prep_kernel(const ChunkArgs a) {
         }
         __syncthreads();
         float* to = out + a.t_at;
-        for (int idx = tid; idx < C * C; idx += NT) {
+        for (int idx = tid * 4; idx < C * C; idx += NT * 4) {
             const int t = idx / C, s = idx % C;
-            to[idx] = s <= t ? As[t * (C + 1) + s] * bs[s] : 0.f;
+            const float* p = As + t * (C + 1) + s;
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = s + e <= t ? p[e] * bs[s + e] : 0.f;
+            *reinterpret_cast<float4*>(to + idx) = make_float4(v[0], v[1], v[2], v[3]);
         }
     }
 }
@@ -373,7 +391,7 @@ template <bool CH, bool DELTA>
 int launch_prep(const ChunkArgs& a, int total_rows, cudaStream_t st) {
     const int chunks = total_rows / C + a.n_seq;     // upper bound on sum(ceil(len / C)); spare CTAs leave at once
     const size_t LD = a.dk + 4, rows = C * LD;
-    const size_t psm = sizeof(float) * (2 * rows + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows + 4 * 128 : 2 * C + 4) + C);
+    const size_t psm = sizeof(float) * (2 * rows + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows + 4 * 128 : C) + C);
     int rc = allow(chunk_prep_kernel<CH, DELTA>, psm);
     if (rc != B2_OK) return rc;
     chunk_prep_kernel<CH, DELTA><<<dim3(chunks, a.H), CH ? 512 : 256, psm, st>>>(a);
@@ -399,9 +417,9 @@ int64_t b2_internal_chunk_scan_floats(int total_rows, int n_seq, int H, int dk, 
 //   chunks   one decay per head without delta (chunk_tc5.cu): 20, 0.2 a chunk of 128 and head for the products (0.14 at 64 x 64) and 0.03 a
 //            sequence and head for its state; at least 33 (29 to dk = 64): three launches
 //            else 0.3 (per channel 20 and 0.27 / 0.46) a chunk of 64 and head for the products, 0.11 a sequence and head for its state, with
-//            delta 2.7 a step of the chain and SM's share of CTAs; at least 60 (39 / 72 per channel; to dk = 64 49, 33 / 58): four launches
-// Measured, tokens -> chunks: 1 x 4096 tokens, 16 heads: 804 -> 121, 1160 -> 442, 963 -> 298, 1255 -> 582; 1 x 500: 102 -> 34,
-// 146 -> 72, 121 -> 43, 158 -> 88; 1500 + 1000 + 501: 411 -> 92, 573 -> 290, 503 -> 235, 631 -> 407; 16 x 100: 121 -> 74, 181 -> 166, but 160 -> 196 and
+//            delta 2.7 a step of the chain and SM's share of CTAs; at least 56 (39 / 72 per channel; to dk = 64 49, 33 / 58): four launches
+// Measured, tokens -> chunks: 1 x 4096 tokens, 16 heads: 804 -> 121, 1160 -> 426, 963 -> 288, 1255 -> 571; 1 x 500: 102 -> 34,
+// 146 -> 69, 121 -> 43, 158 -> 84; 1 x 200 with delta: 62 -> 57; 1500 + 1000 + 501: 411 -> 92, 573 -> 279, 503 -> 225, 631 -> 399; 16 x 100: 121 -> 74, 181 -> 160, but 160 -> 196 and
 // 223 -> 274 with delta, which are left to the tokens, as are 64 x 24: 148 -> 250, 180 -> 415, 193 -> 379, and 1 x 130: 29 -> 33, 41 -> 58, 35 -> 40.
 bool b2_internal_chunk_scan_pays(int total_rows, int n_seq, int H, int dk, int dv, bool ch, bool delta) {
     if (total_rows < 2 * n_seq) return false;
@@ -409,7 +427,7 @@ bool b2_internal_chunk_scan_pays(int total_rows, int n_seq, int H, int dk, int d
     const int kind = (ch ? 2 : 0) + (delta ? 1 : 0), run_as = dk <= 32 ? 32 : dk <= 64 ? 64 : 128;
     const float chain_tok[4] = {0.20f, 0.285f, 0.235f, 0.31f}, rate_few[4] = {5.2e-3f, 7.1e-3f, 10.6e-3f, 12.4e-3f}, rate_many[4] = {5.0e-3f, 6.3e-3f, 6.8e-3f, 8.3e-3f};
     const float per_chunk[4] = {0.f, 0.3f, 0.27f, 0.46f};
-    const float least[4] = {dk <= 64 ? 29.f : 33.f, dk <= 64 ? 49.f : 60.f, dk <= 64 ? 33.f : 39.f, dk <= 64 ? 58.f : 72.f};
+    const float least[4] = {dk <= 64 ? 29.f : 33.f, dk <= 64 ? 49.f : 56.f, dk <= 64 ? 33.f : 39.f, dk <= 64 ? 58.f : 72.f};
     const float many = fminf(1.f, fmaxf(0.f, log2f(n_seq / 2.5f) / 4.f)), rate = rate_few[kind] + (rate_many[kind] - rate_few[kind]) * many;
     const float longest = len * (n_seq > 1 ? 1.25f : 1.f);
     const float tokens = (run_as == dk ? 1.f : 1.33f) * fmaxf(chain_tok[kind] * (dk <= 64 ? 0.75f : 1.f) * longest, rate * (float)total_rows * H * run_as * dv / 16384.f);
