@@ -44,3 +44,38 @@ def test_prompt_rows_equal_those_of_smaller_batches(cuda, dt, H, G, dk, dv, unit
     for x, *y in zip(whole, *parts):
         if x is not None:
             assert torch.equal(torch.cat([x[:100], x[103:]]), torch.cat(y))
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,dk,dv,taps", [(4, 64, 64, 4), (2, 32, 20, 3), (16, 128, 128, 2), (1, 8, 4, 4)])
+@pytest.mark.parametrize("lengths", [[300, 1, 2, 7, 301], [1, 509, 4, 3, 500, 90, 511, 505], [1] * 513, [400, 300] * 3])
+def test_runs_over_several_sequences_equal_each_alone(cuda, dt, H, dk, dv, taps, lengths):
+    """From 512 rows on a CTA goes through a run of rows: a sequence that begins or ends within one keeps its own history.  Alone each is
+    below that, a row a CTA; the sums are the same, so are the bits."""
+    C, T, n = 2 * H * dk + H * dv, sum(lengths), len(lengths)
+    g = torch.Generator(device=cuda).manual_seed(taps + n)
+    proj = torch.randn(T, C + H * dv + 2 * H, generator=g, device=cuda).to(dt)
+    proj = torch.nn.functional.pad(proj, (0, -proj.shape[1] % 8))
+    conv_w = torch.randn(C, taps, generator=g, device=cuda)
+    state = torch.randn(n, taps - 1, C, generator=g, device=cuda).to(dt)
+    bias = torch.rand(H, generator=g, device=cuda)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    cu = [0]
+    for x in lengths:
+        cu.append(cu[-1] + x)
+    ctx = [-1 if s == 3 else s % 2 * 5 for s in range(n)]                # one is padding, every second begins
+
+    def call(rows, cu, ctx, slots, m):
+        kept = state.clone()
+        b = ops.SeqBatch(i32(cu), i32(ctx), None, i32(slots), len(ctx), m)
+        return ops.delta_prep(rows, C + H * dv, C + H * dv + H, H, H, dk, dv, taps, conv_w, bias, bias, b, kept), kept
+
+    whole, states = call(proj, cu, ctx, list(range(n)), T)
+    for s in range(0, n, max(1, n // 8)):
+        if ctx[s] < 0:
+            continue
+        lo, hi = cu[s], cu[s + 1]
+        part, kept = call(proj[lo:hi], [0, hi - lo], [ctx[s]], [s], hi - lo)
+        for x, y in zip(whole, part):
+            assert torch.equal(x[lo:hi], y)
+        assert torch.equal(states[s], kept[s])

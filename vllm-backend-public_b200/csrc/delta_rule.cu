@@ -29,6 +29,8 @@
 // sequence with ctx_start = 0 starts from a zero state whatever the slot holds, so slots need no clearing on reuse.
 #include "b2_act.cuh"
 
+#include <type_traits>
+
 namespace {
 
 constexpr int kMaxTaps = 16;
@@ -138,7 +140,8 @@ __global__ void recur_prep_kernel(const T* __restrict__ proj, int64_t proj_strid
 // and not eight: 64 registers let four CTAs share an SM, and a warp's stores are 512 consecutive bytes.
 // Bound: memory (2 or 4 bytes in and 4 out per channel), with the exact exponentials and divisions of the activation close behind.
 // One CTA a row with scalar accesses and a staging pass took 88 us at 4096 rows of 6144 channels (rotation, no convolution), 174 at 3001
-// rows (four taps, SiLU, unit vectors) and 59 at 64 rows; this one 58, 63 and 27.  Without a convolution recur_prep_heads_kernel takes prompts.
+// rows (four taps, SiLU, unit vectors) and 59 at 64 rows; this one 58, 53 and 27 (the second 63
+// with the inputs moved from place to place and runs of 8).  Without a convolution recur_prep_heads_kernel takes prompts.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(256, 4)
 recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec sp, const float* __restrict__ conv_w,
@@ -154,13 +157,14 @@ recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec 
     const bool turns = head && i0 < sp.rot_dims;
     const bool second = !sp.interleaved && i0 >= half;
     const float scale = c0 < G * dk ? sp.q_scale : sp.k_scale;
-    float w[TAPS][4], hist[TAPS][4];                 // hist[j]: the input j rows back
+    constexpr int RING = TAPS + 1;                   // the last TAPS inputs and the next one: row r_begin + i in place i % RING
+    float w[TAPS][4], ring[RING][4];
 #pragma unroll
-    for (int j = 0; j < TAPS; ++j)
+    for (int j = 0; j < RING; ++j)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            hist[j][c] = 0.f;
-            w[j][c] = 1.f;
+            ring[j][c] = 0.f;
+            if (j < TAPS) w[j][c] = 1.f;
         }
     if (conv_w && channel) {
 #pragma unroll
@@ -185,15 +189,12 @@ recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec 
         for (int c = 0; c < 4; ++c) dbias[c] = sp.bias ? sp.bias[d0 + c] : 0.f;
     }
     int seq = -1, seq_end = r_begin, seq_begin = 0, ctx = -1;
-    float next[4];                                   // a row ahead: nothing of it depends on the row before
-#pragma unroll
-    for (int c = 0; c < 4; ++c) next[c] = 0.f;
-    if (channel) b2::ld4(proj + (size_t)r_begin * proj_stride + c0, next);
-    for (int row = r_begin; row < r_end; ++row) {
-        float now[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) now[c] = next[c];
-        if (channel && row + 1 < r_end) b2::ld4(proj + (size_t)(row + 1) * proj_stride + c0, next);
+    // value columns have neither unit vectors nor a rotation: whole warps of them skip both
+    const bool some_head = __any_sync(0xffffffffu, head), unit = sp.unit && some_head, rotates = sp.rot_dims && some_head;
+    if (channel) b2::ld4(proj + (size_t)r_begin * proj_stride + c0, ring[0]);
+    auto step = [&](auto place, int row) {
+        constexpr int U = decltype(place)::value;
+        if (channel && row + 1 < r_end) b2::ld4(proj + (size_t)(row + 1) * proj_stride + c0, ring[(U + 1) % RING]);
         bool fresh = row == r_begin;
         if (row >= seq_end) {                        // the next sequence with rows
             seq = b2::seq_of_row(cu_q, n_seq, row);
@@ -202,55 +203,50 @@ recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec 
             ctx = ctx_start[seq];
             fresh = true;
         }
-        if (ctx < 0) continue;
+        if (ctx < 0) return;
         const int li = row - seq_begin;
-        if (channel) {
-            if (TAPS > 1) {
-                if (fresh) {                         // inputs before this row: earlier rows of the portion, then the state's tail
-                    const int slot = state_slot[seq];
-                    const T* st = slot >= 0 && ctx > 0 ? conv_state + (size_t)slot * (TAPS - 1) * C : nullptr;
+        if (TAPS > 1 && fresh && channel) {          // inputs before this row: earlier rows of the portion, then the state's tail
+            const int slot = state_slot[seq];
+            const T* st = slot >= 0 && ctx > 0 ? conv_state + (size_t)slot * (TAPS - 1) * C : nullptr;
 #pragma unroll
-                    for (int j = 1; j < TAPS; ++j) {
-                        const int l = li - j;
-                        if (l >= 0) {
-                            b2::ld4(proj + (size_t)(row - j) * proj_stride + c0, hist[j]);
-                        } else if (ctx + l >= 0 && st) {
-                            b2::ld4(st + (size_t)(l + TAPS - 1) * C + c0, hist[j]);
-                        } else {
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) hist[j][c] = 0.f;
-                        }
-                    }
+            for (int j = 1; j < TAPS; ++j) {
+                float (&h)[4] = ring[(U - j + RING) % RING];
+                const int l = li - j;
+                if (l >= 0) {
+                    b2::ld4(proj + (size_t)(row - j) * proj_stride + c0, h);
+                } else if (ctx + l >= 0 && st) {
+                    b2::ld4(st + (size_t)(l + TAPS - 1) * C + c0, h);
                 } else {
 #pragma unroll
-                    for (int j = TAPS - 1; j > 0; --j)
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) hist[j][c] = hist[j - 1][c];
+                    for (int c = 0; c < 4; ++c) h[c] = 0.f;
                 }
             }
-#pragma unroll
-            for (int c = 0; c < 4; ++c) hist[0][c] = now[c];
         }
         float x[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            x[c] = hist[0][c];
+            x[c] = ring[U][c];
             if (TAPS > 1 || conv_w) {
                 x[c] = 0.f;
 #pragma unroll
-                for (int j = 0; j < TAPS; ++j) x[c] = fmaf(w[j][c], hist[j][c], x[c]);
+                for (int j = 0; j < TAPS; ++j) x[c] = fmaf(w[j][c], ring[(U - j + RING) % RING][c], x[c]);
             }
-            if (sp.act && channel) x[c] = b2::silu_f(x[c]);
+        }
+        if (sp.act && channel) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) x[c] = b2::silu_f(x[c]);
         }
         float sc = scale;
-        if (sp.unit) {                               // every lane takes part: heads and value columns may share a warp
+        if (unit) {                                  // every lane takes part: heads and value columns may share a warp
             float ss = 0.f;
 #pragma unroll
             for (int c = 0; c < 4; ++c) ss = fmaf(x[c], x[c], ss);
-            for (int m = 1; m < P; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+#pragma unroll
+            for (int m = 1; m < 32; m <<= 1)
+                if (m < P) ss += __shfl_xor_sync(0xffffffffu, ss, m);
             sc *= rsqrtf(ss + sp.unit_eps);
         }
-        if (sp.rot_dims) {
+        if (rotates) {
             const float* cs = sp.cos_sin + (size_t)min(ctx + li, sp.max_pos - 1) * sp.rot_dims;
             if (sp.interleaved) {
                 if (turns) {
@@ -291,6 +287,13 @@ recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec 
             float* o = decay + (size_t)row * H * dk + d0;
             *reinterpret_cast<float4*>(o) = make_float4(z[0], z[1], z[2], z[3]);
         }
+    };
+    for (int base = r_begin; base < r_end; base += RING) {           // unrolled: nothing moves from place to place
+        step(std::integral_constant<int, 0>(), base);
+        if (base + 1 < r_end) step(std::integral_constant<int, 1>(), base + 1);
+        if constexpr (RING > 2) { if (base + 2 < r_end) step(std::integral_constant<int, 2>(), base + 2); }
+        if constexpr (RING > 3) { if (base + 3 < r_end) step(std::integral_constant<int, 3>(), base + 3); }
+        if constexpr (RING > 4) { if (base + 4 < r_end) step(std::integral_constant<int, 4>(), base + 4); }
     }
     if (blockIdx.y) return;
     for (int idx = threadIdx.x; idx < (r_end - r_begin) * H; idx += 256) {
@@ -874,10 +877,25 @@ int launch_prep(const void* proj, int64_t proj_stride, const PrepSpec& sp, int T
                      (sp.taps == 1 || (b2_aligned16(conv_state) && b2_aligned16(conv_w))) && (!sp.rot_dims || b2_aligned16(sp.cos_sin)) &&
                      (!channel_decay || (b2_aligned16(sp.a) && sp.a_stride % 4 == 0 && b2_aligned16(decay)));
     if (vec) {
-        // rows a CTA: long runs read the convolution's inputs once; small batches spread over the SMs instead.  Runs of 1 / 4 / 16 rows:
-        // 349 / 140 / 85 us at 3001 rows of four taps, 128 / 57 / 46 at 1000, 38 / 42 / 72 at 64 (before the channels went from eight to four)
-        const int run = T >= 2048 ? 8 : T >= 512 ? 4 : 1;
-        const dim3 grid((T + run - 1) / run, ((C + (channel_decay ? sp.H * sp.dk : 0)) / 4 + 255) / 256);
+        // Rows a CTA: long runs read the convolution's inputs once, and the CTAs should fill whole waves (four an SM): a wave of runs of n rows
+        // is taken as n + 3 rows.  4096 rows of 6144 channels: runs of 8 / 15 / 16 / 20 rows 80 / 74 / 77 / 85 us, by this rule (21, just below two waves)
+        // 71; 3001: 8 / 15 / 16 59.5 / 65 / 55, by the rule (31, one wave) 53; 1000: 5 / 8 / 10 24.7 / 24.7 / 26.8, by the rule (11) 20.7.
+        // Below 512 rows one row a CTA, and runs no longer than 4 or 8 over sequences that are shorter: each of them is looked up and its
+        // history fetched, one after another.
+        const int columns = ((C + (channel_decay ? sp.H * sp.dk : 0)) / 4 + 255) / 256, slots = 4 * b2_sm_count();
+        const int most = T < 512 ? 1 : min(32, max(T >= 2048 ? 8 : 4, T / n_seq));
+        int run = 1;
+        int64_t best = INT64_MAX;
+        for (int waves = 1; waves <= 8 && most > 1; ++waves) {
+            const int64_t n = ((int64_t)T * columns + (int64_t)waves * slots - 1) / ((int64_t)waves * slots);
+            const int rows = (int)(n < most ? n : most);
+            const int64_t ctas = (int64_t)((T + rows - 1) / rows) * columns, cost = (ctas + slots - 1) / slots * (rows + 3);
+            if (cost < best) {
+                best = cost;
+                run = rows;
+            }
+        }
+        const dim3 grid((T + run - 1) / run, columns);
 #define B2_PREP_VEC(TAPS)                                                                                                    \
     recur_prep_vec_kernel<A, TAPS><<<grid, 256, 0, st>>>(static_cast<const A*>(proj), proj_stride, sp, conv_w, cu_q, ctx_start, state_slot, \
                                                          n_seq, T, run, static_cast<const A*>(conv_state), qkv, beta, decay)
