@@ -56,6 +56,10 @@ __device__ __forceinline__ void clean(float (&x)[8], F&& bad) {
 // ---------------------------------------------------------------------------------------------------------------- W, U_0 and their products
 // Tiles in shared memory: X0 for G K and later G_C/G K, X1 for V and later U_0, Y for W, T and P; in the end 16 KB and X0 for F, X1 and Y
 // for M, T and P for Q'.
+// Bound by its own phases: with 208 KB of tiles and copies one CTA fits an SM, and an item of 64 tokens goes through ten of them (loads, split,
+// product, read back, split ...), 33e3 cycles, 7e3 of which the copies out take (29 bytes a cycle).  1024 items (4096 tokens, 16 heads of
+// 128) 108 us: 122 with the keys read where they are needed instead of an item ahead, 115 with the decays read per token.  The same work
+// was part of the chain before and took it 196 us on the FMA pipe, where nothing ran beside it.
 template <bool CH, bool DELTA>
 __global__ void __launch_bounds__(512, 1)
 wy_kernel(const Args a) {
@@ -354,6 +358,9 @@ __device__ __forceinline__ int first_chunk(const Args& a, int seq) {
 
 // A CTA per 64 columns of a head's state.  Eight warps keep it in registers, in fp32 (lane a key feature, 32 columns a thread), and
 // write its parts; one warp copies M ahead, three slices of 64 features in a ring; one multiplies and copies the parts out.
+// Bound by one SM's intake: a step's 96 KB of M come at 54 bytes a cycle, 0.95 us, beside which split, product and read-back of the step take
+// place; 64 chunks, 16 heads of 128 x 128, 61 us, where W and U on the FMA pipe within the chain took 196.  32 columns a CTA would
+// put twice the SMs to work, each with the same M.
 template <bool CH>
 __global__ void __launch_bounds__(320, 1)
 chain_kernel(const Args a) {
@@ -541,6 +548,7 @@ state_kernel(const Args a) {
 
 // ---------------------------------------------------------------------------------------------------------------- read-out
 // O^T += S_0^T Q'^T: both operands are copied as they are, three stages of a slice of 64 features (72 KB); two accumulators alternate.
+// Bound by the copies: 4096 tokens, 16 heads of 128, 29 us for 151 MB of images and 67 of outputs, part of them in L2 (the FMA pipe took 84).
 template <bool CH, bool DELTA>
 __global__ void __launch_bounds__(320, 1)
 read_kernel(const Args a) {
