@@ -135,6 +135,8 @@ kv_kernel(const Args a) {
         before = at;
         at = next;
     }
+    // (within the loop the next item's first slice waits for it; commits of different threads promise no order among one another)
+    wait(done(0), (n - 1) & 1, &s_failed);
     finish();
     if (*(volatile int*)&s_failed)
         for (int u = 0; u < 2; ++u) drain(done(u), (n - 1) & 1);
