@@ -179,65 +179,67 @@ chunk_prep_kernel(const ChunkArgs a) {
         __syncthreads();
         // A thread takes a channel of a segment: its decays from the segment's start and to its end, then the copies for delta_tc5.cu.
         // Rows decayed from their segment's start replace q and (in the decays' place) k, k decayed to its segment's end replaces k.
-        float* total = bs + C;                       // [4][128] the segments' whole products
+        double* total = reinterpret_cast<double*>(bs + C);           // [4][128] the segments' whole products
         {
             const int i = tid & 127, b = tid >> 7, t0 = b * 16;
-            float f[16], k[16];
+            double f[16];
             if (i < dk) {
-                float run = 1.f;
+                double run = 1.;
 #pragma unroll
                 for (int t = 0; t < 16; ++t) {
                     run *= gs[(t0 + t) * LD + i];
                     f[t] = run;
-                    k[t] = ks[(t0 + t) * LD + i];
                 }
                 total[b * 128 + i] = run;
             }
             __syncthreads();
             if (i < dk) {
-                float before = 1.f, after = 1.f;
+                double before = 1., after = 1.;
                 for (int m = 0; m < b; ++m) before *= total[m * 128 + i];
                 for (int m = 3; m > b; --m) after *= total[m * 128 + i];
                 if (b == 3) dec[3 * C * dk + i] = before * f[15];
-                float run = 1.f;
+                double run = 1.;
 #pragma unroll
                 for (int t = 15; t >= 0; --t) {
-                    const float to = run * k[t];
-                    dec[(2 * C + t0 + t) * dk + i] = after * to;
-                    ks[(t0 + t) * LD + i] = to;
-                    run *= gs[(t0 + t) * LD + i];
-                }
-#pragma unroll
-                for (int t = 0; t < 16; ++t) {
-                    const float kf = f[t] * k[t], qf = f[t] * qs[(t0 + t) * LD + i];
-                    dec[(t0 + t) * dk + i] = before * kf;
-                    dec[(C + t0 + t) * dk + i] = before * qf;
-                    gs[(t0 + t) * LD + i] = kf;
-                    qs[(t0 + t) * LD + i] = qf;
+                    const int at = (t0 + t) * LD + i;
+                    const float k = ks[at], q = qs[at], g = gs[at], here = f[t], from = before * f[t];
+                    dec[(t0 + t) * dk + i] = from * k;
+                    dec[(C + t0 + t) * dk + i] = from * q;
+                    dec[(2 * C + t0 + t) * dk + i] = (float)(after * run) * k;
+                    ks[at] = (float)run * k;
+                    gs[at] = here * k;
+                    qs[at] = here * q;
+                    run *= g;
                 }
             }
         }
         __syncthreads();
         // a block of 4 rows x 2 columns a thread, all channels; `rows` of q and, with delta, of k
         auto block = [&](int t0, int s0, const float* rows, float* to, bool scale) {
-            float acc[4][2];
+            float sum[4][2] = {};
+            for (int x0 = 0; x0 < dk; x0 += 16) {    // sums of 16, and of these: a chain over all channels has twice the error
+                float acc[4][2] = {};
+                for (int x = x0; x < min(x0 + 16, dk); x += 4) {
+                    const float4 k0 = *reinterpret_cast<const float4*>(ks + s0 * LD + x), k1 = *reinterpret_cast<const float4*>(ks + (s0 + 1) * LD + x);
 #pragma unroll
-            for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = 0.f;
-            for (int x = 0; x < dk; x += 4) {
-                const float4 k0 = *reinterpret_cast<const float4*>(ks + s0 * LD + x), k1 = *reinterpret_cast<const float4*>(ks + (s0 + 1) * LD + x);
+                    for (int r = 0; r < 4; ++r) {
+                        const float4 v = *reinterpret_cast<const float4*>(rows + (t0 + r) * LD + x);
+                        acc[r][0] = fmaf(v.x, k0.x, acc[r][0]); acc[r][0] = fmaf(v.y, k0.y, acc[r][0]);
+                        acc[r][0] = fmaf(v.z, k0.z, acc[r][0]); acc[r][0] = fmaf(v.w, k0.w, acc[r][0]);
+                        acc[r][1] = fmaf(v.x, k1.x, acc[r][1]); acc[r][1] = fmaf(v.y, k1.y, acc[r][1]);
+                        acc[r][1] = fmaf(v.z, k1.z, acc[r][1]); acc[r][1] = fmaf(v.w, k1.w, acc[r][1]);
+                    }
+                }
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    const float4 v = *reinterpret_cast<const float4*>(rows + (t0 + r) * LD + x);
-                    acc[r][0] = fmaf(v.x, k0.x, acc[r][0]); acc[r][0] = fmaf(v.y, k0.y, acc[r][0]);
-                    acc[r][0] = fmaf(v.z, k0.z, acc[r][0]); acc[r][0] = fmaf(v.w, k0.w, acc[r][0]);
-                    acc[r][1] = fmaf(v.x, k1.x, acc[r][1]); acc[r][1] = fmaf(v.y, k1.y, acc[r][1]);
-                    acc[r][1] = fmaf(v.z, k1.z, acc[r][1]); acc[r][1] = fmaf(v.w, k1.w, acc[r][1]);
+                    sum[r][0] += acc[r][0];
+                    sum[r][1] += acc[r][1];
                 }
             }
 #pragma unroll
             for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int c = 0; c < 2; ++c) to[(t0 + r) * (C + 1) + s0 + c] = scale ? bs[t0 + r] * acc[r][c] : acc[r][c];
+                for (int c = 0; c < 2; ++c) to[(t0 + r) * (C + 1) + s0 + c] = scale ? bs[t0 + r] * sum[r][c] : sum[r][c];
         };
         // neighbouring segments of a half: 16 x 16 results, 32 threads; [half][q, k]
         if (wid < (DELTA ? 4 : 2)) {
@@ -248,7 +250,7 @@ chunk_prep_kernel(const ChunkArgs a) {
         __syncthreads();
         // across the halves: on to the boundary, and from it
         if (tid < 128 && tid < dk) {
-            const float to = total[128 + tid], from = total[2 * 128 + tid];
+            const float to = (float)total[128 + tid], from = (float)total[2 * 128 + tid];
 #pragma unroll 4
             for (int t = 0; t < 16; ++t) {
                 ks[t * LD + tid] *= to;
@@ -292,30 +294,45 @@ chunk_prep_kernel(const ChunkArgs a) {
             dec[C + tid] = (float)to;
         }
         __syncthreads();
-        pair_t acc[8][4];                            // sums over even and odd entries; blocks above the diagonal are left out
+        // sums over the even and odd ones of 16 entries, and of these; blocks above the diagonal are left out
+        float sum[8][4];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0;
-        for (int i = 0; i < dk; i += 4) {
-            ulonglong2 kc[4];
+        for (int r = 0; r < 8; ++r) sum[r][0] = sum[r][1] = sum[r][2] = sum[r][3] = 0.f;
+#pragma unroll 1
+        for (int i0 = 0; i0 < dk; i0 += 16) {
+            pair_t acc[8][4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) kc[c] = pairs(ks + (cg + 16 * c) * LD + i);
+            for (int r = 0; r < 8; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0;
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const ulonglong2 x = pairs((r < 4 ? qs : ks) + (rg + 16 * (r & 3)) * LD + i);
+            for (int i = i0; i < i0 + 16; i += 4) {
+                if (i >= dk) break;
+                ulonglong2 kc[4];
 #pragma unroll
-                for (int c = 0; c <= (r & 3); ++c) {
-                    fma2(acc[r][c], x.x, kc[c].x);
-                    fma2(acc[r][c], x.y, kc[c].y);
+                for (int c = 0; c < 4; ++c) kc[c] = pairs(ks + (cg + 16 * c) * LD + i);
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const ulonglong2 x = pairs((r < 4 ? qs : ks) + (rg + 16 * (r & 3)) * LD + i);
+#pragma unroll
+                    for (int c = 0; c <= (r & 3); ++c) {
+                        fma2(acc[r][c], x.x, kc[c].x);
+                        fma2(acc[r][c], x.y, kc[c].y);
+                    }
                 }
             }
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+#pragma unroll
+                for (int c = 0; c <= (r & 3); ++c) {
+                    const float2 h = halves(acc[r][c]);
+                    sum[r][c] += h.x + h.y;
+                }
         }
 #pragma unroll
         for (int r = 7; r >= 0; --r) {          // the k rows still need the ratios that the q rows overwrite (same thread)
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int t = rg + 16 * (r & 3), x = cg + 16 * c;
-                const float2 h = halves(acc[r][c]);
-                const float v = t >= x ? (h.x + h.y) * Ps[t * (C + 1) + x] : 0.f;
+                const float v = t >= x ? sum[r][c] * Ps[t * (C + 1) + x] : 0.f;
                 if (r < 4) Ps[t * (C + 1) + x] = v;
                 else As[t * (C + 1) + x] = t > x ? bs[t] * v : 0.f;
             }
@@ -391,7 +408,7 @@ template <bool CH, bool DELTA>
 int launch_prep(const ChunkArgs& a, int total_rows, cudaStream_t st) {
     const int chunks = total_rows / C + a.n_seq;     // upper bound on sum(ceil(len / C)); spare CTAs leave at once
     const size_t LD = a.dk + 4, rows = C * LD;
-    const size_t psm = sizeof(float) * (2 * rows + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows + 4 * 128 : C) + C);
+    const size_t psm = sizeof(float) * (2 * rows + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows + 2 * 4 * 128 : C) + C);
     int rc = allow(chunk_prep_kernel<CH, DELTA>, psm);
     if (rc != B2_OK) return rc;
     chunk_prep_kernel<CH, DELTA><<<dim3(chunks, a.H), CH ? 512 : 256, psm, st>>>(a);
@@ -410,35 +427,43 @@ int64_t b2_internal_chunk_scan_floats(int total_rows, int n_seq, int H, int dk, 
     return n <= (int64_t)3 << 29 ? n : 0;
 }
 
-// Where the chunked form is the faster one.  Both times are estimated in us from what they measured for heads of 128 x 128 on
-// one B200 (w = dk dv / 16384 scales the products); the host knows the rows and the number of sequences, so the longest of several is taken to be 1.25 times the mean:
+// Where the chunked form is taken.  Both times are estimated in us from what they measured for heads of 128 x 128 on one B200
+// (w = dk dv / 16384 scales the products); the host knows the rows and the number of sequences, so the longest of several is taken to be 1.25 times the mean:
 //   tokens   a chain of 0.20 (delta 0.285, per channel 0.235 / 0.31) a token, or, with several sequences, 5.2 (7.1 / 10.6 / 12.4) ns a
-//            token and head, down to 5.0 (6.3 / 6.8 / 8.3) from 64 sequences on; keys of other sizes than 32, 64, 128 run as the next one, a third slower
+//            token and head, down to 5.0 (6.3 / 6.8 / 8.3) from 64 sequences on; without delta keys of other sizes than 32, 64, 128 run
+//            as the next one, a third slower
 //   chunks   one decay per head without delta (chunk_tc5.cu): 20, 0.2 a chunk of 128 and head for the products (0.14 at 64 x 64) and 0.03 a
 //            sequence and head for its state; at least 33 (29 to dk = 64): three launches
-//            else 0.3 (per channel 20 and 0.27 / 0.46) a chunk of 64 and head for the products, 0.11 a sequence and head for its state, with
-//            delta 2.7 a step of the chain and SM's share of CTAs; at least 56 (39 / 72 per channel; to dk = 64 49, 33 / 58): four launches
-// Measured, tokens -> chunks: 1 x 4096 tokens, 16 heads: 804 -> 121, 1160 -> 426, 963 -> 288, 1255 -> 571; 1 x 500: 102 -> 34,
-// 146 -> 69, 121 -> 43, 158 -> 84; 1 x 200 with delta: 62 -> 57; 1500 + 1000 + 501: 411 -> 92, 573 -> 279, 503 -> 225, 631 -> 399; 16 x 100: 121 -> 74, 181 -> 160, but 160 -> 196 and
+//            a decay per channel without delta: 20, 0.27 a chunk of 64 and head for the products, 0.11 a sequence and head for its
+//            state; at least 39 (33 to dk = 64): four launches
+//            delta: 0.16 (per channel 0.70) a chunk and head for the products, 0.11 a sequence and head for its state, 4.8 a step of the chain
+//            and SM's share of CTAs; at least 40 (110).  That is more than the chunks take (table), and the line lies there for their
+//            error: nearer, 700 to 3100 rows in several sequences would take 10 to 37 % less time, but their outputs would be 1.05 times as far from
+//            64 bits as token by token (28 pairs of sizes and inputs, 0.88 to 1.13; their states 0.92 times).
+// Measured, tokens -> chunks: 1 x 4096 tokens, 16 heads: 804 -> 121, 1160 -> 434, 963 -> 288, 1255 -> 575; 1 x 500: 102 -> 34,
+// 146 -> 70, 121 -> 43, 158 -> 88; 1500 + 1000 + 501: 411 -> 92, 573 -> 279, 503 -> 225, 631 -> 400; 16 x 100: 121 -> 74, 181 -> 160, but 160 -> 196 and
 // 223 -> 274 with delta, which are left to the tokens, as are 64 x 24: 148 -> 250, 180 -> 415, 193 -> 379, and 1 x 130: 29 -> 33, 41 -> 58, 35 -> 40.
 bool b2_internal_chunk_scan_pays(int total_rows, int n_seq, int H, int dk, int dv, bool ch, bool delta) {
     if (total_rows < 2 * n_seq) return false;
     const float len = (float)total_rows / n_seq, w = dk * dv / 16384.f, steps = ceilf(len / C), heads = (float)n_seq * H;
-    const int kind = (ch ? 2 : 0) + (delta ? 1 : 0), run_as = dk <= 32 ? 32 : dk <= 64 ? 64 : 128;
+    const int kind = (ch ? 2 : 0) + (delta ? 1 : 0), run_as = delta ? dk : dk <= 32 ? 32 : dk <= 64 ? 64 : 128;
     const float chain_tok[4] = {0.20f, 0.285f, 0.235f, 0.31f}, rate_few[4] = {5.2e-3f, 7.1e-3f, 10.6e-3f, 12.4e-3f}, rate_many[4] = {5.0e-3f, 6.3e-3f, 6.8e-3f, 8.3e-3f};
-    const float per_chunk[4] = {0.f, 0.3f, 0.27f, 0.46f};
-    const float least[4] = {dk <= 64 ? 29.f : 33.f, dk <= 64 ? 49.f : 56.f, dk <= 64 ? 33.f : 39.f, dk <= 64 ? 58.f : 72.f};
-    const float many = fminf(1.f, fmaxf(0.f, log2f(n_seq / 2.5f) / 4.f)), rate = rate_few[kind] + (rate_many[kind] - rate_few[kind]) * many;
+    const float many = fminf(1.f, fmaxf(0.f, log2f(n_seq / (delta ? 4.f : 2.5f)) / 4.f)), rate = rate_few[kind] + (rate_many[kind] - rate_few[kind]) * many;
     const float longest = len * (n_seq > 1 ? 1.25f : 1.f);
     const float tokens = (run_as == dk ? 1.f : 1.33f) * fmaxf(chain_tok[kind] * (dk <= 64 ? 0.75f : 1.f) * longest, rate * (float)total_rows * H * run_as * dv / 16384.f);
-    float chunks;
+    float chunks, least;
     if (kind == 0) {
         chunks = 20.f + (0.2f * (0.6f + 0.4f * w) * ceilf(len / 128) + 0.03f * w) * heads;
+        least = dk <= 64 ? 29.f : 33.f;
+    } else if (kind == 2) {
+        chunks = 20.f + (0.27f * (0.55f + 0.45f * w) * steps + 0.11f * w) * heads;
+        least = dk <= 64 ? 33.f : 39.f;
     } else {
-        chunks = (ch ? 20.f : 0.f) + (per_chunk[kind] * (ch ? 0.55f + 0.45f * w : 0.35f + 0.65f * w) * steps + 0.11f * w) * heads;
-        if (delta) chunks += 2.7f * fmaxf(ceilf(longest / C), steps * heads * ((dv + 63) / 64) / b2_sm_count());
+        chunks = ((ch ? 0.70f : 0.16f) * (0.35f + 0.65f * w) * steps + 0.11f * w) * heads +
+                 (3.4f + 1.4f * w) * fmaxf(ceilf(longest / C), steps * heads * ((dv + 15) / 16) / b2_sm_count());
+        least = ch ? 110.f : 40.f;
     }
-    return tokens >= fmaxf(chunks, least[kind]);
+    return tokens >= fmaxf(chunks, least);
 }
 
 int b2_internal_chunk_scan(const float* qkv, const float* beta, const float* decay, int total_rows, int H, int G, int dk, int dv,

@@ -309,10 +309,10 @@ out_kernel(const Args a) {
         if (two || qd < 2) {                         // lane: key s; registers: its weight in the tokens' results; takes Q's place
             const int s = qd * 32 + lane;
             unsigned char* to = qb + (s >> 6) * 3 * PART;
-            float run = qd < cg ? from_s : 1.;
+            float run = qd < cg ? from_s : 1.;       // (diagonal: one chain, of at most 31 products)
 #pragma unroll 1
             for (int h = 0; h < 4; ++h) {
-                if (h > 0) {                         // a chain of eight products at most
+                if (h > 0) {                         // below it chains of eight
                     const double x = __shfl_sync(0xffffffffu, in_group, 8 * h - 1);
                     if (qd < cg) run = from_s * x;
                 }

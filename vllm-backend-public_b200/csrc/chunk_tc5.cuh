@@ -88,36 +88,65 @@ struct Fetch {
     }
 };
 
-// D (two accumulators of 128 columns: the leading parts' products, and the five others) += A B over `ksteps` times 16 entries.  The parts
-// of A and B are PART bytes apart, those of B neighbours in N.  AK, BK: bytes >> 4 from one k-step to the next.
+// D (two accumulators of 128 columns) = A B over a first slice of `ksteps` times 16 entries, or += over a second one.  The first accumulator
+// takes the first slice's leading products, the other one the small ones of both and behind these the second's leading ones, so none is cut
+// off eight times at full size.  The parts of A and B are PART bytes apart, those of B neighbours in N.  AK, BK: bytes >> 4
+// from one k-step to the next.
 constexpr int PART = 64 * 256;
 constexpr uint32_t kAmn = 1u << 15, kBmn = 1u << 16;              // operand is MN-major
 template <int AK, int BK>
-__device__ __forceinline__ void mma_parts(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t majors, int ksteps, bool acc) {
+__device__ __forceinline__ void mma_parts(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t majors, int ksteps, bool second) {
     const uint32_t n128 = idesc_bf16(128, 128, 0) | majors, n256 = idesc_bf16(128, 256, 0) | majors;
 #pragma unroll 1
     for (int k = 0; k < ksteps; ++k) {
         const uint64_t a = desc_join(a_lo + k * AK), a1 = desc_join(a_lo + k * AK + (PART >> 4)), a2 = desc_join(a_lo + k * AK + (2 * PART >> 4));
         const uint64_t b = desc_join(b_lo + k * BK), b1 = desc_join(b_lo + k * BK + (PART >> 4)), b2 = desc_join(b_lo + k * BK + (2 * PART >> 4));
-        mma_ss(d, a, b, n256, acc || k > 0);
+        if (second) mma_ss(d + 128, a, b1, n128, true);
+        else mma_ss(d, a, b, n256, k > 0);           // the leading parts' and a b1
         mma_ss(d + 128, a, b2, n128, true);
         mma_ss(d + 128, a1, b, n128, true);
         mma_ss(d + 128, a1, b1, n128, true);
         mma_ss(d + 128, a2, b, n128, true);
     }
+    if (second)
+#pragma unroll 1
+        for (int k = 0; k < ksteps; ++k) mma_ss(d + 128, desc_join(a_lo + k * AK), desc_join(b_lo + k * BK), n128, true);
 }
 
-// The same with 64 columns: D (three accumulators of 64 columns: products of the parts' order 0, 1, 2) += A B over `ksteps` times 16
-// entries, the parts of B side by side as 192 columns.  A_PART: bytes from one part of A to the next.
-template <int A_PART, int AK, int BK>
+// The same over 64 entries at once, and nothing in D before: both accumulators take leading products, every other k-step each, and the first of
+// them all others before these, where what the tensor core cuts off is small.
+template <int AK, int BK>
+__device__ __forceinline__ void mma_parts64(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t majors) {
+    const uint32_t id = idesc_bf16(128, 128, 0) | majors;
+    constexpr int A[5] = {2, 0, 1, 1, 0}, B[5] = {0, 2, 1, 0, 1};
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int p = 0; p < 5; ++p)
+            mma_ss(d, desc_join(a_lo + k * AK + (A[p] * PART >> 4)), desc_join(b_lo + k * BK + (B[p] * PART >> 4)), id, p > 0 || k > 0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) mma_ss(d + 128 * (k & 1), desc_join(a_lo + k * AK), desc_join(b_lo + k * BK), id, k != 1);
+}
+
+// The same with 64 columns: D (accumulators of 64 columns: LEAD that take the leading parts' products in turns, then products of the parts'
+// order 1 and 2) += A B over `ksteps` times 16 entries, at least LEAD of them.  The parts of B are side by side as 192 columns, 8192 bytes
+// apart.  A_PART: bytes from one part of A to the next.
+template <int LEAD, int A_PART, int AK, int BK>
 __device__ __forceinline__ void mma_orders(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t majors, int ksteps, bool acc) {
+    static_assert(LEAD == 1 || LEAD == 2, "");
     const uint32_t n64 = idesc_bf16(128, 64, 0) | majors, n128 = idesc_bf16(128, 128, 0) | majors, n192 = idesc_bf16(128, 192, 0) | majors;
+    const uint32_t order1 = d + 64 * LEAD;
 #pragma unroll 1
     for (int k = 0; k < ksteps; ++k) {
-        const uint64_t b = desc_join(b_lo + k * BK);
-        mma_ss(d, desc_join(a_lo + k * AK), b, n192, acc || k > 0);
-        mma_ss(d + 64, desc_join(a_lo + k * AK + (A_PART >> 4)), b, n128, true);
-        mma_ss(d + 128, desc_join(a_lo + k * AK + (2 * A_PART >> 4)), b, n64, true);
+        const uint64_t a = desc_join(a_lo + k * AK), b = desc_join(b_lo + k * BK);
+        if (LEAD == 2 && (k & 1)) {
+            mma_ss(d, a, b, n64, acc || k > 1);
+            mma_ss(order1, a, desc_join(b_lo + k * BK + (8192 >> 4)), n128, true);
+        } else {
+            mma_ss(order1 - 64, a, b, n192, acc || k > 0);
+        }
+        mma_ss(order1, desc_join(a_lo + k * AK + (A_PART >> 4)), b, n128, true);
+        mma_ss(order1 + 64, desc_join(a_lo + k * AK + (2 * A_PART >> 4)), b, n64, true);
     }
 }
 
@@ -150,14 +179,21 @@ __device__ __forceinline__ void read_parts(uint32_t d, float (&s)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) s[i] += r[i];
 }
-__device__ __forceinline__ void read_orders(uint32_t d, float (&s)[16]) {         // the three accumulators of mma_orders, the smallest first
+template <int LEAD>
+__device__ __forceinline__ void read_orders(uint32_t d, float (&s)[16]) {         // the accumulators of mma_orders, the smallest first
     float r[16], q[16];
-    tmem_ld16(d + 128, s);
-    tmem_ld16(d + 64, r);
-    tmem_ld16(d, q);
+    tmem_ld16(d + 64 * LEAD + 64, s);
+    tmem_ld16(d + 64 * LEAD, r);
+    tmem_ld16(d + 64 * LEAD - 64, q);
     tmem_wait_ld();
 #pragma unroll
     for (int i = 0; i < 16; ++i) s[i] = (s[i] + r[i]) + q[i];
+    if (LEAD == 2) {
+        tmem_ld16(d, r);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) s[i] += r[i];
+    }
 }
 __device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
 

@@ -165,7 +165,7 @@ wy_kernel(const Args a) {
         if (DELTA) store64(tb, tm);
         if (hand_over(&s_full[1])) {
             if (elect_one()) {
-                mma_orders<PART, 128, 2>(tmem + 256, desc_lo(x1, 8192), desc_lo(DELTA ? tb : pb, 16), kAmn, 4, false);
+                mma_orders<2, PART, 128, 2>(tmem + 256, desc_lo(x1, 8192), desc_lo(DELTA ? tb : pb, 16), kAmn, 4, false);
                 mma_commit(done(1));
             }
             __syncwarp();
@@ -186,7 +186,7 @@ wy_kernel(const Args a) {
             }
             k.store(at_sm(x0), PART);
             if (hand_over(&s_full[0]) && elect_one()) {
-                mma_orders<PART, 128, 2>(tmem, desc_lo(x0, 8192), desc_lo(tb, 16), kAmn, 4, false);
+                mma_orders<1, PART, 128, 2>(tmem, desc_lo(x0, 8192), desc_lo(tb, 16), kAmn, 4, false);
                 mma_commit(done(0));
             }
             __syncwarp();
@@ -212,10 +212,10 @@ wy_kernel(const Args a) {
         };
         if (DELTA) {
             settled(1);
-            read_orders(rb + cg * 16, w);
+            read_orders<2>(rb + cg * 16, w);
             store_rows(x1, &col[feature]);
             if (hand_over(&s_full[3]) && elect_one()) {
-                mma_orders<PART, 2, 2>(tmem + 256, desc_lo(x1, 16), desc_lo(pb, 16), 0, 4, false);
+                mma_orders<2, PART, 2, 2>(tmem + 256, desc_lo(x1, 16), desc_lo(pb, 16), 0, 4, false);
                 mma_commit(done(1));
             }
             __syncwarp();
@@ -228,10 +228,10 @@ wy_kernel(const Args a) {
                 for (int e = 0; e < 8; ++e) kd.x[i][e] *= to[i];
         kd.store(at_sm(x0), PART);                   // (its products M and F take all tokens: nothing is kept out)
         if (DELTA) {
-            read_orders(ra + cg * 16, w);
+            read_orders<1>(ra + cg * 16, w);
             store_rows(y, row);
             if (hand_over(&s_full[2]) && elect_one()) {
-                mma_orders<PART, 2, 2>(tmem, desc_lo(y, 16), desc_lo(pb, 16), 0, 4, false);
+                mma_orders<1, PART, 2, 2>(tmem, desc_lo(y, 16), desc_lo(pb, 16), 0, 4, false);
                 mma_commit(done(0));
             }
             __syncwarp();
@@ -241,10 +241,10 @@ wy_kernel(const Args a) {
             for (int i = 0; i < 16; ++i) q[i] *= __shfl_sync(0xffffffffu, from_t, i);
         if (DELTA) {                                 // Q'
             settled(0);                              // (after it, W's marks are final)
-            read_orders(ra + cg * 16, w);
+            read_orders<1>(ra + cg * 16, w);
             if (first) {                             // M
                 if (hand_over(&s_full[4]) && elect_one()) {
-                    mma_parts<128, 2>(tmem, desc_lo(x0, 8192), desc_lo(y, 16), kAmn, 4, false);
+                    mma_parts64<128, 2>(tmem, desc_lo(x0, 8192), desc_lo(y, 16), kAmn);
                     mma_commit(done(0));
                 }
                 __syncwarp();
@@ -254,10 +254,10 @@ wy_kernel(const Args a) {
             for (int i = 0; i < 16; ++i) q[i] = t0 + i >= bad ? kNaN : q[i] - w[i];
         }
         settled(1);                                  // P U_0: lane a column
-        read_orders(rb + cg * 16, w);
+        read_orders<2>(rb + cg * 16, w);
         if (hand_over(&s_full[5]) && elect_one()) {  // F: lane a key feature (no delta: a column), registers the others
-            if (DELTA) mma_parts<128, 2>(tmem + 256, desc_lo(x0, 8192), desc_lo(x1, 16), kAmn, 4, false);
-            else mma_parts<128, 128>(tmem + 256, desc_lo(x1, 8192), desc_lo(x0, 8192), kAmn | kBmn, 4, false);
+            if (DELTA) mma_parts64<128, 2>(tmem + 256, desc_lo(x0, 8192), desc_lo(x1, 16), kAmn);
+            else mma_parts64<128, 128>(tmem + 256, desc_lo(x1, 8192), desc_lo(x0, 8192), kAmn | kBmn);
             mma_commit(done(1));
         }
         __syncwarp();
@@ -431,7 +431,7 @@ chain_kernel(const Args a) {
                 for (int u = 0; u < L.slices; ++u) {
                     const int i = c * L.slices + u, b = i % 3;
                     wait(here(b), (i / 3) & 1, &s_failed);
-                    mma_orders<PART, 2, 128>(tmem, desc_lo(sm + b * 3 * PART, 16), desc_lo(tile + u * 3 * 8192, 8192), kBmn, u + 1 < L.slices ? 4 : k_last, u > 0);
+                    mma_orders<1, PART, 2, 128>(tmem, desc_lo(sm + b * 3 * PART, 16), desc_lo(tile + u * 3 * 8192, 8192), kBmn, u + 1 < L.slices ? 4 : k_last, u > 0);
                     mma_commit(free_(b));
                 }
                 mma_commit(done);
@@ -483,7 +483,7 @@ chain_kernel(const Args a) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 float d[16];
-                read_orders(mine + 16 * h, d);
+                read_orders<1>(mine + 16 * h, d);
 #pragma unroll
                 for (int e = 0; e < 16; ++e) s[16 * h + e] -= d[e];
             }
@@ -601,7 +601,7 @@ read_kernel(const Args a) {
             for (int back = 1; back <= 3 && back <= i; ++back) drain(bar(s_here, (i - back) % 3), ((i - back) / 3) & 1);
         __syncwarp();
     } else if (warp == 9) {
-        const int k_last = (dk - (L.slices - 1) * 64 + 15) / 16;
+        const int k_last = max(2, (dk - (L.slices - 1) * 64 + 15) / 16);           // past dk there are zeros
         int i = 0;
 #pragma unroll 1
         for (int item = blockIdx.x; at.nt > 0; at = locate<C>(a, item += gridDim.x)) {
@@ -613,7 +613,7 @@ read_kernel(const Args a) {
                 wait(bar(s_here, b), (i / 3) & 1, &s_failed);
                 if (elect_one()) {
                     const uint32_t st = sm + b * STAGE;
-                    mma_orders<8192, 128, 128>(tmem + 256 * (n & 1), desc_lo(st, 3 * 8192), desc_lo(st + 6 * 8192, 8192), kAmn | kBmn, u + 1 < L.slices ? 4 : k_last, u > 0);
+                    mma_orders<2, 8192, 128, 128>(tmem + 256 * (n & 1), desc_lo(st, 3 * 8192), desc_lo(st + 6 * 8192, 8192), kAmn | kBmn, u + 1 < L.slices ? 4 : k_last, u > 0);
                     mma_commit(bar(s_free, b));
                     if (u + 1 == L.slices) mma_commit(bar(s_done, n & 1));
                 }
@@ -639,7 +639,7 @@ read_kernel(const Args a) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     float d[16];
-                    read_orders(src + 16 * h, d);
+                    read_orders<2>(src + 16 * h, d);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) x[16 * h + i] += d[i];
                 }
