@@ -138,6 +138,37 @@ def test_error_of_chunks_against_tokens(cuda, delta, per_channel):
     assert mean < 1.0 and max(ratios) < 1.05, ratios
 
 
+@pytest.mark.parametrize("delta,per_channel", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("lens", [[700, 3500, 3, 900], [5103], [40] * 60 + [2800]])
+def test_long_batches_go_through_the_scratch_in_pieces(cuda, lens, delta, per_channel):
+    """Scratch has a limit, past which a batch is taken piece by piece: sequences that a border cuts, one that goes over several pieces, without
+    context, with it, without a slot.  Heads are independent, so 64 of them in pieces give the bits of four at a time, which fit at once."""
+    H, dk, dv, n, T = 64, 128, 128, len(lens), sum(lens)
+    qkv, beta, dec, state = _inputs(cuda, lens, H, H, dk, dv, per_channel, delta, "mild", seed=n)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    cu, ctx, slots = [0], [(7 * i) % 3 for i in range(n)], [-1 if i % 5 == 2 else n - i for i in range(n)]
+    for m in lens:
+        cu.append(cu[-1] + m)
+    keep, lib = (i32(cu), i32(ctx), i32(slots)), _lib.load()
+    ws = torch.empty(1 << 27, device=cuda)               # the limit
+
+    def scan(h0, h1):
+        cols = [slice((p * H + h0) * dk, (p * H + h1) * dk) for p in range(3)]
+        x = torch.cat([qkv[:, c] for c in cols], 1).contiguous()
+        b = beta[:, h0:h1].contiguous() if delta else None
+        d = dec.view(T, H, -1)[:, h0:h1].reshape(T, -1).contiguous()
+        st, o = state[:, h0:h1].clone(), torch.zeros(T, h1 - h0, dv, device=cuda)
+        _lib.check(lib.b2_channel_scan_ws(x.data_ptr(), b.data_ptr() if delta else None, d.data_ptr(), T, h1 - h0, h1 - h0, dk, dv, int(per_channel),
+                                          int(delta), *(t.data_ptr() for t in keep), n, st.data_ptr(), o.data_ptr(), ws.data_ptr(), ws.numel(),
+                                          torch.cuda.current_stream().cuda_stream))
+        return o, st
+
+    out, st = scan(0, H)
+    for h in range(0, H, 4):
+        o, s = scan(h, h + 4)
+        assert torch.equal(out[:, h:h + 4], o) and torch.equal(st[:, h:h + 4], s), h
+
+
 def test_chunked_scan_leaves_short_portions_to_the_token_scan():
     lib = _lib.load()
     for per_channel in (0, 1):

@@ -28,6 +28,30 @@ def test_no_step_asks_for_more_than_the_bound(H, dk, dv):
     assert ops.scan_scratch_bytes(8192, 64, []) == 0
 
 
+LIMIT = 512 << 20
+
+
+@pytest.mark.parametrize("H,dk,dv,rows", [(64, 128, 128, 16384), (32, 128, 256, 32768), (64, 128, 128, 32768), (16, 128, 128, 131072), (48, 64, 64, 32768)])
+def test_scratch_of_long_steps_has_a_limit_and_the_bound_holds(H, dk, dv, rows):
+    """Steps whose scratch would be above the limit go through it in pieces: no step asks for more, and none for more than is kept for it."""
+    lib, r, most = _lib.load(), random.Random(H + rows), 0
+    for seqs in (1, 64, 200):
+        for per_channel in (False, True):
+            for delta in (False, True):
+                bound = ops.scan_scratch_bytes(rows, seqs, [(H, dk, dv, per_channel, delta)])
+                most = max(most, bound)
+                for i in range(600):
+                    T = r.randint(1, rows) if i % 2 else int(rows ** r.random())
+                    n = r.randint(1, min(seqs, T))
+                    assert 4 * lib.b2_channel_scan_workspace(T, n, H, dk, dv, per_channel, delta) <= bound, (T, n)
+    assert most == LIMIT
+
+
+def test_scratch_holds_a_chunk_of_any_number_of_heads():
+    lib = _lib.load()
+    assert LIMIT < 4 * lib.b2_channel_scan_workspace(8192, 1, 4096, 128, 128, False, False) < 3 * LIMIT
+
+
 def test_fewer_than_two_rows_a_sequence_never_use_scratch():
     lib = _lib.load()                                # ops._scan does not ask then
     for H, dk, dv in SIZES:

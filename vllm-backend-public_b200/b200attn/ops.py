@@ -860,14 +860,14 @@ def _scan(lib, dev, qkv, beta, decay, T: int, H: int, G: int, dk: int, dv: int, 
 
 def scan_scratch_bytes(rows: int, seqs: int, mixers) -> int:
     """The most scratch in bytes that one scan of the `mixers` -- (H, dk, dv, per_channel, delta) each -- over up to `rows` batch rows of
-    up to `seqs` sequences asks for.  Scratch grows with rows and sequences wherever the chunked form is taken, so only where its
-    rule ends has to be found: for every number of sequences, all rows and the most rows whose mean length just fills its chunks
-    of 64."""
+    up to `seqs` sequences asks for, 512 MiB at most (unless one chunk of all heads takes more).  Scratch grows with rows and sequences up to
+    that limit wherever the chunked form is taken, so only where its rule ends has to be found: for every number of sequences, all rows
+    and the most rows whose mean length just fills its chunks (of 128 tokens with a decay per head and no delta, of 64 else)."""
     lib = _lib.load()
     most = 0
     for H, dk, dv, per_channel, delta in set(mixers):
         for n in range(1, min(rows, seqs) + 1):
-            for T in (rows, rows // n // 64 * 64 * n):
+            for T in (rows, rows // n // 64 * 64 * n, rows // n // 128 * 128 * n):
                 if T > 0:
                     most = max(most, lib.b2_channel_scan_workspace(T, n, H, dk, dv, per_channel, delta))
     return 4 * most

@@ -17,7 +17,7 @@
 // scan (16 heads of 128), this one about 110: a third of the pairs, and one transposing sum for 16 of them.  Keys and queries come four vectors in flight, P and T
 // leave as vectors, and the triangular solve takes two rows at a time: 76 -> 66 us per head (3001 tokens, delta).  The choice between chunks
 // and tokens is at the end.
-#include "b2_act.cuh"
+#include "chunk_tc5.cuh"
 
 #include <math.h>
 
@@ -30,6 +30,7 @@ struct ChunkArgs {
     int H, G, dk, dv, n_seq;
     const int32_t *cu_q, *ctx_start, *state_slot;
     float* ws;
+    int first, chunks;                               // the chunks of this piece: first .. first + chunks - 1, whose scratch ws holds
     int t_at, dec_at, total;                         // scratch of a (chunk, head) in floats: P at 0, T, the decays (delta_tc5.cu)
 };
 
@@ -68,7 +69,7 @@ chunk_prep_kernel(const ChunkArgs a) {
     __shared__ double s_tail[CH ? 1 : C], s_seg[4];  // per head: the decays from s + 1 to the end of its segment; segments
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, hh = blockIdx.y;
     const int dk = a.dk, dv = a.dv, LD = dk + 4, per = dk / 4;
-    if (tid == 0) find_chunk(a, blockIdx.x, s_at);
+    if (tid == 0) find_chunk(a, a.first + blockIdx.x, s_at);
     __syncthreads();
     const int r0 = s_at[0], nt = s_at[1];
     if (r0 < 0) return;
@@ -203,11 +204,11 @@ chunk_prep_kernel(const ChunkArgs a) {
                 for (int t = 15; t >= 0; --t) {
                     const int at = (t0 + t) * LD + i;
                     const float k = ks[at], q = qs[at], g = gs[at], here = f[t], from = before * f[t];
-                    dec[(t0 + t) * dk + i] = from * k;
+                    if (DELTA) dec[(t0 + t) * dk + i] = from * k;
                     dec[(C + t0 + t) * dk + i] = from * q;
                     dec[(2 * C + t0 + t) * dk + i] = (float)(after * run) * k;
                     ks[at] = (float)run * k;
-                    gs[at] = here * k;
+                    if (DELTA) gs[at] = here * k;
                     qs[at] = here * q;
                     run *= g;
                 }
@@ -219,7 +220,9 @@ chunk_prep_kernel(const ChunkArgs a) {
             float sum[4][2] = {};
             for (int x0 = 0; x0 < dk; x0 += 16) {    // sums of 16, and of these: a chain over all channels has twice the error
                 float acc[4][2] = {};
-                for (int x = x0; x < min(x0 + 16, dk); x += 4) {
+#pragma unroll
+                for (int x = x0; x < x0 + 16; x += 4) {
+                    if (x >= dk) break;
                     const float4 k0 = *reinterpret_cast<const float4*>(ks + s0 * LD + x), k1 = *reinterpret_cast<const float4*>(ks + (s0 + 1) * LD + x);
 #pragma unroll
                     for (int r = 0; r < 4; ++r) {
@@ -405,26 +408,37 @@ int allow(K kern, size_t bytes) {
 }
 
 template <bool CH, bool DELTA>
-int launch_prep(const ChunkArgs& a, int total_rows, cudaStream_t st) {
-    const int chunks = total_rows / C + a.n_seq;     // upper bound on sum(ceil(len / C)); spare CTAs leave at once
+int launch_prep(const ChunkArgs& a, cudaStream_t st) {
     const size_t LD = a.dk + 4, rows = C * LD;
     const size_t psm = sizeof(float) * (2 * rows + (DELTA ? 2 : 1) * C * (C + 1) + (CH ? rows + 2 * 4 * 128 : C) + C);
     int rc = allow(chunk_prep_kernel<CH, DELTA>, psm);
     if (rc != B2_OK) return rc;
-    chunk_prep_kernel<CH, DELTA><<<dim3(chunks, a.H), CH ? 512 : 256, psm, st>>>(a);
+    chunk_prep_kernel<CH, DELTA><<<dim3(a.chunks, a.H), CH ? 512 : 256, psm, st>>>(a);
     B2_CUDA_OK(cudaGetLastError());
     return B2_OK;
 }
 
-}  // namespace
-
-// Scratch (floats) of the chunked form; 0 for sizes it is not built for and for scratch above 6 GiB
-int64_t b2_internal_chunk_scan_floats(int total_rows, int n_seq, int H, int dk, int dv, bool ch, bool delta) {
-    if (dk % 4 || dv % 4 || dk > 128 || n_seq <= 0 || total_rows <= 0) return 0;
+// Scratch of one chunk of all heads, and the tokens that it takes
+int64_t chunk_floats(int H, int dk, int dv, bool ch, bool delta, int* tokens) {
+    *tokens = !ch && !delta ? 128 : C;
+    if (!ch && !delta) return (int64_t)H * b2_internal_chunk_tc5_layout(dk, dv);
     int t, dec, total;
     b2_internal_delta_tc5_layout(dk, dv, ch, delta, &t, &dec, &total);
-    const int64_t n = !ch && !delta ? b2_internal_chunk_tc5_floats(total_rows, n_seq, H, dk, dv) : (int64_t)(total_rows / C + n_seq) * H * total;
-    return n <= (int64_t)3 << 29 ? n : 0;
+    return (int64_t)H * total;
+}
+// Scratch is at most this many floats (512 MiB), or what one chunk takes: longer batches go through it in pieces, one after another, and the
+// state of a sequence that a border cuts is carried.  Cost, all at once -> in pieces: 32 heads of 128 x 128, 8192 tokens with delta
+// 1296 us (1356 MiB) -> 1419, gated channels 1106 (1292 MiB) -> 1238; 16 heads, 32768 tokens 3246 (2697 MiB) -> 3478.
+constexpr int64_t kMostScratch = 1 << 27;
+
+}  // namespace
+
+// Scratch (floats) of the chunked form: grows with rows and sequences up to the limit; 0 for sizes it is not built for
+int64_t b2_internal_chunk_scan_floats(int total_rows, int n_seq, int H, int dk, int dv, bool ch, bool delta) {
+    if (dk % 4 || dv % 4 || dk > 128 || n_seq <= 0 || total_rows <= 0) return 0;
+    int tokens;
+    const int64_t one = chunk_floats(H, dk, dv, ch, delta, &tokens), all = (total_rows / tokens + n_seq) * one, carry = (int64_t)2 * H * dk * dv;
+    return all <= kMostScratch ? all : one + carry > kMostScratch ? one + carry : kMostScratch;
 }
 
 // Where the chunked form is taken.  Both times are estimated in us from what they measured for heads of 128 x 128 on one B200
@@ -469,12 +483,29 @@ bool b2_internal_chunk_scan_pays(int total_rows, int n_seq, int H, int dk, int d
 int b2_internal_chunk_scan(const float* qkv, const float* beta, const float* decay, int total_rows, int H, int G, int dk, int dv,
                            bool ch, bool delta, const int32_t* cu_q, const int32_t* ctx_start, const int32_t* state_slot, int n_seq,
                            float* state, float* o, float* ws, void* stream) {
-    if (!ch && !delta)
-        return b2_internal_chunk_tc5(qkv, decay, total_rows, H, G, dk, dv, cu_q, ctx_start, state_slot, n_seq, state, o, ws, stream);
-    ChunkArgs a{qkv, beta, decay, H, G, dk, dv, n_seq, cu_q, ctx_start, state_slot, ws, 0, 0, 0};
-    b2_internal_delta_tc5_layout(dk, dv, ch, delta, &a.t_at, &a.dec_at, &a.total);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int rc = !ch ? launch_prep<false, true>(a, total_rows, st) : delta ? launch_prep<true, true>(a, total_rows, st) : launch_prep<true, false>(a, total_rows, st);
-    if (rc != B2_OK) return rc;
-    return b2_internal_delta_tc5(qkv, decay, total_rows, H, G, dk, dv, ch, delta, cu_q, ctx_start, state_slot, n_seq, state, o, ws, stream);
+    // upper bound on sum(ceil(len / tokens)): spare CTAs leave at once.  In pieces the scratch starts with the carried states, of which a piece
+    // reads one and writes the other.
+    int tokens;
+    const int64_t one = chunk_floats(H, dk, dv, ch, delta, &tokens), most = b2_internal_chunk_scan_floats(total_rows, n_seq, H, dk, dv, ch, delta);
+    const int chunks = total_rows / tokens + n_seq, blocks = (dv + 127) / 128;
+    const bool whole = chunks * one <= most;
+    const int64_t carry = whole ? 0 : (int64_t)H * dk * dv;
+    const int fit = whole ? chunks : (int)((most - 2 * carry) / one), pieces = (chunks + fit - 1) / fit, piece = (chunks + pieces - 1) / pieces;
+    for (int first = 0, turn = 0; first < chunks; first += piece, turn ^= 1) {
+        const int n = chunks - first < piece ? chunks - first : piece;
+        const chunk_tc5::Args a{qkv, decay, H, G, dk, dv, n_seq, blocks, n * H * blocks, first, n, cu_q, ctx_start, state_slot, state, o, ws + 2 * carry,
+                                ws + turn * carry, ws + (turn ^ 1) * carry};
+        int rc;
+        if (!ch && !delta) {
+            rc = b2_internal_chunk_tc5(a, stream);
+        } else {
+            ChunkArgs p{qkv, beta, decay, H, G, dk, dv, n_seq, cu_q, ctx_start, state_slot, a.ws, first, n, 0, 0, 0};
+            b2_internal_delta_tc5_layout(dk, dv, ch, delta, &p.t_at, &p.dec_at, &p.total);
+            cudaStream_t st = static_cast<cudaStream_t>(stream);
+            rc = !ch ? launch_prep<false, true>(p, st) : delta ? launch_prep<true, true>(p, st) : launch_prep<true, false>(p, st);
+            if (rc == B2_OK) rc = b2_internal_delta_tc5(a, ch, delta, stream);
+        }
+        if (rc != B2_OK) return rc;
+    }
+    return B2_OK;
 }

@@ -146,23 +146,20 @@ kv_kernel(const Args a) {
 // ---------------------------------------------------------------------------------------------------------------- state
 __global__ void __launch_bounds__(128)
 state_kernel(const Args a) {
-    const int seq = blockIdx.x, hh = blockIdx.y, ctx = a.ctx_start[seq];
+    const int seq = blockIdx.x, hh = blockIdx.y;
     // four columns of a row; rows up to the next multiple of 16 are zeros
     const int dk = a.dk, dv = a.dv, e = (blockIdx.z * blockDim.x + threadIdx.x) * 4, row = e / dv, col = e - row * dv;
-    const int nchunks = (a.cu_q[seq + 1] - a.cu_q[seq] + CS - 1) / CS;
-    if (ctx < 0 || row >= ((dk + 15) & ~15) || nchunks == 0) return;
-    int first = 0;
-    for (int s = 0; s < seq; ++s)
-        if (a.ctx_start[s] >= 0) first += (a.cu_q[s + 1] - a.cu_q[s] + CS - 1) / CS;
+    const Portion part = portion<CS>(a, seq);
+    const int nchunks = part.count;
+    if (row >= ((dk + 15) & ~15) || nchunks == 0) return;
     const size_t step = (size_t)a.H * scratch(dk, dv);
-    float* ws = a.ws + ((size_t)first * a.H + hh) * scratch(dk, dv);
+    float* ws = a.ws + ((size_t)part.begin * a.H + hh) * scratch(dk, dv);
     const float *g = ws, *f = ws + F_AT + e;            // the chunk's whole product; F
     unsigned char* to = reinterpret_cast<unsigned char*>(ws + image(dk, dv)) + ((col >> 7) * ((dk + 63) / 64) + (row >> 6)) * (3 * PART) +
                         tile_at(row & 63, (col & 127) >> 3, 64) + (col & 4) * 2;
     const bool pad = row >= dk;
-    const int slot = pad ? -1 : a.state_slot[seq];
-    float* sp = slot >= 0 ? a.state + ((size_t)slot * a.H + hh) * dk * dv + e : nullptr;
-    float4 s = sp && ctx > 0 ? *reinterpret_cast<const float4*>(sp) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* from = pad ? nullptr : state_from(a, part, a.state_slot[seq], hh, a.ctx_start[seq]);
+    float4 s = from ? *reinterpret_cast<const float4*>(from + e) : make_float4(0.f, 0.f, 0.f, 0.f);
     constexpr int AHEAD = 8;                         // loads in flight: they do not depend on the chain
     float4 x[AHEAD];
     float d[AHEAD];
@@ -187,7 +184,8 @@ state_kernel(const Args a) {
             }
         }
     }
-    if (sp) *reinterpret_cast<float4*>(sp) = s;
+    float* dst = pad ? nullptr : state_to(a, part, a.state_slot[seq], hh);
+    if (dst) *reinterpret_cast<float4*>(dst + e) = s;
 }
 
 // ---------------------------------------------------------------------------------------------------------------- output
@@ -406,14 +404,10 @@ out_kernel(const Args a) {
 
 }  // namespace
 
-int64_t b2_internal_chunk_tc5_floats(int total_rows, int n_seq, int H, int dk, int dv) {
-    return (int64_t)(total_rows / CS + n_seq) * H * scratch(dk, dv);
-}
+int b2_internal_chunk_tc5_layout(int dk, int dv) { return scratch(dk, dv); }
 
-int b2_internal_chunk_tc5(const float* qkv, const float* decay, int total_rows, int H, int G, int dk, int dv, const int32_t* cu_q,
-                          const int32_t* ctx_start, const int32_t* state_slot, int n_seq, float* state, float* o, float* ws, void* stream) {
-    const int blocks = (dv + 127) / 128, items = (total_rows / CS + n_seq) * H * blocks;
-    const Args a{qkv, nullptr, decay, H, G, dk, dv, n_seq, blocks, items, cu_q, ctx_start, state_slot, state, o, ws};
+int b2_internal_chunk_tc5(const chunk_tc5::Args& a, void* stream) {
+    const int n_seq = a.n_seq, H = a.H, dk = a.dk, dv = a.dv, items = a.items;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     B2_CUDA_OK(cudaFuncSetAttribute(kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     B2_CUDA_OK(cudaFuncSetAttribute(out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));

@@ -179,6 +179,29 @@ __device__ __forceinline__ void read_parts(uint32_t d, float (&s)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) s[i] += r[i];
 }
+// The same with one accumulator for all small products behind two leading ones: fewer columns to read, more MMAs
+template <int A_PART, int AK, int BK>
+__device__ __forceinline__ void mma_orders3(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t majors, int ksteps, bool acc) {
+    const uint32_t n64 = idesc_bf16(128, 64, 0) | majors;
+    constexpr int A[5] = {2, 0, 1, 1, 0}, B[5] = {0, 2, 1, 0, 1};
+#pragma unroll 1
+    for (int k = 0; k < ksteps; ++k) {
+        const uint64_t a = desc_join(a_lo + k * AK), b = desc_join(b_lo + k * BK);
+        mma_ss(d + 64 * (k & 1), a, b, n64, acc || k > 1);
+#pragma unroll
+        for (int p = 0; p < 5; ++p)
+            mma_ss(d + 128, desc_join(a_lo + k * AK + (A[p] * A_PART >> 4)), desc_join(b_lo + k * BK + (B[p] * 8192 >> 4)), n64, acc || p > 0 || k > 0);
+    }
+}
+__device__ __forceinline__ void read_orders3(uint32_t d, float (&s)[16]) {
+    float r[16], q[16];
+    tmem_ld16(d + 128, s);
+    tmem_ld16(d + 64, r);
+    tmem_ld16(d, q);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s[i] = (s[i] + r[i]) + q[i];
+}
 template <int LEAD>
 __device__ __forceinline__ void read_orders(uint32_t d, float (&s)[16]) {         // the accumulators of mma_orders, the smallest first
     float r[16], q[16];
@@ -198,15 +221,41 @@ __device__ __forceinline__ void read_orders(uint32_t d, float (&s)[16]) {       
 __device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
 
 struct Args {
-    const float *qkv, *beta, *decay;
-    int H, G, dk, dv, n_seq, blocks, items;          // blocks of 128 columns; items = chunks (an upper bound) x heads x blocks
+    const float *qkv, *decay;
+    int H, G, dk, dv, n_seq, blocks, items;          // blocks of 128 columns; items = chunks of this piece (an upper bound) x heads x blocks
+    int first, chunks;                               // the piece: chunks first .. first + chunks - 1 of the batch, whose scratch ws holds
     const int32_t *cu_q, *ctx_start, *state_slot;
     float *state, *o, *ws;
+    const float* carry_in;                           // [H][dk][dv]: state of the sequence that the piece before cut, and of the one that this one cuts
+    float* carry_out;
 };
+
+// A sequence's chunks in this piece.  What goes on after the piece, and into it, is the one sequence that its border cuts.
+struct Portion {
+    int begin, count;                                // first one in the scratch, and how many (0: none)
+    bool starts, ends;                               // the sequence's first and last chunk are among them
+};
+template <int TILE>
+__device__ __forceinline__ Portion portion(const Args& a, int seq) {
+    int base = -a.first;
+    for (int s = 0; s < seq; ++s)
+        if (a.ctx_start[s] >= 0) base += (a.cu_q[s + 1] - a.cu_q[s] + TILE - 1) / TILE;
+    const int n = a.ctx_start[seq] < 0 ? 0 : (a.cu_q[seq + 1] - a.cu_q[seq] + TILE - 1) / TILE, lo = max(base, 0), hi = min(base + n, a.chunks);
+    return {lo, max(hi - lo, 0), base >= 0, base + n <= a.chunks};
+}
+// where a head's state comes from and goes to: the sequence's slot (none: null), or the carried state
+__device__ __forceinline__ const float* state_from(const Args& a, const Portion& p, int slot, int head, int ctx) {
+    const float* src = p.starts ? (slot >= 0 && ctx > 0 ? a.state + (size_t)slot * a.H * a.dk * a.dv : nullptr) : a.carry_in;
+    return src ? src + (size_t)head * a.dk * a.dv : nullptr;
+}
+__device__ __forceinline__ float* state_to(const Args& a, const Portion& p, int slot, int head) {
+    float* dst = p.ends ? (slot >= 0 ? a.state + (size_t)slot * a.H * a.dk * a.dv : nullptr) : a.carry_out;
+    return dst ? dst + (size_t)head * a.dk * a.dv : nullptr;
+}
 
 // Where an item lies.  The whole warp works.
 struct At {
-    int row, nt, chunk, head, block, fresh;          // first row, rows (0: none, and none follow), fresh: the state before it is zero
+    int row, nt, chunk, head, block, fresh;          // first row, rows (0: none, and none follow), chunk of the piece, fresh: the state before it is zero
 };
 template <int TILE>
 __device__ __forceinline__ At locate(const Args& a, int item) {
@@ -216,7 +265,7 @@ __device__ __forceinline__ At locate(const Args& a, int item) {
     at.chunk = item / hz;
     at.head = (item - at.chunk * hz) / a.blocks;
     at.block = (item - at.chunk * hz) % a.blocks;
-    int want = at.chunk;
+    int want = a.first + at.chunk;
     for (int s0 = 0; s0 < a.n_seq; s0 += 32) {
         int lo = 0, len = 0, ctx = -1;
         if (s0 + lane < a.n_seq) {

@@ -349,13 +349,6 @@ wy_kernel(const Args a) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------- the chain
-__device__ __forceinline__ int first_chunk(const Args& a, int seq) {
-    int base = 0;
-    for (int s = 0; s < seq; ++s)
-        if (a.ctx_start[s] >= 0) base += (a.cu_q[s + 1] - a.cu_q[s] + C - 1) / C;
-    return base;
-}
-
 // A CTA per 64 columns of a head's state.  Eight warps keep it in registers, in fp32 (lane a key feature, 32 columns a thread), and
 // write its parts; one warp copies M ahead, three slices of 64 features in a ring; one multiplies and copies the parts out.
 // Bound by one SM's intake: a step's 96 KB of M come at 54 bytes a cycle, 0.95 us, beside which split, product and read-back of the step take
@@ -391,15 +384,16 @@ chain_kernel(const Args a) {
         b2::fence_mbar_init();
     }
     __syncthreads();
-    const int seq = s_seq, hh = blockIdx.y, z = blockIdx.x, ctx = a.ctx_start[seq];
-    const int nchunks = (a.cu_q[seq + 1] - a.cu_q[seq] + C - 1) / C;
-    if (ctx < 0 || nchunks == 0) return;
+    const int seq = s_seq, hh = blockIdx.y, z = blockIdx.x;
+    const Portion part = portion<C>(a, seq);
+    const int nchunks = part.count;
+    if (nchunks == 0) return;
     const int dk = a.dk, dv = a.dv;
     const Layout L(dk, dv, CH, true);
     const uint32_t sm = (b2::smem_u32(sm_raw) + 1023u) & ~1023u, tile = sm + 9 * PART;
     unsigned char* const gen = sm_raw + (sm - b2::smem_u32(sm_raw));
     const size_t step = (size_t)a.H * L.total;
-    float* const ws = a.ws + ((size_t)first_chunk(a, seq) * a.H + hh) * L.total;
+    float* const ws = a.ws + ((size_t)part.begin * a.H + hh) * L.total;
     const uint32_t full = b2::smem_u32(&s_full), done = b2::smem_u32(&s_done), stored = b2::smem_u32(&s_stored);
     auto here = [&](int b) { return b2::smem_u32(&s_here[b]); };
     auto free_ = [&](int b) { return b2::smem_u32(&s_free[b]); };
@@ -445,8 +439,6 @@ chain_kernel(const Args a) {
     } else {
         const int qd = warp & 3, cg = warp >> 2, i0 = qd * 32 + lane, j0 = z * 64 + cg * 32;
         const uint32_t mine = tmem + ((uint32_t)(qd * 32) << 16) + cg * 32;
-        const int slot = a.state_slot[seq];
-        float* sp = slot >= 0 && i0 < dk ? a.state + (((size_t)slot * a.H + hh) * dk + i0) * dv + j0 : nullptr;
         float s[32], f[32];
         auto row32 = [&](const float* p, bool there, float (&x)[32]) {
 #pragma unroll
@@ -456,7 +448,8 @@ chain_kernel(const Args a) {
                 x[e] = v.x; x[e + 1] = v.y; x[e + 2] = v.z; x[e + 3] = v.w;
             }
         };
-        row32(sp, sp && ctx > 0, s);
+        const float* from = state_from(a, part, a.state_slot[seq], hh, a.ctx_start[seq]);
+        row32(from && i0 < dk ? from + (size_t)i0 * dv + j0 : nullptr, from && i0 < dk, s);
         float gc = 0.f;
         const bool pad = i0 >= L.slices * 64;
 #pragma unroll 1
@@ -488,12 +481,14 @@ chain_kernel(const Args a) {
                 for (int e = 0; e < 16; ++e) s[16 * h + e] -= d[e];
             }
         }
-        if (sp) {
+        float* dst = state_to(a, part, a.state_slot[seq], hh);
+        if (dst && i0 < dk) {
+            dst += (size_t)i0 * dv + j0;
             const bool bad = *(volatile int*)&s_failed != 0;
 #pragma unroll
             for (int e = 0; e < 32; e += 4)
                 if (j0 + e < dv)
-                    *reinterpret_cast<float4*>(sp + e) = bad ? make_float4(kNaN, kNaN, kNaN, kNaN) : make_float4(s[e], s[e + 1], s[e + 2], s[e + 3]);
+                    *reinterpret_cast<float4*>(dst + e) = bad ? make_float4(kNaN, kNaN, kNaN, kNaN) : make_float4(s[e], s[e + 1], s[e + 2], s[e + 3]);
         }
     }
     __syncwarp();
@@ -505,20 +500,20 @@ chain_kernel(const Args a) {
 template <bool CH>
 __global__ void __launch_bounds__(128)
 state_kernel(const Args a) {
-    const int seq = blockIdx.x, hh = blockIdx.y, ctx = a.ctx_start[seq], dk = a.dk, dv = a.dv;
+    const int seq = blockIdx.x, hh = blockIdx.y, dk = a.dk, dv = a.dv;
     const int e = (blockIdx.z * blockDim.x + threadIdx.x) * 4, row = e / dv, col = e - row * dv;
-    const int nchunks = (a.cu_q[seq + 1] - a.cu_q[seq] + C - 1) / C;
+    const Portion part = portion<C>(a, seq);
+    const int nchunks = part.count;
     const Layout L(dk, dv, CH, false);
-    if (ctx < 0 || nchunks == 0 || row >= L.slices * 64) return;
+    if (nchunks == 0 || row >= L.slices * 64) return;
     const size_t step = (size_t)a.H * L.total;
-    float* ws = a.ws + ((size_t)first_chunk(a, seq) * a.H + hh) * L.total;
+    float* ws = a.ws + ((size_t)part.begin * a.H + hh) * L.total;
     const bool pad = row >= dk;
     const float *g = ws + L.dec + (CH ? 3 * C * dk + row : C - 1), *f = ws + L.f + e;
     unsigned char* to = reinterpret_cast<unsigned char*>(ws + L.s) + ((col >> 6) * L.slices + (row >> 6)) * (3 * 8192) +
                         tile_at(row & 63, (col & 63) >> 3, 64) + (col & 4) * 2;
-    const int slot = pad ? -1 : a.state_slot[seq];
-    float* sp = slot >= 0 ? a.state + ((size_t)slot * a.H + hh) * dk * dv + e : nullptr;
-    float4 s = sp && ctx > 0 ? *reinterpret_cast<const float4*>(sp) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* from = pad ? nullptr : state_from(a, part, a.state_slot[seq], hh, a.ctx_start[seq]);
+    float4 s = from ? *reinterpret_cast<const float4*>(from + e) : make_float4(0.f, 0.f, 0.f, 0.f);
     constexpr int AHEAD = 8;                         // loads in flight: they do not depend on the chain
     float4 x[AHEAD];
     float d[AHEAD];
@@ -543,7 +538,8 @@ state_kernel(const Args a) {
             }
         }
     }
-    if (sp) *reinterpret_cast<float4*>(sp) = s;
+    float* dst = pad ? nullptr : state_to(a, part, a.state_slot[seq], hh);
+    if (dst) *reinterpret_cast<float4*>(dst + e) = s;
 }
 
 // ---------------------------------------------------------------------------------------------------------------- read-out
@@ -613,7 +609,7 @@ read_kernel(const Args a) {
                 wait(bar(s_here, b), (i / 3) & 1, &s_failed);
                 if (elect_one()) {
                     const uint32_t st = sm + b * STAGE;
-                    mma_orders<2, 8192, 128, 128>(tmem + 256 * (n & 1), desc_lo(st, 3 * 8192), desc_lo(st + 6 * 8192, 8192), kAmn | kBmn, u + 1 < L.slices ? 4 : k_last, u > 0);
+                    mma_orders3<8192, 128, 128>(tmem + 256 * (n & 1), desc_lo(st, 3 * 8192), desc_lo(st + 6 * 8192, 8192), kAmn | kBmn, u + 1 < L.slices ? 4 : k_last, u > 0);
                     mma_commit(bar(s_free, b));
                     if (u + 1 == L.slices) mma_commit(bar(s_done, n & 1));
                 }
@@ -639,7 +635,7 @@ read_kernel(const Args a) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     float d[16];
-                    read_orders<2>(src + 16 * h, d);
+                    read_orders3(src + 16 * h, d);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) x[16 * h + i] += d[i];
                 }
@@ -660,7 +656,7 @@ read_kernel(const Args a) {
 }
 
 template <bool CH, bool DELTA>
-int launch(Args a, int total_rows, cudaStream_t st) {
+int launch(const Args& a, cudaStream_t st) {
     const Layout L(a.dk, a.dv, CH, DELTA);
     constexpr int WY = 10 * PART + 6 * 8192 + 1024, CHAIN = 9 * PART + 6 * 8192 + 1024, READ = 27 * 8192 + 1024;
     B2_CUDA_OK(cudaFuncSetAttribute(wy_kernel<CH, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, WY));
@@ -684,11 +680,8 @@ void b2_internal_delta_tc5_layout(int dk, int dv, bool ch, bool delta, int* t, i
     *total = L.total;
 }
 
-int b2_internal_delta_tc5(const float* qkv, const float* decay, int total_rows, int H, int G, int dk, int dv, bool ch, bool delta, const int32_t* cu_q,
-                          const int32_t* ctx_start, const int32_t* state_slot, int n_seq, float* state, float* o, float* ws, void* stream) {
-    const int blocks = (dv + 127) / 128, items = (total_rows / C + n_seq) * H * blocks;
-    const Args a{qkv, nullptr, decay, H, G, dk, dv, n_seq, blocks, items, cu_q, ctx_start, state_slot, state, o, ws};
+int b2_internal_delta_tc5(const chunk_tc5::Args& a, bool ch, bool delta, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (ch) return delta ? launch<true, true>(a, total_rows, st) : launch<true, false>(a, total_rows, st);
-    return launch<false, true>(a, total_rows, st);
+    if (ch) return delta ? launch<true, true>(a, st) : launch<true, false>(a, st);
+    return launch<false, true>(a, st);
 }
