@@ -217,6 +217,92 @@ def test_nothing_runs_backwards(cuda, at, delta, per_channel, bad):
             assert torch.equal(out[at + 1:], good[at + 1:])
 
 
+def _scan(x, b, d, state, lens, ctx, slots, H, dk, dv, per_channel, delta):
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=x.device)      # noqa: E731
+    cu = [0]
+    for m in lens:
+        cu.append(cu[-1] + m)
+    keep, st, o = (i32(cu), i32(ctx), i32(slots)), state.clone(), torch.zeros(cu[-1], H, dv, device=x.device)
+    ws = torch.empty(1 << 27, device=x.device)
+    _lib.check(_lib.load().b2_channel_scan_ws(x.data_ptr(), b.data_ptr() if delta else None, d.data_ptr(), cu[-1], H, H, dk, dv, int(per_channel), int(delta),
+                                              *(t.data_ptr() for t in keep), len(lens), st.data_ptr(), o.data_ptr(), ws.data_ptr(), ws.numel(),
+                                              torch.cuda.current_stream().cuda_stream))
+    return o, st
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), 3.4e38])
+@pytest.mark.parametrize("delta,per_channel", [(False, False), (True, False), (False, True), (True, True)])
+def test_nothing_runs_backwards_across_items(cuda, delta, per_channel, bad):
+    """The same where a CTA goes on to other items after one with a bad value, with a second block of columns, two slices of features, a sequence
+    that starts fresh behind, and bad values in several chunks, the last column among them: no earlier token, no other head, no other sequence and
+    (a bad value) no other column gets another bit.  3.4e38 is finite, but rounds to an infinity in bf16."""
+    H, dk, dv, lens, ctx, slots = 16, 128, 136, [2100, 700], [9, 0], [0, 1]
+    qkv, beta, dec, state = _inputs(cuda, lens, H, H, dk, dv, per_channel, delta, "mild", seed=3)
+    if not delta:
+        qkv[:, :2 * H * dk] *= 0.05                      # 3.4e38 stays finite in the results
+    run = lambda x, b, d: _scan(x, b, d, state, lens, ctx, slots, H, dk, dv, per_channel, delta)     # noqa: E731
+    good, st_good = run(qkv, beta, dec)
+    plants = ((200, 3, 135), (1029, 3, 7), (1029, 11, 130), (1090, 11, 135))             # token, head, column
+    for what in ("v",) if bad == 3.4e38 else ("q", "k", "v", "decay") + (("beta",) if delta else ()):
+        x, b, d = qkv.clone(), beta.clone() if delta else None, dec.clone()
+        for t, h, c in plants:
+            if what == "decay":
+                d[t, (h * dk + c % dk) if per_channel else h] = bad
+            elif what == "beta":
+                b[t, h] = bad
+            else:
+                x[t, {"q": h * dk + c % dk, "k": (H + h) * dk + c % dk, "v": 2 * H * dk + h * dv + c}[what]] = bad
+        out, st = run(x, b, d)
+        clean = [h for h in range(H) if h not in (3, 11)]
+        assert torch.equal(out[:, clean], good[:, clean]) and torch.equal(out[2100:], good[2100:]) and torch.equal(st[1], st_good[1]), what
+        assert torch.equal(st[0][clean], st_good[0][clean]), what
+        assert torch.equal(out[:200, 3], good[:200, 3]) and torch.equal(out[:1029, 11], good[:1029, 11]), what
+        if what == "q":
+            rest = [t for t in range(2100) if t not in (200, 1029, 1090)]
+            assert torch.equal(out[rest], good[rest]) and torch.equal(st, st_good)
+        if what == "v":
+            for h, cols in ((3, (7, 135)), (11, (130, 135))):
+                rest = [c for c in range(dv) if c not in cols]
+                assert torch.equal(out[:, h][:, rest], good[:, h][:, rest]) and torch.equal(st[0, h][:, rest], st_good[0, h][:, rest])
+            assert torch.equal(out[:1029, 3, 7], good[:1029, 3, 7]) and torch.equal(out[:1090, 11, 135], good[:1090, 11, 135])
+            if bad == 3.4e38:
+                ref, st_ref = _reference(x, b, d, state, lens, ctx, slots, H, H, dk, dv)
+                for a, r in ((out[200:, 3, 135], ref[200:, 3, 135]), (out[1029:, 11, 130], ref[1029:, 11, 130]), (st[0, 3, :, 7], st_ref[0, 3, :, 7])):
+                    assert bool(torch.isfinite(a).all()) and float((a.double() - r).norm() / r.norm()) < 4e-6
+
+
+@pytest.mark.parametrize("delta,per_channel", [(False, False), (True, False), (False, True), (True, True)])
+def test_infinities_stay_infinities(cuda, delta, per_channel):
+    """A value that is an infinity gives infinities of P's sign in its column's outputs of the same chunk (with the delta rule at its own token; behind
+    it different signs meet) and of the key's sign in the state; an infinity in the state those of the query's sign."""
+    H, dk, dv, T = 2, 64, 32, 64
+    qkv, beta, dec, state = _inputs(cuda, [T], H, H, dk, dv, per_channel, delta, "mild", seed=8)
+    run = lambda x, s: _scan(x, beta, dec, s, [T], [4], [0], H, dk, dv, per_channel, delta)      # noqa: E731
+    inf = float("inf")
+    at = T - 1 if delta else 40
+    x = qkv.clone()
+    x[at, 2 * H * dk + 5] = inf
+    out, st = run(x, state)
+    q, k, d = (t.double() for t in (qkv[:, :dk], qkv[:, H * dk:(H + 1) * dk], dec.view(T, H, -1)[:, 0]))
+    ratio = torch.cat([torch.ones_like(d[:1]), torch.cumprod(d[at + 1:], 0)])
+    p = (q[at:] * ratio * k[at]).sum(-1)
+    assert bool((p.abs() > 1e-3).sum() > (T - at) // 2)
+    for t in range(at, T):
+        if abs(float(p[t - at])) > 1e-3:
+            assert float(out[t, 0, 5]) == math.copysign(inf, float(p[t - at])), t
+    assert torch.equal(st[0, 0, :, 5], torch.copysign(torch.full((dk,), inf, device=cuda), k[at].float()))
+    assert bool(torch.isfinite(out[:at]).all()) and bool(torch.isfinite(out[:, 1]).all())
+    if not delta:
+        s = state.clone()
+        s[0, 0, 3, 5] = inf
+        out, st = run(qkv, s)
+        assert torch.equal(out[:, 0, 5], torch.copysign(torch.full((T,), inf, device=cuda), qkv[:, 3])) and float(st[0, 0, 3, 5]) == inf
+        s[0, 0, 3, 5] = 3.4e38
+        out, st = run(qkv * 0.1, s)
+        ref, st_ref = _reference(qkv * 0.1, beta, dec, s, [T], [4], [0], H, H, dk, dv)
+        assert float((out.double() - ref)[:, 0, 5].norm() / ref[:, 0, 5].norm()) < 2e-6 and float((st.double() - st_ref).norm() / st_ref.norm()) < 2e-6
+
+
 @pytest.mark.parametrize("delta", [False, True])
 def test_decode_rows_do_not_ask_for_scratch(cuda, monkeypatch, delta):
     """A decode step's scan is one call into the library, as many of them are launched one by one."""

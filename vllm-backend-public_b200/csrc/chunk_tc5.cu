@@ -7,9 +7,10 @@
 // The first and last take a chunk, a head and 128 columns at a time, one persistent CTA of 16 warps an SM: all of them load, split into parts
 // and read the results back; whichever hands over its share of a tile last issues the tile's MMAs.  The features lie on the tensor core's lanes, the tokens on its columns.  Ratios of decays
 // are products of the decays between (nothing is divided), scanned within each warp.
-// Nothing runs backwards in time: P above its diagonal is selected to zero, and if a result is not finite, the values that are not
-// finite are taken out of V, the product is repeated (so earlier tokens get the very numbers that they get without them) and
-// their columns become NaN from their tokens on.
+// Nothing runs backwards in time: P above its diagonal is selected to zero, and if a result is not finite, the values without parts are
+// taken out of V, the product is repeated (so earlier tokens get the very numbers that they get without them) and
+// their columns become NaN from their tokens on.  When a CTA is through with its items, it sums what is not finite again in plain fp32: infinities
+// stay infinities.
 //
 // 4096 tokens, 16 heads of 128 x 128 in a graph: 121 us (with the products on the FMA pipe 243, token by token 804); 500 tokens 34 (41, 102).
 // out_kernel's item takes 30e3 cycles, of which the MMAs are 9e3: splitting into parts, the copies of S_0 (20 bytes a cycle and SM when all
@@ -28,16 +29,73 @@ constexpr int F_AT = 32;
 __host__ __device__ constexpr int image(int dk, int dv) { return F_AT + (dk * dv + 31) / 32 * 32; }
 __host__ __device__ constexpr int scratch(int dk, int dv) { return image(dk, dv) + (dk + 63) / 64 * ((dv + 127) / 128) * (3 * PART / 4); }
 
+// Results that are not finite, summed again from the inputs (and the state's parts) in plain fp32
+__device__ __noinline__ void again_sums(const Args& a, const Again& again) {
+    const int tid = threadIdx.x, dk = a.dk, dv = a.dv, Cq = 2 * a.G * dk + a.H * dv, group = a.H / a.G;
+    for (int m = again.first; m <= again.last; ++m) {
+        const At t = locate<CS>(a, blockIdx.x + m * gridDim.x);
+        const float* base = a.qkv + (size_t)t.row * Cq, *k = base + (a.G + t.head / group) * dk, *v = base + 2 * a.G * dk + t.head * dv;
+        const float* g = a.decay + (size_t)t.row * a.H + t.head;
+        float* f = a.ws + ((size_t)t.chunk * a.H + t.head) * scratch(dk, dv) + F_AT;
+        for (int e = tid; e < 128 * dk; e += NT) {
+            const int i = e >> 7, j = t.block * 128 + (e & 127);
+            if (j >= dv || finite(f[(size_t)i * dv + j])) continue;
+            double to = 1.;
+            float sum = 0.f;
+            for (int s = t.nt - 1; s >= 0; --s) {
+                sum = fmaf(k[(size_t)s * Cq + i], (float)to * v[(size_t)s * Cq + j], sum);
+                to *= g[(size_t)s * a.H];
+            }
+            f[(size_t)i * dv + j] = sum;
+        }
+    }
+}
+// P: shared memory for P, row after row, and the decays from the chunk's start
+__device__ __noinline__ void again_outputs(const Args& a, const Again& again, float* P) {
+    const int tid = threadIdx.x, dk = a.dk, dv = a.dv, Cq = 2 * a.G * dk + a.H * dv, group = a.H / a.G;
+    float* const from = P + CS * CS;
+    for (int m = again.first; m <= again.last; ++m) {
+        const At t = locate<CS>(a, blockIdx.x + m * gridDim.x);
+        const float* base = a.qkv + (size_t)t.row * Cq, *q = base + (t.head / group) * dk, *k = q + a.G * dk, *v = base + 2 * a.G * dk + t.head * dv;
+        const float* g = a.decay + (size_t)t.row * a.H + t.head;
+        __syncthreads();
+        for (int e = tid; e < CS * CS; e += NT) {
+            const int r = e / CS, s = e % CS;
+            if (s > r || r >= t.nt) continue;
+            double run = 1.;
+            for (int u = s + 1; u <= r; ++u) run *= g[(size_t)u * a.H];
+            float p = 0.f;
+            for (int i = 0; i < dk; ++i) p = fmaf(q[(size_t)r * Cq + i], k[(size_t)s * Cq + i], p);
+            P[e] = p * (float)run;
+            if (s == 0) from[r] = run * g[0];
+        }
+        __syncthreads();
+        const unsigned char* s0 = reinterpret_cast<const unsigned char*>(a.ws + ((size_t)t.chunk * a.H + t.head) * scratch(dk, dv) + image(dk, dv)) +
+                                  t.block * (dk > 64 ? 2 : 1) * (3 * PART);
+        for (int e = tid; e < 128 * t.nt; e += NT) {
+            const int r = e >> 7, c = e & 127, j = t.block * 128 + c;
+            float* o = a.o + ((size_t)(t.row + r) * a.H + t.head) * dv + j;
+            if (j >= dv || finite(*o)) continue;
+            float sum = 0.f;
+            for (int i = 0; i < dk && !t.fresh; ++i)
+                sum = fmaf(from[r] * q[(size_t)r * Cq + i], joined(s0 + (i >> 6) * (3 * PART) + tile_at(i & 63, c >> 3, 64) + (c & 7) * 2, PART), sum);
+            for (int s = 0; s <= r; ++s) sum = fmaf(P[r * CS + s], v[(size_t)s * Cq + j], sum);
+            *o = sum;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------------------------------------------- F
 // Two slices of 64 tokens, each with its own tiles of V and K and its own accumulator; while one is multiplied, the next is split,
 // the one after it is on its way, and the accumulators of two items alternate.
 __global__ void __launch_bounds__(NT, 1)
-kv_kernel(const Args a) {
+kv_kernel(const __grid_constant__ Args a) {
     extern __shared__ unsigned char sm_raw[];
     __shared__ __align__(8) uint64_t s_done[2];
     __shared__ unsigned s_full[2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed;
+    __shared__ Again s_again;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     At at = locate<CS>(a, blockIdx.x);
     if (at.nt == 0) return;
@@ -46,6 +104,7 @@ kv_kernel(const Args a) {
     auto done = [&](int u) { return b2::smem_u32(&s_done[u]); };
     if (tid == 0) {
         s_failed = 0;
+        s_again.none();
         for (int u = 0; u < 2; ++u) {
             s_full[u] = 0;
             b2::mbar_init(done(u), 1);
@@ -82,9 +141,14 @@ kv_kernel(const Args a) {
             float x[16];
             read_parts(src + 16 * h, x);             // the two slices' sums
             if (j < dv) {
+                float sum = 0.f;
 #pragma unroll
                 for (int i = 0; i < 16; ++i, f += dv)
-                    if (i0 + 16 * h + i < dk) *f = bad ? __int_as_float(0x7fc00000) : x[i];
+                    if (i0 + 16 * h + i < dk) {
+                        *f = bad ? __int_as_float(0x7fc00000) : x[i];
+                        sum += fabsf(x[i]);
+                    }
+                if (!finite(sum)) s_again.add(n - 1);
             }
         }
     };
@@ -141,6 +205,7 @@ kv_kernel(const Args a) {
     if (*(volatile int*)&s_failed)
         for (int u = 0; u < 2; ++u) drain(done(u), (n - 1) & 1);
     tmem_free(tmem, warp);
+    if (!*(volatile int*)&s_failed) again_sums(a, s_again);
 }
 
 // ---------------------------------------------------------------------------------------------------------------- state
@@ -174,7 +239,7 @@ state_kernel(const Args a) {
         for (int u = 0; u < AHEAD; ++u) {
             const int c = c0 + u;
             if (c < nchunks) {
-                store_parts4(to + (size_t)c * step * 4, PART, s);
+                store_any4(to + (size_t)c * step * 4, PART, s);
                 if (pad) continue;
                 s = make_float4(fmaf(s.x, d[u], x[u].x), fmaf(s.y, d[u], x[u].y), fmaf(s.z, d[u], x[u].z), fmaf(s.w, d[u], x[u].w));
                 if (c + AHEAD < nchunks) {
@@ -192,26 +257,27 @@ state_kernel(const Args a) {
 // Shared memory: two tiles X for S_0, then K, then V, a slice of 64 features or tokens each, and Q, whose place P takes.  TMEM: S_0^T Q^T,
 // and K Q^T, whose place V^T P^T takes.
 __global__ void __launch_bounds__(NT, 1)
-out_kernel(const Args a) {
+out_kernel(const __grid_constant__ Args a) {
     extern __shared__ unsigned char sm_raw[];
-    __shared__ __align__(8) uint64_t s_done[2], s_copied, s_decided;
+    __shared__ __align__(8) uint64_t s_done[2], s_copied;
     __shared__ unsigned s_full[4];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_failed, s_again;                // s_again: number of the last item (from 1) with a result that was not finite
-    __shared__ int s_bad_from[128];                  // first token whose value in this column is not finite
+    __shared__ int s_failed, s_repeat;               // s_repeat: number of the last item (from 1) with a result that was not finite
+    __shared__ Again s_again;
+    __shared__ int s_bad_from[128];                  // first token whose value in this column has no parts
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     At at = locate<CS>(a, blockIdx.x);
     if (at.nt == 0) return;
     const uint32_t sm = (b2::smem_u32(sm_raw) + 1023u) & ~1023u, q_sm = sm + 6 * PART;
     unsigned char* const gen = sm_raw + (sm - b2::smem_u32(sm_raw)), * const qb = gen + 6 * PART;
     auto done = [&](int u) { return b2::smem_u32(&s_done[u]); };
-    const uint32_t copied = b2::smem_u32(&s_copied), decided = b2::smem_u32(&s_decided);
+    const uint32_t copied = b2::smem_u32(&s_copied);
     if (tid == 0) {
-        s_failed = s_again = 0;
+        s_failed = s_repeat = 0;
+        s_again.none();
         for (int u = 0; u < 4; ++u) s_full[u] = 0;
         for (int u = 0; u < 2; ++u) b2::mbar_init(done(u), 1);
         b2::mbar_init(copied, 1);
-        b2::mbar_init(decided, NT / 32);
         b2::fence_mbar_init();
     }
     const uint32_t tmem = tmem_alloc(&s_tmem, warp);
@@ -367,12 +433,12 @@ out_kernel(const Args a) {
                 }
             }
             if (pass) break;
-            if (bad) s_again = n + 1;
+            if (bad) s_repeat = n + 1;
             tc_fence_before();
-            __syncwarp();
-            if (lane == 0) b2::mbar_arrive(decided);
-            if (!wait(decided, n & 1, &s_failed) || *(volatile int*)&s_again != n + 1) break;
-            // some result is not finite: the values without what is not
+            __syncthreads();                         // (and a volatile flag: __syncthreads_or spills 48 bytes here)
+            if (*(volatile int*)&s_repeat != n + 1) break;
+            // some result is not finite: the values without what has no parts
+            if (tid == 0) s_again.add(n);
             if (tid < 128) s_bad_from[tid] = CS;
             __syncthreads();
 #pragma unroll 1
@@ -383,7 +449,7 @@ out_kernel(const Args a) {
                 for (int i = 0; i < 2; ++i)
 #pragma unroll
                     for (int e = 0; e < 8; ++e)
-                        if (!finite(x.x[i][e])) {
+                        if (!splits(x.x[i][e])) {
                             atomicMin(&s_bad_from[x.col() + e], u * 64 + x.row(i));
                             x.x[i][e] = 0.f;
                         }
@@ -400,6 +466,7 @@ out_kernel(const Args a) {
         if (copies) drain(copied, (copies - 1) & 1);
     }
     tmem_free(tmem, warp);
+    if (!*(volatile int*)&s_failed) again_outputs(a, s_again, reinterpret_cast<float*>(gen));
 }
 
 }  // namespace

@@ -50,6 +50,39 @@ __device__ __forceinline__ void store_parts(unsigned char* dst, int part_bytes, 
     *reinterpret_cast<uint4*>(dst + part_bytes) = s.mid;
     *reinterpret_cast<uint4*>(dst + 2 * part_bytes) = s.lo;
 }
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+// An infinity, and what rounds to one in bf16, has no parts that add up to it: a product with it is NaN.  Kernels find such results and sum
+// them again in plain fp32, as the scan token by token would.
+__device__ __forceinline__ bool splits(float x) { return fabsf(x) < __uint_as_float(0x7f7f8000u); }
+// four floats -> 8 bytes of each part, from which joined() gives back any float: parts by truncation where rounding would overflow, infinities and NaN
+// in the first part alone
+__device__ __forceinline__ void store_any4(unsigned char* dst, int part_bytes, const float4& x) {
+    if (splits(x.x) && splits(x.y) && splits(x.z) && splits(x.w)) {
+        store_parts4(dst, part_bytes, x);
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float v = e == 0 ? x.x : e == 1 ? x.y : e == 2 ? x.z : x.w;
+        const uint32_t bits = __float_as_uint(v);
+        uint32_t hi, mid, lo;
+        split2(v, 0.f, hi, mid, lo);
+        if (!splits(v)) {
+            uint32_t none;
+            hi = v == v ? bits >> 16 : 0x7fffu;
+            split2(finite(v) ? v - __uint_as_float(bits & 0xffff0000u) : 0.f, 0.f, mid, lo, none);
+        }
+        reinterpret_cast<uint16_t*>(dst)[e] = (uint16_t)hi;
+        reinterpret_cast<uint16_t*>(dst + part_bytes)[e] = (uint16_t)mid;
+        reinterpret_cast<uint16_t*>(dst + 2 * part_bytes)[e] = (uint16_t)lo;
+    }
+}
+__device__ __forceinline__ float joined(const unsigned char* src, int part_bytes) {
+    float p[3];
+#pragma unroll
+    for (int u = 0; u < 3; ++u) p[u] = __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t*>(src + u * part_bytes) << 16);
+    return finite(p[0]) ? p[0] + p[1] + p[2] : p[0];
+}
 // 16-byte vector `c` (eight entries) of row `r`, in sub-tiles of 64 entries x `rows` rows
 __device__ __forceinline__ int tile_at(int r, int c, int rows) { return (c >> 3) * rows * 128 + r * 128 + (((c & 7) ^ (r & 7)) << 4); }
 
@@ -218,7 +251,12 @@ __device__ __forceinline__ void read_orders(uint32_t d, float (&s)[16]) {       
         for (int i = 0; i < 16; ++i) s[i] += r[i];
     }
 }
-__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
+// Which of a CTA's items have results that are not finite: once it is through, it looks at those from the first to the last of them again
+struct Again {
+    int first, last;
+    __device__ __forceinline__ void none() { first = 0x7fffffff; last = -1; }
+    __device__ __forceinline__ void add(int item) { atomicMin(&first, item); atomicMax(&last, item); }
+};
 
 struct Args {
     const float *qkv, *decay;

@@ -6,8 +6,9 @@
 //   chain_kernel    S <- G_C S + F - M S over the chunks (no delta: without M); S before each chunk is kept
 //   read_kernel     O = P U_0 + Q' S_0
 // M, Q' and S are written as the parts of the products that read them, so these two only copy them to shared memory.
-// Nothing runs backwards in time: rows of G K, V, W and U_0 that hold something that is not finite enter the products that multiply them
-// with T's and P's zeros without it, and what they reach -- a row of G K all of the later tokens, a value its column -- becomes NaN.
+// Nothing runs backwards in time: rows of G K, V, W and U_0 that hold something without parts enter the products that multiply them
+// with T's and P's zeros without it, and what they reach -- a row of G K all of the later tokens, a value its column -- becomes NaN.  When a
+// CTA is through with its items, it sums what is not finite of F and the outputs again in plain fp32 from P, T and V: infinities stay infinities.
 #include "chunk_tc5.cuh"
 
 namespace {
@@ -34,22 +35,84 @@ struct Layout {
     }
 };
 
-// eight entries without those that are not finite; `bad` is told their places
+// eight entries without those that have no parts; `bad` is told their places
 template <typename F>
 __device__ __forceinline__ void clean(float (&x)[8], F&& bad) {
     float s = 0.f;
 #pragma unroll
     for (int e = 0; e < 8; ++e) s += fabsf(x[e]);
-    if (finite(s)) return;
+    if (splits(s)) return;
 #pragma unroll 1
     for (int e = 0; e < 8; ++e) {
         float v = x[0];
 #pragma unroll
         for (int u = 1; u < 8; ++u) v = e == u ? x[u] : v;
-        if (finite(v)) continue;
+        if (splits(v)) continue;
         bad(e);
 #pragma unroll
         for (int u = 0; u < 8; ++u) x[u] = e == u ? 0.f : x[u];
+    }
+}
+
+// U_0 of a column: 64 tokens in fp32 (no T: V)
+__device__ __forceinline__ void plain_u(const float* T, const float* v, int stride, int nt, float (&u)[C]) {
+#pragma unroll 1
+    for (int t = 0; t < C; ++t) {
+        float sum = t < nt ? v[(size_t)t * stride] : 0.f;
+        if (T) {
+            sum = 0.f;
+            for (int s = 0; s <= t && s < nt; ++s) sum = fmaf(T[t * C + s], v[(size_t)s * stride], sum);
+        }
+        u[t] = sum;
+    }
+}
+// Results of wy_kernel that are not finite, summed again
+template <bool CH, bool DELTA>
+__device__ __noinline__ void again_wy(const Args& a, const Again& again) {
+    const int tid = threadIdx.x, dk = a.dk, dv = a.dv, Cq = 2 * a.G * dk + a.H * dv, c = tid & 127, part = tid >> 7;
+    const Layout L(dk, dv, CH, DELTA);
+    for (int m = again.first; m <= again.last; ++m) {
+        const At at = locate<C>(a, blockIdx.x + m * gridDim.x);
+        const int j = at.block * 128 + c;
+        if (j >= dv) continue;
+        float* ws = a.ws + ((size_t)at.chunk * a.H + at.head) * L.total;
+        const float* k = CH ? ws + L.dec + 2 * C * dk : a.qkv + (size_t)at.row * Cq + (a.G + at.head / (a.H / a.G)) * dk;
+        float u[C];
+        plain_u(DELTA ? ws + L.t : nullptr, a.qkv + (size_t)at.row * Cq + 2 * a.G * dk + at.head * dv + j, Cq, at.nt, u);
+        for (int t = part; t < at.nt; t += 4) {
+            float* o = a.o + ((size_t)(at.row + t) * a.H + at.head) * dv + j;
+            if (finite(*o)) continue;
+            float sum = 0.f;
+            for (int s = 0; s <= t; ++s) sum = fmaf(ws[L.p + t * C + s], u[s], sum);
+            *o = sum;
+        }
+        for (int i = part; i < dk; i += 4) {
+            float* f = ws + L.f + (DELTA ? (size_t)j * dk + i : (size_t)i * dv + j);
+            if (finite(*f)) continue;
+            float sum = 0.f;
+            for (int t = 0; t < at.nt; ++t) sum = fmaf(CH ? k[(size_t)t * dk + i] : ws[L.dec + C + t] * k[(size_t)t * Cq + i], u[t], sum);
+            *f = sum;
+        }
+    }
+}
+// ... of read_kernel without the correction: P V + G Q S_0
+__device__ __noinline__ void again_read(const Args& a, const Again& again) {
+    const int dk = a.dk, dv = a.dv, Cq = 2 * a.G * dk + a.H * dv;
+    const Layout L(dk, dv, true, false);
+    for (int m = again.first; m <= again.last; ++m) {
+        const At at = locate<C>(a, blockIdx.x + m * gridDim.x);
+        const float* ws = a.ws + ((size_t)at.chunk * a.H + at.head) * L.total, *v = a.qkv + (size_t)at.row * Cq + 2 * a.G * dk + at.head * dv;
+        for (int e = threadIdx.x; e < 128 * at.nt; e += blockDim.x) {
+            const int t = e >> 7, j = at.block * 128 + (e & 127);
+            float* o = a.o + ((size_t)(at.row + t) * a.H + at.head) * dv + j;
+            if (j >= dv || finite(*o)) continue;
+            const unsigned char* s0 = reinterpret_cast<const unsigned char*>(ws + L.s) + (j >> 6) * L.slices * (3 * 8192) + (j & 7) * 2;
+            float sum = 0.f;
+            for (int i = 0; i < dk; ++i)
+                sum = fmaf(ws[L.dec + (C + t) * dk + i], joined(s0 + (i >> 6) * (3 * 8192) + tile_at(i & 63, (j & 63) >> 3, 64), 8192), sum);
+            for (int s = 0; s <= t; ++s) sum = fmaf(ws[L.p + t * C + s], v[(size_t)s * Cq + j], sum);
+            *o = sum;
+        }
     }
 }
 
@@ -62,13 +125,14 @@ __device__ __forceinline__ void clean(float (&x)[8], F&& bad) {
 // was part of the chain before and took it 196 us on the FMA pipe, where nothing ran beside it.
 template <bool CH, bool DELTA>
 __global__ void __launch_bounds__(512, 1)
-wy_kernel(const Args a) {
+wy_kernel(const __grid_constant__ Args a) {
     extern __shared__ unsigned char sm_raw[];
     enum { OUT_Q, OUT_M, OUT_F };
     __shared__ __align__(8) uint64_t s_done[2], s_out[3];
     __shared__ unsigned s_full[6], s_staged[3];
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed;
+    __shared__ Again s_again;
     __shared__ int s_row[2], s_col[2][128];          // first token with a bad G K; first bad value of a column
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     At at = locate<C>(a, blockIdx.x);
@@ -80,6 +144,7 @@ wy_kernel(const Args a) {
     auto out = [&](int u) { return b2::smem_u32(&s_out[u]); };
     if (tid == 0) {
         s_failed = 0;
+        s_again.none();
         for (int u = 0; u < 6; ++u) s_full[u] = 0;
         for (int u = 0; u < 3; ++u) {
             s_staged[u] = 0;
@@ -266,9 +331,14 @@ wy_kernel(const Args a) {
             const int j = at.block * 128 + feature, bad = min(*(volatile int*)row, *(volatile int*)&col[feature]);
             if (j < dv) {
                 float* dst = a.o + ((size_t)(at.row + t0) * a.H + at.head) * dv + j;
+                float sum = 0.f;
 #pragma unroll
                 for (int i = 0; i < 16; ++i, dst += a.H * dv)
-                    if (t0 + i < at.nt) *dst = failed || t0 + i >= bad ? kNaN : w[i];
+                    if (t0 + i < at.nt) {
+                        *dst = failed || t0 + i >= bad ? kNaN : w[i];
+                        sum += fabsf(w[i]);
+                    }
+                if (!finite(sum) || bad < C) s_again.add(n);
             }
         }
         // the results go through shared memory, which copies them out as they lie there: Q' where T and P were
@@ -312,7 +382,7 @@ wy_kernel(const Args a) {
         }
         {
             const int cols = min(128, dv - at.block * 128), wide = DELTA ? dk : cols;        // floats a row
-            float* f = reinterpret_cast<float*>(at_sm(x0) - PART) + (size_t)(cg * 32) * wide + feature;
+            float* f = reinterpret_cast<float*>(at_sm(x0) - PART) + (size_t)(cg * 32) * wide + feature, sum = 0.f;
             const bool bad = failed || all_bad || (!DELTA && *(volatile int*)&col[feature] < C);
             // DELTA: a register is a column, and 32 lanes look at 32 marks
             const unsigned bad_cols = DELTA ? __ballot_sync(0xffffffffu, *(volatile int*)&col[cg * 32 + lane] < C) : 0u;
@@ -322,8 +392,12 @@ wy_kernel(const Args a) {
                 read_parts(rb + cg * 32 + 16 * h, x);
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
-                    if (feature < wide) f[(16 * h + i) * wide] = bad || (bad_cols >> (16 * h + i) & 1) ? kNaN : x[i];
+                    if (feature < wide) {
+                        f[(16 * h + i) * wide] = bad || (bad_cols >> (16 * h + i) & 1) ? kNaN : x[i];
+                        sum += fabsf(x[i]);
+                    }
             }
+            if (bad_cols || bad || !finite(sum)) s_again.add(n);
             if (hand_over(&s_staged[OUT_F])) {
                 if (lane == 0) {
                     if (DELTA) copy_out(ws + L.f + (size_t)at.block * 128 * dk, x0 - PART, cols * dk * 4);
@@ -345,7 +419,9 @@ wy_kernel(const Args a) {
         if (turns0) drain(done(0), (turns0 - 1) & 1);
         if (turns1) drain(done(1), (turns1 - 1) & 1);
     }
+    b2::fence_proxy_async();                         // F was copied out
     tmem_free(tmem, warp);
+    if (!*(volatile int*)&s_failed) again_wy<CH, DELTA>(a, s_again);
 }
 
 // ---------------------------------------------------------------------------------------------------------------- the chain
@@ -528,7 +604,7 @@ state_kernel(const Args a) {
         for (int u = 0; u < AHEAD; ++u) {
             const int c = c0 + u;
             if (c < nchunks) {
-                store_parts4(to + (size_t)c * step * 4, 8192, s);
+                store_any4(to + (size_t)c * step * 4, 8192, s);
                 if (pad) continue;
                 s = make_float4(fmaf(s.x, d[u], x[u].x), fmaf(s.y, d[u], x[u].y), fmaf(s.z, d[u], x[u].z), fmaf(s.w, d[u], x[u].w));
                 if (c + AHEAD < nchunks) {
@@ -547,11 +623,12 @@ state_kernel(const Args a) {
 // Bound by the copies: 4096 tokens, 16 heads of 128, 29 us for 151 MB of images and 67 of outputs, part of them in L2 (the FMA pipe took 84).
 template <bool CH, bool DELTA>
 __global__ void __launch_bounds__(320, 1)
-read_kernel(const Args a) {
+read_kernel(const __grid_constant__ Args a) {
     extern __shared__ unsigned char sm_raw[];
     __shared__ __align__(8) uint64_t s_here[3], s_free[3], s_done[2], s_read[2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed;
+    __shared__ Again s_again;
     constexpr int STAGE = 9 * 8192;                  // two slices of S_0's columns, and Q'
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     At at = locate<C>(a, blockIdx.x);
@@ -560,6 +637,7 @@ read_kernel(const Args a) {
     auto bar = [&](uint64_t* b, int i) { return b2::smem_u32(&b[i]); };
     if (tid == 0) {
         s_failed = 0;
+        s_again.none();
         for (int u = 0; u < 3; ++u) {
             b2::mbar_init(bar(s_here, u), 1);
             b2::mbar_init(bar(s_free, u), 1);
@@ -643,9 +721,14 @@ read_kernel(const Args a) {
                 __syncwarp();
                 if (lane == 0) b2::mbar_arrive(bar(s_read, n & 1));
                 const bool bad = *(volatile int*)&s_failed != 0;
+                float sum = 0.f;
 #pragma unroll
                 for (int i = 0; i < 32; ++i)
-                    if (i < rows) o[i * stride] = bad ? kNaN : x[i];
+                    if (i < rows) {
+                        o[i * stride] = bad ? kNaN : x[i];
+                        if (!DELTA) sum += fabsf(x[i]);
+                    }
+                if (!DELTA && !finite(sum)) s_again.add((item - (int)gridDim.x - (int)blockIdx.x) / (int)gridDim.x);
                 ++n;
             }
             at = next;
@@ -653,6 +736,7 @@ read_kernel(const Args a) {
     }
     if (*(volatile int*)&s_failed && n > 0) drain(bar(s_done, (n - 1) & 1), ((n - 1) / 2) & 1);
     tmem_free(tmem, warp);
+    if (!DELTA && !*(volatile int*)&s_failed) again_read(a, s_again);
 }
 
 template <bool CH, bool DELTA>
