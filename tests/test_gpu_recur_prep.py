@@ -47,7 +47,7 @@ def test_prompt_rows_equal_those_of_smaller_batches(cuda, dt, H, G, dk, dv, unit
 
 
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("H,dk,dv,taps", [(4, 64, 64, 4), (2, 32, 20, 3), (16, 128, 128, 2), (1, 8, 4, 4)])
+@pytest.mark.parametrize("H,dk,dv,taps", [(4, 64, 64, 4), (2, 32, 20, 3), (16, 128, 128, 2), (1, 8, 4, 4), (16, 128, 128, 4), (16, 128, 128, 3)])
 @pytest.mark.parametrize("lengths", [[300, 1, 2, 7, 301], [1, 509, 4, 3, 500, 90, 511, 505], [1] * 513, [400, 300] * 3])
 def test_runs_over_several_sequences_equal_each_alone(cuda, dt, H, dk, dv, taps, lengths):
     """From 512 rows on a CTA goes through a run of rows: a sequence that begins or ends within one keeps its own history.  Alone each is
