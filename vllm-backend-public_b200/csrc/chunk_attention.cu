@@ -289,7 +289,8 @@ qk_rope_cache_vec_kernel(const T* __restrict__ qkv, int64_t qkv_stride, int H, i
 // takes one row and loads it itself (a decode step has too few rows for the copies to run ahead).
 // Bound: memory, and the norm, which needs a whole row before its first result.  4096 rows of 32 + 8 heads of 128 with NORM (92 MB): kernel
 // above 39 us, this one 31; without NORM 16 + 4 heads 20.6 -> 10.4, 32 + 8 in neighbours 33 -> 27; a row ahead in registers instead of
-// the ring took 36 with NORM.  380 instructions a warp and row are half of the issue slots.
+// the ring took 36 with NORM.  380 instructions a warp and row are half of the issue slots.  1024 threads a CTA hold it to 64 registers, of
+// which the ring with NORM spills 48 bytes.
 constexpr int kRopeStages = 6;
 struct RopeArgs {
     const __nv_bfloat16* qkv;

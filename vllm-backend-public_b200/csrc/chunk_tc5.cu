@@ -12,10 +12,11 @@
 // their columns become NaN from their tokens on.  When a CTA is through with its items, it sums what is not finite again in plain fp32: infinities
 // stay infinities.
 //
-// 4096 tokens, 16 heads of 128 x 128 in a graph: 121 us (with the products on the FMA pipe 243, token by token 804); 500 tokens 34 (41, 102).
+// 4096 tokens, 16 heads of 128 x 128 in a graph: 124 us (with the products on the FMA pipe 243, token by token 804); 500 tokens 35 (41, 102).  Under
+// ncu, cold: kv 35, state 22, out 75.
 // out_kernel's item takes 30e3 cycles, of which the MMAs are 9e3: splitting into parts, the copies of S_0 (20 bytes a cycle and SM when all
 // ask at once) and the read-back follow one another in the one CTA that an SM's shared memory holds.  Two CTAs of 64 tokens an SM took 89 us
-// instead of 72 (twice the instructions), a warp of its own for the MMAs 78 - 90 (the registers it costs the others spill).
+// instead of the 72 that this one took then (twice the instructions), a warp of its own for the MMAs 78 - 90 (the registers it costs the others spill).
 #include "chunk_tc5.cuh"
 
 namespace {

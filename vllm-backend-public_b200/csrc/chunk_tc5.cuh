@@ -1,12 +1,14 @@
 // chunk_tc5.cuh -- fp32 products on the bf16 tensor cores, as the chunked recurrence uses them.
 //
 // A float is the sum of three bf16 numbers (its rounding to 8 bits, that of the rest, and what is left: exact), and a product of two
-// floats is six of the nine products of their parts: what is left out is below 2^-25 of it.  (Parts by truncation instead of rounding
+// floats is six of the nine products of their parts: what is left out is below 2^-25 of it (Henry, Tang, Heinecke, "Leveraging the bfloat16
+// artificial intelligence datatype for higher-precision computations", 2019).  (Parts by truncation instead of rounding
 // take as many instructions and are all of one sign: errors a third higher.)  Products of parts are exact in fp32, but
 // the tensor core truncates its accumulator at every instruction, so the leading parts' products have an accumulator of their own, which
 // takes one addition per 16 entries, or the small products come first.  Sums of 128 products of normal numbers against 64 bits, relative to
 // the result's norm: 1.2e-7 with two accumulators, 0.8e-7 with one per 64 entries and the small products first, 8.2e-7 with one for all;
-// a chain of 128 FMAs 2.0e-7.
+// a chain of 128 FMAs 2.0e-7.  Of 64 products: 7.0e-8 with one leading accumulator, 5.1e-8 with two in turns, 4.7e-8 with four; FMAs 1.4e-7.
+// Cutting off draws every result towards zero (4.5e-8 of it with one accumulator, 2.3e-8 with two), so more of them help twice.
 //
 // Operands are tiles of 128-byte rows in the 128-byte swizzle: rows of 64 entries of the summed index (K-major), or rows of 64 entries of
 // the result's index, a row per summed index (MN-major).

@@ -141,7 +141,8 @@ __global__ void recur_prep_kernel(const T* __restrict__ proj, int64_t proj_strid
 // Bound: memory (2 or 4 bytes in and 4 out per channel), with the exact exponentials and divisions of the activation close behind.
 // One CTA a row with scalar accesses and a staging pass took 88 us at 4096 rows of 6144 channels (rotation, no convolution), 174 at 3001
 // rows (four taps, SiLU, unit vectors) and 59 at 64 rows; this one 58, 53 and 27 (the second 63
-// with the inputs moved from place to place and runs of 8).  Without a convolution recur_prep_heads_kernel takes prompts.
+// with the inputs moved from place to place and runs of 8).  Four taps spill 32 bytes at these 64 registers, and three CTAs an SM were not tried.
+// Without a convolution recur_prep_heads_kernel takes prompts.
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(256, 4)
 recur_prep_vec_kernel(const T* __restrict__ proj, int64_t proj_stride, PrepSpec sp, const float* __restrict__ conv_w,

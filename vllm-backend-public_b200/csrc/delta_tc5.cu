@@ -120,9 +120,10 @@ __device__ __noinline__ void again_read(const Args& a, const Again& again) {
 // Tiles in shared memory: X0 for G K and later G_C/G K, X1 for V and later U_0, Y for W, T and P; in the end 16 KB and X0 for F, X1 and Y
 // for M, T and P for Q'.
 // Bound by its own phases: with 208 KB of tiles and copies one CTA fits an SM, and an item of 64 tokens goes through ten of them (loads, split,
-// product, read back, split ...), 33e3 cycles, 7e3 of which the copies out take (29 bytes a cycle).  1024 items (4096 tokens, 16 heads of
-// 128) 108 us: 122 with the keys read where they are needed instead of an item ahead, 115 with the decays read per token.  The same work
-// was part of the chain before and took it 196 us on the FMA pipe, where nothing ran beside it.
+// product, read back, split ...), 33e3 cycles, 7e3 of which the copies out take (29 bytes a cycle).  784 items (1119 + 779 + 1103 tokens, 16 heads of
+// 128 x 128) 111 us (ncu, cold; 1024 items of 4096 tokens 131): 122 with the keys read where they are needed instead of an item ahead, 115 with
+// the decays read per token.  U_0 and P U_0 have two leading accumulators, for 3 us: with one their outputs are 1.02 times as far from 64 bits.
+// 128 registers spill 28 bytes per head and 8 per channel, once an item.
 template <bool CH, bool DELTA>
 __global__ void __launch_bounds__(512, 1)
 wy_kernel(const __grid_constant__ Args a) {
@@ -427,9 +428,9 @@ wy_kernel(const __grid_constant__ Args a) {
 // ---------------------------------------------------------------------------------------------------------------- the chain
 // A CTA per 64 columns of a head's state.  Eight warps keep it in registers, in fp32 (lane a key feature, 32 columns a thread), and
 // write its parts; one warp copies M ahead, three slices of 64 features in a ring; one multiplies and copies the parts out.
-// Bound by one SM's intake: a step's 96 KB of M come at 54 bytes a cycle, 0.95 us, beside which split, product and read-back of the step take
-// place; 64 chunks, 16 heads of 128 x 128, 61 us, where W and U on the FMA pipe within the chain took 196.  32 columns a CTA would
-// put twice the SMs to work, each with the same M.
+// Bound by a step's own phases, one after another: split, store, product, read back; 2.9 us a step (64 chunks of one sequence, 16 heads of
+// 128 x 128, 185 us; 18 chunks at most, 1119 + 779 + 1103 tokens, 61 us, where W and U on the FMA pipe within the chain took 196).  Its 96 KB
+// of M a step come a ring ahead, at a quarter of what an SM can take in.
 template <bool CH>
 __global__ void __launch_bounds__(320, 1)
 chain_kernel(const Args a) {
@@ -620,7 +621,8 @@ state_kernel(const Args a) {
 
 // ---------------------------------------------------------------------------------------------------------------- read-out
 // O^T += S_0^T Q'^T: both operands are copied as they are, three stages of a slice of 64 features (72 KB); two accumulators alternate.
-// Bound by the copies: 4096 tokens, 16 heads of 128, 29 us for 151 MB of images and 67 of outputs, part of them in L2 (the FMA pipe took 84).
+// Bound by the copies: 3001 tokens, 16 heads of 128 x 128, 29 us for 116 MB of images and twice 25 MB of outputs, part of them in L2 (the FMA pipe
+// took 84).  Two leading accumulators for Q' S_0, which is a sum over up to 128 features.
 template <bool CH, bool DELTA>
 __global__ void __launch_bounds__(320, 1)
 read_kernel(const __grid_constant__ Args a) {
