@@ -4,7 +4,7 @@ timed on the same seeded problems as bench.py, beside this repo's kernel.  Not t
 that can execute here.  Run by bench_legs.comparator_leg() in a subprocess; writes one JSON file, rewritten after every
 comparator so a time-out keeps what finished.
 
-    python scripts/comparator.py --out gpurun_out/comparator.json [--launches 100]
+    python scripts/comparator.py --out out/comparator.json [--launches 100]
 
   vllm         torch.ops._C.paged_attention_v2 (partition 512), its own cache layout, filled by its reshape_and_cache
   flash_attn   flash_attn_with_kvcache over a paged cache (FA2 needs page_block_size % 256 == 0, so pages of 256 tokens)

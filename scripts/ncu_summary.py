@@ -1,8 +1,8 @@
 #!/usr/bin/env python
-"""Summarise `ncu --set full` reports (gpurun_out/*.ncu-rep) into small text files under profiles/.
+"""Summarise `ncu --set full` reports (out/*.ncu-rep) into small text files under profiles/.
 
-    python scripts/ncu_summary.py gpurun_out/prof_x.ncu-rep [...] --out profiles/r1_ncu_full.md
-    python scripts/ncu_summary.py --launches gpurun_out/launches_x.csv --out profiles/r1_launches.md
+    python scripts/ncu_summary.py out/prof_x.ncu-rep [...] --out profiles/ncu_x.md
+    python scripts/ncu_summary.py --launches out/launches_x.csv --out profiles/launches_x.md
 
 Runs here (no GPU): `ncu -i <rep> --page raw --csv` reads the report offline.
 """

@@ -4,7 +4,7 @@
 The client is the evaluation Job of the reference's loop: b200attn/templates/evaluate.yaml rendered by the
 process_template rule (reference benchmark-eval/main.py:55-58,113) for this model and engine URL, and the Job's
 container command run locally (b200attn.evaljob) -- no Kubernetes on the box.  --tensor-parallel-size N serves on N GPUs.
-Writes gpurun_out/e2e_<tag>.json (raw + standardized EvaluationPayload) and prints the standardized metrics."""
+Writes out/e2e_<tag>.json (raw + standardized EvaluationPayload) and prints the standardized metrics."""
 import argparse
 import os
 import subprocess
@@ -52,7 +52,7 @@ try:
             sys.exit("server not healthy after 600 s")
         time.sleep(0.5)
     print(f"server healthy after {time.time() - t0:.1f}s", flush=True)
-    out = ROOT / "gpurun_out" / f"e2e_{a.tag}.json"
+    out = ROOT / "out" / f"e2e_{a.tag}.json"
     out.parent.mkdir(exist_ok=True)
     # the evaluation Job: template -> process_template -> YAML check -> run its container command here
     text, job = evaljob.render_for_model(a.model, base)

@@ -4,8 +4,8 @@ The reference launches vLLM as an external server (`vllm/vllm-openai:v0.9.1`,
 reference benchmark-vllm/vllm_manager.py:371-374) and holds no vectors for this path.  vLLM is the dependency whose
 `reshape_and_cache` / `paged_attention_v1/v2` semantics the oracle restates, so its kernels, run here on the same
 seeded inputs, are the closest thing to reference outputs.  This script writes
-    gpurun_out/vllm_crosscheck.pt      {case: {"out_v1", "out_v2", "k_cache_sha", "v_cache_sha", ...}}
-    gpurun_out/vllm_crosscheck.json    what ran, versions, or why it could not
+    out/vllm_crosscheck.pt      {case: {"out_v1", "out_v2", "k_cache_sha", "v_cache_sha", ...}}
+    out/vllm_crosscheck.json    what ran, versions, or why it could not
 which are then committed under tests/golden/ and checked by tests/test_vllm_crosscheck.py (oracle, CPU) and
 tests/test_gpu_parity.py (our kernels).  Nothing here is imported by the product.
 
@@ -24,7 +24,7 @@ ROOT = HERE.parent.parent
 sys.path.insert(0, str(ROOT / "oracle"))
 import paged_attention_ref as R  # noqa: E402
 
-OUT = ROOT / "gpurun_out"
+OUT = ROOT / "out"
 OUT.mkdir(exist_ok=True)
 
 CASES = {

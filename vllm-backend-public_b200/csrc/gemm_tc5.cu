@@ -5,7 +5,7 @@
 // rank 3 lets the GEMMs be library calls; at M = 64 the op is a weight STREAM (64 flop per weight byte, HBM-bound), and
 // in-graph cuBLAS reaches 53-88 % of the HBM bandwidth on the Llama-3-8B decode shapes and 13-49 % on the per-rank
 // shapes of --tensor-parallel-size 8.  This kernel was written to beat that and does not yet: 0.47-0.81x of the
-// library's speed (profiles/r2_decode_gemm.jsonl) -- one non-persistent CTA per (feature tile, K slice) pays TMEM
+// library's speed (profiles/later_decode_gemm.jsonl) -- one non-persistent CTA per (feature tile, K slice) pays TMEM
 // allocation, pipeline ramp and two cluster barriers on <= 0.5 MB of weights.  DESIGN.md section 8 says what would.
 //
 // Shape of the kernel (swap-AB, split-K over a thread-block cluster):

@@ -920,7 +920,7 @@ __device__ __forceinline__ uint32_t dyn_runs_of_item_fast(uint32_t ci0, uint32_t
 }
 
 // The four consumer warps (tid128 = 0..127) combine the partial runs of one item into bf16 output rows.
-// (Round 2 experiment, removed again: combining the partials INSIDE the decode kernel -- per-item arrival counters in
+// (Tried and removed again: combining the partials INSIDE the decode kernel -- per-item arrival counters in
 // the workspace header, the CTA that writes an item's last partial merges it -- was parity-green but slower than the
 // PDL merge kernel on every ragged shape (63.1 vs 60.1 us config-2 shape, 99.9 vs 89.6 fp8): two fences + an atomic at
 // every partial run's end sit on the consumers' critical path, the merging CTA stalls its own pipeline, and the extra

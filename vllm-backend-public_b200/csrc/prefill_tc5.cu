@@ -15,15 +15,15 @@
 // Issue order  QK_A(0) QK_B(0) | PV_A(j) QK_A(j+1) PV_B(j) QK_B(j+1) ...  lets the softmax of one tile run under the
 // MMAs of the other; P.V(j) is issued in two halves as the softmax hands over keys 0-63 and 64-127.  Rescaling of O is lazy: a row keeps its stale maximum until the true one exceeds it by 2^8.
 //
-// Round 2, what bounded the kernel and what did not (8k chunk over an 8k prefix, Llama-3-8B heads, block_size 16;
-// clock64 timeline from `make trace` + scripts/trace_prefill.py, profiles/r2_trace_prefill_issuer*.txt):
-//   1055 TF/s  round-1 kernel.  ncu: tensor pipe 48 %, XU pipe 48 %, softmax warps waiting for S in 56 % of samples.
-//   not it     softmax latency hiding: TWO threads per query row (profiles/r2_ncu_prefill_two_threads_per_row.md)
+// What bounded the kernel and what did not (8k chunk over an 8k prefix, Llama-3-8B heads, block_size 16;
+// clock64 timeline from `make trace` + scripts/trace_prefill.py, profiles/later_trace_prefill_issuer*.txt):
+//   1055 TF/s  first kernel.  ncu: tensor pipe 48 %, XU pipe 48 %, softmax warps waiting for S in 56 % of samples.
+//   not it     softmax latency hiding: TWO threads per query row (profiles/later_ncu_prefill_two_threads_per_row.md)
 //              1038; maximum pass off the chain (speculative maximum) 947;
 //              polynomial exp2 for 1-3 of every 4 weights (B2_PREFILL_POLY) slower then and now (1371 / 1266 / 1164).
 //   not it     shared-memory operand bandwidth of cta_group::1 (an earlier reading of the timeline, WRONG):
-//              scripts/umma_rate.cu shows SS, TS, MN-major B, the kernel's own P.V | Q.K^T mix and all of them under
-//              concurrent TMEM traffic at 64.1 cycles per 128x128x16 = full rate (profiles/r2_umma_rate.txt).
+//              a loop of MMAs shows SS, TS, MN-major B, the kernel's own P.V | Q.K^T mix and all of them under
+//              concurrent TMEM traffic at 64.1 cycles per 128x128x16 = full rate (profiles/later_umma_rate.txt).
 //   +8 %       the producer: ONE lane issued the 32 TMA boxes of a step (block_size 16: 2 KiB boxes) one after the other,
 //              ~70 cycles each.  Now warp 8 streams K and warp 10 streams V, one box per lane, and the V stage is released
 //              before the next Q.K^T is issued.  Tiles land ~1500 cycles after their stage frees (1140 TF/s).
@@ -99,7 +99,7 @@ struct Tc5Params {
 };
 
 // 2^x for x <= 0 on the FMA/ALU pipes (the MUFU unit does 16 ex2 per clock and SM: with every weight on it the two
-// tiles' softmax needs as many cycles as their MMAs, profiles/r1_ncu_prefill_tc5.md).  Round x to the nearest integer
+// tiles' softmax needs as many cycles as their MMAs, profiles/first_ncu_prefill_tc5.md).  Round x to the nearest integer
 // n with the 1.5 * 2^23 trick, 2^f on [-0.5, 0.5] by a cubic (relative error 7.5e-5, far below the bf16 rounding of
 // P), n added to the exponent field.
 __device__ __forceinline__ float poly_exp2(float x) {
@@ -201,7 +201,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             // One box = one 64-element half of one (block, kv head) tile = bs x 128 B; at block_size 16 a 128-token tile
             // is 16 boxes.  Each box is issued by its own lane (a lone lane issuing all 32 boxes of a step one after the
             // other took longer than the step: the MMA warp waited ~800 cycles per step for V(j) / K(j+1), see
-            // profiles/r2_trace_prefill_issuer.txt), and K and V wait for their own empty barriers in separate warps.
+            // profiles/later_trace_prefill_issuer.txt), and K and V wait for their own empty barriers in separate warps.
             const int kv = warp == 10;
             const CUtensorMap* tm = kv ? &tmV : &tmK;
             if (lane == 0) {
@@ -266,7 +266,7 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             // group of instructions.  Round 2: with the loop inside `if (lane == 0)` the operands lived in per-thread
             // registers and ptxas wrapped EVERY tcgen05.mma in an ELECT / R2UR.BROADCAST / BRA.U.ANY loop of ~12
             // dependent instructions; sharing its scheduler with two softmax warps, the issuing thread then needed
-            // 80-105 cycles per instruction where the pipe needs 64 (profiles/r2_trace_prefill_issuer.txt).
+            // 80-105 cycles per instruction where the pipe needs 64 (profiles/later_trace_prefill_issuer.txt).
             {
                 constexpr uint32_t ID_QK = idesc_bf16(128, 128, 0), ID_PV = idesc_bf16(128, 128, 1);
                 // low descriptor words of the operands (see desc_lo): Q_x, the K half and the V half of stage 0
