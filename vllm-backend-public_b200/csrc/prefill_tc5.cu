@@ -27,10 +27,8 @@
 //   +8 %       the producer: ONE lane issued the 32 TMA boxes of a step (block_size 16: 2 KiB boxes) one after the other,
 //              ~70 cycles each.  Now warp 8 streams K and warp 10 streams V, one box per lane, and the V stage is released
 //              before the next Q.K^T is issued.  Tiles land ~1500 cycles after their stage frees (1140 TF/s).
-//   +21 %      the issuer: the loop ran inside `if (lane == 0)`, so every operand lived in a per-thread register and ptxas
-//              wrapped EVERY tcgen05.mma in an ELECT / R2UR.BROADCAST / BRA.U.ANY loop, ~12 dependent instructions that
-//              the issuing thread -- sharing its scheduler with two softmax warps -- needed 80-105 cycles for, where the
-//              pipe needs 64.  The whole warp now runs the loop with warp-uniform operands and elect.sync picks the lane
+//   +21 %      the issuer: the loop ran inside `if (lane == 0)`, so no operand was uniform to the compiler, and the issuing thread --
+//              sharing its scheduler with two softmax warps -- needed 80-105 cycles a tcgen05.mma, where the pipe needs 64.  The whole warp now runs the loop with warp-uniform operands and elect.sync picks the lane
 //              per instruction group (what CUTLASS does) (1375 TF/s).
 //   +2.5 %     P is handed over in two halves, so P.V of keys 0-63 runs under the exponentials of keys 64-127 (1409 TF/s,
 //              0.845 of the measured cuBLAS bf16 burst).  Quarters would cost the softmax as much as they save the chain.
@@ -113,7 +111,7 @@ __device__ __forceinline__ float poly_exp2(float x) {
 }
 
 // =============================================================================================
-// the kernel.  POLY of every 4 consecutive softmax weights take poly_exp2, the rest MUFU.EX2.
+// the kernel.  POLY of every 4 consecutive softmax weights take poly_exp2, the rest ex2.approx.
 // =============================================================================================
 // SPLIT (rows_per_cta = 128: launches that would leave SMs idle at 256 rows per CTA, e.g. a 512-token chunk over a long
 // prefix): both slots work on the SAME 128 query rows and share the keys between them -- slot x takes the 128-key
@@ -263,9 +261,8 @@ prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             // ------------------------------------------ MMA issuer ------------------------------------------
             // The WHOLE warp runs this loop with warp-uniform control flow and operands (`warp` comes from a shuffle,
             // every address below derives from kernel parameters and loop counters), and one elected lane issues each
-            // group of instructions.  Round 2: with the loop inside `if (lane == 0)` the operands lived in per-thread
-            // registers and ptxas wrapped EVERY tcgen05.mma in an ELECT / R2UR.BROADCAST / BRA.U.ANY loop of ~12
-            // dependent instructions; sharing its scheduler with two softmax warps, the issuing thread then needed
+            // group of instructions.  With the loop inside `if (lane == 0)` no operand was uniform to the compiler, and the
+            // issuing thread, sharing its scheduler with two softmax warps, needed
             // 80-105 cycles per instruction where the pipe needs 64 (profiles/later_trace_prefill_issuer.txt).
             {
                 constexpr uint32_t ID_QK = idesc_bf16(128, 128, 0), ID_PV = idesc_bf16(128, 128, 1);
