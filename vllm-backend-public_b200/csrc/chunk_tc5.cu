@@ -30,7 +30,8 @@ constexpr int F_AT = 32;
 __host__ __device__ constexpr int image(int dk, int dv) { return F_AT + (dk * dv + 31) / 32 * 32; }
 __host__ __device__ constexpr int scratch(int dk, int dv) { return image(dk, dv) + (dk + 63) / 64 * ((dv + 127) / 128) * (3 * PART / 4); }
 
-// Results that are not finite, summed again from the inputs (and the state's parts) in plain fp32
+// Results that are not finite, summed again from the inputs (and the state's parts) in plain fp32, as far as they are no NaN.  It is for broken inputs: 4096
+// tokens of 16 heads take 2 ms with one infinite value, 3 with states of NaN, 5 with values of NaN.
 __device__ __noinline__ void again_sums(const Args& a, const Again& again) {
     const int tid = threadIdx.x, dk = a.dk, dv = a.dv, Cq = 2 * a.G * dk + a.H * dv, group = a.H / a.G;
     for (int m = again.first; m <= again.last; ++m) {
@@ -43,7 +44,7 @@ __device__ __noinline__ void again_sums(const Args& a, const Again& again) {
             if (j >= dv || finite(f[(size_t)i * dv + j])) continue;
             double to = 1.;
             float sum = 0.f;
-            for (int s = t.nt - 1; s >= 0; --s) {
+            for (int s = t.nt - 1; s >= 0 && sum == sum; --s) {
                 sum = fmaf(k[(size_t)s * Cq + i], (float)to * v[(size_t)s * Cq + j], sum);
                 to *= g[(size_t)s * a.H];
             }
@@ -78,9 +79,9 @@ __device__ __noinline__ void again_outputs(const Args& a, const Again& again, fl
             float* o = a.o + ((size_t)(t.row + r) * a.H + t.head) * dv + j;
             if (j >= dv || finite(*o)) continue;
             float sum = 0.f;
-            for (int i = 0; i < dk && !t.fresh; ++i)
+            for (int i = 0; i < dk && !t.fresh && sum == sum; ++i)
                 sum = fmaf(from[r] * q[(size_t)r * Cq + i], joined(s0 + (i >> 6) * (3 * PART) + tile_at(i & 63, c >> 3, 64) + (c & 7) * 2, PART), sum);
-            for (int s = 0; s <= r; ++s) sum = fmaf(P[r * CS + s], v[(size_t)s * Cq + j], sum);
+            for (int s = 0; s <= r && sum == sum; ++s) sum = fmaf(P[r * CS + s], v[(size_t)s * Cq + j], sum);
             *o = sum;
         }
     }

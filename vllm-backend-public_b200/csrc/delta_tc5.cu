@@ -83,14 +83,14 @@ __device__ __noinline__ void again_wy(const Args& a, const Again& again) {
             float* o = a.o + ((size_t)(at.row + t) * a.H + at.head) * dv + j;
             if (finite(*o)) continue;
             float sum = 0.f;
-            for (int s = 0; s <= t; ++s) sum = fmaf(ws[L.p + t * C + s], u[s], sum);
+            for (int s = 0; s <= t && sum == sum; ++s) sum = fmaf(ws[L.p + t * C + s], u[s], sum);
             *o = sum;
         }
         for (int i = part; i < dk; i += 4) {
             float* f = ws + L.f + (DELTA ? (size_t)j * dk + i : (size_t)i * dv + j);
             if (finite(*f)) continue;
             float sum = 0.f;
-            for (int t = 0; t < at.nt; ++t) sum = fmaf(CH ? k[(size_t)t * dk + i] : ws[L.dec + C + t] * k[(size_t)t * Cq + i], u[t], sum);
+            for (int t = 0; t < at.nt && sum == sum; ++t) sum = fmaf(CH ? k[(size_t)t * dk + i] : ws[L.dec + C + t] * k[(size_t)t * Cq + i], u[t], sum);
             *f = sum;
         }
     }
@@ -108,9 +108,9 @@ __device__ __noinline__ void again_read(const Args& a, const Again& again) {
             if (j >= dv || finite(*o)) continue;
             const unsigned char* s0 = reinterpret_cast<const unsigned char*>(ws + L.s) + (j >> 6) * L.slices * (3 * 8192) + (j & 7) * 2;
             float sum = 0.f;
-            for (int i = 0; i < dk; ++i)
+            for (int i = 0; i < dk && sum == sum; ++i)
                 sum = fmaf(ws[L.dec + (C + t) * dk + i], joined(s0 + (i >> 6) * (3 * 8192) + tile_at(i & 63, (j & 63) >> 3, 64), 8192), sum);
-            for (int s = 0; s <= t; ++s) sum = fmaf(ws[L.p + t * C + s], v[(size_t)s * Cq + j], sum);
+            for (int s = 0; s <= t && sum == sum; ++s) sum = fmaf(ws[L.p + t * C + s], v[(size_t)s * Cq + j], sum);
             *o = sum;
         }
     }
