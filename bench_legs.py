@@ -172,7 +172,7 @@ def tp_parity_leg(dev, group, model: str = "tiny8", seed: int = 1, gap: float = 
         if group.rank == 0:
             if str(ROOT / "oracle") not in sys.path:
                 sys.path.insert(0, str(ROOT / "oracle"))
-            import layer_ref as L                                       # the checker (oracle/), never the product path
+            import layer_ref as L                                       # the oracle (oracle/), never the product path
             full = LlamaModel(cfg, dev, num_blocks=1, seed=seed)        # same seed -> the unsharded weights
             w = {k: v.cpu() for k, v in full.w.items()}
             table = full.cos_sin.cpu()

@@ -20,7 +20,7 @@
     tests/test_vllm_crosscheck.py.  That wheel is not the reference's pinned v0.9.1 image.
 
 Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl reference legs
-may import this module -- as the checker or the timed CPU baseline, never as a product
+may import this module -- as the oracle or the timed CPU baseline, never as a product
 path.  The product (`b200attn`) has no CPU fallback and never imports it.
 
 Semantics:
