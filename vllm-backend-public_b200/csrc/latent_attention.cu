@@ -1156,7 +1156,7 @@ extern "C" int b2_window_attention_rows(void* out, const void* qn, int64_t qn_ro
     pa.q0 = qn; pa.q0_row = qn_row; pa.q0_head = qn_head;
     pa.q1 = qr; pa.q1_row = qr_row; pa.q1_head = qr_head;
     pa.k0 = kn; pa.k1 = kt; pa.k1_row = kt_row; pa.v = v;
-    pa.cu_k = cu_k; pa.k_lo = k_lo; pa.cu_q = cu_q; pa.ctx_start = ctx_start; pa.n_seq = n_seq; pa.T = T;
+    pa.cu_k = cu_k; pa.k_lo = k_lo; pa.k_rows = n_keys; pa.cu_q = cu_q; pa.ctx_start = ctx_start; pa.n_seq = n_seq; pa.T = T;
     pa.H = pa.G = H; pa.bs = 1; pa.dk0 = dn; pa.dk = dn + dr; pa.dv = dv; pa.maps = 1; pa.min_rows = 1;
     pa.scale = scale; pa.window = window;
     pa.sink = sink_logits ? 1.f : 0.f; pa.sink_logits = sink_logits;

@@ -2,13 +2,9 @@
 // kv head) and of b2_window_attention (keys and values rebuilt per head in gathered buffers), with every option of those entry
 // points: sliding window with kept first tokens, mask blocks, sinks, capped scores, sigmoid weights, two maps per head, gates.
 //
-// One CTA = two slots of 128 query rows; warps 0-3 / 4-7 are the softmax of slot 0 / 1 (a thread per row = TMEM lane), warp 9
-// issues the MMAs, warps 8 and 11 copy K tiles, warp 10 V tiles (all three Q), 128 keys at a time.  The slots are
-//   two query heads of one kv head on the same rows   where a kv head serves an even number of heads: both see the same keys, a
-//                                                     window of W keys costs W + 127 rounded up to tiles instead of W + 255
-//   two row tiles of one head                         otherwise
-//   the two maps of a head on the same rows           differential attention: slot x multiplies the keys of map x
-//   one slot                                          launches that would leave SMs idle
+// A CTA takes one tile: 128 query rows of a head in one slot, or its two maps on the same rows in two (differential attention: slot x
+// multiplies the keys of map x).  Warps 0-3 / 4-7 are the softmax of slot 0 / 1 (a thread per row = TMEM lane), warp 9 issues the MMAs, warps
+// 8 and 11 copy K tiles, warp 10 V tiles (all three Q), 128 keys at a time.  Launches of more tiles are prompt_turns_tc5.cu's.
 // Keys are walked in the compact order of KeySpan (kept first keys, then the union of the rows' windows), so a window costs no
 // tiles between its parts and neither page size nor alignment shows: the copies are 16-byte cp.async gathers with a page lookup
 // per key row, written in the 128-byte swizzle that the MMA descriptors name (gathered rows: TMA boxes).  A mask is tested per
@@ -22,27 +18,22 @@
 // score would need two more XU operations (the exponential and the division of tanh): where a whole warp's scores are below 3/16
 // of the cap, tanh is its Taylor polynomial to x^7 on the packed FMA pipe instead (remainder below 7e-9; the exponential form's
 // error is one fp32 rounding, 6e-8).
-// Measured (clock64, 128 keys x two slots): 3.3k cycles with heads of 192 / 128, of which the tensor pipe is busy 2.6k; 4.8k with
-// capped scores (the packed polynomial and the exponentials of both slots share the issue slots).
-//   4096 rows x 16 heads of 128 + 64 / 128, causal: 648 us (mma.sync, 64-row tiles) -> 78 us, in a graph
-//   4096 rows x 32 heads of 128, window 1024, capped: 461 us (mma.sync) -> 124 us; causal, not capped 877 -> 152 us
+// Measured in a graph with the kernels around it: 300 rows x 16 heads of 128, window 500: 15 us; 1000 rows 22; 1200 gathered rows x 16 heads of
+// 128 + 64 / 128, causal, 41.  A step of 128 keys is the softmax of the tile (0.5k cycles for the maximum, 0.6k to bring O along, 1.4k for the
+// weights) and the MMAs behind it, one after the other.
 // What cost most on the way: code size (95 - 145 KB with everything unrolled: every warp waited for instructions, 10.9k cycles per
 // tile; loops are rolled wherever registers are not indexed), and a divergent branch per row in the copies (~100 cycles an
 // instruction, serialised; zero-filling copies need none).
-#include "b2_mask.cuh"
-#include "b2_tc5.cuh"
+#include "prompt_tc5.cuh"
 
 #include <algorithm>
 
 namespace {
 
 using namespace b2tc;
+using namespace b2prompt;
 
-constexpr int BM = 128, BN = 128, NTHREADS = 384;
-constexpr int SUB = 128 * 128;                       // bytes of a [128 rows][64 el] sub-tile
-constexpr float LOG2E = 1.4426950408889634f;
-constexpr float FLOOR = -1e30f;                      // a row that has seen no key yet: exp2(-inf - FLOOR) = 0, not NaN
-enum { KIND_SOFTMAX = 0, KIND_CAPPED = 1, KIND_SIGMOID = 2 };
+constexpr int NTHREADS = 384;
 
 // NH: 64-column sub-tiles of a slot's Q and K; DVH: of V.  Three sub-tiles of K leave room for one V stage beside two of K.
 template <int NH, int DVH, bool TWO_MAPS>
@@ -58,17 +49,12 @@ struct Shape {
 
 struct Params {
     b2_prompt_args a;
-    int rows_per_cta, heads_per_cta;
     int bs_shift;                                    // log2 of the page size, or -1
     float scale_log2;
     int tma;                                         // gathered form: whole key tiles come by TMA boxes of 128 rows x 64 columns
     CUtensorMap map_k0, map_k1, map_v;
 };
 
-// 16 bytes, or zeros without reading `src` (no branch: a divergent one would serialise the copies of a warp)
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool ok) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
-}
 // (s0, s1) (1 + z a1 + z^2 a2 + z^3 a3), z = s^2, on the packed pipe: s tanh(x) / x of a score s = x / c, a_i = t_i c^2i with the
 // Taylor coefficients -1/3, 2/15, -17/315
 __device__ __forceinline__ void tanh_small_x2(uint32_t& s0, uint32_t& s1, float a1, float a2, float a3) {
@@ -77,25 +63,6 @@ __device__ __forceinline__ void tanh_small_x2(uint32_t& s0, uint32_t& s1, float 
         "mul.rn.f32x2 z, s, s;\n\tfma.rn.f32x2 p, z, c3, c2;\n\tfma.rn.f32x2 p, z, p, c1;\n\tmul.rn.f32x2 p, z, p;\n\t"
         "fma.rn.f32x2 s, s, p, s;\n\tmov.b64 {%0, %1}, s;\n\t}"
         : "+r"(s0), "+r"(s1) : "f"(a1), "f"(a2), "f"(a3));
-}
-// bits 0..31 of the columns [lo, hi) of a 32-column group that starts at column 0
-__device__ __forceinline__ uint32_t col_bits(int lo, int hi) {
-    lo = min(max(lo, 0), 32);
-    hi = min(max(hi, 0), 32);
-    return hi > lo ? (0xffffffffu >> (32 - (hi - lo))) << lo : 0u;
-}
-// what a query row sees of the compact key order: c <= hi and (c >= low or block <= c < keep)
-struct RowRange {
-    int hi, low, block;
-};
-__device__ __forceinline__ RowRange range_of(const KeySpan& span, int i, int chunk, int window) {
-    RowRange r;
-    r.hi = span.index(i);
-    r.block = 0;
-    if (chunk > 0) r.block = span.index((i / chunk) * chunk);
-    r.low = r.block;
-    if (window > 0) r.low = max(r.block, span.index(i - window + 1));
-    return r;
 }
 // what one thread works out for the CTA
 struct Plan {
@@ -126,14 +93,14 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
 
     // This CTA's tile: counted from the batch's last row backwards (late rows see more keys, and the spare CTAs of a grid that is an
     // upper bound come behind all tiles), by every warp for itself, 32 sequences at a time, so that a spare CTA leaves at once.
-    const int groups = a.H / prm.heads_per_cta, group = blockIdx.x % groups;
+    const int groups = a.H, group = blockIdx.x % groups;
     int seq = -1, q0 = 0, len = 0;
     {
         int want = blockIdx.x / groups;
 #pragma unroll 1
         for (int top = a.n_seq - 1; top >= 0; top -= 32) {
             const int s = top - lane, n = s >= 0 ? a.cu_q[s + 1] - a.cu_q[s] : 0;
-            const int nt = n >= a.min_rows ? (n + prm.rows_per_cta - 1) / prm.rows_per_cta : 0;
+            const int nt = n >= a.min_rows ? (n + BM - 1) / BM : 0;
             int upto = nt;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -145,7 +112,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                 const int who = __ffs(hit) - 1;
                 seq = top - who;
                 len = __shfl_sync(0xffffffffu, n, who);
-                q0 = (__shfl_sync(0xffffffffu, upto, who) - 1 - want) * prm.rows_per_cta;
+                q0 = (__shfl_sync(0xffffffffu, upto, who) - 1 - want) * BM;
                 break;
             }
             want -= __shfl_sync(0xffffffffu, upto, 31);
@@ -154,7 +121,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
     if (seq < 0) return;
     const int ctx = a.ctx_start[seq], row0 = a.cu_q[seq] + q0;
     if (ctx < 0) {                                                   // padding: zero rows (the paged form's are another kernel's)
-        const int rows = GATHERED ? min(len - q0, prm.rows_per_cta) : 0, v8 = a.dv / 8;
+        const int rows = GATHERED ? min(len - q0, BM) : 0, v8 = a.dv / 8;
         for (int idx = tid; idx < rows * v8; idx += NTHREADS)
             *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + (size_t)(row0 + idx / v8) * a.out_stride + (size_t)group * a.dv + (idx % v8) * 8) =
                 make_uint4(0, 0, 0, 0);
@@ -166,8 +133,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
         Plan& pl = s_plan;
         pl.rows[0] = pl.rows[1] = pl.t0[0] = pl.t0[1] = pl.t1[0] = pl.t1[1] = 0;
         {
-            const int left = len - q0, p0 = ctx + q0, p_last = p0 + min(left, prm.rows_per_cta) - 1;
-            const bool two = prm.rows_per_cta > BM;
+            const int left = len - q0, p0 = ctx + q0, p_last = p0 + min(left, BM) - 1;
             KeySpan span = key_span(p0, p_last, a.chunk, a.window, a.keep_first);
             if (GATHERED && span.wlo < a.k_lo[seq]) {                // the gathered rows begin at k_lo
                 span.wlo = span.lo = a.k_lo[seq];
@@ -176,11 +142,11 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             pl.span = span;
             pl.keep = a.window > 0 ? span.index(a.keep_first) : 0;
             pl.rows[0] = min(BM, left);
-            pl.rows[1] = two ? min(BM, max(0, left - BM)) : (TWO_MAPS || prm.heads_per_cta == 2) ? pl.rows[0] : 0;
+            pl.rows[1] = TWO_MAPS ? pl.rows[0] : 0;
 #pragma unroll 1
             for (int x = 0; x < 2; ++x) {
                 if (pl.rows[x] == 0) continue;
-                const int pf = p0 + (two && x ? BM : 0);
+                const int pf = p0;
                 const RowRange f = range_of(span, pf, a.chunk, a.window), l = range_of(span, pf + pl.rows[x] - 1, a.chunk, a.window);
                 pl.first_row[x] = pf;
                 pl.t0[x] = (f.block < pl.keep ? f.block : f.low) / BN;
@@ -209,10 +175,8 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    const int hpc = prm.heads_per_cta;
-    const bool two_rows = prm.rows_per_cta > BM;
-    const int n_tiles = max(s_plan.t1[0], s_plan.t1[1]), n_keys = s_plan.span.n;
-    const int kvh = (group * hpc) / (a.H / a.G);                // kv head of the paged pools
+        const int n_tiles = max(s_plan.t1[0], s_plan.t1[1]), n_keys = s_plan.span.n;
+    const int kvh = group / (a.H / a.G);                // kv head of the paged pools
 
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
@@ -252,8 +216,8 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             {                                                        // Q, by all three warps: rows past the tile are zeros
 #pragma unroll 1
                 for (int x = 0; x < 2; ++x) {
-                    const int hh = group * hpc + (hpc == 2 ? x : 0), nrows = s_plan.rows[x];
-                    const int rbase = row0 + (two_rows && x ? BM : 0);
+                    const int hh = group, nrows = s_plan.rows[x];
+                    const int rbase = row0;
                     if (nrows == 0) continue;
                     const int col0 = TWO_MAPS ? x * a.dk : 0;
                     const char* qh = reinterpret_cast<const char*>(static_cast<const bf16*>(a.q0) + (size_t)rbase * a.q0_row + (size_t)hh * a.q0_head + col0 + c8 * 8);
@@ -420,7 +384,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             const int row = wq * 32 + lane;                          // query row of the slot = TMEM lane
             const uint32_t lane_off = (uint32_t)(wq * 32) << 16;
             const uint32_t s_addr = tmem + lane_off + x * 128, o_addr = tmem + lane_off + 256 + x * 128;
-            const int hh = group * hpc + (hpc == 2 ? x : 0);
+            const int hh = group;
             const RowRange mine = range_of(s_plan.span, s_plan.first_row[x] + min(row, nrows - 1), a.chunk, a.window);
             const int all_hi = s_plan.all_hi[x], all_low = s_plan.all_low[x], keep = s_plan.keep;
             const float sl2 = prm.scale_log2;
@@ -550,7 +514,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             // ------------------------------------------ output rows
             const int n = te - tb;
             const bool valid = row < nrows;
-            const size_t brow = (size_t)row0 + (two_rows && x ? BM : 0) + row;
+            const size_t brow = (size_t)row0 + row;
             wait(bar(L::BAR_PV + x), (n - 1) & 1, failed);
             float inv = KIND == KIND_SIGMOID ? 1.f : (l > 0.f ? 1.f / l : 0.f);
             if (*failed) inv = __int_as_float(0x7fc00000);           // behind the last wait, which may be the one that gave up
@@ -661,7 +625,12 @@ bool b2_internal_prompt_tc5_ok(const b2_prompt_args& a) {
 }
 
 int b2_internal_prompt_tc5(const b2_prompt_args& a, void* stream) {
-    const int n_sm = b2_sm_count();
+    // A CTA a tile of one slot (two maps: two) up to one and a half waves; more tiles are taken in turns.  In a graph, this kernel / turns: 300 rows x
+    // 16 heads 15.0 / 15.4 us, 1000 x 16 22.2 / 23.6, 1200 gathered x 16 40.7 / 41.8, 1300 x 16 (176 tiles) 27.4 / 27.1, 4 x 146 x 32 (256) 26.6 / 25.2.
+    const int64_t longs = std::min(a.n_seq, a.T / a.min_rows);       // sequences of min_rows rows or more
+    const int64_t tiles = (int64_t)a.T / BM + longs, ctas = tiles * a.H;         // upper bound on sum(ceil(len / rows)); spare CTAs leave at once
+    if (tiles == 0) return B2_OK;
+    if (ctas > b2_sm_count() * 3 / 2) return b2_internal_prompt_turns(a, stream);
     Params p;
     p.a = a;
     p.scale_log2 = a.scale * LOG2E;
@@ -693,21 +662,6 @@ int b2_internal_prompt_tc5(const b2_prompt_args& a, void* stream) {
         }
         if (rc != B2_OK) return rc;
     }
-    // Two slots a CTA share the copies of a key tile and cover each other's softmax; a launch of fewer than one wave of such CTAs
-    // takes one slot each (twice the CTAs, each a little faster).  Two heads of a kv head before two row tiles: see above.
-    const int64_t longs = std::min(a.n_seq, a.T / a.min_rows);       // sequences of min_rows rows or more
-    const int64_t tiles128 = (int64_t)a.T / BM + longs, tiles256 = (int64_t)a.T / (2 * BM) + longs;
-    p.rows_per_cta = BM;
-    p.heads_per_cta = 1;
-    if (a.maps == 1) {
-        const bool pair = !gathered && (a.H / a.G) % 2 == 0;
-        if (pair && tiles128 * (a.H / 2) >= n_sm) p.heads_per_cta = 2;
-        else if (!pair && tiles256 * a.H >= n_sm) p.rows_per_cta = 2 * BM;
-    }
-    const int64_t tiles = p.rows_per_cta == BM ? tiles128 : tiles256;        // upper bound on sum(ceil(len / rows)); spare CTAs leave at once
-    if (tiles == 0) return B2_OK;
-    const int64_t ctas = tiles * (a.H / p.heads_per_cta);
-    B2_REQUIRE(ctas <= 0x7fffffff, B2_EUNSUPPORTED, "prompt attention: %lld row tiles exceed the grid", (long long)tiles);
     const dim3 grid((unsigned)ctas);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nh = (a.dk + 63) / 64, dvh = (a.dv + 63) / 64;
