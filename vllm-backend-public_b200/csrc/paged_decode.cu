@@ -1533,8 +1533,8 @@ size_t workspace_bound(int B, int Hq, int Hkv, int bs, int max_nb, int num_split
 
 // NSTAGE / NSTAGE_D: ring depth of the grid-split / dynamic kernel.  bf16: 3 x 32 KiB, two CTAs per SM.
 // fp8 (16 KiB stages): 4 / 3 stages with three CTAs per SM (default), or 6 / 5 with two.
-// zero_first: launch the tiny kernel that zeroes the claim counter (stateless API); a b2_decode_plan zeroes it once
-// at creation and every merge kernel leaves it at zero, so its calls are two launches.
+// zero_first: launch the tiny kernel that zeroes the claim counter (stateless API without a KV write in front, which would do it); a
+// b2_decode_plan zeroes it once at creation and every merge kernel leaves it at zero, so its calls are two launches.
 template <int BS, bool FP8, int NT, int NSTAGE, int NSTAGE_D>
 int launch_decode(const CUtensorMap& tmK, const CUtensorMap& tmV, const DecodeParams& p, const Plan& pl,
                   bool zero_first, cudaStream_t st) {
@@ -1746,15 +1746,13 @@ int run_decode(const DecodeGeom& g, const CacheMaps& maps, const Knobs& kn, bool
     }
     if (ap && !p.append) {
         // a schedule that cuts rows over several CTAs: the KV write goes in front of the grid (after every argument
-        // check above, so a refused call has written nothing)
-        const int rc = ap->bt_update
-            ? b2_reshape_and_cache_decode(ap->k_new, ap->v_new, ap->k_cache, ap->v_cache, ap->slot_mapping,
-                                          ap->bt_update, seq_lens, B, g.Hkv, D, g.bs, g.max_nb, ap->k_token_stride,
-                                          ap->v_token_stride, ap->cache_block_stride, ap->cache_head_stride,
-                                          g.kv_dtype, g.k_scale, g.v_scale, st)
-            : b2_reshape_and_cache(ap->k_new, ap->v_new, ap->k_cache, ap->v_cache, ap->slot_mapping, B, g.Hkv, D,
-                                   g.bs, ap->k_token_stride, ap->v_token_stride, ap->cache_block_stride,
-                                   ap->cache_head_stride, g.kv_dtype, g.k_scale, g.v_scale, st);
+        // check above, so a refused call has written nothing), and takes the zeroing of the claim counter along
+        const bool zeroes = zero_first && pl.num_splits == 0;
+        const int rc = b2_internal_write_kv(ap->k_new, ap->v_new, ap->k_cache, ap->v_cache, ap->slot_mapping, ap->bt_update,
+                                            ap->bt_update ? seq_lens : nullptr, B, g.Hkv, D, g.bs, ap->bt_update ? g.max_nb : 0, ap->k_token_stride,
+                                            ap->v_token_stride, ap->cache_block_stride, ap->cache_head_stride, g.kv_dtype,
+                                            g.k_scale, g.v_scale, zeroes ? p.counter : nullptr, st);
+        if (zeroes) zero_first = false;
         if (rc != B2_OK) return rc;
     }
     if (g.bs == 8) return dispatch_decode<8>(maps.k, maps.v, p, pl, fp8, kn.fp8_ctas, zero_first, st);

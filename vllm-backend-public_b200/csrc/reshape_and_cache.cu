@@ -23,11 +23,13 @@ reshape_and_cache_kernel(const __nv_bfloat16* __restrict__ k_new,
                          int64_t k_token_stride, int64_t v_token_stride,
                          int64_t cache_block_stride, int64_t cache_head_stride,
                          const float* __restrict__ k_scale, const float* __restrict__ v_scale,
-                         int32_t* __restrict__ block_tables, const int32_t* __restrict__ seq_lens, int max_nb) {
+                         int32_t* __restrict__ block_tables, const int32_t* __restrict__ seq_lens, int max_nb,
+                         uint32_t* __restrict__ counter) {
     // the decode kernel that follows in the stream may be launched now (programmatic dependent launch): its prologue
     // runs under this kernel; it waits (griddepcontrol.wait) before it touches the cache or the block tables
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int t = blockIdx.x;
+    if (counter && t == 0 && threadIdx.x == 0) *counter = 0u;        // the claim counter of the decode grid behind this kernel
     const int64_t slot = slot_mapping[t];
     if (slot < 0) return;  // padding token
     const int64_t blk = slot / bs;
@@ -104,7 +106,7 @@ int reshape_and_cache_impl(const void* k_new, const void* v_new, void* k_cache,
                            int d, int bs, int64_t k_token_stride, int64_t v_token_stride,
                            int64_t cache_block_stride, int64_t cache_head_stride,
                            int kv_dtype, const float* k_scale, const float* v_scale,
-                           int32_t* block_tables, const int32_t* seq_lens, int max_nb, void* stream) {
+                           int32_t* block_tables, const int32_t* seq_lens, int max_nb, uint32_t* counter, void* stream) {
     B2_REQUIRE(T >= 0 && Hkv > 0 && d > 0 && bs > 0, B2_EINVAL,
                "reshape_and_cache: bad sizes T=%d Hkv=%d d=%d bs=%d", T, Hkv, d, bs);
     if (T == 0) return B2_OK;
@@ -133,11 +135,11 @@ int reshape_and_cache_impl(const void* k_new, const void* v_new, void* k_cache,
     if (kv_dtype == B2_KV_BF16) {
         reshape_and_cache_kernel<false><<<T, threads, 0, st>>>(
             kn, vn, k_cache, v_cache, slot_mapping, Hkv, d, bs, k_token_stride, v_token_stride,
-            cache_block_stride, cache_head_stride, nullptr, nullptr, block_tables, seq_lens, max_nb);
+            cache_block_stride, cache_head_stride, nullptr, nullptr, block_tables, seq_lens, max_nb, counter);
     } else {
         reshape_and_cache_kernel<true><<<T, threads, 0, st>>>(
             kn, vn, k_cache, v_cache, slot_mapping, Hkv, d, bs, k_token_stride, v_token_stride,
-            cache_block_stride, cache_head_stride, k_scale, v_scale, block_tables, seq_lens, max_nb);
+            cache_block_stride, cache_head_stride, k_scale, v_scale, block_tables, seq_lens, max_nb, counter);
     }
     B2_CUDA_OK(cudaGetLastError());
     return B2_OK;
@@ -153,7 +155,15 @@ extern "C" int b2_reshape_and_cache(const void* k_new, const void* v_new, void* 
                                     void* stream) {
     return reshape_and_cache_impl(k_new, v_new, k_cache, v_cache, slot_mapping, T, Hkv, d, bs, k_token_stride,
                                   v_token_stride, cache_block_stride, cache_head_stride, kv_dtype, k_scale, v_scale,
-                                  nullptr, nullptr, 0, stream);
+                                  nullptr, nullptr, 0, nullptr, stream);
+}
+
+int b2_internal_write_kv(const void* k_new, const void* v_new, void* k_cache, void* v_cache, const int64_t* slot_mapping, int32_t* block_tables,
+                         const int32_t* seq_lens, int B, int Hkv, int d, int bs, int max_nb, int64_t k_token_stride, int64_t v_token_stride,
+                         int64_t cache_block_stride, int64_t cache_head_stride, int kv_dtype, const float* k_scale, const float* v_scale,
+                         uint32_t* counter, void* stream) {
+    return reshape_and_cache_impl(k_new, v_new, k_cache, v_cache, slot_mapping, B, Hkv, d, bs, k_token_stride, v_token_stride, cache_block_stride,
+                                  cache_head_stride, kv_dtype, k_scale, v_scale, block_tables, seq_lens, max_nb, counter, stream);
 }
 
 extern "C" int b2_reshape_and_cache_decode(const void* k_new, const void* v_new, void* k_cache, void* v_cache,
@@ -165,7 +175,7 @@ extern "C" int b2_reshape_and_cache_decode(const void* k_new, const void* v_new,
                "reshape_and_cache_decode: block_tables / seq_lens / max_nb");
     return reshape_and_cache_impl(k_new, v_new, k_cache, v_cache, slot_mapping, B, Hkv, d, bs, k_token_stride,
                                   v_token_stride, cache_block_stride, cache_head_stride, kv_dtype, k_scale, v_scale,
-                                  block_tables, seq_lens, max_nb, stream);
+                                  block_tables, seq_lens, max_nb, nullptr, stream);
 }
 
 extern "C" int b2_dequant_kv_blocks(void* k_out, void* v_out, const void* k_cache, const void* v_cache,
