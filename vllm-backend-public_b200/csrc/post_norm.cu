@@ -323,6 +323,28 @@ __global__ void relu_sq_kernel(T* __restrict__ out, int64_t out_stride, const T*
     }
 }
 
+// bf16 rows that lie on 16 bytes: two vectors of eight a thread, both on their way before the first is used.  4096 x 4096: 15.4 us with four entries
+// an access, 9.8 with this (under ncu; 67 MB).  in and out may be the same: a thread writes what it has read.
+__global__ void __launch_bounds__(256)
+relu_sq_rows_kernel(__nv_bfloat16* out, int64_t out_stride, const __nv_bfloat16* in, int64_t in_stride, int vecs) {
+    const uint4* src = reinterpret_cast<const uint4*>(in + (size_t)blockIdx.x * in_stride);
+    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * out_stride);
+    auto square = [](uint4 r) {
+        uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float a = fmaxf(__uint_as_float(w[c] << 16), 0.f), b = fmaxf(__uint_as_float(w[c] & 0xffff0000u), 0.f);
+            w[c] = b2::pack_bf16x2(a * a, b * b);
+        }
+        return make_uint4(w[0], w[1], w[2], w[3]);
+    };
+    for (int i = blockIdx.y * 512 + threadIdx.x; i < vecs; i += gridDim.y * 512) {
+        const uint4 a = src[i], b = i + 256 < vecs ? src[i + 256] : make_uint4(0, 0, 0, 0);
+        dst[i] = square(a);
+        if (i + 256 < vecs) dst[i + 256] = square(b);
+    }
+}
+
 template <typename T, int W>
 __global__ void glu_and_mul_kernel(T* __restrict__ out, int64_t out_stride, const T* __restrict__ in, int64_t in_stride, int I,
                                    int glu, float alpha, float limit) {
@@ -516,6 +538,12 @@ extern "C" int b2_relu_sq(void* out, int64_t out_stride, const void* in, int64_t
     B2_REQUIRE(out && in, B2_EINVAL, "relu_sq: null pointer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool vec = I % 4 == 0 && in_stride % 4 == 0 && out_stride % 4 == 0 && b2_aligned16(in) && b2_aligned16(out);
+    if (act_dtype == B2_ACT_BF16 && vec && I % 8 == 0 && in_stride % 8 == 0 && out_stride % 8 == 0) {
+        relu_sq_rows_kernel<<<rows_grid((I / 8 + 1) / 2, T), 256, 0, st>>>(static_cast<__nv_bfloat16*>(out), out_stride, static_cast<const __nv_bfloat16*>(in),
+                                                                 in_stride, I / 8);
+        B2_CUDA_OK(cudaGetLastError());
+        return B2_OK;
+    }
     B2_DISPATCH_ACT(act_dtype, A, {
         A* o = static_cast<A*>(out);
         const A* i = static_cast<const A*>(in);
