@@ -566,24 +566,40 @@ __global__ void moe_gather_kernel(const T* __restrict__ h, int64_t h_stride, con
     }
 }
 
+// A row's columns over blockIdx.y, the rows of four choices on their way at once; the sum runs over the choices in their order.  64 rows of 8 choices of
+// 4096 columns: 10.7 us with a CTA a row and one choice behind the other, 5.9 (under ncu; 8.9 MB).
 template <typename T, typename R, int W>
-__global__ void moe_combine_kernel(const R* __restrict__ rows, const int32_t* __restrict__ place,
-                                   const float* __restrict__ wts, int top, int D, const T* __restrict__ add, int64_t add_stride,
-                                   T* __restrict__ y, int64_t y_stride) {
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(const R* __restrict__ rows, const int32_t* __restrict__ place, const float* __restrict__ wts, int top, int D,
+                   const T* __restrict__ add, int64_t add_stride, T* __restrict__ y, int64_t y_stride) {
+    constexpr int AHEAD = 4;
     const int t = blockIdx.x;
-    for (int d = threadIdx.x * W; d < D; d += blockDim.x * W) {
+    for (int d = (blockIdx.y * 256 + threadIdx.x) * W; d < D; d += gridDim.y * 256 * W) {
         float a[4] = {0.f, 0.f, 0.f, 0.f};
         if (add) {
             if (W == 4) b2::ld4(add + (size_t)t * add_stride + d, a); else a[0] = b2::ld(add + (size_t)t * add_stride + d);
         }
-        for (int j = 0; j < top; ++j) {
-            const int p = place[(size_t)t * top + j];
-            if (p < 0) continue;
-            const float wt = wts ? wts[(size_t)t * top + j] : 1.f;
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-            if (W == 4) b2::ld4(rows + (size_t)p * D + d, v); else v[0] = b2::ld(rows + (size_t)p * D + d);
+        for (int j0 = 0; j0 < top; j0 += AHEAD) {
+            int p[AHEAD];
+            float wt[AHEAD], v[AHEAD][4];
 #pragma unroll
-            for (int c = 0; c < W; ++c) a[c] = fmaf(wt, v[c], a[c]);
+            for (int u = 0; u < AHEAD; ++u) {
+                p[u] = j0 + u < top ? place[(size_t)t * top + j0 + u] : -1;
+                wt[u] = wts && j0 + u < top ? wts[(size_t)t * top + j0 + u] : 1.f;
+            }
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                v[u][0] = v[u][1] = v[u][2] = v[u][3] = 0.f;
+                if (p[u] >= 0) {
+                    if (W == 4) b2::ld4(rows + (size_t)p[u] * D + d, v[u]); else v[u][0] = b2::ld(rows + (size_t)p[u] * D + d);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                if (p[u] < 0) continue;
+#pragma unroll
+                for (int c = 0; c < W; ++c) a[c] = fmaf(wt[u], v[u][c], a[c]);
+            }
         }
         if (W == 4) b2::st4(y + (size_t)t * y_stride + d, a); else b2::st(y + (size_t)t * y_stride + d, a[0]);
     }
@@ -595,10 +611,10 @@ int launch_combine(const void* rows, const int32_t* place, const float* wts, int
     const bool vec = D % 4 == 0 && y_stride % 4 == 0 && b2_aligned16(rows) && b2_aligned16(y) &&
                      (!add || (add_stride % 4 == 0 && b2_aligned16(add)));
     if (vec)
-        moe_combine_kernel<T, R, 4><<<rows_n, 256, 0, st>>>(static_cast<const R*>(rows), place, wts, top, D, static_cast<const T*>(add),
+        moe_combine_kernel<T, R, 4><<<dim3(rows_n, (D / 4 + 255) / 256 < 64 ? (D / 4 + 255) / 256 : 64), 256, 0, st>>>(static_cast<const R*>(rows), place, wts, top, D, static_cast<const T*>(add),
                                                            add_stride, static_cast<T*>(y), y_stride);
     else
-        moe_combine_kernel<T, R, 1><<<rows_n, 256, 0, st>>>(static_cast<const R*>(rows), place, wts, top, D, static_cast<const T*>(add),
+        moe_combine_kernel<T, R, 1><<<dim3(rows_n, (D + 255) / 256 < 64 ? (D + 255) / 256 : 64), 256, 0, st>>>(static_cast<const R*>(rows), place, wts, top, D, static_cast<const T*>(add),
                                                            add_stride, static_cast<T*>(y), y_stride);
     B2_CUDA_OK(cudaGetLastError());
     return B2_OK;
