@@ -13,7 +13,7 @@
 // stay infinities.
 //
 // 4096 tokens, 16 heads of 128 x 128 in a graph: 124 us (with the products on the FMA pipe 243, token by token 804); 500 tokens 35 (41, 102).  Under
-// ncu, cold: kv 35, state 22, out 75.
+// ncu, cold: kv 35, state 20, out 75.
 // out_kernel's item takes 30e3 cycles, of which the MMAs are 9e3: splitting into parts, the copies of S_0 (20 bytes a cycle and SM when all
 // ask at once) and the read-back follow one another in the one CTA that an SM's shared memory holds.  Two CTAs of 64 tokens an SM took 89 us
 // instead of the 72 that this one took then (twice the instructions), a warp of its own for the MMAs 78 - 90 (the registers it costs the others spill).
@@ -227,7 +227,8 @@ state_kernel(const Args a) {
     const bool pad = row >= dk;
     const float* from = pad ? nullptr : state_from(a, part, a.state_slot[seq], hh, a.ctx_start[seq]);
     float4 s = from ? *reinterpret_cast<const float4*>(from + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-    constexpr int AHEAD = 8;                         // loads in flight: they do not depend on the chain
+    constexpr int AHEAD = 16;                        // loads in flight: they do not depend on the chain (4096 tokens x 16 heads, 84 MB: eight 22 us, sixteen
+                                                     // 19.6 under ncu; more would leave registers for fewer than the four CTAs an SM)
     float4 x[AHEAD];
     float d[AHEAD];
 #pragma unroll

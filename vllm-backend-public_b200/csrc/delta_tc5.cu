@@ -591,7 +591,7 @@ state_kernel(const Args a) {
                         tile_at(row & 63, (col & 63) >> 3, 64) + (col & 4) * 2;
     const float* from = pad ? nullptr : state_from(a, part, a.state_slot[seq], hh, a.ctx_start[seq]);
     float4 s = from ? *reinterpret_cast<const float4*>(from + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-    constexpr int AHEAD = 8;                         // loads in flight: they do not depend on the chain
+    constexpr int AHEAD = 16;                        // loads in flight: they do not depend on the chain (as in chunk_tc5.cu)
     float4 x[AHEAD];
     float d[AHEAD];
 #pragma unroll
