@@ -494,7 +494,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                 const bool boxes_of_all = prm.tma && (!GATHERED || a.k_rows > 0);
                 uint32_t rows[4];
                 auto lookup = [&](int it) {
-                    if (!GATHERED && prm.tma) {                      // rows[0], rows[1]: this lane's box, or its first two: page, row in it
+                    if (!GATHERED && prm.tma) {                      // rows[0], rows[1]: page of this lane's box, row in it
                         const int c = it * BN + ((lane % (BN >> box_shift)) << box_shift);
                         rows[0] = NONE;
                         if (c < n_keys) {
