@@ -411,6 +411,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                 }
                 tiles = max(tiles, __shfl_sync(0xffffffffu, tiles, 1));
                 if (t == 0) meet();
+                __syncwarp();                                        // lane 0's word covers what lane 1 wrote: a shuffle orders no memory
                 if (lane == 0) {
                     pl.n_tiles = tiles;
                     b2::mbar_arrive(bar(L::BAR_PLAN + (t & 1)));
