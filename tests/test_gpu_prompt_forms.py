@@ -1,0 +1,18 @@
+"""The forms that prompt rows go through by what the host knows of their batch -- a tile of one slot a CTA, two heads of a kv head or two row tiles a
+CTA, CTAs that take tiles in turns -- on both sides of each rule.  Oracle and tolerance are those of test_gpu_prompt_tc5."""
+import pytest
+
+from test_gpu_prompt_tc5 import test_gathered_prompt_rows as gathered_rows, test_masked_prompt_rows as masked_rows
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("c", [
+    # lens, ctx, heads, kv heads, dk, dv, page, chunk, window, keep, cap, sink, maps, sigmoid, gate, scale factor
+    # most sequences are decode rows: counted as more tiles than there are, which turn out to be one wave
+    ([1] * 40 + [200, 130], [60] * 40 + [0, 77], 32, 8, 64, 64, 16, 0, 100, 3, 0.0, True, 1, False, True, 1.0),
+    ([1] * 40 + [300, 16], [60] * 41 + [5], 28, 4, 64, 64, 16, 0, 0, 0, 0.0, False, 1, False, True, 1.0),
+    ([1] * 33 + [250], [60] * 33 + [9], 16, 2, 128, 64, 16, 128, 0, 0, 0.0, False, 1, True, False, 1.0),
+])
+def test_forms(cuda, c):
+    masked_rows(cuda, c)

@@ -124,7 +124,7 @@ struct Plan {
     int t0[2], t1[2];                                // a slot works on the key tiles t0 .. t1 - 1
     int all_hi[2], all_low[2];                       // keys all_low .. all_hi are visible to every row of the slot
     int n_tiles;                                     // key tiles of the slots together; 0: no more tiles for this CTA
-    int seq, row0, group;                            // row0: first row in q and out
+    int seq, row0, head;                             // row0: first row in q and out; head: slot 0's
 };
 
 // The order of the tiles: by the number of key tiles they walk, most first, so that the CTAs, which take tiles in boustrophedon
@@ -162,21 +162,18 @@ struct TileOrder {
     __device__ __forceinline__ int total(int L) const {
         return __reduce_add_sync(0xffffffffu, ((mine.len + (1 << shift) - 1) >> shift) - first_at(L, mine));
     }
-    __device__ __forceinline__ void init(const b2_prompt_args& args, int rows_per_cta, int groups, int ln) {
+    // rows, heads: of a tile; both become those of one slot where the batch turns out to hold no more tiles of one slot than there are CTAs
+    __device__ __forceinline__ void init(const b2_prompt_args& args, int& rows, int& heads, int ln) {
         a = &args;
         lane = ln;
-        shift = rows_per_cta == BM ? 7 : 8;
-        cap = 0x7fffff;
-        if (a->window > 0) cap = min(cap, (a->window + rows_per_cta) / BN + 1);
-        if (a->chunk > 0) cap = min(cap, a->chunk / BN + 2);
         n_long = 0;
         mine = {0, 0, 0, 0};
-        max_level = 1;
+        int level = 1;
 #pragma unroll 1
         for (int s0 = 0; s0 < a->n_seq && n_long <= 32; s0 += 32) {
             const Prompt p = read(s0 + lane);
             uint32_t longs = __ballot_sync(0xffffffffu, p.len > 0);
-            if (p.len > 0) max_level = max(max_level, min(cap, (max(p.ctx, 0) + p.len + BN - 1) / BN));
+            if (p.len > 0) level = max(level, (max(p.ctx, 0) + p.len + BN - 1) / BN);
             if (a->n_seq <= 32) {
                 mine = p;
                 break;
@@ -190,10 +187,18 @@ struct TileOrder {
                 ++n_long;                            // 33: more than the lanes hold
             }
         }
-        max_level = __reduce_max_sync(0xffffffffu, max_level);
+        if (n_long <= 32 && __reduce_add_sync(0xffffffffu, (mine.len + BM - 1) / BM) * a->H <= (int)gridDim.x) {
+            rows = BM;
+            heads = 1;
+        }
+        shift = rows == BM ? 7 : 8;
+        cap = 0x7fffff;
+        if (a->window > 0) cap = min(cap, (a->window + rows) / BN + 1);
+        if (a->chunk > 0) cap = min(cap, a->chunk / BN + 2);
+        max_level = min(cap, (int)__reduce_max_sync(0xffffffffu, level));
         from = before = 0;
         if (n_long > 32) cap = max_level = 1;        // one level: in the order of the batch
-        else if (total(1) * groups <= (int)gridDim.x) cap = max_level = 1;       // a tile a CTA in any order
+        else if (total(1) * (a->H / heads) <= (int)gridDim.x) cap = max_level = 1;       // a tile a CTA in any order
     }
     // row tile of rank r: its prompt and first row in it (false: there are no more)
     __device__ __forceinline__ bool find(int r, Prompt& at, int& q0) {
@@ -314,8 +319,6 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(b2::smem_u32(&s_tmem)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    const int hpc = prm.heads_per_cta;
-    const uint32_t groups = (uint32_t)(a.H / hpc);
     TileOrder order;
     // The plan warp comes to this barrier with its first plan in hand, made while the others set up what it does not need.
     auto meet = [] { asm volatile("bar.sync 2, 512;" ::: "memory"); };
@@ -326,7 +329,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
         tc_fence_after();
     }
     const uint32_t tmem = warp != W_PLAN ? s_tmem : 0u;
-    const bool two_rows = prm.rows_per_cta > BM;
+    const bool two_rows = prm.rows_per_cta > BM, two_heads = prm.heads_per_cta == 2;     // slot 1's rows or head, where it is not empty
     // the plan of tile t: its place, which stays the tile's until every warp has said that it is done with it
     auto plan_of = [&](int t) -> const Plan* {
         const bool ok = wait(bar(L::BAR_PLAN + (t & 1)), (t >> 1) & 1, failed);
@@ -348,28 +351,30 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                 if (!GATHERED || a.dk0 > 0) b2::tma_prefetch_desc(&prm.map_q0);
                 if (GATHERED && a.dk0 < a.dk) b2::tma_prefetch_desc(&prm.map_q1);
             }
-            order.init(a, prm.rows_per_cta, (int)groups, lane);
+            int tile_rows = prm.rows_per_cta, hpc = prm.heads_per_cta;
+            order.init(a, tile_rows, hpc, lane);
+            const uint32_t groups = (uint32_t)(a.H / hpc);
             int t = 0, q_0 = 0, q_1 = 0;                             // tiles published, Q tiles of the slots
 #pragma unroll 1
             for (uint32_t turn = 0;; ++turn) {
                 const uint32_t rank = tile_rank(turn);
-                const int group = (int)(rank % groups);
+                const int head = (int)(rank % groups) * hpc;
                 Prompt at = {0, 0, 0, 0};
                 int q0 = 0;
                 const bool more = order.find((int)(rank / groups), at, q0);
                 const int seq = at.seq, len = at.len, ctx = at.ctx, row0 = at.row + q0;
                 if (more && ctx < 0) {                               // padding: zero rows (the paged form's are another kernel's)
-                    const int rows = GATHERED ? min(len - q0, prm.rows_per_cta) : 0, v8 = a.dv / 8;
+                    const int rows = GATHERED ? min(len - q0, tile_rows) : 0, v8 = a.dv / 8;
 #pragma unroll 1
                     for (int idx = lane; idx < rows * v8; idx += 32)
-                        *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + (size_t)(row0 + idx / v8) * a.out_stride + (size_t)group * a.dv + (idx % v8) * 8) =
+                        *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + (size_t)(row0 + idx / v8) * a.out_stride + (size_t)head * a.dv + (idx % v8) * 8) =
                             make_uint4(0, 0, 0, 0);
                     continue;
                 }
-                const int nrows0 = min(BM, len - q0), nrows1 = two_rows ? min(BM, max(0, len - q0 - BM)) : (TWO_MAPS || hpc == 2) ? nrows0 : 0;
+                const int nrows0 = min(BM, len - q0), nrows1 = tile_rows > BM ? min(BM, max(0, len - q0 - BM)) : (TWO_MAPS || hpc == 2) ? nrows0 : 0;
                 auto q_boxes = [&](int x) {                          // rows behind the tile are the next ones' (zeros behind the last): their results go nowhere
                     if (lane == 0) {
-                        const int hh = group * hpc + (hpc == 2 ? x : 0), rb = row0 + (two_rows && x ? BM : 0);
+                        const int hh = head + (two_heads ? x : 0), rb = row0 + (two_rows && x ? BM : 0);
                         b2::mbar_arrive_expect_tx(bar(L::BAR_Q + x), NH * SUB);
 #pragma unroll 1
                         for (int h = 0; h < NH; ++h) {
@@ -385,7 +390,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                 int tiles = 0;
                 if (lane < 2 && more) {                              // a lane a slot
                     const int x = lane, rows = x ? nrows1 : nrows0;
-                    const int p0 = ctx + q0, p_last = p0 + min(len - q0, prm.rows_per_cta) - 1;
+                    const int p0 = ctx + q0, p_last = p0 + min(len - q0, tile_rows) - 1;
                     KeySpan keys = key_span(p0, p_last, a.chunk, a.window, a.keep_first);
                     if (GATHERED && keys.wlo < a.k_lo[seq]) keys.wlo = keys.lo = a.k_lo[seq];     // the gathered rows begin at k_lo
                     const TileSpan span = tile_span(keys, p_last, prm.align);
@@ -406,7 +411,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                         pl.keep = kept;
                         pl.seq = seq;
                         pl.row0 = row0;
-                        pl.group = group;
+                        pl.head = head;
                     }
                 }
                 tiles = max(tiles, __shfl_sync(0xffffffffu, tiles, 1));
@@ -430,7 +435,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                         continue;
                     }
                     {                                                // rows past the tile are zeros
-                        const int hh = group * hpc + (hpc == 2 ? x : 0), nrows = x ? nrows1 : nrows0;
+                        const int hh = head + (two_heads ? x : 0), nrows = x ? nrows1 : nrows0;
                         const int rbase = row0 + (two_rows && x ? BM : 0);
                         const int col0 = TWO_MAPS ? x * a.dk : 0;
                         const char* qh = reinterpret_cast<const char*>(static_cast<const bf16*>(a.q0) + (size_t)rbase * a.q0_row + (size_t)hh * a.q0_head + col0 + c8 * 8);
@@ -484,13 +489,13 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                 const Plan* pl = plan_of(t);
                 if (!pl) break;
                 const TileSpan span = pl->span;
-                const int n_tiles = pl->n_tiles, n_keys = span.n, seq = pl->seq, group = pl->group;
+                const int n_tiles = pl->n_tiles, n_keys = span.n, seq = pl->seq, head = pl->head;
                 plan_done(t);
-                const int kvh = (group * hpc) / (a.H / a.G);         // kv head of the paged pools
+                const int kvh = head / (a.H / a.G);                  // kv head of the paged pools
                 const int32_t* bt = GATHERED ? nullptr : a.block_tables + (int64_t)seq * a.max_nb;
                 const uint32_t g0 = GATHERED ? (uint32_t)a.cu_k[seq] - (uint32_t)a.k_lo[seq] : 0u;
                 const uint32_t head0 = (uint32_t)(TWO_MAPS && !is_v ? 2 * kvh : kvh);
-                const char* p0 = reinterpret_cast<const char*>(static_cast<const bf16*>(is_v ? a.v : a.k0) + (GATHERED ? (size_t)group * split : 0) + c8 * 8);
+                const char* p0 = reinterpret_cast<const char*>(static_cast<const bf16*>(is_v ? a.v : a.k0) + (GATHERED ? (size_t)head * split : 0) + c8 * 8);
                 const char* p1g = GATHERED && !is_v ? p1 : p0;
                 const bool boxes_of_all = prm.tma && (!GATHERED || a.k_rows > 0);
                 uint32_t rows[4];
@@ -555,7 +560,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                             if (GATHERED) {
                                 const int row = (int)g0 + span.key(it * BN + r);
                                 if (!is_v && h * 64 >= split) tma_load_2d(dst, &prm.map_k1, full, h * 64 - split, row);
-                                else tma_load_3d(dst, is_v ? &prm.map_v : &prm.map_k0, full, h * 64, group, row);
+                                else tma_load_3d(dst, is_v ? &prm.map_v : &prm.map_k0, full, h * 64, head, row);
                             } else {
                                 const bool second = TWO_MAPS && !is_v;
                                 tma_load_4d(dst, is_v ? &prm.map_v : &prm.map_k0, full, second ? 0 : h * 64, (int)rows[1], (int)head0 + (second ? h : 0), (int)rows[0]);
@@ -744,7 +749,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
         for (int t = 0;; ++t) {
             const Plan* pl = plan_of(t);
             if (!pl) break;
-            const int n_tiles = pl->n_tiles, group = pl->group, row0 = pl->row0;
+            const int n_tiles = pl->n_tiles, head = pl->head, row0 = pl->row0;
             const int tb0 = pl->t0[0], tb1 = pl->t0[1], te0 = pl->t1[0], te1 = pl->t1[1], nrows0 = pl->rows[0], nrows1 = pl->rows[1];
             plan_done(t);
 #pragma unroll 1
@@ -796,7 +801,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                     wait(bar(L::BAR_PV + x), ((x ? steps1 : steps0) + i) & 1, failed);
                     __syncwarp();
                     tc_fence_after();
-                    const int hh = group * hpc + (hpc == 2 ? x : 0);
+                    const int hh = head + (two_heads ? x : 0);
                     const uint32_t out0 = TWO_MAPS ? tmem + lane_off + 256 : o_addr;
                     const int brow0 = row0 + (two_rows && x ? BM : 0) + wq * 32, left = (x ? nrows1 : nrows0) - wq * 32;      // the warp's rows
                     float f = s_inv[TWO_MAPS ? 0 : x][row], f2 = TWO_MAPS ? -a.map_lambda * s_inv[1][row] : 0.f;
@@ -892,13 +897,13 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
         for (int t = 0;; ++t) {
             const Plan* pl = plan_of(t);
             if (!pl) break;
-            const int tb = pl->t0[x], te = pl->t1[x], nrows = pl->rows[x], group = pl->group;
+            const int tb = pl->t0[x], te = pl->t1[x], nrows = pl->rows[x], head = pl->head;
             const int all_hi = pl->all_hi[x], all_low = pl->all_low[x], keep = pl->keep;
             RowRange mine = {0, 0, 0};
             if (te > tb) mine = range_of(pl->span, pl->first_row[x] + min(row, nrows - 1), a.chunk, a.window);
             plan_done(t);
             if (te <= tb) continue;
-            const int hh = group * hpc + (hpc == 2 ? x : 0);
+            const int hh = head + (two_heads ? x : 0);
             const float bias2 = KIND == KIND_SIGMOID && a.head_bias ? a.head_bias[hh] * LOG2E : 0.f;
             float m = a.sink > 0.f ? (a.sink_logits ? a.sink_logits[hh] : a.sink_logit) * LOG2E : -INFINITY, l = a.sink;
 #pragma unroll 1
@@ -1057,7 +1062,9 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     }
     if (*failed) {                                                   // a wait gave up: every row of this CTA's tiles is NaN
-        order.init(a, prm.rows_per_cta, (int)groups, lane);
+        int tile_rows = prm.rows_per_cta, hpc = prm.heads_per_cta;
+        order.init(a, tile_rows, hpc, lane);
+        const uint32_t groups = (uint32_t)(a.H / hpc);
 #pragma unroll 1
         for (uint32_t turn = 0;; ++turn) {
             const uint32_t rank = tile_rank(turn);
@@ -1065,7 +1072,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
             int q0 = 0;
             if (!order.find((int)(rank / groups), at, q0)) break;
             if (at.ctx < 0) continue;
-            const int rows = min(at.len - q0, prm.rows_per_cta), wide = hpc * a.dv;
+            const int rows = min(at.len - q0, tile_rows), wide = hpc * a.dv;
 #pragma unroll 1
             for (int idx = tid; idx < rows * wide; idx += NTHREADS)
                 static_cast<bf16*>(a.out)[(size_t)(at.row + q0 + idx / wide) * a.out_stride + (size_t)(rank % groups) * wide + idx % wide] =
@@ -1147,21 +1154,20 @@ int b2_internal_prompt_turns(const b2_prompt_args& a, void* stream) {
     }
     if (rc != B2_OK) return rc;
     // Two slots a CTA share the copies of a key tile and cover each other's softmax; row tiles, whose later one sees more keys, only where they
-    // fill the SMs (1200 gathered rows x 16 heads: 43.8 us in pairs, 41.8 one by one).  Two heads of a kv head before two row tiles: see above.
+    // fill the SMs (2000 gathered rows x 16 heads: 42.8 us in pairs, 38.1 one by one).  Two heads of a kv head before two row tiles: see above.
+    // These counts are bounds, far too large where most sequences are decode rows: TileOrder::init counts, and takes one slot a tile where
+    // that is all in one wave (64 decode rows and a prompt of 300, 16 heads of sigmoid weights: 67.3 us in pairs, 64.4 one by one).
     const int64_t longs = std::min(a.n_seq, a.T / a.min_rows);       // sequences of min_rows rows or more
     const int64_t tiles128 = (int64_t)a.T / BM + longs, tiles256 = (int64_t)a.T / (2 * BM) + longs;
     p.rows_per_cta = BM;
     p.heads_per_cta = 1;
     if (a.maps == 1) {
         const bool pair = !gathered && (a.H / a.G) % 2 == 0;
-        if (pair && tiles128 * a.H > n_sm) p.heads_per_cta = 2;
-        else if (!pair && tiles256 * a.H >= n_sm) p.rows_per_cta = 2 * BM;
+        if (pair) p.heads_per_cta = 2;
+        else if (tiles256 * a.H >= n_sm) p.rows_per_cta = 2 * BM;
     }
-    const int64_t tiles = p.rows_per_cta == BM ? tiles128 : tiles256;        // upper bound on sum(ceil(len / rows)); spare CTAs leave at once
-    if (tiles == 0) return B2_OK;
-    const int64_t ctas = tiles * (a.H / p.heads_per_cta);
-    B2_REQUIRE(ctas <= 0x7fffffff, B2_EUNSUPPORTED, "prompt attention: %lld row tiles exceed the grid", (long long)tiles);
-    const dim3 grid((unsigned)std::min<int64_t>(ctas, n_sm));
+    B2_REQUIRE(tiles128 * a.H <= 0x7fffffff, B2_EUNSUPPORTED, "prompt attention: %lld row tiles exceed the grid", (long long)tiles128);
+    const dim3 grid((unsigned)n_sm);                 // CTAs without a tile leave at once; a grid of fewer leaves the kernel behind it unevenly spread
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nh = (a.dk + 63) / 64, dvh = (a.dv + 63) / 64;
     const bool one_by_one = a.cap > 0.f || !(a.scale > 0.f);         // the capped form takes any score and any sign of the scale
