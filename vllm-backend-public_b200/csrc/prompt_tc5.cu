@@ -2,9 +2,10 @@
 // kv head) and of b2_window_attention (keys and values rebuilt per head in gathered buffers), with every option of those entry
 // points: sliding window with kept first tokens, mask blocks, sinks, capped scores, sigmoid weights, two maps per head, gates.
 //
-// A CTA takes one tile: 128 query rows of a head in one slot, or its two maps on the same rows in two (differential attention: slot x
-// multiplies the keys of map x).  Warps 0-3 / 4-7 are the softmax of slot 0 / 1 (a thread per row = TMEM lane), warp 9 issues the MMAs, warps
-// 8 and 11 copy K tiles, warp 10 V tiles (all three Q), 128 keys at a time.  Launches of more tiles are prompt_turns_tc5.cu's.
+// A CTA takes one tile: 128 query rows of a head in one slot, or two slots: two heads of a kv head on the same rows, two row tiles of a head, or
+// its two maps on the same rows (differential attention: slot x multiplies the keys of map x).  Warps 0-3 / 4-7 are the softmax of slot 0 / 1 (a
+// thread per row = TMEM lane), warp 9 issues the MMAs, warps 8 and 11 copy K tiles, warp 10 V tiles (all three Q), 128 keys at a time.  Launches
+// of more tiles are prompt_turns_tc5.cu's.
 // Keys are walked in the compact order of KeySpan (kept first keys, then the union of the rows' windows), so a window costs no
 // tiles between its parts and neither page size nor alignment shows: the copies are 16-byte cp.async gathers with a page lookup
 // per key row, written in the 128-byte swizzle that the MMA descriptors name (gathered rows: TMA boxes).  A mask is tested per
@@ -49,6 +50,7 @@ struct Shape {
 
 struct Params {
     b2_prompt_args a;
+    int rows_per_cta, heads_per_cta;
     int bs_shift;                                    // log2 of the page size, or -1
     float scale_log2;
     int tma;                                         // gathered form: whole key tiles come by TMA boxes of 128 rows x 64 columns
@@ -73,7 +75,7 @@ struct Plan {
     int all_hi[2], all_low[2];                       // keys all_low .. all_hi are visible to every row of the slot
 };
 
-template <int NH, int DVH, int KIND, bool TWO_MAPS, bool GATHERED>
+template <int NH, int DVH, int KIND, bool TWO_MAPS, bool GATHERED, bool PAIRS>
 __global__ void __launch_bounds__(NTHREADS, 1)
 prompt_tc5_kernel(const __grid_constant__ Params prm) {
     using L = Shape<NH, DVH, TWO_MAPS>;
@@ -93,14 +95,16 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
 
     // This CTA's tile: counted from the batch's last row backwards (late rows see more keys, and the spare CTAs of a grid that is an
     // upper bound come behind all tiles), by every warp for itself, 32 sequences at a time, so that a spare CTA leaves at once.
-    const int groups = a.H, group = blockIdx.x % groups;
+    const int hpc = PAIRS ? prm.heads_per_cta : 1, rows_per_cta = PAIRS ? prm.rows_per_cta : BM;
+    const bool two_rows = rows_per_cta > BM;
+    const int groups = a.H / hpc, group = blockIdx.x % groups;
     int seq = -1, q0 = 0, len = 0;
     {
         int want = blockIdx.x / groups;
 #pragma unroll 1
         for (int top = a.n_seq - 1; top >= 0; top -= 32) {
             const int s = top - lane, n = s >= 0 ? a.cu_q[s + 1] - a.cu_q[s] : 0;
-            const int nt = n >= a.min_rows ? (n + BM - 1) / BM : 0;
+            const int nt = n >= a.min_rows ? (n + rows_per_cta - 1) / rows_per_cta : 0;
             int upto = nt;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -112,7 +116,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
                 const int who = __ffs(hit) - 1;
                 seq = top - who;
                 len = __shfl_sync(0xffffffffu, n, who);
-                q0 = (__shfl_sync(0xffffffffu, upto, who) - 1 - want) * BM;
+                q0 = (__shfl_sync(0xffffffffu, upto, who) - 1 - want) * rows_per_cta;
                 break;
             }
             want -= __shfl_sync(0xffffffffu, upto, 31);
@@ -121,7 +125,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
     if (seq < 0) return;
     const int ctx = a.ctx_start[seq], row0 = a.cu_q[seq] + q0;
     if (ctx < 0) {                                                   // padding: zero rows (the paged form's are another kernel's)
-        const int rows = GATHERED ? min(len - q0, BM) : 0, v8 = a.dv / 8;
+        const int rows = GATHERED ? min(len - q0, rows_per_cta) : 0, v8 = a.dv / 8;
         for (int idx = tid; idx < rows * v8; idx += NTHREADS)
             *reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + (size_t)(row0 + idx / v8) * a.out_stride + (size_t)group * a.dv + (idx % v8) * 8) =
                 make_uint4(0, 0, 0, 0);
@@ -133,7 +137,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
         Plan& pl = s_plan;
         pl.rows[0] = pl.rows[1] = pl.t0[0] = pl.t0[1] = pl.t1[0] = pl.t1[1] = 0;
         {
-            const int left = len - q0, p0 = ctx + q0, p_last = p0 + min(left, BM) - 1;
+            const int left = len - q0, p0 = ctx + q0, p_last = p0 + min(left, rows_per_cta) - 1;
             KeySpan span = key_span(p0, p_last, a.chunk, a.window, a.keep_first);
             if (GATHERED && span.wlo < a.k_lo[seq]) {                // the gathered rows begin at k_lo
                 span.wlo = span.lo = a.k_lo[seq];
@@ -142,11 +146,11 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             pl.span = span;
             pl.keep = a.window > 0 ? span.index(a.keep_first) : 0;
             pl.rows[0] = min(BM, left);
-            pl.rows[1] = TWO_MAPS ? pl.rows[0] : 0;
+            pl.rows[1] = two_rows ? min(BM, max(0, left - BM)) : (TWO_MAPS || hpc == 2) ? pl.rows[0] : 0;
 #pragma unroll 1
             for (int x = 0; x < 2; ++x) {
                 if (pl.rows[x] == 0) continue;
-                const int pf = p0;
+                const int pf = p0 + (two_rows && x ? BM : 0);
                 const RowRange f = range_of(span, pf, a.chunk, a.window), l = range_of(span, pf + pl.rows[x] - 1, a.chunk, a.window);
                 pl.first_row[x] = pf;
                 pl.t0[x] = (f.block < pl.keep ? f.block : f.low) / BN;
@@ -175,8 +179,8 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-        const int n_tiles = max(s_plan.t1[0], s_plan.t1[1]), n_keys = s_plan.span.n;
-    const int kvh = group / (a.H / a.G);                // kv head of the paged pools
+    const int n_tiles = max(s_plan.t1[0], s_plan.t1[1]), n_keys = s_plan.span.n;
+    const int kvh = (group * hpc) / (a.H / a.G);                     // kv head of the paged pools
 
     if (warp >= 8) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
@@ -216,8 +220,8 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             {                                                        // Q, by all three warps: rows past the tile are zeros
 #pragma unroll 1
                 for (int x = 0; x < 2; ++x) {
-                    const int hh = group, nrows = s_plan.rows[x];
-                    const int rbase = row0;
+                    const int hh = group * hpc + (hpc == 2 ? x : 0), nrows = s_plan.rows[x];
+                    const int rbase = row0 + (two_rows && x ? BM : 0);
                     if (nrows == 0) continue;
                     const int col0 = TWO_MAPS ? x * a.dk : 0;
                     const char* qh = reinterpret_cast<const char*>(static_cast<const bf16*>(a.q0) + (size_t)rbase * a.q0_row + (size_t)hh * a.q0_head + col0 + c8 * 8);
@@ -384,7 +388,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             const int row = wq * 32 + lane;                          // query row of the slot = TMEM lane
             const uint32_t lane_off = (uint32_t)(wq * 32) << 16;
             const uint32_t s_addr = tmem + lane_off + x * 128, o_addr = tmem + lane_off + 256 + x * 128;
-            const int hh = group;
+            const int hh = group * hpc + (hpc == 2 ? x : 0);
             const RowRange mine = range_of(s_plan.span, s_plan.first_row[x] + min(row, nrows - 1), a.chunk, a.window);
             const int all_hi = s_plan.all_hi[x], all_low = s_plan.all_low[x], keep = s_plan.keep;
             const float sl2 = prm.scale_log2;
@@ -514,7 +518,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
             // ------------------------------------------ output rows
             const int n = te - tb;
             const bool valid = row < nrows;
-            const size_t brow = (size_t)row0 + row;
+            const size_t brow = (size_t)row0 + (two_rows && x ? BM : 0) + row;
             wait(bar(L::BAR_PV + x), (n - 1) & 1, failed);
             float inv = KIND == KIND_SIGMOID ? 1.f : (l > 0.f ? 1.f / l : 0.f);
             if (*failed) inv = __int_as_float(0x7fc00000);           // behind the last wait, which may be the one that gave up
@@ -607,12 +611,42 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
 
 template <int NH, int DVH, int KIND, bool TWO_MAPS, bool GATHERED>
 int launch(const Params& p, dim3 grid, cudaStream_t st) {
-    auto kern = prompt_tc5_kernel<NH, DVH, KIND, TWO_MAPS, GATHERED>;
+    auto kern = prompt_tc5_kernel<NH, DVH, KIND, TWO_MAPS, GATHERED, false>;
+    if constexpr (!TWO_MAPS)
+        if (p.rows_per_cta > BM || p.heads_per_cta > 1) kern = prompt_tc5_kernel<NH, DVH, KIND, TWO_MAPS, GATHERED, true>;
     constexpr int smem = Shape<NH, DVH, TWO_MAPS>::SMEM;
     B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     kern<<<grid, NTHREADS, smem, st>>>(p);
     B2_CUDA_OK(cudaGetLastError());
     return B2_OK;
+}
+
+// A tile a CTA, of one slot, of two heads of a kv head or of two row tiles; or CTAs that take tiles in turns (prompt_turns_tc5.cu), whose first
+// scores come 1.3 us later.  Times below: in a graph, this kernel / turns.
+enum Form { ONE_SLOT, HEAD_PAIRS, ROW_PAIRS, TURNS };
+
+int64_t longs_of(const b2_prompt_args& a) { return std::min(a.n_seq, a.T / a.min_rows); }      // most sequences of min_rows rows or more
+
+Form form_of(const b2_prompt_args& a) {
+    const int64_t n_sm = b2_sm_count(), longs = longs_of(a);
+    if (longs == 0) return ONE_SLOT;
+    // One slot to one and a half waves: 300 rows x 16 heads 15.0 / 15.4 us, 1000 x 16 22.2 / 23.6, 1200 gathered x 16 40.7 / 41.8, 1300 x 16 (176 tiles)
+    // 27.4 / 27.1, 4 x 146 x 32 (256) 26.6 / 25.2.  The count is a bound: every sequence may begin a tile more.
+    int64_t tiles = (int64_t)a.T / BM + longs;
+    const bool rows_of_few = a.T < (int64_t)a.min_rows * a.n_seq;             // mostly decode rows
+    if (tiles * a.H <= n_sm * 3 / 2) return ONE_SLOT;
+    if (a.cu_k || a.maps == 2 || (a.H / a.G) % 2 || rows_of_few) return TURNS;
+    // Two heads a CTA, if that is one wave with remainders of half a tile (the host does not have the lengths) and short: 8 x 200 rows x 16 heads
+    // 13.7 / 15.4, 4 x 400 17.0 / 18.9, 2 x 900 (8 steps) 25.2 / 26.6, 1000 x 32 26.6 / 27.2.  Not at 9 steps (1750 x 16, window 1024, 30.2 / 29.6),
+    // beyond one wave (4 x 600 x 16, 160 CTAs, 23.7 / 21.6; 830 + 577 + 817 x 16 in blocks of 510, 152 CTAs, 26.7 / 23.0), with capped scores
+    // (1000 + 800 x 16 34.9 / 32.3) or heads of 96 (570 + 396 x 32, window 152, 19.8 / 18.9).  The ragged 187 + 750 + 187 + 375 x 16 take 22.7 in
+    // either, and would take 20.0 in one slot each.
+    const int64_t pairs = (a.T + longs * (BM / 2)) * (a.H / 2) / BM;
+    int64_t steps = ((int64_t)a.max_nb * a.bs + BN - 1) / BN;                 // of the longest tile, at most
+    if (a.window > 0) steps = std::min<int64_t>(steps, (a.window + BM) / BN + 1);
+    if (a.chunk > 0) steps = std::min<int64_t>(steps, a.chunk / BN + 2);
+    if (a.cap == 0.f && a.dk % 64 == 0 && steps <= 8 && pairs <= n_sm) return HEAD_PAIRS;
+    return TURNS;
 }
 
 }  // namespace
@@ -625,13 +659,15 @@ bool b2_internal_prompt_tc5_ok(const b2_prompt_args& a) {
 }
 
 int b2_internal_prompt_tc5(const b2_prompt_args& a, void* stream) {
-    // A CTA a tile of one slot (two maps: two) up to one and a half waves; more tiles are taken in turns.  In a graph, this kernel / turns: 300 rows x
-    // 16 heads 15.0 / 15.4 us, 1000 x 16 22.2 / 23.6, 1200 gathered x 16 40.7 / 41.8, 1300 x 16 (176 tiles) 27.4 / 27.1, 4 x 146 x 32 (256) 26.6 / 25.2.
-    const int64_t longs = std::min(a.n_seq, a.T / a.min_rows);       // sequences of min_rows rows or more
-    const int64_t tiles = (int64_t)a.T / BM + longs, ctas = tiles * a.H;         // upper bound on sum(ceil(len / rows)); spare CTAs leave at once
-    if (tiles == 0) return B2_OK;
-    if (ctas > b2_sm_count() * 3 / 2) return b2_internal_prompt_turns(a, stream);
+    const Form form = form_of(a);
+    if (form == TURNS) return b2_internal_prompt_turns(a, stream);
     Params p;
+    p.rows_per_cta = form == ROW_PAIRS ? 2 * BM : BM;
+    p.heads_per_cta = form == HEAD_PAIRS ? 2 : 1;
+    const int64_t tiles = (int64_t)a.T / p.rows_per_cta + longs_of(a);       // upper bound on sum(ceil(len / rows)); spare CTAs leave at once
+    if (tiles == 0) return B2_OK;
+    const int64_t ctas = tiles * (a.H / p.heads_per_cta);
+    B2_REQUIRE(ctas <= 0x7fffffff, B2_EUNSUPPORTED, "prompt attention: %lld row tiles exceed the grid", (long long)tiles);
     p.a = a;
     p.scale_log2 = a.scale * LOG2E;
     p.bs_shift = -1;
