@@ -19,6 +19,12 @@ pytestmark = pytest.mark.gpu
     ([500, 300], [3, 0], 32, 4, 96, 128, 16, 0, 200, 0, 0.0, False, 1, True, False, 1.0),
     ([1020], [30], 32, 8, 64, 64, 16, 0, 0, 0, 0.0, False, 1, False, False, 1.0),
     ([300] * 7, [0] * 7, 16, 4, 64, 64, 16, 0, 0, 0, 0.0, False, 1, False, False, 1.0),
+    # capped scores in short windows or blocks: two heads a CTA, scores on both sides of the polynomial; one slot; two row tiles; a longer window
+    ([600, 333], [0, 40], 32, 8, 128, 128, 16, 0, 150, 5, 30.0, True, 1, False, True, 1.0),
+    ([600, 333], [0, 40], 32, 8, 64, 64, 24, 256, 0, 0, 1.5, False, 1, False, False, 1.0),
+    ([400, 500], [5, 0], 28, 4, 64, 64, 16, 0, 200, 0, 30.0, True, 1, False, False, 1.0),
+    ([700, 640], [5, 0], 28, 4, 64, 128, 16, 0, 384, 3, 30.0, False, 1, False, True, -1.0),
+    ([700, 640], [5, 0], 28, 4, 64, 64, 16, 0, 900, 0, 30.0, False, 1, False, False, 1.0),
 ])
 def test_forms(cuda, c):
     masked_rows(cuda, c)

@@ -635,7 +635,21 @@ Form form_of(const b2_prompt_args& a) {
     int64_t tiles = (int64_t)a.T / BM + longs;
     const bool rows_of_few = a.T < (int64_t)a.min_rows * a.n_seq;             // mostly decode rows
     if (tiles * a.H <= n_sm * 3 / 2) return ONE_SLOT;
-    if (a.cu_k || a.maps == 2 || (a.H / a.G) % 2 || rows_of_few) return TURNS;
+    if (a.cu_k || a.maps == 2 || rows_of_few) return TURNS;
+    const bool heads = (a.H / a.G) % 2 == 0;
+    // Capped scores of which a mask cuts most key tiles, up to two waves: such a step takes 6k cycles in turns.  Windows of 150: 4096 rows x 16 heads on 4
+    // kv heads 37.2 / 40.6, 16 on 16 40.7 / 44.1, 8 on 8 25.9 / 32.4, 2000 x 16 20.4 / 24.1; of 500: 50.7 / 52.4, 54.3 / 61.3, 34.7 / 41.9, 26.9 / 31.8;
+    // of 1024 75.1 / 70.0, and of 500 in 3.4 waves (4096 x 32) 97.5 / 93.0; three waves of row tiles (600 + 417 + 591 + 1055 x 28) 54.3 / 59.3 but
+    // 52.0 / 45.7 with windows of 150.  The tiles of 1.1 to 1.4 waves go either way (600 + 417 + 591 + 1055 x 16, 150, 500 and 850: 30.8 / 30.7, 35.4 /
+    // 30.2, 36.2 / 37.4).
+    const int reach = a.chunk > 0 && (a.window == 0 || a.chunk < a.window) ? a.chunk : a.window;
+    if (a.cap > 0.f && reach > 0 && reach <= 7 * BN) {
+        const int64_t rows256 = ((int64_t)a.T / (2 * BM) + longs) * a.H;
+        const Form form = heads ? HEAD_PAIRS : rows256 >= n_sm ? ROW_PAIRS : ONE_SLOT;
+        const int64_t ctas = form == ROW_PAIRS ? rows256 : (a.T + longs * (BM / 2)) * (heads ? a.H / 2 : a.H) / BM;
+        return ctas <= (form == ROW_PAIRS && reach > 2 * BN ? 3 : 2) * n_sm ? form : TURNS;
+    }
+    if (!heads) return TURNS;
     // Two heads a CTA, if that is one wave with remainders of half a tile (the host does not have the lengths) and short: 8 x 200 rows x 16 heads
     // 13.7 / 15.4, 4 x 400 17.0 / 18.9, 2 x 900 (8 steps) 25.2 / 26.6, 1000 x 32 26.6 / 27.2.  Not at 9 steps (1750 x 16, window 1024, 30.2 / 29.6),
     // beyond one wave (4 x 600 x 16, 160 CTAs, 23.7 / 21.6; 830 + 577 + 817 x 16 in blocks of 510, 152 CTAs, 26.7 / 23.0), with capped scores
