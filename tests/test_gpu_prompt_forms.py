@@ -28,3 +28,13 @@ pytestmark = pytest.mark.gpu
 ])
 def test_forms(cuda, c):
     masked_rows(cuda, c)
+
+
+@pytest.mark.parametrize("lens,ctx,H,dn,dr,dv,window,sink,gate", [
+    ([1792], [0], 16, 128, 64, 128, 0, True, 2),                         # one causal portion: one slot to 1.6 waves
+    ([2400], [0], 16, 64, 64, 64, 0, False, 1),                          # ... two row tiles a CTA, the last one half a slot
+    ([2049], [0], 19, 24, 8, 112, 0, True, 0),                           # ... a row in the last tile
+    ([2305], [3], 16, 64, 64, 64, 0, False, 1),                          # behind a context: in turns
+])
+def test_one_gathered_portion(cuda, lens, ctx, H, dn, dr, dv, window, sink, gate):
+    gathered_rows(cuda, lens, ctx, H, dn, dr, dv, window, sink, gate)

@@ -635,6 +635,16 @@ Form form_of(const b2_prompt_args& a) {
     int64_t tiles = (int64_t)a.T / BM + longs;
     const bool rows_of_few = a.T < (int64_t)a.min_rows * a.n_seq;             // mostly decode rows
     if (tiles * a.H <= n_sm * 3 / 2) return ONE_SLOT;
+    // One causal portion without context is as long as its longest tile, which turns do not shorten.  One slot: 1792 gathered rows x 16 heads (224
+    // tiles) 32.4 / 34.1 us, 1800 x 16 (240) 36.3 / 34.9; past 16 steps 3584 x 8 (224) 56.6 / 59.0, 4000 x 8 (256) 62.6 / 65.0.  Two row tiles past 16
+    // steps: 2400 x 16 (160 CTAs) 46.2 / 47.4, 3584 x 16 (224) 66.0 / 68.4, 4000 x 16 (256) 76.6 / 75.8, 1792 x 32 (14 steps, 224) 41.2 / 39.3; 2000 x 16,
+    // which would leave SMs without a CTA, 42.5 / 38.1.
+    if (a.cu_k && a.n_seq == 1 && a.window == 0 && a.k_rows == a.T) {
+        const int64_t one = ((int64_t)a.T + BM - 1) / BM * a.H, two = ((int64_t)a.T + 2 * BM - 1) / (2 * BM) * a.H;
+        const bool longer = a.T > 16 * BM;
+        if (longer ? one * 4 <= n_sm * 7 : one * 5 <= n_sm * 8) return ONE_SLOT;
+        if (longer && two >= n_sm && two * 5 <= n_sm * 8) return ROW_PAIRS;
+    }
     if (a.cu_k || a.maps == 2 || rows_of_few) return TURNS;
     const bool heads = (a.H / a.G) % 2 == 0;
     // Capped scores of which a mask cuts most key tiles, up to two waves: such a step takes 6k cycles in turns.  Windows of 150: 4096 rows x 16 heads on 4
