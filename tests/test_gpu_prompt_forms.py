@@ -13,6 +13,9 @@ pytestmark = pytest.mark.gpu
     ([1] * 40 + [200, 130], [60] * 40 + [0, 77], 32, 8, 64, 64, 16, 0, 100, 3, 0.0, True, 1, False, True, 1.0),
     ([1] * 40 + [300, 16], [60] * 41 + [5], 28, 4, 64, 64, 16, 0, 0, 0, 0.0, False, 1, False, True, 1.0),
     ([1] * 33 + [250], [60] * 33 + [9], 16, 2, 128, 64, 16, 128, 0, 0, 0.0, False, 1, True, False, 1.0),
+    # ... and where capped scores or two maps make the start in turns a long one
+    ([1] * 40 + [200], [60] * 40 + [9], 32, 8, 64, 64, 16, 0, 100, 3, 30.0, True, 1, False, True, 1.0),
+    ([1] * 40 + [150] + [16] * 9, [60] * 40 + [9] * 10, 32, 8, 64, 64, 16, 0, 100, 3, 0.0, True, 2, False, True, 1.0),
     # portions of a few key tiles, two heads a CTA: one wave, the last tile's edges, pages that are no power of two; nine steps, and more than a wave
     ([200, 129, 128, 16, 250, 201, 127, 255], [0, 40, 0, 9, 0, 1, 600, 0], 16, 4, 128, 128, 16, 0, 0, 0, 0.0, True, 1, False, True, 1.0),
     ([290, 411, 130], [0, 33, 5], 32, 8, 64, 64, 24, 300, 100, 7, 0.0, True, 1, False, False, 1.0),

@@ -633,7 +633,11 @@ Form form_of(const b2_prompt_args& a) {
     // One slot to one and a half waves: 300 rows x 16 heads 15.0 / 15.4 us, 1000 x 16 22.2 / 23.6, 1200 gathered x 16 40.7 / 41.8, 1300 x 16 (176 tiles)
     // 27.4 / 27.1, 4 x 146 x 32 (256) 26.6 / 25.2.  The count is a bound: every sequence may begin a tile more.
     int64_t tiles = (int64_t)a.T / BM + longs;
-    const bool rows_of_few = a.T < (int64_t)a.min_rows * a.n_seq;             // mostly decode rows
+    // Where most sequences must be decode rows it is far too large: if those of one or two portions are one wave, capped scores and two maps, whose
+    // start in turns is the longer one, stay here.  64 decode rows and a prompt of 200, with the decode kernel: 16 heads, capped 61.2 / 70.4, two maps
+    // 63.7 / 68.2, but ten prompts of 20 x 32 heads, capped, 83.4 / 81.3; other weights 73.1 / 73.6 and 81.6 / 77.4 (32 heads).
+    const bool rows_of_few = a.T < (int64_t)a.min_rows * a.n_seq;
+    if (rows_of_few && (a.cap > 0.f || a.maps == 2) && ((a.T - a.n_seq) / BM + 2) * a.H <= n_sm) return ONE_SLOT;
     if (tiles * a.H <= n_sm * 3 / 2) return ONE_SLOT;
     // One causal portion without context is as long as its longest tile, which turns do not shorten.  One slot: 1792 gathered rows x 16 heads (224
     // tiles) 32.4 / 34.1 us, 1800 x 16 (240) 36.3 / 34.9; past 16 steps 3584 x 8 (224) 56.6 / 59.0, 4000 x 8 (256) 62.6 / 65.0.  Two row tiles past 16
