@@ -16,6 +16,7 @@ pytestmark = pytest.mark.gpu
     # ... and where capped scores or two maps make the start in turns a long one
     ([1] * 40 + [200], [60] * 40 + [9], 32, 8, 64, 64, 16, 0, 100, 3, 30.0, True, 1, False, True, 1.0),
     ([1] * 40 + [150] + [16] * 9, [60] * 40 + [9] * 10, 32, 8, 64, 64, 16, 0, 100, 3, 0.0, True, 2, False, True, 1.0),
+    ([100, 140, 30], [0, 9, 200], 49, 7, 64, 64, 16, 0, 0, 0, 0.0, True, 1, False, False, 1.0),          # two row tiles a CTA of odd heads
     # portions of a few key tiles, two heads a CTA: one wave, the last tile's edges, pages that are no power of two; nine steps, and more than a wave
     ([200, 129, 128, 16, 250, 201, 127, 255], [0, 40, 0, 9, 0, 1, 600, 0], 16, 4, 128, 128, 16, 0, 0, 0, 0.0, True, 1, False, True, 1.0),
     ([290, 411, 130], [0, 33, 5], 32, 8, 64, 64, 24, 300, 100, 7, 0.0, True, 1, False, False, 1.0),
@@ -34,10 +35,11 @@ def test_forms(cuda, c):
 
 
 @pytest.mark.parametrize("lens,ctx,H,dn,dr,dv,window,sink,gate", [
+    ([85, 58, 83, 148], [555, 0, 30, 9], 32, 128, 64, 128, 0, True, 1),  # two row tiles a CTA where one a CTA would be more than a wave
     ([1792], [0], 16, 128, 64, 128, 0, True, 2),                         # one causal portion: one slot to 1.6 waves
     ([2400], [0], 16, 64, 64, 64, 0, False, 1),                          # ... two row tiles a CTA, the last one half a slot
     ([2049], [0], 19, 24, 8, 112, 0, True, 0),                           # ... a row in the last tile
     ([2305], [3], 16, 64, 64, 64, 0, False, 1),                          # behind a context: in turns
 ])
-def test_one_gathered_portion(cuda, lens, ctx, H, dn, dr, dv, window, sink, gate):
+def test_gathered_forms(cuda, lens, ctx, H, dn, dr, dv, window, sink, gate):
     gathered_rows(cuda, lens, ctx, H, dn, dr, dv, window, sink, gate)

@@ -638,15 +638,18 @@ Form form_of(const b2_prompt_args& a) {
     // 63.7 / 68.2, but ten prompts of 20 x 32 heads, capped, 83.4 / 81.3; other weights 73.1 / 73.6 and 81.6 / 77.4 (32 heads).
     const bool rows_of_few = a.T < (int64_t)a.min_rows * a.n_seq;
     if (rows_of_few && (a.cap > 0.f || a.maps == 2) && ((a.T - a.n_seq) / BM + 2) * a.H <= n_sm) return ONE_SLOT;
-    if (tiles * a.H <= n_sm * 3 / 2) return ONE_SLOT;
+    // Tiles of two rows, where they are the form in turns too, leave fewer tiles: 85 + 58 + 83 + 148 gathered rows behind 555 x 32, 128 CTAs of two and
+    // 160 of one, 18.7 against 26.4.
+    const bool row_pairs = a.maps == 1 && (a.cu_k || (a.H / a.G) % 2) && ((int64_t)a.T / (2 * BM) + longs) * a.H >= n_sm;
+    if (tiles * a.H <= n_sm * 3 / 2) return row_pairs ? ROW_PAIRS : ONE_SLOT;
     // One causal portion without context is as long as its longest tile, which turns do not shorten.  One slot: 1792 gathered rows x 16 heads (224
-    // tiles) 32.4 / 34.1 us, 1800 x 16 (240) 36.3 / 34.9; past 16 steps 3584 x 8 (224) 56.6 / 59.0, 4000 x 8 (256) 62.6 / 65.0.  Two row tiles past 16
-    // steps: 2400 x 16 (160 CTAs) 46.2 / 47.4, 3584 x 16 (224) 66.0 / 68.4, 4000 x 16 (256) 76.6 / 75.8, 1792 x 32 (14 steps, 224) 41.2 / 39.3; 2000 x 16,
-    // which would leave SMs without a CTA, 42.5 / 38.1.
+    // tiles) 32.4 / 34.1 us, 1800 x 16 (240) 36.3 / 34.9, 871 x 32 (224) 23.8 / 22.1; past 16 steps 3584 x 8 (224) 56.6 / 59.0, 4000 x 8 (256) 62.6 /
+    // 65.0.  Two row tiles past 16 steps: 2400 x 16 (160 CTAs) 46.2 / 47.4, 3584 x 16 (224) 66.0 / 68.4, 4000 x 16 (256) 76.6 / 75.8, 1792 x 32 (14
+    // steps, 224) 41.2 / 39.3; 2000 x 16, which would leave SMs without a CTA, 42.5 / 38.1.
     if (a.cu_k && a.n_seq == 1 && a.window == 0 && a.k_rows == a.T) {
         const int64_t one = ((int64_t)a.T + BM - 1) / BM * a.H, two = ((int64_t)a.T + 2 * BM - 1) / (2 * BM) * a.H;
         const bool longer = a.T > 16 * BM;
-        if (longer ? one * 4 <= n_sm * 7 : one * 5 <= n_sm * 8) return ONE_SLOT;
+        if (longer ? one * 4 <= n_sm * 7 : a.T > 12 * BM && one * 5 <= n_sm * 8) return ONE_SLOT;
         if (longer && two >= n_sm && two * 5 <= n_sm * 8) return ROW_PAIRS;
     }
     if (a.cu_k || a.maps == 2 || rows_of_few) return TURNS;
@@ -658,23 +661,22 @@ Form form_of(const b2_prompt_args& a) {
     // 30.2, 36.2 / 37.4).
     const int reach = a.chunk > 0 && (a.window == 0 || a.chunk < a.window) ? a.chunk : a.window;
     if (a.cap > 0.f && reach > 0 && reach <= 7 * BN) {
-        const int64_t rows256 = ((int64_t)a.T / (2 * BM) + longs) * a.H;
-        const Form form = heads ? HEAD_PAIRS : rows256 >= n_sm ? ROW_PAIRS : ONE_SLOT;
-        const int64_t ctas = form == ROW_PAIRS ? rows256 : (a.T + longs * (BM / 2)) * (heads ? a.H / 2 : a.H) / BM;
+        const Form form = heads ? HEAD_PAIRS : row_pairs ? ROW_PAIRS : ONE_SLOT;
+        const int64_t ctas = form == ROW_PAIRS ? ((int64_t)a.T / (2 * BM) + longs) * a.H : (a.T + longs * (BM / 2)) * (heads ? a.H / 2 : a.H) / BM;
         return ctas <= (form == ROW_PAIRS && reach > 2 * BN ? 3 : 2) * n_sm ? form : TURNS;
     }
-    if (!heads) return TURNS;
     // Two heads a CTA, if that is one wave with remainders of half a tile (the host does not have the lengths) and short: 8 x 200 rows x 16 heads
     // 13.7 / 15.4, 4 x 400 17.0 / 18.9, 2 x 900 (8 steps) 25.2 / 26.6, 1000 x 32 26.6 / 27.2.  Not at 9 steps (1750 x 16, window 1024, 30.2 / 29.6),
     // beyond one wave (4 x 600 x 16, 160 CTAs, 23.7 / 21.6; 830 + 577 + 817 x 16 in blocks of 510, 152 CTAs, 26.7 / 23.0), with capped scores
     // (1000 + 800 x 16 34.9 / 32.3) or heads of 96 (570 + 396 x 32, window 152, 19.8 / 18.9).  The ragged 187 + 750 + 187 + 375 x 16 take 22.7 in
     // either, and would take 20.0 in one slot each.
+    // Not two row tiles: 66 + 101 + 257 + 94 + 97 + 30 + 32 + 137 gathered rows x 16 13.1 / 13.6, but 292 + 211 + 298 x 32 22.9 / 20.1.
+    if (!heads || a.cap > 0.f || a.dk % 64) return TURNS;
     const int64_t pairs = (a.T + longs * (BM / 2)) * (a.H / 2) / BM;
     int64_t steps = ((int64_t)a.max_nb * a.bs + BN - 1) / BN;                 // of the longest tile, at most
     if (a.window > 0) steps = std::min<int64_t>(steps, (a.window + BM) / BN + 1);
     if (a.chunk > 0) steps = std::min<int64_t>(steps, a.chunk / BN + 2);
-    if (a.cap == 0.f && a.dk % 64 == 0 && steps <= 8 && pairs <= n_sm) return HEAD_PAIRS;
-    return TURNS;
+    return pairs <= n_sm && steps <= 8 ? HEAD_PAIRS : TURNS;
 }
 
 }  // namespace
