@@ -39,3 +39,28 @@ def test_one_lane_arrives_behind_a_warp_barrier(name):
             if not ok and (name, m.group(1)) not in OWN:
                 loose.append((i + 1, line.strip()))
     assert not loose, loose
+
+
+# kernels whose waits may give up, and the barriers that their boxes or MMAs complete
+IN_FLIGHT = [
+    ("prompt_turns_tc5.cu", "prompt_turns_kernel", ["L::BAR_Q)", "L::BAR_Q + 1)", "L::BAR_V : L::BAR_K"]),
+    ("prompt_tc5.cu", "prompt_tc5_kernel", ["L::BAR_V : L::BAR_K"]),
+    ("latent_tc5.cu", "latent_tc5_kernel", ["FULL"]),
+    ("moe_tc5.cu", "moe_tc5_kernel", ["full(", "s_end"]),
+    ("delta_tc5.cu", "chain_kernel", ["here(", "done"]),
+    ("delta_tc5.cu", "read_kernel", ["s_here", "s_done"]),
+]
+
+
+@pytest.mark.parametrize("name,kernel,bars", IN_FLIGHT)
+def test_what_is_in_flight_is_waited_for_when_a_wait_gave_up(name, kernel, bars):
+    """A wait of any role may give up last, when those that copy have left their loops: what is under way is waited for behind a barrier of the
+    whole CTA, not where a copying warp's own wait failed."""
+    text = "\n".join(_code(name))
+    body = text[text.index(kernel + "("):]
+    body = body[:body.index("\n}\n")]
+    at_end = body[body.rindex("__syncthreads();"):]
+    drained = re.findall(r"drain\((.*)", at_end)
+    assert re.search(r"if \([^{]*failed", at_end)
+    for bar in bars:
+        assert any(bar in d for d in drained), (bar, drained)

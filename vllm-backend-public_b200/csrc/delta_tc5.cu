@@ -476,15 +476,14 @@ chain_kernel(const Args a) {
     auto free_ = [&](int b) { return b2::smem_u32(&s_free[b]); };
     const uint32_t tmem = tmem_alloc(&s_tmem, warp);
     const int total = nchunks * L.slices;
+    int sent = 0;                                    // slices of M that this thread has asked for
     if (warp == 8) {
         if (lane == 0) {
 #pragma unroll 1
             for (int i = 0; i < total; ++i) {
                 const int b = i % 3;
-                if (i >= 3 && !wait(free_(b), (i / 3 - 1) & 1, &s_failed)) {
-                    for (int back = 1; back <= 3; ++back) drain(here((i - back) % 3), ((i - back) / 3) & 1);
-                    break;
-                }
+                if (i >= 3 && !wait(free_(b), (i / 3 - 1) & 1, &s_failed)) break;
+                sent = i + 1;
                 b2::mbar_arrive_expect_tx(here(b), 3 * PART);
                 b2::bulk_load(sm + b * 3 * PART, ws + (i / L.slices) * step + L.m + (i % L.slices) * (3 * PART / 4), 3 * PART, here(b));
             }
@@ -568,8 +567,12 @@ chain_kernel(const Args a) {
                     *reinterpret_cast<float4*>(dst + e) = bad ? make_float4(kNaN, kNaN, kNaN, kNaN) : make_float4(s[e], s[e + 1], s[e + 2], s[e + 3]);
         }
     }
+    __syncthreads();
+    if (*(volatile int*)&s_failed) {                 // what nobody has waited for: every role is done now
+        drain(done, (nchunks - 1) & 1);
+        for (int back = 1; back <= min(3, sent); ++back) drain(here((sent - back) % 3), ((sent - back) / 3) & 1);
+    }
     __syncwarp();
-    if (*(volatile int*)&s_failed) drain(done, (nchunks - 1) & 1);
     tmem_free(tmem, warp);
 }
 
@@ -653,7 +656,7 @@ read_kernel(const __grid_constant__ Args a) {
     const uint32_t tmem = tmem_alloc(&s_tmem, warp);
     const int dk = a.dk, dv = a.dv;
     const Layout L(dk, dv, CH, DELTA);
-    int n = 0;                                       // items with a state so far
+    int n = 0, sent = 0;                             // items with a state so far; slices that this thread has asked for
     if (warp == 8) {
         int i = 0;
 #pragma unroll 1
@@ -665,6 +668,7 @@ read_kernel(const __grid_constant__ Args a) {
                 const int b = i % 3;
                 if (i >= 3) wait(bar(s_free, b), (i / 3 - 1) & 1, &s_failed);
                 if (lane == 0 && !*(volatile int*)&s_failed) {
+                    sent = i + 1;
                     b2::mbar_arrive_expect_tx(bar(s_here, b), (zn + 1) * 3 * 8192);
                     for (int z = 0; z < zn; ++z)
                         b2::bulk_load(sm + b * STAGE + z * 3 * 8192, ws + L.s + ((2 * at.block + z) * L.slices + u) * (3 * 8192 / 4), 3 * 8192, bar(s_here, b));
@@ -673,9 +677,6 @@ read_kernel(const __grid_constant__ Args a) {
                 __syncwarp();
             }
         }
-        if (*(volatile int*)&s_failed && lane == 0)
-            for (int back = 1; back <= 3 && back <= i; ++back) drain(bar(s_here, (i - back) % 3), ((i - back) / 3) & 1);
-        __syncwarp();
     } else if (warp == 9) {
         const int k_last = max(2, (dk - (L.slices - 1) * 64 + 15) / 16);           // past dk there are zeros
         int i = 0;
@@ -736,7 +737,12 @@ read_kernel(const __grid_constant__ Args a) {
             at = next;
         }
     }
-    if (*(volatile int*)&s_failed && n > 0) drain(bar(s_done, (n - 1) & 1), ((n - 1) / 2) & 1);
+    __syncthreads();
+    if (*(volatile int*)&s_failed) {                 // what nobody has waited for: every role is done now
+        if (n > 0) drain(bar(s_done, (n - 1) & 1), ((n - 1) / 2) & 1);
+        for (int back = 1; back <= min(3, sent); ++back) drain(bar(s_here, (sent - back) % 3), ((sent - back) / 3) & 1);
+    }
+    __syncwarp();
     tmem_free(tmem, warp);
     if (!DELTA && !*(volatile int*)&s_failed) again_read(a, s_again);
 }

@@ -159,10 +159,7 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
             for (int t = 0; t < nt; ++t) {
                 const int it = it0 + t, s = it & 1, kv0 = kbase + (t0 + t) * KT;
                 const uint32_t base = ring + s * (KT * 128), full = bar(FULL + s);
-                if (it >= 2 && !__all_sync(0xffffffffu, wait(bar(EMPTY + s), ((it >> 1) - 1) & 1, failed))) {
-                    for (int back = 1; lane == 0 && back <= 2; ++back) drain(bar(FULL + ((it - back) & 1)), ((it - back) >> 1) & 1);
-                    break;
-                }
+                if (it >= 2 && !__all_sync(0xffffffffu, wait(bar(EMPTY + s), ((it >> 1) - 1) & 1, failed))) break;
                 if (whole(t)) {
                     if (cw == 0) {
                         if (lane == 0) b2::mbar_arrive_expect_tx(full, (uint32_t)NS * KT * 128);      // columns past Dc are zero-filled and count
@@ -388,6 +385,10 @@ latent_tc5_kernel(const __grid_constant__ LatentArgs p) {
     __syncthreads();
     tc_fence_after();
     if (warp == 4) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(COLS) : "memory");
+    if (*failed && lane == 0) {                      // boxes that nobody has waited for: every role is done now
+        const int n = s_redo ? 2 * nt : nt;          // (a tile that was never begun takes the whole millisecond, which is as good)
+        for (int it = max(0, n - 2); it < n; ++it) drain(bar(FULL + (it & 1)), (it >> 1) & 1);
+    }
 }
 
 size_t smem_bytes(int Dc) { return (size_t)((Dc + 63) / 64) * (SUB + Q_SUB) + SUB + 1024; }

@@ -66,15 +66,14 @@ moe_tc5_kernel(const __grid_constant__ ExpertArgs p) {
     const uint32_t tmem = s_tmem;
     const int nk = (p.K + KSTEP - 1) / KSTEP;
 
+    int sent = 0;                                    // k-steps whose weights this thread has asked for
     if (warp == 0) {
         if (lane == 0) {
 #pragma unroll 1
             for (int it = 0; it < nk; ++it) {
                 const int s = it % ST;
-                if (it >= ST && !wait(empty(s), (it / ST - 1) & 1, failed)) {
-                    for (int back = 1; back <= ST; ++back) drain(full((it - back) % ST), ((it - back) / ST) & 1);
-                    break;
-                }
+                if (it >= ST && !wait(empty(s), (it / ST - 1) & 1, failed)) break;
+                sent = it + 1;
                 b2::mbar_arrive_expect_tx(full(s), W_STAGE);         // columns and rows past the matrix are zero-filled and count
                 tma_load_3d(sm + s * W_STAGE, &p.map0, full(s), it * KSTEP, n0, e);
                 tma_load_3d(sm + s * W_STAGE + W_STAGE / 2, &p.map1, full(s), it * KSTEP, KIND == PAIR ? n0 : n0 + 64, e);
@@ -167,9 +166,13 @@ moe_tc5_kernel(const __grid_constant__ ExpertArgs p) {
             b2::st(static_cast<bf16*>(p.out) + (size_t)(m0 + r) * p.N + n0 + c, bad ? __int_as_float(0x7fc00000) : v);
         }
     }
-    if (bad) drain(b2::smem_u32(&s_end), 0);
     tc_fence_before();
     __syncthreads();
+    if (*failed) {                                   // what nobody has waited for: every role is done now
+        drain(b2::smem_u32(&s_end), 0);
+        for (int back = 1; back <= min(ST, sent); ++back) drain(full((sent - back) % ST), ((sent - back) / ST) & 1);
+        __syncwarp();
+    }
     tc_fence_after();
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(tmem) : "memory");
 }

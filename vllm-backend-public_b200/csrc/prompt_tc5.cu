@@ -252,11 +252,7 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
 #pragma unroll 1
             for (int it = 0; it < n_tiles; ++it) {
                 const int s = it % nst, ph = (it / nst) & 1;
-                if (!__all_sync(0xffffffffu, wait(bar((is_v ? L::BAR_VE : L::BAR_KE) + s), ph ^ 1, failed))) {
-                    for (int back = 1; GATHERED && lane == 0 && back <= min(nst, it); ++back)
-                        drain(bar((is_v ? L::BAR_V : L::BAR_K) + (it - back) % nst), ((it - back) / nst) & 1);
-                    break;
-                }
+                if (!__all_sync(0xffffffffu, wait(bar((is_v ? L::BAR_VE : L::BAR_KE) + s), ph ^ 1, failed))) break;
                 const uint32_t base = is_v ? v_ring + s * L::V_STAGE : k_ring + s * L::K_STAGE;
                 const uint32_t full = bar((is_v ? L::BAR_V : L::BAR_K) + s);
                 const bool whole = GATHERED && prm.tma && (it + 1) * BN <= n_keys;      // all 128 rows are this sequence's
@@ -606,6 +602,10 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
     if (warp == 9) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    }
+    if (GATHERED && *failed && lane == 0 && (warp == 8 || warp == 10)) {     // boxes that nobody has waited for: every role is done now
+        const int nst = warp == 10 ? L::VST : L::KST;                // (a tile that was never begun takes the whole millisecond, which is as good)
+        for (int it = max(0, n_tiles - nst); it < n_tiles; ++it) drain(bar((warp == 10 ? L::BAR_V : L::BAR_K) + it % nst), (it / nst) & 1);
     }
 }
 

@@ -329,6 +329,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
         tc_fence_after();
     }
     const uint32_t tmem = warp != W_PLAN ? s_tmem : 0u;
+    int sent0 = 0, sent1 = 0;                                        // Q tiles of the slots that the plan warp has asked for; key tiles of a copying warp
     const bool two_rows = prm.rows_per_cta > BM, two_heads = prm.heads_per_cta == 2;     // slot 1's rows or head, where it is not empty
     // the plan of tile t: its place, which stays the tile's until every warp has said that it is done with it
     auto plan_of = [&](int t) -> const Plan* {
@@ -354,7 +355,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
             int tile_rows = prm.rows_per_cta, hpc = prm.heads_per_cta;
             order.init(a, tile_rows, hpc, lane);
             const uint32_t groups = (uint32_t)(a.H / hpc);
-            int t = 0, q_0 = 0, q_1 = 0;                             // tiles published, Q tiles of the slots
+            int t = 0;                                               // tiles published
 #pragma unroll 1
             for (uint32_t turn = 0;; ++turn) {
                 const uint32_t rank = tile_rank(turn);
@@ -427,9 +428,10 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
 #pragma unroll 1
                 for (int x = 0; x < 2; ++x) {
                     if ((x ? nrows1 : nrows0) == 0) continue;
-                    const int qn = x ? q_1++ : q_0++;
-                    ok = __all_sync(0xffffffffu, wait(bar(L::BAR_QE + x), (qn & 1) ^ 1, failed));
+                    ok = __all_sync(0xffffffffu, wait(bar(L::BAR_QE + x), ((x ? sent1 : sent0) & 1) ^ 1, failed));
                     if (!ok) break;
+                    if (x) ++sent1;
+                    else ++sent0;
                     if (prm.tma_q) {
                         q_boxes(x);
                         continue;
@@ -482,7 +484,8 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                 else if (!GATHERED || a.dk0 > 0) b2::tma_prefetch_desc(&prm.map_k0);
                 if (GATHERED && !is_v && a.dk0 < a.dk) b2::tma_prefetch_desc(&prm.map_k1);
             }
-            int g = 0, unit = is_v ? L::NK : 0;                      // key tiles of this CTA so far, first of this one's units
+            int& g = sent0;                                          // key tiles of this CTA so far
+            int unit = is_v ? L::NK : 0;                             // first of this one's units
             bool going = true;
 #pragma unroll 1
             for (int t = 0; going; ++t) {
@@ -533,8 +536,6 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                     const int lap = g * L::NS + (is_v ? L::NS : L::NK) - 1 - L::UNITS, before = lap / L::NS;
                     const int taken = lap % L::NS < L::NK ? L::BAR_KE : L::BAR_VE;
                     if (lap >= 0 && !__all_sync(0xffffffffu, wait(bar(taken + (before & 3)), (before >> 2) & 1, failed))) {
-                        for (int back = 1; lane == 0 && back <= min(4, g); ++back)
-                            drain(bar((is_v ? L::BAR_V : L::BAR_K) + ((g - back) & 3)), ((g - back) >> 2) & 1);
                         going = false;
                         break;
                     }
@@ -1060,6 +1061,14 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
     if (warp == W_MMA) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    }
+    if (*failed && lane == 0) {                                      // boxes that nobody has waited for, whichever wait gave up: every role is done now
+        if (warp == W_PLAN) {
+            if (sent0 > 0) drain(bar(L::BAR_Q), (sent0 - 1) & 1);
+            if (sent1 > 0) drain(bar(L::BAR_Q + 1), (sent1 - 1) & 1);
+        } else if (warp == W_K || warp == W_V) {
+            for (int back = 1; back <= min(4, sent0); ++back) drain(bar((warp == W_V ? L::BAR_V : L::BAR_K) + ((sent0 - back) & 3)), ((sent0 - back) >> 2) & 1);
+        }
     }
     if (*failed) {                                                   // a wait gave up: every row of this CTA's tiles is NaN
         int tile_rows = prm.rows_per_cta, hpc = prm.heads_per_cta;
