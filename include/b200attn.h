@@ -677,8 +677,8 @@ B2_API int b2_window_attention(void* out, const void* qn, int64_t qn_row, int qn
                                int n_seq, int T, int H, int dn, int dr, int dv, float scale, int window,
                                const float* sink_logits, const void* gate, int64_t gate_stride, int gate_channels,
                                int64_t out_stride, void* stream);
-/* the same, told how many gathered rows there are (n_keys = cu_k[n_seq]; 0: not known): it helps to choose between two kernels, and the
- * last rows of a portion are copied in whole boxes, none of which goes past row n_keys of kn, kt and v */
+/* the same, told how many gathered rows there are (n_keys = cu_k[n_seq]; 0: not known): it helps to choose between kernels and ways of copying the
+ * last rows; the results do not depend on it, and no row from cu_k[n_seq] on is read */
 B2_API int b2_window_attention_rows(void* out, const void* qn, int64_t qn_row, int qn_head, const void* qr, int64_t qr_row,
                                     int qr_head, const void* kn, const void* kt, int64_t kt_row, const void* v,
                                     const int32_t* cu_q, const int32_t* ctx_start, const int32_t* cu_k, const int32_t* k_lo,

@@ -76,21 +76,44 @@ def test_keys_beside_the_visible_ones(cuda, bs, cap, sigmoid):
         assert bool(((out[i] - ref).abs() <= 2.0 ** -8 * (spr + ref.abs()) + 1e-6).all()), i
 
 
-@pytest.mark.parametrize("N", [0, 1])
-def test_gathered_rows_of_unknown_number(cuda, N):
-    """n_keys 0: the last keys of a portion come row by row and not in boxes; the results are the same bits."""
-    lens, ctx, H, dn, dr, dv = [300, 129, 257], [0, 60, 5], 32, 128, 64, 128
+@pytest.mark.parametrize("lens,ctx,H,window", [([300, 129, 257], [0, 60, 5], 32, 0), ([1300, 700], [0, 33], 16, 200)])
+def test_gathered_rows_of_any_number(cuda, lens, ctx, H, window):
+    """The number of gathered rows is a hint: the true one, none, one that is too small or larger than the rows give the same bits (the last keys come in
+    boxes or row by row), and those are right.  One portion's keys and values, and the rows behind the last one, are NaN and infinity: boxes reach into
+    them, the other portions must not."""
+    dn, dr, dv, scale, bad = 128, 64, 128, 0.1, 1
     g = torch.Generator(device=cuda).manual_seed(9)
     rnd = lambda *s: torch.randn(*s, generator=g, device=cuda).bfloat16()        # noqa: E731
     i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
-    T = sum(lens)
-    rows, cu_k, k_lo = ops.latent_prompt_plan(lens, [a + b for a, b in zip(lens, ctx)], 0, 1 << 30, cuda)
-    q, kn, kt, v = rnd(T, H, dn + dr), rnd(rows, H, dn), rnd(rows, dr), rnd(rows, H, dv)
-    cu_q, start = i32([0, 300, 429, 686]), i32(ctx)
-    want = ops.window_attention(q[:, :, :dn], q[:, :, dn:], kn, kt, v, cu_q, start, cu_k, k_lo, 3, 0.1)
-    out = torch.empty_like(want)
+    T, cu = sum(lens), [0]
+    for m in lens:
+        cu.append(cu[-1] + m)
+    rows, cu_k, k_lo = ops.latent_prompt_plan(lens, [a + b for a, b in zip(lens, ctx)], window, 1 << 30, cuda)
+    ck, lo = cu_k.tolist(), k_lo.tolist()
+    spare = 300                                                          # rows of the buffers behind the last one
+    q, kn, kt, v = rnd(T, H, dn + dr), rnd(rows + spare, H, dn), rnd(rows + spare, dr), rnd(rows + spare, H, dv)
+    for t, x in ((kn, math.nan), (kt, math.nan), (v, math.inf)):
+        t[ck[bad]:ck[bad + 1]] = x
+        t[rows:] = x
+    cu_q, start = i32(cu), i32(ctx)
     p = lambda t: t.data_ptr()                                           # noqa: E731
-    _lib.check(_lib.load().b2_window_attention_rows(p(out), p(q), H * (dn + dr), dn + dr, p(q) + 2 * dn, H * (dn + dr), dn + dr, p(kn), p(kt), dr,
-                                                    p(v), p(cu_q), p(start), p(cu_k), p(k_lo), 3, T, H, dn, dr, dv, 0.1, 0, None, None, 0, 0,
-                                                    H * dv, rows * N, torch.cuda.current_stream().cuda_stream))
-    assert torch.equal(out, want)
+
+    def run(n_keys):
+        out = torch.empty(T, H, dv, dtype=torch.bfloat16, device=cuda)
+        _lib.check(_lib.load().b2_window_attention_rows(p(out), p(q), H * (dn + dr), dn + dr, p(q) + 2 * dn, H * (dn + dr), dn + dr, p(kn), p(kt), dr,
+                                                        p(v), p(cu_q), p(start), p(cu_k), p(k_lo), len(lens), T, H, dn, dr, dv, scale, window, None, None, 0,
+                                                        0, H * dv, n_keys, torch.cuda.current_stream().cuda_stream))
+        return out
+
+    want = run(rows)
+    for n_keys in (0, 1, rows - 150, rows + 200, 1 << 40):
+        assert torch.equal(run(n_keys).view(torch.int16), want.view(torch.int16)), n_keys
+    for i in range(len(lens)):
+        if i == bad:
+            continue
+        K = torch.cat([kn[ck[i]:ck[i + 1]].double(), kt[ck[i]:ck[i + 1], None].double().expand(-1, H, -1)], 2).transpose(0, 1)
+        V = v[ck[i]:ck[i + 1]].double().transpose(0, 1)
+        ok = _visible(torch.arange(ctx[i], ctx[i] + lens[i], device=cuda), ctx[i] + lens[i], 0, window, 0)[:, lo[i]:]
+        w = _weights(torch.bmm(q[cu[i]:cu[i + 1]].double().transpose(0, 1), K.transpose(1, 2)) * scale, ok, None, False, None)
+        ref, spr = torch.bmm(w, V).transpose(0, 1), torch.bmm(w, V.abs()).transpose(0, 1)
+        assert bool(((want[cu[i]:cu[i + 1]].double() - ref).abs() <= 2.0 ** -8 * (spr + ref.abs()) + 1e-6).all()), i

@@ -468,7 +468,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
         } else if (warp != W_MMA) {
             // ------------------------------------------ copies: K tiles / V tiles, on through all tiles of the CTA
             // By TMA, a box a page and 64 columns (gathered rows: 128 rows), a lane each.  Forms without boxes -- pages that do not lie on a
-            // tile's eight-row groups, gathered rows whose end is not known -- are cp.async gathers: eight lanes copy the 128 bytes of a row
+            // tile's eight-row groups, gathered rows at an end that the host does not know -- are cp.async gathers: eight lanes copy the 128 bytes of a row
             // and sub-tile, four rows (a group) an instruction, the pool rows of a tile's 128 keys (four a lane) looked up before the
             // stage is free: a lookup in front of its copies would put its latency on the path of every tile.
             const bool is_v = warp == W_V;
@@ -487,6 +487,13 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
             int& g = sent0;                                          // key tiles of this CTA so far
             int unit = is_v ? L::NK : 0;                             // first of this one's units
             bool going = true;
+            // A box of gathered rows must not read behind the last one, which the device knows (cu_k[n_seq]) whatever the host was told: where both
+            // agree the maps end there and zeros come behind, else the box has to end before either.
+            int box_end = -1;
+            if (GATHERED && prm.tma) {
+                const int last = a.cu_k[a.n_seq];
+                if (a.k_rows != last) box_end = a.k_rows > 0 && a.k_rows < last ? (int)a.k_rows : last;
+            }
 #pragma unroll 1
             for (int t = 0; going; ++t) {
                 const Plan* pl = plan_of(t);
@@ -500,7 +507,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                 const uint32_t head0 = (uint32_t)(TWO_MAPS && !is_v ? 2 * kvh : kvh);
                 const char* p0 = reinterpret_cast<const char*>(static_cast<const bf16*>(is_v ? a.v : a.k0) + (GATHERED ? (size_t)head * split : 0) + c8 * 8);
                 const char* p1g = GATHERED && !is_v ? p1 : p0;
-                const bool boxes_of_all = prm.tma && (!GATHERED || a.k_rows > 0);
+                const int in_boxes = !prm.tma ? 0 : GATHERED && box_end >= 0 ? (box_end - (int)g0 - span.w0) / BN : n_tiles;     // the first key tiles
                 uint32_t rows[4];
                 auto lookup = [&](int it) {
                     if (!GATHERED && prm.tma) {                      // rows[0], rows[1]: page of this lane's box, row in it
@@ -548,7 +555,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                         return (DVH == 2 ? ring + (uint32_t)((unit + half) % L::UNITS) * SUB : ring + (uint32_t)unit * SUB + half * (SUB / 2)) +
                                h * (SUB / 2) + (uint32_t)(r & 63) * 128;
                     };
-                    if (boxes_of_all || (GATHERED && prm.tma && left >= BN)) {
+                    if (it < in_boxes) {
                         // columns past the head are zero-filled and count; so do rows past the last one of a gathered buffer
                         const int there = GATHERED ? BN >> box_shift : min(BN >> box_shift, (left + (1 << box_shift) - 1) >> box_shift);
                         if (lane == 0) b2::mbar_arrive_expect_tx(full, (uint32_t)(there * n_sub) << (box_shift + 7));
@@ -1113,7 +1120,7 @@ int b2_internal_prompt_turns(const b2_prompt_args& a, void* stream) {
     const bool gathered = a.cu_k != nullptr;
     // Boxes: gathered rows are consecutive, 128 (V: 64) of them one a sub-tile; a page is one, if it fills whole groups of eight rows of a
     // tile.  A head's columns from two tensors (dk0) have to change between sub-tiles.  Pages: no limit, the tables' entries are the
-    // caller's; gathered rows: k_rows, behind which zeros come, or where it is not known only boxes whose rows are all the sequence's.
+    // caller's; gathered rows: k_rows, behind which zeros come, or none where it is not known (the kernel looks at their number itself).
     const uint64_t many = 0x7fffffff;
     const bool sides = !gathered || a.dk0 % 64 == 0 || a.dk0 >= a.dk;
     const int dr = a.dk - a.dk0;
@@ -1125,7 +1132,7 @@ int b2_internal_prompt_turns(const b2_prompt_args& a, void* stream) {
               (!gathered || dr == 0 || (a.q1_row % 8 == 0 && a.q1_head % 8 == 0 && b2_aligned16(a.q1)));
     int rc = B2_OK;
     if (p.tma && gathered) {
-        const uint64_t rows = a.k_rows > 0 ? (uint64_t)a.k_rows : many;
+        const uint64_t rows = a.k_rows > 0 && (uint64_t)a.k_rows < many ? (uint64_t)a.k_rows : many;
         const uint32_t box3[3] = {64, 1, BN}, box2[2] = {64, BN}, boxv[3] = {64, 1, 64};
         if (a.dk0 > 0) {
             const uint64_t dims[3] = {(uint64_t)a.dk0, (uint64_t)a.H, rows}, st[2] = {(uint64_t)a.dk0 * 2, (uint64_t)a.H * a.dk0 * 2};
