@@ -117,3 +117,18 @@ def test_gathered_rows_of_any_number(cuda, lens, ctx, H, window):
         w = _weights(torch.bmm(q[cu[i]:cu[i + 1]].double().transpose(0, 1), K.transpose(1, 2)) * scale, ok, None, False, None)
         ref, spr = torch.bmm(w, V).transpose(0, 1), torch.bmm(w, V.abs()).transpose(0, 1)
         assert bool(((want[cu[i]:cu[i + 1]].double() - ref).abs() <= 2.0 ** -8 * (spr + ref.abs()) + 1e-6).all()), i
+
+
+def test_gathered_rows_that_repeat(cuda):
+    """Queries and shared key parts with a row stride of zero (one row for all): no box has such a stride."""
+    T, H, dn, dr, dv = 1500, 16, 128, 64, 128
+    g = torch.Generator(device=cuda).manual_seed(4)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=cuda).bfloat16()        # noqa: E731
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=cuda)      # noqa: E731
+    rows, cu_k, k_lo = ops.latent_prompt_plan([T - 500, 500], [T - 500, 700], 300, 1 << 30, cuda)
+    kn, v = rnd(rows, H, dn), rnd(rows, H, dv)
+    args = (i32([0, T - 500, T]), i32([0, 200]), cu_k, k_lo, 2, 0.1, 300)
+    for qn, qr, kt in ((rnd(1, H, dn).expand(T, -1, -1), rnd(T, H, dr), rnd(rows, dr)), (rnd(T, H, dn), rnd(T, 1, dr).expand(-1, H, -1), rnd(rows, dr)),
+                       (rnd(T, H, dn), rnd(T, H, dr), rnd(1, dr).expand(rows, -1))):
+        want = ops.window_attention(qn.contiguous(), qr.contiguous(), kn, kt.contiguous(), v, *args)
+        assert torch.equal(ops.window_attention(qn, qr, kn, kt, v, *args), want)
