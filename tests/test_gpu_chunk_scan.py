@@ -65,6 +65,11 @@ def _reference(qkv, beta, dec, state, lens, ctx, slots, H, G, dk, dv):
     ([90, 70], [3, 0], [-1, 1], 2, 2, 20, 36, "one"),                    # a sequence without state; sizes with remainders
     ([257], [8], [1], 2, 2, 128, 64, "strong"),                          # products of a chunk far below the smallest float
     ([140], [8], [0], 3, 3, 4, 4, "zero"),
+    # chains of eight to thirty-three chunks of 64 or 128 tokens, and a short one beside a long one: eight or sixteen loads of a state in flight
+    ([576], [3], [0], 2, 2, 32, 32, "mild"),
+    ([1151], [0], [0], 2, 1, 20, 36, "mild"),
+    ([2100], [5], [0], 2, 2, 32, 32, "mild"),
+    ([1500, 40], [0, 7], [1, 0], 2, 2, 64, 16, "mild"),
 ])
 def test_chunked_scan(cuda, lens, ctx, slots, H, G, dk, dv, decay, delta, per_channel):
     qkv, beta, dec, state = _inputs(cuda, lens, H, G, dk, dv, per_channel, delta, decay, seed=len(lens) * 100 + dk + dv)

@@ -211,6 +211,7 @@ kv_kernel(const __grid_constant__ Args a) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------- state
+template <int AHEAD>
 __global__ void __launch_bounds__(128)
 state_kernel(const Args a) {
     const int seq = blockIdx.x, hh = blockIdx.y;
@@ -227,9 +228,7 @@ state_kernel(const Args a) {
     const bool pad = row >= dk;
     const float* from = pad ? nullptr : state_from(a, part, a.state_slot[seq], hh, a.ctx_start[seq]);
     float4 s = from ? *reinterpret_cast<const float4*>(from + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-    constexpr int AHEAD = 16;                        // loads in flight: they do not depend on the chain (4096 tokens x 16 heads, 84 MB: eight 22 us, sixteen
-                                                     // 19.6 under ncu; more would leave registers for fewer than the four CTAs an SM)
-    float4 x[AHEAD];
+    float4 x[AHEAD];                                 // they do not depend on the chain
     float d[AHEAD];
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u)
@@ -483,7 +482,9 @@ int b2_internal_chunk_tc5(const chunk_tc5::Args& a, void* stream) {
     B2_CUDA_OK(cudaFuncSetAttribute(out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     const int ctas = items < b2_sm_count() ? items : b2_sm_count();
     kv_kernel<<<ctas, NT, SMEM, st>>>(a);
-    state_kernel<<<dim3(n_seq, H, (((dk + 15) & ~15) * dv / 4 + 127) / 128), 128, 0, st>>>(a);
+    const dim3 grid(n_seq, H, (((dk + 15) & ~15) * dv / 4 + 127) / 128);
+    if (long_chains(a, grid.x * grid.y * grid.z)) state_kernel<16><<<grid, 128, 0, st>>>(a);
+    else state_kernel<8><<<grid, 128, 0, st>>>(a);
     out_kernel<<<ctas, NT, SMEM, st>>>(a);
     B2_CUDA_OK(cudaGetLastError());
     return B2_OK;

@@ -270,6 +270,12 @@ struct Args {
     float* carry_out;
 };
 
+// Loads that a thread of a state kernel has in flight: eight (72 registers, seven CTAs an SM), or sixteen (128, four) where the chains are longer than that,
+// but not where eight would keep all CTAs resident and sixteen would not.  Scans of 16 heads of 128 x 128, eight / sixteen: one sequence of 4096 tokens
+// 123.5 / 120.8 us, of 2000 63.9 / 62.7, of 500 33.4 / 34.0; 2 x 4096 229.7 / 239.0, 4 x 2000 214.5 / 211.3, 4 x 200 36.8 / 40.2, 8 x 500 119.8 / 125.8; channel
+// decays 1 x 4096 294.2 / 290.8, 2 x 2048 296.5 / 305.4, 3 x 1000 226.9 / 224.1, 8 x 200 146.2 / 153.1.
+inline bool long_chains(const Args& a, int ctas) { return a.chunks > 9 * a.n_seq && (ctas <= 4 * b2_sm_count() || ctas > 7 * b2_sm_count()); }
+
 // A sequence's chunks in this piece.  What goes on after the piece, and into it, is the one sequence that its border cuts.
 struct Portion {
     int begin, count;                                // first one in the scratch, and how many (0: none)

@@ -577,7 +577,7 @@ chain_kernel(const Args a) {
 }
 
 // Without the correction: element by element, four columns of a row a thread; rows up to the end of a slice are zeros
-template <bool CH>
+template <bool CH, int AHEAD>
 __global__ void __launch_bounds__(128)
 state_kernel(const Args a) {
     const int seq = blockIdx.x, hh = blockIdx.y, dk = a.dk, dv = a.dv;
@@ -594,8 +594,7 @@ state_kernel(const Args a) {
                         tile_at(row & 63, (col & 63) >> 3, 64) + (col & 4) * 2;
     const float* from = pad ? nullptr : state_from(a, part, a.state_slot[seq], hh, a.ctx_start[seq]);
     float4 s = from ? *reinterpret_cast<const float4*>(from + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-    constexpr int AHEAD = 16;                        // loads in flight: they do not depend on the chain (as in chunk_tc5.cu)
-    float4 x[AHEAD];
+    float4 x[AHEAD];                                 // they do not depend on the chain
     float d[AHEAD];
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u)
@@ -756,8 +755,13 @@ int launch(const Args& a, cudaStream_t st) {
     B2_CUDA_OK(cudaFuncSetAttribute(read_kernel<CH, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, READ));
     const int ctas = a.items < b2_sm_count() ? a.items : b2_sm_count();
     wy_kernel<CH, DELTA><<<ctas, 512, WY, st>>>(a);
-    if (DELTA) chain_kernel<CH><<<dim3(L.zs, a.H, a.n_seq), 320, CHAIN, st>>>(a);
-    else state_kernel<CH><<<dim3(a.n_seq, a.H, (L.slices * 64 * a.dv / 4 + 127) / 128), 128, 0, st>>>(a);
+    if constexpr (DELTA) {
+        chain_kernel<CH><<<dim3(L.zs, a.H, a.n_seq), 320, CHAIN, st>>>(a);
+    } else {
+        const dim3 grid(a.n_seq, a.H, (L.slices * 64 * a.dv / 4 + 127) / 128);
+        if (long_chains(a, grid.x * grid.y * grid.z)) state_kernel<CH, 16><<<grid, 128, 0, st>>>(a);
+        else state_kernel<CH, 8><<<grid, 128, 0, st>>>(a);
+    }
     read_kernel<CH, DELTA><<<ctas, 320, READ, st>>>(a);
     B2_CUDA_OK(cudaGetLastError());
     return B2_OK;
