@@ -1020,10 +1020,10 @@ paged_decode_dynamic_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     if (tid == 0) B2_TRACE_AT(x, 0);
     const int gs = (p.B + C::PMAX - 1) / C::PMAX, E = (p.B + gs - 1) / gs;
     const uint32_t Ctot = build_chunk_prefix<NTHREADS>(p.seq_lens, p.B, IPB, ct, gs, E, s_pre);
-    // The claim counter is zeroed by the preceding (tiny) kernel of this call.  Only the producer warp touches
-    // it, and only after its static share, so it orders itself after that kernel (griddepcontrol.wait) right
-    // before its first claim -- and at the latest before it exits, which keeps "this grid finished" =>
-    // "that grid finished" for whatever follows in the stream.
+    // The claim counter is zero before this grid (a plan's, or a KV write that zeroed it on its way: the grid is ordered behind it as usual),
+    // or zeroed by the tiny kernel in front, under which this grid may start.  Only the producer warp touches the counter, and only after
+    // its static share, so it orders itself after that kernel (griddepcontrol.wait, which returns at once in the other case) right before
+    // its first claim -- and at the latest before it exits, which keeps "this grid finished" => "that grid finished" for whatever follows.
     if (Ctot == 0) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         return;
@@ -1453,9 +1453,10 @@ struct Plan {
 };
 
 // num_splits = 0 with block tables too narrow for long rows and all items in one wave: the single-pass grid.  It is one launch (KV
-// write included) and streams a CTA's tokens at about 10.7 ns each behind 3.3 us; the dynamic schedule starts at 9.6 us whatever the
-// batch (write, counter, decode, merge).  Measured with 1 - 32 rows in a graph, single / dynamic, bf16: 4.7 / 10.5 us at 128 tokens,
-// 8.4 / 11.6 at 512, 13.8 / 13.7 at 1024; fp8: 4.9 / 10.2, 7.8 / 11.7, 12.5 / 13.5.  Launched one by one 20 / 29 at 512.
+// write included) and streams a CTA's tokens at about 10.7 ns each behind 3.6 us; the dynamic schedule starts at 11.5 us (write, which zeroes
+// the counter, decode, merge).  With the write, in a graph, 32 heads on 8, one row, single / dynamic: bf16 5.0 / 11.6 us at 128 tokens, 9.0 / 11.7
+// at 512, 10.5 / 11.8 at 640, 11.8 / 11.8 at 768, 14.6 / 12.5 at 1024; fp8 5.4 / 11.6, 8.2 / 11.6, 9.4 / 11.8, 10.6 / 12.0, 13.1 / 12.3.  More rows put
+// the point where they meet further out: 8 rows of 640 11.1 / 18.1, of 1024 15.1 / 19.6; 32 of 640 13.6 / 27.8, of 1024 22.1 / 36.5.
 constexpr int SHORT_ROW_TOKENS = 640;
 bool short_rows(int64_t B, int ipb, int bs, int max_nb) { return (int64_t)max_nb * bs <= SHORT_ROW_TOKENS && B * ipb <= 2 * (int64_t)sm_count(); }
 
