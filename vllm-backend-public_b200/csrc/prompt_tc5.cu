@@ -19,8 +19,8 @@
 // score would need two more XU operations (the exponential and the division of tanh): where a whole warp's scores are below 3/16
 // of the cap, tanh is its Taylor polynomial to x^7 on the packed FMA pipe instead (remainder below 7e-9; the exponential form's
 // error is one fp32 rounding, 6e-8).
-// Measured in a graph with the kernels around it: 300 rows x 16 heads of 128, window 500: 15 us; 1000 rows 22; 1200 gathered rows x 16 heads of
-// 128 + 64 / 128, causal, 41.  A step of 128 keys is the softmax of the tile (0.5k cycles for the maximum, 0.6k to bring O along, 1.4k for the
+// Attention alone in a graph: 300 rows x 16 heads of 128 on 4 kv heads, causal, 12.9 us; 1000 rows 23.3; 1200 gathered rows x 16 heads of
+// 128 + 64 / 128, causal, 24.4 (25.4 with one V stage, which the second slot's Q once cost the form of one).  A step of 128 keys is the softmax of the tile (0.5k cycles for the maximum, 0.6k to bring O along, 1.4k for the
 // weights) and the MMAs behind it, one after the other.
 // What cost most on the way: code size (95 - 145 KB with everything unrolled: every warp waited for instructions, 10.9k cycles per
 // tile; loops are rolled wherever registers are not indexed), and a divergent branch per row in the copies (~100 cycles an
@@ -36,12 +36,13 @@ using namespace b2prompt;
 
 constexpr int NTHREADS = 384;
 
-// NH: 64-column sub-tiles of a slot's Q and K; DVH: of V.  Three sub-tiles of K leave room for one V stage beside two of K.
-template <int NH, int DVH, bool TWO_MAPS>
+// NH: 64-column sub-tiles of a slot's Q and K; DVH: of V.  Three sub-tiles of two slots leave room for one V stage beside two of K.
+template <int NH, int DVH, bool TWO_MAPS, bool PAIRS>
 struct Shape {
-    static constexpr int VST = NH <= 2 ? 2 : 1, KST = 2;
+    static constexpr int SLOTS = TWO_MAPS || PAIRS ? 2 : 1;
+    static constexpr int VST = SLOTS * NH <= 4 ? 2 : 1, KST = 2;
     static constexpr int KSUBS = TWO_MAPS ? 2 : NH;
-    static constexpr int Q_BYTES = 2 * NH * SUB, K_STAGE = KSUBS * SUB, V_STAGE = DVH * SUB;
+    static constexpr int Q_BYTES = SLOTS * NH * SUB, K_STAGE = KSUBS * SUB, V_STAGE = DVH * SUB;
     static constexpr int BAR_Q = 0, BAR_K = 1, BAR_V = BAR_K + KST, BAR_KE = BAR_V + VST, BAR_VE = BAR_KE + KST, BAR_S = BAR_VE + VST,
                          BAR_P = BAR_S + 2, BAR_P2 = BAR_P + 2, BAR_PV = BAR_P2 + 2, BAR_END = BAR_PV + 2, BARS = BAR_END + 1;
     static constexpr int SMEM = Q_BYTES + KST * K_STAGE + VST * V_STAGE + 256;
@@ -78,7 +79,7 @@ struct Plan {
 template <int NH, int DVH, int KIND, bool TWO_MAPS, bool GATHERED, bool PAIRS>
 __global__ void __launch_bounds__(NTHREADS, 1)
 prompt_tc5_kernel(const __grid_constant__ Params prm) {
-    using L = Shape<NH, DVH, TWO_MAPS>;
+    using L = Shape<NH, DVH, TWO_MAPS, PAIRS>;
     using bf16 = __nv_bfloat16;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     __shared__ Plan s_plan;
@@ -612,9 +613,12 @@ prompt_tc5_kernel(const __grid_constant__ Params prm) {
 template <int NH, int DVH, int KIND, bool TWO_MAPS, bool GATHERED>
 int launch(const Params& p, dim3 grid, cudaStream_t st) {
     auto kern = prompt_tc5_kernel<NH, DVH, KIND, TWO_MAPS, GATHERED, false>;
+    int smem = Shape<NH, DVH, TWO_MAPS, false>::SMEM;
     if constexpr (!TWO_MAPS)
-        if (p.rows_per_cta > BM || p.heads_per_cta > 1) kern = prompt_tc5_kernel<NH, DVH, KIND, TWO_MAPS, GATHERED, true>;
-    constexpr int smem = Shape<NH, DVH, TWO_MAPS>::SMEM;
+        if (p.rows_per_cta > BM || p.heads_per_cta > 1) {
+            kern = prompt_tc5_kernel<NH, DVH, KIND, TWO_MAPS, GATHERED, true>;
+            smem = Shape<NH, DVH, TWO_MAPS, true>::SMEM;
+        }
     B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     kern<<<grid, NTHREADS, smem, st>>>(p);
     B2_CUDA_OK(cudaGetLastError());

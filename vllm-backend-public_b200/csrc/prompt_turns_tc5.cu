@@ -23,11 +23,14 @@
 // row's largest capped score is that of its largest score and needs no pass.
 // Measured with clock64, 128 keys x two slots: 3.3 - 3.9k cycles with heads of 192 / 128 (softmax 0.5k for the maximum and 1.5 - 2k for the
 // weights, then the P V of its last 64 keys and the next Q K^T one after another, 1.3k), 4.4k with capped scores.
-// A CTA a tile needed 9k cycles to its first scores and 5k to write its rows, and took tiles in the order of the rows: with 16 heads of
-// 128 + 64 / 128 and 4096 ragged causal rows the SMs ended between 29 and 56 us.  Here, in a graph with the kernels around it: 4096 rows x 32 heads
-// of 128, window 1024, capped 153 -> 140 us; those causal rows 96 -> 87; 2500 rows x 16 heads of two maps 55 -> 47; 2000 gathered rows x 32 heads in
-// windows of 300 101 -> 91.
-// What is left of the first steps is fetching code, 12k cycles to the first scores: launches of a tile a CTA are prompt_tc5.cu's.
+// A CTA a tile needs 7.5 - 9k cycles to its first scores and 5k to write its rows, and takes tiles in the order of the rows: with 16 heads of
+// 128 + 64 / 128 and 4096 ragged causal rows the SMs ended between 29 and 56 us.  Attention alone in a graph, a CTA a tile -> here: 4096 rows x 32
+// heads of 128, window 1024, capped 122 -> 107 us, not capped 93.6 -> 77.2; those causal rows 52.8 -> 42.6; 4 x 625 rows x 16 heads of two maps 37.0 ->
+// 30.2; 3500 gathered rows x 16 heads in windows of 300 39.0 -> 34.5; 1000 rows x 32 heads of sigmoid weights 30.8 -> 22.6.
+// What is left of the first steps is fetching code, 9 - 12k cycles to the first scores: which launches are prompt_tc5.cu's, and why, stands there.
+// Mask blocks are walked from their beginning, so their tiles are not in the order of their length: 1424 + 991 rows x 16 behind 777 in blocks of 589 take
+// 36.8 us and 30.0 with a CTA a tile, other sizes (830 + 577 + 817, blocks of 510) 23.0 and 26.7.
+// The forms of two maps spill 12 - 60 bytes a thread, the others nothing.
 // What cost most on the way: an MMA loop with the slot as a variable, whose operands are not uniform to the compiler (3.6k cycles between a
 // softmax and the next instead of 1.3k); the weights in a rolled loop over 32 keys (2.3k cycles instead of 1.5k); stores by a thread a row
 // (32 lines each) and gates per column in the same kernel (10k cycles a tile's output instead of 3k).
