@@ -1,15 +1,15 @@
 #!/usr/bin/env python
-"""bench.py -- paged-attention decode on B200: achieved HBM GB/s on BASELINE.json's headline config.
+"""bench.py -- paged-attention decode on B200: achieved HBM GB/s on the headline configuration.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference] [--workload NAME]
 
 One "step" = one pass of the hot path over one decode batch of one layer:
     reshape_and_cache (the step's new K/V token of every sequence)  ->  paged_decode.
-Workload at N = 1 (BASELINE.json configs[1], the configuration the metric is quoted on):
+Workload at N = 1 (the configuration the metric is quoted on):
     Llama-3-8B attention geometry, 32 q / 8 kv heads, d = 128, block_size 16, batch 64, ctx 4096, bf16 KV.
 At N > 1 (torchrun, one rank per GPU, NCCL only for the timing barrier) the KV heads are sharded over the
 ranks and the batch grows with N (global batch 64*N), so per-GPU work is fixed: "scaling": "weak".  There is
-no collective on the data path (SURVEY.md section 8(e)).
+no collective on the data path.
 
 Printed on rank 0: ONE JSON line (see the keys below).  `value` is whole-job GB/s with every input resident
 in HBM; `e2e` is the same metric through the public API with HOST (pinned) buffers, H2D/D2H copies inside
@@ -40,18 +40,18 @@ NOMINAL_HBM_GBS = 8000.0
 
 WORKLOADS = {
     # name: (B per GPU-equivalent, Hq, Hkv, ctx, kv dtype)
-    "llama3-8b_b64_ctx4k_bf16kv": dict(B=64, Hq=32, Hkv=8, ctx=4096, fp8=False),
-    "llama3-8b_b128_ctx8k_fp8kv": dict(B=128, Hq=32, Hkv=8, ctx=8192, fp8=True),
-    "llama3-70b_b256_ctx8k_bf16kv": dict(B=256, Hq=64, Hkv=8, ctx=8192, fp8=False),
-    "oracle_b4_ctx512": dict(B=4, Hq=8, Hkv=2, ctx=512, fp8=False),
-    "llama3-70b_tp8_shard": dict(B=256, Hq=8, Hkv=1, ctx=8192, fp8=False),           # one rank's share of configs[3] at tp = 8
+    "llama3-8b_b64_ctx4k_bf16kv": dict(B=64, Hq=32, Hkv=8, ctx=4096, fp8=False),     # the headline
+    "llama3-8b_b128_ctx8k_fp8kv": dict(B=128, Hq=32, Hkv=8, ctx=8192, fp8=True),     # long fp8
+    "llama3-70b_b256_ctx8k_bf16kv": dict(B=256, Hq=64, Hkv=8, ctx=8192, fp8=False),  # 70B
+    "oracle_b4_ctx512": dict(B=4, Hq=8, Hkv=2, ctx=512, fp8=False),                 # the oracle's
+    "llama3-70b_tp8_shard": dict(B=256, Hq=8, Hkv=1, ctx=8192, fp8=False),           # one rank's share at tp = 8
 }
 D = 128
-BS = int(os.environ.get("B2_BENCH_BLOCK_SIZE", "16"))   # BASELINE fixes 16; other sizes are experiments only
+BS = int(os.environ.get("B2_BENCH_BLOCK_SIZE", "16"))   # the metric fixes 16; other sizes are experiments only
 
 
 def algorithmic_bytes(B, Hq, Hkv, ctx, kv_bytes):
-    """SURVEY.md section 8(d): K+V read once, q read, out written, block table, seq_lens."""
+    """K+V read once, q read, out written, block table, seq_lens."""
     nb = (ctx + BS - 1) // BS
     return B * ctx * 2 * Hkv * D * kv_bytes + 2 * B * Hq * D * 2 + B * nb * 4 + B * 4
 
@@ -132,7 +132,7 @@ def physical_gpu_index(local_rank: int) -> int:
 
 
 # --------------------------------------------------------------------------------------------
-# synthetic problem (device-side generation; SURVEY.md section 8(d))
+# synthetic problem (device-side generation)
 # --------------------------------------------------------------------------------------------
 def _seq_gen(dev, seed, b):
     return torch.Generator(device=dev).manual_seed(seed * 1000003 + b)
@@ -392,7 +392,7 @@ def committed_traffic(wl_name, B, Hq_l, Hkv_l):
 
 
 def sub_config_record(dev, name, K, W, splits_arg):
-    """One more BASELINE config measured the same way as the headline (device-resident steps, CUDA events): the
+    """One more configuration measured the same way as the headline (device-resident steps, CUDA events): the
     record that goes under `configs` in the JSON line."""
     wl = WORKLOADS[name]
     prob = build_problem(dev, wl["B"], wl["Hq"], wl["Hkv"], wl["ctx"], wl["fp8"], seed=0)
@@ -419,7 +419,7 @@ def sub_config_record(dev, name, K, W, splits_arg):
 def sharded_parity_check(dev, dist, rank, wl, shard, out_local, seed, n_rows=8, n_oracle=4):
     """The head-sharded result, gathered once (outside every timed region), against (1) rank 0 running the UNSHARDED
     problem (all heads, b2_paged_decode) on a slice of the batch and (2) the CPU oracle on some of those rows.
-    Rows: first, last and random ones.  Bound: |d| <= 2e-3 + 1e-2 |ref| (north_star, bf16 KV)."""
+    Rows: first, last and random ones.  Bound: |d| <= 2e-3 + 1e-2 |ref| (bf16 KV)."""
     import b200attn
     from b200attn import parallel
     B, Hq, Hkv, ctx = wl["B"], wl["Hq"], wl["Hkv"], wl["ctx"]
@@ -485,7 +485,7 @@ def run_ours(args, wl_name, wl):
     if wl["Hkv"] % tp:
         raise SystemExit(f"Hkv={wl['Hkv']} is not divisible by tp={tp}")
     # KV-head sharding, weak scaling: rank r owns kv heads [r*Hkv/tp, (r+1)*Hkv/tp) of a batch of B*tp sequences
-    # (--strong keeps the batch fixed instead: BASELINE configs[3], B = 256 sharded over tp = 2/4/8)
+    # (--strong keeps the batch fixed instead: B = 256 sharded over tp = 2/4/8)
     from b200attn import parallel
     shard = parallel.HeadShard(tp, rank, wl["Hq"], wl["Hkv"])
     B = wl["B"] if args.strong else wl["B"] * tp
@@ -495,7 +495,7 @@ def run_ours(args, wl_name, wl):
     prob = build_problem(dev, B, wl["Hq"], wl["Hkv"], ctx, fp8, seed=0, shard=shard)
     bytes_rank = algorithmic_bytes(B, Hq_l, Hkv_l, ctx, kv_bytes)
     if args.ragged:
-        # experiment (not a BASELINE config): sequence lengths log-uniform in [128, ctx], the shape of a serving batch
+        # experiment: sequence lengths log-uniform in [128, ctx], the shape of a serving batch
         g = torch.Generator().manual_seed(1234)
         lens = torch.exp(torch.empty(B).uniform_(math.log(128.0), math.log(float(ctx)), generator=g)).to(torch.int32)
         lens = lens.clamp_(128, ctx)
@@ -618,7 +618,7 @@ def run_ours(args, wl_name, wl):
     del prob, out
     torch.cuda.empty_cache()
 
-    # ---------------- the other BASELINE configs, the model-level half of the metric, the comparator (N = 1) ----------
+    # ---------------- the other configurations, the model-level half of the metric, the comparator (N = 1) ----------
     extras = not args.lean and not args.ragged and wl_name == "llama3-8b_b64_ctx4k_bf16kv"
     if extras and world == 1:
         import bench_legs
@@ -632,7 +632,7 @@ def run_ours(args, wl_name, wl):
         line["comparator"] = bench_legs.comparator_leg()
         line["decode_tok_s"] = bench_legs.decode_tok_s_leg(dev, steps=max(20, min(K, 100)))
 
-    # ---------------- BASELINE configs[3], strong scaling over the ranks + sharded-vs-unsharded parity (N > 1) --------
+    # ---------------- B = 256, 64 q heads, strong scaling over the ranks + sharded-vs-unsharded parity (N > 1) --------
     if extras and world > 1:
         wl4 = WORKLOADS["llama3-70b_b256_ctx8k_bf16kv"]
         sh4 = parallel.HeadShard(tp, rank, wl4["Hq"], wl4["Hkv"])
@@ -704,7 +704,7 @@ def main():
                     help="num_splits for b2_paged_decode: -1 = host planner (default), 0 = dynamic persistent, 1 = single pass")
     ap.add_argument("--no-cpu", action="store_true", help="skip the cpu_baseline leg")
     ap.add_argument("--lean", action="store_true",
-                    help="headline leg only: skip the sub-records (other BASELINE configs, decode tok/s, comparator, "
+                    help="headline leg only: skip the sub-records (other configurations, decode tok/s, comparator, "
                          "strong scaling + sharded parity)")
     ap.add_argument("--strong", action="store_true", help="N > 1: keep the global batch fixed (strong scaling)")
     ap.add_argument("--batch", type=int, default=0, help="override the workload batch size (experiments only)")

@@ -1,9 +1,9 @@
 """Secondary legs of bench.py (and scripts/bench_model.py): measurements that ride along in the one JSON line.
 
-  decode_tok_s_leg   the model-level half of BASELINE.json's metric: whole-model decode tok/s, Llama-3-8B geometry,
+  decode_tok_s_leg   the model-level half of the metric: whole-model decode tok/s, Llama-3-8B geometry,
                      batch 64, ctx 4096, random-init weights, through b200attn.engine.LLMEngine (C++ scheduler,
                      CUDA-graph decode steps), with its weights + KV HBM roofline.
-  comparator_leg     the same-box comparator BASELINE.md section 4 plans: the paged-decode kernels of the vLLM /
+  comparator_leg     the same-box comparator: the paged-decode kernels of the vLLM /
                      flash-attn / flashinfer wheels that happen to be in this image, timed on the same seeded problem.
                      Runs in a SUBPROCESS (scripts/comparator.py) with a time limit: those imports log to stdout, may
                      JIT-compile, and must never be able to break or pollute the bench line.  Absent wheel, import
@@ -114,7 +114,7 @@ def decode_tok_s_leg(dev, model: str = "llama-3-8b", B: int = 64, ctx: int = 409
 
 
 def comparator_leg(timeout_s: int = 420) -> dict:
-    """vLLM paged_attention_v2 / flash_attn_with_kvcache / flashinfer decode on BASELINE configs 2 and 3, same box.
+    """vLLM paged_attention_v2 / flash_attn_with_kvcache / flashinfer decode on the headline and the fp8 configuration, same box.
     See scripts/comparator.py; this function only runs it under a time limit and reads its JSON."""
     script = ROOT / "scripts" / "comparator.py"
     if os.environ.get("B2_BENCH_COMPARATOR", "1") != "1":

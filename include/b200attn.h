@@ -1,7 +1,7 @@
 /*
  * b200attn.h -- C ABI of libb200attn.so: the B200 (sm_100a) paged-attention decode backend.
  *
- * This is the drop-in boundary "b2" of SURVEY.md section 8(b).  The reference
+ * This is the drop-in boundary below the engine.  The reference
  * (ThakiCloud/vllm-backend-public) has no FFI for this path -- it launches an external vLLM
  * server process (reference benchmark-vllm/vllm_manager.py:371-374,744-773) and never sees
  * the kernels -- so every entry point below cites (a) the vLLM operation an engine behind that
@@ -164,7 +164,7 @@ B2_API int b2_paged_decode_append(void* out, const void* q,
                            void* stream);
 
 /* b2_paged_decode for callers that may not allocate: code under CUDA graph capture, tight serving loops, harnesses
- * that forbid cudaMalloc.  No counterpart in the reference; added at the request of the run's operators.
+ * that forbid cudaMalloc.  No counterpart in the reference.
  * Same operation, arguments and results as b2_paged_decode, minus the workspace: the split-K partials and the claim
  * counter live in a file-scope device array of B2_STATIC_SCRATCH_BYTES inside the library (every GPU that loads the
  * library holds it until exit).  The call allocates nothing (no cudaMalloc / cudaFree, no allocating library routine).
@@ -218,7 +218,7 @@ B2_API int b2_decode_plan_run_append(b2_decode_plan* plan, void* out, const void
                               int32_t* block_tables, const int32_t* seq_lens, int B,
                               int64_t q_stride, int64_t out_stride, int num_splits, void* stream);
 
-/* Diagnostic / A-B variant kept for the ncu comparison DESIGN.md cites: the same contract as
+/* Diagnostic / A-B variant kept for the ncu comparison in profiles/: the same contract as
  * b2_paged_decode, computed by a plain CUDA-core kernel (no TMA, no tensor cores).  Not used by
  * the engine. */
 B2_API int b2_paged_decode_simt(void* out, const void* q,
@@ -232,7 +232,7 @@ B2_API int b2_paged_decode_simt(void* out, const void* q,
                          void* stream);
 
 /* ---------------------------------------------------------------------------------------------
- * Prompt-chunk (prefill) attention over the paged cache (SURVEY.md section 8(f) rank 2).  Replaces vLLM's
+ * Prompt-chunk (prefill) attention over the paged cache.  Replaces vLLM's
  * chunked-prefill / prefix attention (flash_attn_varlen_func with a block table, `context_attention_fwd`) in the
  * engine behind the reference's launch contract; chunk sizes follow the scheduler's token budget, table rows
  * max_nb = ceil(max_model_len / block_size) (reference benchmark-vllm/models.py:15,10).
@@ -266,7 +266,7 @@ B2_API int b2_dequant_kv_blocks(void* k_out, void* v_out, const void* k_cache, c
                          int64_t cache_block_stride, int64_t cache_head_stride, void* stream);
 
 /* ---------------------------------------------------------------------------------------------
- * Element-wise ops of one decoder layer around the attention path (SURVEY.md section 8(f) rank 3): what the
+ * Element-wise ops of one decoder layer around the attention path: what the
  * launched engine runs between its GEMMs.  bf16 activations (VLLMConfig.dtype, reference
  * benchmark-vllm/models.py:14), fp32 math, one rounding on the way out; strides in elements.
  *
@@ -349,7 +349,7 @@ B2_API int     b2_bm_plan_decode(b2_block_manager* bm, const int64_t* seq_ids, i
                           int64_t* slot_mapping_out);
 
 /* ---------------------------------------------------------------------------------------------
- * Continuous-batching scheduler (host only; SURVEY.md section 8(f) rank 1): the caller of the hot path.
+ * Continuous-batching scheduler (host only): the caller of the hot path.
  * It owns a block manager and turns a stream of requests into per-step plans under the limits of the
  * reference's launch contract: max_num_seqs (models.py:9), max_model_len (:15), block_size (:10), the block
  * pool sized from gpu_memory_utilization (:8), plus a per-step token budget for chunked prefill.

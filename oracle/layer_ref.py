@@ -1,4 +1,4 @@
-"""CPU oracle for the rows either side of the decode hot path (SURVEY.md section 8(f) ranks 2-3):
+"""CPU oracle for the rows either side of the decode hot path:
 prompt-chunk attention over the paged cache, RMSNorm, SwiGLU, rotary + KV write, token choice, and a whole
 random-init Llama forward built from them.  TEST INFRASTRUCTURE ONLY.
 

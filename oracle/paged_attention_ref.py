@@ -8,7 +8,7 @@
     benchmark-vllm/vllm_templates.py:124).  vLLM is not vendored under /root/reference,
     so this file restates vLLM's *published* paged-attention semantics (v0.9.1
     `csrc/cache_kernels.cu::reshape_and_cache`, `csrc/attention/attention_kernels.cuh`)
-    in plain fp32 PyTorch, as BASELINE.json's north_star prescribes.  The parameters
+    in plain fp32 PyTorch, an oracle that shares no code with the kernels.  The parameters
     that shape it do come from the reference: `block_size` (benchmark-vllm/models.py:10),
     `max_num_seqs` / `max_model_len` (models.py:9,15), `tensor_parallel_size`
     (models.py:11), `dtype` (models.py:14).
@@ -23,7 +23,7 @@ Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl refere
 may import this module -- as the oracle or the timed CPU baseline, never as a product
 path.  The product (`b200attn`) has no CPU fallback and never imports it.
 
-Semantics (SURVEY.md section 8(a), rows a5-a8):
+Semantics:
   * slot -> (block, offset) = (slot // bs, slot % bs); slot < 0 means "skip this token".
   * caches are [num_blocks, Hkv, bs, d]; bf16, or uint8 holding e4m3 bit patterns.
   * GQA: q head hq reads kv head hq // (Hq // Hkv).
@@ -220,7 +220,7 @@ def paged_decode_partitioned_ref(
 
 
 # --------------------------------------------------------------------------------------
-# Seeded synthetic inputs (SURVEY.md section 8(d)).  Pure CPU; used by tests and bench.
+# Seeded synthetic inputs.  Pure CPU; used by tests and bench.
 # --------------------------------------------------------------------------------------
 def make_inputs(
     B: int, Hq: int, Hkv: int, d: int, bs: int, ctx: int,
@@ -257,7 +257,7 @@ def make_inputs(
 
 
 def algorithmic_bytes(B: int, Hq: int, Hkv: int, d: int, bs: int, seq_lens, kv_bytes: int) -> int:
-    """SURVEY.md section 8(d): K+V read once, q read, out written, block table, seq_lens."""
+    """K+V read once, q read, out written, block table, seq_lens."""
     total = 0
     for L in seq_lens:
         L = int(L)

@@ -1,6 +1,6 @@
-"""Measurements for the rows next to the hot path (SURVEY.md section 8(f)), one JSON line each:
+"""Measurements for the rows next to the hot path, one JSON line each:
   prefill attention TFLOP/s (Llama-3-8B heads, 8k-token chunks at several prefix lengths), element-wise ops GB/s,
-  whole-model decode tok/s at Llama-3-8B b64 ctx4k (BASELINE.json's second headline figure; roofline = weights + KV bytes).
+  whole-model decode tok/s at Llama-3-8B b64 ctx4k (the second headline figure; roofline = weights + KV bytes).
     python scripts/bench_model.py [--skip-model] > out/bench_model.jsonl
 CUDA events on the launching stream, >= 3 warm-ups, inputs larger than L2 or L2 flushed (said per line)."""
 import argparse

@@ -1,4 +1,4 @@
-"""Same-box comparator (BASELINE.md section 4): the paged-decode kernels of the wheels that happen to be in this image,
+"""Same-box comparator: the paged-decode kernels of the wheels that happen to be in this image,
 timed on the same seeded problems as bench.py, beside this repo's kernel.  Not the reference's pinned vLLM v0.9.1 image
 (reference benchmark-vllm/vllm_manager.py:371-374) -- the closest thing to "the kernel the launched engine would run"
 that can execute here.  Run by bench_legs.comparator_leg() in a subprocess; writes one JSON file, rewritten after every

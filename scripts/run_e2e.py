@@ -1,5 +1,5 @@
-"""random-init Llama-3-8B behind the OpenAI endpoint on port 8005, driven by the load generator
-(mixed prompt lengths 128-32k, log-uniform, seed 0).  Usage (on the GPU box):
+"""Random-init Llama-3-8B behind the OpenAI endpoint on port 8005, driven by the load generator
+(mixed prompt lengths 128-32k, log-uniform, seed 0).  Usage (on a machine with a B200):
     python scripts/run_e2e.py [--num-requests 256] [--concurrency 64] [--max-tokens 128] [--model llama-3.1-8b] [--tag x]
 The client is the evaluation Job of the reference's loop: b200attn/templates/evaluate.yaml rendered by the
 process_template rule (reference benchmark-eval/main.py:55-58,113) for this model and engine URL, and the Job's

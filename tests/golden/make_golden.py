@@ -1,7 +1,7 @@
-"""Regenerates tests/golden/config1.json + config1_out.pt from the oracle (
+"""Regenerates tests/golden/config1.json + config1_out.pt from the oracle (the oracle configuration:
 8 q / 2 kv heads, head_dim 128, block_size 16, batch 4, ctx 512).  The reference repository has no
 implementation or vectors for this path, so the fixture is the oracle's own frozen output; it is
-cross-checked on the GPU box against the vLLM wheel's paged_attention_v1 by
+cross-checked on a B200 against the vLLM wheel's paged_attention_v1 by
 tests/golden/make_vllm_crosscheck.py when that wheel loads there."""
 import hashlib
 import json

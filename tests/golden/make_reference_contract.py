@@ -1,5 +1,5 @@
 """Generates tests/golden/reference_contract.json by IMPORTING the reference's own Python modules from
-/root/reference (read-only, in this container only; it does not exist on the GPU box):
+/root/reference (read-only):
 
   * benchmark-vllm/models.py::VLLMConfig parsed from every benchmark-vllm/configs/*.yaml
   * benchmark-vllm/vllm_templates.py::create_vllm_deployment_template / _statefulset_template -> container args

@@ -1,4 +1,4 @@
-"""Pin the oracle against vLLM's own CUDA kernels (run on the GPU box; the wheel in the image is vllm 0.22).
+"""Pin the oracle against vLLM's own CUDA kernels (run on a machine with a B200; written against vllm 0.22).
 
 The reference launches vLLM as an external server (`vllm/vllm-openai:v0.9.1`,
 reference benchmark-vllm/vllm_manager.py:371-374) and holds no vectors for this path.  vLLM is the dependency whose
@@ -33,7 +33,7 @@ CASES = {
     "ragged_b16_hq32_hkv8_ctx700": (dict(B=16, Hq=32, Hkv=8, d=128, bs=16, ctx=700, seed=3, ragged=True), False),
     "ragged_b8_hq64_hkv8_ctx1100": (dict(B=8, Hq=64, Hkv=8, d=128, bs=16, ctx=1100, seed=5, ragged=True), False),
     "fp8_b8_hq32_hkv8_ctx600": (dict(B=8, Hq=32, Hkv=8, d=128, bs=16, ctx=600, seed=4, ragged=True), True),
-    # r2 (VERDICT r1 "the vLLM pin is thin"): other block sizes, contexts long enough that v2 really partitions
+    # other block sizes, contexts long enough that v2 really partitions
     # (512-token partitions), G = 1 and G = 16, single-token sequences, a long fp8 case
     "bs8_b6_hq8_hkv2_ctx300": (dict(B=6, Hq=8, Hkv=2, d=128, bs=8, ctx=300, seed=6, ragged=True), False),
     "bs32_b6_hq32_hkv8_ctx900": (dict(B=6, Hq=32, Hkv=8, d=128, bs=32, ctx=900, seed=7, ragged=True), False),

@@ -64,7 +64,7 @@ def test_argument_validation_without_gpu():
 
 
 def test_workspace_bound_is_monotone_in_batch():
-    """the automatic schedule cuts smaller batches into finer chunks, so the bytes ONE batch size
+    """The automatic schedule cuts smaller batches into finer chunks, so the bytes ONE batch size
     needs are not monotone in B (B=24 needed more than B=32 at max_nb 512).  The exported size must serve every
     batch 1..B, i.e. never shrink as B grows -- an engine sizes the workspace once for max_num_seqs and captures CUDA
     graphs for every smaller bucket against that one buffer."""

@@ -1,4 +1,4 @@
-"""GPU parity for the rows either side of the decode path (SURVEY.md section 8(f) ranks 2-3), through the C ABI:
+"""GPU parity for the rows either side of the decode path, through the C ABI:
 prompt-chunk attention over the paged cache, RMSNorm (+ fused residual add), SwiGLU, rotary + KV write, token choice.
 
 Bars (written here because the north star only states the decode bound):

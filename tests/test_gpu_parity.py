@@ -1,12 +1,12 @@
 """GPU parity tests proper: the sm_100a kernels, called through the C ABI (ctypes ->
 libb200attn.so), against the CPU oracle on the same seeded inputs.
 
-Bars (BASELINE.json north_star):
+Bars:
   * reshape_and_cache: bit-exact.
   * decode, bf16 KV: |delta| <= 2e-3 + 1e-2 * |ref|.
   * decode, fp8 KV vs the oracle reading the *same quantised cache*: same bound; vs the
     unquantised oracle the looser stated bound 5e-2 + 1e-1 * |ref| (quantisation error).
-At BASELINE.json's full sizes the oracle is run on a subset of sequences and the rest is covered
+At the benchmark's full sizes the oracle is run on a subset of sequences and the rest is covered
 by size-independent properties (split-count invariance, block-table permutation invariance,
 agreement of two independent kernels)."""
 import json
@@ -133,7 +133,7 @@ def run_decode(inp, kc, vc, dev, **kw):
 
 @pytest.mark.parametrize("impl,splits", [("tma", 1), ("tma", 2), ("tma", 0), ("tma", 7), ("simt", 1)])
 def test_decode_config1(cuda, impl, splits):
-    """8 q / 2 kv heads, d 128, bs 16, batch 4, ctx 512."""
+    """The oracle configuration: 8 q / 2 kv heads, d 128, bs 16, batch 4, ctx 512."""
     inp = R.make_inputs(4, 8, 2, 128, 16, 512, seed=0)
     kc, vc, kc_ref, vc_ref, _ = build_caches(inp, cuda)
     ref = R.paged_decode_ref(inp["q"], kc_ref, vc_ref, inp["block_tables"], inp["seq_lens"], return_f32=True)
@@ -336,22 +336,22 @@ def _full_size(cuda, B, Hq, Hkv, ctx, fp8, seed, n_oracle=8):
 
 
 def test_full_size_config2_llama3_8b_b64_ctx4k(cuda):
-    """32 q / 8 kv heads, batch 64, ctx 4096, bf16 KV."""
+    """The headline: 32 q / 8 kv heads, batch 64, ctx 4096, bf16 KV."""
     _full_size(cuda, 64, 32, 8, 4096, fp8=False, seed=0)
 
 
 def test_full_size_config3_fp8_b128_ctx8k(cuda):
-    """BASELINE.json configs[2]: fp8 e4m3 KV, batch 128, ctx 8192."""
+    """fp8 e4m3 KV, batch 128, ctx 8192."""
     _full_size(cuda, 128, 32, 8, 8192, fp8=True, seed=1)
 
 
 def test_full_size_config4_per_gpu_shard_tp8(cuda):
-    """BASELINE.json configs[3] as seen by one of 8 ranks: 8 q / 1 kv head, batch 256, ctx 8192."""
+    """A 70B model as seen by one of 8 ranks: 8 q / 1 kv head, batch 256, ctx 8192."""
     _full_size(cuda, 256, 8, 1, 8192, fp8=False, seed=2)
 
 
 def test_full_size_config4_tp1_llama3_70b_b256_ctx8k(cuda):
-    """BASELINE.json configs[3] unsharded: 64 q / 8 kv heads (G = 8), batch 256, ctx 8192, bf16 KV -- 8.6 GB of cache.
+    """A 70B model unsharded: 64 q / 8 kv heads (G = 8), batch 256, ctx 8192, bf16 KV -- 8.6 GB of cache.
     The problem is generated on the device (bench.build_problem: per-sequence seeds); the oracle regenerates the tokens
     of 8 rows (first, last, random), builds its own cache from them and is compared on the KV bits and on the output."""
     import bench
@@ -574,7 +574,7 @@ def test_decode_two_box_fallback_map_dynamic_schedule(cuda, monkeypatch):
 
 
 def test_workspace_for_max_batch_serves_every_smaller_batch(cuda):
-    """one workspace sized for max_num_seqs = 32 at max_model_len 8192 must be accepted by every
+    """One workspace sized for max_num_seqs = 32 at max_model_len 8192 must be accepted by every
     batch size below it under the dynamic schedule (B = 24 needs more partial slots than B = 32)."""
     Hq, Hkv, bs, max_nb = 32, 8, 16, 512
     ws = torch.empty(b200attn.decode_workspace_bytes(32, Hq, Hkv, 128, bs, max_nb, 0), dtype=torch.uint8, device=cuda)

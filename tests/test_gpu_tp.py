@@ -1,6 +1,6 @@
 """GPU (>= 2 devices): the served engine at --tensor-parallel-size 2 (reference benchmark-vllm/models.py:11,
 vllm_templates.py:55) -- one process per GPU under torchrun, teacher-forcing parity against the dense CPU oracle.
-Skipped on a single-GPU box; bench.py --gpus N runs the same check (`tp_serving.parity`) where the driver sees it."""
+Skipped with one GPU; bench.py --gpus N runs the same check (`tp_serving.parity`)."""
 import json
 import subprocess
 import sys

@@ -148,7 +148,7 @@ def test_fp8_cache_decode_close_to_unquantised():
 
 
 def test_algorithmic_bytes_matches_baseline_md():
-    # BASELINE.md section 3
+    # the headline's algorithmic bytes
     assert R.algorithmic_bytes(4, 8, 2, 128, 16, [512] * 4, 2) == 2_114_064
     assert R.algorithmic_bytes(64, 32, 8, 128, 16, [4096] * 64, 2) == 1_074_856_192
     assert R.algorithmic_bytes(128, 32, 8, 128, 16, [8192] * 128, 1) == 2_149_843_456

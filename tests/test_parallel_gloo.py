@@ -1,4 +1,4 @@
-"""KV-head sharding (SURVEY.md section 8(e)) on CPU: world_size-2 and -4 gloo groups.
+"""KV-head sharding on CPU: world_size-2 and -4 gloo groups.
 
 Each rank owns Hkv/tp kv heads and the q heads that read them; block tables / seq_lens / slots are replicated.
 The ranks compute their heads with the CPU oracle (stand-in for the CUDA kernel, which needs a GPU), then
@@ -69,7 +69,7 @@ def test_head_sharding_gather_matches_unsharded(world):
 def test_shard_arithmetic():
     sys.path.insert(0, str(ROOT / "vllm-backend-public_b200"))
     from b200attn.parallel import HeadShard
-    s = HeadShard(8, 3, 64, 8)                       # BASELINE configs[3] at tp = 8
+    s = HeadShard(8, 3, 64, 8)                       # 64 q / 8 kv heads at tp = 8
     assert (s.Hq_local, s.Hkv_local) == (8, 1) and s.q_heads == slice(24, 32) and s.kv_heads == slice(3, 4)
     assert s.cache_bytes_per_block(16, 128, 2) == 2 * 16 * 128 * 2
     for bad in [(3, 0, 64, 8), (2, 2, 64, 8), (2, 0, 30, 8)]:

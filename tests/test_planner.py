@@ -10,10 +10,10 @@ def plan(lens, Hq=32, Hkv=8):
 
 
 def test_uniform_large_batches_take_the_single_pass_grid():
-    assert plan([4096] * 64) == 1                 # 512 items on 296 CTA slots
-    assert plan([8192] * 128) == 1                # configs[2]
-    assert plan([8192] * 256, 64, 8) == 1         # configs[3], tp = 1
-    assert plan([8192] * 256, 8, 1) == 1          # configs[3] at tp = 8: 256 equal items fill 86 % of one wave (measured
+    assert plan([4096] * 64) == 1                 # the headline: 512 items on 296 CTA slots
+    assert plan([8192] * 128) == 1                # 128 x 8k, fp8
+    assert plan([8192] * 256, 64, 8) == 1         # 64 q / 8 kv heads
+    assert plan([8192] * 256, 8, 1) == 1          # one of 8 ranks: 256 equal items fill 86 % of one wave (measured
                                                   # 6.7 TB/s single pass vs 6.1 dynamic)
     KV_FP8 = b200attn.KV_FP8_E4M3
     lens = torch.tensor([8192] * 128, dtype=torch.int32)
@@ -21,7 +21,7 @@ def test_uniform_large_batches_take_the_single_pass_grid():
 
 
 def test_small_or_skewed_batches_take_the_dynamic_schedule():
-    assert plan([512] * 4, 8, 2) == 0             # configs[0]: 8 items
+    assert plan([512] * 4, 8, 2) == 0             # 8 items
     assert plan([8192] * 100, 8, 1) == 0          # 100 items on 296 slots: a third of the SMs would idle
     assert plan([32768] + [200] * 63) == 0        # one long prompt among short ones
     assert plan(list(range(100, 6500, 100))) == 0
@@ -29,7 +29,7 @@ def test_small_or_skewed_batches_take_the_dynamic_schedule():
 
 def test_ragged_serving_batches_take_the_dynamic_schedule():
     """log-uniform 128..ctx lengths: the per-item pipeline ramp of the single-pass grid costs more than the dynamic
-    schedule's ~4 % (measured +9 % / +7 % for configs[3] / configs[1] shapes, bench.py --ragged)."""
+    schedule's ~4 % (measured +9 % / +7 % at 256 x 8k and 64 x 4k, bench.py --ragged)."""
     import math
     g = torch.Generator().manual_seed(1234)
     for B, ctx, Hq, Hkv in ((256, 8192, 64, 8), (64, 4096, 32, 8)):

@@ -165,7 +165,7 @@ def test_repeated_preemption_of_the_same_request():
 
 
 def test_request_that_outgrows_the_whole_pool_ends_by_length_instead_of_livelocking():
-    """ADVICE r1: 4 blocks of 16, prompt 40, 100 new tokens -- alone in the running set the request used to be
+    """4 blocks of 16, prompt 40, 100 new tokens -- alone in the running set the request used to be
     preempted, recomputed and preempted again for ever (175 preemptions in 200 steps, generated stuck at 25).
     Its budget is now cut to what the pool can hold (64 cached tokens = 40 + 25 - 1) and it finishes by length."""
     s = make(4, 16, 2, 4096, 64)
@@ -188,7 +188,7 @@ def test_request_that_outgrows_the_whole_pool_ends_by_length_instead_of_livelock
 
 
 def test_memory_pressure_does_not_thrash_preempted_requests():
-    """ADVICE r1: 8 requests (prompts ~100 tokens, 400 new tokens) on a 64-block pool.  A victim used to be re-admitted
+    """8 requests (prompts ~100 tokens, 400 new tokens) on a 64-block pool.  A victim used to be re-admitted
     in the very step that preempted it, on the blocks it had just freed, and be evicted again at the next block
     boundary: 171 preemptions and 26 176 prefill tokens scheduled for 908 prompt tokens.  Now a step that preempts
     admits nothing, and a preempted request returns only when its whole recompute fits."""

@@ -290,7 +290,7 @@ def test_process_template_placeholders():
 
 
 def test_chat_uses_the_models_own_template_when_the_tokenizer_ships_one(tmp_path):
-    """ADVICE r1: /v1/chat/completions must prompt instruct weights with THEIR chat template (tokenizer_config.json),
+    """/v1/chat/completions must prompt instruct weights with THEIR chat template (tokenizer_config.json),
     not a hard-coded format; the byte tokenizer (random-init weights) has none and keeps the plain fallback."""
     import json
     from tokenizers import Tokenizer, models, pre_tokenizers

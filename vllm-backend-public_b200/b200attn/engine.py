@@ -6,7 +6,7 @@ state slot per live sequence (alloc_state); the scheduler hands out blocks, cach
 
 This is the process the reference deploys and probes (reference benchmark-vllm/vllm_manager.py:371-374,
 888-983); its limits are the launch parameters of `VLLMConfig` (reference benchmark-vllm/models.py:8-15):
-max_num_seqs, max_model_len, block_size, gpu_memory_utilization.  SURVEY.md section 8(f) ranks 1-3.
+max_num_seqs, max_model_len, block_size, gpu_memory_utilization.
 
 Per step:  plan = scheduler.step()  (decode rows first, then prompt chunks within the token budget)
   * decode-only plan  -> one CUDA-graph replay per (batch bucket, schedule): H2D of the step's int32/int64 rows from

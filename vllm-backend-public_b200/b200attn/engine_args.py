@@ -1,4 +1,4 @@
-"""Launch contract of the engine process (SURVEY.md section 8(b) boundary b1).
+"""Launch contract of the engine process.
 
 The reference describes an engine by `VLLMConfig` (reference benchmark-vllm/models.py:5-31) and starts it with the
 argument vector built in reference benchmark-vllm/vllm_templates.py:50-87 (StatefulSet) / :221-258 (Deployment), or

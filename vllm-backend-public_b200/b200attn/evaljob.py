@@ -1,4 +1,4 @@
-"""The evaluation-job side of the reference's loop, without Kubernetes (SURVEY.md section 8(f) rank 4).
+"""The evaluation-job side of the reference's loop, without Kubernetes.
 
 benchmark-eval renders a Job template by literal placeholder replacement and hands the YAML to benchmark-deployer,
 which creates a Kubernetes Job whose container talks to the engine (reference benchmark-eval/main.py:55-58,108-127;

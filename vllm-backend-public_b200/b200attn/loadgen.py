@@ -1,4 +1,4 @@
-"""Benchmark client: what a reference benchmark Job does to an engine (SURVEY.md section 8(f) rank 4).
+"""Benchmark client: what a reference benchmark Job does to an engine.
 
 It is the container side of `benchmark-deployer /run`: the engine URL arrives as env `VLLM_MODEL_ENDPOINT`
 (reference benchmark-deployer/deployer_manager.py:2195-2199, e.g. http://host:8000/v1/completions), an optional JSON
@@ -8,7 +8,7 @@ POSTed as `EvaluationPayload` (reference benchmark-results/models.py:6-19) to `{
 `{results}/standardized_output` (reference benchmark-results/main.py:55-63), whose primary key is
 f"{timestamp}-{benchmark_name}-{run_id}" (reference benchmark-results/results_manager.py:22).
 
-Workload (BASELINE.json configs[4]): `num_requests` prompts with lengths drawn log-uniformly from
+Workload: `num_requests` prompts with lengths drawn log-uniformly from
 [min_prompt, max_prompt] tokens (seed 0), sent as token-id prompts, `max_tokens` each, at most `concurrency` in
 flight, streamed so TTFT and inter-token latency are measured at the client.
 

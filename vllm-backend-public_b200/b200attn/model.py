@@ -1,4 +1,4 @@
-"""Llama-family decoder on the b200attn ops (SURVEY.md section 8(f) rank 3): the caller of the hot path.
+"""Llama-family decoder on the b200attn ops: the caller of the hot path.
 
 What the engine launched by the reference (reference benchmark-vllm/vllm_manager.py:371-374, flags from
 benchmark-vllm/vllm_templates.py:50-87) computes for every scheduled token.  The projections are plain library
@@ -6,7 +6,7 @@ GEMMs (torch.matmul -> cuBLAS); everything between them is this repo's sm_100a k
 b2_rms_norm (fused residual add), b2_rope_and_cache (rotary + KV write in one pass over the fused QKV rows),
 b2_paged_decode / b2_prefill_attention, b2_silu_and_mul, b2_sample.  There is no CPU path.
 
-Weights: random-init from a seed (BASELINE.json configs[4] is random-init; the box has no network), or a local
+Weights: random-init from a seed, or a local
 HF directory (config.json + *.safetensors) when `model` is a path.  Geometry comes from the registry below or
 from that config.json.  head_dim must be 128 (what the attention kernels are built for).
 """

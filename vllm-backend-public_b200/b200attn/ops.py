@@ -421,7 +421,7 @@ class DecodePlan:
 
 
 # ------------------------------------------------------------------------------------------------
-# prompt-chunk attention and the element-wise ops of a decoder layer
+# Prompt-chunk attention and the element-wise ops of a decoder layer
 # ------------------------------------------------------------------------------------------------
 def dequant_kv_blocks(k_cache: torch.Tensor, v_cache: torch.Tensor, src_blocks: torch.Tensor,
                       k_out: Optional[torch.Tensor] = None, v_out: Optional[torch.Tensor] = None):

@@ -1,4 +1,4 @@
-"""KV-head sharding across the GPUs of one box (SURVEY.md section 8(e)).
+"""KV-head sharding across the GPUs of one box.
 
 `tensor_parallel_size` comes from the reference's launch contract (reference benchmark-vllm/models.py:11 ->
 `--tensor-parallel-size`, benchmark-vllm/vllm_templates.py:55).  One process per GPU (torchrun), rank r of tp owns
@@ -74,7 +74,7 @@ def from_env(Hq: int, Hkv: int) -> HeadShard:
 
 def gather_heads(out_local: torch.Tensor, shard: HeadShard, group: Optional[dist.ProcessGroup] = None) -> torch.Tensor:
     """All-gather [B, Hq/tp, d] over the ranks -> [B, Hq, d] (head axis in rank order).  4 MiB in total at
-    BASELINE configs[3]; microseconds over NVLink 5 / NVSwitch, and off the attention path."""
+    256 rows; microseconds over NVLink 5 / NVSwitch, and off the attention path."""
     if shard.tp == 1:
         return out_local
     B, Hl, d = out_local.shape

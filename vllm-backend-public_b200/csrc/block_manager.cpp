@@ -1,5 +1,4 @@
-// block_manager.cpp -- host side of libb200attn.so: error text + the KV page allocator
-// (SURVEY.md section 8(a) row a9, section 8(f) rank 1).
+// block_manager.cpp -- host side of libb200attn.so: error text + the KV page allocator.
 //
 // The reference never allocates KV pages itself; it passes the knobs that size the pool to the
 // engine it launches: block_size (reference benchmark-vllm/models.py:10), max_num_seqs (:9),

@@ -1,5 +1,4 @@
-// comm.cu -- tensor-parallel exchange of one decoder layer over NVLink peer memory (SURVEY.md section 8 rows a4 / e:
-// `--tensor-parallel-size N`, reference benchmark-vllm/models.py:11 -> vllm_templates.py:55,226).
+// comm.cu -- tensor-parallel exchange of one decoder layer over NVLink peer memory (`--tensor-parallel-size N`, reference benchmark-vllm/models.py:11 -> vllm_templates.py:55,226).
 //
 // With the heads (and the MLP columns) sharded over tp GPUs, `o_proj` and `down_proj` are row-parallel: every rank
 // holds a PARTIAL [T, hidden] sum, and the layer needs  h = resid + sum_r partial_r ;  x = RMSNorm(h) * w  next.

@@ -1,5 +1,5 @@
 // model_ops.cu -- the HBM-bound element-wise ops either side of the attention path in one decoder layer
-// (SURVEY.md section 8(f) rank 3: the random-init Llama forward that calls the hot path every step).
+// (the random-init Llama forward that calls the hot path every step).
 //
 //   b2_rms_norm        (optional fused residual add)           vLLM: rms_norm / fused_add_rms_norm
 //   b2_rope_and_cache  neox rotary on q and k in place + KV write through slot_mapping in the same pass

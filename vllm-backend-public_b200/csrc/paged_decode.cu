@@ -1,12 +1,12 @@
 // paged_decode.cu -- paged-attention decode for B200 (sm_100a).
-// SURVEY.md section 8(a) rows a6 (single pass), a7 (split-K + merge), a8 (fp8 dequant in load).
+// Single pass, split-K + merge, fp8 dequant in load.
 //
 // Contract: include/b200attn.h `b2_paged_decode`.  Semantics follow vLLM paged_attention_v1/v2,
 // the op run each decode step by the engine the reference launches
 // (reference benchmark-vllm/vllm_manager.py:371-374); block_size / max_num_seqs / max_model_len
 // come from reference benchmark-vllm/models.py:9,10,15.
 //
-// Design (HBM-bound gather; DESIGN.md section 3):
+// Design (HBM-bound gather):
 //   * One CTA serves all G = Hq/Hkv query heads that share a kv head, so KV bytes are read once
 //     per kv head, not once per q head.  An "item" is one (sequence, kv head [, head group]).
 //   * warp 4 is the producer: it walks the block table and issues ONE TMA box per (block, head)
@@ -1793,7 +1793,7 @@ extern "C" int b2_paged_decode_plan_splits(const int32_t* seq_lens_host, int B, 
     // The ipb items of a sequence are equal and adjacent in grid order: they are placed together on a group of ipb
     // slots (NC / ipb groups), which keeps this at one heap operation per sequence -- it runs on the host every step.
     // (fewer items than slots is not special: 256 equal items on 296 slots stream at 6.7 TB/s in one wave, the
-    // dynamic schedule at 6.1 -- BASELINE configs[3] at tp = 8; the model below rejects the really short grids)
+    // dynamic schedule at 6.1 -- 256 x 8k, 8 q / 1 kv heads a rank; the model below rejects the really short grids)
     const int n_groups = NC / ipb > 0 ? NC / ipb : 1;
     static thread_local std::vector<int64_t> slot;     // min-heap of group finish times (reused: no allocation per step)
     slot.assign((size_t)n_groups, 0);
@@ -1902,7 +1902,7 @@ extern "C" int b2_paged_decode_append(void* out, const void* q, const void* k_ne
 // b2_paged_decode_static: b2_paged_decode for callers that may not allocate (CUDA graph capture, tight serving
 // loops, harnesses that forbid cudaMalloc).  The split-K partials and the claim counter live in a file-scope device
 // array of B2_STATIC_SCRATCH_BYTES that every GPU loading this library holds until exit.  No counterpart in the
-// reference; added at the request of the run's operators.  Nothing here allocates: no cudaMalloc / cudaFree, no
+// reference.  Nothing here allocates: no cudaMalloc / cudaFree, no
 // allocating library call.  Every call on a GPU shares the ONE array (it keeps the previous call's partials; the
 // claim counter is re-zeroed on `stream` by the stateless path, and partials are always written before they are
 // read), so two calls whose kernels overlap on the GPU (different streams) race.

@@ -1,7 +1,7 @@
 // paged_decode_simt.cu -- plain CUDA-core paged-attention decode (no TMA, no tensor cores).
 //
 // Same contract as b2_paged_decode (include/b200attn.h).  This is NOT the product path: it is the
-// "recompiled baseline" variant kept for the ncu A/B comparison in DESIGN.md / profiles/ and as an
+// "recompiled baseline" variant kept for the ncu A/B comparison in profiles/ and as an
 // independent second implementation for the parity tests.  One CTA per (sequence, kv head); each
 // of 8 warps walks tokens warp, warp+8, ...; a lane owns 4 of the 128 head_dim elements, so one
 // warp-wide load is one contiguous token row.  Dot products are reduced with xor-shuffles.

@@ -1,5 +1,5 @@
 // prefill_attention.cu -- causal attention of prompt chunks over the paged KV cache (sm_100a).
-// the step on the other side of the cache (it produces, through
+// The step on the other side of the cache (it produces, through
 // b2_rope_and_cache / b2_reshape_and_cache, the KV the decode kernel reads).
 //
 // Contract: include/b200attn.h `b2_prefill_attention`.  Semantics follow vLLM's chunked-prefill /

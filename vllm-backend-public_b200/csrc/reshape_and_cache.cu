@@ -1,4 +1,4 @@
-// reshape_and_cache.cu -- KV write through slot_mapping (SURVEY.md section 8(a) row a5).
+// reshape_and_cache.cu -- KV write through slot_mapping.
 //
 // Contract: include/b200attn.h `b2_reshape_and_cache`.  Semantics follow vLLM's
 // `reshape_and_cache` (the op the engine launched by reference

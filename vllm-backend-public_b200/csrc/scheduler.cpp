@@ -1,5 +1,5 @@
 // scheduler.cpp -- continuous-batching step planner of libb200attn.so (host only).
-// the caller of the hot path; it decides B and the raggedness every step.
+// The caller of the hot path; it decides B and the raggedness every step.
 //
 // Limits come from the reference's launch contract: max_num_seqs (reference benchmark-vllm/models.py:9),
 // max_model_len (:15), block_size (:10), the pool sized from gpu_memory_utilization (:8).  Policy and the
