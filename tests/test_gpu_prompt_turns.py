@@ -24,6 +24,13 @@ pytestmark = pytest.mark.gpu
     ([640, 500], [5, 31], 32, 8, 128, 128, 16, 0, 0, 0, 1.5, False, 1, False, False, 1.0),                    # scores far above the cap
     ([640, 500], [5, 31], 32, 8, 32, 64, 24, 256, 0, 0, 30.0, True, 1, False, True, -1.0),                    # pages that are no box, a negative scale
     ([640, 500], [5, 31], 32, 8, 128, 64, 16, 0, 150, 0, 0.0, False, 1, True, True, 1.0),
+    # mask blocks, whose tiles are listed by their length: behind contexts, with an empty prompt between, rows in pairs, blocks beyond every prompt, blocks
+    # with a window; more row tiles than the list holds
+    ([700, 0, 1290, 16], [777, 5, 33, 299], 32, 8, 64, 64, 16, 300, 0, 0, 0.0, True, 1, False, False, 1.0),
+    ([1100, 900], [50, 2000], 28, 4, 64, 64, 16, 589, 0, 0, 0.0, False, 1, False, True, 1.0),
+    ([1200, 333], [700, 0], 32, 8, 64, 64, 24, 100000, 0, 0, 0.0, False, 1, True, False, 1.0),
+    ([1500, 600], [130, 0], 32, 8, 64, 64, 16, 700, 260, 9, 0.0, True, 1, False, False, 1.0),
+    ([1100] * 32, [37 * i for i in range(32)], 2, 1, 32, 32, 16, 400, 0, 0, 0.0, False, 1, False, False, 1.0),
 ])
 def test_tiles_in_turns(cuda, c):
     masked_rows(cuda, c)

@@ -28,8 +28,6 @@
 // heads of 128, window 1024, capped 122 -> 107 us, not capped 93.6 -> 77.2; those causal rows 52.8 -> 42.6; 4 x 625 rows x 16 heads of two maps 37.0 ->
 // 30.2; 3500 gathered rows x 16 heads in windows of 300 39.0 -> 34.5; 1000 rows x 32 heads of sigmoid weights 30.8 -> 22.6.
 // What is left of the first steps is fetching code, 9 - 12k cycles to the first scores: which launches are prompt_tc5.cu's, and why, stands there.
-// Mask blocks are walked from their beginning, so their tiles are not in the order of their length: 1424 + 991 rows x 16 behind 777 in blocks of 589 take
-// 36.8 us and 30.0 with a CTA a tile, other sizes (830 + 577 + 817, blocks of 510) 23.0 and 26.7.
 // The forms of two maps spill 12 - 60 bytes a thread, the others nothing.
 // What cost most on the way: an MMA loop with the slot as a variable, whose operands are not uniform to the compiler (3.6k cycles between a
 // softmax and the next instead of 1.3k); the weights in a rolled loop over 32 keys (2.3k cycles instead of 1.5k); stores by a thread a row
@@ -137,8 +135,16 @@ struct Plan {
 struct Prompt {
     int seq, row, len, ctx;                          // first row in q, rows (0: not this kernel's), first position (< 0: padding)
 };
+// In mask blocks a tile's steps go up and down with its place in the block: then they are listed, for as many row tiles as the list holds (more
+// average out).  In the order of their positions, which is none, two long tiles could meet in a CTA; order of positions -> list (a CTA a tile), heads
+// of 128 behind 2000 keys: 666 + 1593 rows x 16, blocks of 1273, 49.4 -> 36.4 us (37.1); 3309 x 16, 1649, 52.8 -> 44.2 (45.0); 3860 x 16, 463, 33.4 -> 27.9
+// (35.5); 298 + 891 x 32, 1946, 45.6 -> 28.7 (27.6); three long portions behind 0, blocks of 947, 29.3 -> 30.4 (33.0).
+constexpr int LISTED = 256;
+template <bool BLOCKS>
 struct TileOrder {
     const b2_prompt_args* a;
+    uint8_t* list;                                   // steps of the row tiles in the order of the batch (at most 255)
+    int n_list, ahead;                               // row tiles listed (0: none are); of the prompts before this lane's
     int shift, cap;                                  // log2 of the rows per tile; windows and mask blocks: steps beyond which tiles cost the same
     int lane, n_long, max_level;
     int from, before;                                // more prompts than lanes: batch of 32 at which the search goes on, row tiles before it
@@ -166,9 +172,11 @@ struct TileOrder {
         return __reduce_add_sync(0xffffffffu, ((mine.len + (1 << shift) - 1) >> shift) - first_at(L, mine));
     }
     // rows, heads: of a tile; both become those of one slot where the batch turns out to hold no more tiles of one slot than there are CTAs
-    __device__ __forceinline__ void init(const b2_prompt_args& args, int& rows, int& heads, int ln) {
+    __device__ __forceinline__ void init(const b2_prompt_args& args, uint8_t* s_list, int& rows, int& heads, int ln) {
         a = &args;
+        list = s_list;
         lane = ln;
+        n_list = 0;
         n_long = 0;
         mine = {0, 0, 0, 0};
         int level = 1;
@@ -202,9 +210,70 @@ struct TileOrder {
         from = before = 0;
         if (n_long > 32) cap = max_level = 1;        // one level: in the order of the batch
         else if (total(1) * (a->H / heads) <= (int)gridDim.x) cap = max_level = 1;       // a tile a CTA in any order
+        else if (BLOCKS && total(1) <= LISTED) make_list();
+    }
+    __device__ __forceinline__ int scan(int n) const {               // inclusive sum over the lanes
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int below = __shfl_up_sync(0xffffffffu, n, d);
+            if (lane >= d) n += below;
+        }
+        return n;
+    }
+    __device__ __forceinline__ void make_list() {
+        const int nt = (mine.len + (1 << shift) - 1) >> shift, upto = scan(nt), prompts = 32 - __clz(__ballot_sync(0xffffffffu, nt > 0));
+        ahead = upto - nt;
+        n_list = __shfl_sync(0xffffffffu, upto, 31);
+        max_level = min(max_level, 255);
+#pragma unroll 1
+        for (int u0 = 0; u0 < n_list; u0 += 32) {
+            int k = 0, ctx = 0, len = 0;             // of the last prompt that begins at or before this lane's tile
+#pragma unroll 1
+            for (int s = 0; s < prompts; ++s) {
+                const int b = __shfl_sync(0xffffffffu, ahead, s), c = __shfl_sync(0xffffffffu, mine.ctx, s), l = __shfl_sync(0xffffffffu, mine.len, s);
+                if (u0 + lane >= b) { k = u0 + lane - b; ctx = max(c, 0); len = l; }
+            }
+            const int q0 = k << shift;
+            if (u0 + lane < n_list) list[u0 + lane] = (uint8_t)min(max_level, ((ctx + q0) % a->chunk + min(len - q0, 1 << shift) + BN - 1) / BN);
+        }
+        __syncwarp();
+    }
+    __device__ __forceinline__ int listed(int L) const {             // row tiles of at least L steps
+        int n = 0;
+#pragma unroll 1
+        for (int u = lane; u < n_list; u += 32) n += list[u] >= L;
+        return __reduce_add_sync(0xffffffffu, n);
+    }
+    __device__ __forceinline__ bool find_listed(int r, Prompt& at, int& q0) const {
+        if (r >= n_list) return false;
+        int lo = 1, hi = max_level + 1;              // listed(lo) > r >= listed(hi) = 0
+#pragma unroll 1
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (listed(mid) > r) lo = mid;
+            else hi = mid;
+        }
+        r -= listed(lo + 1);
+        int u = 0;
+#pragma unroll 1
+        for (;; u += 32) {
+            const uint32_t bits = __ballot_sync(0xffffffffu, u + lane < n_list && list[u + lane] == lo);
+            if (r < __popc(bits)) {
+                u += __ffs(__ballot_sync(0xffffffffu, (bits >> lane & 1) && __popc(bits & ((1u << lane) - 1)) == r)) - 1;
+                break;
+            }
+            r -= __popc(bits);
+        }
+        const int nt = (mine.len + (1 << shift) - 1) >> shift;
+        const int who = __ffs(__ballot_sync(0xffffffffu, u >= ahead && u < ahead + nt)) - 1;
+        at = {__shfl_sync(0xffffffffu, mine.seq, who), __shfl_sync(0xffffffffu, mine.row, who), __shfl_sync(0xffffffffu, mine.len, who),
+              __shfl_sync(0xffffffffu, mine.ctx, who)};
+        q0 = (u - __shfl_sync(0xffffffffu, ahead, who)) << shift;
+        return true;
     }
     // row tile of rank r: its prompt and first row in it (false: there are no more)
     __device__ __forceinline__ bool find(int r, Prompt& at, int& q0) {
+        if (BLOCKS && n_list > 0) return find_listed(r, at, q0);
         int lo = 1, hi = max_level + 1;              // total(lo) > r >= total(hi) = 0
         if (n_long <= 32) {
             if (r >= total(1)) return false;
@@ -222,12 +291,7 @@ struct TileOrder {
         for (int b = from; b < batches(); ++b) {
             const Prompt p = load(b);
             const int first = first_at(lo, p), n = first_at(lo + 1, p) - first;
-            int upto = n;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int below = __shfl_up_sync(0xffffffffu, upto, d);
-                if (lane >= d) upto += below;
-            }
+            const int upto = scan(n);
             const uint32_t hit = __ballot_sync(0xffffffffu, r < upto);
             if (hit) {
                 const int who = __ffs(hit) - 1;
@@ -282,7 +346,7 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
                  : "r"(taddr));
 }
 
-template <int NH, int DVH, int KIND, bool TWO_MAPS, bool GATHERED, bool GATE_COLUMNS>
+template <int NH, int DVH, int KIND, bool TWO_MAPS, bool GATHERED, bool GATE_COLUMNS, bool BLOCKS>
 __global__ void __launch_bounds__(NTHREADS, 1)
 prompt_turns_kernel(const __grid_constant__ Params prm) {
     using L = Shape<NH, DVH, TWO_MAPS>;
@@ -292,6 +356,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
     __shared__ Plan s_plan[2];
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed;
+    __shared__ uint8_t s_list[BLOCKS ? LISTED : 1];
     __shared__ float s_alpha[2][BM], s_inv[2][BM];                   // softmax -> output warps: factor of O, 1 / denominator
     const b2_prompt_args& a = prm.a;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -322,7 +387,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(b2::smem_u32(&s_tmem)) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    TileOrder order;
+    TileOrder<BLOCKS> order;
     // The plan warp comes to this barrier with its first plan in hand, made while the others set up what it does not need.
     auto meet = [] { asm volatile("bar.sync 2, 512;" ::: "memory"); };
     static_assert(NTHREADS == 512, "the barrier's threads");
@@ -356,7 +421,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
                 if (GATHERED && a.dk0 < a.dk) b2::tma_prefetch_desc(&prm.map_q1);
             }
             int tile_rows = prm.rows_per_cta, hpc = prm.heads_per_cta;
-            order.init(a, tile_rows, hpc, lane);
+            order.init(a, s_list, tile_rows, hpc, lane);
             const uint32_t groups = (uint32_t)(a.H / hpc);
             int t = 0;                                               // tiles published
 #pragma unroll 1
@@ -1082,7 +1147,7 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
     }
     if (*failed) {                                                   // a wait gave up: every row of this CTA's tiles is NaN
         int tile_rows = prm.rows_per_cta, hpc = prm.heads_per_cta;
-        order.init(a, tile_rows, hpc, lane);
+        order.init(a, s_list, tile_rows, hpc, lane);
         const uint32_t groups = (uint32_t)(a.H / hpc);
 #pragma unroll 1
         for (uint32_t turn = 0;; ++turn) {
@@ -1102,7 +1167,9 @@ prompt_turns_kernel(const __grid_constant__ Params prm) {
 
 template <int NH, int DVH, int KIND, bool TWO_MAPS, bool GATHERED, bool GATE_COLUMNS = false>
 int launch(const Params& p, dim3 grid, cudaStream_t st) {
-    auto kern = prompt_turns_kernel<NH, DVH, KIND, TWO_MAPS, GATHERED, GATE_COLUMNS>;
+    auto kern = prompt_turns_kernel<NH, DVH, KIND, TWO_MAPS, GATHERED, GATE_COLUMNS, false>;
+    if constexpr (!GATHERED)                         // instances of their own: the list's code would cost all others 0.3 us
+        if (p.a.chunk > 0) kern = prompt_turns_kernel<NH, DVH, KIND, TWO_MAPS, GATHERED, GATE_COLUMNS, true>;
     constexpr int smem = Shape<NH, DVH, TWO_MAPS>::SMEM;
     B2_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     kern<<<grid, NTHREADS, smem, st>>>(p);
